@@ -9,6 +9,8 @@ from __future__ import annotations
 import ctypes as C
 import os
 
+import torch  # noqa: F401  (before _native, which uses its libraries)
+
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libtc_attn.so")
 
@@ -230,6 +232,11 @@ def load(path: str = LIB_PATH) -> C.CDLL:
 
 
 lib = load()
+try:
+    from . import _native as native  # noqa: E402  (links against libtc_attn.so: after it)
+except ImportError as e:
+    raise ImportError("_native.so is missing or does not fit the installed torch: build it with "
+                      "`python -c 'import __graft_entry__ as g; g.build()'`.  There is no fallback path.") from e
 
 
 def check(code: int) -> None:

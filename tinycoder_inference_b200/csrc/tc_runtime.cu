@@ -76,25 +76,46 @@ static EncodeTiledFn encodeFn() {
 }
 
 struct CacheEntry {
-    int dev;
+    int dev;  // -1: empty
     TensorMapKey key;
     CUtensorMap map;
 };
 
-// The cache is a fixed ring (no heap growth): entry points that promise not to
-// allocate go through here too.
+// The cache is a fixed table (no heap growth: entry points that promise not to allocate go through here
+// too), set-associative by a hash of the key.  A program holds one map per pool and layer -- 64 layers of K and
+// V at a time -- and a call looks up two to four of them: scanning a list of 256 keys took 0.5 to 2 us of
+// every launch, and programs with more maps than that re-encoded them on every call.
+constexpr uint32_t kMapSets = 512, kMapWays = 4;
+struct CacheSet {
+    CacheEntry way[kMapWays] = {{-1, {}, {}}, {-1, {}, {}}, {-1, {}, {}}, {-1, {}, {}}};
+    uint32_t next = 0;
+};
+
+static uint32_t mapSet(const TensorMapKey &key, int dev) {
+    static_assert(sizeof(TensorMapKey) % 8 == 0, "hashed in 64-bit words");
+    uint64_t w[sizeof(TensorMapKey) / 8], h = 0x9e3779b97f4a7c15ull + static_cast<uint64_t>(dev);
+    std::memcpy(w, &key, sizeof(key));
+    for (uint64_t x : w) {
+        h = (h ^ x) * 0xff51afd7ed558ccdull;
+        h ^= h >> 32;
+    }
+    return static_cast<uint32_t>(h % kMapSets);
+}
+
 int getTensorMap(const TensorMapKey &key, CUtensorMap *out) {
     static std::mutex mu;
-    constexpr int kSlots = 256;
-    static CacheEntry cache[kSlots];
-    static int used = 0, next = 0;
+    static CacheSet *cache = [] {
+        static CacheSet sets[kMapSets];
+        return sets;
+    }();
     int dev = 0;
     cudaGetDevice(&dev);
+    CacheSet &set = cache[mapSet(key, dev)];
     {
         std::lock_guard<std::mutex> lk(mu);
-        for (int i = 0; i < used; ++i) {
-            if (cache[i].dev == dev && std::memcmp(&cache[i].key, &key, sizeof(key)) == 0) {
-                *out = cache[i].map;
+        for (const CacheEntry &e : set.way) {
+            if (e.dev == dev && std::memcmp(&e.key, &key, sizeof(key)) == 0) {
+                *out = e.map;
                 return TC_OK;
             }
         }
@@ -124,12 +145,11 @@ int getTensorMap(const TensorMapKey &key, CUtensorMap *out) {
     TC_REQUIRE(r == CUDA_SUCCESS, TC_ECUDA, "cuTensorMapEncodeTiled failed with CUresult %d", (int) r);
     {
         std::lock_guard<std::mutex> lk(mu);
-        CacheEntry &e = cache[next];
+        CacheEntry &e = set.way[set.next];
         e.dev = dev;
         e.key = key;
         e.map = m;
-        next = (next + 1) % kSlots;
-        if (used < kSlots) ++used;
+        set.next = (set.next + 1) % kMapWays;
     }
     *out = m;
     return TC_OK;

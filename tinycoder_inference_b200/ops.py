@@ -2,6 +2,8 @@
 
 torch is used for device memory and streams only; every call goes through
 libtc_attn.so.  Tensors must live on the current CUDA device and be contiguous.
+Launching calls go through `_native` (csrc/python/native.cpp), which reads the
+tensors' addresses and the current stream in C++; host-only calls use ctypes.
 """
 from __future__ import annotations
 
@@ -11,7 +13,7 @@ import math
 import torch
 
 from . import capi
-from .capi import check, lib
+from .capi import check, lib, native as _n
 
 
 def _ptr(t):
@@ -42,33 +44,30 @@ def kv_quantize_i8(k, v, k8, v8, ks, vs, tokens, nKV, hd, dst_base=0, src_base=0
     """k, v f32 [rows][nKV][hd] -> rows dst_base.. of the int8 pool k8/v8 + scales ks/vs."""
     if max_rows is None:
         max_rows = k8.numel() // (nKV * hd)
-    check(lib.tc_kv_quantize_i8(_ptr(k), _ptr(v), _ptr(k8), _ptr(v8), _ptr(ks), _ptr(vs), tokens, nKV, hd,
-                                dst_base, src_base, _ptr(dev_dst_base), max_rows, _stream()))
+    check(_n.kv_quantize_i8(k, v, k8, v8, ks, vs, tokens, nKV, hd, dst_base, src_base, dev_dst_base, max_rows))
 
 
 def kv_quantize_i8_batch(k, v, k8, v8, ks, vs, batch, nKV, hd, rows_per_seq=0, row_base=None, pos=0, lens=None,
                          len_add=0, total_rows=None):
     """The new token of every sequence of a batch into one pool, one launch."""
     total = k8.numel() // (nKV * hd) if total_rows is None else total_rows
-    check(lib.tc_kv_quantize_i8_batch(_ptr(k), _ptr(v), _ptr(k8), _ptr(v8), _ptr(ks), _ptr(vs), batch, nKV, hd,
-                                      rows_per_seq, _ptr(row_base), pos, _ptr(lens), len_add, total, _stream()))
+    check(_n.kv_quantize_i8_batch(k, v, k8, v8, ks, vs, batch, nKV, hd, rows_per_seq, row_base, pos, lens, len_add,
+                                  total))
 
 
 def kv_append(kSrc, vSrc, kDst, vDst, seqLen, nKV, hd, cachePos, dev_pos=None, max_rows=None):
     half = kDst.dtype == torch.float16
     if max_rows is None:
         max_rows = kDst.numel() // (nKV * hd)
-    check(lib.tc_kv_append(_ptr(kSrc), _ptr(vSrc), _ptr(kDst), _ptr(vDst), int(half), seqLen, nKV, hd, cachePos,
-                           _ptr(dev_pos), max_rows, _stream()))
+    check(_n.kv_append(kSrc, vSrc, kDst, vDst, int(half), seqLen, nKV, hd, cachePos, dev_pos, max_rows))
 
 
 def kv_append_rope(q, kSrc, vSrc, kDst, vDst, seqLen, nHeads, nKV, hd, cachePos, ropePos, cosT, sinT,
                    dev_pos=None):
     half = kDst.dtype == torch.float16
     max_rows = kDst.numel() // (nKV * hd)
-    check(lib.tc_kv_append_rope(_ptr(q), _ptr(kSrc), _ptr(vSrc), _ptr(kDst), _ptr(vDst), int(half), seqLen,
-                                nHeads, nKV, hd, cachePos, ropePos, _ptr(dev_pos), _ptr(cosT), _ptr(sinT),
-                                max_rows, _stream()))
+    check(_n.kv_append_rope(q, kSrc, vSrc, kDst, vDst, int(half), seqLen, nHeads, nKV, hd, cachePos, ropePos, dev_pos,
+                            cosT, sinT, max_rows))
 
 
 def qk_norm_rope(qIn, qOut, k, wq, wk, hd, nDims, nHeads, nKV, seqLen, pos, cosT, sinT, dev_pos=None,
@@ -76,8 +75,8 @@ def qk_norm_rope(qIn, qOut, k, wq, wk, hd, nDims, nHeads, nKV, seqLen, pos, cosT
     """Per-head RMSNorm of q (out of place, rows of stride q_in_stride) and k (in place) + partial rotation."""
     stride = (2 * hd if q_in_stride is None else q_in_stride) if qIn is not None else 0
     rows = cosT.numel() // max(1, nDims // 2)
-    check(lib.tc_qk_norm_rope(_ptr(qIn), stride, _ptr(qOut), _ptr(k), _ptr(wq), _ptr(wk), hd, nDims, nHeads, nKV,
-                              seqLen, pos, _ptr(dev_pos), _ptr(cosT), _ptr(sinT), rows, _stream()))
+    check(_n.qk_norm_rope(qIn, stride, qOut, k, wq, wk, hd, nDims, nHeads, nKV, seqLen, pos, dev_pos, cosT, sinT,
+                          rows))
 
 
 def rope_tables(rows, headDim, theta):
@@ -98,7 +97,7 @@ def mrope_tables(rows, nDims, thetaBase):
 
 
 def rope_q(q, cosT, sinT, seqLen, nHeads, hd, pos, dev_pos=None):
-    check(lib.tc_rope_q(_ptr(q), _ptr(cosT), _ptr(sinT), seqLen, nHeads, hd, pos, _ptr(dev_pos), _stream()))
+    check(_n.rope_q(q, cosT, sinT, seqLen, nHeads, hd, pos, dev_pos))
 
 
 # ---- decode -------------------------------------------------------------------
@@ -126,9 +125,8 @@ def decode_i8(q, k8, v8, ks, vs, out, ws, nHeads, nKV, hd, cachePos, numChunks, 
         invSqrt = 1.0 / math.sqrt(hd)
     total_rows = k8.numel() // (nKV * hd)
     pAcc, pM, pL = ws
-    check(lib.tc_attn_decode_i8(_ptr(q), _ptr(k8), _ptr(v8), _ptr(ks), _ptr(vs), _ptr(out), _ptr(pAcc),
-                                _ptr(pM), _ptr(pL), nHeads, nKV, hd, cachePos, _ptr(dev_pos), total_rows,
-                                numChunks, chunkSize, invSqrt, _stream()))
+    check(_n.decode_i8(q, k8, v8, ks, vs, out, pAcc, pM, pL, nHeads, nKV, hd, cachePos, dev_pos, total_rows,
+                       numChunks, chunkSize, invSqrt))
 
 
 def decode_i8_noalloc(q, k8, v8, ks, vs, out, nHeads, nKV, hd, cachePos, invSqrt=None):
@@ -137,8 +135,7 @@ def decode_i8_noalloc(q, k8, v8, ks, vs, out, nHeads, nKV, hd, cachePos, invSqrt
     if invSqrt is None:
         invSqrt = 1.0 / math.sqrt(hd)
     total_rows = k8.numel() // (nKV * hd)
-    check(lib.tc_attn_decode_i8_noalloc(_ptr(q), _ptr(k8), _ptr(v8), _ptr(ks), _ptr(vs), _ptr(out), nHeads, nKV,
-                                        hd, cachePos, total_rows, invSqrt, _stream()))
+    check(_n.decode_i8_noalloc(q, k8, v8, ks, vs, out, nHeads, nKV, hd, cachePos, total_rows, invSqrt))
 
 
 def decode_i8_batch(q, k8, v8, ks, vs, out, ws, lens, batch, nHeads, nKV, hd, maxLen, numChunks,
@@ -151,31 +148,16 @@ def decode_i8_batch(q, k8, v8, ks, vs, out, ws, lens, batch, nHeads, nKV, hd, ma
     if invSqrt is None:
         invSqrt = 1.0 / math.sqrt(hd)
     pAcc, pM, pL = ws
-    used = C.c_uint32(0)
-    d = capi.DecodeI8Batch()
-    d.q, d.out = q.data_ptr(), out.data_ptr()
-    d.k8, d.v8, d.ks, d.vs = k8.data_ptr(), v8.data_ptr(), ks.data_ptr(), vs.data_ptr()
-    d.pAcc, d.pM, d.pL = pAcc.data_ptr(), pM.data_ptr(), pL.data_ptr()
-    d.lens = lens.data_ptr() if lens is not None else None
-    d.flags = capi.TC_DECODE_PDL if pdl else 0
-    d.prefetchRows = prefetch_rows
-    if next_kv is not None:
-        d.nextK8, d.nextV8 = next_kv[0].data_ptr(), next_kv[1].data_ptr()
     if tickets is not None:      # zeroed uint32 [batch * nKV]: the kernel merges its own partials
         assert tickets.dtype == torch.int32 and tickets.numel() >= batch * nKV
-        d.mergeTickets = tickets.data_ptr()
-    if append is not None:
-        d.appendK, d.appendV = append[0].data_ptr(), append[1].data_ptr()
-    d.rowBase = row_base.data_ptr() if row_base is not None else None
-    d.rowsPerSeq = rows_per_seq
-    d.totalRows = k8.numel() // (nKV * hd)
-    d.batch, d.nHeads, d.nKV, d.hd = batch, nHeads, nKV, hd
-    d.maxLen, d.numChunks = maxLen, numChunks
-    d.invSqrt = invSqrt
-    d.partialsOnly = int(partials_only)
-    d.chunksUsed = C.pointer(used)
-    check(lib.tc_attn_decode_i8_batch(C.byref(d), _stream()))
-    return used.value
+    nextK8, nextV8 = next_kv if next_kv is not None else (None, None)
+    appendK, appendV = append if append is not None else (None, None)
+    used = _n.decode_i8_batch(q, k8, v8, ks, vs, out, pAcc, pM, pL, lens, row_base, nextK8, nextV8, tickets, appendK,
+                              appendV, rows_per_seq, k8.numel() // (nKV * hd), batch, nHeads, nKV, hd, maxLen,
+                              numChunks, invSqrt, int(partials_only), capi.TC_DECODE_PDL if pdl else 0, prefetch_rows)
+    if used < 0:
+        check(-used)
+    return used
 
 
 def decode_kv(q, kvK, kvV, out, ws, seqLen, nHeads, nKV, hd, pos, numChunks, chunkSize=0, invSqrt=None,
@@ -185,19 +167,17 @@ def decode_kv(q, kvK, kvV, out, ws, seqLen, nHeads, nKV, hd, pos, numChunks, chu
     half = kvK.dtype == torch.float16
     total_rows = kvK.numel() // (nKV * hd)
     pAcc, pM, pL = ws
-    check(lib.tc_attn_decode_kv(_ptr(q), _ptr(kvK), _ptr(kvV), _ptr(out), _ptr(pAcc), _ptr(pM), _ptr(pL),
-                                seqLen, nHeads, nKV, hd, pos, _ptr(dev_pos), total_rows, numChunks, chunkSize,
-                                invSqrt, int(half), _ptr(q81), _stream()))
+    check(_n.decode_kv(q, kvK, kvV, out, pAcc, pM, pL, seqLen, nHeads, nKV, hd, pos, dev_pos, total_rows, numChunks,
+                       chunkSize, invSqrt, int(half), q81))
 
 
 def merge_partials(pAcc, pM, pL, out, seqLen, nHeads, numChunks, hd, q81=None):
-    check(lib.tc_attn_merge_partials(_ptr(pAcc), _ptr(pM), _ptr(pL), _ptr(out), seqLen, nHeads, numChunks, hd,
-                                     _ptr(q81), _stream()))
+    check(_n.merge_partials(pAcc, pM, pL, out, seqLen, nHeads, numChunks, hd, q81))
 
 
 def merge_gathered(gathered, out, nHeads, ranks, chunksPerRank, hd):
     """Merge the all-gathered [acc | m | l] blocks of `ranks` context shards."""
-    check(lib.tc_attn_merge_gathered(_ptr(gathered), _ptr(out), nHeads, ranks, chunksPerRank, hd, _stream()))
+    check(_n.merge_gathered(gathered, out, nHeads, ranks, chunksPerRank, hd))
 
 
 def exchange_bytes(nHeads, hd, world):
@@ -243,32 +223,28 @@ def prefill_f16(q, kvK, kvV, out, scratch, seqLen, nHeads, nKV, hd, invSqrt=None
         invSqrt = 1.0 / math.sqrt(hd)
     if kv8 is not None:
         k8, v8, ks, vs = kv8
-        check(lib.tc_attn_prefill_f16_kv8(_ptr(q), _ptr(kvK), _ptr(kvV), _ptr(out), _ptr(scratch),
-                                          scratch.numel() * scratch.element_size(), seqLen, cachePos, nHeads, nKV, hd,
-                                          invSqrt, _ptr(k8), _ptr(v8), _ptr(ks), _ptr(vs),
-                                          cachePos if kv8_row is None else kv8_row, ks.numel() // nKV, _stream()))
+        check(_n.prefill_f16_kv8(q, kvK, kvV, out, scratch, scratch.numel() * scratch.element_size(), seqLen,
+                                 cachePos, nHeads, nKV, hd, invSqrt, k8, v8, ks, vs,
+                                 cachePos if kv8_row is None else kv8_row, ks.numel() // nKV))
         return
-    check(lib.tc_attn_prefill_f16(_ptr(q), _ptr(kvK), _ptr(kvV), _ptr(out), _ptr(scratch),
-                                  scratch.numel() * scratch.element_size(), seqLen, cachePos, nHeads, nKV, hd,
-                                  invSqrt, _stream()))
+    check(_n.prefill_f16(q, kvK, kvV, out, scratch, scratch.numel() * scratch.element_size(), seqLen, cachePos,
+                         nHeads, nKV, hd, invSqrt))
 
 
 def prefill_f16_kvhalf(q, kvK16, kvV16, out, scratch, seqLen, nHeads, nKV, hd, invSqrt=None, cachePos=0):
     """The tcgen05 prefill over an fp16 store (read in place; the scratch holds q's twin only)."""
     if invSqrt is None:
         invSqrt = 1.0 / math.sqrt(hd)
-    check(lib.tc_attn_prefill_f16_kvhalf(_ptr(q), _ptr(kvK16), _ptr(kvV16), _ptr(out), _ptr(scratch),
-                                         scratch.numel() * scratch.element_size(), seqLen, cachePos, nHeads, nKV, hd,
-                                         invSqrt, _stream()))
+    check(_n.prefill_f16_kvhalf(q, kvK16, kvV16, out, scratch, scratch.numel() * scratch.element_size(), seqLen,
+                                cachePos, nHeads, nKV, hd, invSqrt))
 
 
 def prefill_f16_i8(q, k8, v8, ks, vs, out, scratch, seqLen, nHeads, nKV, hd, invSqrt=None, cachePos=0):
     """The tcgen05 prefill over an int8 store whose rows [0, cachePos + seqLen) are written."""
     if invSqrt is None:
         invSqrt = 1.0 / math.sqrt(hd)
-    check(lib.tc_attn_prefill_f16_i8(_ptr(q), _ptr(k8), _ptr(v8), _ptr(ks), _ptr(vs), _ptr(out), _ptr(scratch),
-                                     scratch.numel() * scratch.element_size(), seqLen, cachePos, nHeads, nKV, hd,
-                                     invSqrt, _stream()))
+    check(_n.prefill_f16_i8(q, k8, v8, ks, vs, out, scratch, scratch.numel() * scratch.element_size(), seqLen,
+                            cachePos, nHeads, nKV, hd, invSqrt))
 
 
 def prefill_kv(q, kvK, kvV, out, seqLen, nHeads, nKV, hd, cachePos, invSqrt=None, dev_pos=None):
@@ -276,20 +252,18 @@ def prefill_kv(q, kvK, kvV, out, seqLen, nHeads, nKV, hd, cachePos, invSqrt=None
         invSqrt = 1.0 / math.sqrt(hd)
     half = kvK.dtype == torch.float16
     total_rows = kvK.numel() // (nKV * hd)
-    check(lib.tc_attn_prefill_kv(_ptr(q), _ptr(kvK), _ptr(kvV), _ptr(out), seqLen, nHeads, nKV, hd, cachePos,
-                                 _ptr(dev_pos), total_rows, invSqrt, int(half), _stream()))
+    check(_n.prefill_kv(q, kvK, kvV, out, seqLen, nHeads, nKV, hd, cachePos, dev_pos, total_rows, invSqrt, int(half)))
 
 
 def prefill_i8(q, k8, v8, ks, vs, out, seqLen, nHeads, nKV, hd, cachePos, invSqrt=None, dev_pos=None):
     if invSqrt is None:
         invSqrt = 1.0 / math.sqrt(hd)
     total_rows = k8.numel() // (nKV * hd)
-    check(lib.tc_attn_prefill_i8(_ptr(q), _ptr(k8), _ptr(v8), _ptr(ks), _ptr(vs), _ptr(out), seqLen, nHeads,
-                                 nKV, hd, cachePos, _ptr(dev_pos), total_rows, invSqrt, _stream()))
+    check(_n.prefill_i8(q, k8, v8, ks, vs, out, seqLen, nHeads, nKV, hd, cachePos, dev_pos, total_rows, invSqrt))
 
 
 def sigmoid_gate(attnOut, qGate, seqLen, nHeads, hd):
-    check(lib.tc_attn_sigmoid_gate(_ptr(attnOut), _ptr(qGate), seqLen, nHeads, hd, _stream()))
+    check(_n.sigmoid_gate(attnOut, qGate, seqLen, nHeads, hd))
 
 
 # ---- planner (host) -------------------------------------------------------------
@@ -386,6 +360,7 @@ class KvSession:
         h = C.c_void_p()
         check(lib.tc_kv_session_create(C.byref(cfg), C.byref(h)))
         self.h = h
+        self._s = h.value    # the handle as `_native` takes it
 
     def __del__(self):
         if getattr(self, "h", None):
@@ -393,12 +368,13 @@ class KvSession:
             self.h = None
 
     def clear(self):
-        check(lib.tc_kv_session_clear(self.h, _stream()))
+        check(_n.clear(self._s))
 
     def begin(self, n):
-        pos = C.c_uint32(0)
-        check(lib.tc_kv_session_begin(self.h, n, C.byref(pos)))
-        return pos.value
+        pos = _n.begin(self._s, n)
+        if pos < 0:
+            check(-pos)
+        return pos
 
     def commit(self, n):
         check(lib.tc_kv_session_commit(self.h, n))
@@ -415,6 +391,4 @@ class KvSession:
         return lib.tc_kv_session_rows8(self.h, slot)
 
     def attend(self, slot, q, k, v, out, pos, dev_pos=None, graph_capture=False):
-        seqLen = q.shape[0]
-        check(lib.tc_kv_session_attend(self.h, slot, _ptr(q), _ptr(k), _ptr(v), _ptr(out), seqLen, pos, _ptr(dev_pos),
-                                       int(graph_capture), _stream()))
+        check(_n.attend(self._s, slot, q, k, v, out, pos, dev_pos, graph_capture))
