@@ -21,11 +21,20 @@ namespace tc {
 
 constexpr int kNormMaxPer = 4;  // elements per reference thread: hd <= 512
 
+// What bounds it: latency for a token (18 slices of a 16 + 2 head model), HBM for prompts.  Every load of a lane --
+// its elements, the norm weights, the table row -- is requested before the first one is used, and with the
+// rotated half a multiple of 32 (HB = half / 32) an element's partner sits in the same lane, HB registers further on.
+// (16 + 2 heads of 256, in a graph: 1 row 1.3 us, 333 rows 2.8, 4096 rows 26.4; with partners, weights and table
+// entries fetched behind the reduction 3.2, 6.0 and 50.0.)  HB = 0: any other half; partners come from the row
+// again (it is in L1).  PER: 128-element groups of a slice.
+template <int PER, int HB>
 __global__ void __launch_bounds__(256)
 qkNormRopeKernel(const float *__restrict__ qIn, uint32_t qInStride, float *qOut, float *k,
                  const float *__restrict__ wq, const float *__restrict__ wk, uint32_t hd, uint32_t nDims,
                  uint32_t nHeads, uint32_t nKV, uint32_t seqLen, uint32_t pos, const uint32_t *__restrict__ devPos,
                  const float *__restrict__ cosT, const float *__restrict__ sinT) {
+    gridDepWait();
+    gridDepLaunch();
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t slices = (qIn ? nHeads : 0u) + (k ? nKV : 0u);
     const uint64_t idx = static_cast<uint64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -39,59 +48,70 @@ qkNormRopeKernel(const float *__restrict__ qIn, uint32_t qInStride, float *qOut,
     float *op = isQ ? qOut + (static_cast<uint64_t>(s) * nHeads + h) * hd : k + (static_cast<uint64_t>(s) * nKV + h) * hd;
     const float *w = isQ ? wq : wk;
 
-    // element j = lane + 32 i + 128 kk  (reference thread lane + 32 i, its kk-th element)
-    float x[4][kNormMaxPer];
+    // element e of a lane is j = lane + 32 e: e = i + 4 kk is the kk-th element of reference thread lane + 32 i
+    constexpr int E = 4 * PER;
+    float x[E], wv[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const uint32_t j = lane + 32u * e;
+        x[e] = j < hd ? rp[j] : 0.0f;
+        wv[e] = j < hd ? w[j] : 0.0f;
+    }
+    const uint32_t p = (devPos != nullptr ? devPos[0] : pos) + s;
+    const uint32_t half = HB ? HB * 32u : nDims / 2;
+    const float *c = cosT + static_cast<uint64_t>(p) * half;
+    const float *sn = sinT + static_cast<uint64_t>(p) * half;
+    constexpr int kHalfRegs = HB ? HB : 1;
+    float cv[kHalfRegs], sv[kHalfRegs];
+    if (HB) {
+#pragma unroll
+        for (int e = 0; e < kHalfRegs; ++e) cv[e] = c[lane + 32u * e], sv[e] = sn[lane + 32u * e];
+    }
     float a[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         a[i] = 0.0f;
 #pragma unroll
-        for (int kk = 0; kk < kNormMaxPer; ++kk) {
-            const uint32_t j = lane + 32u * i + 128u * kk;
-            x[i][kk] = j < hd ? rp[j] : 0.0f;
-            if (j < hd) a[i] = fmaf(x[i][kk], x[i][kk], a[i]);
-        }
+        for (int kk = 0; kk < PER; ++kk)
+            if (lane + 32u * i + 128u * kk < hd) a[i] = fmaf(x[i + 4 * kk], x[i + 4 * kk], a[i]);
     }
     float sum = (a[0] + a[2]) + (a[1] + a[3]);  // threads 64 apart, then 32 apart
 #pragma unroll
     for (int o = 16; o; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
     sum = __shfl_sync(0xffffffffu, sum, 0);
     const float rms = rsqrtf(sum / static_cast<float>(hd) + 1e-6f);
-    const uint32_t p = (devPos != nullptr ? devPos[0] : pos) + s;
-    const uint32_t half = nDims / 2;
-    const float *c = cosT + static_cast<uint64_t>(p) * half;
-    const float *sn = sinT + static_cast<uint64_t>(p) * half;
-    // The partner of element j sits `half` away: it is fetched from global memory again rather
-    // than shuffled (half is a run-time value; the row was just read and is in L1).  K is
-    // rotated in place, so every read happens before the first write.
-    float y[4][kNormMaxPer];
+    float y[E];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int e = 0; e < E; ++e) y[e] = x[e] * rms * wv[e];
+    if (HB) {
 #pragma unroll
-        for (int kk = 0; kk < kNormMaxPer; ++kk) {
-            const uint32_t j = lane + 32u * i + 128u * kk;
-            y[i][kk] = 0.0f;
+        for (int e = 0; e < HB && e + HB < E; ++e) {
+            const float y0 = y[e], y1 = y[e + HB];
+            y[e] = fmaf(y0, cv[e], -y1 * sv[e]);
+            y[e + HB] = fmaf(y0, sv[e], y1 * cv[e]);
+        }
+    } else {
+        // (K is rotated in place: every read happens before the first write)
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const uint32_t j = lane + 32u * e;
             if (j >= hd) continue;
-            const float yj = x[i][kk] * rms * w[j];
             if (j < half) {
                 const float y1 = rp[j + half] * rms * w[j + half];
-                y[i][kk] = fmaf(yj, c[j], -y1 * sn[j]);
+                y[e] = fmaf(y[e], c[j], -y1 * sn[j]);
             } else if (j < nDims) {
                 const uint32_t j0 = j - half;
                 const float y0 = rp[j0] * rms * w[j0];
-                y[i][kk] = fmaf(y0, sn[j0], yj * c[j0]);
-            } else {
-                y[i][kk] = yj;
+                y[e] = fmaf(y0, sn[j0], y[e] * c[j0]);
             }
         }
-    __syncwarp();
+        __syncwarp();
+    }
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int kk = 0; kk < kNormMaxPer; ++kk) {
-            const uint32_t j = lane + 32u * i + 128u * kk;
-            if (j < hd) op[j] = y[i][kk];
-        }
+    for (int e = 0; e < E; ++e) {
+        const uint32_t j = lane + 32u * e;
+        if (j < hd) op[j] = y[e];
+    }
 }
 
 }  // namespace tc
@@ -120,8 +140,15 @@ extern "C" int tc_qk_norm_rope(const float *qIn, uint32_t qInStride, float *qOut
     }
     const uint64_t warps = static_cast<uint64_t>(seqLen) * ((qIn ? nHeads : 0u) + (k ? nKV : 0u));
     const uint32_t blocks = static_cast<uint32_t>((warps + 7) / 8);
-    tc::qkNormRopeKernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-            qIn, qInStride, qOut, k, wq, wk, hd, nDims, nHeads, nKV, seqLen, pos, devPos, cosT, sinT);
-    TC_CUDA_OK(cudaGetLastError());
-    return TC_OK;
+    // partners in the lane when the rotated half is 1, 2 or 4 x 32 elements (64, 128 or 256 rotated dims)
+    const uint32_t hb = nDims == 64 ? 1u : (nDims == 128 ? 2u : (nDims == 256 ? 4u : 0u));
+    const uint32_t per = hd <= 128 ? 1u : (hd <= 256 ? 2u : 4u);
+    using Kern = decltype(&tc::qkNormRopeKernel<1, 0>);
+    static const Kern kerns[3][4] = {
+            {tc::qkNormRopeKernel<1, 0>, tc::qkNormRopeKernel<1, 1>, tc::qkNormRopeKernel<1, 2>, tc::qkNormRopeKernel<1, 0>},
+            {tc::qkNormRopeKernel<2, 0>, tc::qkNormRopeKernel<2, 1>, tc::qkNormRopeKernel<2, 2>, tc::qkNormRopeKernel<2, 4>},
+            {tc::qkNormRopeKernel<4, 0>, tc::qkNormRopeKernel<4, 1>, tc::qkNormRopeKernel<4, 2>, tc::qkNormRopeKernel<4, 4>}};
+    const Kern kern = kerns[per == 1 ? 0 : (per == 2 ? 1 : 2)][hb == 4 ? 3 : hb];
+    return tc::launchDependent(kern, dim3(blocks), 256, 0, static_cast<cudaStream_t>(stream), 1, qIn, qInStride, qOut, k, wq, wk,
+                               hd, nDims, nHeads, nKV, seqLen, pos, devPos, cosT, sinT);
 }

@@ -61,6 +61,32 @@ int getTensorMap(const TensorMapKey &key, CUtensorMap *out);
 
 #ifdef __CUDACC__
 
+// Launch under programmatic dependent launch: the grid may be scheduled while the one in front of it drains, so
+// the kernel has to call gridDepWait() before it touches anything that grid may have written or may still read --
+// every kernel launched through here does so first thing.  Kernels that write K/V rows call gridDepLaunch() after
+// that wait: a decode launch that requests old rows early (TC_DECODE_PDL) then has at most the kernel right in front of
+// it in flight, as it had when these were plain launches.  (In stream order a dependent launch takes 3.1 - 3.7 us on
+// B200, like this 2.0; as nodes of a graph 1.2 and 0.8.)  cluster: blocks per cluster along x.
+template <typename... P, typename... A>
+int launchDependent(void (*kern)(P...), dim3 grid, uint32_t threads, size_t smem, cudaStream_t st, uint32_t cluster,
+                    const A &...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    TC_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, args...));
+    return TC_OK;
+}
+
 // ---- mbarrier ----------------------------------------------------------------
 constexpr uint32_t kMbarSuspendNs = 20000u;  // upper bound of one hardware-parked poll
 __device__ __forceinline__ uint32_t smemAddr(const void *p) {
