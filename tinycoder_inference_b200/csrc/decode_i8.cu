@@ -6,31 +6,23 @@
 // head), score = dot(q, float(k8)*sk) * invSqrt, online softmax with exp2,
 // out = sum p * float(v8)*sv / sum p.
 //
-// How it is built for B200:
-//   * split-K flash-decoding.  grid = (chunks, kv-head groups, sequences); a CTA
-//     streams one contiguous token range of HPC kv heads and serves ALL q heads
-//     of those kv heads, so every KV byte leaves HBM exactly once.
-//   * KV streaming by TMA (cp.async.bulk.tensor, 128-byte swizzle) from one
-//     producer warp into an mbarrier ring; the per-row scales ride in the same
-//     stage through cp.async.  8 consumer warps, one (kv head, 16-token) tile
-//     each per stage.
-//   * at group 5..7 the dequant+FMA work (2*group flop per KV byte) is beyond the
-//     CUDA cores at HBM speed, so QK^T and PV run on tensor cores
-//     (mma.sync.m16n8k16): int8 is converted to fp16 exactly (prmt + one hsub2),
-//     q and p*sv are carried as fp16 hi+lo pairs (two MMAs, ~22 mantissa bits)
-//     after a power-of-two normalisation, accumulation is f32.  The per-row K
-//     scale is applied to the score column after the MMA, the V scale is folded
-//     into p before it.
-//   * S is produced transposed (tokens x heads) so no MMA row is padding; the
-//     probabilities reach the PV operand layout through movmatrix.trans.
-//   * softmax reductions are warp shuffles; (m, l, acc) partials per chunk go to
-//     the caller's partial buffers in the reference's layout and are merged by
-//     the merge kernel (merge.cu).
-#include "tc_common.cuh"
-#include <cstdlib>
+// This file: the mma.sync form, for head_dim 256 and for causal query rows over the store (head_dim 128 decode is
+// decode_i8_tc.cu's), and the entry points of both.
+//   * decode: a block streams a token range of one kv head and serves ALL its q heads, so every KV byte leaves
+//     HBM exactly once; the split over clusters of blocks and the fold of their results are decode_cluster.cuh's,
+//     and the launch quantises the new token's row itself.
+//   * the warps of a block take tiles of MT x 16 tokens in turn, each with copies (16-byte cp.async) and slots of its
+//     own: a warp spends a microsecond on 16 tokens, HBM half of that for an SM, so it takes many independent warps.
+//   * at group 5..8 the dequant+FMA work (2*group flop per KV byte) is beyond the CUDA cores at HBM speed, so
+//     QK^T and PV run on tensor cores (mma.sync.m16n8k16): int8 is fed as exact fp16 subnormals, q and p*sv are
+//     carried as fp16 hi+lo pairs (two MMAs, ~22 mantissa bits) after a power-of-two normalisation, accumulation
+//     is f32.  The per-row K scale is applied to the score column after the MMA, the V scale is folded into p
+//     before it.
+//   * S is produced transposed (tokens x heads) so no MMA row is padding; the probabilities reach the PV operand
+//     layout through movmatrix.trans.
 #include <mutex>
 
-#include "decode_shared.cuh"
+#include "decode_cluster.cuh"
 
 namespace tc {
 
@@ -44,189 +36,144 @@ struct DecodeI8Params {
     uint64_t rowsPerSeq, totalRows;
     uint32_t lenHost, lenAdd;
     uint32_t nHeads, nKV, group;
-    uint32_t colBase;  // heads mode: the 8 MMA columns are q heads colBase .. colBase + 7 of the kv head
+    uint32_t colBase;  // decode: the 8 MMA columns are q heads colBase .. colBase + 7 of the kv head
     uint32_t chunkTokens, numChunks;
-    uint32_t prefetchRows;  // rows [0, prefetchRows) of a sequence may be read before the dependency wait
+    const float *appendK, *appendV;  // nullable: [batch][nKV][hd] rows to quantise into row len - 1 first
+    uint32_t *k8w, *v8w;             // the pools
+    F32Mirror mir;                   // and the f32 store that gets it verbatim
     // rows mode (causal prefill over the store): the 8 MMA columns of a CTA are 8
     // consecutive query rows of ONE q head instead of the q heads of one kv head;
     // row s attends pool rows [0, cachePos + s].  grid = (1, nHeads, ceil(qRows / 8)).
-    uint32_t rowsMode, qRows, cachePos;
+    uint32_t qRows, cachePos;
     const uint32_t *devPos;
     float invSqrt;
     int directOut;
-    int prefetchNext;  // tmKn / tmVn describe the pools of the next call: pull this block's rows of them into L2
     unsigned int *err;
 };
 
 constexpr int kHD = 128;
 
-// TC_ATTN_LEGACY_DECODE=1 keeps head_dim 128 on the mma.sync kernel (comparison runs)
-static bool forceLegacyDecode() {
-    static const bool v = [] {
-        const char *e = getenv("TC_ATTN_LEGACY_DECODE");
-        return e != nullptr && e[0] == '1';
-    }();
-    return v;
-}
-// MT = 16-row MMA tiles one consumer warp folds per stage: 2 amortises the softmax
-// bookkeeping over 32 tokens (large problems), 1 halves the work quantum so that a
-// small problem still spreads evenly over 148 SMs x 8 warps.
+// MT = 16-row MMA tiles a consumer warp folds at a time: 2 amortises the softmax bookkeeping over 32
+// tokens (causal rows at head_dim 128).
 //
-// A stage holds K then V; each is stored as HD/128 half-tiles of [rows][128 bytes]
-// (the 128-byte swizzle spans exactly one half-row), half-tile h covering dims
-// [128h, 128h + 128).
-template <int HD, int HPC, int NW, int NSTAGE, int MT>
+// Every warp has NS slots for tiles of 16 MT tokens of K and as many of V, each as HD/128 half-tiles of [rows][128 bytes],
+// half-tile h covering dims [128h, 128h + 128); the rows' scales lie behind all slots.
+template <int HD, int NW, int NS, int MT>
 struct DecodeI8Smem {
-    static constexpr int kTokPerWarp = 16 * MT;
-    static constexpr int kRows = NW * kTokPerWarp;       // (token, head) rows per stage
-    static constexpr int T = kRows / HPC;                 // tokens per stage
-    static constexpr int kHalfBytes = kRows * 128;        // one half-tile, all HPC heads
-    static constexpr int kTileBytes = kRows * HD;         // K (or V) bytes per stage, all HPC heads
-    static constexpr int kScaleBytes = kRows * 4;
-    static constexpr int kStageBytes = 2 * kTileBytes + 2 * kScaleBytes;
-    static constexpr int kBarOffset = NSTAGE * kStageBytes;
-    static constexpr int kTotal = kBarOffset + 2 * NSTAGE * 8 + 1024;  // + alignment slack
-    static_assert(kStageBytes % 1024 == 0, "stage must keep 1024-byte alignment for the 128B swizzle");
-    static_assert(T <= 256, "TMA box rows");
+    static constexpr int T = 16 * MT;
+    static constexpr int kHalfBytes = T * 128;            // one half-tile
+    static constexpr int kTileBytes = T * HD;             // K (or V) bytes of a tile
+    static constexpr int kScales = NW * NS * 2 * kTileBytes;   // [warp][slot][K, V][T] floats
+    static constexpr int kSlots = kScales + NW * NS * 2 * T * 4, kScratch = (NW + 1) * (8 * HD + 16) * 4;  // (the fold reuses the slots)
+    static constexpr int kTotal = (kSlots > kScratch ? kSlots : kScratch) + 128;
+    static_assert(kTotal <= 227 * 1024, "shared memory of an SM");
 };
 
 // How far the running reference point of the softmax may lag behind the true
 // maximum (log2 units) before the accumulators are rescaled.  p stays <= 2^8.
 constexpr float kLazyLog2 = 8.0f;
-// Stages a producer may request before the grids it depends on have completed.
-constexpr uint32_t kEarlyStages = 1;
 
-template <int HD, int HPC, int NW, int NSTAGE, int MT>
-__global__ void __launch_bounds__((NW + 1) * 32, 1)
-decodeI8Kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
-               const __grid_constant__ CUtensorMap tmKn, const __grid_constant__ CUtensorMap tmVn,
-               const DecodeI8Params p) {
-    using L = DecodeI8Smem<HD, HPC, NW, NSTAGE, MT>;
+// What a launch does: a token's q heads over chunks of the store; causal query rows; or a token's q heads with the
+// accumulation order of the causal form -- tile j of the store belongs to stream j % 8, a stream's tiles are folded one
+// after the other -- each stream a block (one warp) of an 8-block cluster per kv head.
+enum class I8Mode { kChunks, kRows, kStreams };
+
+template <int HD, int NW, int NS, int MT, I8Mode MODE>
+__global__ void __launch_bounds__(NW * 32, MODE == I8Mode::kChunks && NW <= 4 ? 2 : 1)
+decodeI8Kernel(const __grid_constant__ DecodeI8Params p) {
+    using L = DecodeI8Smem<HD, NW, NS, MT>;
+    constexpr bool ROWS = MODE == I8Mode::kRows, STREAMS = MODE == I8Mode::kStreams;
     constexpr int T = L::T;
     constexpr int NC = HD / 16;  // 16-dim groups of a head vector
-    constexpr int kTokPerWarp = L::kTokPerWarp;
     constexpr int NR = 2 * MT;  // 8-token row groups of a warp's tile
-    constexpr int NSUB = NW / HPC;  // consumer warps per kv head
     constexpr float k2p24 = 16777216.0f;
 
     const uint32_t chunk = blockIdx.x, hg = blockIdx.y, b = blockIdx.z;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
 
     extern __shared__ uint8_t smemRaw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
-    uint64_t *fullBar = reinterpret_cast<uint64_t *>(smem + L::kBarOffset);
-    uint64_t *emptyBar = fullBar + NSTAGE;
+    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smemRaw) + 127) & ~uintptr_t(127));
 
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < NSTAGE; ++s) {
-            mbarInit(&fullBar[s], 1 + 32);
-            mbarInit(&emptyBar[s], NW);
-        }
-        fenceBarrierInit();
-        tmaPrefetchDesc(&tmK);
-        tmaPrefetchDesc(&tmV);
-    }
-    __syncthreads();
-    gridDepLaunch();  // the dependent grid (the merge) may be scheduled as soon as room frees up
+    gridDepWait();
+    gridDepLaunch();
 
-    // The length may live in device memory written by an earlier kernel; only a
-    // host-known length lets the producer start before the dependency wait.
-    uint32_t len = p.lenHost;
-    const bool earlyOk = p.devLens == nullptr && p.devRowBase == nullptr && p.prefetchRows != 0 && !p.rowsMode;
-    if (!earlyOk) {
-        gridDepWait();
-        if (p.devLens) len = p.devLens[b] + p.lenAdd;
-    }
-    uint32_t rowsPos = p.cachePos;  // rows mode: first query row sits at pool row rowsPos
-    if (p.rowsMode) {
+    uint32_t len, rowsPos = p.cachePos;  // rows mode: first query row sits at pool row rowsPos
+    if (ROWS) {
         if (p.devPos) rowsPos = p.devPos[0];
-        const uint32_t sEnd = min(p.qRows, b * 8u + 8u);  // b = row block
-        len = rowsPos + sEnd;                             // the block's last row sees [0, rowsPos + sEnd)
+        len = rowsPos + min(p.qRows, b * 8u + 8u);  // b = row block; its last row sees [0, len)
+    } else {
+        // (the host's length is the upper bound of a device length)
+        len = p.devLens ? min(p.devLens[b] + p.lenAdd, p.lenHost) : p.lenHost;
+        // a cluster behind the last row leaves as a whole: the merge derives the active count from len
+        if (!STREAMS && (chunk - clusterRank()) * p.chunkTokens >= len) return;
     }
-    const uint32_t t0 = chunk * p.chunkTokens;
-    if (t0 >= len) return;  // inactive chunk: the merge derives the active count from len
-    const uint32_t t1 = min(len, t0 + p.chunkTokens);
-    const uint32_t nTiles = (t1 - t0 + T - 1) / T;
-    const uint64_t rowBase = p.rowsMode ? 0ull
-                                        : (p.devRowBase ? p.devRowBase[b] : static_cast<uint64_t>(b) * p.rowsPerSeq);
-    // kv heads of this CTA: heads mode streams HPC of them, rows mode the one behind q head `hg`
-    const uint32_t kvHead0 = p.rowsMode ? hg / p.group : hg * HPC;
+    const uint32_t t0 = MODE != I8Mode::kChunks ? 0u : chunk * p.chunkTokens;
+    const uint32_t t1 = MODE != I8Mode::kChunks ? len : min(len, t0 + p.chunkTokens);
+    const uint32_t nTiles = t0 < t1 ? (t1 - t0 + T - 1) / T : 0u;
+    const uint64_t rowBase = ROWS ? 0ull : (p.devRowBase ? p.devRowBase[b] : static_cast<uint64_t>(b) * p.rowsPerSeq);
+    const uint32_t kvHead = ROWS ? hg / p.group : hg;
 
-    if (warp == NW) {
-        // ------------------------------ producer ------------------------------
-        bool waited = !earlyOk;
-        for (uint32_t it = 0; it < nTiles; ++it) {
-            const uint32_t s = it % NSTAGE;
-            if (it >= NSTAGE) {
-                if (!mbarWaitClock(&emptyBar[s], ((it / NSTAGE) - 1) & 1, p.err, kDevErrEmptyWait)) break;
-            }
-            const uint32_t tok = t0 + it * T;
-            if (!waited && (tok + T > p.prefetchRows || it >= kEarlyStages)) {
-                // this tile may hold rows appended by the kernel we depend on -- or it is not
-                // the first one: the kernels ahead (the merge above all) are short and
-                // latency-bound, and a deeper prefetch would put a whole ring of KV loads
-                // in front of theirs in the memory system
-                gridDepWait();
-                waited = true;
-            }
-            uint8_t *st = smem + s * L::kStageBytes;
-            const uint64_t row = rowBase + tok;
-            if (lane == 0) {
-                mbarExpectTx(&fullBar[s], 2 * L::kTileBytes);
-#pragma unroll
-                for (int h = 0; h < HPC; ++h) {
-#pragma unroll
-                    for (int hf = 0; hf < HD / 128; ++hf) {
-                        uint8_t *dst = st + hf * L::kHalfBytes + h * T * 128;
-                        tmaLoad3D(dst, &tmK, &fullBar[s], hf * 128, kvHead0 + h, static_cast<int>(row));
-                        tmaLoad3D(dst + L::kTileBytes, &tmV, &fullBar[s], hf * 128, kvHead0 + h,
-                                  static_cast<int>(row));
-                    }
+    // Tile j belongs to warp (or stream) j % step, its slot (j / step) % NS.  A warp copies its own tiles: with one slot the next
+    // tile's K while it works on this one's V and the next V while it works on K.
+    const uint32_t first = STREAMS ? clusterRank() : warp;
+    constexpr uint32_t step = STREAMS ? 8 : NW;
+    auto slotK = [&](uint32_t i) { return smem + (warp * NS + i % NS) * 2 * L::kTileBytes; };
+    auto scaleK = [&](uint32_t i) { return reinterpret_cast<float *>(smem + L::kScales) + (warp * NS + i % NS) * 2 * T; };
+    const uint32_t stride = p.nKV * HD;
+    const uint8_t *storeK = reinterpret_cast<const uint8_t *>(p.k8w) + static_cast<size_t>(kvHead) * HD;
+    const uint8_t *storeV = reinterpret_cast<const uint8_t *>(p.v8w) + static_cast<size_t>(kvHead) * HD;
+    auto copyScales = [&](float *dst, const float *src, uint64_t row) {
+        if (lane < T) cpAsync4(dst + lane, src + min(row + lane, p.totalRows - 1) * p.nKV + kvHead);
+    };
+    auto requestK = [&](uint32_t i) {
+        const uint32_t j = first + i * step;
+        if (j < nTiles) {
+            if (!ROWS && p.appendK != nullptr && j + 1 == nTiles && t1 == len) {
+                // the tile that holds the new token's row: the row goes in first
+                const uint64_t row = rowBase + (p.devLens ? p.devLens[b] + p.lenAdd : len) - 1u;
+                if (row >= p.totalRows) {  // a device length outside the pool: no row written, and said so
+                    if (lane == 0) atomicOr(p.err, kDevErrRowBound);
+                } else {
+                    const size_t src = (static_cast<size_t>(b) * p.nKV + kvHead) * (HD / 4);
+                    const uint64_t dst = row * p.nKV + kvHead;
+                    float4 *mk = nullptr, *mv = nullptr;
+                    if (p.mir.k != nullptr)
+                        mk = reinterpret_cast<float4 *>(p.mir.k) + dst * (HD / 4), mv = reinterpret_cast<float4 *>(p.mir.v) + dst * (HD / 4);
+                    appendQuantRow<HD>(reinterpret_cast<const float4 *>(p.appendK) + src,
+                                       reinterpret_cast<const float4 *>(p.appendV) + src, p.k8w, p.v8w,
+                                       const_cast<float *>(p.ks), const_cast<float *>(p.vs), dst, mk, mv, lane);
                 }
             }
-            float *sK = reinterpret_cast<float *>(st + 2 * L::kTileBytes);
-            float *sV = sK + L::kRows;
-#pragma unroll
-            for (int idx = lane; idx < L::kRows; idx += 32) {
-                const int h = idx / T, tt = idx % T;
-                uint64_t r = row + tt;
-                r = r < p.totalRows ? r : p.totalRows - 1;
-                cpAsync4(&sK[idx], p.ks + r * p.nKV + kvHead0 + h);
-                cpAsync4(&sV[idx], p.vs + r * p.nKV + kvHead0 + h);
-            }
-            cpAsyncMbarArriveNoinc(&fullBar[s]);
+            const uint64_t row = rowBase + t0 + j * T;
+            copyTile<T, HD>(smemAddr(slotK(i)), storeK, stride, row, p.totalRows - 1, lane);
+            copyScales(scaleK(i), p.ks, row);
         }
-        if (p.prefetchNext && lane == 0) {
-            // This block's own tiles are all requested.  DRAM would now idle through the fold, the
-            // merge and the next call's start-up: have it fetch the same rows of the next call's
-            // pools into L2 meanwhile (the next call's TMA loads then hit L2).
-            for (uint32_t it = 0; it < nTiles; ++it) {
-                const int row = static_cast<int>(rowBase + t0 + it * T);
-#pragma unroll
-                for (int h = 0; h < HPC; ++h)
-#pragma unroll
-                    for (int hf = 0; hf < HD / 128; ++hf) {
-                        tmaPrefetchL2_3D(&tmKn, hf * 128, kvHead0 + h, row);
-                        tmaPrefetchL2_3D(&tmVn, hf * 128, kvHead0 + h, row);
-                    }
-            }
+        cpAsyncCommit();
+    };
+    auto requestV = [&](uint32_t i) {
+        const uint32_t j = first + i * step;
+        if (j < nTiles) {
+            const uint64_t row = rowBase + t0 + j * T;
+            copyTile<T, HD>(smemAddr(slotK(i) + L::kTileBytes), storeV, stride, row, p.totalRows - 1, lane);
+            copyScales(scaleK(i) + T, p.vs, row);
         }
-        return;
+        cpAsyncCommit();
+    };
+#pragma unroll
+    for (uint32_t i = 0; i < NS; ++i) {
+        requestK(i);
+        requestV(i);
     }
 
-    // -------------------------------- consumers --------------------------------
-    if (earlyOk) gridDepWait();  // q comes from a kernel that may still be running
     const uint32_t g = lane >> 2, t = lane & 3u;
-    const uint32_t hL = warp % HPC, sub = warp / HPC;
-    const uint32_t kvHead = kvHead0 + hL;
     // What MMA column j (0..7) of this warp stands for.
-    auto colValid = [&](uint32_t j) { return p.rowsMode ? (b * 8u + j < p.qRows) : (p.colBase + j < p.group); };
+    auto colValid = [&](uint32_t j) { return ROWS ? (b * 8u + j < p.qRows) : (p.colBase + j < p.group); };
     auto colIndex = [&](uint32_t j) -> size_t {  // index of the column's q / out vector, in units of HD
-        return p.rowsMode ? (static_cast<size_t>(b) * 8u + j) * p.nHeads + hg
-                          : static_cast<size_t>(b) * p.nHeads + kvHead * p.group + p.colBase + j;
+        return ROWS ? (static_cast<size_t>(b) * 8u + j) * p.nHeads + hg
+                    : static_cast<size_t>(b) * p.nHeads + kvHead * p.group + p.colBase + j;
     };
-    // exclusive row bound of a column: everything in heads mode, causal in rows mode
-    auto colLen = [&](uint32_t j) { return p.rowsMode ? min(t1, rowsPos + b * 8u + j + 1u) : t1; };
+    // exclusive row bound of a column: everything in decode, causal in rows mode
+    auto colLen = [&](uint32_t j) { return ROWS ? min(t1, rowsPos + b * 8u + j + 1u) : t1; };
 
     // q fragments for head column n = g of this kv head's group: power-of-two
     // normalised, split into fp16 hi + lo, laid out as the B operand whose k
@@ -290,14 +237,10 @@ decodeI8Kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
     const uint32_t lco = lane >> 4;                             // and which chunk of the pair
     const uint32_t lmOff = lr * 128;
 
-    for (uint32_t it = 0; it < nTiles; ++it) {
-        const uint32_t s = it % NSTAGE;
-        if (!mbarWaitClock(&fullBar[s], (it / NSTAGE) & 1, p.err, kDevErrFullWait)) break;
-        uint8_t *st = smem + s * L::kStageBytes;
-        const uint32_t rowInTile = hL * T + sub * kTokPerWarp;
-        const float *sK = reinterpret_cast<const float *>(st + 2 * L::kTileBytes) + rowInTile;
-        const float *sV = sK + L::kRows;
-        const uint32_t tokBase = t0 + it * T + sub * kTokPerWarp + g;
+    for (uint32_t i = 0, tile = first; tile < nTiles; ++i, tile += step) {
+        cpAsyncWait<2 * NS - 1>();  // K of this tile is in, what was requested behind it may still be on its way
+        const float *sK = scaleK(i), *sV = sK + T;
+        const uint32_t tokBase = t0 + tile * T + g;
         bool vl0[NR], vl1[NR];
         float skr[NR], svr[NR];
 #pragma unroll
@@ -305,7 +248,6 @@ decodeI8Kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
             vl0[r] = tokBase + 8 * r < len0;
             vl1[r] = tokBase + 8 * r < len1;
             skr[r] = sK[g + 8 * r];
-            svr[r] = tokBase + 8 * r < t1 ? sV[g + 8 * r] : 0.0f;
         }
 
         // ---- S^T = K . Q^T, two 16-token tiles x 8 heads ----
@@ -314,7 +256,7 @@ decodeI8Kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
         for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
             for (int i = 0; i < 4; ++i) sh[mt][i] = sl[mt][i] = 0.0f;
-        const uint32_t kTile = smemAddr(st + rowInTile * 128);
+        const uint32_t kTile = smemAddr(slotK(i));
 #pragma unroll
         for (int cp = 0; cp < NC / 2; ++cp) {
             const uint32_t sw = (((2 * (cp & 3) + lco) ^ (lr & 7u)) << 4) + (cp >> 2) * L::kHalfBytes;
@@ -355,6 +297,11 @@ decodeI8Kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
             }
         }
         float mx0 = fmaxf(sc[0][0], sc[1][0]), mx1 = fmaxf(sc[0][1], sc[1][1]);
+        __syncwarp();  // every lane has read its part of K
+        requestK(i + NS);
+        cpAsyncWait<2 * NS - 1>();  // V of this tile is in
+#pragma unroll
+        for (int r = 0; r < NR; ++r) svr[r] = tokBase + 8 * r < t1 ? sV[g + 8 * r] : 0.0f;
         float svmax = fmaxf(svr[0], svr[1]);
 #pragma unroll
         for (int r = 2; r < NR; ++r) {
@@ -421,7 +368,7 @@ decodeI8Kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
             }
         }
         // ---- O^T += V^T . P^T (HD dims x 8 heads), V bytes read transposed ----
-        const uint32_t vTile = smemAddr(st + L::kTileBytes + rowInTile * 128);
+        const uint32_t vTile = smemAddr(slotK(i) + L::kTileBytes);
 #pragma unroll
         for (int cp = 0; cp < NC / 2; ++cp) {
             const uint32_t sw = (((2 * (cp & 3) + lco) ^ (lr & 7u)) << 4) + (cp >> 2) * L::kHalfBytes;
@@ -449,7 +396,7 @@ decodeI8Kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
             }
         }
         __syncwarp();
-        if (lane == 0) mbarArrive(&emptyBar[s]);
+        requestV(i + NS);
     }
 
     // ---- fold the consumer warps of each kv head, write the chunk partial ----
@@ -484,80 +431,167 @@ decodeI8Kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
         wO[8 * HD + 8 + 2 * t + 1] = l1;
     }
     namedBarSync(1, NW * 32);
-    // NW*32 threads, HPC*8*(HD/4) float4 outputs
+    if (!ROWS) {
+        FoldTarget f;
+        f.out = p.out, f.pAcc = p.pAcc, f.pM = p.pM, f.pL = p.pL;
+        f.numChunks = p.numChunks, f.slot = chunk / clusterSize();
+        f.firstHead = static_cast<uint32_t>(colIndex(0)), f.nValid = min(8u, p.group - p.colBase);
+        f.direct = p.directOut;
+        f.qRot = nullptr, f.cosT = nullptr, f.sinT = nullptr, f.tableRow = 0;
+        clusterFold<HD, NW>(scr, f, threadIdx.x);
+        return;
+    }
     constexpr uint32_t V4 = HD / 4;
-    for (uint32_t idx = threadIdx.x; idx < HPC * 8 * V4; idx += NW * 32) {
-        const uint32_t d4 = idx % V4, j = (idx / V4) & 7u, h = idx / (8 * V4);
+    for (uint32_t idx = threadIdx.x; idx < 8 * V4; idx += NW * 32) {
+        const uint32_t d4 = idx % V4, j = idx / V4;
         if (!colValid(j)) continue;
         float M = kNegBig;
 #pragma unroll
-        for (int sb = 0; sb < NSUB; ++sb) M = fmaxf(M, scr[(sb * HPC + h) * kWarpScr + 8 * HD + j]);
+        for (int w = 0; w < NW; ++w) M = fmaxf(M, scr[w * kWarpScr + 8 * HD + j]);
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
         float lsum = 0.0f;
 #pragma unroll
-        for (int sb = 0; sb < NSUB; ++sb) {
-            const float *w = scr + (sb * HPC + h) * kWarpScr;
-            const float wgt = fastExp2(w[8 * HD + j] - M);
-            lsum += wgt * w[8 * HD + 8 + j];
-            const float4 a = *reinterpret_cast<const float4 *>(w + j * HD + 4 * d4);
+        for (int w = 0; w < NW; ++w) {
+            const float *s = scr + w * kWarpScr;
+            const float wgt = fastExp2(s[8 * HD + j] - M);
+            lsum += wgt * s[8 * HD + 8 + j];
+            const float4 a = *reinterpret_cast<const float4 *>(s + j * HD + 4 * d4);
             acc.x = fmaf(wgt, a.x, acc.x);
             acc.y = fmaf(wgt, a.y, acc.y);
             acc.z = fmaf(wgt, a.z, acc.z);
             acc.w = fmaf(wgt, a.w, acc.w);
         }
-        // column -> output vector (same rule as colIndex, for kv head kvHead0 + h)
-        const size_t oidx = p.rowsMode ? (static_cast<size_t>(b) * 8u + j) * p.nHeads + hg
-                                       : static_cast<size_t>(b) * p.nHeads + (kvHead0 + h) * p.group + p.colBase + j;
-        if (p.directOut) {
-            const float inv = lsum > 0.0f ? 1.0f / lsum : 0.0f;
-            *reinterpret_cast<float4 *>(p.out + oidx * HD + 4 * d4) =
-                    make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
-        } else {
-            const size_t pidx = oidx * p.numChunks + chunk;
-            *reinterpret_cast<float4 *>(p.pAcc + pidx * HD + 4 * d4) = acc;
-            if (d4 == 0) {
-                // back to natural-log units: the merge contract is w = exp2((m - M) * log2e)
-                p.pM[pidx] = M > -1e29f ? M * 0.6931471805599453f : kNegBig;
-                p.pL[pidx] = lsum;
-            }
-        }
+        const float inv = lsum > 0.0f ? 1.0f / lsum : 0.0f;
+        *reinterpret_cast<float4 *>(p.out + colIndex(j) * HD + 4 * d4) =
+                make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
     }
 }
 
-template <int HD, int HPC, int MT>
-static int launchDecodeI8(const CUtensorMap &tmK, const CUtensorMap &tmV, const CUtensorMap &tmKn,
-                          const CUtensorMap &tmVn, const DecodeI8Params &prm, const DecodePlan &pl, uint32_t batch,
-                          bool pdl, cudaStream_t st) {
-    constexpr int NW = 8, NSTAGE = (MT == 2 || HD == 256) ? 3 : 6;
-    using L = DecodeI8Smem<HD, HPC, NW, NSTAGE, MT>;
-    static_assert(L::kTotal <= 227 * 1024, "stage ring exceeds the shared memory of an SM");
-    auto kern = decodeI8Kernel<HD, HPC, NW, NSTAGE, MT>;
-    static bool attrDone[64] = {false};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 64 && !attrDone[dev]) {
-        TC_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
-        attrDone[dev] = true;
+// The split at head_dim 256.  Which tokens one warp accumulates in a row decides the roundings of the result: the V
+// bytes enter the products with an offset of 128 that is taken out at the end, so the running sums are large next to the
+// result.  Short runs keep that small, and the runs stay what they are whatever the clusters look like: chunks of
+// planDecode (one wave of blocks that stream up to four kv heads), a chunk's tokens dealt to 8 / hpc warps.  A chunk is a
+// block here; the cluster only decides how the blocks' results come together.
+static ClusterPlan decodeI8Plan(const tc_decode_i8_batch *d, const uint32_t *maxClusters) {
+    const DecodePlan dp = planDecode(d->batch, d->nKV, d->maxLen, d->numChunks, 8u * 16u, d->lens == nullptr);
+    ClusterPlan best = {1, dp.chunksPerSeq, dp.chunkTokens};
+    // up to 16 chunks one cluster per kv head folds them all; more take the merge
+    for (uint32_t lg = 1; lg < 5; ++lg)
+        if (dp.chunksPerSeq > 1 && dp.chunksPerSeq <= (1u << lg) && maxClusters[lg] >= d->nKV * d->batch) {
+            best.cluster = 1u << lg, best.clusters = 1;
+            break;
+        }
+#ifdef TC_TUNE
+    if (const char *e = getenv("TC_PLAN")) {
+        unsigned C = 1, n = 1;
+        sscanf(e, "%u,%u", &C, &n);
+        best.cluster = C, best.clusters = (dp.chunksPerSeq + C - 1) / C;
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(pl.chunksPerSeq, pl.headGroups, batch);
-    cfg.blockDim = dim3((NW + 1) * 32);
-    cfg.dynamicSmemBytes = L::kTotal;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    TC_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, tmK, tmV, tmKn, tmVn, prm));
+#endif
+    return best;
+}
+
+template <int NW>
+static int decodeI8Hd256(const tc_decode_i8_batch *d, DecodeI8Params prm, cudaStream_t st) {
+    constexpr int HD = 256;
+    using L = DecodeI8Smem<HD, NW, 1, 1>;
+    auto kern = decodeI8Kernel<HD, NW, 1, 1, I8Mode::kChunks>;
+    static ClusterSetup setup;
+    const uint32_t *limits = nullptr;
+    int rc = setupCluster(setup, kern, NW * 32, L::kTotal, &limits);
+    if (rc != TC_OK) return rc;
+    const ClusterPlan pl = decodeI8Plan(d, limits);
+    const bool direct = pl.clusters == 1 && !d->partialsOnly;
+    if (!direct)
+        TC_REQUIRE(d->pAcc && d->pM && d->pL, TC_EWORKSPACE, "decode_i8: partial buffers are required");
+    if (d->chunksUsed) *d->chunksUsed = pl.clusters;
+    prm.chunkTokens = pl.chunkTokens;
+    prm.directOut = direct ? 1 : 0;
+    // a launch serves 8 q heads per kv head (the MMA columns); wider groups take one launch per
+    // block of 8 and stream the rows again
+    for (uint32_t cb = 0; cb < prm.group; cb += 8) {
+        prm.colBase = cb;
+        if (cb) prm.appendK = prm.appendV = nullptr;  // the row is in
+        rc = launchDependent(kern, dim3(pl.clusters * pl.cluster, d->nKV, d->batch), NW * 32, L::kTotal, st, pl.cluster,
+                             prm);
+        if (rc != TC_OK) return rc;
+    }
+    if (direct || d->partialsOnly) return TC_OK;
+    // merge: the active partial count of a sequence follows from its length (read on
+    // the device when the length lives there); slots past it were never written.
+    return launchMerge(d->pAcc, d->pM, d->pL, d->out, d->batch, d->nHeads, d->numChunks, pl.clusters, HD, d->lens, prm.lenAdd,
+                       pl.chunkTokens * pl.cluster, nullptr, true, st);
+}
+
+static int i8Params(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, const F32Mirror &mir, DecodeI8Params *o) {
+    memset(o, 0, sizeof(*o));
+    o->q = d->q;
+    o->out = d->out;
+    o->ks = d->ks;
+    o->vs = d->vs;
+    o->pAcc = d->pAcc;
+    o->pM = d->pM;
+    o->pL = d->pL;
+    o->devLens = d->lens;
+    o->devRowBase = d->rowBase;
+    o->rowsPerSeq = d->rowsPerSeq;
+    o->totalRows = d->totalRows;
+    o->lenHost = lenHost;
+    o->lenAdd = lenAdd;
+    o->nHeads = d->nHeads;
+    o->nKV = d->nKV;
+    o->group = d->nHeads / d->nKV;
+    o->numChunks = d->numChunks;
+    o->appendK = d->appendK;
+    o->appendV = d->appendV;
+    o->k8w = reinterpret_cast<uint32_t *>(const_cast<int8_t *>(d->k8));
+    o->v8w = reinterpret_cast<uint32_t *>(const_cast<int8_t *>(d->v8));
+    o->mir = mir;
+    o->invSqrt = d->invSqrt;
+    o->err = devErrorWord();
+    TC_REQUIRE(o->err != nullptr, TC_ECUDA, "decode_i8: no device error word");
     return TC_OK;
 }
 
-static int decodeI8Common(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, cudaStream_t st) {
+// One sequence, any length up to lenHost rows, no partial buffers: what a captured decode step of the int8 store takes.
+// The causal kernel (a block per q head, 8 warps of which 7 / 8 of the MMA columns were padding) took 27.5 us for
+// 5000 rows of 28 q / 4 kv heads of 128; this form, with the same roundings, 26.
+template <int HD, int MT>
+static int launchStreamsI8(DecodeI8Params prm, cudaStream_t st) {
+    constexpr int NS = 4;
+    using L = DecodeI8Smem<HD, 1, NS, MT>;
+    auto kern = decodeI8Kernel<HD, 1, NS, MT, I8Mode::kStreams>;
+    static ClusterSetup setup;
+    const uint32_t *limits = nullptr;
+    int rc = setupCluster(setup, kern, 32, L::kTotal, &limits);
+    if (rc != TC_OK) return rc;
+    prm.directOut = 1;
+    for (uint32_t cb = 0; cb < prm.group; cb += 8) {
+        prm.colBase = cb;
+        if (cb) prm.appendK = prm.appendV = nullptr;  // the row is in
+        rc = launchDependent(kern, dim3(8, prm.nKV, 1), 32, L::kTotal, st, 8, prm);
+        if (rc != TC_OK) return rc;
+    }
+    return TC_OK;
+}
+int decodeI8Streams(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, cudaStream_t st) {
+    TC_REQUIRE(d->hd == 128 || d->hd == 256, TC_EUNSUPPORTED, "decode_i8: head_dim %u (built for 128 and 256)", d->hd);
+    TC_REQUIRE(d->nHeads / d->nKV <= 64, TC_EUNSUPPORTED, "decode_i8: %u q heads per kv head (built for <= 64)",
+               d->nHeads / d->nKV);
+    TC_REQUIRE(((reinterpret_cast<uintptr_t>(d->k8) | reinterpret_cast<uintptr_t>(d->v8) |
+                 reinterpret_cast<uintptr_t>(d->q) | reinterpret_cast<uintptr_t>(d->out) |
+                 reinterpret_cast<uintptr_t>(d->appendK) | reinterpret_cast<uintptr_t>(d->appendV)) & 15u) == 0,
+               TC_EINVAL, "decode_i8: q/out/k8/v8 and the new row need 16-byte alignment");
+    DecodeI8Params prm;
+    const int rc = i8Params(d, lenHost, lenAdd, F32Mirror{nullptr, nullptr}, &prm);
+    if (rc != TC_OK) return rc;
+    return d->hd == 256 ? launchStreamsI8<256, 1>(prm, st) : launchStreamsI8<128, 2>(prm, st);
+}
+
+int decodeI8Common(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, const F32Mirror &mir, cudaStream_t st) {
     TC_REQUIRE(d->q && d->out && d->k8 && d->v8 && d->ks && d->vs, TC_EINVAL, "decode_i8: null pointer");
     TC_REQUIRE(d->hd == 128 || d->hd == 256, TC_EUNSUPPORTED, "decode_i8: head_dim %u (built for 128 and 256)",
                d->hd);
-    const uint32_t hd = d->hd;
     TC_REQUIRE(d->nKV > 0 && d->nHeads % d->nKV == 0, TC_EINVAL, "decode_i8: nHeads %u not a multiple of nKV %u",
                d->nHeads, d->nKV);
     const uint32_t group = d->nHeads / d->nKV;
@@ -570,123 +604,32 @@ static int decodeI8Common(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_
                  reinterpret_cast<uintptr_t>(d->q) | reinterpret_cast<uintptr_t>(d->out)) & 15u) == 0,
                TC_EINVAL, "decode_i8: q/out/k8/v8 need 16-byte alignment");
     TC_REQUIRE(d->numChunks >= 1, TC_EWORKSPACE, "decode_i8: no chunk slots");
-    // head_dim 128 runs on the tcgen05 integer path; this file's mma.sync kernel keeps head_dim
-    // 256 and the causal rows mode
     TC_REQUIRE((d->appendK == nullptr) == (d->appendV == nullptr), TC_EINVAL, "decode_i8: appendK and appendV come together");
-    if (hd == 128 && !forceLegacyDecode()) return decodeI8Tc(d, lenHost, lenAdd, st);
-    if (d->appendK != nullptr) {
-        // this file's kernel reads the pool only: the new rows go in with the quantise launch
-        const int rc = tc_kv_quantize_i8_batch(d->appendK, d->appendV, const_cast<int8_t *>(d->k8),
-                                               const_cast<int8_t *>(d->v8), const_cast<float *>(d->ks),
-                                               const_cast<float *>(d->vs), d->batch, d->nKV, hd, d->rowsPerSeq, d->rowBase,
-                                               lenHost - 1u, d->lens, static_cast<int32_t>(lenAdd) - 1, d->totalRows, st);
-        if (rc != TC_OK) return rc;
-    }
-    // work quantum: 32 tokens per warp when every warp of the machine gets at least ~12
-    // of them, 16 otherwise (see DecodeI8Smem)
-    const uint64_t warpTiles32 = static_cast<uint64_t>(d->batch) * d->nKV * ((d->maxLen + 31) / 32);
-    // (head_dim 256: a 32-token tile of K and V no longer leaves room for a second stage)
-    const uint32_t mt = hd == 128 && warpTiles32 >= 2ull * 8ull * static_cast<uint64_t>(numSMs()) ? 2u : 1u;
-    const DecodePlan pl = planDecode(d->batch, d->nKV, d->maxLen, d->numChunks, 8u * 16u * mt, d->lens == nullptr);
-    const bool pdl = (d->flags & TC_DECODE_PDL) != 0;
-    const bool direct = pl.chunksPerSeq == 1 && !d->partialsOnly;
-    if (!direct)
-        TC_REQUIRE(d->pAcc && d->pM && d->pL, TC_EWORKSPACE, "decode_i8: partial buffers are required");
-    if (d->chunksUsed) *d->chunksUsed = pl.chunksPerSeq;
-
-    TensorMapKey key;
-    memset(&key, 0, sizeof(key));
-    key.rank = 3;
-    key.elemBytes = 1;
-    key.swizzle = 3;
-    key.dims[0] = hd;
-    key.dims[1] = d->nKV;
-    key.dims[2] = d->totalRows;
-    key.strides[0] = hd;
-    key.strides[1] = static_cast<uint64_t>(d->nKV) * hd;
-    key.box[0] = 128;  // one swizzle span; a 256-dim row is fetched as two boxes
-    key.box[1] = 1;
-    key.box[2] = pl.tileTokens;
-    CUtensorMap tmK, tmV;
-    key.base = d->k8;
-    int rc = getTensorMap(key, &tmK);
-    if (rc != TC_OK) return rc;
-    key.base = d->v8;
-    rc = getTensorMap(key, &tmV);
-    if (rc != TC_OK) return rc;
-    // the pools of the next call, for the L2 prefetch hint (same geometry)
-    CUtensorMap tmKn = tmK, tmVn = tmV;
-    // Only when a call's rows fit into L2 next to the rows still in flight: a prefetch of more than
-    // that is evicted before it is used and costs the DRAM traffic twice (8 sequences of 32768 rows,
-    // 277 MB per call: 0.87 of the copy peak without the hint, 0.74 with it).
-    const uint64_t callBytes = static_cast<uint64_t>(d->batch) * d->maxLen * d->nKV * hd * 2ull;
-    const bool prefetchNext = d->nextK8 != nullptr && d->nextV8 != nullptr && callBytes <= (48ull << 20);
-    if (prefetchNext) {
-        TC_REQUIRE(((reinterpret_cast<uintptr_t>(d->nextK8) | reinterpret_cast<uintptr_t>(d->nextV8)) & 15u) == 0,
-                   TC_EINVAL, "decode_i8: nextK8/nextV8 need 16-byte alignment");
-        key.base = d->nextK8;
-        rc = getTensorMap(key, &tmKn);
-        if (rc != TC_OK) return rc;
-        key.base = d->nextV8;
-        rc = getTensorMap(key, &tmVn);
-        if (rc != TC_OK) return rc;
-    }
+    // head_dim 128 runs on the tcgen05 integer path
+    if (d->hd == 128) return decodeI8Tc(d, lenHost, lenAdd, mir, st);
 
     DecodeI8Params prm;
-    prm.q = d->q;
-    prm.out = d->out;
-    prm.ks = d->ks;
-    prm.vs = d->vs;
-    prm.pAcc = d->pAcc;
-    prm.pM = d->pM;
-    prm.pL = d->pL;
-    prm.devLens = d->lens;
-    prm.devRowBase = d->rowBase;
-    prm.rowsPerSeq = d->rowsPerSeq;
-    prm.totalRows = d->totalRows;
-    prm.lenHost = lenHost;
-    prm.lenAdd = lenAdd;
-    prm.nHeads = d->nHeads;
-    prm.nKV = d->nKV;
-    prm.group = group;
-    prm.chunkTokens = pl.chunkTokens;
-    prm.numChunks = d->numChunks;
-    prm.prefetchRows = pdl ? d->prefetchRows : 0;
-    prm.rowsMode = 0;
-    prm.qRows = 0;
-    prm.cachePos = 0;
-    prm.devPos = nullptr;
-    prm.invSqrt = d->invSqrt;
-    prm.directOut = direct ? 1 : 0;
-    prm.prefetchNext = prefetchNext ? 1 : 0;
-    prm.err = devErrorWord();
-    TC_REQUIRE(prm.err != nullptr, TC_ECUDA, "decode_i8: no device error word");
-
-    // a launch serves 8 q heads per kv head (the MMA columns); wider groups take one launch per
-    // block of 8 and stream the rows again
-    for (uint32_t cb = 0; cb < group; cb += 8) {
-        prm.colBase = cb;
-        if (hd == 256) {
-            if (pl.hpc == 4) rc = launchDecodeI8<256, 4, 1>(tmK, tmV, tmKn, tmVn, prm, pl, d->batch, pdl, st);
-            else if (pl.hpc == 2) rc = launchDecodeI8<256, 2, 1>(tmK, tmV, tmKn, tmVn, prm, pl, d->batch, pdl, st);
-            else rc = launchDecodeI8<256, 1, 1>(tmK, tmV, tmKn, tmVn, prm, pl, d->batch, pdl, st);
-        } else if (mt == 2) {
-            if (pl.hpc == 4) rc = launchDecodeI8<128, 4, 2>(tmK, tmV, tmKn, tmVn, prm, pl, d->batch, pdl, st);
-            else if (pl.hpc == 2) rc = launchDecodeI8<128, 2, 2>(tmK, tmV, tmKn, tmVn, prm, pl, d->batch, pdl, st);
-            else rc = launchDecodeI8<128, 1, 2>(tmK, tmV, tmKn, tmVn, prm, pl, d->batch, pdl, st);
-        } else {
-            if (pl.hpc == 4) rc = launchDecodeI8<128, 4, 1>(tmK, tmV, tmKn, tmVn, prm, pl, d->batch, pdl, st);
-            else if (pl.hpc == 2) rc = launchDecodeI8<128, 2, 1>(tmK, tmV, tmKn, tmVn, prm, pl, d->batch, pdl, st);
-            else rc = launchDecodeI8<128, 1, 1>(tmK, tmV, tmKn, tmVn, prm, pl, d->batch, pdl, st);
-        }
-        if (rc != TC_OK) return rc;
-    }
+    const int rc = i8Params(d, lenHost, lenAdd, mir, &prm);
     if (rc != TC_OK) return rc;
-    if (direct || d->partialsOnly) return TC_OK;
-    // merge: the active chunk count of a sequence follows from its length (read on
-    // the device when the length lives there); slots past it were never written.
-    return launchMerge(d->pAcc, d->pM, d->pL, d->out, d->batch, d->nHeads, d->numChunks, pl.chunksPerSeq, hd,
-                       d->lens, lenAdd, pl.chunkTokens, nullptr, pdl, st);
+    // warps that share a chunk's tokens, by the kv heads (see decodeI8Plan)
+    if (d->nKV % 4u == 0) return decodeI8Hd256<2>(d, prm, st);
+    if (d->nKV % 2u == 0) return decodeI8Hd256<4>(d, prm, st);
+    return decodeI8Hd256<8>(d, prm, st);
+}
+
+template <int HD, int MT>
+static int launchRowsI8(const DecodeI8Params &prm, cudaStream_t st) {
+    constexpr int NW = 8, NS = 3;
+    using L = DecodeI8Smem<HD, NW, NS, MT>;
+    auto kern = decodeI8Kernel<HD, NW, NS, MT, I8Mode::kRows>;
+    static bool attrDone[64] = {false};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 0 && dev < 64 && !attrDone[dev]) {
+        TC_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
+        attrDone[dev] = true;
+    }
+    return launchDependent(kern, dim3(1, prm.nHeads, (prm.qRows + 7) / 8), NW * 32, L::kTotal, st, 1, prm);
 }
 
 // Causal prefill over the int8 store: the decode kernel with query rows as MMA columns.
@@ -711,41 +654,19 @@ static int prefillI8(const float *q, const int8_t *k8, const int8_t *v8, const f
     const uint32_t rowBlocks = (seqLen + 7) / 8;
     TC_REQUIRE(rowBlocks <= 65535 && nHeads <= 65535, TC_EUNSUPPORTED, "prefill_i8: %u rows x %u heads", seqLen,
                nHeads);
-    // tokens per stage: 8 warps x 32 rows (head_dim 128) or x 16 rows (head_dim 256)
-    const uint32_t tileTokens = hd == 256 ? 128u : 256u;
-    TensorMapKey key;
-    memset(&key, 0, sizeof(key));
-    key.rank = 3;
-    key.elemBytes = 1;
-    key.swizzle = 3;
-    key.dims[0] = hd;
-    key.dims[1] = nKV;
-    key.dims[2] = totalRows;
-    key.strides[0] = hd;
-    key.strides[1] = static_cast<uint64_t>(nKV) * hd;
-    key.box[0] = 128;
-    key.box[1] = 1;
-    key.box[2] = tileTokens;
-    CUtensorMap tmK, tmV;
-    key.base = k8;
-    int rc = getTensorMap(key, &tmK);
-    if (rc != TC_OK) return rc;
-    key.base = v8;
-    rc = getTensorMap(key, &tmV);
-    if (rc != TC_OK) return rc;
     DecodeI8Params prm;
     memset(&prm, 0, sizeof(prm));
     prm.q = q;
     prm.out = out;
     prm.ks = ks;
     prm.vs = vs;
+    prm.k8w = reinterpret_cast<uint32_t *>(const_cast<int8_t *>(k8));
+    prm.v8w = reinterpret_cast<uint32_t *>(const_cast<int8_t *>(v8));
     prm.totalRows = totalRows;
     prm.nHeads = nHeads;
     prm.nKV = nKV;
     prm.group = nHeads / nKV;
-    prm.chunkTokens = 0xffffff00u;  // one chunk: a block streams its whole causal prefix
     prm.numChunks = 1;
-    prm.rowsMode = 1;
     prm.qRows = seqLen;
     prm.cachePos = cachePos;
     prm.devPos = devPos;
@@ -753,16 +674,10 @@ static int prefillI8(const float *q, const int8_t *k8, const int8_t *v8, const f
     prm.directOut = 1;
     prm.err = devErrorWord();
     TC_REQUIRE(prm.err != nullptr, TC_ECUDA, "prefill_i8: no device error word");
-    DecodePlan pl;
-    pl.hpc = 1;
-    pl.headGroups = nHeads;
-    pl.chunksPerSeq = 1;
-    pl.chunkTokens = prm.chunkTokens;
-    pl.tileTokens = tileTokens;
     // heaviest row blocks first would need a reversed grid; the hardware scheduler
     // hands out blocks in z-major order, so late (long) blocks start last -- acceptable here
-    if (hd == 256) return launchDecodeI8<256, 1, 1>(tmK, tmV, tmK, tmV, prm, pl, rowBlocks, false, st);
-    return launchDecodeI8<128, 1, 2>(tmK, tmV, tmK, tmV, prm, pl, rowBlocks, false, st);
+    if (hd == 256) return launchRowsI8<256, 1>(prm, st);
+    return launchRowsI8<128, 2>(prm, st);
 }
 
 }  // namespace tc
@@ -778,7 +693,7 @@ int tc_attn_prefill_i8(const float *q, const int8_t *k8, const int8_t *v8, const
 
 int tc_attn_decode_i8_batch(const tc_decode_i8_batch *d, tc_stream stream) {
     TC_REQUIRE(d != nullptr, TC_EINVAL, "tc_attn_decode_i8_batch: null descriptor");
-    return tc::decodeI8Common(d, d->maxLen, 0, static_cast<cudaStream_t>(stream));
+    return tc::decodeI8Common(d, d->maxLen, 0, tc::F32Mirror{nullptr, nullptr}, static_cast<cudaStream_t>(stream));
 }
 
 int tc_attn_decode_i8(const float *q, const int8_t *k8, const int8_t *v8, const float *ks, const float *vs,
@@ -811,7 +726,7 @@ int tc_attn_decode_i8(const float *q, const int8_t *k8, const int8_t *v8, const 
     d.maxLen = cachePos + 1;
     d.numChunks = numChunks;
     d.invSqrt = invSqrt;
-    return tc::decodeI8Common(&d, cachePos + 1, devPos ? 1u : 0u, static_cast<cudaStream_t>(stream));
+    return tc::decodeI8Common(&d, cachePos + 1, devPos ? 1u : 0u, tc::F32Mirror{nullptr, nullptr}, static_cast<cudaStream_t>(stream));
 }
 
 // ---------------------------------------------------------------------------------
@@ -885,7 +800,7 @@ int tc_attn_decode_i8_noalloc(const float *q, const int8_t *k8, const int8_t *v8
     d.maxLen = cachePos + 1;
     d.numChunks = kNoAllocChunks;
     d.invSqrt = invSqrt;
-    return tc::decodeI8Common(&d, cachePos + 1, 0u, static_cast<cudaStream_t>(stream));
+    return tc::decodeI8Common(&d, cachePos + 1, 0u, tc::F32Mirror{nullptr, nullptr}, static_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

@@ -45,6 +45,7 @@ struct DecodeTcParams {
     const float *ks, *vs;
     const float *appendK, *appendV;  // nullable: [batch][nKV][128] rows to quantise into row len - 1 first
     int8_t *k8w, *v8w;               // the pools, for that row
+    float *mirK, *mirV;              // nullable: an f32 store that gets the row verbatim
     const int8_t *nextK8, *nextV8;  // nullable: pools of the next call (L2 prefetch)
     float *pAcc, *pM, *pL;
     uint32_t *tickets;           // nullable: [batch][nKV] arrival counters of the in-kernel merge (zero between calls)
@@ -159,40 +160,6 @@ __device__ __forceinline__ bool barOr(uint32_t id, uint32_t threads, bool pred) 
 }
 __device__ __forceinline__ float i2f(uint32_t x) { return __int2float_rn(static_cast<int>(x)); }
 
-// The new token's K and V row of one kv head into the int8 pool, by one warp (the arithmetic of
-// kvQuantKernel: amax / 127, IEEE divide, round-half-even; lane i owns dims 4 i .. 4 i + 3 of the 128).
-// Blocks that share the kv head write the same bytes.  Both rows are loaded at once (they were pulled
-// towards L2 when the block started); the block's own TMA load and scale copies read the row back, so
-// the stores are ordered before the async proxy and nothing wider.  srcK / srcV: the rows' 32 float4;
-// dst: row x nKV + kv head of the pool.
-__device__ __forceinline__ void appendNewRow(const float4 *srcK, const float4 *srcV, uint32_t *k8w, uint32_t *v8w,
-                                             float *ksw, float *vsw, uint64_t dst, uint32_t lane) {
-    const float4 kx = __ldg(srcK + lane);
-    const float4 vx = __ldg(srcV + lane);
-    float mk = fmaxf(fmaxf(fabsf(kx.x), fabsf(kx.y)), fmaxf(fabsf(kx.z), fabsf(kx.w)));
-    float mv = fmaxf(fmaxf(fabsf(vx.x), fabsf(vx.y)), fmaxf(fabsf(vx.z), fabsf(vx.w)));
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-        mk = fmaxf(mk, __shfl_xor_sync(0xffffffffu, mk, o));
-        mv = fmaxf(mv, __shfl_xor_sync(0xffffffffu, mv, o));
-    }
-    const float sk = mk > 0.0f ? __fdiv_rn(mk, 127.0f) : 1.0f;
-    const float sv = mv > 0.0f ? __fdiv_rn(mv, 127.0f) : 1.0f;
-    if (lane == 0) {
-        ksw[dst] = sk;
-        vsw[dst] = sv;
-    }
-    auto q8 = [](float x, float sc) -> uint32_t {
-        int qv = __float2int_rn(__fdiv_rn(x, sc));
-        qv = qv < -128 ? -128 : (qv > 127 ? 127 : qv);
-        return static_cast<uint32_t>(qv) & 0xffu;
-    };
-    k8w[dst * 32u + lane] = q8(kx.x, sk) | (q8(kx.y, sk) << 8) | (q8(kx.z, sk) << 16) | (q8(kx.w, sk) << 24);
-    v8w[dst * 32u + lane] = q8(vx.x, sv) | (q8(vx.y, sv) << 8) | (q8(vx.z, sv) << 16) | (q8(vx.w, sv) << 24);
-    asm volatile("fence.proxy.async.global;" ::: "memory");
-    __syncwarp();
-}
-
 // APPEND: the instantiation for calls that hand in the new token's rows.  It is a kernel of its own
 // because the mere presence of that (cold) code -- inlined or called, inside or behind the producer's
 // loop -- cost the 7B-shaped batch-1 step 0.5 us; calls without new rows run the other instantiation.
@@ -243,7 +210,7 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     const bool earlyOk = p.devLens == nullptr && p.devRowBase == nullptr && p.prefetchRows != 0;
     if (!earlyOk) {
         gridDepWait();
-        if (p.devLens) len = p.devLens[b] + p.lenAdd;
+        if (p.devLens) len = min(p.devLens[b] + p.lenAdd, p.lenHost);  // (the host's length is the upper bound)
     }
     const uint32_t t0 = chunk * p.chunkTokens;
     if (t0 >= len) return;  // inactive chunk (block-uniform): the merge derives the active count from len
@@ -333,16 +300,19 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
                 waited = true;
             }
             const size_t srcRow = (static_cast<size_t>(b) * p.nKV + kvHead) * 32u;
-            const uint64_t dst = (rowBase + len - 1u) * p.nKV + kvHead;
+            const uint64_t row = rowBase + (p.devLens ? p.devLens[b] + p.lenAdd : len) - 1u;
+            const uint64_t dst = row * p.nKV + kvHead;
             // a length read from device memory is checked where it is known: outside the pool the
             // store is skipped and the error word says so
-            if (rowBase + len - 1u >= p.totalRows) {
+            if (row >= p.totalRows) {
                 if (lane == 0) atomicOr(p.err, kDevErrRowBound);
             } else {
-                appendNewRow(reinterpret_cast<const float4 *>(p.appendK) + srcRow,
-                             reinterpret_cast<const float4 *>(p.appendV) + srcRow, reinterpret_cast<uint32_t *>(p.k8w),
-                             reinterpret_cast<uint32_t *>(p.v8w), const_cast<float *>(p.ks), const_cast<float *>(p.vs), dst,
-                             lane);
+                float4 *mk = nullptr, *mv = nullptr;
+                if (p.mirK != nullptr) mk = reinterpret_cast<float4 *>(p.mirK) + dst * 32u, mv = reinterpret_cast<float4 *>(p.mirV) + dst * 32u;
+                appendQuantRow<128>(reinterpret_cast<const float4 *>(p.appendK) + srcRow,
+                                    reinterpret_cast<const float4 *>(p.appendV) + srcRow, reinterpret_cast<uint32_t *>(p.k8w),
+                                    reinterpret_cast<uint32_t *>(p.v8w), const_cast<float *>(p.ks), const_cast<float *>(p.vs), dst,
+                                    mk, mv, lane);
             }
             requestTile(nTiles - 1u);
         }
@@ -739,7 +709,7 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
 }
 
 // Host side: arguments were validated by the caller (decodeI8Common in decode_i8.cu).
-int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, cudaStream_t st) {
+int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, const F32Mirror &mir, cudaStream_t st) {
     const uint32_t hd = 128;
     const uint32_t group = d->nHeads / d->nKV;
     const DecodePlan pl = planDecode(d->batch, d->nKV, d->maxLen, d->numChunks, kTcTile, d->lens == nullptr, 1u);
@@ -794,6 +764,7 @@ int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, c
     prm.nextV8 = d->nextV8;
     prm.appendK = d->appendK;
     prm.appendV = d->appendV;
+    prm.mirK = mir.k, prm.mirV = mir.v;
     prm.k8w = const_cast<int8_t *>(d->k8);
     prm.v8w = const_cast<int8_t *>(d->v8);
     prm.pAcc = d->pAcc;
@@ -854,25 +825,18 @@ int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, c
                                         Smem::kTotal));
         attrDone[dev] = true;
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(pl.chunksPerSeq, d->nKV, d->batch);
-    cfg.blockDim = dim3(Smem::kThreads);
-    cfg.dynamicSmemBytes = Smem::kTotal;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    // (without TC_DECODE_PDL prefetchRows is 0 and every block waits for the kernels ahead first thing)
     // a launch serves 8 q heads per kv head (the MMA columns); wider groups take one launch per
     // block of 8 and stream the rows again
     for (uint32_t cb = 0; cb < group; cb += 8) {
         prm.colBase = cb;
-        TC_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, tmK, tmV, tmKn, tmVn, prm));
+        rc = launchDependent(kern, dim3(pl.chunksPerSeq, d->nKV, d->batch), Smem::kThreads, Smem::kTotal, st, 1, tmK, tmV,
+                             tmKn, tmVn, prm);
+        if (rc != TC_OK) return rc;
     }
     if (direct || d->partialsOnly || fused) return TC_OK;
     return launchMerge(d->pAcc, d->pM, d->pL, d->out, d->batch, d->nHeads, d->numChunks, pl.chunksPerSeq, hd, d->lens,
-                       lenAdd, pl.chunkTokens, nullptr, pdl, st);
+                       lenAdd, pl.chunkTokens, nullptr, true, st);
 }
 
 #ifdef TC_TRACE

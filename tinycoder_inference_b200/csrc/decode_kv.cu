@@ -9,47 +9,27 @@
 // models (include/gpu/GpuQwen35Kernels.hpp:2437-2492): score = dot(q, k) *
 // invSqrt, online softmax with exp2, out = sum p v / sum p, all f32.
 //
-// Same skeleton as the int8 kernel (decode_i8.cu): grid = (chunks, kv-head groups,
-// sequences), one TMA producer warp feeding an mbarrier ring with 128-byte
-// swizzled [tokens][32 floats] boxes, consumer warps that own a (kv head, 16
-// token) tile per stage and serve every q head of that kv head, partials in the
-// reference's layout, merge by merge.cu.  The arithmetic differs: K and V are
+// A block streams a token range of one kv head; its warps take 16-token tiles in
+// turn, each with copies and slots of its own, and serve every q head of the kv head.  The split
+// over clusters of blocks, the fold of their results and the new token's row are
+// decode_cluster.cuh's.  The arithmetic differs from the int8 kernel's: K and V are
 // arbitrary f32, so QK^T and PV run as 3xTF32 tensor-core products
 // (mma.sync.m16n8k8: x = hi + lo with both parts tf32; hi*hi + lo*hi + hi*lo keeps
 // ~21 mantissa bits and the full f32 exponent range, f32 accumulation).  f32 rows
 // are four times the bytes of int8 rows, so per byte this costs a quarter of the
 // instructions and the kernel stays HBM-bound.
-#include "decode_shared.cuh"
+#include "decode_cluster.cuh"
 
 namespace tc {
 
-struct DecodeKvParams {
-    const float *q;
-    float *out;
-    float *pAcc, *pM, *pL;
-    const uint32_t *devPos;  // nullable: position read at kernel time
-    uint64_t totalRows;
-    uint32_t lenHost;        // rows to attend in heads mode when devPos == nullptr
-    uint32_t nHeads, nKV, group;
-    uint32_t colBase;  // heads mode: the 8 MMA columns are q heads colBase .. colBase + 7 of the kv head
-    uint32_t chunkTokens, numChunks;
-    uint32_t rowsMode, qRows, cachePos;  // rows mode: see decode_i8.cu
-    float invSqrt;
-    int directOut;
-    unsigned int *err;
-};
-
-template <int HD, int NW, int HPC, int NSTAGE>
+// Every warp has a slot for a 16-token tile of K and one of V, each as HD / 32 boxes of [16 rows][32 floats].
+template <int HD, int NW>
 struct DecodeKvSmem {
-    static constexpr int NB = HD / 32;                  // 32-float boxes per row
-    static constexpr int kRows = NW * 16;               // (token, head) rows per stage
-    static constexpr int T = kRows / HPC;               // tokens per stage
-    static constexpr int kTileBytes = kRows * HD * 4;   // K (or V) bytes per stage
-    static constexpr int kStageBytes = 2 * kTileBytes;
-    static constexpr int kBarOffset = NSTAGE * kStageBytes;
-    static constexpr int kTotal = kBarOffset + 2 * NSTAGE * 8 + 1024;
-    static_assert(T % 8 == 0 && T <= 256, "box rows");
-    static_assert(NW % HPC == 0, "warps per head");
+    static constexpr int NB = HD / 32;             // 32-float boxes per row
+    static constexpr int kTileBytes = 16 * HD * 4; // K (or V) bytes of a tile
+    static constexpr int kSlots = NW * 2 * kTileBytes, kScratch = (NW + 1) * (8 * HD + 16) * 4;  // (the fold reuses the slots)
+    static constexpr int kTotal = (kSlots > kScratch ? kSlots : kScratch) + 128;
+    static_assert(kTotal <= 227 * 1024, "shared memory of an SM");
 };
 
 __device__ __forceinline__ void splitTf32(float x, uint32_t &hi, uint32_t &lo) {
@@ -57,13 +37,18 @@ __device__ __forceinline__ void splitTf32(float x, uint32_t &hi, uint32_t &lo) {
     lo = toTf32(x - __uint_as_float(hi));
 }
 
-template <int HD, int NW, int HPC, int NSTAGE>
-__global__ void __launch_bounds__((NW + 1) * 32, 1)
-decodeKvKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
-               const DecodeKvParams p) {
-    using L = DecodeKvSmem<HD, NW, HPC, NSTAGE>;
-    constexpr int T = L::T, NB = L::NB;
-    constexpr int NSUB = NW / HPC;
+// ROWS: the causal kernel (one block per 8 query rows and q head); otherwise decode, blocks of a cluster
+// share a kv head's tokens.
+//
+// What bounds it: a warp needs about 800 instructions and six dependent chains of tensor-core products for 16
+// tokens (1 - 2 us alone), HBM delivers 16 tokens of one kv head to an SM in 0.4 us at head_dim 128: it takes
+// many warps per SM, each with a tile of its own, to keep up.  16-byte copies by the warp itself serve that: small TMA
+// boxes from one producer thread do not (22 us for 18.8 MB of one layer), and boxes shared by a block's warps leave
+// too few of them (17 us; this form 15).  192 MB of one layer (28 / 4 / 128 at 47000 rows): 42 us.
+template <int HD, int NW, bool ROWS>
+__global__ void __launch_bounds__(NW * 32, ROWS ? 1 : 2) decodeKvKernel(const __grid_constant__ DecodeKvParams p) {
+    using L = DecodeKvSmem<HD, NW>;
+    constexpr int T = 16, NB = L::NB;
     constexpr int KS = HD / 8;   // tf32 k-steps of the QK product
     constexpr int MTO = HD / 16;  // 16-dim output tiles
 
@@ -71,71 +56,64 @@ decodeKvKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
 
     extern __shared__ uint8_t smemRaw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
-    uint64_t *fullBar = reinterpret_cast<uint64_t *>(smem + L::kBarOffset);
-    uint64_t *emptyBar = fullBar + NSTAGE;
+    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smemRaw) + 127) & ~uintptr_t(127));
     __shared__ float pScratch[NW][16 * 8];
 
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < NSTAGE; ++s) {
-            mbarInit(&fullBar[s], 1);
-            mbarInit(&emptyBar[s], NW);
-        }
-        fenceBarrierInit();
-        tmaPrefetchDesc(&tmK);
-        tmaPrefetchDesc(&tmV);
-    }
-    __syncthreads();
+    gridDepWait();
+    gridDepLaunch();
 
     uint32_t pos = p.devPos ? p.devPos[0] : 0u;
-    uint32_t len;
-    uint32_t rowsPos = p.cachePos;
-    if (p.rowsMode) {
+    uint32_t len, rowsPos = p.cachePos;
+    if (ROWS) {
         if (p.devPos) rowsPos = pos;
         len = rowsPos + min(p.qRows, b * 8u + 8u);
     } else {
-        len = p.devPos ? pos + 1u : p.lenHost;
+        len = p.devPos ? min(pos, p.lenHost - 1u) + 1u : p.lenHost;  // (the host's length is the upper bound)
     }
-    const uint32_t t0 = chunk * p.chunkTokens;
-    if (t0 >= len) return;
-    const uint32_t t1 = min(len, t0 + p.chunkTokens);
-    const uint32_t nTiles = (t1 - t0 + T - 1) / T;
-    const uint32_t kvHead0 = p.rowsMode ? hg / p.group : hg * HPC;
+    // A launch sized for a window shares the rows there are among all its blocks; the merge counts them the same way.
+    const uint32_t share = ROWS ? len : (p.devPos ? tokensPerBlock(len, gridDim.x) : p.chunkTokens);
+    const uint32_t t0 = ROWS ? 0u : chunk * share;
+    if (!ROWS && t0 >= len && clusterSize() == 1) return;
+    const uint32_t t1 = min(len, t0 + share);
+    const uint32_t nTiles = t0 < t1 ? (t1 - t0 + T - 1) / T : 0u;
+    const uint32_t kvHead = ROWS ? hg / p.group : hg;
 
-    if (warp == NW) {
-        if (lane == 0) {
-            for (uint32_t it = 0; it < nTiles; ++it) {
-                const uint32_t s = it % NSTAGE;
-                if (it >= NSTAGE) {
-                    if (!mbarWaitClock(&emptyBar[s], ((it / NSTAGE) - 1) & 1, p.err, kDevErrEmptyWait)) break;
-                }
-                uint8_t *st = smem + s * L::kStageBytes;
-                const int row = static_cast<int>(t0 + it * T);
-                mbarExpectTx(&fullBar[s], L::kStageBytes);
-#pragma unroll
-                for (int h = 0; h < HPC; ++h) {
-#pragma unroll
-                    for (int bx = 0; bx < NB; ++bx) {
-                        const int sub = (h * NB + bx) * T * 128;
-                        tmaLoad3D(st + sub, &tmK, &fullBar[s], 32 * bx, kvHead0 + h, row);
-                        tmaLoad3D(st + L::kTileBytes + sub, &tmV, &fullBar[s], 32 * bx, kvHead0 + h, row);
-                    }
+    // Tile j belongs to warp j % NW.  A warp copies its own tiles: the next tile's K while it works on this one's V,
+    // the next V while it works on K.
+    uint8_t *slotK = smem + warp * 2 * L::kTileBytes, *slotV = slotK + L::kTileBytes;
+    const uint32_t stride = p.nKV * HD * 4;
+    const uint8_t *storeK = static_cast<const uint8_t *>(p.kvK) + static_cast<size_t>(kvHead) * HD * 4;
+    const uint8_t *storeV = static_cast<const uint8_t *>(p.kvV) + static_cast<size_t>(kvHead) * HD * 4;
+    auto requestK = [&](uint32_t j) {
+        if (j < nTiles) {
+            if (!ROWS && p.tok.k != nullptr && j + 1 == nTiles && t1 == len) {
+                // the tile that holds the new token's row: the row goes in first
+                if (p.devPos && pos >= p.totalRows) {  // a device position outside the store: no row written, and said so
+                    if (lane == 0) atomicOr(p.err, kDevErrRowBound);
+                } else {
+                    const size_t at = (static_cast<size_t>(len - 1u) * p.nKV + kvHead) * HD;
+                    appendRow<HD, float>(p.tok, kvHead, static_cast<float *>(p.kvK) + at, static_cast<float *>(p.kvV) + at,
+                                         len - 1u, lane);
                 }
             }
+            copyTile<T, HD * 4>(smemAddr(slotK), storeK, stride, t0 + j * T, p.totalRows - 1, lane);
         }
-        return;
-    }
-
-    // -------------------------------- consumers --------------------------------
-    const uint32_t g = lane >> 2, t = lane & 3u;
-    const uint32_t hL = warp % HPC, sub = warp / HPC;
-    const uint32_t kvHead = kvHead0 + hL;
-    auto colValid = [&](uint32_t j) { return p.rowsMode ? (b * 8u + j < p.qRows) : (p.colBase + j < p.group); };
-    auto colIndex = [&](uint32_t j) -> size_t {
-        return p.rowsMode ? (static_cast<size_t>(b) * 8u + j) * p.nHeads + hg
-                          : static_cast<size_t>(b) * p.nHeads + kvHead * p.group + p.colBase + j;
+        cpAsyncCommit();
     };
-    auto colLen = [&](uint32_t j) { return p.rowsMode ? min(t1, rowsPos + b * 8u + j + 1u) : t1; };
+    auto requestV = [&](uint32_t j) {
+        if (j < nTiles) copyTile<T, HD * 4>(smemAddr(slotV), storeV, stride, t0 + j * T, p.totalRows - 1, lane);
+        cpAsyncCommit();
+    };
+    requestK(warp);
+    requestV(warp);
+
+    const uint32_t g = lane >> 2, t = lane & 3u;
+    auto colValid = [&](uint32_t j) { return ROWS ? (b * 8u + j < p.qRows) : (p.colBase + j < p.group); };
+    auto colIndex = [&](uint32_t j) -> size_t {
+        return ROWS ? (static_cast<size_t>(b) * 8u + j) * p.nHeads + hg
+                    : static_cast<size_t>(kvHead) * p.group + p.colBase + j;
+    };
+    auto colLen = [&](uint32_t j) { return ROWS ? min(t1, rowsPos + b * 8u + j + 1u) : t1; };
 
     // q of column n = g as the B operand: k slot t / t+4 of step (bx, h, e) is
     // dim 32bx + 8t + 4h + 2e / +1 -- the order the swizzled 16-byte loads deliver.
@@ -143,12 +121,41 @@ decodeKvKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
     {
         const bool valid = colValid(g);
         const float *qp = p.q + colIndex(valid ? g : 0) * HD;
+        float4 qv[NB][2];
+        // (plain loads: with a rotation q is written in place at the end of the launch)
+#pragma unroll
+        for (int bx = 0; bx < NB; ++bx)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                qv[bx][h] = valid ? *reinterpret_cast<const float4 *>(qp + 32 * bx + 8 * t + 4 * h)
+                                  : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (!ROWS && p.tok.cosT != nullptr) {
+            // NEOX rotation: the partner of dim d is d + HD / 2, NB / 2 boxes further on
+            const size_t row = static_cast<size_t>(len - 1u) * (HD / 2);
+#pragma unroll
+            for (int bx = 0; bx < NB / 2; ++bx)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int d = 32 * bx + 8 * t + 4 * h;
+                    const float4 c = __ldg(reinterpret_cast<const float4 *>(p.tok.cosT + row + d));
+                    const float4 s = __ldg(reinterpret_cast<const float4 *>(p.tok.sinT + row + d));
+                    float4 &x = qv[bx][h], &y = qv[bx + NB / 2][h];
+                    auto rot = [](float &x0, float &x1, float cc, float ss) {
+                        const float a = fmaf(x0, cc, -__fmul_rn(x1, ss));
+                        x1 = fmaf(x0, ss, __fmul_rn(x1, cc));
+                        x0 = a;
+                    };
+                    rot(x.x, y.x, c.x, s.x);
+                    rot(x.y, y.y, c.y, s.y);
+                    rot(x.z, y.z, c.z, s.z);
+                    rot(x.w, y.w, c.w, s.w);
+                }
+        }
 #pragma unroll
         for (int bx = 0; bx < NB; ++bx)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const float4 v = valid ? __ldg(reinterpret_cast<const float4 *>(qp + 32 * bx + 8 * t + 4 * h))
-                                       : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 v = qv[bx][h];
                 const int ks = (bx * 2 + h) * 2;
                 splitTf32(v.x, qhi[ks][0], qlo[ks][0]);
                 splitTf32(v.y, qhi[ks][1], qlo[ks][1]);
@@ -165,17 +172,17 @@ decodeKvKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
     for (int i = 0; i < MTO; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
     float *pS = pScratch[warp];
 
-    for (uint32_t it = 0; it < nTiles; ++it) {
-        const uint32_t s = it % NSTAGE;
-        if (!mbarWaitClock(&fullBar[s], (it / NSTAGE) & 1, p.err, kDevErrFullWait)) break;
-        const uint8_t *st = smem + s * L::kStageBytes;
-        const uint32_t tokA = t0 + it * T + sub * 16 + g, tokB = tokA + 8;
+    for (uint32_t tile = warp; tile < nTiles; tile += NW) {
+        cpAsyncWait<1>();  // K of this tile is in, V may still be on its way
+        const uint32_t tok0 = t0 + tile * T;
+        const uint32_t tokA = tok0 + g, tokB = tokA + 8;
 
         // ---- S^T = K . Q^T (16 tokens x 8 columns), 3xTF32 ----
-        float sa[4] = {0.f, 0.f, 0.f, 0.f}, sb[4] = {0.f, 0.f, 0.f, 0.f};
+        // (two k steps in flight, the three products of a step in chains of their own)
+        float sa[2][4] = {}, sb[2][4] = {}, sc[2][4] = {};
 #pragma unroll
         for (int bx = 0; bx < NB; ++bx) {
-            const uint8_t *kT = st + ((hL * NB + bx) * T + sub * 16) * 128;
+            const uint8_t *kT = slotK + bx * T * 128;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const uint32_t off = ((2 * t + h) ^ g) << 4;
@@ -188,9 +195,9 @@ decodeKvKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
                     splitTf32(xb.x, h1, l1_);
                     splitTf32(xa.y, h2, l2_);
                     splitTf32(xb.y, h3, l3_);
-                    mmaTf32(sa, h0, h1, h2, h3, qhi[ks][0], qhi[ks][1]);
-                    mmaTf32(sb, l0_, l1_, l2_, l3_, qhi[ks][0], qhi[ks][1]);
-                    mmaTf32(sb, h0, h1, h2, h3, qlo[ks][0], qlo[ks][1]);
+                    mmaTf32(sa[0], h0, h1, h2, h3, qhi[ks][0], qhi[ks][1]);
+                    mmaTf32(sb[0], l0_, l1_, l2_, l3_, qhi[ks][0], qhi[ks][1]);
+                    mmaTf32(sc[0], h0, h1, h2, h3, qlo[ks][0], qlo[ks][1]);
                 }
                 {
                     uint32_t h0, l0_, h1, l1_, h2, l2_, h3, l3_;
@@ -198,16 +205,19 @@ decodeKvKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
                     splitTf32(xb.z, h1, l1_);
                     splitTf32(xa.w, h2, l2_);
                     splitTf32(xb.w, h3, l3_);
-                    mmaTf32(sa, h0, h1, h2, h3, qhi[ks + 1][0], qhi[ks + 1][1]);
-                    mmaTf32(sb, l0_, l1_, l2_, l3_, qhi[ks + 1][0], qhi[ks + 1][1]);
-                    mmaTf32(sb, h0, h1, h2, h3, qlo[ks + 1][0], qlo[ks + 1][1]);
+                    mmaTf32(sa[1], h0, h1, h2, h3, qhi[ks + 1][0], qhi[ks + 1][1]);
+                    mmaTf32(sb[1], l0_, l1_, l2_, l3_, qhi[ks + 1][0], qhi[ks + 1][1]);
+                    mmaTf32(sc[1], h0, h1, h2, h3, qlo[ks + 1][0], qlo[ks + 1][1]);
                 }
             }
         }
-        const float s00 = tokA < len0 ? (sa[0] + sb[0]) * cs : -INFINITY;
-        const float s01 = tokA < len1 ? (sa[1] + sb[1]) * cs : -INFINITY;
-        const float s10 = tokB < len0 ? (sa[2] + sb[2]) * cs : -INFINITY;
-        const float s11 = tokB < len1 ? (sa[3] + sb[3]) * cs : -INFINITY;
+        __syncwarp();  // every lane has read its part of K
+        requestK(tile + NW);
+        auto dot = [&](int i) { return (sa[0][i] + sa[1][i]) + ((sb[0][i] + sb[1][i]) + (sc[0][i] + sc[1][i])); };
+        const float s00 = tokA < len0 ? dot(0) * cs : -INFINITY;
+        const float s01 = tokA < len1 ? dot(1) * cs : -INFINITY;
+        const float s10 = tokB < len0 ? dot(2) * cs : -INFINITY;
+        const float s11 = tokB < len1 ? dot(3) * cs : -INFINITY;
         float mx0 = fmaxf(s00, s10), mx1 = fmaxf(s01, s11);
 #pragma unroll
         for (int off = 4; off <= 16; off <<= 1) {
@@ -247,13 +257,14 @@ decodeKvKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
         }
         __syncwarp();
         // ---- O^T += V^T . P^T (HD dims x 8 columns), 3xTF32 ----
+        cpAsyncWait<1>();  // V of this tile is in, the next K may still be on its way
 #pragma unroll
         for (int kk = 0; kk < 2; ++kk) {
             const uint32_t ra = 8 * kk + 2 * t, rb = ra + 1;  // token rows of k slots t and t+4
-            const bool okA = t0 + it * T + sub * 16 + ra < t1, okB = t0 + it * T + sub * 16 + rb < t1;
+            const bool okA = tok0 + ra < t1, okB = tok0 + rb < t1;
 #pragma unroll
             for (int bx = 0; bx < NB; ++bx) {
-                const uint8_t *vT = st + L::kTileBytes + ((hL * NB + bx) * T + sub * 16) * 128;
+                const uint8_t *vT = slotV + bx * T * 128;
                 float4 xa = *reinterpret_cast<const float4 *>(vT + ra * 128 + ((g ^ (ra & 7u)) << 4));
                 float4 xb = *reinterpret_cast<const float4 *>(vT + rb * 128 + ((g ^ (rb & 7u)) << 4));
                 if (!okA) xa = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -281,10 +292,10 @@ decodeKvKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
             }
         }
         __syncwarp();
-        if (lane == 0) mbarArrive(&emptyBar[s]);
+        requestV(tile + NW);
     }
 
-    // ---- fold the consumer warps of each kv head, write the chunk partial ----
+    // ---- fold the consumer warps, then the blocks of the cluster ----
 #pragma unroll
     for (int off = 4; off <= 16; off <<= 1) {
         l0 += __shfl_xor_sync(0xffffffffu, l0, off);
@@ -309,49 +320,56 @@ decodeKvKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
         wO[8 * HD + 8 + 2 * t + 1] = l1;
     }
     namedBarSync(1, NW * 32);
+    if (!ROWS) {
+        FoldTarget f;
+        f.out = p.out, f.pAcc = p.pAcc, f.pM = p.pM, f.pL = p.pL;
+        f.numChunks = p.numChunks, f.slot = chunk / clusterSize();
+        f.firstHead = static_cast<uint32_t>(colIndex(0)), f.nValid = min(8u, p.group - p.colBase);
+        f.direct = p.directOut;
+        f.qRot = p.tok.qRot != nullptr ? p.tok.qRot + colIndex(0) * HD : nullptr;
+        f.cosT = p.tok.cosT, f.sinT = p.tok.sinT, f.tableRow = len - 1u;
+        clusterFold<HD, NW>(scr, f, threadIdx.x);
+        return;
+    }
     constexpr int NV = HD / 4;  // float4 per output vector
-    for (uint32_t idx = threadIdx.x; idx < HPC * 8 * NV; idx += NW * 32) {
-        const uint32_t d4 = idx % NV, j = (idx / NV) & 7u, h = idx / (NV * 8);
+    for (uint32_t idx = threadIdx.x; idx < 8 * NV; idx += NW * 32) {
+        const uint32_t d4 = idx % NV, j = idx / NV;
         if (!colValid(j)) continue;
         float M = kNegBig;
 #pragma unroll
-        for (int sb2 = 0; sb2 < NSUB; ++sb2) M = fmaxf(M, scr[(sb2 * HPC + h) * kWarpScr + 8 * HD + j]);
+        for (int w = 0; w < NW; ++w) M = fmaxf(M, scr[w * kWarpScr + 8 * HD + j]);
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
         float lsum = 0.0f;
 #pragma unroll
-        for (int sb2 = 0; sb2 < NSUB; ++sb2) {
-            const float *w = scr + (sb2 * HPC + h) * kWarpScr;
-            const float wgt = fastExp2(w[8 * HD + j] - M);
-            lsum += wgt * w[8 * HD + 8 + j];
-            const float4 a = *reinterpret_cast<const float4 *>(w + j * HD + 4 * d4);
+        for (int w = 0; w < NW; ++w) {
+            const float *s = scr + w * kWarpScr;
+            const float wgt = fastExp2(s[8 * HD + j] - M);
+            lsum += wgt * s[8 * HD + 8 + j];
+            const float4 a = *reinterpret_cast<const float4 *>(s + j * HD + 4 * d4);
             acc.x = fmaf(wgt, a.x, acc.x);
             acc.y = fmaf(wgt, a.y, acc.y);
             acc.z = fmaf(wgt, a.z, acc.z);
             acc.w = fmaf(wgt, a.w, acc.w);
         }
-        const size_t oidx = p.rowsMode ? (static_cast<size_t>(b) * 8u + j) * p.nHeads + hg
-                                       : static_cast<size_t>(b) * p.nHeads + (kvHead0 + h) * p.group + p.colBase + j;
-        if (p.directOut) {
-            const float inv = lsum > 0.0f ? 1.0f / lsum : 0.0f;
-            *reinterpret_cast<float4 *>(p.out + oidx * HD + 4 * d4) =
-                    make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
-        } else {
-            const size_t pidx = oidx * p.numChunks + chunk;
-            *reinterpret_cast<float4 *>(p.pAcc + pidx * HD + 4 * d4) = acc;
-            if (d4 == 0) {
-                p.pM[pidx] = M > -1e29f ? M * 0.6931471805599453f : kNegBig;
-                p.pL[pidx] = lsum;
-            }
-        }
+        const float inv = lsum > 0.0f ? 1.0f / lsum : 0.0f;
+        *reinterpret_cast<float4 *>(p.out + colIndex(j) * HD + 4 * d4) =
+                make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
     }
 }
 
-template <int HD, int NW, int HPC>
-static int launchKv(const CUtensorMap &tmK, const CUtensorMap &tmV, const DecodeKvParams &prm, dim3 grid,
-                    cudaStream_t st) {
-    constexpr int NSTAGE = 3;
-    using L = DecodeKvSmem<HD, NW, HPC, NSTAGE>;
-    auto kern = decodeKvKernel<HD, NW, HPC, NSTAGE>;
+// As many warps as the registers and the shared memory of an SM carry for two decode blocks (16-block clusters find room
+// twice per GPC then), or for one block of the causal form.
+template <int HD>
+struct KvShape {
+    static constexpr int kWarps = HD == 64 ? 8 : (HD == 128 ? 6 : 3);
+    static constexpr int kRowsWarps = HD == 64 ? 16 : (HD == 128 ? 12 : 6);
+};
+
+template <int HD>
+static int launchRows(const DecodeKvParams &prm, cudaStream_t st) {
+    constexpr int NW = KvShape<HD>::kRowsWarps;
+    using L = DecodeKvSmem<HD, NW>;
+    auto kern = decodeKvKernel<HD, NW, true>;
     static bool attrDone[64] = {false};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -359,41 +377,7 @@ static int launchKv(const CUtensorMap &tmK, const CUtensorMap &tmV, const Decode
         TC_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
         attrDone[dev] = true;
     }
-    kern<<<grid, (NW + 1) * 32, L::kTotal, st>>>(tmK, tmV, prm);
-    TC_CUDA_OK(cudaGetLastError());
-    return TC_OK;
-}
-
-template <int HD, int NW>
-static int launchKvHpc(uint32_t hpc, const CUtensorMap &tmK, const CUtensorMap &tmV, const DecodeKvParams &prm,
-                       dim3 grid, cudaStream_t st) {
-    if constexpr (NW % 4 == 0) {
-        if (hpc == 4) return launchKv<HD, NW, 4>(tmK, tmV, prm, grid, st);
-    }
-    if (hpc == 2) return launchKv<HD, NW, 2>(tmK, tmV, prm, grid, st);
-    return launchKv<HD, NW, 1>(tmK, tmV, prm, grid, st);
-}
-
-static int kvMaps(const void *kvK, const void *kvV, uint32_t nKV, uint32_t hd, uint64_t totalRows, uint32_t boxRows,
-                  CUtensorMap *tmK, CUtensorMap *tmV) {
-    TensorMapKey key;
-    memset(&key, 0, sizeof(key));
-    key.rank = 3;
-    key.elemBytes = 4;
-    key.swizzle = 3;
-    key.dims[0] = hd;
-    key.dims[1] = nKV;
-    key.dims[2] = totalRows;
-    key.strides[0] = static_cast<uint64_t>(hd) * 4;
-    key.strides[1] = static_cast<uint64_t>(nKV) * hd * 4;
-    key.box[0] = 32;
-    key.box[1] = 1;
-    key.box[2] = boxRows;
-    key.base = kvK;
-    int rc = getTensorMap(key, tmK);
-    if (rc != TC_OK) return rc;
-    key.base = kvV;
-    return getTensorMap(key, tmV);
+    return launchDependent(kern, dim3(1, prm.nHeads, (prm.qRows + 7) / 8), NW * 32, L::kTotal, st, 1, prm);
 }
 
 static int kvCommonChecks(const char *who, const float *q, const void *kvK, const void *kvV, float *out,
@@ -425,12 +409,6 @@ static int prefillKv(const float *q, const void *kvK, const void *kvV, float *ou
     }
     const uint32_t rowBlocks = (seqLen + 7) / 8;
     TC_REQUIRE(rowBlocks <= 65535 && nHeads <= 65535, TC_EUNSUPPORTED, "prefill_kv: %u rows x %u heads", seqLen, nHeads);
-    if (kvHalf)
-        return prefillKv16(q, kvK, kvV, out, seqLen, nHeads, nKV, hd, cachePos, devPos, totalRows, invSqrt, st);
-    const uint32_t nw = hd == 64 ? 8u : (hd == 128 ? 4u : 2u);  // consumer warps: 16 rows of K and V each per stage
-    CUtensorMap tmK, tmV;
-    rc = kvMaps(kvK, kvV, nKV, hd, totalRows, nw * 16u, &tmK, &tmV);
-    if (rc != TC_OK) return rc;
     DecodeKvParams prm;
     memset(&prm, 0, sizeof(prm));
     prm.q = q;
@@ -440,19 +418,62 @@ static int prefillKv(const float *q, const void *kvK, const void *kvV, float *ou
     prm.nHeads = nHeads;
     prm.nKV = nKV;
     prm.group = nHeads / nKV;
-    prm.chunkTokens = 0xffffff00u;
     prm.numChunks = 1;
-    prm.rowsMode = 1;
+    prm.kvK = const_cast<void *>(kvK), prm.kvV = const_cast<void *>(kvV);
     prm.qRows = seqLen;
     prm.cachePos = cachePos;
     prm.invSqrt = invSqrt;
     prm.directOut = 1;
     prm.err = devErrorWord();
     TC_REQUIRE(prm.err != nullptr, TC_ECUDA, "prefill_kv: no device error word");
-    dim3 grid(1, nHeads, rowBlocks);
-    if (hd == 64) return launchKv<64, 8, 1>(tmK, tmV, prm, grid, st);
-    if (hd == 256) return launchKv<256, 2, 1>(tmK, tmV, prm, grid, st);
-    return launchKv<128, 4, 1>(tmK, tmV, prm, grid, st);
+    if (kvHalf) return prefillKv16(prm, hd, st);
+    if (hd == 64) return launchRows<64>(prm, st);
+    if (hd == 256) return launchRows<256>(prm, st);
+    return launchRows<128>(prm, st);
+}
+
+template <int HD>
+static int decodeKv32(const DecodeKvParams &prm, uint8_t *q81Out, cudaStream_t st) {
+    constexpr int NW = KvShape<HD>::kWarps;
+    using L = DecodeKvSmem<HD, NW>;
+    static ClusterSetup setup;
+    return launchKvDecode(setup, decodeKvKernel<HD, NW, false>, NW * 32, L::kTotal, HD, NW, 2 * L::kTileBytes,
+                          HD == 256 ? 4.2f : (HD == 128 ? 2.85f : 1.7f), HD == 256 ? 1.2f : (HD == 128 ? 0.38f : 0.2f), prm, q81Out, st);
+}
+
+int decodeKvToken(const float *q, const void *kvK, const void *kvV, float *attnOut, float *pAcc, float *pM, float *pL,
+                  uint32_t nHeads, uint32_t nKV, uint32_t hd, uint32_t pos, const uint32_t *devPos, uint64_t totalRows,
+                  uint32_t numChunks, float invSqrt, int kvHalf, uint8_t *q81Out, const NewToken &tok, cudaStream_t st) {
+    int rc = kvCommonChecks("tc_attn_decode_kv", q, kvK, kvV, attnOut, nHeads, nKV, hd, totalRows, kvHalf);
+    if (rc != TC_OK) return rc;
+    TC_REQUIRE(static_cast<uint64_t>(pos) + 1 <= totalRows, TC_ECONTEXT_FULL,
+               "tc_attn_decode_kv: position %u is outside the cache of %llu rows", pos,
+               (unsigned long long) totalRows);
+    TC_REQUIRE(numChunks >= 1, TC_EWORKSPACE, "tc_attn_decode_kv: no chunk slots");
+    DecodeKvParams prm;
+    memset(&prm, 0, sizeof(prm));
+    prm.q = q;
+    prm.out = attnOut;
+    prm.pAcc = pAcc;
+    prm.pM = pM;
+    prm.pL = pL;
+    prm.devPos = devPos;
+    prm.totalRows = totalRows;
+    prm.lenHost = pos + 1;
+    prm.nHeads = nHeads;
+    prm.nKV = nKV;
+    prm.group = nHeads / nKV;
+    prm.numChunks = numChunks;
+    prm.invSqrt = invSqrt;
+    prm.tok = tok;
+    prm.kvHalf = kvHalf != 0;
+    prm.kvK = const_cast<void *>(kvK), prm.kvV = const_cast<void *>(kvV);
+    prm.err = devErrorWord();
+    TC_REQUIRE(prm.err != nullptr, TC_ECUDA, "tc_attn_decode_kv: no device error word");
+    if (kvHalf) return decodeKv16(prm, hd, q81Out, st);
+    if (hd == 64) return decodeKv32<64>(prm, q81Out, st);
+    if (hd == 128) return decodeKv32<128>(prm, q81Out, st);
+    return decodeKv32<256>(prm, q81Out, st);
 }
 
 }  // namespace tc
@@ -470,60 +491,17 @@ int tc_attn_decode_kv(const float *q, const void *kvK, const void *kvV, float *a
                       float *pL, uint32_t seqLen, uint32_t nHeads, uint32_t nKV, uint32_t hd, uint32_t pos,
                       const uint32_t *devPos, uint64_t totalRows, uint32_t numChunks, uint32_t chunkSize,
                       float invSqrt, int kvHalf, uint8_t *q81Out, tc_stream stream) {
-    using namespace tc;
     (void) chunkSize;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (seqLen != 1) {
         // the reference only splits single-token decode; several rows take the causal kernel
         TC_REQUIRE(q81Out == nullptr, TC_EUNSUPPORTED, "tc_attn_decode_kv: Q8_1 output needs seqLen == 1");
-        return prefillKv(q, kvK, kvV, attnOut, seqLen, nHeads, nKV, hd, pos, devPos, totalRows, invSqrt, kvHalf, st);
+        return tc::prefillKv(q, kvK, kvV, attnOut, seqLen, nHeads, nKV, hd, pos, devPos, totalRows, invSqrt, kvHalf, st);
     }
-    int rc = kvCommonChecks("tc_attn_decode_kv", q, kvK, kvV, attnOut, nHeads, nKV, hd, totalRows, kvHalf);
-    if (rc != TC_OK) return rc;
-    TC_REQUIRE(static_cast<uint64_t>(pos) + 1 <= totalRows, TC_ECONTEXT_FULL,
-               "tc_attn_decode_kv: position %u is outside the cache of %llu rows", pos,
-               (unsigned long long) totalRows);
-    TC_REQUIRE(numChunks >= 1, TC_EWORKSPACE, "tc_attn_decode_kv: no chunk slots");
-    if (kvHalf)
-        return decodeKv16(q, kvK, kvV, attnOut, pAcc, pM, pL, nHeads, nKV, hd, pos, devPos, totalRows, numChunks,
-                          invSqrt, q81Out, st);
-    const uint32_t nw = hd == 64 ? 8u : (hd == 128 ? 4u : 2u);
-    DecodePlan pl = planDecode(1, nKV, pos + 1, numChunks, nw * 16u, true, nw >= 4u ? 4u : 2u);
-    const bool direct = pl.chunksPerSeq == 1 && q81Out == nullptr;
-    if (!direct) TC_REQUIRE(pAcc && pM && pL, TC_EWORKSPACE, "tc_attn_decode_kv: partial buffers are required");
-    CUtensorMap tmK, tmV;
-    rc = kvMaps(kvK, kvV, nKV, hd, totalRows, pl.tileTokens, &tmK, &tmV);
-    if (rc != TC_OK) return rc;
-    DecodeKvParams prm;
-    memset(&prm, 0, sizeof(prm));
-    prm.q = q;
-    prm.out = attnOut;
-    prm.pAcc = pAcc;
-    prm.pM = pM;
-    prm.pL = pL;
-    prm.devPos = devPos;
-    prm.totalRows = totalRows;
-    prm.lenHost = pos + 1;
-    prm.nHeads = nHeads;
-    prm.nKV = nKV;
-    prm.group = nHeads / nKV;
-    prm.chunkTokens = pl.chunkTokens;
-    prm.numChunks = numChunks;
-    prm.invSqrt = invSqrt;
-    prm.directOut = direct ? 1 : 0;
-    prm.err = devErrorWord();
-    TC_REQUIRE(prm.err != nullptr, TC_ECUDA, "tc_attn_decode_kv: no device error word");
-    dim3 grid(pl.chunksPerSeq, pl.headGroups, 1);
-    for (uint32_t cb = 0; cb < prm.group; cb += 8) {  // 8 q heads of a kv head per launch
-        prm.colBase = cb;
-        rc = hd == 64    ? launchKvHpc<64, 8>(pl.hpc, tmK, tmV, prm, grid, st)
-             : hd == 128 ? launchKvHpc<128, 4>(pl.hpc, tmK, tmV, prm, grid, st)
-                         : launchKvHpc<256, 2>(pl.hpc, tmK, tmV, prm, grid, st);
-        if (rc != TC_OK) return rc;
-    }
-    if (direct) return TC_OK;
-    return launchMerge(pAcc, pM, pL, attnOut, 1, nHeads, numChunks, pl.chunksPerSeq, hd, devPos, devPos ? 1u : 0u,
-                       pl.chunkTokens, q81Out, false, st);
+    tc::NewToken none;
+    memset(&none, 0, sizeof(none));
+    return tc::decodeKvToken(q, kvK, kvV, attnOut, pAcc, pM, pL, nHeads, nKV, hd, pos, devPos, totalRows, numChunks, invSqrt,
+                             kvHalf, q81Out, none, st);
 }
 
 }  // extern "C"

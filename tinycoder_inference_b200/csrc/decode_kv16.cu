@@ -7,129 +7,99 @@
 // dense models' optional fp16 cache (src/cpp/core/cuda/forward/GPUComputeUpload.cu:1252):
 // score = dot(q, float(k)) * invSqrt, online softmax with exp2, out = sum p float(v) / sum p.
 //
-// Same skeleton as the int8 kernel (decode_i8.cu) -- grid (chunks, kv-head groups, sequences
-// or row blocks), a TMA producer warp feeding an mbarrier ring, eight consumer warps that own
-// a (kv head, 16-token) tile per stage and serve every q head of the kv head -- with the
-// natural operands: fp16 K and V go into mma.sync.m16n8k16 as they are (ldmatrix for K,
+// Same skeleton as the f32 kernel (decode_kv.cu) -- a block streams a token range of one kv head,
+// its warps take 16-token tiles in turn and serve every q head of the kv head, decode_cluster.cuh
+// around it -- with the natural operands: fp16 K and V go into mma.sync.m16n8k16 as they are (ldmatrix for K,
 // ldmatrix.trans for V, both straight from the 128-byte-swizzled TMA tiles), q and p are
 // carried as fp16 hi + lo pairs (two MMAs, ~22 mantissa bits) after a power-of-two
 // normalisation of q, accumulation is f32.  Nothing is rounded that the reference does not
 // round: float(k) and float(v) are exact.
-#include "decode_shared.cuh"
+#include "decode_cluster.cuh"
 
 namespace tc {
 
-struct DecodeKv16Params {
-    const float *q;
-    float *out;
-    float *pAcc, *pM, *pL;
-    const uint32_t *devPos;  // nullable: position read at kernel time
-    uint64_t totalRows;
-    uint32_t lenHost;
-    uint32_t nHeads, nKV, group;
-    uint32_t colBase;  // heads mode: the 8 MMA columns are q heads colBase .. colBase + 7 of the kv head
-    uint32_t chunkTokens, numChunks;
-    uint32_t rowsMode, qRows, cachePos;  // rows mode: see decode_i8.cu
-    float invSqrt;
-    int directOut;
-    unsigned int *err;
-};
-
-// A stage holds K then V; each as HD/64 half-tiles of [rows][64 halves = 128 bytes] (one
-// swizzle span), half-tile a covering dims [64a, 64a + 64).
-template <int HD, int HPC, int NW, int NSTAGE>
+// Every warp has a slot for a 16-token tile of K and one of V, each as HD / 64 half-tiles of [16 rows][64 halves =
+// 128 bytes], half-tile a covering dims [64a, 64a + 64).
+template <int HD, int NW>
 struct DecodeKv16Smem {
-    static constexpr int kAtoms = HD / 64;
-    static constexpr int kRows = NW * 16;            // (token, head) rows per stage
-    static constexpr int T = kRows / HPC;            // tokens per stage
-    static constexpr int kAtomBytes = kRows * 128;   // one half-tile, all HPC heads
-    static constexpr int kTileBytes = kRows * HD * 2;
-    static constexpr int kStageBytes = 2 * kTileBytes;
-    static constexpr int kBarOffset = NSTAGE * kStageBytes;
-    static constexpr int kTotal = kBarOffset + 2 * NSTAGE * 8 + 1024;
-    static_assert(T % 8 == 0 && T <= 256, "box rows");
-    static_assert(kTotal <= 227 * 1024, "ring exceeds the shared memory of an SM");
+    static constexpr int kAtomBytes = 16 * 128;      // one half-tile
+    static constexpr int kTileBytes = 16 * HD * 2;
+    static constexpr int kSlots = NW * 2 * kTileBytes, kScratch = (NW + 1) * (8 * HD + 16) * 4;  // (the fold reuses the slots)
+    static constexpr int kTotal = (kSlots > kScratch ? kSlots : kScratch) + 128;
+    static_assert(kTotal <= 227 * 1024, "shared memory of an SM");
 };
 
 constexpr float kLazyLog2Kv16 = 8.0f;  // see decode_i8.cu: p stays <= 2^8, exact enough as fp16 hi + lo
 
-template <int HD, int HPC, int NW, int NSTAGE>
-__global__ void __launch_bounds__((NW + 1) * 32, 1)
-decodeKv16Kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
-                 const DecodeKv16Params p) {
-    using L = DecodeKv16Smem<HD, HPC, NW, NSTAGE>;
-    constexpr int T = L::T;
+// ROWS: the causal kernel (one block per 8 query rows and q head); otherwise decode, blocks of a cluster
+// share a kv head's tokens.
+template <int HD, int NW, bool ROWS>
+__global__ void __launch_bounds__(NW * 32, ROWS ? 1 : 2) decodeKv16Kernel(const __grid_constant__ DecodeKvParams p) {
+    using L = DecodeKv16Smem<HD, NW>;
+    constexpr int T = 16;
     constexpr int NS = HD / 16;     // k16 steps of QK^T = 16-dim output tiles of PV
-    constexpr int NSUB = NW / HPC;  // consumer warps per kv head
 
     const uint32_t chunk = blockIdx.x, hg = blockIdx.y, b = blockIdx.z;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
 
     extern __shared__ uint8_t smemRaw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
-    uint64_t *fullBar = reinterpret_cast<uint64_t *>(smem + L::kBarOffset);
-    uint64_t *emptyBar = fullBar + NSTAGE;
+    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smemRaw) + 127) & ~uintptr_t(127));
 
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < NSTAGE; ++s) {
-            mbarInit(&fullBar[s], 1);
-            mbarInit(&emptyBar[s], NW);
-        }
-        fenceBarrierInit();
-        tmaPrefetchDesc(&tmK);
-        tmaPrefetchDesc(&tmV);
-    }
-    __syncthreads();
+    gridDepWait();
+    gridDepLaunch();
 
-    const uint32_t pos = p.devPos ? p.devPos[0] : 0u;
-    uint32_t len;
-    uint32_t rowsPos = p.cachePos;
-    if (p.rowsMode) {
+    uint32_t pos = p.devPos ? p.devPos[0] : 0u;
+    uint32_t len, rowsPos = p.cachePos;
+    if (ROWS) {
         if (p.devPos) rowsPos = pos;
         len = rowsPos + min(p.qRows, b * 8u + 8u);
     } else {
-        len = p.devPos ? pos + 1u : p.lenHost;
+        len = p.devPos ? min(pos, p.lenHost - 1u) + 1u : p.lenHost;  // (the host's length is the upper bound)
     }
-    const uint32_t t0 = chunk * p.chunkTokens;
-    if (t0 >= len) return;
-    const uint32_t t1 = min(len, t0 + p.chunkTokens);
-    const uint32_t nTiles = (t1 - t0 + T - 1) / T;
-    const uint32_t kvHead0 = p.rowsMode ? hg / p.group : hg * HPC;
+    // A launch sized for a window shares the rows there are among all its blocks; the merge counts them the same way.
+    const uint32_t share = ROWS ? len : (p.devPos ? tokensPerBlock(len, gridDim.x) : p.chunkTokens);
+    const uint32_t t0 = ROWS ? 0u : chunk * share;
+    if (!ROWS && t0 >= len && clusterSize() == 1) return;
+    const uint32_t t1 = min(len, t0 + share);
+    const uint32_t nTiles = t0 < t1 ? (t1 - t0 + T - 1) / T : 0u;
+    const uint32_t kvHead = ROWS ? hg / p.group : hg;
 
-    if (warp == NW) {
-        if (lane == 0) {
-            for (uint32_t it = 0; it < nTiles; ++it) {
-                const uint32_t s = it % NSTAGE;
-                if (it >= NSTAGE) {
-                    if (!mbarWaitClock(&emptyBar[s], ((it / NSTAGE) - 1) & 1, p.err, kDevErrEmptyWait)) break;
-                }
-                uint8_t *st = smem + s * L::kStageBytes;
-                const int row = static_cast<int>(t0 + it * T);
-                mbarExpectTx(&fullBar[s], L::kStageBytes);
-#pragma unroll
-                for (int h = 0; h < HPC; ++h) {
-#pragma unroll
-                    for (int a = 0; a < L::kAtoms; ++a) {
-                        uint8_t *dst = st + a * L::kAtomBytes + h * T * 128;
-                        tmaLoad3D(dst, &tmK, &fullBar[s], 64 * a, kvHead0 + h, row);
-                        tmaLoad3D(dst + L::kTileBytes, &tmV, &fullBar[s], 64 * a, kvHead0 + h, row);
-                    }
+    // Tile j belongs to warp j % NW.  A warp copies its own tiles: the next tile's K while it works on this one's V,
+    // the next V while it works on K.
+    uint8_t *slotK = smem + warp * 2 * L::kTileBytes, *slotV = slotK + L::kTileBytes;
+    const uint32_t stride = p.nKV * HD * 2;
+    const uint8_t *storeK = static_cast<const uint8_t *>(p.kvK) + static_cast<size_t>(kvHead) * HD * 2;
+    const uint8_t *storeV = static_cast<const uint8_t *>(p.kvV) + static_cast<size_t>(kvHead) * HD * 2;
+    auto requestK = [&](uint32_t j) {
+        if (j < nTiles) {
+            if (!ROWS && p.tok.k != nullptr && j + 1 == nTiles && t1 == len) {
+                // the tile that holds the new token's row: the row goes in first
+                if (p.devPos && pos >= p.totalRows) {  // a device position outside the store: no row written, and said so
+                    if (lane == 0) atomicOr(p.err, kDevErrRowBound);
+                } else {
+                    const size_t at = (static_cast<size_t>(len - 1u) * p.nKV + kvHead) * HD;
+                    appendRow<HD, __half>(p.tok, kvHead, static_cast<__half *>(p.kvK) + at, static_cast<__half *>(p.kvV) + at,
+                                          len - 1u, lane);
                 }
             }
+            copyTile<T, HD * 2>(smemAddr(slotK), storeK, stride, t0 + j * T, p.totalRows - 1, lane);
         }
-        return;
-    }
-
-    // -------------------------------- consumers --------------------------------
-    const uint32_t g = lane >> 2, t = lane & 3u;
-    const uint32_t hL = warp % HPC, sub = warp / HPC;
-    const uint32_t kvHead = kvHead0 + hL;
-    auto colValid = [&](uint32_t j) { return p.rowsMode ? (b * 8u + j < p.qRows) : (p.colBase + j < p.group); };
-    auto colIndex = [&](uint32_t j) -> size_t {
-        return p.rowsMode ? (static_cast<size_t>(b) * 8u + j) * p.nHeads + hg
-                          : static_cast<size_t>(b) * p.nHeads + kvHead * p.group + p.colBase + j;
+        cpAsyncCommit();
     };
-    auto colLen = [&](uint32_t j) { return p.rowsMode ? min(t1, rowsPos + b * 8u + j + 1u) : t1; };
+    auto requestV = [&](uint32_t j) {
+        if (j < nTiles) copyTile<T, HD * 2>(smemAddr(slotV), storeV, stride, t0 + j * T, p.totalRows - 1, lane);
+        cpAsyncCommit();
+    };
+    requestK(warp);
+    requestV(warp);
+
+    const uint32_t g = lane >> 2, t = lane & 3u;
+    auto colValid = [&](uint32_t j) { return ROWS ? (b * 8u + j < p.qRows) : (p.colBase + j < p.group); };
+    auto colIndex = [&](uint32_t j) -> size_t {
+        return ROWS ? (static_cast<size_t>(b) * 8u + j) * p.nHeads + hg
+                    : static_cast<size_t>(kvHead) * p.group + p.colBase + j;
+    };
+    auto colLen = [&](uint32_t j) { return ROWS ? min(t1, rowsPos + b * 8u + j + 1u) : t1; };
 
     // q of column n = g as the B operand of k16 step s: b0 = dims 16s + 2t, +1; b1 = dims
     // 16s + 8 + 2t, +1.  Power-of-two normalised, split into fp16 hi + lo.
@@ -144,10 +114,30 @@ decodeKv16Kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         for (int s = 0; s < NS; ++s)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                qv[s][h] = valid ? __ldg(reinterpret_cast<const float2 *>(qp + 16 * s + 8 * h + 2 * t))
+                // (a plain load: with a rotation q is written in place at the end of the launch)
+                qv[s][h] = valid ? *reinterpret_cast<const float2 *>(qp + 16 * s + 8 * h + 2 * t)
                                  : make_float2(0.f, 0.f);
-                amax = fmaxf(amax, fmaxf(fabsf(qv[s][h].x), fabsf(qv[s][h].y)));
             }
+        if (!ROWS && p.tok.cosT != nullptr) {
+            // NEOX rotation: the partner of dim d is d + HD / 2, NS / 2 steps further on
+            const size_t row = static_cast<size_t>(len - 1u) * (HD / 2);
+#pragma unroll
+            for (int s = 0; s < NS / 2; ++s)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int d = 16 * s + 8 * h + 2 * t;
+                    const float2 c = __ldg(reinterpret_cast<const float2 *>(p.tok.cosT + row + d));
+                    const float2 sn = __ldg(reinterpret_cast<const float2 *>(p.tok.sinT + row + d));
+                    float2 &x = qv[s][h], &y = qv[s + NS / 2][h];
+                    const float2 x0 = x, x1 = y;
+                    x = make_float2(fmaf(x0.x, c.x, -__fmul_rn(x1.x, sn.x)), fmaf(x0.y, c.y, -__fmul_rn(x1.y, sn.y)));
+                    y = make_float2(fmaf(x0.x, sn.x, __fmul_rn(x1.x, c.x)), fmaf(x0.y, sn.y, __fmul_rn(x1.y, c.y)));
+                }
+        }
+#pragma unroll
+        for (int s = 0; s < NS; ++s)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) amax = fmaxf(amax, fmaxf(fabsf(qv[s][h].x), fabsf(qv[s][h].y)));
         amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
         amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
         int e = static_cast<int>((__float_as_uint(amax) >> 23) & 0xffu) - 127;  // floor(log2 amax)
@@ -179,17 +169,14 @@ decodeKv16Kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     const uint32_t lco = lane >> 4;                             // and which 16-byte chunk of the pair
     const uint32_t lmOff = lr * 128;
 
-    for (uint32_t it = 0; it < nTiles; ++it) {
-        const uint32_t s = it % NSTAGE;
-        if (!mbarWaitClock(&fullBar[s], (it / NSTAGE) & 1, p.err, kDevErrFullWait)) break;
-        uint8_t *st = smem + s * L::kStageBytes;
-        const uint32_t rowInTile = hL * T + sub * 16;
-        const uint32_t tokW = t0 + it * T + sub * 16;  // first token of this warp's tile
+    for (uint32_t tile = warp; tile < nTiles; tile += NW) {
+        cpAsyncWait<1>();  // K of this tile is in, V may still be on its way
+        const uint32_t tokW = t0 + tile * T;  // first token of the tile
         const uint32_t tokA = tokW + g, tokB = tokA + 8;
 
         // ---- S^T = K . Q^T (16 tokens x 8 columns) ----
         float sh[4] = {0.f, 0.f, 0.f, 0.f}, sl[4] = {0.f, 0.f, 0.f, 0.f};
-        const uint32_t kTile = smemAddr(st + rowInTile * 128);
+        const uint32_t kTile = smemAddr(slotK);
 #pragma unroll
         for (int ks = 0; ks < NS; ++ks) {
             const uint32_t sw = (((2 * (ks & 3) + lco) ^ (lr & 7u)) << 4) + (ks >> 2) * L::kAtomBytes;
@@ -198,6 +185,8 @@ decodeKv16Kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
             mmaF16(sh, r0, r1, r2, r3, qhi[ks][0], qhi[ks][1]);
             mmaF16(sl, r0, r1, r2, r3, qlo[ks][0], qlo[ks][1]);
         }
+        __syncwarp();  // every lane has read its part of K
+        requestK(tile + NW);
         // a stale or foreign row behind the range may hold anything, NaN included: select, never scale
         const float s00 = tokA < len0 ? (sh[0] + sl[0]) * cs0 : -INFINITY;
         const float s01 = tokA < len1 ? (sh[1] + sl[1]) * cs1 : -INFINITY;
@@ -250,7 +239,8 @@ decodeKv16Kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
             mk0 = (tokW + 2 * t < t1 ? 0x0000ffffu : 0u) | (tokW + 2 * t + 1 < t1 ? 0xffff0000u : 0u);
             mk1 = (tokW + 8 + 2 * t < t1 ? 0x0000ffffu : 0u) | (tokW + 8 + 2 * t + 1 < t1 ? 0xffff0000u : 0u);
         }
-        const uint32_t vTile = smemAddr(st + L::kTileBytes + rowInTile * 128);
+        cpAsyncWait<1>();  // V of this tile is in, the next K may still be on its way
+        const uint32_t vTile = smemAddr(slotV);
 #pragma unroll
         for (int ks = 0; ks < NS; ++ks) {
             const uint32_t sw = (((2 * (ks & 3) + lco) ^ (lr & 7u)) << 4) + (ks >> 2) * L::kAtomBytes;
@@ -265,7 +255,7 @@ decodeKv16Kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
             mmaF16(o[ks], r0, r2, r1, r3, bl[0], bl[1]);
         }
         __syncwarp();
-        if (lane == 0) mbarArrive(&emptyBar[s]);
+        requestV(tile + NW);
     }
 
     // ---- fold the consumer warps of each kv head, write the chunk partial ----
@@ -293,49 +283,64 @@ decodeKv16Kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         wO[8 * HD + 8 + 2 * t + 1] = l1;
     }
     namedBarSync(1, NW * 32);
-    constexpr uint32_t V4 = HD / 4;
-    for (uint32_t idx = threadIdx.x; idx < HPC * 8 * V4; idx += NW * 32) {
-        const uint32_t d4 = idx % V4, j = (idx / V4) & 7u, h = idx / (8 * V4);
+    if (!ROWS) {
+        FoldTarget f;
+        f.out = p.out, f.pAcc = p.pAcc, f.pM = p.pM, f.pL = p.pL;
+        f.numChunks = p.numChunks, f.slot = chunk / clusterSize();
+        f.firstHead = static_cast<uint32_t>(colIndex(0)), f.nValid = min(8u, p.group - p.colBase);
+        f.direct = p.directOut;
+        f.qRot = p.tok.qRot != nullptr ? p.tok.qRot + colIndex(0) * HD : nullptr;
+        f.cosT = p.tok.cosT, f.sinT = p.tok.sinT, f.tableRow = len - 1u;
+        clusterFold<HD, NW>(scr, f, threadIdx.x);
+        return;
+    }
+    constexpr int NV = HD / 4;  // float4 per output vector
+    for (uint32_t idx = threadIdx.x; idx < 8 * NV; idx += NW * 32) {
+        const uint32_t d4 = idx % NV, j = idx / NV;
         if (!colValid(j)) continue;
         float M = kNegBig;
 #pragma unroll
-        for (int sb = 0; sb < NSUB; ++sb) M = fmaxf(M, scr[(sb * HPC + h) * kWarpScr + 8 * HD + j]);
+        for (int w = 0; w < NW; ++w) M = fmaxf(M, scr[w * kWarpScr + 8 * HD + j]);
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
         float lsum = 0.0f;
 #pragma unroll
-        for (int sb = 0; sb < NSUB; ++sb) {
-            const float *w = scr + (sb * HPC + h) * kWarpScr;
-            const float wgt = fastExp2(w[8 * HD + j] - M);
-            lsum += wgt * w[8 * HD + 8 + j];
-            const float4 a = *reinterpret_cast<const float4 *>(w + j * HD + 4 * d4);
+        for (int w = 0; w < NW; ++w) {
+            const float *s = scr + w * kWarpScr;
+            const float wgt = fastExp2(s[8 * HD + j] - M);
+            lsum += wgt * s[8 * HD + 8 + j];
+            const float4 a = *reinterpret_cast<const float4 *>(s + j * HD + 4 * d4);
             acc.x = fmaf(wgt, a.x, acc.x);
             acc.y = fmaf(wgt, a.y, acc.y);
             acc.z = fmaf(wgt, a.z, acc.z);
             acc.w = fmaf(wgt, a.w, acc.w);
         }
-        const size_t oidx = p.rowsMode ? (static_cast<size_t>(b) * 8u + j) * p.nHeads + hg
-                                       : static_cast<size_t>(b) * p.nHeads + (kvHead0 + h) * p.group + p.colBase + j;
-        if (p.directOut) {
-            const float inv = lsum > 0.0f ? 1.0f / lsum : 0.0f;
-            *reinterpret_cast<float4 *>(p.out + oidx * HD + 4 * d4) =
-                    make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
-        } else {
-            const size_t pidx = oidx * p.numChunks + chunk;
-            *reinterpret_cast<float4 *>(p.pAcc + pidx * HD + 4 * d4) = acc;
-            if (d4 == 0) {
-                p.pM[pidx] = M > -1e29f ? M * 0.6931471805599453f : kNegBig;
-                p.pL[pidx] = lsum;
-            }
-        }
+        const float inv = lsum > 0.0f ? 1.0f / lsum : 0.0f;
+        *reinterpret_cast<float4 *>(p.out + colIndex(j) * HD + 4 * d4) =
+                make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
     }
 }
 
-template <int HD, int HPC>
-static int launchKv16(const CUtensorMap &tmK, const CUtensorMap &tmV, const DecodeKv16Params &prm, dim3 grid,
-                      cudaStream_t st) {
-    constexpr int NW = 8, NSTAGE = HD == 128 ? 3 : 6;
-    using L = DecodeKv16Smem<HD, HPC, NW, NSTAGE>;
-    auto kern = decodeKv16Kernel<HD, HPC, NW, NSTAGE>;
+// As many warps as the registers of an SM carry for two decode blocks (16-block clusters find room twice per GPC then),
+// or for one block of the causal form.
+template <int HD>
+static int decodeKv16Hd(const DecodeKvParams &prm, uint8_t *q81Out, cudaStream_t st) {
+    constexpr int NW = 8;
+    using L = DecodeKv16Smem<HD, NW>;
+    static ClusterSetup setup;
+    return launchKvDecode(setup, decodeKv16Kernel<HD, NW, false>, NW * 32, L::kTotal, HD, NW, 2 * L::kTileBytes,
+                          HD == 128 ? 0.87f : 0.73f, HD == 128 ? 0.12f : 0.08f, prm, q81Out, st);
+}
+
+// Both are called from decode_kv.cu when kvHalf is set; arguments were validated there.
+int decodeKv16(const DecodeKvParams &prm, uint32_t hd, uint8_t *q81Out, cudaStream_t st) {
+    return hd == 64 ? decodeKv16Hd<64>(prm, q81Out, st) : decodeKv16Hd<128>(prm, q81Out, st);
+}
+
+template <int HD>
+static int rowsKv16Hd(const DecodeKvParams &prm, cudaStream_t st) {
+    constexpr int NW = 16;
+    using L = DecodeKv16Smem<HD, NW>;
+    auto kern = decodeKv16Kernel<HD, NW, true>;
     static bool attrDone[64] = {false};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -343,110 +348,11 @@ static int launchKv16(const CUtensorMap &tmK, const CUtensorMap &tmV, const Deco
         TC_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
         attrDone[dev] = true;
     }
-    kern<<<grid, (NW + 1) * 32, L::kTotal, st>>>(tmK, tmV, prm);
-    TC_CUDA_OK(cudaGetLastError());
-    return TC_OK;
+    return launchDependent(kern, dim3(1, prm.nHeads, (prm.qRows + 7) / 8), NW * 32, L::kTotal, st, 1, prm);
 }
 
-template <int HD>
-static int launchKv16Hpc(uint32_t hpc, const CUtensorMap &tmK, const CUtensorMap &tmV, const DecodeKv16Params &prm,
-                         dim3 grid, cudaStream_t st) {
-    if (hpc == 4) return launchKv16<HD, 4>(tmK, tmV, prm, grid, st);
-    if (hpc == 2) return launchKv16<HD, 2>(tmK, tmV, prm, grid, st);
-    return launchKv16<HD, 1>(tmK, tmV, prm, grid, st);
-}
-
-static int kv16Maps(const void *kvK, const void *kvV, uint32_t nKV, uint32_t hd, uint64_t totalRows,
-                    uint32_t boxRows, CUtensorMap *tmK, CUtensorMap *tmV) {
-    TensorMapKey key;
-    memset(&key, 0, sizeof(key));
-    key.rank = 3;
-    key.elemBytes = 2;
-    key.swizzle = 3;
-    key.dims[0] = hd;
-    key.dims[1] = nKV;
-    key.dims[2] = totalRows;
-    key.strides[0] = static_cast<uint64_t>(hd) * 2;
-    key.strides[1] = static_cast<uint64_t>(nKV) * hd * 2;
-    key.box[0] = 64;
-    key.box[1] = 1;
-    key.box[2] = boxRows;
-    key.base = kvK;
-    int rc = getTensorMap(key, tmK);
-    if (rc != TC_OK) return rc;
-    key.base = kvV;
-    return getTensorMap(key, tmV);
-}
-
-// Called from decode_kv.cu when kvHalf is set; arguments were validated there.
-int decodeKv16(const float *q, const void *kvK, const void *kvV, float *attnOut, float *pAcc, float *pM, float *pL,
-               uint32_t nHeads, uint32_t nKV, uint32_t hd, uint32_t pos, const uint32_t *devPos, uint64_t totalRows,
-               uint32_t numChunks, float invSqrt, uint8_t *q81Out, cudaStream_t st) {
-    DecodePlan pl = planDecode(1, nKV, pos + 1, numChunks, 8u * 16u);
-    const bool direct = pl.chunksPerSeq == 1 && q81Out == nullptr;
-    if (!direct) TC_REQUIRE(pAcc && pM && pL, TC_EWORKSPACE, "tc_attn_decode_kv: partial buffers are required");
-    CUtensorMap tmK, tmV;
-    int rc = kv16Maps(kvK, kvV, nKV, hd, totalRows, pl.tileTokens, &tmK, &tmV);
-    if (rc != TC_OK) return rc;
-    DecodeKv16Params prm;
-    memset(&prm, 0, sizeof(prm));
-    prm.q = q;
-    prm.out = attnOut;
-    prm.pAcc = pAcc;
-    prm.pM = pM;
-    prm.pL = pL;
-    prm.devPos = devPos;
-    prm.totalRows = totalRows;
-    prm.lenHost = pos + 1;
-    prm.nHeads = nHeads;
-    prm.nKV = nKV;
-    prm.group = nHeads / nKV;
-    prm.chunkTokens = pl.chunkTokens;
-    prm.numChunks = numChunks;
-    prm.invSqrt = invSqrt;
-    prm.directOut = direct ? 1 : 0;
-    prm.err = devErrorWord();
-    TC_REQUIRE(prm.err != nullptr, TC_ECUDA, "tc_attn_decode_kv: no device error word");
-    dim3 grid(pl.chunksPerSeq, pl.headGroups, 1);
-    for (uint32_t cb = 0; cb < prm.group; cb += 8) {  // 8 q heads of a kv head per launch
-        prm.colBase = cb;
-        rc = hd == 64 ? launchKv16Hpc<64>(pl.hpc, tmK, tmV, prm, grid, st)
-                      : launchKv16Hpc<128>(pl.hpc, tmK, tmV, prm, grid, st);
-        if (rc != TC_OK) return rc;
-    }
-    if (direct) return TC_OK;
-    return launchMerge(pAcc, pM, pL, attnOut, 1, nHeads, numChunks, pl.chunksPerSeq, hd, devPos, devPos ? 1u : 0u,
-                       pl.chunkTokens, q81Out, false, st);
-}
-
-int prefillKv16(const float *q, const void *kvK, const void *kvV, float *out, uint32_t seqLen, uint32_t nHeads,
-                uint32_t nKV, uint32_t hd, uint32_t cachePos, const uint32_t *devPos, uint64_t totalRows,
-                float invSqrt, cudaStream_t st) {
-    const uint32_t rowBlocks = (seqLen + 7) / 8;
-    CUtensorMap tmK, tmV;
-    int rc = kv16Maps(kvK, kvV, nKV, hd, totalRows, 8u * 16u, &tmK, &tmV);
-    if (rc != TC_OK) return rc;
-    DecodeKv16Params prm;
-    memset(&prm, 0, sizeof(prm));
-    prm.q = q;
-    prm.out = out;
-    prm.devPos = devPos;
-    prm.totalRows = totalRows;
-    prm.nHeads = nHeads;
-    prm.nKV = nKV;
-    prm.group = nHeads / nKV;
-    prm.chunkTokens = 0xffffff00u;
-    prm.numChunks = 1;
-    prm.rowsMode = 1;
-    prm.qRows = seqLen;
-    prm.cachePos = cachePos;
-    prm.invSqrt = invSqrt;
-    prm.directOut = 1;
-    prm.err = devErrorWord();
-    TC_REQUIRE(prm.err != nullptr, TC_ECUDA, "prefill_kv: no device error word");
-    dim3 grid(1, nHeads, rowBlocks);
-    if (hd == 64) return launchKv16<64, 1>(tmK, tmV, prm, grid, st);
-    return launchKv16<128, 1>(tmK, tmV, prm, grid, st);
+int prefillKv16(DecodeKvParams prm, uint32_t hd, cudaStream_t st) {
+    return hd == 64 ? rowsKv16Hd<64>(prm, st) : rowsKv16Hd<128>(prm, st);
 }
 
 }  // namespace tc

@@ -6,21 +6,39 @@
 
 namespace tc {
 
+// What a block of n takes of len tokens, in whole 16-token tiles (the decode kernels whose blocks share a device length,
+// and the merge behind them).
+__host__ __device__ inline uint32_t tokensPerBlock(uint32_t len, uint32_t n) {
+    return (((len + 15u) >> 4) + n - 1u) / n * 16u;
+}
+
+// q of one token rotated in place by the merge (decode launches whose blocks all still read it leave that to it):
+// table row = the token's position = attended rows - 1, at most maxLen - 1.
+struct QRotation {
+    float *q;                  // nullable: [nHeads][hd]
+    const float *cosT, *sinT;  // [rows][hd / 2]
+    uint32_t maxLen;
+};
+
+// devLens (nullable): the merge works out on the device how many of the activeHost partials were written, from the
+// length devLens[s] + lenAdd and chunkTokens per partial (0: tokensPerBlock of the length, at most rot.maxLen).
 int launchMerge(const float *pAcc, const float *pM, const float *pL, float *out, uint32_t seqLen,
                 uint32_t nHeads, uint32_t numChunks, uint32_t activeHost, uint32_t hd, const uint32_t *devLens,
                 uint32_t lenAdd, uint32_t chunkTokens, uint8_t *q81, bool pdl, cudaStream_t st,
-                uint32_t chunksPerRank = 0, uint64_t rankStride = 0);
+                uint32_t chunksPerRank = 0, uint64_t rankStride = 0, QRotation rot = {nullptr, nullptr, nullptr, 0});
 
-// int8 decode on tcgen05 (decode_i8_tc.cu): head_dim 128, heads mode; arguments already validated
-int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, cudaStream_t st);
+// An f32 store kept beside an int8 pool: where the appended row of a decode call also goes, verbatim (one
+// sequence; row = its last).
+struct F32Mirror {
+    float *k, *v;  // nullable: [rows][nKV][hd]
+};
 
-// fp16-cache twins of the f32 decode / causal kernels (decode_kv16.cu); arguments already validated
-int decodeKv16(const float *q, const void *kvK, const void *kvV, float *attnOut, float *pAcc, float *pM, float *pL,
-               uint32_t nHeads, uint32_t nKV, uint32_t hd, uint32_t pos, const uint32_t *devPos, uint64_t totalRows,
-               uint32_t numChunks, float invSqrt, uint8_t *q81Out, cudaStream_t st);
-int prefillKv16(const float *q, const void *kvK, const void *kvV, float *out, uint32_t seqLen, uint32_t nHeads,
-                uint32_t nKV, uint32_t hd, uint32_t cachePos, const uint32_t *devPos, uint64_t totalRows,
-                float invSqrt, cudaStream_t st);
+// int8 decode (decode_i8.cu): tc_attn_decode_i8_batch plus the mirror; lens[b] + lenAdd is the length on the device
+int decodeI8Common(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, const F32Mirror &mir, cudaStream_t st);
+// one sequence whose length the launch need not know (captured decode steps): no partials, one launch
+int decodeI8Streams(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, cudaStream_t st);
+// its head_dim 128 form on tcgen05 (decode_i8_tc.cu); arguments already validated
+int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, const F32Mirror &mir, cudaStream_t st);
 
 #ifdef __CUDACC__
 __device__ __forceinline__ bool mbarWaitClock(uint64_t *bar, uint32_t parity, unsigned int *err,
@@ -35,6 +53,58 @@ __device__ __forceinline__ bool mbarWaitClock(uint64_t *bar, uint32_t parity, un
     }
     atomicOr(err, errBit);
     return false;
+}
+
+// The new token's K and V row of one kv head into an int8 pool, by one warp (the arithmetic of kvQuantKernel: amax / 127,
+// IEEE divide, round-half-even; lane i owns float4 i, i + 32 of the row).  Blocks that share the kv head write the same
+// bytes.  Both rows are loaded at once; the block's own TMA load and scale copies read the row back, so the stores are
+// ordered before the async proxy and nothing wider.  srcK / srcV: the rows; dst: row x nKV + kv head of the pool.
+// mirK / mirV (nullable): the same row of an f32 store beside the pool, written verbatim.
+template <int HD>
+__device__ __forceinline__ void appendQuantRow(const float4 *srcK, const float4 *srcV, uint32_t *k8w, uint32_t *v8w,
+                                               float *ksw, float *vsw, uint64_t dst, float4 *mirK, float4 *mirV,
+                                               uint32_t lane) {
+    constexpr int N = HD / 128;
+    float4 kx[N], vx[N];
+    float mk = 0.0f, mv = 0.0f;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        kx[i] = __ldg(srcK + lane + 32 * i);
+        vx[i] = __ldg(srcV + lane + 32 * i);
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        mk = fmaxf(mk, fmaxf(fmaxf(fabsf(kx[i].x), fabsf(kx[i].y)), fmaxf(fabsf(kx[i].z), fabsf(kx[i].w))));
+        mv = fmaxf(mv, fmaxf(fmaxf(fabsf(vx[i].x), fabsf(vx[i].y)), fmaxf(fabsf(vx[i].z), fabsf(vx[i].w))));
+        if (mirK != nullptr) {
+            mirK[lane + 32 * i] = kx[i];
+            mirV[lane + 32 * i] = vx[i];
+        }
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        mk = fmaxf(mk, __shfl_xor_sync(0xffffffffu, mk, o));
+        mv = fmaxf(mv, __shfl_xor_sync(0xffffffffu, mv, o));
+    }
+    const float sk = mk > 0.0f ? __fdiv_rn(mk, 127.0f) : 1.0f;
+    const float sv = mv > 0.0f ? __fdiv_rn(mv, 127.0f) : 1.0f;
+    if (lane == 0) {
+        ksw[dst] = sk;
+        vsw[dst] = sv;
+    }
+    auto q8 = [](float x, float sc) -> uint32_t {
+        int qv = __float2int_rn(__fdiv_rn(x, sc));
+        qv = qv < -128 ? -128 : (qv > 127 ? 127 : qv);
+        return static_cast<uint32_t>(qv) & 0xffu;
+    };
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const uint64_t at = dst * (HD / 4) + lane + 32 * i;
+        k8w[at] = q8(kx[i].x, sk) | (q8(kx[i].y, sk) << 8) | (q8(kx[i].z, sk) << 16) | (q8(kx[i].w, sk) << 24);
+        v8w[at] = q8(vx[i].x, sv) | (q8(vx[i].y, sv) << 8) | (q8(vx[i].z, sv) << 16) | (q8(vx[i].w, sv) << 24);
+    }
+    asm volatile("fence.proxy.async.global;" ::: "memory");
+    __syncwarp();
 }
 
 #endif

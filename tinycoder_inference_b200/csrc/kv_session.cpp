@@ -17,7 +17,7 @@
 
 #include <cuda_runtime.h>
 
-#include "../../include/tc_attn.h"
+#include "decode_cluster.cuh"
 
 struct tc_kv_session {
     tc_kv_session_config c;
@@ -144,6 +144,21 @@ int tc_kv_session_attend(tc_kv_session *s, uint32_t slot, float *q, const float 
         kvV = slotPtr(c.kvV, s->g.kvLayerStride, slot);
     }
     int rc;
+    // one query row over the int8 pool; the decode launch quantises the new row into it first
+    tc_decode_i8_batch d;
+    auto describe = [&](uint32_t maxLen, const uint32_t *posOnDevice) {
+        memset(&d, 0, sizeof(d));
+        d.q = q, d.out = attnOut;
+        d.k8 = k8, d.v8 = v8, d.ks = ks, d.vs = vs;
+        d.pAcc = c.pAcc, d.pM = c.pM, d.pL = c.pL;
+        d.lens = posOnDevice;
+        d.totalRows = rows8Cap;
+        d.batch = 1, d.nHeads = nH, d.nKV = nKV, d.hd = hd;
+        d.maxLen = maxLen;
+        d.numChunks = c.numChunks;
+        d.invSqrt = s->invSqrt;
+        d.appendK = kSrc, d.appendV = vSrc;
+    };
 
     // ---- decode over the int8 pool (kv8Decode) ----
     // One row, not under graph capture (the row counts below are host state the replay could
@@ -159,30 +174,27 @@ int tc_kv_session_attend(tc_kv_session *s, uint32_t slot, float *q, const float 
                 if (rc != TC_OK) return rc;
                 rows8 = pos;
             }
-            // The reference leaves the f32 row of a token decoded through the pool unwritten;
-            // writing it costs one row and keeps a later multi-row call (which reads the f32
-            // cache) looking at the whole history.  The attention of this call does not read it.
-            rc = tc_kv_append(kSrc, vSrc, kvK, kvV, c.kvHalf, 1, nKV, hd, pos, nullptr, c.maxSeqLen, stream);
-            if (rc != TC_OK) return rc;
         }
-        // the decode launch quantises the new row into the pool itself (one launch instead of two)
-        tc_decode_i8_batch d;
-        memset(&d, 0, sizeof(d));
-        d.q = q, d.out = attnOut;
-        d.k8 = k8, d.v8 = v8, d.ks = ks, d.vs = vs;
-        d.pAcc = c.pAcc, d.pM = c.pM, d.pL = c.pL;
-        d.totalRows = rows8Cap;
-        d.batch = 1, d.nHeads = nH, d.nKV = nKV, d.hd = hd;
-        d.maxLen = pos + 1u;
-        d.numChunks = c.numChunks;
-        d.invSqrt = s->invSqrt;
-        d.appendK = kSrc, d.appendV = vSrc;
-        rc = tc_attn_decode_i8_batch(&d, stream);
+        // The reference leaves the f32 row of a token decoded through the pool unwritten;
+        // writing it (the decode launch does) costs one row and keeps a later multi-row call (which
+        // reads the f32 cache) looking at the whole history.  The attention of this call does not read it.
+        tc::F32Mirror mir = {nullptr, nullptr};
+        if (!c.kvStoreI8) mir.k = static_cast<float *>(kvK), mir.v = static_cast<float *>(kvV);
+        describe(pos + 1u, nullptr);
+        rc = tc::decodeI8Common(&d, pos + 1u, 0u, mir, static_cast<cudaStream_t>(stream));
         if (rc == TC_OK) rows8 = pos + 1u;
         return rc;
     }
 
     // ---- int8 as the store: quantise the rows straight into the pool, attend over it ----
+    if (c.kvStoreI8 && seqLen == 1) {
+        // the captured / device-position form of the decode step
+        const uint32_t maxLen = devPos != nullptr ? static_cast<uint32_t>(rows8Cap) : pos + 1u;
+        describe(maxLen, devPos);
+        rc = tc::decodeI8Streams(&d, maxLen, devPos != nullptr ? 1u : 0u, static_cast<cudaStream_t>(stream));
+        if (rc == TC_OK) s->rows8[slot] = pos + 1u;
+        return rc;
+    }
     if (c.kvStoreI8) {
         rc = tc_kv_quantize_i8(kSrc, vSrc, k8, v8, ks, vs, seqLen, nKV, hd, pos, 0, devPos, rows8Cap, stream);
         if (rc != TC_OK) return rc;
@@ -199,6 +211,20 @@ int tc_kv_session_attend(tc_kv_session *s, uint32_t slot, float *q, const float 
     }
 
     // ---- f32 / fp16 store ----
+    if (seqLen == 1) {
+        // The decode launch stores the new row itself (and rotates it and q).
+        // A launch whose position lives on the device (the form a captured graph replays) is sized
+        // for the whole window: the host position is only the value at capture time, the grid and
+        // the chunk length must cover every position a replay can reach (the reference's *Pos
+        // decode launches its fixed attnChunk_ x attnChunks_ grid for the same reason).
+        const uint32_t hostBound = devPos != nullptr ? c.maxSeqLen - 1u : pos;
+        tc::NewToken tok;
+        memset(&tok, 0, sizeof(tok));
+        tok.k = kSrc, tok.v = vSrc;
+        if (c.ropeCos != nullptr) tok.cosT = c.ropeCos, tok.sinT = c.ropeSin, tok.qRot = q;
+        return tc::decodeKvToken(q, kvK, kvV, attnOut, c.pAcc, c.pM, c.pL, nH, nKV, hd, hostBound, devPos, c.maxSeqLen,
+                                 c.numChunks, s->invSqrt, c.kvHalf, nullptr, tok, static_cast<cudaStream_t>(stream));
+    }
     if (c.ropeCos != nullptr)
         rc = tc_kv_append_rope(q, kSrc, vSrc, kvK, kvV, c.kvHalf, seqLen, nH, nKV, hd, pos, pos, devPos, c.ropeCos,
                                c.ropeSin, c.maxSeqLen, stream);
@@ -206,15 +232,6 @@ int tc_kv_session_attend(tc_kv_session *s, uint32_t slot, float *q, const float 
         rc = tc_kv_append(kSrc, vSrc, kvK, kvV, c.kvHalf, seqLen, nKV, hd, pos, devPos, c.maxSeqLen, stream);
     if (rc != TC_OK) return rc;
     // (no int8 bookkeeping here: the next decode's rebuild converts exactly the rows the pool lacks)
-    if (seqLen == 1) {
-        // A launch whose position lives on the device (the form a captured graph replays) is sized
-        // for the whole window: the host position is only the value at capture time, the grid and
-        // the chunk length must cover every position a replay can reach (the reference's *Pos
-        // decode launches its fixed attnChunk_ x attnChunks_ grid for the same reason).
-        const uint32_t hostBound = devPos != nullptr ? c.maxSeqLen - 1u : pos;
-        return tc_attn_decode_kv(q, kvK, kvV, attnOut, c.pAcc, c.pM, c.pL, 1, nH, nKV, hd, hostBound, devPos,
-                                 c.maxSeqLen, c.numChunks, 0, s->invSqrt, c.kvHalf, nullptr, stream);
-    }
     // every multi-row call on the f32 cache -- the first chunk of a prompt and the chunks behind it
     // (ModelForward.cpp:115-127 cuts prompts into 512-token calls) -- takes the tensor-core prefill
     // when the caller's scratch holds the fp16 twins of the rows it attends over

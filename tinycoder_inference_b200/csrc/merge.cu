@@ -12,11 +12,25 @@
 // attention (40-byte slots {fp16 d, fp16 sum, int8 q[32]}, :1068-1096).  The
 // block sum is folded in the reference's order (lane = element index inside the
 // block, xor butterfly 16..1) so the fp16 sum matches bit for bit on equal input.
-#include "tc_common.cuh"
+#include "decode_shared.cuh"
 
 namespace tc {
 
 constexpr int kMergeMaxChunks = 1024;
+
+// The rotation of q in place (see QRotation), block `part` of `parts` of a head.
+__device__ __forceinline__ void rotateHead(const QRotation &rot, uint32_t head, uint32_t hd, const uint32_t *devLens,
+                                           uint32_t lenAdd, uint32_t part, uint32_t parts) {
+    const uint32_t H = hd >> 1;
+    const uint32_t len = devLens != nullptr ? min(devLens[0] + lenAdd, rot.maxLen) : rot.maxLen;
+    const float *c = rot.cosT + static_cast<size_t>(len - 1u) * H, *s = rot.sinT + static_cast<size_t>(len - 1u) * H;
+    float *x = rot.q + static_cast<size_t>(head) * hd;
+    for (uint32_t j = part * blockDim.x + threadIdx.x; j < H; j += parts * blockDim.x) {
+        const float x0 = x[j], x1 = x[j + H];
+        x[j] = fmaf(x0, c[j], -__fmul_rn(x1, s[j]));
+        x[j + H] = fmaf(x0, s[j], __fmul_rn(x1, c[j]));
+    }
+}
 
 // Phase 1: all 256 threads read (m, l) of the active chunks at once, the block
 // takes the max, and the per-chunk weights w_c = exp2((m_c - M) * log2e) (0 for
@@ -29,7 +43,7 @@ __global__ void __launch_bounds__(256)
 mergePartialsKernel(const float *__restrict__ pAcc, const float *__restrict__ pM, const float *__restrict__ pL,
                     float *__restrict__ out, uint32_t nHeads, uint32_t numChunks, uint32_t activeHost,
                     uint32_t hd, const uint32_t *__restrict__ devLens, uint32_t lenAdd, uint32_t chunkTokens,
-                    uint8_t *__restrict__ q81, uint32_t chunksPerRank, uint64_t rankStride) {
+                    uint8_t *__restrict__ q81, uint32_t chunksPerRank, uint64_t rankStride, QRotation rot) {
     constexpr int NW = 8;
     const uint32_t head = blockIdx.x, s = blockIdx.y;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
@@ -56,12 +70,14 @@ mergePartialsKernel(const float *__restrict__ pAcc, const float *__restrict__ pM
     // numChunks is the slot stride; only the first `active` slots were written
     uint32_t active = activeHost < numChunks ? activeHost : numChunks;
     if (devLens != nullptr) {
-        const uint32_t len = devLens[s] + lenAdd;
-        const uint32_t need = (len + chunkTokens - 1) / chunkTokens;
+        uint32_t len = devLens[s] + lenAdd, per = chunkTokens;
+        if (per == 0) len = min(len, rot.maxLen), per = tokensPerBlock(len, activeHost);
+        const uint32_t need = (len + per - 1) / per;
         // never past the slots the launch that wrote the partials covered (activeHost): a device
         // length beyond the host bound the plan was built from must not pull in stale slots
         active = need < active ? need : active;
     }
+    if (rot.q != nullptr) rotateHead(rot, head, hd, devLens, lenAdd, 0, 1);
     __shared__ float sw[kMergeMaxChunks], sl[kMergeMaxChunks];
     __shared__ float sred[NW];
     __shared__ float4 sacc[NW][NV4][32];
@@ -204,7 +220,7 @@ __global__ void __launch_bounds__(T)
 mergeSliceKernel(const float *__restrict__ pAcc, const float *__restrict__ pM, const float *__restrict__ pL,
                  float *__restrict__ out, uint32_t nHeads, uint32_t numChunks, uint32_t activeHost, uint32_t hd,
                  const uint32_t *__restrict__ devLens, uint32_t lenAdd, uint32_t chunkTokens, uint32_t chunksPerRank,
-                 uint64_t rankStride) {
+                 uint64_t rankStride, QRotation rot) {
     constexpr int NW = T / 32;
     const uint32_t head = blockIdx.x, s = blockIdx.y, slice = blockIdx.z;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
@@ -225,8 +241,9 @@ mergeSliceKernel(const float *__restrict__ pAcc, const float *__restrict__ pM, c
     gridDepWait();
     uint32_t active = activeHost < numChunks ? activeHost : numChunks;
     if (devLens != nullptr) {
-        const uint32_t len = devLens[s] + lenAdd;
-        const uint32_t need = (len + chunkTokens - 1) / chunkTokens;
+        uint32_t len = devLens[s] + lenAdd, per = chunkTokens;
+        if (per == 0) len = min(len, rot.maxLen), per = tokensPerBlock(len, activeHost);
+        const uint32_t need = (len + per - 1) / per;
         // never past the slots the launch that wrote the partials covered (activeHost): a device
         // length beyond the host bound the plan was built from must not pull in stale slots
         active = need < active ? need : active;
@@ -322,6 +339,7 @@ mergeSliceKernel(const float *__restrict__ pAcc, const float *__restrict__ pM, c
             }
         }
     }  // more than 64 chunks
+    if (rot.q != nullptr && slice == gridDim.z - 1) rotateHead(rot, head, hd, devLens, lenAdd, 0, 1);
     // a warp holds 32 / SL4 chunk lanes x SL4 float4: fold the chunk lanes, then the warps
 #pragma unroll
     for (int o = SL4; o <= 16; o <<= 1) {
@@ -351,7 +369,7 @@ mergeSliceKernel(const float *__restrict__ pAcc, const float *__restrict__ pM, c
 int launchMerge(const float *pAcc, const float *pM, const float *pL, float *out, uint32_t seqLen,
                 uint32_t nHeads, uint32_t numChunks, uint32_t activeHost, uint32_t hd, const uint32_t *devLens,
                 uint32_t lenAdd, uint32_t chunkTokens, uint8_t *q81, bool pdl, cudaStream_t st,
-                uint32_t chunksPerRank, uint64_t rankStride) {
+                uint32_t chunksPerRank, uint64_t rankStride, QRotation rot) {
     if (chunksPerRank == 0) chunksPerRank = numChunks;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(nHeads, seqLen);
@@ -374,20 +392,20 @@ int launchMerge(const float *pAcc, const float *pM, const float *pL, float *out,
         if (static_cast<uint64_t>(nHeads) * seqLen <= 64u) {
             cfg.gridDim = dim3(nHeads, seqLen, hd / 16u);
             TC_CUDA_OK(cudaLaunchKernelEx(&cfg, mergeSliceKernel<4, 256>, pAcc, pM, pL, out, nHeads, numChunks, activeHost, hd,
-                                          devLens, lenAdd, chunkTokens, chunksPerRank, rankStride));
+                                          devLens, lenAdd, chunkTokens, chunksPerRank, rankStride, rot));
             return TC_OK;
         }
         cfg.gridDim = dim3(nHeads, seqLen, hd / 32u);
         TC_CUDA_OK(cudaLaunchKernelEx(&cfg, mergeSliceKernel<8, 256>, pAcc, pM, pL, out, nHeads, numChunks, activeHost, hd,
-                                      devLens, lenAdd, chunkTokens, chunksPerRank, rankStride));
+                                      devLens, lenAdd, chunkTokens, chunksPerRank, rankStride, rot));
         return TC_OK;
     }
     if (hd <= 128)
         TC_CUDA_OK(cudaLaunchKernelEx(&cfg, mergePartialsKernel<1>, pAcc, pM, pL, out, nHeads, numChunks,
-                                      activeHost, hd, devLens, lenAdd, chunkTokens, q81, chunksPerRank, rankStride));
+                                      activeHost, hd, devLens, lenAdd, chunkTokens, q81, chunksPerRank, rankStride, rot));
     else
         TC_CUDA_OK(cudaLaunchKernelEx(&cfg, mergePartialsKernel<2>, pAcc, pM, pL, out, nHeads, numChunks,
-                                      activeHost, hd, devLens, lenAdd, chunkTokens, q81, chunksPerRank, rankStride));
+                                      activeHost, hd, devLens, lenAdd, chunkTokens, q81, chunksPerRank, rankStride, rot));
     return TC_OK;
 }
 
