@@ -18,6 +18,7 @@
 #include <cuda_runtime.h>
 
 #include "decode_cluster.cuh"
+#include "prefill_rows.cuh"
 
 struct tc_kv_session {
     tc_kv_session_config c;
@@ -144,6 +145,17 @@ int tc_kv_session_attend(tc_kv_session *s, uint32_t slot, float *q, const float 
         kvV = slotPtr(c.kvV, s->g.kvLayerStride, slot);
     }
     int rc;
+    // the launches that take the new rows along move them (and the tables) 16 bytes at a time; rows at any other
+    // address go in with a launch of their own
+    const bool aligned = ((reinterpret_cast<uintptr_t>(kSrc) | reinterpret_cast<uintptr_t>(vSrc) |
+                           reinterpret_cast<uintptr_t>(c.ropeCos) | reinterpret_cast<uintptr_t>(c.ropeSin) |
+                           reinterpret_cast<uintptr_t>(kvK) | reinterpret_cast<uintptr_t>(kvV)) & 15u) == 0;
+    auto append = [&]() {
+        if (c.ropeCos != nullptr)
+            return tc_kv_append_rope(q, kSrc, vSrc, kvK, kvV, c.kvHalf, seqLen, nH, nKV, hd, pos, pos, devPos, c.ropeCos,
+                                     c.ropeSin, c.maxSeqLen, stream);
+        return tc_kv_append(kSrc, vSrc, kvK, kvV, c.kvHalf, seqLen, nKV, hd, pos, devPos, c.maxSeqLen, stream);
+    };
     // one query row over the int8 pool; the decode launch quantises the new row into it first
     tc_decode_i8_batch d;
     auto describe = [&](uint32_t maxLen, const uint32_t *posOnDevice) {
@@ -179,7 +191,8 @@ int tc_kv_session_attend(tc_kv_session *s, uint32_t slot, float *q, const float 
         // writing it (the decode launch does) costs one row and keeps a later multi-row call (which
         // reads the f32 cache) looking at the whole history.  The attention of this call does not read it.
         tc::F32Mirror mir = {nullptr, nullptr};
-        if (!c.kvStoreI8) mir.k = static_cast<float *>(kvK), mir.v = static_cast<float *>(kvV);
+        if (!c.kvStoreI8 && aligned) mir.k = static_cast<float *>(kvK), mir.v = static_cast<float *>(kvV);
+        if (!c.kvStoreI8 && !aligned && (rc = append()) != TC_OK) return rc;
         describe(pos + 1u, nullptr);
         rc = tc::decodeI8Common(&d, pos + 1u, 0u, mir, static_cast<cudaStream_t>(stream));
         if (rc == TC_OK) rows8 = pos + 1u;
@@ -195,17 +208,37 @@ int tc_kv_session_attend(tc_kv_session *s, uint32_t slot, float *q, const float 
         if (rc == TC_OK) s->rows8[slot] = pos + 1u;
         return rc;
     }
+    // A multi-row call takes the tensor-core prefill when the caller's scratch holds the fp16 twins it needs -- the first
+    // chunk of a prompt and the chunks behind it alike (ModelForward.cpp:115-127 cuts prompts into 512-token calls).
+    // Its first launch rotates, stores and quantises the new rows on their way to the twins.  (An fp16 store is read in
+    // place: the scratch only has to hold q's twin.)
+    if (seqLen > 1 && devPos == nullptr && !graphCapture && (hd == 64 || hd == 128 || hd == 256) && c.prefillScratch != nullptr) {
+        size_t need = 0;
+        if (tc_attn_prefill_f16_scratch_bytes(seqLen, c.kvHalf ? 0 : pos, nH, c.kvHalf ? 0 : nKV, hd, &need) == TC_OK &&
+            need <= c.prefillScratchBytes) {
+            tc::PrefillKvStore st = {c.kvHalf ? 1 : 0, kvK, kvV, nullptr, nullptr};
+            if (c.kvStoreI8) st = {2, k8, v8, ks, vs};
+            tc::PrefillNewRows nr = {kSrc, vSrc, c.ropeCos, c.ropeSin};
+            if (!aligned && !c.kvStoreI8) {
+                if ((rc = append()) != TC_OK) return rc;
+                nr = {nullptr, nullptr, nullptr, nullptr};
+            }
+            tc::PrefillMirror mir;
+            memset(&mir, 0, sizeof(mir));
+            // With a decode pool that is current up to this call's first row its rows of the new positions are written
+            // too: the mirror stays current through the chunks of a prompt and the first decode step has nothing to rebuild.
+            const bool keepMirror = c.kvMirror && s->rows8[slot] == pos;
+            if (keepMirror) mir = {k8, v8, ks, vs, pos, rows8Cap};
+            rc = tc::prefillF16(q, st, attnOut, c.prefillScratch, c.prefillScratchBytes, seqLen, pos, nH, nKV, hd, s->invSqrt,
+                                mir, nr, static_cast<cudaStream_t>(stream));
+            if (rc == TC_OK && (keepMirror || c.kvStoreI8)) s->rows8[slot] = pos + seqLen;
+            return rc;
+        }
+    }
     if (c.kvStoreI8) {
         rc = tc_kv_quantize_i8(kSrc, vSrc, k8, v8, ks, vs, seqLen, nKV, hd, pos, 0, devPos, rows8Cap, stream);
         if (rc != TC_OK) return rc;
         s->rows8[slot] = pos + seqLen;
-        // a multi-row call with scratch for the twins (bytes x row scale) takes the tensor-core prefill
-        if (seqLen > 1 && devPos == nullptr && !graphCapture && (hd == 64 || hd == 128 || hd == 256) && c.prefillScratch != nullptr) {
-            size_t need = 0;
-            if (tc_attn_prefill_f16_scratch_bytes(seqLen, pos, nH, nKV, hd, &need) == TC_OK && need <= c.prefillScratchBytes)
-                return tc_attn_prefill_f16_i8(q, k8, v8, ks, vs, attnOut, c.prefillScratch, c.prefillScratchBytes, seqLen,
-                                              pos, nH, nKV, hd, s->invSqrt, stream);
-        }
         return tc_attn_prefill_i8(q, k8, v8, ks, vs, attnOut, seqLen, nH, nKV, hd, pos, devPos, rows8Cap, s->invSqrt,
                                   stream);
     }
@@ -220,46 +253,17 @@ int tc_kv_session_attend(tc_kv_session *s, uint32_t slot, float *q, const float 
         const uint32_t hostBound = devPos != nullptr ? c.maxSeqLen - 1u : pos;
         tc::NewToken tok;
         memset(&tok, 0, sizeof(tok));
-        tok.k = kSrc, tok.v = vSrc;
-        if (c.ropeCos != nullptr) tok.cosT = c.ropeCos, tok.sinT = c.ropeSin, tok.qRot = q;
+        if (aligned) {
+            tok.k = kSrc, tok.v = vSrc;
+            if (c.ropeCos != nullptr) tok.cosT = c.ropeCos, tok.sinT = c.ropeSin, tok.qRot = q;
+        } else if ((rc = append()) != TC_OK) {
+            return rc;
+        }
         return tc::decodeKvToken(q, kvK, kvV, attnOut, c.pAcc, c.pM, c.pL, nH, nKV, hd, hostBound, devPos, c.maxSeqLen,
                                  c.numChunks, s->invSqrt, c.kvHalf, nullptr, tok, static_cast<cudaStream_t>(stream));
     }
-    if (c.ropeCos != nullptr)
-        rc = tc_kv_append_rope(q, kSrc, vSrc, kvK, kvV, c.kvHalf, seqLen, nH, nKV, hd, pos, pos, devPos, c.ropeCos,
-                               c.ropeSin, c.maxSeqLen, stream);
-    else
-        rc = tc_kv_append(kSrc, vSrc, kvK, kvV, c.kvHalf, seqLen, nKV, hd, pos, devPos, c.maxSeqLen, stream);
-    if (rc != TC_OK) return rc;
+    if ((rc = append()) != TC_OK) return rc;
     // (no int8 bookkeeping here: the next decode's rebuild converts exactly the rows the pool lacks)
-    // every multi-row call on the f32 cache -- the first chunk of a prompt and the chunks behind it
-    // (ModelForward.cpp:115-127 cuts prompts into 512-token calls) -- takes the tensor-core prefill
-    // when the caller's scratch holds the fp16 twins of the rows it attends over
-    if (devPos == nullptr && !graphCapture && c.kvHalf && (hd == 64 || hd == 128 || hd == 256) && c.prefillScratch != nullptr) {
-        // the fp16 store is read in place: the scratch only has to hold q's twin
-        size_t need = 0;
-        if (tc_attn_prefill_f16_scratch_bytes(seqLen, 0, nH, 0, hd, &need) == TC_OK && need <= c.prefillScratchBytes)
-            return tc_attn_prefill_f16_kvhalf(q, kvK, kvV, attnOut, c.prefillScratch, c.prefillScratchBytes, seqLen, pos,
-                                              nH, nKV, hd, s->invSqrt, stream);
-    }
-    if (devPos == nullptr && !graphCapture && !c.kvHalf && (hd == 64 || hd == 128 || hd == 256) && c.prefillScratch != nullptr) {
-        size_t need = 0;
-        if (tc_attn_prefill_f16_scratch_bytes(seqLen, pos, nH, nKV, hd, &need) == TC_OK && need <= c.prefillScratchBytes) {
-            // With a decode pool that is current up to this call's first row, the launch that makes
-            // the fp16 twins writes the pool's rows of the new positions too: the mirror stays
-            // current through the chunks of a prompt and the first decode step has nothing to rebuild.
-            if (c.kvMirror && s->rows8[slot] == pos) {
-                rc = tc_attn_prefill_f16_kv8(q, static_cast<const float *>(kvK), static_cast<const float *>(kvV),
-                                             attnOut, c.prefillScratch, c.prefillScratchBytes, seqLen, pos, nH, nKV, hd,
-                                             s->invSqrt, k8, v8, ks, vs, pos, rows8Cap, stream);
-                if (rc == TC_OK) s->rows8[slot] = pos + seqLen;
-                return rc;
-            }
-            return tc_attn_prefill_f16(q, static_cast<const float *>(kvK), static_cast<const float *>(kvV), attnOut,
-                                       c.prefillScratch, c.prefillScratchBytes, seqLen, pos, nH, nKV, hd, s->invSqrt,
-                                       stream);
-        }
-    }
     return tc_attn_prefill_kv(q, kvK, kvV, attnOut, seqLen, nH, nKV, hd, pos, devPos, c.maxSeqLen, s->invSqrt,
                               c.kvHalf, stream);
 }

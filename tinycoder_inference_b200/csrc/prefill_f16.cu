@@ -11,8 +11,11 @@
 // never exists and the sequence length is not capped at 512.
 //
 // One persistent block per SM walks work items: a q head x 256 query rows = two 128-row query
-// tiles A and B (one tile per item for short calls and at head_dim 256), KV tiles of 64 tokens (32
-// at head_dim 256).  The first item of a block is its index, the following ones come from a
+// tiles A and B, KV tiles of 64 tokens.  A call with fewer such items than SMs takes items of ONE query
+// tile whose KV tiles the two halves of the block share (even / odd) and put together at the end: 512 rows
+// behind 3584 of 28 q heads of 128 take 48.6 us, with one half idle 55.5.  At head_dim 256 a block
+// holds one query tile (2000 rows of 16 heads: 55.9 us, with 32-token KV tiles 79.0).
+// The first item of a block is its index, the following ones come from a
 // counter, heavy (late) query blocks first; the mbarriers are initialised once, every ring index
 // counts on from item to item, so the next item's loads and first score products run under the
 // current item's epilogue.  Warp roles:
@@ -21,10 +24,10 @@
 //              first columns of the same S buffer (tcgen05.st) as the A operand of the PV product,
 //              rescales O in TMEM only when the row maximum ran ahead by 2^8 (lazy rescale);
 //              packed f32x2 arithmetic; normalises and stores the output rows (32-byte stores);
-//   warp 8     TMA producer and scheduler: the query tiles and K_0, K_1 per item, then a four-stage
-//              ring whose stage j holds what step j of the MMA warps consumes, K_{j+2} and V_j
-//              (cp.async.bulk.tensor, 128-byte swizzle = the canonical UMMA shared-memory layout,
-//              so no register pass touches the operands); draws the next item late in the current;
+//   warp 8     TMA producer and scheduler: the query tiles per item, then K two tiles ahead of V
+//              into rings of their own (cp.async.bulk.tensor, 128-byte swizzle = the canonical UMMA
+//              shared-memory layout, so no register pass touches the operands); draws the next
+//              item late in the current;
 //   warps 9, 10  issue the score products of tile A / B: S_X(t) = Q_X K^T (M128 N64 K16 per
 //              instruction), tcgen05.commit onto the softmax warps' barrier;
 //   warps 11, 12  issue the P.V products of tile A / B: O_X += P_X(t) V (A from TMEM, B = V
@@ -35,70 +38,99 @@
 // columns): O_A, O_B (128 each, f32; one O of 256 at head_dim 256), S_{A,0}, S_{A,1}, S_{B,0},
 // S_{B,1} (64 each).  Causality: a query tile only visits KV tiles up to its diagonal, the last
 // two or three are masked element-wise; the query rows may sit behind an existing cache.
-// In front of the kernel one launch makes the fp16 twins of q, K and V (from the f32 store, or
-// from the int8 store's bytes and scales; an fp16 store is read in place) and, on request, the int8
-// pool rows of the call's new positions; the attention kernel is its programmatic dependent.
+// In front of the kernel one launch (prefillRowsKernel) makes the fp16 twins of q, K and V and puts the
+// call's new rows into the store; the attention kernel is its programmatic dependent.
 // Every wait is bounded; a wait that runs out records an error bit, every other wait of the launch
 // then gives up at once, the block frees its TMEM and returns.
 #include <algorithm>
+#include <cstring>
 
+#include "prefill_rows.cuh"
 #include "tc_tcgen05.cuh"
 
 namespace tc {
 
 constexpr int kPfBM = 128;    // query rows per tile (two tiles per CTA)
-constexpr int kPfStages = 4;  // K and V ring depth
+constexpr int kPfBN = 64;     // tokens per KV tile
 constexpr float kPfLazyLog2 = 8.0f;
 
-// Where the int8 mirror of the call's new K/V rows goes (the reference keeps such a pool beside its
-// f32 store and rebuilds it before the first decode step, GPUComputeMoE.cu:3049-3063): rows
-// [cachePos, cachePos + seqLen) of the cache become pool rows dstRow ..; null k8 = no mirror.
-struct PrefillMirror {
-    int8_t *k8, *v8;   // [rows][nKV][hd]
-    float *ks, *vs;    // [rows][nKV]
-    uint64_t dstRow;   // pool row of cache row cachePos
-    uint64_t maxRows;  // rows the pool holds
+// Everything between a call's f32 rows and the attention launch, in ONE launch: q to fp16 (the reference's kF32ToF16,
+// GpuElementwiseKernels.hpp:92-101; GPUComputeForward.cu:3957-3968), rotated in place first in the dense models; the new
+// K/V rows -- if the call brings them -- rotated and stored into the f32 / fp16 / int8 store (the arithmetic of
+// kvAppendKernel and kvQuantKernel, bit for bit); the fp16 twins of all rows the call attends over (an fp16 store needs
+// none: its layout is the twins'); and the int8 pool rows of the new positions beside an f32 store.  q goes four
+// rotation pairs per thread; a K/V row of one kv head goes to a warp, lane i holding dims 4 i .. 4 i + 3 (and 128
+// further on at head_dim 256), so its maximum is a shuffle away.
+// HBM-bound for prompts: 4096 rows of 28 q / 4 kv heads of 128 with the mirror move 134 MB in 23.6 us, 5.7 TB/s (append and
+// twins as launches of their own: 33 us, and the rows went through HBM twice); launch-bound for short ones.
+struct PrefillRowsParams {
+    float *q;              // [seqLen][nHeads][hd]; written back only when it is rotated
+    uint2 *q16, *k16, *v16;
+    PrefillKvStore st;
+    PrefillNewRows nr;
+    PrefillMirror mir;
+    uint32_t seqLen, cachePos, nHeads, nKV;
+    unsigned int *err, *workCounter;
 };
 
-// What the K/V rows of a call are read from: the f32 store (twins made here), the fp16 store (used in
-// place: its layout is the twins'), or the int8 store (twins made here: byte x the row's scale).
-struct PrefillKvSource {
-    int kind;             // 0 f32, 1 fp16, 2 int8
-    const void *k, *v;    // [rows][nKV][hd] of float / __half / int8_t
-    const float *ks, *vs; // int8: [rows][nKV] scales
-};
-
-// f32 -> fp16 twins of q, K and V in ONE launch (the reference's kF32ToF16 x3,
-// GpuElementwiseKernels.hpp:92-101; GPUComputeForward.cu:3957-3968), and -- the K/V rows being in
-// registers anyway -- the int8 rows of the new positions (one scale per row and kv head, amax / 127,
-// round-half-even: the arithmetic of kvQuantKernel, bit for bit).  q goes float4 by float4; a K/V
-// row of one kv head goes to a warp, lane i holding dims 4 i .. 4 i + 3 (and 128 further on at head_dim 256).
-// With an int8 source (k8 != nullptr) the K/V rows are bytes and a scale per row and kv head instead of
-// floats, and there is no mirror to write.
-// MAXV: float4 per lane and row, 1 up to head_dim 128, 2 at 256.
-template <int MAXV>
-__global__ void __launch_bounds__(256)
-f32ToF16MirrorKernel(const float4 *__restrict__ q, const float4 *__restrict__ k, const float4 *__restrict__ v,
-                     const uint32_t *__restrict__ k8, const uint32_t *__restrict__ v8, const float *__restrict__ ks8,
-                     const float *__restrict__ vs8, uint2 *__restrict__ q16, uint2 *__restrict__ k16,
-                     uint2 *__restrict__ v16, size_t nq4, size_t kvRowHeads, uint32_t nvec, size_t mirrorFrom,
-                     PrefillMirror mir, uint32_t nKV, unsigned int *__restrict__ err,
-                     unsigned int *__restrict__ workCounter) {
-    // the attention launch that follows in the stream hands out its work items through this counter
-    if (blockIdx.x == 0 && threadIdx.x == 0) *workCounter = 0u;
+template <int HD>
+__global__ void __launch_bounds__(256) prefillRowsKernel(const __grid_constant__ PrefillRowsParams p) {
+    gridDepWait();
     gridDepLaunch();  // the attention launch may set itself up while this one drains
+    // the attention launch that follows in the stream hands out its work items through this counter
+    if (blockIdx.x == 0 && threadIdx.x == 0) *p.workCounter = 0u;
     const size_t tid = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
-    for (size_t i = tid; i < nq4; i += stride) {
-        const float4 x = __ldg(q + i);
-        uint2 o;
-        o.x = packHalf2(x.x, x.y);
-        o.y = packHalf2(x.z, x.w);
-        q16[i] = o;
+    constexpr uint32_t half = HD / 2, perRow = half / 4, nvec = HD / 4;
+    constexpr int MAXV = HD > 128 ? 2 : 1;  // float4 per lane and K/V row
+    auto half4 = [](const float4 &x) { return make_uint2(packHalf2(x.x, x.y), packHalf2(x.z, x.w)); };
+    auto rotate = [](float4 &a, float4 &b, const float4 &c, const float4 &s) {
+        auto rot = [](float &x0, float &x1, float cc, float ss) {
+            const float y = fmaf(x0, cc, -__fmul_rn(x1, ss));
+            x1 = fmaf(x0, ss, __fmul_rn(x1, cc));
+            x0 = y;
+        };
+        rot(a.x, b.x, c.x, s.x);
+        rot(a.y, b.y, c.y, s.y);
+        rot(a.z, b.z, c.z, s.z);
+        rot(a.w, b.w, c.w, s.w);
+    };
+    const size_t qUnits = static_cast<size_t>(p.seqLen) * p.nHeads * perRow;
+    constexpr int N = 4;  // units of a thread in flight
+    for (size_t i0 = tid; i0 < qUnits; i0 += N * stride) {
+        float4 x[N], y[N];
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            const size_t i = i0 + u * stride;
+            if (i >= qUnits) continue;
+            const float4 *a = reinterpret_cast<const float4 *>(p.q) + i / perRow * nvec + i % perRow;
+            x[u] = a[0];
+            y[u] = a[perRow];
+        }
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            const size_t i = i0 + u * stride;
+            if (i >= qUnits) continue;
+            const size_t row = i / perRow, at = row * nvec + i % perRow;
+            if (p.nr.cosT != nullptr) {
+                const size_t t = (static_cast<size_t>(p.cachePos) + row / p.nHeads) * perRow + i % perRow;
+                rotate(x[u], y[u], __ldg(reinterpret_cast<const float4 *>(p.nr.cosT) + t),
+                       __ldg(reinterpret_cast<const float4 *>(p.nr.sinT) + t));
+                reinterpret_cast<float4 *>(p.q)[at] = x[u];
+                reinterpret_cast<float4 *>(p.q)[at + perRow] = y[u];
+            }
+            p.q16[at] = half4(x[u]);
+            p.q16[at + perRow] = half4(y[u]);
+        }
     }
     const uint32_t lane = threadIdx.x & 31u;
-    for (size_t rh = tid >> 5; rh < kvRowHeads; rh += stride >> 5) {
-        // lane i holds float4 i and, at head_dim 256, float4 i + 32 of the row
+    const size_t newFrom = static_cast<size_t>(p.cachePos) * p.nKV;            // first (row, kv head) of the call's rows
+    const size_t end = newFrom + static_cast<size_t>(p.seqLen) * p.nKV;
+    const bool bring = p.nr.k != nullptr;
+    // (an fp16 store has nothing to do for rows that it already holds)
+    const size_t begin = p.k16 != nullptr ? 0 : (bring ? newFrom : end);
+    for (size_t rh = begin + (tid >> 5); rh < end; rh += stride >> 5) {
+        const bool fresh = bring && rh >= newFrom;
         float4 kx[MAXV], vx[MAXV];
         bool active[MAXV];
 #pragma unroll
@@ -107,57 +139,105 @@ f32ToF16MirrorKernel(const float4 *__restrict__ q, const float4 *__restrict__ k,
             active[u] = i4 < nvec;
             kx[u] = make_float4(0.f, 0.f, 0.f, 0.f), vx[u] = kx[u];
             if (!active[u]) continue;
-            if (k8 != nullptr) {
-                const uint32_t kb = __ldg(k8 + rh * nvec + i4), vb = __ldg(v8 + rh * nvec + i4);
-                const float sk = __ldg(ks8 + rh), sv = __ldg(vs8 + rh);
+            if (fresh) {
+                kx[u] = __ldg(reinterpret_cast<const float4 *>(p.nr.k) + (rh - newFrom) * nvec + i4);
+                vx[u] = __ldg(reinterpret_cast<const float4 *>(p.nr.v) + (rh - newFrom) * nvec + i4);
+            } else if (p.st.kind == 2) {
+                const uint32_t kb = __ldg(static_cast<const uint32_t *>(p.st.k) + rh * nvec + i4),
+                               vb = __ldg(static_cast<const uint32_t *>(p.st.v) + rh * nvec + i4);
+                const float sk = __ldg(p.st.ks + rh), sv = __ldg(p.st.vs + rh);
                 auto b = [](uint32_t w, int i) { return static_cast<float>(static_cast<int8_t>((w >> (8 * i)) & 0xffu)); };
                 kx[u] = make_float4(b(kb, 0) * sk, b(kb, 1) * sk, b(kb, 2) * sk, b(kb, 3) * sk);
                 vx[u] = make_float4(b(vb, 0) * sv, b(vb, 1) * sv, b(vb, 2) * sv, b(vb, 3) * sv);
             } else {
-                kx[u] = __ldg(k + rh * nvec + i4);
-                vx[u] = __ldg(v + rh * nvec + i4);
+                kx[u] = __ldg(static_cast<const float4 *>(p.st.k) + rh * nvec + i4);
+                vx[u] = __ldg(static_cast<const float4 *>(p.st.v) + rh * nvec + i4);
             }
-            uint2 o;
-            o.x = packHalf2(kx[u].x, kx[u].y);
-            o.y = packHalf2(kx[u].z, kx[u].w);
-            k16[rh * nvec + i4] = o;
-            o.x = packHalf2(vx[u].x, vx[u].y);
-            o.y = packHalf2(vx[u].z, vx[u].w);
-            v16[rh * nvec + i4] = o;
         }
-        if (mir.k8 == nullptr || rh < mirrorFrom) continue;  // warp-uniform
-        const size_t dst = mir.dstRow * nKV + (rh - mirrorFrom);
-        if (dst >= mir.maxRows * nKV) {
-            if (lane == 0) atomicOr(err, kDevErrRowBound);
-            continue;
+        if (fresh && p.nr.cosT != nullptr) {  // warp-uniform
+            const size_t at = static_cast<size_t>(rh / p.nKV) * half;
+            if (MAXV > 1) {
+                // the partner of a lane's first float4 is its second one
+                rotate(kx[0], kx[MAXV - 1], __ldg(reinterpret_cast<const float4 *>(p.nr.cosT + at) + lane),
+                       __ldg(reinterpret_cast<const float4 *>(p.nr.sinT + at) + lane));
+            } else {
+                // perRow lanes apart
+                const bool low = lane < perRow;
+                const uint32_t j = low ? lane : lane - perRow;
+                float4 o;
+                o.x = __shfl_xor_sync(0xffffffffu, kx[0].x, perRow);
+                o.y = __shfl_xor_sync(0xffffffffu, kx[0].y, perRow);
+                o.z = __shfl_xor_sync(0xffffffffu, kx[0].z, perRow);
+                o.w = __shfl_xor_sync(0xffffffffu, kx[0].w, perRow);
+                if (active[0]) {
+                    float4 a = low ? kx[0] : o, b = low ? o : kx[0];
+                    rotate(a, b, __ldg(reinterpret_cast<const float4 *>(p.nr.cosT + at) + j),
+                           __ldg(reinterpret_cast<const float4 *>(p.nr.sinT + at) + j));
+                    kx[0] = low ? a : b;
+                }
+            }
         }
-        auto amax4 = [](const float4 &x) { return fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))); };
-        float mk = amax4(kx[0]), mv = amax4(vx[0]);
-        if (MAXV > 1) mk = fmaxf(mk, amax4(kx[MAXV - 1])), mv = fmaxf(mv, amax4(vx[MAXV - 1]));
+        // int8 rows: of the store itself, or of the pool beside an f32 store
+        const bool toStore8 = fresh && p.st.kind == 2;
+        const bool toMirror = p.mir.k8 != nullptr && rh >= newFrom;
+        if (toStore8 || toMirror) {  // warp-uniform
+            auto amax4 = [](const float4 &x) { return fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))); };
+            float mk = amax4(kx[0]), mv = amax4(vx[0]);
+            if (MAXV > 1) mk = fmaxf(mk, amax4(kx[MAXV - 1])), mv = fmaxf(mv, amax4(vx[MAXV - 1]));
 #pragma unroll
-        for (int o = 16; o; o >>= 1) {
-            mk = fmaxf(mk, __shfl_xor_sync(0xffffffffu, mk, o));
-            mv = fmaxf(mv, __shfl_xor_sync(0xffffffffu, mv, o));
+            for (int o = 16; o; o >>= 1) {
+                mk = fmaxf(mk, __shfl_xor_sync(0xffffffffu, mk, o));
+                mv = fmaxf(mv, __shfl_xor_sync(0xffffffffu, mv, o));
+            }
+            const float sk = mk > 0.0f ? __fdiv_rn(mk, 127.0f) : 1.0f;
+            const float sv = mv > 0.0f ? __fdiv_rn(mv, 127.0f) : 1.0f;
+            const size_t dst = toStore8 ? rh : static_cast<size_t>(p.mir.dstRow) * p.nKV + (rh - newFrom);
+            uint32_t *k8 = toStore8 ? static_cast<uint32_t *>(p.st.k) : reinterpret_cast<uint32_t *>(p.mir.k8);
+            uint32_t *v8 = toStore8 ? static_cast<uint32_t *>(p.st.v) : reinterpret_cast<uint32_t *>(p.mir.v8);
+            float *ks = toStore8 ? p.st.ks : p.mir.ks, *vs = toStore8 ? p.st.vs : p.mir.vs;
+            if (!toStore8 && dst >= p.mir.maxRows * p.nKV) {
+                if (lane == 0) atomicOr(p.err, kDevErrRowBound);
+            } else {
+                if (lane == 0) {
+                    ks[dst] = sk;
+                    vs[dst] = sv;
+                }
+                auto q8 = [](float x, float sc) -> int {
+                    const int qv = __float2int_rn(__fdiv_rn(x, sc));
+                    return qv < -128 ? -128 : (qv > 127 ? 127 : qv);
+                };
+#pragma unroll
+                for (int u = 0; u < MAXV; ++u) {
+                    if (!active[u]) continue;
+                    const uint32_t i4 = lane + 32u * u;
+                    auto pack = [&](float4 &x, float sc) -> uint32_t {
+                        const int a = q8(x.x, sc), b = q8(x.y, sc), c = q8(x.z, sc), d = q8(x.w, sc);
+                        if (toStore8)  // attention over an int8 store sees what the store holds
+                            x = make_float4(static_cast<float>(a) * sc, static_cast<float>(b) * sc, static_cast<float>(c) * sc,
+                                            static_cast<float>(d) * sc);
+                        return (static_cast<uint32_t>(a) & 0xffu) | ((static_cast<uint32_t>(b) & 0xffu) << 8) |
+                               ((static_cast<uint32_t>(c) & 0xffu) << 16) | ((static_cast<uint32_t>(d) & 0xffu) << 24);
+                    };
+                    k8[dst * nvec + i4] = pack(kx[u], sk);
+                    v8[dst * nvec + i4] = pack(vx[u], sv);
+                }
+            }
         }
-        const float sk = mk > 0.0f ? __fdiv_rn(mk, 127.0f) : 1.0f;
-        const float sv = mv > 0.0f ? __fdiv_rn(mv, 127.0f) : 1.0f;
-        if (lane == 0) {
-            mir.ks[dst] = sk;
-            mir.vs[dst] = sv;
-        }
-        auto q8 = [](float x, float sc) -> uint32_t {
-            int qv = __float2int_rn(__fdiv_rn(x, sc));
-            qv = qv < -128 ? -128 : (qv > 127 ? 127 : qv);
-            return static_cast<uint32_t>(qv) & 0xffu;
-        };
 #pragma unroll
         for (int u = 0; u < MAXV; ++u) {
             if (!active[u]) continue;
-            const uint32_t i4 = lane + 32u * u;
-            reinterpret_cast<uint32_t *>(mir.k8)[dst * nvec + i4] =
-                    q8(kx[u].x, sk) | (q8(kx[u].y, sk) << 8) | (q8(kx[u].z, sk) << 16) | (q8(kx[u].w, sk) << 24);
-            reinterpret_cast<uint32_t *>(mir.v8)[dst * nvec + i4] =
-                    q8(vx[u].x, sv) | (q8(vx[u].y, sv) << 8) | (q8(vx[u].z, sv) << 16) | (q8(vx[u].w, sv) << 24);
+            const size_t at = rh * nvec + lane + 32u * u;
+            if (fresh && p.st.kind == 0) {
+                static_cast<float4 *>(p.st.k)[at] = kx[u];
+                static_cast<float4 *>(p.st.v)[at] = vx[u];
+            } else if (fresh && p.st.kind == 1) {
+                static_cast<uint2 *>(p.st.k)[at] = half4(kx[u]);
+                static_cast<uint2 *>(p.st.v)[at] = half4(vx[u]);
+            }
+            if (p.k16 != nullptr) {
+                p.k16[at] = half4(kx[u]);
+                p.v16[at] = half4(vx[u]);
+            }
         }
     }
 }
@@ -167,7 +247,8 @@ struct PrefillF16Params {
     uint32_t seqLen, nHeads, nKV, group;
     uint32_t cachePos;  // query row r sits at position cachePos + r and sees K/V rows [0, cachePos + r]
     uint32_t nQTiles;   // query blocks of itemRows rows
-    uint32_t itemRows;  // 256: two query tiles per work item; 128: one (short calls, so that every SM gets an item)
+    uint32_t itemRows;  // 256: two query tiles per work item; 128: one
+    uint32_t split;     // one-tile items whose KV tiles the two halves of the block share (even / odd)
     float scaleLog2;   // invSqrt * log2(e)
     unsigned int *err;
     unsigned int *workCounter;  // zero at launch; item gridDim.x + n goes to the n-th request
@@ -193,26 +274,29 @@ __device__ __forceinline__ unsigned long long pfTime() {
 #endif
 
 // HD = head_dim (64, 128 or 256): a tile is HD / 64 halves of 64 columns (128 bytes, one swizzle span)
-// each.  BN = tokens per KV tile: 64, or 32 at head_dim 256, where one query tile and its 256-column
-// accumulator take the room two tiles take at head_dim 128 (a block then serves one query tile).
-template <int HD, int BN>
+// each.  K and V tiles (64 tokens) have rings of their own: the score products run two tiles ahead of the P.V
+// products.  At head_dim 256 one query tile and its 256-column accumulator take the room two tiles take at head_dim 128,
+// and the rings are two tiles deep.
+template <int HD>
 struct PrefillF16Smem {
     static constexpr int kHalves = HD / 64;
     static constexpr int kQTiles = HD > 128 ? 1 : 2;   // query tiles a block holds
+    static constexpr int NK = HD > 128 ? 2 : 6, NV = HD > 128 ? 2 : 4;
     static constexpr int kQHalf = kPfBM * 128;         // 16 KB: 128 rows x 64 fp16
-    static constexpr int kKvHalf = BN * 128;           // BN rows x 64 fp16
+    static constexpr int kKvHalf = kPfBN * 128;        // kPfBN rows x 64 fp16
     static constexpr int kQTile = kHalves * kQHalf;    // head_dim 128: 32 KB
     static constexpr int kKvTile = kHalves * kKvHalf;  // head_dim 128: 16 KB
-    static constexpr int kQ = 0;                       // two query tiles
-    static constexpr int kK01 = kQTiles * kQTile;      // K_0, K_1 (the products issued before the loop)
-    static constexpr int kStage = kK01 + 2 * kKvTile;  // stage s: K slot, then V slot
-    static constexpr int kStageBytes = 2 * kKvTile;
-    static constexpr int kBars = kStage + kPfStages * kStageBytes;
-    // qFull, k01Full, stage full + empty, sFull[2][2], pFull[2][2], pvDone[2], pvBuf[2][2], qFree[2], itemFull[4]
-    static constexpr int kNumBars = 2 + 2 * kPfStages + 4 + 4 + 2 + 4 + 2 + 4;
+    static constexpr int kQ = 0;
+    static constexpr int kK = kQTiles * kQTile;
+    static constexpr int kV = kK + NK * kKvTile;
+    static constexpr int kBars = kV + NV * kKvTile;
+    // qFull, kFull + kEmpty, vFull + vEmpty, sFull[2][2], pFull[2][2], pvDone[2], pvBuf[2][2], qFree[2], itemFull[4],
+    // exFull, exRead
+    static constexpr int kNumBars = 1 + 2 * NK + 2 * NV + 4 + 4 + 2 + 4 + 2 + 4 + 2;
     static constexpr int kTmemSlot = kBars + kNumBars * 8;
     static constexpr int kItemSlots = kTmemSlot + 16;  // four work item indices
     static constexpr int kTotal = kItemSlots + 16 + 1024;
+    static_assert(kTotal <= 227 * 1024, "shared memory of an SM");
 };
 
 __device__ __forceinline__ bool pfWait(uint64_t *bar, uint32_t parity, unsigned int *err, uint32_t bit) {
@@ -249,24 +333,27 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 // never carries out of the field).
 __device__ __forceinline__ uint64_t descAdvance(uint64_t d, uint32_t bytes) { return d + (bytes >> 4); }
 
-// What one work item (a 256-row query block of one head) covers.  Query tile X (0 = A, 1 = B) holds
-// rows m0 + 128 X .. at positions cachePos + row; it sees KV tiles 0 .. nX - 1 (64 tokens each; the
-// last two or three straddle its diagonal).  B may lie wholly past the sequence; a call with fewer
-// 256-row items than SMs is cut into 128-row items instead, which have no tile B.
+// What one work item covers.  Two-tile items (256 query rows of one head): query tile X (0 = A, 1 = B) holds rows
+// m0 + 128 X .. at positions cachePos + row and sees KV tiles 0 .. nX - 1 (the last two or three straddle its diagonal); B
+// may lie wholly past the sequence.  Split items (128 query rows): both halves of the block work on the same query
+// tile, A on the even KV tiles, B on the odd ones, and put their results together at the end -- a call too short to give
+// every SM a two-tile item is bound by the chain of one tile's steps, not by the tensor pipe.
 struct PfItem {
     uint32_t head, kvHead, m0, nA, nB, nTiles;
 };
-template <int BN>
 __device__ __forceinline__ PfItem pfItem(const PrefillF16Params &p, uint32_t item) {
     PfItem it;
     const uint32_t qb = p.nQTiles - 1u - item / p.nHeads;  // heavy query blocks (long causal prefixes) first
     it.head = item % p.nHeads;
     it.kvHead = it.head / p.group;
     it.m0 = qb * p.itemRows;
-    const bool activeB = p.itemRows > kPfBM && it.m0 + kPfBM < p.seqLen;
-    it.nA = (p.cachePos + it.m0 + kPfBM + BN - 1u) / BN;
-    it.nB = activeB ? (p.cachePos + it.m0 + 2u * kPfBM + BN - 1u) / BN : 0u;
-    it.nTiles = activeB ? it.nB : it.nA;
+    auto tilesOf = [&](uint32_t row0) {  // KV tiles the rows row0 .. row0 + 127 of the sequence see
+        return (p.cachePos + min(row0 + kPfBM, p.seqLen) + kPfBN - 1u) / kPfBN;
+    };
+    it.nA = tilesOf(it.m0);
+    it.nB = p.itemRows > kPfBM && it.m0 + kPfBM < p.seqLen ? tilesOf(it.m0 + kPfBM) : 0u;
+    it.nTiles = max(it.nA, it.nB);
+    if (p.split) it.nB = it.nTiles / 2u, it.nA = it.nTiles - it.nB;
     return it;
 }
 
@@ -282,29 +369,38 @@ __device__ __forceinline__ PfItem pfItem(const PrefillF16Params &p, uint32_t ite
 // product has been issued, its first scores are in TMEM while the softmax threads still write this
 // item's output, and tile A moves on while tile B finishes its two extra diagonal tiles.
 constexpr int kPfThreads = 416;
-template <int HD, int BN>
+template <int HD>
 __global__ void __launch_bounds__(kPfThreads, 1)
 prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const PrefillF16Params p) {
-    using L = PrefillF16Smem<HD, BN>;
+    using L = PrefillF16Smem<HD>;
+    constexpr int BN = kPfBN;
     constexpr int NC = BN / 32;  // 32-column chunks of a score row
-    constexpr uint32_t NS = kPfStages;
+    constexpr uint32_t NK = L::NK, NV = L::NV;
+    constexpr bool kOne = L::kQTiles == 1;  // the second half of the block has nothing to do
     extern __shared__ uint8_t smemRaw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L::kBars);
-    uint64_t *qFull = bars, *k01Full = bars + 1, *stFull = bars + 2, *stEmpty = stFull + NS,
-             *sFull = stEmpty + NS /* [x][b] */, *pFull = sFull + 4 /* [x][b] */, *pvDone = pFull + 4 /* [x] */,
-             *pvBuf = pvDone + 2 /* [x][b] */, *qFree = pvBuf + 4 /* [x] */, *itemFull = qFree + 2 /* [4] */;
+    uint64_t *qFull = bars, *kFull = bars + 1, *kEmpty = kFull + NK, *vFull = kEmpty + NK, *vEmpty = vFull + NV,
+             *sFull = vEmpty + NV /* [x][b] */, *pFull = sFull + 4 /* [x][b] */, *pvDone = pFull + 4 /* [x] */,
+             *pvBuf = pvDone + 2 /* [x][b] */, *qFree = pvBuf + 4 /* [x] */, *itemFull = qFree + 2 /* [4] */,
+             *exFull = itemFull + 4, *exRead = exFull + 1;
     uint32_t *tmemSlot = reinterpret_cast<uint32_t *>(smem + L::kTmemSlot);
     volatile uint32_t *itemSlots = reinterpret_cast<volatile uint32_t *>(smem + L::kItemSlots);  // [4]
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const bool split = !kOne && p.split != 0;
 
     if (threadIdx.x == 0) {
         mbarInit(qFull, 1);
-        mbarInit(k01Full, 1);
-        for (uint32_t s = 0; s < NS; ++s) {
-            mbarInit(&stFull[s], 1);
-            mbarInit(&stEmpty[s], 4);  // all four MMA warps release a stage
+        // a K (V) tile is released by the score (P.V) warps of the query tiles that it serves
+        const uint32_t users = kOne || split ? 1u : 2u;
+        for (uint32_t s = 0; s < NK; ++s) {
+            mbarInit(&kFull[s], 1);
+            mbarInit(&kEmpty[s], users);
+        }
+        for (uint32_t s = 0; s < NV; ++s) {
+            mbarInit(&vFull[s], 1);
+            mbarInit(&vEmpty[s], users);
         }
         for (int i = 0; i < 4; ++i) {
             mbarInit(&sFull[i], 1);
@@ -314,8 +410,10 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         }
         mbarInit(&pvDone[0], 1);
         mbarInit(&pvDone[1], 1);
-        mbarInit(&qFree[0], 1);  // score warp X is done with the query tiles and K_0, K_1
+        mbarInit(&qFree[0], 1);  // score warp X is done with the query tiles
         mbarInit(&qFree[1], 1);
+        mbarInit(exFull, 2 * kPfBM);  // split items: every softmax thread has left its (m, l) / has read the accumulators
+        mbarInit(exRead, 2 * kPfBM);
         fenceBarrierInit();
         tmaPrefetchDesc(&tmQ);
         tmaPrefetchDesc(&tmK);
@@ -343,63 +441,63 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     if (warp == 8) {
         // ------------------------ TMA producer and scheduler ------------------------
         if (lane == 0) {
-            uint32_t item = blockIdx.x, g = 0;  // g: K/V tiles requested so far, over all items
+            uint32_t item = blockIdx.x, gk = 0, gv = 0;  // gk / gv: K / V tiles requested so far, over all items
             gridDepWait();  // the twins and the work counter come from the launch in front
+            gridDepLaunch();
             itemSlots[0] = item;
             mbarArrive(&itemFull[0]);
             bool ok = true;
+            auto requestK = [&](uint32_t kvHead, uint32_t j) {
+                const uint32_t s = gk % NK;
+                if (gk >= NK && !pfWait(&kEmpty[s], ((gk / NK) - 1u) & 1u, p.err, kDevErrEmptyWait)) return false;
+                mbarExpectTx(&kFull[s], L::kKvTile);
+#pragma unroll
+                for (int h = 0; h < L::kHalves; ++h)
+                    tmaLoad3D(smem + L::kK + s * L::kKvTile + h * L::kKvHalf, &tmK, &kFull[s], 64 * h, kvHead, j * BN);
+                ++gk;
+                return true;
+            };
+            auto requestV = [&](uint32_t kvHead, uint32_t j) {
+                const uint32_t s = gv % NV;
+                if (gv >= NV && !pfWait(&vEmpty[s], ((gv / NV) - 1u) & 1u, p.err, kDevErrEmptyWait)) return false;
+                mbarExpectTx(&vFull[s], L::kKvTile);
+#pragma unroll
+                for (int h = 0; h < L::kHalves; ++h)
+                    tmaLoad3D(smem + L::kV + s * L::kKvTile + h * L::kKvHalf, &tmV, &vFull[s], 64 * h, kvHead, j * BN);
+                ++gv;
+                return true;
+            };
             for (uint32_t n = 0; ok && item < p.totalItems; ++n) {
-                const PfItem it = pfItem<BN>(p, item);
+                const PfItem it = pfItem(p, item);
                 PF_BLK(0);
 #ifdef TC_TRACE
                 if (p.trace) { unsigned sm; asm("mov.u32 %0, %%smid;" : "=r"(sm)); p.trace[8u * 64u * 4u + item * 8u + 6] = sm; }
 #endif
-                // the query tiles and K_0, K_1 are free once both score warps have issued the last
-                // product of the previous item that reads them, and those products are complete
-                if (n > 0 && !(pfWait(&qFree[0], (n - 1u) & 1u, p.err, kDevErrEmptyWait) &&
-                               pfWait(&qFree[1], (n - 1u) & 1u, p.err, kDevErrEmptyWait))) {
-                    ok = false;
-                    break;
-                }
-                mbarExpectTx(qFull, L::kQTiles * L::kQTile);
-#pragma unroll
-                for (int x = 0; x < L::kQTiles; ++x)
+                // the query tiles are free once the score warps have issued the last product of the previous item and
+                // those products are complete
+                if (n > 0)
+                    ok = pfWait(&qFree[0], (n - 1u) & 1u, p.err, kDevErrEmptyWait) &&
+                         (kOne || pfWait(&qFree[1], (n - 1u) & 1u, p.err, kDevErrEmptyWait));
+                if (!ok) break;
+                const int qTiles = kOne || split ? 1 : 2;
+                mbarExpectTx(qFull, qTiles * L::kQTile);
+                for (int x = 0; x < qTiles; ++x)
 #pragma unroll
                     for (int h = 0; h < L::kHalves; ++h)
                         tmaLoad3D(smem + L::kQ + x * L::kQTile + h * L::kQHalf, &tmQ, qFull, 64 * h, it.head,
                                   it.m0 + x * kPfBM);
-                // K_0 and K_1 feed the products issued ahead of the loop (nTiles >= 2 always)
-                mbarExpectTx(k01Full, 2 * L::kKvTile);
-#pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    uint8_t *kd = smem + L::kK01 + j * L::kKvTile;
-#pragma unroll
-                    for (int h = 0; h < L::kHalves; ++h)
-                        tmaLoad3D(kd + h * L::kKvHalf, &tmK, k01Full, 64 * h, it.kvHead, j * BN);
-                }
+                ok = requestK(it.kvHead, 0) && (it.nTiles < 2u || requestK(it.kvHead, 1));
                 // The next item is drawn late -- with the third last tile request, some six tiles before
                 // the consumers finish this item -- so that the blocks which finish first take the
                 // heavier of the remaining items.
                 const uint32_t drawAt = it.nTiles >= 3u ? it.nTiles - 3u : 0u;
                 uint32_t drawn = 0, flags = 0;
-                for (uint32_t j = 0; j < it.nTiles; ++j, ++g) {
+                for (uint32_t j = 0; ok && j < it.nTiles; ++j) {
                     if (j == drawAt) {
                         flags = *reinterpret_cast<volatile unsigned int *>(p.err);
                         drawn = gridDim.x + atomicAdd(p.workCounter, 1u);
                     }
-                    const uint32_t s = g % NS;
-                    if (g >= NS && !pfWait(&stEmpty[s], ((g / NS) - 1u) & 1u, p.err, kDevErrEmptyWait)) {
-                        ok = false;
-                        break;
-                    }
-                    uint8_t *kd = smem + L::kStage + s * L::kStageBytes, *vd = kd + L::kKvTile;
-                    const bool withK = j + 2 < it.nTiles;
-                    mbarExpectTx(&stFull[s], withK ? 2 * L::kKvTile : L::kKvTile);
-#pragma unroll
-                    for (int h = 0; h < L::kHalves; ++h) {
-                        if (withK) tmaLoad3D(kd + h * L::kKvHalf, &tmK, &stFull[s], 64 * h, it.kvHead, (j + 2) * BN);
-                        tmaLoad3D(vd + h * L::kKvHalf, &tmV, &stFull[s], 64 * h, it.kvHead, j * BN);
-                    }
+                    ok = (j + 2u >= it.nTiles || requestK(it.kvHead, j + 2u)) && requestV(it.kvHead, j);
                 }
                 if (!ok) break;
                 // a wait that ran out anywhere ends the launch: the flag is the caller's to read
@@ -409,10 +507,14 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 mbarArrive(&itemFull[(n + 1u) & 3u]);
                 item = next;
             }
-            // the last release of every stage has to have arrived before the block leaves
-            for (uint32_t back = 0; ok && back < NS && back < g; ++back) {
-                const uint32_t gg = g - 1u - back;
-                ok = pfWait(&stEmpty[gg % NS], (gg / NS) & 1u, p.err, kDevErrEmptyWait);
+            // the last release of every slot has to have arrived before the block leaves
+            for (uint32_t back = 0; ok && back < NK && back < gk; ++back) {
+                const uint32_t g = gk - 1u - back;
+                ok = pfWait(&kEmpty[g % NK], (g / NK) & 1u, p.err, kDevErrEmptyWait);
+            }
+            for (uint32_t back = 0; ok && back < NV && back < gv; ++back) {
+                const uint32_t g = gv - 1u - back;
+                ok = pfWait(&vEmpty[g % NV], (g / NV) & 1u, p.err, kDevErrEmptyWait);
             }
         }
     } else if (warp >= 9) {
@@ -430,76 +532,77 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         const uint32_t issue = lane == 0 ? 1u : 0u;
         constexpr uint32_t idQK = umaInstrDescF16(kPfBM, BN, 0, 0);
         constexpr uint32_t idPV = umaInstrDescF16(kPfBM, HD, 0, 1);
-        const uint64_t dQ = umaSmemDesc(smemAddr(smem + L::kQ + x * L::kQTile), 16, 1024);
-        const uint64_t dK01 = umaSmemDesc(smemAddr(smem + L::kK01), 16, 1024);
-        const uint64_t dKs = umaSmemDesc(smemAddr(smem + L::kStage), 16, 1024);
-        const uint64_t dVs = umaSmemDesc(smemAddr(smem + L::kStage + L::kKvTile), L::kKvHalf, 1024);
+        const uint64_t dQ = umaSmemDesc(smemAddr(smem + L::kQ + (split ? 0u : x) * L::kQTile), 16, 1024);
+        const uint64_t dK0 = umaSmemDesc(smemAddr(smem + L::kK), 16, 1024);
+        const uint64_t dV0 = umaSmemDesc(smemAddr(smem + L::kV), L::kKvHalf, 1024);
         const uint32_t tO = tmemBase + 128u * x, tS0 = tmemBase + 256u + 128u * x;
-        // score product of running tile tt from the K tile at descriptor dK; tt >= 2 first waits
-        // until the P.V product of tile tt - 2 has left the buffer
-        auto issueQK = [&](uint64_t dK, uint32_t tt) -> bool {
-            if (tt >= 2u && !pfWait(&pvBuf[2u * x + (tt & 1u)], ((tt - 2u) >> 1) & 1u, p.err, kDevErrMmaWait)) return false;
-            tcFenceAfter();
-#pragma unroll
-            for (uint32_t ks = 0; ks < HD / 16; ++ks) {
-                // k step ks: dims 16 ks .. +15 = 32 bytes inside the (ks >> 2)-th 64-dim half
-                umaMmaSSIf(issue, tS0 + 64u * (tt & 1u), descAdvance(dQ, (ks >> 2) * L::kQHalf + (ks & 3u) * 32u),
-                           descAdvance(dK, (ks >> 2) * L::kKvHalf + (ks & 3u) * 32u), idQK, ks > 0 ? 1u : 0u);
-            }
-            umaCommitIf(issue, &sFull[2u * x + (tt & 1u)]);
-            return true;
-        };
-        uint32_t g = 0, t = 0, item = 0;  // K/V tiles consumed, tiles of X done, over all items
-        bool ok = true;
+        uint32_t g = 0, t = 0, item = 0;  // K (V) tiles of the items done, tiles of X done, over all items
+        bool ok = !(kOne && x == 1u);
         for (uint32_t n = 0; ok && takeItem(n, item); ++n) {
-            const PfItem it = pfItem<BN>(p, item);
+            const PfItem it = pfItem(p, item);
             const uint32_t myTiles = x == 0 ? it.nA : it.nB;
-            if (!pvRole) {
-                if (myTiles != 0) {
-                    ok = pfWait(qFull, n & 1u, p.err, kDevErrFullWait) && pfWait(k01Full, n & 1u, p.err, kDevErrFullWait);
-                    ok = ok && issueQK(dK01, t) && issueQK(descAdvance(dK01, L::kKvTile), t + 1u);
-                    if (myTiles <= 2u) umaCommitIf(issue, &qFree[x]);
-                }
-            }
-            // Every stage is released by all four warps, also the ones past a tile's diagonal -- but
-            // only after the stage has been filled: a warp with nothing to do must not run ahead and
-            // hand in the release of a later round, or the barrier would complete without the warp
-            // that still reads the stage.
-            for (uint32_t j = 0; ok && j < it.nTiles; ++j, ++g) {
-                const uint32_t s = g % NS;
-                ok = pfWait(&stFull[s], (g / NS) & 1u, p.err, kDevErrFullWait);
-                if (!ok) break;
-                if (pvRole && j < myTiles) {
-                    const uint32_t tt = t + j;
-                    if (lane == 0) PF_STAMP(4u + x, j, 0);
-                    ok = pfWait(&pFull[2u * x + (tt & 1u)], (tt >> 1) & 1u, p.err, kDevErrMmaWait);
-                    if (lane == 0) PF_STAMP(4u + x, j, 1);
-                    if (!ok) break;
-                    tcFenceAfter();
-                    const uint64_t dV = descAdvance(dVs, s * L::kStageBytes);
-                    const uint32_t tP = tS0 + 64u * (tt & 1u);
-#pragma unroll
-                    for (uint32_t ks = 0; ks < BN / 16; ++ks)  // 16 tokens per step: 8 columns of fp16 P, 2 KB of V
-                        umaMmaTSIf(issue, tO, tP + ks * 8u, descAdvance(dV, ks * 2048u), idPV, (j > 0 || ks > 0) ? 1u : 0u);
-                    umaCommitIf(issue, &pvDone[x]);
-                    umaCommitIf(issue, &pvBuf[2u * x + (tt & 1u)]);
-                    if (lane == 0) PF_STAMP(4u + x, j, 2);
-                } else if (!pvRole && j + 2 < myTiles) {
+            // A split item's warps look at their own KV tiles only.  In a two-tile item every tile is released by both
+            // query tiles' warps, also the ones past a tile's diagonal -- but only after it has been filled: a warp with
+            // nothing to do must not run ahead and hand in the release of a later round, or the barrier would complete
+            // without the warp that still reads the slot.
+            const uint32_t j0 = split ? x : 0u, step = split ? 2u : 1u;
+            uint32_t tt = t;
+            for (uint32_t j = j0; ok && j < it.nTiles; j += step, ++tt) {
+                const uint32_t gg = g + j;
+                const bool mine = split || j < myTiles;
+                if (!pvRole) {
+                    const uint32_t s = gg % NK;
+                    if (mine && j == j0) ok = pfWait(qFull, n & 1u, p.err, kDevErrFullWait);
                     if (lane == 0) PF_STAMP(2u + x, j, 0);
-                    ok = issueQK(descAdvance(dKs, s * L::kStageBytes), t + j + 2u);
-                    if (!ok) break;
-                    if (lane == 0) PF_STAMP(2u + x, j, 2);
-                    // the item's last score product: the query tiles may be replaced once it is complete
-                    if (j + 3u == myTiles) umaCommitIf(issue, &qFree[x]);
+                    ok = ok && pfWait(&kFull[s], (gg / NK) & 1u, p.err, kDevErrFullWait);
+                    if (mine) {
+                        if (ok && tt >= 2u) ok = pfWait(&pvBuf[2u * x + (tt & 1u)], ((tt - 2u) >> 1) & 1u, p.err, kDevErrMmaWait);
+                        if (!ok) break;
+                        tcFenceAfter();
+                        const uint64_t dK = descAdvance(dK0, s * L::kKvTile);
+#pragma unroll
+                        for (uint32_t ks = 0; ks < HD / 16; ++ks) {
+                            // k step ks: dims 16 ks .. +15 = 32 bytes inside the (ks >> 2)-th 64-dim half
+                            umaMmaSSIf(issue, tS0 + 64u * (tt & 1u), descAdvance(dQ, (ks >> 2) * L::kQHalf + (ks & 3u) * 32u),
+                                       descAdvance(dK, (ks >> 2) * L::kKvHalf + (ks & 3u) * 32u), idQK, ks > 0 ? 1u : 0u);
+                        }
+                        umaCommitIf(issue, &sFull[2u * x + (tt & 1u)]);
+                        if (lane == 0) PF_STAMP(2u + x, j, 2);
+                        // the item's last score product: the query tiles may be replaced once it is complete
+                        if (tt + 1u == t + myTiles) umaCommitIf(issue, &qFree[x]);
+                    }
+                    if (ok) umaCommitIf(issue, &kEmpty[s]);
+                } else {
+                    const uint32_t s = gg % NV;
+                    ok = pfWait(&vFull[s], (gg / NV) & 1u, p.err, kDevErrFullWait);
+                    if (mine) {
+                        if (lane == 0) PF_STAMP(4u + x, j, 0);
+                        ok = ok && pfWait(&pFull[2u * x + (tt & 1u)], (tt >> 1) & 1u, p.err, kDevErrMmaWait);
+                        if (lane == 0) PF_STAMP(4u + x, j, 1);
+                        if (!ok) break;
+                        tcFenceAfter();
+                        const uint64_t dV = descAdvance(dV0, s * L::kKvTile);
+                        const uint32_t tP = tS0 + 64u * (tt & 1u);
+#pragma unroll
+                        for (uint32_t ks = 0; ks < BN / 16; ++ks)  // 16 tokens per step: 8 columns of fp16 P, 2 KB of V
+                            umaMmaTSIf(issue, tO, tP + ks * 8u, descAdvance(dV, ks * 2048u), idPV, (tt > t || ks > 0) ? 1u : 0u);
+                        umaCommitIf(issue, &pvDone[x]);
+                        umaCommitIf(issue, &pvBuf[2u * x + (tt & 1u)]);
+                        if (lane == 0) PF_STAMP(4u + x, j, 2);
+                    }
+                    if (ok) umaCommitIf(issue, &vEmpty[s]);
                 }
-                umaCommitIf(issue, &stEmpty[s]);
             }
-            // A tile that is not there still hands in its phase of qFree, one per item -- but only
-            // behind the item's last stage: the producer fills that stage after it has looked at the
-            // previous phase, so this warp cannot complete two phases before the producer has seen
-            // the first (a parity wait cannot tell those apart).
-            if (!pvRole && myTiles == 0u && ok) umaCommitIf(issue, &qFree[x]);
+            // A half without tiles still hands in its phase of qFree, one per item -- but only behind the item's last
+            // K tile: the producer fills that tile after it has looked at the previous phase, so this warp cannot
+            // complete two phases before the producer has seen the first (a parity wait cannot tell those apart).
+            // (A split item without odd tiles has one tile: its own full barrier stands for the last K tile.)
+            if (!pvRole && myTiles == 0u && ok) {
+                if (split) ok = pfWait(&kFull[g % NK], (g / NK) & 1u, p.err, kDevErrFullWait);
+                if (ok) umaCommitIf(issue, &qFree[x]);
+            }
             t += myTiles;
+            g += it.nTiles;
         }
         if (pvRole && ok) {
             // nobody waits for the last two buffer commits; they have to land before the block leaves
@@ -511,19 +614,23 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         const uint32_t x = warp >> 2;                         // which query tile this warpgroup owns
         const uint32_t row = (warp & 3u) * 32u + lane;        // row of that tile = TMEM lane
         const uint32_t laneBase = ((warp & 3u) * 32u) << 16;  // TMEM lane field
-        const uint32_t rowInBlock = x * kPfBM + row;          // row inside the 256-row block
+        const uint32_t tileRow0 = split ? 0u : x * kPfBM;     // the tile's first row inside the item
+        const uint32_t rowInBlock = tileRow0 + row;
         const uint32_t tO = tmemBase + 128u * x;
+        // split items: (m, l) of a half's rows, in the room of the query tile that they do not have
+        float2 *exch = reinterpret_cast<float2 *>(smem + L::kQ + (kOne ? 0 : L::kQTile));
         uint32_t t = 0, item = 0;  // tiles of X done over all items
         bool ok = true;
         for (uint32_t n = 0; ok && takeItem(n, item); ++n) {
-            const PfItem it = pfItem<BN>(p, item);
+            const PfItem it = pfItem(p, item);
             const uint32_t m0 = it.m0, head = it.head;
             const uint32_t rq = m0 + rowInBlock;  // query position
             const uint32_t myTiles = x == 0 ? it.nA : it.nB;
-            if (myTiles == 0) continue;
+            if (myTiles == 0 && !split) continue;
             float m = kNegBig, l = 0.0f;
             for (uint32_t j = 0; j < myTiles; ++j) {
                 const uint32_t tt = t + j, b = tt & 1u;
+                const uint32_t kt = split ? 2u * j + x : j;  // KV tile
                 const uint32_t tS = tmemBase + 256u + 128u * x + 64u * b;
                 if (row == 0) PF_STAMP(x, j, 0);
                 if (!pfWait(&sFull[2u * x + b], (tt >> 1) & 1u, p.err, kDevErrMmaWait)) {
@@ -538,11 +645,11 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 for (int c = 0; c < NC; ++c) tmemLd32(tS + laneBase + 32u * c, r[c]);
                 tmemLdWait();
                 if (row == 0 && x == 0) PF_STAMP(6u, j, 0);
-                if (BN * j + (BN - 1u) > p.cachePos + m0 + x * kPfBM) {
+                if (BN * kt + (BN - 1u) > p.cachePos + m0 + tileRow0) {
                     // causal edge (the tile reaches past the position of this tile's first row): token
-                    // 64 j + c is visible iff it is not past the query position; relative to the block's
-                    // first row that is 64 j - (cachePos + m0) + c <= rowInBlock
-                    const int32_t first = static_cast<int32_t>(BN * j) - static_cast<int32_t>(p.cachePos + m0);
+                    // 64 kt + c is visible iff it is not past the query position; relative to the item's
+                    // first row that is 64 kt - (cachePos + m0) + c <= rowInBlock
+                    const int32_t first = static_cast<int32_t>(BN * kt) - static_cast<int32_t>(p.cachePos + m0);
 #pragma unroll
                     for (int c = 0; c < NC; ++c)
 #pragma unroll
@@ -627,34 +734,81 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 if (row == 0) PF_STAMP(x, j, 2);
                 if (row == 0 && j + 1u == myTiles) PF_BLK(3u + x);
             }
-            if (!ok || !pfWait(&pvDone[x], (t + myTiles - 1u) & 1u, p.err, kDevErrMmaWait)) {
-                ok = false;
-                break;
+            ok = ok && (myTiles == 0 || pfWait(&pvDone[x], (t + myTiles - 1u) & 1u, p.err, kDevErrMmaWait));
+            if (!ok) break;
+            // Split items: each half leaves (m, l) of its rows for the other one and stores half of the dims, out of both
+            // accumulators (they lie in the same TMEM lanes).
+            float inv, wOther = 0.0f;
+            bool both = false;
+            if (split) {
+                exch[x * kPfBM + row] = make_float2(m, l);
+                tcFenceBefore();
+                mbarArrive(exFull);
+                ok = pfWait(exFull, n & 1u, p.err, kDevErrMmaWait);
+                if (!ok) break;
+                tcFenceAfter();
+                const float2 o = exch[(x ^ 1u) * kPfBM + row];
+                const float M = fmaxf(m, o.x), wMine = fastExp2(m - M);
+                wOther = fastExp2(o.x - M);
+                const float lAll = fmaf(wMine, l, wOther * o.y);
+                inv = lAll > 0.0f ? 1.0f / lAll : 0.0f;
+                wOther *= inv;
+                inv *= wMine;
+                both = it.nB != 0u;
+            } else {
+                tcFenceAfter();
+                inv = l > 0.0f ? 1.0f / l : 0.0f;
             }
-            tcFenceAfter();
-            const float inv = l > 0.0f ? 1.0f / l : 0.0f;
             float *orow = p.out + (static_cast<size_t>(rq) * p.nHeads + head) * HD;
+            // this half's 32-column chunks
+            constexpr uint32_t kChunks = HD / 32;
+            const uint32_t c0 = split ? x * (kChunks / 2) : 0u, c1 = split ? c0 + kChunks / 2 : kChunks;
+            if (split && x == 1u && !both) inv = 0.0f;  // no odd tiles: accumulator B was never written
 #pragma unroll 1
-            for (uint32_t c = 0; c < HD / 32; ++c) {
+            for (uint32_t c = c0; c < c1; ++c) {
                 uint32_t o[32];
-                tmemLd32(tO + laneBase + c * 32u, o);
-                tmemLdWait();
+                if (split && x == 1u && !both) {
+                    // everything is in accumulator A
+                    tmemLd32(tmemBase + laneBase + c * 32u, o);
+                    tmemLdWait();
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * wOther);
+                } else if (both) {
+                    uint32_t o2[32];
+                    tmemLd32(tO + laneBase + c * 32u, o);
+                    tmemLd32(tmemBase + 128u * (x ^ 1u) + laneBase + c * 32u, o2);
+                    tmemLdWait();
+#pragma unroll
+                    for (int i = 0; i < 32; ++i)
+                        o[i] = __float_as_uint(fmaf(__uint_as_float(o2[i]), wOther, __uint_as_float(o[i]) * inv));
+                } else {
+                    tmemLd32(tO + laneBase + c * 32u, o);
+                    tmemLdWait();
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * inv);
+                }
                 if (rq < p.seqLen && !p.out32) {
 #pragma unroll
                     for (int i = 0; i < 8; ++i)
                         *reinterpret_cast<float4 *>(orow + c * 32 + 4 * i) =
-                                make_float4(__uint_as_float(o[4 * i]) * inv, __uint_as_float(o[4 * i + 1]) * inv,
-                                            __uint_as_float(o[4 * i + 2]) * inv, __uint_as_float(o[4 * i + 3]) * inv);
+                                make_float4(__uint_as_float(o[4 * i]), __uint_as_float(o[4 * i + 1]),
+                                            __uint_as_float(o[4 * i + 2]), __uint_as_float(o[4 * i + 3]));
                 } else if (rq < p.seqLen) {
                     // 32 bytes per store: a thread owns its row, so a warp's store touches 32 rows, and
                     // whole sectors halve the number of transactions against 16-byte stores
 #pragma unroll
                     for (int i = 0; i < 4; ++i)
-                        stGlobalV8(orow + c * 32 + 8 * i, __uint_as_float(o[8 * i]) * inv, __uint_as_float(o[8 * i + 1]) * inv,
-                                   __uint_as_float(o[8 * i + 2]) * inv, __uint_as_float(o[8 * i + 3]) * inv,
-                                   __uint_as_float(o[8 * i + 4]) * inv, __uint_as_float(o[8 * i + 5]) * inv,
-                                   __uint_as_float(o[8 * i + 6]) * inv, __uint_as_float(o[8 * i + 7]) * inv);
+                        stGlobalV8(orow + c * 32 + 8 * i, __uint_as_float(o[8 * i]), __uint_as_float(o[8 * i + 1]),
+                                   __uint_as_float(o[8 * i + 2]), __uint_as_float(o[8 * i + 3]),
+                                   __uint_as_float(o[8 * i + 4]), __uint_as_float(o[8 * i + 5]),
+                                   __uint_as_float(o[8 * i + 6]), __uint_as_float(o[8 * i + 7]));
                 }
+            }
+            if (split) {
+                // the next item's first P.V product may overwrite an accumulator once both halves have read it
+                tcFenceBefore();
+                mbarArrive(exRead);
+                ok = pfWait(exRead, n & 1u, p.err, kDevErrMmaWait);
             }
             if (threadIdx.x == 0) PF_BLK(5);
             t += myTiles;
@@ -710,10 +864,13 @@ int tc_attn_prefill_f16_scratch_bytes(uint32_t seqLen, uint32_t cachePos, uint32
     return TC_OK;
 }
 
-static int prefillF16Impl(const float *q, const tc::PrefillKvSource &src, float *out, void *scratch,
-                          size_t scratchBytes, uint32_t seqLen, uint32_t cachePos, uint32_t nHeads, uint32_t nKV,
-                          uint32_t hd, float invSqrt, const tc::PrefillMirror &mir, tc_stream stream) {
-    using namespace tc;
+}  // extern "C"
+
+namespace tc {
+
+int prefillF16(float *q, const PrefillKvStore &src, float *out, void *scratch, size_t scratchBytes, uint32_t seqLen,
+               uint32_t cachePos, uint32_t nHeads, uint32_t nKV, uint32_t hd, float invSqrt, const PrefillMirror &mir,
+               const PrefillNewRows &nr, cudaStream_t st) {
     const void *kvK = src.k, *kvV = src.v;
     TC_REQUIRE(q && kvK && kvV && out && scratch, TC_EINVAL, "tc_attn_prefill_f16: null pointer");
     TC_REQUIRE(src.kind != 2 || (src.ks && src.vs), TC_EINVAL, "tc_attn_prefill_f16: null scale pointer");
@@ -721,7 +878,9 @@ static int prefillF16Impl(const float *q, const tc::PrefillKvSource &src, float 
     TC_REQUIRE(nKV > 0 && nHeads % nKV == 0, TC_EINVAL, "tc_attn_prefill_f16: nHeads %u not a multiple of nKV %u",
                nHeads, nKV);
     TC_REQUIRE(((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(kvK) | reinterpret_cast<uintptr_t>(kvV) |
-                 reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(scratch)) & 15u) == 0,
+                 reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(scratch) | reinterpret_cast<uintptr_t>(nr.k) |
+                 reinterpret_cast<uintptr_t>(nr.v) | reinterpret_cast<uintptr_t>(nr.cosT) |
+                 reinterpret_cast<uintptr_t>(nr.sinT)) & 15u) == 0,
                TC_EINVAL, "tc_attn_prefill_f16: pointers need 16-byte alignment");
     if (seqLen == 0) return TC_OK;
     TC_REQUIRE(static_cast<uint64_t>(cachePos) + seqLen < (1ull << 31), TC_EUNSUPPORTED,
@@ -741,11 +900,9 @@ static int prefillF16Impl(const float *q, const tc::PrefillKvSource &src, float 
             hd == 256 || static_cast<uint64_t>((seqLen + 2 * kPfBM - 1) / (2 * kPfBM)) * nHeads < static_cast<uint64_t>(sms)
                     ? kPfBM
                     : 2 * kPfBM;
-    const uint32_t bn = hd == 256 ? 32u : 64u;  // tokens per KV tile
     const uint32_t nQTiles = (seqLen + itemRows - 1) / itemRows;
     TC_REQUIRE(static_cast<uint64_t>(nQTiles) * nHeads < (1ull << 31), TC_EUNSUPPORTED,
                "tc_attn_prefill_f16: grid too large");
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
     auto al = [](size_t x) { return (x + 1023) & ~size_t(1023); };
     const size_t qElems = static_cast<size_t>(seqLen) * nHeads * hd;
     const uint32_t kvRows = cachePos + seqLen;  // the cache rows this call attends over
@@ -761,25 +918,28 @@ static int prefillF16Impl(const float *q, const tc::PrefillKvSource &src, float 
     unsigned int *err = devErrorWord();
     TC_REQUIRE(err != nullptr, TC_ECUDA, "tc_attn_prefill_f16: no device error word");
     {
-        const size_t nq4 = qElems / 4, kvRowHeads = src.kind == 1 ? 0 : static_cast<size_t>(kvRows) * nKV;
-        const size_t threads = std::max(nq4, kvRowHeads * 32);
+        PrefillRowsParams rp;
+        rp.q = q;
+        rp.q16 = static_cast<uint2 *>(q16);
+        rp.k16 = src.kind == 1 ? nullptr : static_cast<uint2 *>(k16);
+        rp.v16 = src.kind == 1 ? nullptr : static_cast<uint2 *>(v16);
+        rp.st = src;
+        rp.nr = nr;
+        rp.mir = mir;
+        rp.seqLen = seqLen, rp.cachePos = cachePos, rp.nHeads = nHeads, rp.nKV = nKV;
+        rp.err = err, rp.workCounter = workCounter;
+        const size_t rowHeads = static_cast<size_t>(src.kind == 1 ? (nr.k != nullptr ? seqLen : 0) : kvRows) * nKV;
+        const size_t threads = std::max(qElems / 8, rowHeads * 32);
         const uint32_t blocks = static_cast<uint32_t>(std::min<size_t>((threads + 255) / 256, static_cast<size_t>(sms) * 16));
-        const bool i8 = src.kind == 2;
-        auto conv = hd > 128 ? f32ToF16MirrorKernel<2> : f32ToF16MirrorKernel<1>;
-        conv<<<blocks, 256, 0, st>>>(
-                reinterpret_cast<const float4 *>(q), i8 ? nullptr : static_cast<const float4 *>(kvK),
-                i8 ? nullptr : static_cast<const float4 *>(kvV), i8 ? static_cast<const uint32_t *>(kvK) : nullptr,
-                i8 ? static_cast<const uint32_t *>(kvV) : nullptr, src.ks, src.vs, static_cast<uint2 *>(q16),
-                static_cast<uint2 *>(k16), static_cast<uint2 *>(v16), nq4, kvRowHeads, hd / 4,
-                static_cast<size_t>(cachePos) * nKV, mir, nKV, err, workCounter);
+        const int rc = launchDependent(hd == 64 ? prefillRowsKernel<64> : (hd == 128 ? prefillRowsKernel<128> : prefillRowsKernel<256>), dim3(blocks), 256, 0, st, 1, rp);
+        if (rc != TC_OK) return rc;
     }
-    TC_CUDA_OK(cudaGetLastError());
     CUtensorMap tmQ, tmK, tmV;
     int rc = f16Map(q16, hd, nHeads, seqLen, kPfBM, &tmQ);
     if (rc != TC_OK) return rc;
-    rc = f16Map(k16, hd, nKV, kvRows, bn, &tmK);
+    rc = f16Map(k16, hd, nKV, kvRows, kPfBN, &tmK);
     if (rc != TC_OK) return rc;
-    rc = f16Map(v16, hd, nKV, kvRows, bn, &tmV);
+    rc = f16Map(v16, hd, nKV, kvRows, kPfBN, &tmV);
     if (rc != TC_OK) return rc;
     PrefillF16Params prm;
     prm.out = out;
@@ -790,6 +950,7 @@ static int prefillF16Impl(const float *q, const tc::PrefillKvSource &src, float 
     prm.group = nHeads / nKV;
     prm.nQTiles = nQTiles;
     prm.itemRows = itemRows;
+    prm.split = itemRows == kPfBM && hd != 256 ? 1u : 0u;
     prm.scaleLog2 = invSqrt * kLog2e;
     prm.err = err;
     prm.workCounter = workCounter;
@@ -802,44 +963,44 @@ static int prefillF16Impl(const float *q, const tc::PrefillKvSource &src, float 
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !attrDone[dev]) {
-        TC_CUDA_OK(cudaFuncSetAttribute(prefillF16Kernel<64, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        PrefillF16Smem<64, 64>::kTotal));
-        TC_CUDA_OK(cudaFuncSetAttribute(prefillF16Kernel<128, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        PrefillF16Smem<128, 64>::kTotal));
-        TC_CUDA_OK(cudaFuncSetAttribute(prefillF16Kernel<256, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        PrefillF16Smem<256, 32>::kTotal));
+        TC_CUDA_OK(cudaFuncSetAttribute(prefillF16Kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        PrefillF16Smem<64>::kTotal));
+        TC_CUDA_OK(cudaFuncSetAttribute(prefillF16Kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        PrefillF16Smem<128>::kTotal));
+        TC_CUDA_OK(cudaFuncSetAttribute(prefillF16Kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        PrefillF16Smem<256>::kTotal));
         attrDone[dev] = true;
     }
     const uint32_t grid = std::min<uint32_t>(prm.totalItems, static_cast<uint32_t>(sms));  // one block per SM
-    // programmatic dependent launch: the blocks allocate TMEM and set up their barriers while the twins
-    // launch drains; the producer waits for it before its first load (nothing else reads its outputs)
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(kPfThreads);
-    cfg.dynamicSmemBytes = hd == 64 ? PrefillF16Smem<64, 64>::kTotal
-                                    : (hd == 128 ? PrefillF16Smem<128, 64>::kTotal : PrefillF16Smem<256, 32>::kTotal);
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    // (the blocks allocate TMEM and set up their barriers while the rows launch drains; the producer waits for it before its
+    // first load, nothing else reads its outputs)
     if (hd == 64)
-        TC_CUDA_OK(cudaLaunchKernelEx(&cfg, prefillF16Kernel<64, 64>, tmQ, tmK, tmV, prm));
-    else if (hd == 128)
-        TC_CUDA_OK(cudaLaunchKernelEx(&cfg, prefillF16Kernel<128, 64>, tmQ, tmK, tmV, prm));
-    else
-        TC_CUDA_OK(cudaLaunchKernelEx(&cfg, prefillF16Kernel<256, 32>, tmQ, tmK, tmV, prm));
-    return TC_OK;
+        return launchDependent(prefillF16Kernel<64>, dim3(grid), kPfThreads, PrefillF16Smem<64>::kTotal, st, 1, tmQ, tmK, tmV, prm);
+    if (hd == 128)
+        return launchDependent(prefillF16Kernel<128>, dim3(grid), kPfThreads, PrefillF16Smem<128>::kTotal, st, 1, tmQ, tmK, tmV, prm);
+    return launchDependent(prefillF16Kernel<256>, dim3(grid), kPfThreads, PrefillF16Smem<256>::kTotal, st, 1, tmQ, tmK, tmV, prm);
 }
+
+static int prefillStore(const float *q, const PrefillKvStore &src, float *out, void *scratch, size_t scratchBytes,
+                        uint32_t seqLen, uint32_t cachePos, uint32_t nHeads, uint32_t nKV, uint32_t hd, float invSqrt,
+                        const PrefillMirror &mir, tc_stream stream) {
+    PrefillNewRows none;
+    memset(&none, 0, sizeof(none));
+    return prefillF16(const_cast<float *>(q), src, out, scratch, scratchBytes, seqLen, cachePos, nHeads, nKV, hd, invSqrt, mir,
+                      none, static_cast<cudaStream_t>(stream));
+}
+
+}  // namespace tc
+
+extern "C" {
 
 int tc_attn_prefill_f16(const float *q, const float *kvK, const float *kvV, float *out, void *scratch,
                         size_t scratchBytes, uint32_t seqLen, uint32_t cachePos, uint32_t nHeads, uint32_t nKV,
                         uint32_t hd, float invSqrt, tc_stream stream) {
     tc::PrefillMirror none;
     memset(&none, 0, sizeof(none));
-    const tc::PrefillKvSource src = {0, kvK, kvV, nullptr, nullptr};
-    return prefillF16Impl(q, src, out, scratch, scratchBytes, seqLen, cachePos, nHeads, nKV, hd, invSqrt, none, stream);
+    const tc::PrefillKvStore src = {0, const_cast<float *>(kvK), const_cast<float *>(kvV), nullptr, nullptr};
+    return tc::prefillStore(q, src, out, scratch, scratchBytes, seqLen, cachePos, nHeads, nKV, hd, invSqrt, none, stream);
 }
 
 int tc_attn_prefill_f16_kvhalf(const float *q, const void *kvK16, const void *kvV16, float *out, void *scratch,
@@ -847,8 +1008,8 @@ int tc_attn_prefill_f16_kvhalf(const float *q, const void *kvK16, const void *kv
                                uint32_t hd, float invSqrt, tc_stream stream) {
     tc::PrefillMirror none;
     memset(&none, 0, sizeof(none));
-    const tc::PrefillKvSource src = {1, kvK16, kvV16, nullptr, nullptr};
-    return prefillF16Impl(q, src, out, scratch, scratchBytes, seqLen, cachePos, nHeads, nKV, hd, invSqrt, none, stream);
+    const tc::PrefillKvStore src = {1, const_cast<void *>(kvK16), const_cast<void *>(kvV16), nullptr, nullptr};
+    return tc::prefillStore(q, src, out, scratch, scratchBytes, seqLen, cachePos, nHeads, nKV, hd, invSqrt, none, stream);
 }
 
 int tc_attn_prefill_f16_i8(const float *q, const int8_t *k8, const int8_t *v8, const float *ks, const float *vs,
@@ -856,8 +1017,9 @@ int tc_attn_prefill_f16_i8(const float *q, const int8_t *k8, const int8_t *v8, c
                            uint32_t nHeads, uint32_t nKV, uint32_t hd, float invSqrt, tc_stream stream) {
     tc::PrefillMirror none;
     memset(&none, 0, sizeof(none));
-    const tc::PrefillKvSource src = {2, k8, v8, ks, vs};
-    return prefillF16Impl(q, src, out, scratch, scratchBytes, seqLen, cachePos, nHeads, nKV, hd, invSqrt, none, stream);
+    const tc::PrefillKvStore src = {2, const_cast<int8_t *>(k8), const_cast<int8_t *>(v8), const_cast<float *>(ks),
+                                    const_cast<float *>(vs)};
+    return tc::prefillStore(q, src, out, scratch, scratchBytes, seqLen, cachePos, nHeads, nKV, hd, invSqrt, none, stream);
 }
 
 int tc_attn_prefill_f16_kv8(const float *q, const float *kvK, const float *kvV, float *out, void *scratch,
@@ -874,8 +1036,8 @@ int tc_attn_prefill_f16_kv8(const float *q, const float *kvK, const float *kvV, 
     }
     tc::PrefillMirror mir;
     mir.k8 = k8, mir.v8 = v8, mir.ks = ks, mir.vs = vs, mir.dstRow = kv8Row, mir.maxRows = kv8MaxRows;
-    const tc::PrefillKvSource src = {0, kvK, kvV, nullptr, nullptr};
-    return prefillF16Impl(q, src, out, scratch, scratchBytes, seqLen, cachePos, nHeads, nKV, hd, invSqrt, mir, stream);
+    const tc::PrefillKvStore src = {0, const_cast<float *>(kvK), const_cast<float *>(kvV), nullptr, nullptr};
+    return tc::prefillStore(q, src, out, scratch, scratchBytes, seqLen, cachePos, nHeads, nKV, hd, invSqrt, mir, stream);
 }
 
 }  // extern "C"
