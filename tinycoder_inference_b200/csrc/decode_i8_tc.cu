@@ -35,7 +35,7 @@
 #include <cstdlib>
 
 #include "tc_tcgen05.cuh"
-#include "decode_shared.cuh"
+#include "decode_cluster.cuh"
 
 namespace tc {
 
@@ -163,7 +163,10 @@ __device__ __forceinline__ float i2f(uint32_t x) { return __int2float_rn(static_
 // APPEND: the instantiation for calls that hand in the new token's rows.  It is a kernel of its own
 // because the mere presence of that (cold) code -- inlined or called, inside or behind the producer's
 // loop -- cost the 7B-shaped batch-1 step 0.5 us; calls without new rows run the other instantiation.
-template <int NWG, int NS, bool APPEND, bool TICKETS>
+// FOLD: how a sequence's blocks come together: a merge launch (or one block per sequence, which writes the output), the
+// last block to arrive (tickets), or a cluster that holds them all and folds through distributed shared memory.
+enum class TcFold { kLaunch, kTickets, kCluster };
+template <int NWG, int NS, bool APPEND, TcFold FOLD>
 __global__ void __launch_bounds__((4 * NWG + 9) * 32, 1)
 decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                  const __grid_constant__ CUtensorMap tmKn, const __grid_constant__ CUtensorMap tmVn,
@@ -208,14 +211,29 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     // length lets the producer start before the dependency wait.
     uint32_t len = p.lenHost;
     const bool earlyOk = p.devLens == nullptr && p.devRowBase == nullptr && p.prefetchRows != 0;
+    // a cluster shares the tiles that its sequence has, whatever the launch was sized for (a block may get none)
+    auto tokensOfBlock = [&]() {
+        return FOLD == TcFold::kCluster ? ((len + T - 1u) / T + gridDim.x - 1u) / gridDim.x * T : p.chunkTokens;
+    };
     if (!earlyOk) {
+        // pulling this block's rows into L2 is right at any time: a row that a kernel in flight writes is read after the wait
+        if (p.devLens == nullptr && p.devRowBase == nullptr && warp == kProducerWarp && lane < NS) {
+            const uint32_t tok = chunk * tokensOfBlock() + lane * T, end = min(len, (chunk + 1u) * tokensOfBlock());
+            if (tok < end) {
+                const int row = static_cast<int>(static_cast<uint64_t>(b) * p.rowsPerSeq + tok);
+                tmaPrefetchL2_3D(&tmK, 0, kvHead, row);
+                tmaPrefetchL2_3D(&tmV, 0, kvHead, row);
+            }
+        }
         gridDepWait();
         if (p.devLens) len = min(p.devLens[b] + p.lenAdd, p.lenHost);  // (the host's length is the upper bound)
     }
-    const uint32_t t0 = chunk * p.chunkTokens;
-    if (t0 >= len) return;  // inactive chunk (block-uniform): the merge derives the active count from len
-    const uint32_t t1 = min(len, t0 + p.chunkTokens);
-    const uint32_t nTiles = (t1 - t0 + T - 1) / T;
+    const uint32_t share = tokensOfBlock();
+    const uint32_t t0 = chunk * share;
+    // inactive chunk (block-uniform): the merge derives the active count from len
+    if (FOLD != TcFold::kCluster && t0 >= len) return;
+    const uint32_t t1 = min(len, t0 + share);
+    const uint32_t nTiles = t0 >= len ? 0u : (t1 - t0 + T - 1) / T;
     const uint64_t rowBase = p.devRowBase ? p.devRowBase[b] : static_cast<uint64_t>(b) * p.rowsPerSeq;
 
     if (warp == 0) {
@@ -245,7 +263,7 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
                 }
             }
         };
-        if (APPEND && p.appendK != nullptr && t1 == len && lane < 8u) {
+        if (APPEND && p.appendK != nullptr && t1 == len && nTiles != 0u && lane < 8u) {
             // the rows this block will append, towards L2 (their final contents arrive there too)
             const char *src = reinterpret_cast<const char *>((lane < 4u ? p.appendK : p.appendV) +
                                                              (static_cast<size_t>(b) * p.nKV + kvHead) * 128u) + (lane & 3u) * 128u;
@@ -290,7 +308,7 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         // The tile that holds the row of a token being appended (the last tile of the sequence's last
         // chunk) is requested apart from the loop: the row goes into the pool first, once the kernels
         // ahead have completed.
-        const bool appendHere = APPEND && p.appendK != nullptr && t1 == len;
+        const bool appendHere = APPEND && p.appendK != nullptr && t1 == len && nTiles != 0u;
         const uint32_t nLoop = appendHere ? nTiles - 1u : nTiles;
         bool okP = true;
         for (uint32_t it = 0; okP && it < nLoop; ++it) okP = requestTile(it);
@@ -600,6 +618,7 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         float *mF = scr + 8 * 128;
         float *mS = mF + 8;                       // [NWG][8]
         float *lS = mS + NWG * 8;                 // [4 NWG warps][8]
+        float *clusterL = lS + 4 * NWG * 8;       // [8]: row sums against mF (cluster fold)
         namedBarSync(kEndBar, kEndThreads);       // the fold warpgroup is through: every P tile has been consumed
         if (lane == 0) {
 #pragma unroll
@@ -627,7 +646,9 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
                     lsum = fmaf(a, lg, lsum);
                 }
                 const size_t oidx = static_cast<size_t>(b) * p.nHeads + kvHead * p.group + p.colBase + h;
-                if (p.directOut) {
+                if (FOLD == TcFold::kCluster) {
+                    if (d4 == 0) clusterL[h] = lsum;  // (the accumulators stay where they are, in oS)
+                } else if (p.directOut) {
                     const float inv = lsum > 0.0f ? 1.0f / lsum : 0.0f;
                     *reinterpret_cast<float4 *>(p.out + oidx * 128u + 4u * d4) =
                             make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
@@ -642,7 +663,7 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
                 }
             }
         }
-        if (TICKETS && !p.directOut && p.tickets != nullptr) {
+        if (FOLD == TcFold::kTickets && !p.directOut && p.tickets != nullptr) {
             // ---- merge inside the kernel: the block that arrives last at its (sequence, kv head)
             // counter folds all chunk partials of the kv head's q heads.  Nobody waits: every block
             // publishes its partial, takes a ticket and leaves unless the ticket is the last one.
@@ -701,6 +722,47 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     }
     if (threadIdx.x == 0) TC_STAMP(12);
     tcFenceBefore();
+    if (FOLD == TcFold::kCluster) {
+        // every block of the cluster has its accumulators, reference points and row sums in place: rank r puts together and
+        // stores the r-th share of the 8 x 128 outputs
+        clusterSync();
+        const uint32_t n = clusterSize(), per = 256u / n, base = smemAddr(smem + L::kP);
+        if (threadIdx.x < per) {
+            const uint32_t idx = clusterRank() * per + threadIdx.x, h = idx >> 5, d4 = idx & 31u;
+            if (p.colBase + h < p.group) {
+                float m[16], ls[16];
+                float4 a[16];
+#pragma unroll
+                for (uint32_t r = 0; r < 16; ++r) {
+                    m[r] = kNegBig, ls[r] = 0.0f, a[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (r < n) {
+                        const uint32_t q = mapRank(base, r);
+                        m[r] = ldCluster(q + (8 * 128 + h) * 4);
+                        ls[r] = ldCluster(q + (8 * 128 + 8 + 8 * NWG + 32 * NWG + h) * 4);
+                        a[r] = ldCluster4(q + (h * 128 + 4 * d4) * 4);
+                    }
+                }
+                float M = m[0], lsum = 0.0f;
+#pragma unroll
+                for (uint32_t r = 1; r < 16; ++r) M = fmaxf(M, m[r]);
+                float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (uint32_t r = 0; r < 16; ++r) {
+                    const float w = fastExp2(m[r] - M);
+                    lsum = fmaf(w, ls[r], lsum);
+                    acc.x = fmaf(w, a[r].x, acc.x);
+                    acc.y = fmaf(w, a[r].y, acc.y);
+                    acc.z = fmaf(w, a[r].z, acc.z);
+                    acc.w = fmaf(w, a[r].w, acc.w);
+                }
+                const float inv = lsum > 0.0f ? 1.0f / lsum : 0.0f;
+                const size_t oidx = static_cast<size_t>(b) * p.nHeads + kvHead * p.group + p.colBase + h;
+                *reinterpret_cast<float4 *>(p.out + oidx * 128u + 4u * d4) =
+                        make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
+            }
+        }
+        clusterSync();  // nobody leaves while its shared memory may still be read
+    }
     __syncthreads();
     if (warp == 0) {
         tcFenceAfter();
@@ -712,9 +774,31 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
 int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, const F32Mirror &mir, cudaStream_t st) {
     const uint32_t hd = 128;
     const uint32_t group = d->nHeads / d->nKV;
-    const DecodePlan pl = planDecode(d->batch, d->nKV, d->maxLen, d->numChunks, kTcTile, d->lens == nullptr, 1u);
+    using Smem = DecodeTcSmem<2, 6>;
+    // A cluster per (sequence, kv head) folds without partials and merge launch.  It is taken when all of them are resident
+    // at once (16 blocks: 7, 8: 15, 4: 33, 2: 74, a block filling an SM) and their blocks, fewer than the merge form's, do not
+    // cost more than the launch: a tile more per block takes 0.3 us while latency is what bounds it.  7B shape, per layer in
+    // a graph: 8192 rows 8.4 -> 7.1 us, 8 sequences of 2048 / 8192 rows 10.7 -> 8.3 / 18.1 -> 16.1, 16384 rows 9.0 in
+    // either form.  With ragged device lengths the cluster also shares every sequence evenly among its blocks, where the
+    // merge form cuts chunks by the longest one.
+    static ClusterSetup setup;
+    const uint32_t *limits = nullptr;
+    int rc = setupCluster(setup, decodeI8TcKernel<2, 6, true, TcFold::kCluster>, Smem::kThreads, Smem::kTotal, &limits);
+    if (rc != TC_OK) return rc;
+    DecodePlan pl = planDecode(d->batch, d->nKV, d->maxLen, d->numChunks, kTcTile, d->lens == nullptr, 1u);
+    uint32_t cluster = 1;
+    if (pl.chunksPerSeq > 1 && !d->partialsOnly && d->mergeTickets == nullptr) {
+        const uint32_t tiles = (d->maxLen + kTcTile - 1) / kTcTile;
+        const uint32_t most = d->lens == nullptr || d->batch == 1 ? pl.chunkTokens / kTcTile + 3u : 20u;  // tiles per block
+        for (uint32_t lg = 4; lg >= 1 && cluster == 1; --lg) {
+            const uint32_t n = 1u << lg;
+            if (n / 2u >= tiles || limits[lg] < d->nKV * d->batch || (tiles + n - 1u) / n > most) continue;
+            cluster = n;
+            pl.chunksPerSeq = n;
+        }
+    }
     const bool pdl = (d->flags & TC_DECODE_PDL) != 0;
-    const bool direct = pl.chunksPerSeq == 1 && !d->partialsOnly;
+    const bool direct = (pl.chunksPerSeq == 1 || cluster > 1) && !d->partialsOnly;
     if (!direct) TC_REQUIRE(d->pAcc && d->pM && d->pL, TC_EWORKSPACE, "decode_i8: partial buffers are required");
     if (d->chunksUsed) *d->chunksUsed = pl.chunksPerSeq;
     TC_REQUIRE(d->nKV <= 65535, TC_EUNSUPPORTED, "decode_i8: %u kv heads", d->nKV);
@@ -734,7 +818,7 @@ int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, c
     key.box[2] = kTcTile;
     CUtensorMap tmK, tmV;
     key.base = d->k8;
-    int rc = getTensorMap(key, &tmK);
+    rc = getTensorMap(key, &tmK);
     if (rc != TC_OK) return rc;
     key.base = d->v8;
     rc = getTensorMap(key, &tmV);
@@ -807,36 +891,37 @@ int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, c
 
     // (Four softmax warpgroups with a five-stage ring were measured and dropped: 11.5 against 8.3 us
     // per layer for the split launch alone at 32768 rows, 53.9 against 47.0 us at batch 8.)
-    using Smem = DecodeTcSmem<2, 6>;
-    // (the in-kernel merge is an instantiation of its own for the same reason as the append)
-    auto kern = d->appendK != nullptr ? (fused ? decodeI8TcKernel<2, 6, true, true> : decodeI8TcKernel<2, 6, true, false>)
-                                      : (fused ? decodeI8TcKernel<2, 6, false, true> : decodeI8TcKernel<2, 6, false, false>);
+    // (each way of coming together is an instantiation of its own for the same reason as the append)
+    using Kern = decltype(&decodeI8TcKernel<2, 6, true, TcFold::kLaunch>);
+    static const Kern kerns[2][3] = {
+            {decodeI8TcKernel<2, 6, false, TcFold::kLaunch>, decodeI8TcKernel<2, 6, false, TcFold::kTickets>,
+             decodeI8TcKernel<2, 6, false, TcFold::kCluster>},
+            {decodeI8TcKernel<2, 6, true, TcFold::kLaunch>, decodeI8TcKernel<2, 6, true, TcFold::kTickets>,
+             decodeI8TcKernel<2, 6, true, TcFold::kCluster>}};
     static bool attrDone[64] = {false};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !attrDone[dev]) {
-        TC_CUDA_OK(cudaFuncSetAttribute(decodeI8TcKernel<2, 6, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        Smem::kTotal));
-        TC_CUDA_OK(cudaFuncSetAttribute(decodeI8TcKernel<2, 6, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        Smem::kTotal));
-        TC_CUDA_OK(cudaFuncSetAttribute(decodeI8TcKernel<2, 6, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        Smem::kTotal));
-        TC_CUDA_OK(cudaFuncSetAttribute(decodeI8TcKernel<2, 6, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        Smem::kTotal));
+        for (auto &row : kerns)
+            for (Kern k : row) {
+                TC_CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem::kTotal));
+                TC_CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            }
         attrDone[dev] = true;
     }
+    const Kern kern = kerns[d->appendK != nullptr ? 1 : 0][cluster > 1 ? 2 : (fused ? 1 : 0)];
     // (without TC_DECODE_PDL prefetchRows is 0 and every block waits for the kernels ahead first thing)
     // a launch serves 8 q heads per kv head (the MMA columns); wider groups take one launch per
     // block of 8 and stream the rows again
     for (uint32_t cb = 0; cb < group; cb += 8) {
         prm.colBase = cb;
-        rc = launchDependent(kern, dim3(pl.chunksPerSeq, d->nKV, d->batch), Smem::kThreads, Smem::kTotal, st, 1, tmK, tmV,
-                             tmKn, tmVn, prm);
+        rc = launchDependent(kern, dim3(pl.chunksPerSeq, d->nKV, d->batch), Smem::kThreads, Smem::kTotal, st, cluster, tmK,
+                             tmV, tmKn, tmVn, prm);
         if (rc != TC_OK) return rc;
     }
     if (direct || d->partialsOnly || fused) return TC_OK;
     return launchMerge(d->pAcc, d->pM, d->pL, d->out, d->batch, d->nHeads, d->numChunks, pl.chunksPerSeq, hd, d->lens,
-                       lenAdd, pl.chunkTokens, nullptr, true, st);
+                       lenAdd, pl.chunkTokens, nullptr, pdl, st);
 }
 
 #ifdef TC_TRACE

@@ -194,6 +194,9 @@ int tc_kv_session_attend(tc_kv_session *s, uint32_t slot, float *q, const float 
         if (!c.kvStoreI8 && aligned) mir.k = static_cast<float *>(kvK), mir.v = static_cast<float *>(kvV);
         if (!c.kvStoreI8 && !aligned && (rc = append()) != TC_OK) return rc;
         describe(pos + 1u, nullptr);
+        // the layers of a token come one after the other: the next slot's rows towards L2
+        const uint32_t next = (slot + 1u) % c.slots;
+        if (next != slot) d.nextK8 = c.kvK8 + s->g.kv8LayerStride * next, d.nextV8 = c.kvV8 + s->g.kv8LayerStride * next;
         rc = tc::decodeI8Common(&d, pos + 1u, 0u, mir, static_cast<cudaStream_t>(stream));
         if (rc == TC_OK) rows8 = pos + 1u;
         return rc;

@@ -43,7 +43,8 @@ __global__ void __launch_bounds__(256)
 mergePartialsKernel(const float *__restrict__ pAcc, const float *__restrict__ pM, const float *__restrict__ pL,
                     float *__restrict__ out, uint32_t nHeads, uint32_t numChunks, uint32_t activeHost,
                     uint32_t hd, const uint32_t *__restrict__ devLens, uint32_t lenAdd, uint32_t chunkTokens,
-                    uint8_t *__restrict__ q81, uint32_t chunksPerRank, uint64_t rankStride, QRotation rot) {
+                    uint8_t *__restrict__ q81, uint32_t chunksPerRank, uint64_t rankStride, QRotation rot,
+                    uint32_t early) {
     constexpr int NW = 8;
     const uint32_t head = blockIdx.x, s = blockIdx.y;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
@@ -63,10 +64,11 @@ mergePartialsKernel(const float *__restrict__ pAcc, const float *__restrict__ pM
         const uint32_t r = c / chunksPerRank;
         return static_cast<uint64_t>(r) * rankStride + (headRow * chunksPerRank + (c - r * chunksPerRank)) * hd;
     };
-    // under programmatic dependent launch: let the next grid start its prologue, then
-    // wait until the grid that wrote the partials has finished (a no-op otherwise)
-    gridDepLaunch();
+    // let the next grid start its prologue -- ahead of the grid that wrote the partials only when that one's caller works
+    // under programmatic dependent launch itself -- and wait until the partials are complete
+    if (early) gridDepLaunch();
     gridDepWait();
+    if (!early) gridDepLaunch();
     // numChunks is the slot stride; only the first `active` slots were written
     uint32_t active = activeHost < numChunks ? activeHost : numChunks;
     if (devLens != nullptr) {
@@ -220,7 +222,7 @@ __global__ void __launch_bounds__(T)
 mergeSliceKernel(const float *__restrict__ pAcc, const float *__restrict__ pM, const float *__restrict__ pL,
                  float *__restrict__ out, uint32_t nHeads, uint32_t numChunks, uint32_t activeHost, uint32_t hd,
                  const uint32_t *__restrict__ devLens, uint32_t lenAdd, uint32_t chunkTokens, uint32_t chunksPerRank,
-                 uint64_t rankStride, QRotation rot) {
+                 uint64_t rankStride, QRotation rot, uint32_t early) {
     constexpr int NW = T / 32;
     const uint32_t head = blockIdx.x, s = blockIdx.y, slice = blockIdx.z;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
@@ -237,8 +239,9 @@ mergeSliceKernel(const float *__restrict__ pAcc, const float *__restrict__ pM, c
         const uint32_t r = c / chunksPerRank;
         return static_cast<uint64_t>(r) * rankStride + (headRow * chunksPerRank + (c - r * chunksPerRank)) * hd;
     };
-    gridDepLaunch();
+    if (early) gridDepLaunch();
     gridDepWait();
+    if (!early) gridDepLaunch();
     uint32_t active = activeHost < numChunks ? activeHost : numChunks;
     if (devLens != nullptr) {
         uint32_t len = devLens[s] + lenAdd, per = chunkTokens;
@@ -366,47 +369,134 @@ mergeSliceKernel(const float *__restrict__ pAcc, const float *__restrict__ pM, c
     }
 }
 
+// The merge of a batch: W warps of a 128-thread block per (token, head), each taking every W-th chunk; lane c of a warp
+// holds (m, l) of chunk c of a group of 32, a lane owns four dims (and 128 further on at head_dim 256).  With some thousand
+// (token, head) pairs of a few chunks each it is the number of blocks that costs: 64 sequences x 28 heads took 17 us
+// behind their decode launch with a 256-thread block per pair, NEWMERGE with a warp.
+template <int NV4, int W>
+__global__ void __launch_bounds__(128)
+mergeWarpKernel(const float *__restrict__ pAcc, const float *__restrict__ pM, const float *__restrict__ pL,
+                float *__restrict__ out, uint32_t units, uint32_t nHeads, uint32_t numChunks, uint32_t activeHost, uint32_t hd,
+                const uint32_t *__restrict__ devLens, uint32_t lenAdd, uint32_t chunkTokens, uint32_t early) {
+    __shared__ float4 sacc[W > 1 ? W : 1][NV4][32];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, part = warp % W;
+    const uint32_t unit = blockIdx.x * (4u / W) + warp / W;
+    if (early) gridDepLaunch();
+    gridDepWait();
+    if (!early) gridDepLaunch();
+    if (unit >= units) return;  // (W == 4: a block is one unit, nobody leaves alone)
+    uint32_t active = activeHost < numChunks ? activeHost : numChunks;
+    if (devLens != nullptr) {
+        const uint32_t need = (devLens[unit / nHeads] + lenAdd + chunkTokens - 1) / chunkTokens;
+        active = need < active ? need : active;  // never past the slots that the launch in front covered
+    }
+    const uint32_t nvec = hd >> 2;
+    const float *gm = pM + static_cast<uint64_t>(unit) * numChunks, *gl = pL + static_cast<uint64_t>(unit) * numChunks;
+    const float4 *ga = reinterpret_cast<const float4 *>(pAcc) + static_cast<uint64_t>(unit) * numChunks * nvec;
+    float4 acc[NV4];
+#pragma unroll
+    for (int j = 0; j < NV4; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    float M = kNegBig, lsum = 0.0f;
+    for (uint32_t c0 = 0; c0 < active; c0 += 32u) {
+        const uint32_t n = min(32u, active - c0);
+        constexpr uint32_t kB = 32u / W;  // chunks of this warp per group
+        // (addresses do not depend on the weights: everything is requested at once)
+        float4 a[kB < 8u ? kB : 8u][NV4];
+        constexpr uint32_t kHeld = kB < 8u ? kB : 8u;
+        auto load = [&](uint32_t i0) {
+#pragma unroll
+            for (uint32_t u = 0; u < kHeld; ++u) {
+                const uint32_t i = part + (i0 + u) * W;
+#pragma unroll
+                for (int j = 0; j < NV4; ++j) {
+                    a[u][j] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (i < n && lane + 32u * j < nvec) a[u][j] = __ldcg(ga + static_cast<uint64_t>(c0 + i) * nvec + lane + 32u * j);
+                }
+            }
+        };
+        load(0);
+        float mc = kNegBig, lc = 0.0f;
+        if (lane < n) mc = __ldcg(gm + c0 + lane), lc = __ldcg(gl + c0 + lane);
+        if (!(lc > 0.0f)) mc = kNegBig;
+        float Mn = mc;
+#pragma unroll
+        for (int o = 16; o; o >>= 1) Mn = fmaxf(Mn, __shfl_xor_sync(0xffffffffu, Mn, o));
+        Mn = fmaxf(M, Mn);
+        const float old = exp2f((M - Mn) * kLog2e);
+        const float w = lc > 0.0f ? exp2f((mc - Mn) * kLog2e) : 0.0f;
+        float wl = lc > 0.0f ? w * lc : 0.0f;
+#pragma unroll
+        for (int o = 16; o; o >>= 1) wl += __shfl_xor_sync(0xffffffffu, wl, o);
+        lsum = fmaf(lsum, old, wl);
+        M = Mn;
+#pragma unroll
+        for (int j = 0; j < NV4; ++j) acc[j].x *= old, acc[j].y *= old, acc[j].z *= old, acc[j].w *= old;
+        for (uint32_t i0 = 0; part + i0 * W < n; i0 += kHeld) {
+            if (i0) load(i0);
+#pragma unroll
+            for (uint32_t u = 0; u < kHeld; ++u) {
+                const uint32_t i = part + (i0 + u) * W;
+                const float wi = __shfl_sync(0xffffffffu, w, i & 31u);
+                if (i < n && wi != 0.0f) {  // an empty chunk is left out, never multiplied in
+#pragma unroll
+                    for (int j = 0; j < NV4; ++j) {
+                        acc[j].x = fmaf(wi, a[u][j].x, acc[j].x);
+                        acc[j].y = fmaf(wi, a[u][j].y, acc[j].y);
+                        acc[j].z = fmaf(wi, a[u][j].z, acc[j].z);
+                        acc[j].w = fmaf(wi, a[u][j].w, acc[j].w);
+                    }
+                }
+            }
+        }
+    }
+    if constexpr (W > 1) {
+#pragma unroll
+        for (int j = 0; j < NV4; ++j) sacc[part][j][lane] = acc[j];
+        __syncthreads();
+        if (part != 0) return;
+#pragma unroll
+        for (int j = 0; j < NV4; ++j)
+#pragma unroll
+            for (int w2 = 1; w2 < W; ++w2) {
+                const float4 x = sacc[w2][j][lane];
+                acc[j].x += x.x, acc[j].y += x.y, acc[j].z += x.z, acc[j].w += x.w;
+            }
+    }
+    const float inv = lsum > 0.0f ? 1.0f / lsum : 0.0f;
+#pragma unroll
+    for (int j = 0; j < NV4; ++j)
+        if (lane + 32u * j < nvec)
+            reinterpret_cast<float4 *>(out)[static_cast<uint64_t>(unit) * nvec + lane + 32u * j] =
+                    make_float4(acc[j].x * inv, acc[j].y * inv, acc[j].z * inv, acc[j].w * inv);
+}
+
 int launchMerge(const float *pAcc, const float *pM, const float *pL, float *out, uint32_t seqLen,
                 uint32_t nHeads, uint32_t numChunks, uint32_t activeHost, uint32_t hd, const uint32_t *devLens,
                 uint32_t lenAdd, uint32_t chunkTokens, uint8_t *q81, bool pdl, cudaStream_t st,
                 uint32_t chunksPerRank, uint64_t rankStride, QRotation rot) {
     if (chunksPerRank == 0) chunksPerRank = numChunks;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(nHeads, seqLen);
-    cfg.blockDim = dim3(256);
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    // The sliced form (a block per head and 32-dim slice) is the faster merge in plain stream order.
-    // Under programmatic dependent launch its blocks are resident next to the decode blocks they wait
-    // for: with one sequence that still wins (7B shape, 32768 rows: 11.7 us per layer against 12.5 with
-    // a block per head; 131072 rows of the 32B shape 48.1 against 49.2), with a batch of sequences the
-    // 4x as many blocks get in the way (batch 8: 49.4 against 46.1 us; 64 ragged sequences 201 against
-    // 190), so a batch keeps the block-per-head form there.
-    if (q81 == nullptr && (!pdl || static_cast<uint64_t>(nHeads) * seqLen <= 64u)) {
-        // one sequence: 16-dim slices, twice the blocks (7B shape at 32768 rows: 11.36 us per layer
-        // against 11.67 with 32-dim slices, 11.38 with 8-dim, 12.17 with 4-dim ones)
-        if (static_cast<uint64_t>(nHeads) * seqLen <= 64u) {
-            cfg.gridDim = dim3(nHeads, seqLen, hd / 16u);
-            TC_CUDA_OK(cudaLaunchKernelEx(&cfg, mergeSliceKernel<4, 256>, pAcc, pM, pL, out, nHeads, numChunks, activeHost, hd,
-                                          devLens, lenAdd, chunkTokens, chunksPerRank, rankStride, rot));
-            return TC_OK;
-        }
-        cfg.gridDim = dim3(nHeads, seqLen, hd / 32u);
-        TC_CUDA_OK(cudaLaunchKernelEx(&cfg, mergeSliceKernel<8, 256>, pAcc, pM, pL, out, nHeads, numChunks, activeHost, hd,
-                                      devLens, lenAdd, chunkTokens, chunksPerRank, rankStride, rot));
-        return TC_OK;
+    const uint64_t units = static_cast<uint64_t>(nHeads) * seqLen;
+    const uint32_t early = pdl ? 1u : 0u;
+    // (under dependent launch the blocks of a merge are resident next to the blocks they wait for: few and small)
+    if (q81 == nullptr && units <= 64u) {
+        // one sequence: 16-dim slices (7B shape at 32768 rows: 11.36 us per layer against 11.67 with 32-dim slices, 11.38
+        // with 8-dim, 12.17 with 4-dim ones, 12.5 with a block per head)
+        return launchDependent(mergeSliceKernel<4, 256>, dim3(nHeads, seqLen, hd / 16u), 256, 0, st, 1, pAcc, pM, pL, out,
+                               nHeads, numChunks, activeHost, hd, devLens, lenAdd, chunkTokens, chunksPerRank, rankStride, rot,
+                               early);
     }
-    if (hd <= 128)
-        TC_CUDA_OK(cudaLaunchKernelEx(&cfg, mergePartialsKernel<1>, pAcc, pM, pL, out, nHeads, numChunks,
-                                      activeHost, hd, devLens, lenAdd, chunkTokens, q81, chunksPerRank, rankStride, rot));
-    else
-        TC_CUDA_OK(cudaLaunchKernelEx(&cfg, mergePartialsKernel<2>, pAcc, pM, pL, out, nHeads, numChunks,
-                                      activeHost, hd, devLens, lenAdd, chunkTokens, q81, chunksPerRank, rankStride, rot));
-    return TC_OK;
+    if (q81 == nullptr && rankStride == 0 && rot.q == nullptr && chunkTokens != 0) {
+        // a batch: a warp per (token, head) up to 8 chunks, four from there on
+        const bool wide = activeHost > 8u;
+        const uint32_t blocks = static_cast<uint32_t>(wide ? units : (units + 3) / 4), u32 = static_cast<uint32_t>(units);
+        auto kern = hd <= 128 ? (wide ? mergeWarpKernel<1, 4> : mergeWarpKernel<1, 1>)
+                              : (wide ? mergeWarpKernel<2, 4> : mergeWarpKernel<2, 1>);
+        return launchDependent(kern, dim3(blocks), 128, 0, st, 1, pAcc, pM, pL, out, u32, nHeads, numChunks, activeHost, hd,
+                               devLens, lenAdd, chunkTokens, early);
+    }
+    return launchDependent(hd <= 128 ? mergePartialsKernel<1> : mergePartialsKernel<2>, dim3(nHeads, seqLen), 256, 0, st, 1,
+                           pAcc, pM, pL, out, nHeads, numChunks, activeHost, hd, devLens, lenAdd, chunkTokens, q81,
+                           chunksPerRank, rankStride, rot, early);
 }
 
 }  // namespace tc
