@@ -217,7 +217,9 @@ mergePartialsKernel(const float *__restrict__ pAcc, const float *__restrict__ pM
 // t % SL4 of the slice and the chunks t / SL4, t / SL4 + CL, ...; (m, l) and the weights are recomputed
 // by every slice's block -- a few hundred bytes.  No Q8_1 epilogue here (that needs the whole head).
 // SL4 = float4 per slice (8: 32-dim slices, 4: 16-dim slices); 256 / SL4 chunk lanes.
-template <int SL4, int T>
+// TOKEN: the merge behind an f32 / fp16 decode launch, which may have q to rotate and a length to share out; a form of its
+// own because the mere presence of that code cost the others 0.3 us.
+template <int SL4, int T, bool TOKEN>
 __global__ void __launch_bounds__(T)
 mergeSliceKernel(const float *__restrict__ pAcc, const float *__restrict__ pM, const float *__restrict__ pL,
                  float *__restrict__ out, uint32_t nHeads, uint32_t numChunks, uint32_t activeHost, uint32_t hd,
@@ -245,7 +247,7 @@ mergeSliceKernel(const float *__restrict__ pAcc, const float *__restrict__ pM, c
     uint32_t active = activeHost < numChunks ? activeHost : numChunks;
     if (devLens != nullptr) {
         uint32_t len = devLens[s] + lenAdd, per = chunkTokens;
-        if (per == 0) len = min(len, rot.maxLen), per = tokensPerBlock(len, activeHost);
+        if (TOKEN && per == 0) len = min(len, rot.maxLen), per = tokensPerBlock(len, activeHost);
         const uint32_t need = (len + per - 1) / per;
         // never past the slots the launch that wrote the partials covered (activeHost): a device
         // length beyond the host bound the plan was built from must not pull in stale slots
@@ -342,7 +344,7 @@ mergeSliceKernel(const float *__restrict__ pAcc, const float *__restrict__ pM, c
             }
         }
     }  // more than 64 chunks
-    if (rot.q != nullptr && slice == gridDim.z - 1) rotateHead(rot, head, hd, devLens, lenAdd, 0, 1);
+    if (TOKEN && rot.q != nullptr && slice == gridDim.z - 1) rotateHead(rot, head, hd, devLens, lenAdd, 0, 1);
     // a warp holds 32 / SL4 chunk lanes x SL4 float4: fold the chunk lanes, then the warps
 #pragma unroll
     for (int o = SL4; o <= 16; o <<= 1) {
@@ -372,7 +374,7 @@ mergeSliceKernel(const float *__restrict__ pAcc, const float *__restrict__ pM, c
 // The merge of a batch: W warps of a 128-thread block per (token, head), each taking every W-th chunk; lane c of a warp
 // holds (m, l) of chunk c of a group of 32, a lane owns four dims (and 128 further on at head_dim 256).  With some thousand
 // (token, head) pairs of a few chunks each it is the number of blocks that costs: 64 sequences x 28 heads took 17 us
-// behind their decode launch with a 256-thread block per pair, NEWMERGE with a warp.
+// behind their decode launch with a 256-thread block per pair, a few with a warp (205 -> 190 us for the layer).
 template <int NV4, int W>
 __global__ void __launch_bounds__(128)
 mergeWarpKernel(const float *__restrict__ pAcc, const float *__restrict__ pM, const float *__restrict__ pL,
@@ -481,7 +483,8 @@ int launchMerge(const float *pAcc, const float *pM, const float *pL, float *out,
     if (q81 == nullptr && units <= 64u) {
         // one sequence: 16-dim slices (7B shape at 32768 rows: 11.36 us per layer against 11.67 with 32-dim slices, 11.38
         // with 8-dim, 12.17 with 4-dim ones, 12.5 with a block per head)
-        return launchDependent(mergeSliceKernel<4, 256>, dim3(nHeads, seqLen, hd / 16u), 256, 0, st, 1, pAcc, pM, pL, out,
+        const bool token = rot.q != nullptr || chunkTokens == 0;
+        return launchDependent(token ? mergeSliceKernel<4, 256, true> : mergeSliceKernel<4, 256, false>, dim3(nHeads, seqLen, hd / 16u), 256, 0, st, 1, pAcc, pM, pL, out,
                                nHeads, numChunks, activeHost, hd, devLens, lenAdd, chunkTokens, chunksPerRank, rankStride, rot,
                                early);
     }
