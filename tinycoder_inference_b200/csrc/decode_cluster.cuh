@@ -17,10 +17,6 @@
 
 #include <cstring>
 #include <mutex>
-#ifdef TC_TUNE
-#include <cstdio>
-#include <cstdlib>
-#endif
 
 #include "decode_shared.cuh"
 
@@ -106,14 +102,6 @@ inline ClusterPlan searchClusterPlan(uint32_t nKV, uint32_t maxLen, uint32_t slo
         if ((tiles + perBlock - 1) / perBlock != n) continue;  // the last blocks would have no rows
         consider(1, n, workUs(perBlock, n * nKV, 1) + 1.7f + (n > 32 ? 0.035f * (n - 32) : 0.0f));
     }
-#ifdef TC_TUNE
-    if (const char *e = getenv("TC_PLAN")) {
-        unsigned C = 1, n = 1;
-        sscanf(e, "%u,%u", &C, &n);
-        const uint32_t perBlock = (tiles + n * C - 1) / (n * C);
-        best.cluster = C, best.clusters = (tiles + perBlock * C - 1) / (perBlock * C), best.chunkTokens = perBlock * 16;
-    }
-#endif
     return best;
 }
 
@@ -274,14 +262,14 @@ __device__ __forceinline__ void foldStore(const FoldTarget &f, uint32_t j, uint3
     }
 }
 
-// Every consumer warp has left [8 columns][HD] accumulators, m[8] (log2 units) and l[8] in its part of
+// Every warp has left [8 columns][HD] accumulators, m[8] (log2 units) and l[8] in its part of
 // scr ([NW][8 HD + 16]).  Called by all NW * 32 threads of the block (tid) with the warps' parts complete.
-template <int HD, int NW>
+template <int HD, int NW, int THREADS = NW * 32>
 __device__ __forceinline__ void clusterFold(float *scr, const FoldTarget &f, uint32_t tid) {
     constexpr uint32_t kWarpScr = 8 * HD + 16, V4 = HD / 4;
     const uint32_t n = clusterSize(), rank = clusterRank();
     float *part = scr + NW * kWarpScr;  // this block's partial: [8][HD], m[8], l[8]
-    for (uint32_t idx = tid; idx < f.nValid * V4; idx += NW * 32) {
+    for (uint32_t idx = tid; idx < f.nValid * V4; idx += THREADS) {
         const uint32_t d4 = idx % V4, j = idx / V4;
         float M = kNegBig;
 #pragma unroll
@@ -312,13 +300,13 @@ __device__ __forceinline__ void clusterFold(float *scr, const FoldTarget &f, uin
     if (n > 1) clusterSync();
     // (in a cluster of one block the caller's barrier has every warp's q in registers)
     if (f.qRot != nullptr)
-        rotateQ<HD>(f.qRot, f.cosT, f.sinT, f.tableRow, f.nValid, rank * NW * 32 + tid, n * NW * 32);
+        rotateQ<HD>(f.qRot, f.cosT, f.sinT, f.tableRow, f.nValid, rank * THREADS + tid, n * THREADS);
     if (n == 1) return;
     // the blocks of the cluster share the output: rank r takes the r-th slice of its float4s.  Everything a
     // thread needs from the other blocks is requested before anything is consumed.
     const uint32_t total = f.nValid * V4, per = (total + n - 1) / n;
     const uint32_t end = min(total, (rank + 1) * per), base = smemAddr(part);
-    for (uint32_t idx = rank * per + tid; idx < end; idx += NW * 32) {
+    for (uint32_t idx = rank * per + tid; idx < end; idx += THREADS) {
         const uint32_t d4 = idx % V4, j = idx / V4;
         float m[16], ls[16];
         float4 a[16];

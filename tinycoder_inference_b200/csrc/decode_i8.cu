@@ -22,34 +22,9 @@
 //     layout through movmatrix.trans.
 #include <mutex>
 
-#include "decode_cluster.cuh"
+#include "decode_i8.cuh"
 
 namespace tc {
-
-struct DecodeI8Params {
-    const float *q;
-    float *out;
-    const float *ks, *vs;
-    float *pAcc, *pM, *pL;
-    const uint32_t *devLens;     // nullable
-    const uint64_t *devRowBase;  // nullable
-    uint64_t rowsPerSeq, totalRows;
-    uint32_t lenHost, lenAdd;
-    uint32_t nHeads, nKV, group;
-    uint32_t colBase;  // decode: the 8 MMA columns are q heads colBase .. colBase + 7 of the kv head
-    uint32_t chunkTokens, numChunks;
-    const float *appendK, *appendV;  // nullable: [batch][nKV][hd] rows to quantise into row len - 1 first
-    uint32_t *k8w, *v8w;             // the pools
-    F32Mirror mir;                   // and the f32 store that gets it verbatim
-    // rows mode (causal prefill over the store): the 8 MMA columns of a CTA are 8
-    // consecutive query rows of ONE q head instead of the q heads of one kv head;
-    // row s attends pool rows [0, cachePos + s].  grid = (1, nHeads, ceil(qRows / 8)).
-    uint32_t qRows, cachePos;
-    const uint32_t *devPos;
-    float invSqrt;
-    int directOut;
-    unsigned int *err;
-};
 
 constexpr int kHD = 128;
 
@@ -69,24 +44,15 @@ struct DecodeI8Smem {
     static_assert(kTotal <= 227 * 1024, "shared memory of an SM");
 };
 
-// How far the running reference point of the softmax may lag behind the true
-// maximum (log2 units) before the accumulators are rescaled.  p stays <= 2^8.
-constexpr float kLazyLog2 = 8.0f;
-
-// What a launch does: a token's q heads over chunks of the store; causal query rows; or a token's q heads with the
-// accumulation order of the causal form -- tile j of the store belongs to stream j % 8, a stream's tiles are folded one
-// after the other -- each stream a block (one warp) of an 8-block cluster per kv head.
-enum class I8Mode { kChunks, kRows, kStreams };
-
-template <int HD, int NW, int NS, int MT, I8Mode MODE>
-__global__ void __launch_bounds__(NW * 32, MODE == I8Mode::kChunks && NW <= 4 ? 2 : 1)
+// ROWS: causal query rows; otherwise a token's q heads over chunks of the store.
+template <int HD, int NW, int NS, int MT, bool ROWS>
+__global__ void __launch_bounds__(NW * 32, !ROWS && NW <= 4 ? 2 : 1)
 decodeI8Kernel(const __grid_constant__ DecodeI8Params p) {
     using L = DecodeI8Smem<HD, NW, NS, MT>;
-    constexpr bool ROWS = MODE == I8Mode::kRows, STREAMS = MODE == I8Mode::kStreams;
     constexpr int T = L::T;
     constexpr int NC = HD / 16;  // 16-dim groups of a head vector
     constexpr int NR = 2 * MT;  // 8-token row groups of a warp's tile
-    constexpr float k2p24 = 16777216.0f;
+    constexpr float k2p24 = kI8Unscale;
 
     const uint32_t chunk = blockIdx.x, hg = blockIdx.y, b = blockIdx.z;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
@@ -105,18 +71,16 @@ decodeI8Kernel(const __grid_constant__ DecodeI8Params p) {
         // (the host's length is the upper bound of a device length)
         len = p.devLens ? min(p.devLens[b] + p.lenAdd, p.lenHost) : p.lenHost;
         // a cluster behind the last row leaves as a whole: the merge derives the active count from len
-        if (!STREAMS && (chunk - clusterRank()) * p.chunkTokens >= len) return;
+        if ((chunk - clusterRank()) * p.chunkTokens >= len) return;
     }
-    const uint32_t t0 = MODE != I8Mode::kChunks ? 0u : chunk * p.chunkTokens;
-    const uint32_t t1 = MODE != I8Mode::kChunks ? len : min(len, t0 + p.chunkTokens);
+    const uint32_t t0 = ROWS ? 0u : chunk * p.chunkTokens;
+    const uint32_t t1 = ROWS ? len : min(len, t0 + p.chunkTokens);
     const uint32_t nTiles = t0 < t1 ? (t1 - t0 + T - 1) / T : 0u;
     const uint64_t rowBase = ROWS ? 0ull : (p.devRowBase ? p.devRowBase[b] : static_cast<uint64_t>(b) * p.rowsPerSeq);
     const uint32_t kvHead = ROWS ? hg / p.group : hg;
 
-    // Tile j belongs to warp (or stream) j % step, its slot (j / step) % NS.  A warp copies its own tiles: with one slot the next
+    // Tile j belongs to warp j % NW, its slot (j / NW) % NS.  A warp copies its own tiles: with one slot the next
     // tile's K while it works on this one's V and the next V while it works on K.
-    const uint32_t first = STREAMS ? clusterRank() : warp;
-    constexpr uint32_t step = STREAMS ? 8 : NW;
     auto slotK = [&](uint32_t i) { return smem + (warp * NS + i % NS) * 2 * L::kTileBytes; };
     auto scaleK = [&](uint32_t i) { return reinterpret_cast<float *>(smem + L::kScales) + (warp * NS + i % NS) * 2 * T; };
     const uint32_t stride = p.nKV * HD;
@@ -126,7 +90,7 @@ decodeI8Kernel(const __grid_constant__ DecodeI8Params p) {
         if (lane < T) cpAsync4(dst + lane, src + min(row + lane, p.totalRows - 1) * p.nKV + kvHead);
     };
     auto requestK = [&](uint32_t i) {
-        const uint32_t j = first + i * step;
+        const uint32_t j = warp + i * NW;
         if (j < nTiles) {
             if (!ROWS && p.appendK != nullptr && j + 1 == nTiles && t1 == len) {
                 // the tile that holds the new token's row: the row goes in first
@@ -151,7 +115,7 @@ decodeI8Kernel(const __grid_constant__ DecodeI8Params p) {
         cpAsyncCommit();
     };
     auto requestV = [&](uint32_t i) {
-        const uint32_t j = first + i * step;
+        const uint32_t j = warp + i * NW;
         if (j < nTiles) {
             const uint64_t row = rowBase + t0 + j * T;
             copyTile<T, HD>(smemAddr(slotK(i) + L::kTileBytes), storeV, stride, row, p.totalRows - 1, lane);
@@ -175,54 +139,8 @@ decodeI8Kernel(const __grid_constant__ DecodeI8Params p) {
     // exclusive row bound of a column: everything in decode, causal in rows mode
     auto colLen = [&](uint32_t j) { return ROWS ? min(t1, rowsPos + b * 8u + j + 1u) : t1; };
 
-    // q fragments for head column n = g of this kv head's group: power-of-two
-    // normalised, split into fp16 hi + lo, laid out as the B operand whose k
-    // slots follow the byte order ldmatrix hands out (dims 16c + 4t + {0..3}).
-    uint32_t qhi[NC][2], qlo[NC][2];
-    float headScale, headOff;
-    {
-        float4 qv[NC];
-        float amax = 0.0f;
-        const bool valid = colValid(g);
-        const float *qp = p.q + colIndex(valid ? g : 0) * HD;
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-            qv[c] = valid ? __ldg(reinterpret_cast<const float4 *>(qp + 16 * c + 4 * t))
-                          : make_float4(0.f, 0.f, 0.f, 0.f);
-            amax = fmaxf(amax, fmaxf(fmaxf(fabsf(qv[c].x), fabsf(qv[c].y)), fmaxf(fabsf(qv[c].z), fabsf(qv[c].w))));
-        }
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-        int e = static_cast<int>((__float_as_uint(amax) >> 23) & 0xffu) - 127;  // floor(log2 amax)
-        e = amax > 0.0f ? max(-100, min(100, e)) : 0;
-        const float down = __uint_as_float(static_cast<uint32_t>(127 - e) << 23);  // 2^-e
-        const float up = __uint_as_float(static_cast<uint32_t>(127 + e) << 23);    // 2^e
-        headScale = p.invSqrt * up * kLog2e;
-        float qsum = 0.0f;
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-            float h0, l0, h1, l1, h2, l2, h3, l3;
-            splitHalf(qv[c].x * down, h0, l0);
-            splitHalf(qv[c].y * down, h1, l1);
-            splitHalf(qv[c].z * down, h2, l2);
-            splitHalf(qv[c].w * down, h3, l3);
-            qhi[c][0] = packHalf2(h0, h1);
-            qhi[c][1] = packHalf2(h2, h3);
-            qlo[c][0] = packHalf2(l0, l1);
-            qlo[c][1] = packHalf2(l2, l3);
-            // the column sum the MMA really sees: the fp16-rounded parts
-            const __half2 a = *reinterpret_cast<__half2 *>(&qlo[c][0]), bb = *reinterpret_cast<__half2 *>(&qlo[c][1]);
-            qsum += (h0 + __low2float(a)) + (h1 + __high2float(a)) + (h2 + __low2float(bb)) + (h3 + __high2float(bb));
-        }
-        qsum += __shfl_xor_sync(0xffffffffu, qsum, 1);
-        qsum += __shfl_xor_sync(0xffffffffu, qsum, 2);
-        headOff = 128.0f * qsum;  // K bytes enter the MMA as x + 128
-    }
-    // score columns of this thread are heads 2t and 2t+1: fetch their constants
-    const float cs0 = __shfl_sync(0xffffffffu, headScale, (2 * t) * 4);
-    const float cs1 = __shfl_sync(0xffffffffu, headScale, (2 * t + 1) * 4);
-    const float off0 = __shfl_sync(0xffffffffu, headOff, (2 * t) * 4);
-    const float off1 = __shfl_sync(0xffffffffu, headOff, (2 * t + 1) * 4);
+    I8Query<HD> qf;
+    i8LoadQuery<HD>(qf, p.q + colIndex(colValid(g) ? g : 0) * HD, colValid(g), p.invSqrt, lane);
     const uint32_t len0 = colLen(2 * t), len1 = colLen(2 * t + 1);
 
     float m0 = kNegBig, m1 = kNegBig, l0 = 0.0f, l1 = 0.0f;
@@ -237,65 +155,12 @@ decodeI8Kernel(const __grid_constant__ DecodeI8Params p) {
     const uint32_t lco = lane >> 4;                             // and which chunk of the pair
     const uint32_t lmOff = lr * 128;
 
-    for (uint32_t i = 0, tile = first; tile < nTiles; ++i, tile += step) {
+    for (uint32_t i = 0, tile = warp; tile < nTiles; ++i, tile += NW) {
         cpAsyncWait<2 * NS - 1>();  // K of this tile is in, what was requested behind it may still be on its way
         const float *sK = scaleK(i), *sV = sK + T;
         const uint32_t tokBase = t0 + tile * T + g;
-        bool vl0[NR], vl1[NR];
-        float skr[NR], svr[NR];
-#pragma unroll
-        for (int r = 0; r < NR; ++r) {  // rows g, g+8, ... of this warp's tokens
-            vl0[r] = tokBase + 8 * r < len0;
-            vl1[r] = tokBase + 8 * r < len1;
-            skr[r] = sK[g + 8 * r];
-        }
-
-        // ---- S^T = K . Q^T, two 16-token tiles x 8 heads ----
-        float sh[MT][4], sl[MT][4];
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) sh[mt][i] = sl[mt][i] = 0.0f;
-        const uint32_t kTile = smemAddr(slotK(i));
-#pragma unroll
-        for (int cp = 0; cp < NC / 2; ++cp) {
-            const uint32_t sw = (((2 * (cp & 3) + lco) ^ (lr & 7u)) << 4) + (cp >> 2) * L::kHalfBytes;
-#pragma unroll
-            for (int mt = 0; mt < MT; ++mt) {
-                uint32_t r0, r1, r2, r3;
-                ldmatrixX4(r0, r1, r2, r3, kTile + mt * 2048 + lmOff + sw);
-                r0 ^= 0x80808080u;
-                r1 ^= 0x80808080u;
-                r2 ^= 0x80808080u;
-                r3 ^= 0x80808080u;
-                {
-                    const uint32_t a0 = subnormalPair<0x4140>(r0), a1 = subnormalPair<0x4140>(r1),
-                                   a2 = subnormalPair<0x4342>(r0), a3 = subnormalPair<0x4342>(r1);
-                    mmaF16(sh[mt], a0, a1, a2, a3, qhi[2 * cp][0], qhi[2 * cp][1]);
-                    mmaF16(sl[mt], a0, a1, a2, a3, qlo[2 * cp][0], qlo[2 * cp][1]);
-                }
-                {
-                    const uint32_t a0 = subnormalPair<0x4140>(r2), a1 = subnormalPair<0x4140>(r3),
-                                   a2 = subnormalPair<0x4342>(r2), a3 = subnormalPair<0x4342>(r3);
-                    mmaF16(sh[mt], a0, a1, a2, a3, qhi[2 * cp + 1][0], qhi[2 * cp + 1][1]);
-                    mmaF16(sl[mt], a0, a1, a2, a3, qlo[2 * cp + 1][0], qlo[2 * cp + 1][1]);
-                }
-            }
-        }
-        // log2-domain scores: undo the 2^-24 of the subnormal operand and the +128 offset,
-        // apply the row's K scale; rows past the range are masked out
-        float sc[NR][2];  // [row r][head 2t / 2t+1]
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt) {
-#pragma unroll
-            for (int hf = 0; hf < 2; ++hf) {
-                const int r = 2 * mt + hf;
-                const float d0 = fmaf(sh[mt][2 * hf] + sl[mt][2 * hf], k2p24, -off0);
-                const float d1 = fmaf(sh[mt][2 * hf + 1] + sl[mt][2 * hf + 1], k2p24, -off1);
-                sc[r][0] = vl0[r] ? d0 * (skr[r] * cs0) : -INFINITY;
-                sc[r][1] = vl1[r] ? d1 * (skr[r] * cs1) : -INFINITY;
-            }
-        }
+        float svr[NR], sc[NR][2];
+        i8Scores<HD, MT>(qf, smemAddr(slotK(i)), sK, tokBase, len0, len1, lane, sc);
         float mx0 = fmaxf(sc[0][0], sc[1][0]), mx1 = fmaxf(sc[0][1], sc[1][1]);
         __syncwarp();  // every lane has read its part of K
         requestK(i + NS);
@@ -481,13 +346,6 @@ static ClusterPlan decodeI8Plan(const tc_decode_i8_batch *d, const uint32_t *max
             best.cluster = 1u << lg, best.clusters = 1;
             break;
         }
-#ifdef TC_TUNE
-    if (const char *e = getenv("TC_PLAN")) {
-        unsigned C = 1, n = 1;
-        sscanf(e, "%u,%u", &C, &n);
-        best.cluster = C, best.clusters = (dp.chunksPerSeq + C - 1) / C;
-    }
-#endif
     return best;
 }
 
@@ -495,7 +353,7 @@ template <int NW>
 static int decodeI8Hd256(const tc_decode_i8_batch *d, DecodeI8Params prm, cudaStream_t st) {
     constexpr int HD = 256;
     using L = DecodeI8Smem<HD, NW, 1, 1>;
-    auto kern = decodeI8Kernel<HD, NW, 1, 1, I8Mode::kChunks>;
+    auto kern = decodeI8Kernel<HD, NW, 1, 1, false>;
     static ClusterSetup setup;
     const uint32_t *limits = nullptr;
     int rc = setupCluster(setup, kern, NW * 32, L::kTotal, &limits);
@@ -553,27 +411,6 @@ static int i8Params(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenA
     return TC_OK;
 }
 
-// One sequence, any length up to lenHost rows, no partial buffers: what a captured decode step of the int8 store takes.
-// The causal kernel (a block per q head, 8 warps of which 7 / 8 of the MMA columns were padding) took 27.5 us for
-// 5000 rows of 28 q / 4 kv heads of 128; this form, with the same roundings, 26.
-template <int HD, int MT>
-static int launchStreamsI8(DecodeI8Params prm, cudaStream_t st) {
-    constexpr int NS = 4;
-    using L = DecodeI8Smem<HD, 1, NS, MT>;
-    auto kern = decodeI8Kernel<HD, 1, NS, MT, I8Mode::kStreams>;
-    static ClusterSetup setup;
-    const uint32_t *limits = nullptr;
-    int rc = setupCluster(setup, kern, 32, L::kTotal, &limits);
-    if (rc != TC_OK) return rc;
-    prm.directOut = 1;
-    for (uint32_t cb = 0; cb < prm.group; cb += 8) {
-        prm.colBase = cb;
-        if (cb) prm.appendK = prm.appendV = nullptr;  // the row is in
-        rc = launchDependent(kern, dim3(8, prm.nKV, 1), 32, L::kTotal, st, 8, prm);
-        if (rc != TC_OK) return rc;
-    }
-    return TC_OK;
-}
 int decodeI8Streams(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, cudaStream_t st) {
     TC_REQUIRE(d->hd == 128 || d->hd == 256, TC_EUNSUPPORTED, "decode_i8: head_dim %u (built for 128 and 256)", d->hd);
     TC_REQUIRE(d->nHeads / d->nKV <= 64, TC_EUNSUPPORTED, "decode_i8: %u q heads per kv head (built for <= 64)",
@@ -585,7 +422,8 @@ int decodeI8Streams(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenA
     DecodeI8Params prm;
     const int rc = i8Params(d, lenHost, lenAdd, F32Mirror{nullptr, nullptr}, &prm);
     if (rc != TC_OK) return rc;
-    return d->hd == 256 ? launchStreamsI8<256, 1>(prm, st) : launchStreamsI8<128, 2>(prm, st);
+    prm.directOut = 1;
+    return launchStreamsI8(prm, d->hd, st);
 }
 
 int decodeI8Common(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, const F32Mirror &mir, cudaStream_t st) {
@@ -621,7 +459,7 @@ template <int HD, int MT>
 static int launchRowsI8(const DecodeI8Params &prm, cudaStream_t st) {
     constexpr int NW = 8, NS = 3;
     using L = DecodeI8Smem<HD, NW, NS, MT>;
-    auto kern = decodeI8Kernel<HD, NW, NS, MT, I8Mode::kRows>;
+    auto kern = decodeI8Kernel<HD, NW, NS, MT, true>;
     static bool attrDone[64] = {false};
     int dev = 0;
     cudaGetDevice(&dev);

@@ -1,0 +1,355 @@
+// decode_i8_streams.cu -- one query token over the int8 store, any length up to the launch's bound, no partial buffers:
+// what a captured decode step of the int8 store replays.
+//
+// What it replaces: kQ35WarpAttention8Prefill / kQ35PrefillAttnSharedKV8 with one query row (include/gpu/
+// GpuQwen35Kernels.hpp:2306-2435), the reference's graph-safe form of the int8 decode.
+//
+// The roundings of the result are those of the causal kernel (decode_i8.cu): its V bytes enter the products with an offset
+// of 128 that is taken out at the end, so the running sums are large next to the result and the order in which tiles are
+// accumulated shows.  That order is eight streams -- tile j (16 MT tokens) belongs to stream j % 8, a stream's tiles are
+// folded one after the other -- and it is kept: a block is a stream, an 8-block cluster a kv head.  Inside a stream only
+// three things depend on the tile before: the reference point of the maximum, the scale of the V factors, and the
+// accumulators, each dimension on its own.  So
+//   * eight score warps take tiles in turn: scores (K product), then -- once the warps of a round have told each other
+//     their tiles' maxima and each has walked through them in tile order -- probabilities as MMA operands;
+//   * four value warps own HD / 4 dimensions each and walk through all tiles of the stream: rescale, four to eight products;
+//   * a sum warp walks along with the row sums.
+// A tile costs the walk some 150 cycles where one warp doing all of it took 2500: 5000 rows of 28 q / 4 kv heads of 128
+// (157 tiles of 32 tokens, 20 per stream) take 13.8 us, 26 with a warp per stream, 27.5 with a block per q head.
+#include "decode_i8.cuh"
+
+namespace tc {
+
+template <int HD, int MT>
+struct I8StreamSmem {
+    static constexpr int T = 16 * MT, NR = 2 * MT;
+    static constexpr int kScoreWarps = 8, kValueWarps = 4, kWarps = kScoreWarps + kValueWarps + 1;
+    static constexpr int kSlots = 2 * kScoreWarps;                 // V tiles and probability records in flight
+    static constexpr int kHalfBytes = T * 128;                     // half-tile of 128 dims
+    static constexpr int kTileBytes = T * HD;
+    static constexpr int kRecord = 1536 * MT + 128;                // P operands, P and P x scale per row, factors
+    static constexpr int kK = 0;                                   // [score warp][2] K tiles
+    static constexpr int kV = kK + kScoreWarps * 2 * kTileBytes;   // [slot] V tiles
+    static constexpr int kRec = kV + kSlots * kTileBytes;          // [slot]
+    static constexpr int kScales = kRec + kSlots * kRecord;        // [score warp][2][K, V][T]
+    static constexpr int kMax = kScales + kScoreWarps * 4 * T * 4; // [2][score warp][12]: column maxima, V scale bits
+    static constexpr int kEnd = kMax + 2 * kScoreWarps * 12 * 4;   // m[8], E, then l[8], sums of P x scale [8]
+    static constexpr int kBars = kEnd + 32 * 4;                    // full, empty per slot
+    static constexpr int kTotal = kBars + 2 * kSlots * 8 + 128;
+    static_assert(2 * (8 * HD + 16) * 4 <= kV, "the fold reuses the K tiles");
+    static_assert(kTotal <= 227 * 1024, "shared memory of an SM");
+};
+
+template <int HD, int MT>
+__global__ void __launch_bounds__(I8StreamSmem<HD, MT>::kWarps * 32, 1)
+decodeI8StreamsKernel(const __grid_constant__ DecodeI8Params p) {
+    using L = I8StreamSmem<HD, MT>;
+    constexpr int T = L::T, NR = L::NR;
+    constexpr uint32_t SW = L::kScoreWarps, VW = L::kValueWarps, NSLOT = L::kSlots, kThreads = L::kWarps * 32;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, g = lane >> 2, t = lane & 3u;
+    const uint32_t stream = clusterRank(), kvHead = blockIdx.y;
+
+    extern __shared__ uint8_t smemRaw[];
+    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smemRaw) + 127) & ~uintptr_t(127));
+    uint64_t *fullBar = reinterpret_cast<uint64_t *>(smem + L::kBars), *emptyBar = fullBar + NSLOT;
+    float *sEnd = reinterpret_cast<float *>(smem + L::kEnd);
+    if (threadIdx.x == 0) {
+        for (uint32_t s = 0; s < NSLOT; ++s) {
+            mbarInit(&fullBar[s], 32);
+            mbarInit(&emptyBar[s], VW + 1);
+        }
+        fenceBarrierInit();
+    }
+    __syncthreads();
+    gridDepWait();
+    gridDepLaunch();
+
+    const uint32_t want = p.devLens ? p.devLens[0] + p.lenAdd : p.lenHost;
+    const uint32_t len = min(want, p.lenHost);  // (the host's length is the upper bound of a device length)
+    const uint32_t nTiles = (len + T - 1) / T;
+    const uint32_t n = nTiles > stream ? (nTiles - stream + 7u) / 8u : 0u;  // tiles of this stream: stream + 8 i
+    const uint32_t head0 = kvHead * p.group + p.colBase, nValid = min(8u, p.group - p.colBase);
+    // record of a slot: P operands [MT][32 lanes] uint4, P [2 NR][32], P x scale [2 NR][32], then al[8], as[8], flag
+    auto record = [&](uint32_t i) { return smem + L::kRec + (i % NSLOT) * L::kRecord; };
+    constexpr uint32_t kRecP = 512 * MT, kRecX = 1024 * MT, kRecF = 1536 * MT;
+
+    const uint32_t lr = (lane & 7u) + ((lane >> 3) & 1u) * 8u, lco = lane >> 4;  // ldmatrix row and chunk of this lane
+    constexpr int CP = HD / 128;  // 32-dim groups of a value warp
+    float o[2 * CP][4];           // its accumulators, by 16-dim group
+#pragma unroll
+    for (int c = 0; c < 2 * CP; ++c) o[c][0] = o[c][1] = o[c][2] = o[c][3] = 0.0f;
+
+    if (warp < SW) {
+        // ---------------------------------- scores and probabilities ----------------------------------
+        const uint32_t stride = p.nKV * HD;
+        const uint8_t *storeK = reinterpret_cast<const uint8_t *>(p.k8w) + static_cast<size_t>(kvHead) * HD;
+        const uint8_t *storeV = reinterpret_cast<const uint8_t *>(p.v8w) + static_cast<size_t>(kvHead) * HD;
+        auto slotK = [&](uint32_t i) { return smem + L::kK + (warp * 2 + (i / SW) % 2) * L::kTileBytes; };
+        auto scales = [&](uint32_t i) { return reinterpret_cast<float *>(smem + L::kScales) + (warp * 2 + (i / SW) % 2) * 2 * T; };
+        auto copyScales = [&](float *dst, const float *src, uint64_t row) {
+            if (lane < T) cpAsync4(dst + lane, src + min(row + lane, p.totalRows - 1) * p.nKV + kvHead);
+        };
+        auto requestK = [&](uint32_t i) {
+            if (i < n) {
+                const uint32_t j = stream + 8u * i;
+                if (p.appendK != nullptr && j + 1 == nTiles) {
+                    // the tile that holds the new token's row: the row goes in first
+                    const uint64_t row = static_cast<uint64_t>(want) - 1u;
+                    if (row >= p.totalRows) {  // a device position outside the pool: no row written, and said so
+                        if (lane == 0) atomicOr(p.err, kDevErrRowBound);
+                    } else {
+                        const size_t src = static_cast<size_t>(kvHead) * (HD / 4);
+                        appendQuantRow<HD>(reinterpret_cast<const float4 *>(p.appendK) + src,
+                                           reinterpret_cast<const float4 *>(p.appendV) + src, p.k8w, p.v8w,
+                                           const_cast<float *>(p.ks), const_cast<float *>(p.vs), row * p.nKV + kvHead, nullptr,
+                                           nullptr, lane);
+                    }
+                }
+                const uint64_t row = static_cast<uint64_t>(j) * T;
+                copyTile<T, HD>(smemAddr(slotK(i)), storeK, stride, row, p.totalRows - 1, lane);
+                copyScales(scales(i), p.ks, row);
+            }
+            cpAsyncCommit();
+        };
+        bool ok = true;
+        auto requestV = [&](uint32_t i) {
+            if (ok && i < n) {
+                // the slot's tile of a round before has been folded by everybody
+                if (i >= NSLOT) ok = mbarWaitClock(&emptyBar[i % NSLOT], (i / NSLOT - 1u) & 1u, p.err, kDevErrEmptyWait);
+                const uint64_t row = static_cast<uint64_t>(stream + 8u * i) * T;
+                copyTile<T, HD>(smemAddr(smem + L::kV + (i % NSLOT) * L::kTileBytes), storeV, stride, row, p.totalRows - 1, lane);
+                copyScales(scales(i) + T, p.vs, row);
+            }
+            cpAsyncCommit();
+        };
+        requestK(warp);
+        requestV(warp);
+        requestK(warp + SW);
+        I8Query<HD> qf;
+        i8LoadQuery<HD>(qf, p.q + static_cast<size_t>(head0 + (g < nValid ? g : 0u)) * HD, g < nValid, p.invSqrt, lane);
+        float *sMax = reinterpret_cast<float *>(smem + L::kMax);
+        float m0 = kNegBig, m1 = kNegBig;  // at the start of the round
+        uint32_t Ebits = 0;                // running power-of-two scale of the V row scales (0 = unset)
+        for (uint32_t round = 0; round * SW < n; ++round) {
+            const uint32_t i = round * SW + warp;
+            requestV(i + SW);
+            cpAsyncWait<2>();  // K and V of this tile are in
+            const uint32_t tokBase = (stream + 8u * i) * T + g;
+            float sc[NR][2], svr[NR];
+            float mx0 = -INFINITY, mx1 = -INFINITY, svmax = 0.0f;
+            if (i < n) {  // warp-uniform
+                i8Scores<HD, MT>(qf, smemAddr(slotK(i)), scales(i), tokBase, len, len, lane, sc);
+#pragma unroll
+                for (int r = 0; r < NR; ++r) {
+                    svr[r] = tokBase + 8 * r < len ? scales(i)[T + g + 8 * r] : 0.0f;
+                    mx0 = fmaxf(mx0, sc[r][0]);
+                    mx1 = fmaxf(mx1, sc[r][1]);
+                    svmax = fmaxf(svmax, svr[r]);
+                }
+#pragma unroll
+                for (int off = 4; off <= 16; off <<= 1) {
+                    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, off));
+                    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, off));
+                }
+            }
+            const uint32_t ebMine = min(__reduce_max_sync(0xffffffffu, __float_as_uint(svmax)) & 0x7f800000u, 253u << 23);
+            requestK(i + 2 * SW);  // (the shuffles above have every lane through with K)
+            // ---- the round's maxima, in tile order ----
+            float *mine = sMax + ((round & 1u) * SW + warp) * 12u;
+            if (g == 0) *reinterpret_cast<float2 *>(mine + 2 * t) = make_float2(mx0, mx1);
+            if (lane == 0) mine[8] = __uint_as_float(ebMine);
+            namedBarSync(1, SW * 32);
+            float a0 = 1.0f, a1 = 1.0f, fMine = 1.0f, r0 = m0, r1 = m1, invE = 0.0f;
+            bool moved = false;
+#pragma unroll
+            for (uint32_t w = 0; w < SW; ++w) {
+                const float *other = sMax + ((round & 1u) * SW + w) * 12u;
+                const float2 mx = *reinterpret_cast<const float2 *>(other + 2 * t);
+                const uint32_t eb = __float_as_uint(other[8]);
+                // lazy reference point: move it only when the maximum ran ahead by 2^8
+                const float mn0 = mx.x > m0 + kLazyLog2 ? mx.x : m0;
+                const float mn1 = mx.y > m1 + kLazyLog2 ? mx.y : m1;
+                float fE = 1.0f;
+                if (eb > Ebits) {
+                    fE = Ebits ? __uint_as_float(Ebits) * __uint_as_float((254u << 23) - eb) : 1.0f;
+                    Ebits = eb;
+                }
+                if (w == warp) {
+                    a0 = fastExp2(m0 - mn0), a1 = fastExp2(m1 - mn1), fMine = fE;
+                    moved = mn0 != m0 || mn1 != m1 || fE != 1.0f;
+                    r0 = mn0, r1 = mn1;
+                    invE = Ebits ? __uint_as_float((254u << 23) - Ebits) : 0.0f;
+                }
+                m0 = mn0, m1 = mn1;
+            }
+            const bool any = __any_sync(0xffffffffu, moved);
+            if (i >= n) continue;
+            // ---- p, then p * sv scaled into fp16 range, hi + lo, transposed to the B layout ----
+            uint8_t *rec = record(i);
+            float *recP = reinterpret_cast<float *>(rec + kRecP) + lane, *recX = reinterpret_cast<float *>(rec + kRecX) + lane;
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt) {
+                uint32_t bh[2], bl[2];
+#pragma unroll
+                for (int hf = 0; hf < 2; ++hf) {
+                    const int r = 2 * mt + hf;
+                    const float p0 = fastExp2(sc[r][0] - r0), p1 = fastExp2(sc[r][1] - r1);
+                    const float w = svr[r] * invE;
+                    const float x0 = p0 * w, x1 = p1 * w;
+                    const uint32_t hi = packHalf2(x0, x1);
+                    const __half2 hh = *reinterpret_cast<const __half2 *>(&hi);
+                    const float d0 = x0 - __low2float(hh), d1 = x1 - __high2float(hh);
+                    const uint32_t lo = packHalf2(d0, d1);
+                    const __half2 ll = *reinterpret_cast<const __half2 *>(&lo);
+                    recP[(2 * r) * 32] = p0, recP[(2 * r + 1) * 32] = p1;
+                    recX[(2 * r) * 32] = __low2float(hh) + __low2float(ll);
+                    recX[(2 * r + 1) * 32] = __high2float(hh) + __high2float(ll);
+                    bh[hf] = movmatrixTrans(hi);
+                    bl[hf] = movmatrixTrans(lo);
+                }
+                *reinterpret_cast<uint4 *>(rec + (mt * 32 + lane) * 16) = make_uint4(bh[0], bh[1], bl[0], bl[1]);
+            }
+            float *fac = reinterpret_cast<float *>(rec + kRecF);
+            if (g == 0) {
+                *reinterpret_cast<float2 *>(fac + 2 * t) = make_float2(a0 * fMine, a1 * fMine);
+                *reinterpret_cast<float2 *>(fac + 8 + 2 * t) = make_float2(a0, a1);
+            }
+            if (lane == 0) *reinterpret_cast<uint32_t *>(fac + 16) = any ? 1u : 0u;
+            // (a warp whose wait ran out stays with the others' barrier and hands nothing on: their waits end too)
+            if (ok) mbarArrive(&fullBar[i % NSLOT]);
+        }
+        if (warp == 0) {
+            if (g == 0) sEnd[2 * t] = m0, sEnd[2 * t + 1] = m1;
+            if (lane == 0) sEnd[8] = __uint_as_float(Ebits);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    } else if (warp < SW + VW) {
+        // ---------------------------------- accumulators ----------------------------------
+        const uint32_t cp0 = (warp - SW) * CP;  // dims 32 cp0 .. 32 (cp0 + CP) - 1
+        for (uint32_t i = 0; i < n; ++i) {
+            if (!mbarWaitClock(&fullBar[i % NSLOT], (i / NSLOT) & 1u, p.err, kDevErrFullWait)) break;
+            const uint8_t *rec = record(i);
+            const float *fac = reinterpret_cast<const float *>(rec + kRecF);
+            uint4 b[MT];
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt) b[mt] = *reinterpret_cast<const uint4 *>(rec + (mt * 32 + lane) * 16);
+            uint32_t v[CP][MT][4];
+            const uint32_t vTile = smemAddr(smem + L::kV + (i % NSLOT) * L::kTileBytes) + lr * 128;
+#pragma unroll
+            for (int c = 0; c < CP; ++c) {
+                const uint32_t cp = cp0 + c;
+                const uint32_t sw = (((2 * (cp & 3u) + lco) ^ (lr & 7u)) << 4) + (cp >> 2) * L::kHalfBytes;
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt)
+                    ldmatrixX4Trans(v[c][mt][0], v[c][mt][1], v[c][mt][2], v[c][mt][3], vTile + mt * 2048 + sw);
+            }
+            if (*reinterpret_cast<const uint32_t *>(fac + 16) != 0u) {
+                const float2 al = *reinterpret_cast<const float2 *>(fac + 2 * t);
+#pragma unroll
+                for (int c = 0; c < 2 * CP; ++c) o[c][0] *= al.x, o[c][1] *= al.y, o[c][2] *= al.x, o[c][3] *= al.y;
+            }
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt) {
+                // rows g / g + 8 of an MMA tile are dims 16 c + 2 g / 16 c + 2 g + 1
+                uint32_t x[2 * CP][4];
+#pragma unroll
+                for (int c = 0; c < 2 * CP; ++c) {
+                    const uint32_t r0 = v[c / 2][mt][c % 2 * 2] ^ 0x80808080u, r1 = v[c / 2][mt][c % 2 * 2 + 1] ^ 0x80808080u;
+                    x[c][0] = subnormalPair<0x4240>(r0), x[c][1] = subnormalPair<0x4341>(r0);
+                    x[c][2] = subnormalPair<0x4240>(r1), x[c][3] = subnormalPair<0x4341>(r1);
+                }
+#pragma unroll
+                for (int c = 0; c < 2 * CP; ++c) mmaF16(o[c], x[c][0], x[c][1], x[c][2], x[c][3], b[mt].x, b[mt].y);
+#pragma unroll
+                for (int c = 0; c < 2 * CP; ++c) mmaF16(o[c], x[c][0], x[c][1], x[c][2], x[c][3], b[mt].z, b[mt].w);
+            }
+            __syncwarp();
+            if (lane == 0) mbarArrive(&emptyBar[i % NSLOT]);
+        }
+    } else {
+        // ---------------------------------- row sums ----------------------------------
+        float l0 = 0.0f, l1 = 0.0f, ps0 = 0.0f, ps1 = 0.0f;
+        for (uint32_t i = 0; i < n; ++i) {
+            if (!mbarWaitClock(&fullBar[i % NSLOT], (i / NSLOT) & 1u, p.err, kDevErrFullWait)) break;
+            const uint8_t *rec = record(i);
+            const float *fac = reinterpret_cast<const float *>(rec + kRecF);
+            const float *recP = reinterpret_cast<const float *>(rec + kRecP) + lane;
+            const float *recX = reinterpret_cast<const float *>(rec + kRecX) + lane;
+            float pv[2 * NR], xv[2 * NR];
+#pragma unroll
+            for (int r = 0; r < 2 * NR; ++r) pv[r] = recP[r * 32], xv[r] = recX[r * 32];
+            if (*reinterpret_cast<const uint32_t *>(fac + 16) != 0u) {
+                const float2 al = *reinterpret_cast<const float2 *>(fac + 2 * t);
+                const float2 as = *reinterpret_cast<const float2 *>(fac + 8 + 2 * t);
+                l0 *= as.x, l1 *= as.y;
+                ps0 *= al.x, ps1 *= al.y;
+            }
+#pragma unroll
+            for (int r = 0; r < NR; ++r) {
+                l0 += pv[2 * r], l1 += pv[2 * r + 1];
+                ps0 += xv[2 * r], ps1 += xv[2 * r + 1];
+            }
+            __syncwarp();
+            if (lane == 0) mbarArrive(&emptyBar[i % NSLOT]);
+        }
+#pragma unroll
+        for (int off = 4; off <= 16; off <<= 1) {
+            l0 += __shfl_xor_sync(0xffffffffu, l0, off);
+            l1 += __shfl_xor_sync(0xffffffffu, l1, off);
+            ps0 += __shfl_xor_sync(0xffffffffu, ps0, off);
+            ps1 += __shfl_xor_sync(0xffffffffu, ps1, off);
+        }
+        if (g == 0) {
+            sEnd[16 + 2 * t] = l0, sEnd[17 + 2 * t] = l1;
+            sEnd[24 + 2 * t] = ps0, sEnd[25 + 2 * t] = ps1;
+        }
+    }
+    __syncthreads();
+    float *scr = reinterpret_cast<float *>(smem);  // [8 heads][HD], then m[8], l[8]
+    if (warp >= SW && warp < SW + VW) {
+        // true accumulator = 2^24 * raw - 128 * sum(p*sv), then back from the E-scaled domain
+        const float E = sEnd[8], c0 = 128.0f * sEnd[24 + 2 * t], c1 = 128.0f * sEnd[25 + 2 * t];
+#pragma unroll
+        for (int c = 0; c < 2 * CP; ++c) {
+            const uint32_t d = (warp - SW) * (HD / 4) + 16 * c + 2 * g;
+            *reinterpret_cast<float2 *>(scr + (2 * t) * HD + d) =
+                    make_float2(fmaf(o[c][0], kI8Unscale, -c0) * E, fmaf(o[c][2], kI8Unscale, -c0) * E);
+            *reinterpret_cast<float2 *>(scr + (2 * t + 1) * HD + d) =
+                    make_float2(fmaf(o[c][1], kI8Unscale, -c1) * E, fmaf(o[c][3], kI8Unscale, -c1) * E);
+        }
+    } else if (warp == 0 && lane < 8u) {
+        scr[8 * HD + lane] = sEnd[lane];
+        scr[8 * HD + 8 + lane] = sEnd[16 + lane];
+    }
+    __syncthreads();
+    FoldTarget f;
+    f.out = p.out, f.pAcc = nullptr, f.pM = nullptr, f.pL = nullptr;
+    f.numChunks = 1, f.slot = 0;
+    f.firstHead = head0, f.nValid = nValid;
+    f.direct = 1;
+    f.qRot = nullptr, f.cosT = nullptr, f.sinT = nullptr, f.tableRow = 0;
+    clusterFold<HD, 1, kThreads>(scr, f, threadIdx.x);
+}
+
+template <int HD, int MT>
+static int launchStreams(DecodeI8Params prm, cudaStream_t st) {
+    using L = I8StreamSmem<HD, MT>;
+    auto kern = decodeI8StreamsKernel<HD, MT>;
+    static ClusterSetup setup;
+    const uint32_t *limits = nullptr;
+    int rc = setupCluster(setup, kern, L::kWarps * 32, L::kTotal, &limits);
+    if (rc != TC_OK) return rc;
+    for (uint32_t cb = 0; cb < prm.group; cb += 8) {  // 8 q heads of a kv head per launch
+        prm.colBase = cb;
+        if (cb) prm.appendK = prm.appendV = nullptr;  // the row is in
+        rc = launchDependent(kern, dim3(8, prm.nKV, 1), L::kWarps * 32, L::kTotal, st, 8, prm);
+        if (rc != TC_OK) return rc;
+    }
+    return TC_OK;
+}
+
+int launchStreamsI8(DecodeI8Params prm, uint32_t hd, cudaStream_t st) {
+    return hd == 256 ? launchStreams<256, 1>(prm, st) : launchStreams<128, 2>(prm, st);
+}
+
+}  // namespace tc
