@@ -185,6 +185,19 @@ __device__ __forceinline__ void copyTile(uint32_t dst, const uint8_t *base, uint
     }
 }
 
+// The rows of one 16-token tile of K and V (ROWB bytes each) towards L2, by one warp.  Right at any time, also ahead of the
+// dependency wait: a row that a kernel in flight still writes is read after the wait.  The launches of a token's
+// layers overlap by their prologues, so DRAM streams the next layer's rows while this one computes.
+template <int ROWB>
+__device__ __forceinline__ void prefetchTile(const uint8_t *k, const uint8_t *v, size_t stride, uint64_t row, uint64_t lastRow,
+                                             uint32_t lane) {
+    const uint64_t r = row + (lane & 15u);
+    const uint8_t *p = (lane < 16u ? k : v) + (r < lastRow ? r : lastRow) * stride;
+#pragma unroll
+    for (int i = 0; i < ROWB / 128; ++i) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + i * 128));
+}
+constexpr uint32_t kPrefetchTiles = 2;  // of a warp, ahead of the wait
+
 // ---- distributed shared memory -------------------------------------------------------------------
 __device__ __forceinline__ uint32_t clusterRank() {
     uint32_t r;

@@ -60,6 +60,19 @@ decodeI8Kernel(const __grid_constant__ DecodeI8Params p) {
     extern __shared__ uint8_t smemRaw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smemRaw) + 127) & ~uintptr_t(127));
 
+    if (!ROWS && p.devLens == nullptr && p.devRowBase == nullptr) {
+        const uint64_t base = static_cast<uint64_t>(b) * p.rowsPerSeq;
+        const uint32_t t0 = chunk * p.chunkTokens, t1 = min(p.lenHost, t0 + p.chunkTokens);
+        const uint8_t *k = reinterpret_cast<const uint8_t *>(p.k8w) + static_cast<size_t>(hg) * HD;
+        const uint8_t *v = reinterpret_cast<const uint8_t *>(p.v8w) + static_cast<size_t>(hg) * HD;
+        for (uint32_t i = 0, tok = t0 + warp * T; i < kPrefetchTiles && tok < t1; ++i, tok += NW * T) {
+            prefetchTile<HD>(k, v, static_cast<size_t>(p.nKV) * HD, base + tok, p.totalRows - 1, lane);
+            if (lane < 2u) {
+                const float *s = (lane ? p.vs : p.ks) + min(base + tok, p.totalRows - 1) * p.nKV + hg;
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(s));
+            }
+        }
+    }
     gridDepWait();
     gridDepLaunch();
 

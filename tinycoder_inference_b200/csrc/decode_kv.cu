@@ -22,12 +22,12 @@
 
 namespace tc {
 
-// Every warp has a slot for a 16-token tile of K and one of V, each as HD / 32 boxes of [16 rows][32 floats].
-template <int HD, int NW>
+// Every warp has SLOTS slots for 16-token tiles of K and as many of V, each as HD / 32 boxes of [16 rows][32 floats].
+template <int HD, int NW, int SLOTS>
 struct DecodeKvSmem {
     static constexpr int NB = HD / 32;             // 32-float boxes per row
     static constexpr int kTileBytes = 16 * HD * 4; // K (or V) bytes of a tile
-    static constexpr int kSlots = NW * 2 * kTileBytes, kScratch = (NW + 1) * (8 * HD + 16) * 4;  // (the fold reuses the slots)
+    static constexpr int kSlots = NW * SLOTS * 2 * kTileBytes, kScratch = (NW + 1) * (8 * HD + 16) * 4;  // (the fold reuses the slots)
     static constexpr int kTotal = (kSlots > kScratch ? kSlots : kScratch) + 128;
     static_assert(kTotal <= 227 * 1024, "shared memory of an SM");
 };
@@ -45,9 +45,9 @@ __device__ __forceinline__ void splitTf32(float x, uint32_t &hi, uint32_t &lo) {
 // many warps per SM, each with a tile of its own, to keep up.  16-byte copies by the warp itself serve that: small TMA
 // boxes from one producer thread do not (22 us for 18.8 MB of one layer), and boxes shared by a block's warps leave
 // too few of them (17 us; this form 15).  192 MB of one layer (28 / 4 / 128 at 47000 rows): 42 us.
-template <int HD, int NW, bool ROWS>
-__global__ void __launch_bounds__(NW * 32, ROWS ? 1 : 2) decodeKvKernel(const __grid_constant__ DecodeKvParams p) {
-    using L = DecodeKvSmem<HD, NW>;
+template <int HD, int NW, int SLOTS, int BPS, bool ROWS>
+__global__ void __launch_bounds__(NW * 32, BPS) decodeKvKernel(const __grid_constant__ DecodeKvParams p) {
+    using L = DecodeKvSmem<HD, NW, SLOTS>;
     constexpr int T = 16, NB = L::NB;
     constexpr int KS = HD / 8;   // tf32 k-steps of the QK product
     constexpr int MTO = HD / 16;  // 16-dim output tiles
@@ -59,6 +59,15 @@ __global__ void __launch_bounds__(NW * 32, ROWS ? 1 : 2) decodeKvKernel(const __
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smemRaw) + 127) & ~uintptr_t(127));
     __shared__ float pScratch[NW][16 * 8];
 
+    if (!ROWS) {
+        // (a device position read here may be a step old: good enough to know which rows to pull)
+        const uint32_t hint = p.devPos ? min(p.devPos[0], p.lenHost - 1u) + 1u : p.lenHost;
+        const uint32_t per = p.devPos ? tokensPerBlock(hint, gridDim.x) : p.chunkTokens;
+        const uint8_t *k = static_cast<const uint8_t *>(p.kvK) + static_cast<size_t>(hg) * HD * 4;
+        const uint8_t *v = static_cast<const uint8_t *>(p.kvV) + static_cast<size_t>(hg) * HD * 4;
+        for (uint32_t i = 0, tok = chunk * per + warp * T; i < kPrefetchTiles && tok < min(hint, (chunk + 1u) * per); ++i, tok += NW * T)
+            prefetchTile<HD * 4>(k, v, static_cast<size_t>(p.nKV) * HD * 4, tok, p.totalRows - 1, lane);
+    }
     gridDepWait();
     gridDepLaunch();
 
@@ -78,13 +87,14 @@ __global__ void __launch_bounds__(NW * 32, ROWS ? 1 : 2) decodeKvKernel(const __
     const uint32_t nTiles = t0 < t1 ? (t1 - t0 + T - 1) / T : 0u;
     const uint32_t kvHead = ROWS ? hg / p.group : hg;
 
-    // Tile j belongs to warp j % NW.  A warp copies its own tiles: the next tile's K while it works on this one's V,
-    // the next V while it works on K.
-    uint8_t *slotK = smem + warp * 2 * L::kTileBytes, *slotV = slotK + L::kTileBytes;
+    // Tile j belongs to warp j % NW, its slot (j / NW) % SLOTS.  A warp copies its own tiles: with one slot the
+    // next tile's K while it works on this one's V and the next V while it works on K.
+    auto slotK = [&](uint32_t i) { return smem + (warp * SLOTS + i % SLOTS) * 2 * L::kTileBytes; };
     const uint32_t stride = p.nKV * HD * 4;
     const uint8_t *storeK = static_cast<const uint8_t *>(p.kvK) + static_cast<size_t>(kvHead) * HD * 4;
     const uint8_t *storeV = static_cast<const uint8_t *>(p.kvV) + static_cast<size_t>(kvHead) * HD * 4;
-    auto requestK = [&](uint32_t j) {
+    auto requestK = [&](uint32_t i) {
+        const uint32_t j = warp + i * NW;
         if (j < nTiles) {
             if (!ROWS && p.tok.k != nullptr && j + 1 == nTiles && t1 == len) {
                 // the tile that holds the new token's row: the row goes in first
@@ -96,16 +106,20 @@ __global__ void __launch_bounds__(NW * 32, ROWS ? 1 : 2) decodeKvKernel(const __
                                          len - 1u, lane);
                 }
             }
-            copyTile<T, HD * 4>(smemAddr(slotK), storeK, stride, t0 + j * T, p.totalRows - 1, lane);
+            copyTile<T, HD * 4>(smemAddr(slotK(i)), storeK, stride, t0 + j * T, p.totalRows - 1, lane);
         }
         cpAsyncCommit();
     };
-    auto requestV = [&](uint32_t j) {
-        if (j < nTiles) copyTile<T, HD * 4>(smemAddr(slotV), storeV, stride, t0 + j * T, p.totalRows - 1, lane);
+    auto requestV = [&](uint32_t i) {
+        const uint32_t j = warp + i * NW;
+        if (j < nTiles) copyTile<T, HD * 4>(smemAddr(slotK(i) + L::kTileBytes), storeV, stride, t0 + j * T, p.totalRows - 1, lane);
         cpAsyncCommit();
     };
-    requestK(warp);
-    requestV(warp);
+#pragma unroll
+    for (uint32_t i = 0; i < SLOTS; ++i) {
+        requestK(i);
+        requestV(i);
+    }
 
     const uint32_t g = lane >> 2, t = lane & 3u;
     auto colValid = [&](uint32_t j) { return ROWS ? (b * 8u + j < p.qRows) : (p.colBase + j < p.group); };
@@ -172,8 +186,8 @@ __global__ void __launch_bounds__(NW * 32, ROWS ? 1 : 2) decodeKvKernel(const __
     for (int i = 0; i < MTO; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
     float *pS = pScratch[warp];
 
-    for (uint32_t tile = warp; tile < nTiles; tile += NW) {
-        cpAsyncWait<1>();  // K of this tile is in, V may still be on its way
+    for (uint32_t i = 0, tile = warp; tile < nTiles; ++i, tile += NW) {
+        cpAsyncWait<2 * SLOTS - 1>();  // K of this tile is in, V may still be on its way
         const uint32_t tok0 = t0 + tile * T;
         const uint32_t tokA = tok0 + g, tokB = tokA + 8;
 
@@ -182,7 +196,7 @@ __global__ void __launch_bounds__(NW * 32, ROWS ? 1 : 2) decodeKvKernel(const __
         float sa[2][4] = {}, sb[2][4] = {}, sc[2][4] = {};
 #pragma unroll
         for (int bx = 0; bx < NB; ++bx) {
-            const uint8_t *kT = slotK + bx * T * 128;
+            const uint8_t *kT = slotK(i) + bx * T * 128;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const uint32_t off = ((2 * t + h) ^ g) << 4;
@@ -212,7 +226,7 @@ __global__ void __launch_bounds__(NW * 32, ROWS ? 1 : 2) decodeKvKernel(const __
             }
         }
         __syncwarp();  // every lane has read its part of K
-        requestK(tile + NW);
+        requestK(i + SLOTS);
         auto dot = [&](int i) { return (sa[0][i] + sa[1][i]) + ((sb[0][i] + sb[1][i]) + (sc[0][i] + sc[1][i])); };
         const float s00 = tokA < len0 ? dot(0) * cs : -INFINITY;
         const float s01 = tokA < len1 ? dot(1) * cs : -INFINITY;
@@ -257,14 +271,14 @@ __global__ void __launch_bounds__(NW * 32, ROWS ? 1 : 2) decodeKvKernel(const __
         }
         __syncwarp();
         // ---- O^T += V^T . P^T (HD dims x 8 columns), 3xTF32 ----
-        cpAsyncWait<1>();  // V of this tile is in, the next K may still be on its way
+        cpAsyncWait<2 * SLOTS - 1>();  // V of this tile is in, the next K may still be on its way
 #pragma unroll
         for (int kk = 0; kk < 2; ++kk) {
             const uint32_t ra = 8 * kk + 2 * t, rb = ra + 1;  // token rows of k slots t and t+4
             const bool okA = tok0 + ra < t1, okB = tok0 + rb < t1;
 #pragma unroll
             for (int bx = 0; bx < NB; ++bx) {
-                const uint8_t *vT = slotV + bx * T * 128;
+                const uint8_t *vT = slotK(i) + L::kTileBytes + bx * T * 128;
                 float4 xa = *reinterpret_cast<const float4 *>(vT + ra * 128 + ((g ^ (ra & 7u)) << 4));
                 float4 xb = *reinterpret_cast<const float4 *>(vT + rb * 128 + ((g ^ (rb & 7u)) << 4));
                 if (!okA) xa = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -292,7 +306,7 @@ __global__ void __launch_bounds__(NW * 32, ROWS ? 1 : 2) decodeKvKernel(const __
             }
         }
         __syncwarp();
-        requestV(tile + NW);
+        requestV(i + SLOTS);
     }
 
     // ---- fold the consumer warps, then the blocks of the cluster ----
@@ -357,19 +371,17 @@ __global__ void __launch_bounds__(NW * 32, ROWS ? 1 : 2) decodeKvKernel(const __
     }
 }
 
-// As many warps as the registers and the shared memory of an SM carry for two decode blocks (16-block clusters find room
-// twice per GPC then), or for one block of the causal form.
+// Warps of the causal form: as many as the registers and the shared memory of an SM carry.
 template <int HD>
 struct KvShape {
-    static constexpr int kWarps = HD == 64 ? 8 : (HD == 128 ? 6 : 3);
     static constexpr int kRowsWarps = HD == 64 ? 16 : (HD == 128 ? 12 : 6);
 };
 
 template <int HD>
 static int launchRows(const DecodeKvParams &prm, cudaStream_t st) {
     constexpr int NW = KvShape<HD>::kRowsWarps;
-    using L = DecodeKvSmem<HD, NW>;
-    auto kern = decodeKvKernel<HD, NW, true>;
+    using L = DecodeKvSmem<HD, NW, 1>;
+    auto kern = decodeKvKernel<HD, NW, 1, 1, true>;
     static bool attrDone[64] = {false};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -432,13 +444,13 @@ static int prefillKv(const float *q, const void *kvK, const void *kvV, float *ou
     return launchRows<128>(prm, st);
 }
 
-template <int HD>
+template <int HD, int NW, int SLOTS, int BPS>
 static int decodeKv32(const DecodeKvParams &prm, uint8_t *q81Out, cudaStream_t st) {
-    constexpr int NW = KvShape<HD>::kWarps;
-    using L = DecodeKvSmem<HD, NW>;
+    using L = DecodeKvSmem<HD, NW, SLOTS>;
     static ClusterSetup setup;
-    return launchKvDecode(setup, decodeKvKernel<HD, NW, false>, NW * 32, L::kTotal, HD, NW, 2 * L::kTileBytes,
-                          HD == 256 ? 4.2f : (HD == 128 ? 2.85f : 1.7f), HD == 256 ? 1.2f : (HD == 128 ? 0.38f : 0.2f), prm, q81Out, st);
+    return launchKvDecode(setup, decodeKvKernel<HD, NW, SLOTS, BPS, false>, NW * 32, L::kTotal, HD, NW, 2 * L::kTileBytes,
+                          HD == 256 ? 4.2f : (HD == 128 ? 2.85f : 1.7f), HD == 256 ? 1.2f : (HD == 128 ? 0.38f : 0.2f), prm,
+                          q81Out, st);
 }
 
 int decodeKvToken(const float *q, const void *kvK, const void *kvV, float *attnOut, float *pAcc, float *pM, float *pL,
@@ -471,9 +483,14 @@ int decodeKvToken(const float *q, const void *kvK, const void *kvV, float *attnO
     prm.err = devErrorWord();
     TC_REQUIRE(prm.err != nullptr, TC_ECUDA, "tc_attn_decode_kv: no device error word");
     if (kvHalf) return decodeKv16(prm, hd, q81Out, st);
-    if (hd == 64) return decodeKv32<64>(prm, q81Out, st);
-    if (hd == 128) return decodeKv32<128>(prm, q81Out, st);
-    return decodeKv32<256>(prm, q81Out, st);
+    // Warps of a block, slots of a warp, blocks per SM.  Rows that a 16-block cluster covers with one tile per warp (head_dim
+    // 128: 1536) want small blocks; longer ones as many warps per SM as fit (head_dim 128, per layer: 2048 rows 8.6 against
+    // 9.5 us, 20000 rows 23.8 against 26.4, 200 rows 7.2 against 6.5; head_dim 256: 8191 / 20000 rows 19.5 / 36.2 us with
+    // four warps per SM, 21.5 / 29.8 with six).
+    if (hd == 64) return decodeKv32<64, 8, 2, 1>(prm, q81Out, st);
+    if (hd == 128)
+        return prm.lenHost <= 1536u ? decodeKv32<128, 6, 1, 2>(prm, q81Out, st) : decodeKv32<128, 8, 1, 1>(prm, q81Out, st);
+    return prm.lenHost <= 12288u ? decodeKv32<256, 4, 1, 1>(prm, q81Out, st) : decodeKv32<256, 6, 1, 1>(prm, q81Out, st);
 }
 
 }  // namespace tc

@@ -18,13 +18,13 @@
 
 namespace tc {
 
-// Every warp has a slot for a 16-token tile of K and one of V, each as HD / 64 half-tiles of [16 rows][64 halves =
+// Every warp has SLOTS slots for 16-token tiles of K and as many of V, each as HD / 64 half-tiles of [16 rows][64 halves =
 // 128 bytes], half-tile a covering dims [64a, 64a + 64).
-template <int HD, int NW>
+template <int HD, int NW, int SLOTS>
 struct DecodeKv16Smem {
     static constexpr int kAtomBytes = 16 * 128;      // one half-tile
     static constexpr int kTileBytes = 16 * HD * 2;
-    static constexpr int kSlots = NW * 2 * kTileBytes, kScratch = (NW + 1) * (8 * HD + 16) * 4;  // (the fold reuses the slots)
+    static constexpr int kSlots = NW * SLOTS * 2 * kTileBytes, kScratch = (NW + 1) * (8 * HD + 16) * 4;  // (the fold reuses the slots)
     static constexpr int kTotal = (kSlots > kScratch ? kSlots : kScratch) + 128;
     static_assert(kTotal <= 227 * 1024, "shared memory of an SM");
 };
@@ -33,9 +33,9 @@ constexpr float kLazyLog2Kv16 = 8.0f;  // see decode_i8.cu: p stays <= 2^8, exac
 
 // ROWS: the causal kernel (one block per 8 query rows and q head); otherwise decode, blocks of a cluster
 // share a kv head's tokens.
-template <int HD, int NW, bool ROWS>
-__global__ void __launch_bounds__(NW * 32, ROWS ? 1 : 2) decodeKv16Kernel(const __grid_constant__ DecodeKvParams p) {
-    using L = DecodeKv16Smem<HD, NW>;
+template <int HD, int NW, int SLOTS, int BPS, bool ROWS>
+__global__ void __launch_bounds__(NW * 32, BPS) decodeKv16Kernel(const __grid_constant__ DecodeKvParams p) {
+    using L = DecodeKv16Smem<HD, NW, SLOTS>;
     constexpr int T = 16;
     constexpr int NS = HD / 16;     // k16 steps of QK^T = 16-dim output tiles of PV
 
@@ -45,6 +45,15 @@ __global__ void __launch_bounds__(NW * 32, ROWS ? 1 : 2) decodeKv16Kernel(const 
     extern __shared__ uint8_t smemRaw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smemRaw) + 127) & ~uintptr_t(127));
 
+    if (!ROWS) {
+        // (a device position read here may be a step old: good enough to know which rows to pull)
+        const uint32_t hint = p.devPos ? min(p.devPos[0], p.lenHost - 1u) + 1u : p.lenHost;
+        const uint32_t per = p.devPos ? tokensPerBlock(hint, gridDim.x) : p.chunkTokens;
+        const uint8_t *k = static_cast<const uint8_t *>(p.kvK) + static_cast<size_t>(hg) * HD * 2;
+        const uint8_t *v = static_cast<const uint8_t *>(p.kvV) + static_cast<size_t>(hg) * HD * 2;
+        for (uint32_t i = 0, tok = chunk * per + warp * T; i < kPrefetchTiles && tok < min(hint, (chunk + 1u) * per); ++i, tok += NW * T)
+            prefetchTile<HD * 2>(k, v, static_cast<size_t>(p.nKV) * HD * 2, tok, p.totalRows - 1, lane);
+    }
     gridDepWait();
     gridDepLaunch();
 
@@ -64,13 +73,14 @@ __global__ void __launch_bounds__(NW * 32, ROWS ? 1 : 2) decodeKv16Kernel(const 
     const uint32_t nTiles = t0 < t1 ? (t1 - t0 + T - 1) / T : 0u;
     const uint32_t kvHead = ROWS ? hg / p.group : hg;
 
-    // Tile j belongs to warp j % NW.  A warp copies its own tiles: the next tile's K while it works on this one's V,
-    // the next V while it works on K.
-    uint8_t *slotK = smem + warp * 2 * L::kTileBytes, *slotV = slotK + L::kTileBytes;
+    // Tile j belongs to warp j % NW, its slot (j / NW) % SLOTS.  A warp copies its own tiles: with one slot the
+    // next tile's K while it works on this one's V and the next V while it works on K.
+    auto slotK = [&](uint32_t i) { return smem + (warp * SLOTS + i % SLOTS) * 2 * L::kTileBytes; };
     const uint32_t stride = p.nKV * HD * 2;
     const uint8_t *storeK = static_cast<const uint8_t *>(p.kvK) + static_cast<size_t>(kvHead) * HD * 2;
     const uint8_t *storeV = static_cast<const uint8_t *>(p.kvV) + static_cast<size_t>(kvHead) * HD * 2;
-    auto requestK = [&](uint32_t j) {
+    auto requestK = [&](uint32_t i) {
+        const uint32_t j = warp + i * NW;
         if (j < nTiles) {
             if (!ROWS && p.tok.k != nullptr && j + 1 == nTiles && t1 == len) {
                 // the tile that holds the new token's row: the row goes in first
@@ -82,16 +92,20 @@ __global__ void __launch_bounds__(NW * 32, ROWS ? 1 : 2) decodeKv16Kernel(const 
                                           len - 1u, lane);
                 }
             }
-            copyTile<T, HD * 2>(smemAddr(slotK), storeK, stride, t0 + j * T, p.totalRows - 1, lane);
+            copyTile<T, HD * 2>(smemAddr(slotK(i)), storeK, stride, t0 + j * T, p.totalRows - 1, lane);
         }
         cpAsyncCommit();
     };
-    auto requestV = [&](uint32_t j) {
-        if (j < nTiles) copyTile<T, HD * 2>(smemAddr(slotV), storeV, stride, t0 + j * T, p.totalRows - 1, lane);
+    auto requestV = [&](uint32_t i) {
+        const uint32_t j = warp + i * NW;
+        if (j < nTiles) copyTile<T, HD * 2>(smemAddr(slotK(i) + L::kTileBytes), storeV, stride, t0 + j * T, p.totalRows - 1, lane);
         cpAsyncCommit();
     };
-    requestK(warp);
-    requestV(warp);
+#pragma unroll
+    for (uint32_t i = 0; i < SLOTS; ++i) {
+        requestK(i);
+        requestV(i);
+    }
 
     const uint32_t g = lane >> 2, t = lane & 3u;
     auto colValid = [&](uint32_t j) { return ROWS ? (b * 8u + j < p.qRows) : (p.colBase + j < p.group); };
@@ -169,14 +183,14 @@ __global__ void __launch_bounds__(NW * 32, ROWS ? 1 : 2) decodeKv16Kernel(const 
     const uint32_t lco = lane >> 4;                             // and which 16-byte chunk of the pair
     const uint32_t lmOff = lr * 128;
 
-    for (uint32_t tile = warp; tile < nTiles; tile += NW) {
-        cpAsyncWait<1>();  // K of this tile is in, V may still be on its way
+    for (uint32_t i = 0, tile = warp; tile < nTiles; ++i, tile += NW) {
+        cpAsyncWait<2 * SLOTS - 1>();  // K of this tile is in, V may still be on its way
         const uint32_t tokW = t0 + tile * T;  // first token of the tile
         const uint32_t tokA = tokW + g, tokB = tokA + 8;
 
         // ---- S^T = K . Q^T (16 tokens x 8 columns) ----
         float sh[4] = {0.f, 0.f, 0.f, 0.f}, sl[4] = {0.f, 0.f, 0.f, 0.f};
-        const uint32_t kTile = smemAddr(slotK);
+        const uint32_t kTile = smemAddr(slotK(i));
 #pragma unroll
         for (int ks = 0; ks < NS; ++ks) {
             const uint32_t sw = (((2 * (ks & 3) + lco) ^ (lr & 7u)) << 4) + (ks >> 2) * L::kAtomBytes;
@@ -186,7 +200,7 @@ __global__ void __launch_bounds__(NW * 32, ROWS ? 1 : 2) decodeKv16Kernel(const 
             mmaF16(sl, r0, r1, r2, r3, qlo[ks][0], qlo[ks][1]);
         }
         __syncwarp();  // every lane has read its part of K
-        requestK(tile + NW);
+        requestK(i + SLOTS);
         // a stale or foreign row behind the range may hold anything, NaN included: select, never scale
         const float s00 = tokA < len0 ? (sh[0] + sl[0]) * cs0 : -INFINITY;
         const float s01 = tokA < len1 ? (sh[1] + sl[1]) * cs1 : -INFINITY;
@@ -239,8 +253,8 @@ __global__ void __launch_bounds__(NW * 32, ROWS ? 1 : 2) decodeKv16Kernel(const 
             mk0 = (tokW + 2 * t < t1 ? 0x0000ffffu : 0u) | (tokW + 2 * t + 1 < t1 ? 0xffff0000u : 0u);
             mk1 = (tokW + 8 + 2 * t < t1 ? 0x0000ffffu : 0u) | (tokW + 8 + 2 * t + 1 < t1 ? 0xffff0000u : 0u);
         }
-        cpAsyncWait<1>();  // V of this tile is in, the next K may still be on its way
-        const uint32_t vTile = smemAddr(slotV);
+        cpAsyncWait<2 * SLOTS - 1>();  // V of this tile is in, the next K may still be on its way
+        const uint32_t vTile = smemAddr(slotK(i) + L::kTileBytes);
 #pragma unroll
         for (int ks = 0; ks < NS; ++ks) {
             const uint32_t sw = (((2 * (ks & 3) + lco) ^ (lr & 7u)) << 4) + (ks >> 2) * L::kAtomBytes;
@@ -255,7 +269,7 @@ __global__ void __launch_bounds__(NW * 32, ROWS ? 1 : 2) decodeKv16Kernel(const 
             mmaF16(o[ks], r0, r2, r1, r3, bl[0], bl[1]);
         }
         __syncwarp();
-        requestV(tile + NW);
+        requestV(i + SLOTS);
     }
 
     // ---- fold the consumer warps of each kv head, write the chunk partial ----
@@ -320,27 +334,29 @@ __global__ void __launch_bounds__(NW * 32, ROWS ? 1 : 2) decodeKv16Kernel(const 
     }
 }
 
-// As many warps as the registers of an SM carry for two decode blocks (16-block clusters find room twice per GPC then),
-// or for one block of the causal form.
-template <int HD>
+template <int HD, int NW, int SLOTS, int BPS>
 static int decodeKv16Hd(const DecodeKvParams &prm, uint8_t *q81Out, cudaStream_t st) {
-    constexpr int NW = 8;
-    using L = DecodeKv16Smem<HD, NW>;
+    using L = DecodeKv16Smem<HD, NW, SLOTS>;
     static ClusterSetup setup;
-    return launchKvDecode(setup, decodeKv16Kernel<HD, NW, false>, NW * 32, L::kTotal, HD, NW, 2 * L::kTileBytes,
+    return launchKvDecode(setup, decodeKv16Kernel<HD, NW, SLOTS, BPS, false>, NW * 32, L::kTotal, HD, NW, 2 * L::kTileBytes,
                           HD == 128 ? 0.87f : 0.73f, HD == 128 ? 0.12f : 0.08f, prm, q81Out, st);
 }
 
 // Both are called from decode_kv.cu when kvHalf is set; arguments were validated there.
+// Warps of a block, slots of a warp, blocks per SM: rows beyond what a 16-block cluster covers with one tile per warp
+// (2048) want two tiles of a warp in flight (head_dim 128, per layer: 20000 rows 14.3 against 15.8 us, 47000 rows 24.2
+// against 28.3; 2047 rows 6.0 against 5.9).
 int decodeKv16(const DecodeKvParams &prm, uint32_t hd, uint8_t *q81Out, cudaStream_t st) {
-    return hd == 64 ? decodeKv16Hd<64>(prm, q81Out, st) : decodeKv16Hd<128>(prm, q81Out, st);
+    if (hd == 64)
+        return prm.lenHost <= 2048u ? decodeKv16Hd<64, 8, 1, 2>(prm, q81Out, st) : decodeKv16Hd<64, 8, 2, 1>(prm, q81Out, st);
+    return prm.lenHost <= 2048u ? decodeKv16Hd<128, 8, 1, 2>(prm, q81Out, st) : decodeKv16Hd<128, 8, 2, 1>(prm, q81Out, st);
 }
 
 template <int HD>
 static int rowsKv16Hd(const DecodeKvParams &prm, cudaStream_t st) {
     constexpr int NW = 16;
-    using L = DecodeKv16Smem<HD, NW>;
-    auto kern = decodeKv16Kernel<HD, NW, true>;
+    using L = DecodeKv16Smem<HD, NW, 1>;
+    auto kern = decodeKv16Kernel<HD, NW, 1, 1, true>;
     static bool attrDone[64] = {false};
     int dev = 0;
     cudaGetDevice(&dev);
