@@ -145,11 +145,11 @@ __device__ __forceinline__ void cpAsyncWait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
     __syncwarp();
 }
-// ROWS rows of ROWB bytes (a multiple of 128) by one warp, from row `row` of a [rows][stride bytes] matrix on (rows past
-// the last one re-read it: the caller masks them), as ROWB / 128 boxes of [ROWS][128 bytes], 16-byte units
-// xor-swizzled by the row: what ldmatrix and 16-byte loads down the rows read without bank conflicts.
+// ROWS rows of ROWB bytes (a multiple of 128) by one warp, from row `row` of a [rows][stride bytes] matrix on -- the first
+// `count` of them: what lies behind is left as it is, and masked by the caller -- as ROWB / 128 boxes of [ROWS][128
+// bytes], 16-byte units xor-swizzled by the row: what ldmatrix and 16-byte loads down the rows read without bank conflicts.
 template <int ROWS, int ROWB>
-__device__ __forceinline__ void copyTile(uint32_t dst, const uint8_t *base, uint32_t stride, uint64_t row, uint64_t lastRow,
+__device__ __forceinline__ void copyTile(uint32_t dst, const uint8_t *base, uint32_t stride, uint64_t row, uint32_t count,
                                          uint32_t lane) {
     constexpr uint32_t U = ROWB / 16;  // 16-byte units per row
     if constexpr (U <= 32) {
@@ -157,8 +157,8 @@ __device__ __forceinline__ void copyTile(uint32_t dst, const uint8_t *base, uint
         constexpr uint32_t R = 32 / U;
         const uint32_t r0 = lane / U, u = lane % U;
         const uint32_t d0 = dst + (u / 8) * (ROWS * 128) + r0 * 128 + (((u & 7u) ^ (r0 & 7u)) << 4);
-        if (row + ROWS - 1 <= lastRow) {
-            const uint8_t *src = base + (row + r0) * stride + u * 16;
+        const uint8_t *src = base + (row + r0) * stride + u * 16;
+        if (count >= ROWS) {
 #pragma unroll
             for (uint32_t k = 0; k < ROWS / R; ++k) {
                 cpAsync16((d0 ^ (((k * R) & 7u) << 4)) + k * R * 128, src);
@@ -167,22 +167,28 @@ __device__ __forceinline__ void copyTile(uint32_t dst, const uint8_t *base, uint
         } else {
 #pragma unroll
             for (uint32_t k = 0; k < ROWS / R; ++k) {
-                const uint64_t gr = row + r0 + k * R < lastRow ? row + r0 + k * R : lastRow;
-                cpAsync16((d0 ^ (((k * R) & 7u) << 4)) + k * R * 128, base + gr * stride + u * 16);
+                if (r0 + k * R < count) cpAsync16((d0 ^ (((k * R) & 7u) << 4)) + k * R * 128, src);
+                src += R * stride;
             }
         }
     } else {
         constexpr uint32_t N = U / 32;  // copy instructions per row
+        const uint8_t *src = base + row * stride + lane * 16;
 #pragma unroll
         for (uint32_t r = 0; r < ROWS; ++r) {
-            const uint8_t *src = base + (row + r < lastRow ? row + r : lastRow) * stride + lane * 16;
 #pragma unroll
             for (uint32_t k = 0; k < N; ++k) {
                 const uint32_t u = k * 32 + lane;
-                cpAsync16(dst + (u / 8) * (ROWS * 128) + r * 128 + (((u & 7u) ^ (r & 7u)) << 4), src + k * 512);
+                if (r < count) cpAsync16(dst + (u / 8) * (ROWS * 128) + r * 128 + (((u & 7u) ^ (r & 7u)) << 4), src + k * 512);
             }
+            src += stride;
         }
     }
+}
+// Where byte `off` of row r of such a tile lies.
+template <int ROWS>
+__device__ __forceinline__ uint32_t tileOffset(uint32_t r, uint32_t off) {
+    return (off >> 7) * (ROWS * 128) + r * 128 + ((((off >> 4) & 7u) ^ (r & 7u)) << 4) + (off & 15u);
 }
 
 // The rows of one 16-token tile of K and V (ROWB bytes each) towards L2, by one warp.  Right at any time, also ahead of the
@@ -212,23 +218,13 @@ __device__ __forceinline__ uint32_t clusterSize() {
 __device__ __forceinline__ void clusterSync() {
     asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
+// "This block runs": the other blocks may write its shared memory once they have waited for it.
+__device__ __forceinline__ void clusterHello() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
+__device__ __forceinline__ void clusterHelloWait() { asm volatile("barrier.cluster.wait;" ::: "memory"); }
 __device__ __forceinline__ uint32_t mapRank(uint32_t addr, uint32_t rank) {
     uint32_t r;
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
     return r;
-}
-__device__ __forceinline__ float ldCluster(uint32_t addr) {
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-    return v;
-}
-__device__ __forceinline__ float4 ldCluster4(uint32_t addr) {
-    float4 v;
-    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-                 : "r"(addr)
-                 : "memory");
-    return v;
 }
 
 // The rotated q of nValid heads, written in place: pairs [first, ...) of the heads, a share per caller.
@@ -275,14 +271,53 @@ __device__ __forceinline__ void foldStore(const FoldTarget &f, uint32_t j, uint3
     }
 }
 
+// The blocks of a cluster share the output: rank r takes the r-th slice of its nValid x HD / 4 float4s (`per` of them), and
+// every block writes its results for that slice into rank r's inbox.  One cluster barrier lies between the writes and the
+// reads (which are local); a block may leave after it.  (With the results read from the other blocks' memory instead it
+// took a round trip and a second barrier more: 0.5 us of a launch.)
+template <int V4>
+struct FoldInbox {
+    float4 acc[8 * V4 + 16];
+    float2 ml[8 * V4 + 16];
+};
+template <int V4>
+__device__ __forceinline__ void inboxPush(FoldInbox<V4> &in, uint32_t idx, uint32_t per, uint32_t rank, float M, float l,
+                                          float4 acc) {
+    const uint32_t owner = idx / per, at = rank * per + (idx - owner * per);
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(mapRank(smemAddr(&in.acc[at]), owner)), "f"(acc.x),
+                 "f"(acc.y), "f"(acc.z), "f"(acc.w)
+                 : "memory");
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(mapRank(smemAddr(&in.ml[at]), owner)), "f"(M), "f"(l) : "memory");
+}
+template <int V4>
+__device__ __forceinline__ void inboxTake(const FoldInbox<V4> &in, uint32_t i, uint32_t per, uint32_t n, float &M, float &l,
+                                          float4 &acc) {
+    M = kNegBig, l = 0.0f, acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (uint32_t r = 0; r < n; ++r) M = fmaxf(M, in.ml[r * per + i].x);
+#pragma unroll 4
+    for (uint32_t r = 0; r < n; ++r) {
+        const float2 ml = in.ml[r * per + i];
+        const float4 a = in.acc[r * per + i];
+        const float wgt = fastExp2(ml.x - M);
+        l = fmaf(wgt, ml.y, l);
+        acc.x = fmaf(wgt, a.x, acc.x);
+        acc.y = fmaf(wgt, a.y, acc.y);
+        acc.z = fmaf(wgt, a.z, acc.z);
+        acc.w = fmaf(wgt, a.w, acc.w);
+    }
+}
+
 // Every warp has left [8 columns][HD] accumulators, m[8] (log2 units) and l[8] in its part of
-// scr ([NW][8 HD + 16]).  Called by all NW * 32 threads of the block (tid) with the warps' parts complete.
+// scr ([NW][8 HD + 16]).  Called by all THREADS threads of the block (tid) with the warps' parts complete; in a cluster
+// every thread has said clusterHello() before.
 template <int HD, int NW, int THREADS = NW * 32>
-__device__ __forceinline__ void clusterFold(float *scr, const FoldTarget &f, uint32_t tid) {
+__device__ __forceinline__ void clusterFold(const float *scr, const FoldTarget &f, uint32_t tid) {
     constexpr uint32_t kWarpScr = 8 * HD + 16, V4 = HD / 4;
+    __shared__ FoldInbox<V4> inbox;
     const uint32_t n = clusterSize(), rank = clusterRank();
-    float *part = scr + NW * kWarpScr;  // this block's partial: [8][HD], m[8], l[8]
-    for (uint32_t idx = tid; idx < f.nValid * V4; idx += THREADS) {
+    const uint32_t total = f.nValid * V4, per = (total + n - 1) / n;
+    if (n > 1) clusterHelloWait();
+    for (uint32_t idx = tid; idx < total; idx += THREADS) {
         const uint32_t d4 = idx % V4, j = idx / V4;
         float M = kNegBig;
 #pragma unroll
@@ -300,57 +335,23 @@ __device__ __forceinline__ void clusterFold(float *scr, const FoldTarget &f, uin
             acc.z = fmaf(wgt, a.z, acc.z);
             acc.w = fmaf(wgt, a.w, acc.w);
         }
-        if (n == 1) {
-            foldStore<HD>(f, j, d4, M, l, acc);
-        } else {
-            *reinterpret_cast<float4 *>(part + j * HD + 4 * d4) = acc;
-            if (d4 == 0) {
-                part[8 * HD + j] = M;
-                part[8 * HD + 8 + j] = l;
-            }
-        }
+        if (n == 1) foldStore<HD>(f, j, d4, M, l, acc);
+        else inboxPush<V4>(inbox, idx, per, rank, M, l, acc);
     }
     if (n > 1) clusterSync();
     // (in a cluster of one block the caller's barrier has every warp's q in registers)
     if (f.qRot != nullptr)
         rotateQ<HD>(f.qRot, f.cosT, f.sinT, f.tableRow, f.nValid, rank * THREADS + tid, n * THREADS);
     if (n == 1) return;
-    // the blocks of the cluster share the output: rank r takes the r-th slice of its float4s.  Everything a
-    // thread needs from the other blocks is requested before anything is consumed.
-    const uint32_t total = f.nValid * V4, per = (total + n - 1) / n;
-    const uint32_t end = min(total, (rank + 1) * per), base = smemAddr(part);
-    for (uint32_t idx = rank * per + tid; idx < end; idx += THREADS) {
-        const uint32_t d4 = idx % V4, j = idx / V4;
-        float m[16], ls[16];
-        float4 a[16];
-#pragma unroll
-        for (uint32_t r = 0; r < 16; ++r) {
-            m[r] = kNegBig, ls[r] = 0.0f, a[r] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (r < n) {
-                const uint32_t p = mapRank(base, r);
-                m[r] = ldCluster(p + (8 * HD + j) * 4);
-                ls[r] = ldCluster(p + (8 * HD + 8 + j) * 4);
-                a[r] = ldCluster4(p + (j * HD + 4 * d4) * 4);
-            }
-        }
-        float M = m[0];
-#pragma unroll
-        for (uint32_t r = 1; r < 16; ++r) M = fmaxf(M, m[r]);
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-        float l = 0.0f;
-#pragma unroll
-        for (uint32_t r = 0; r < 16; ++r) {
-            const float wgt = fastExp2(m[r] - M);
-            l = fmaf(wgt, ls[r], l);
-            acc.x = fmaf(wgt, a[r].x, acc.x);
-            acc.y = fmaf(wgt, a[r].y, acc.y);
-            acc.z = fmaf(wgt, a[r].z, acc.z);
-            acc.w = fmaf(wgt, a[r].w, acc.w);
-        }
-        foldStore<HD>(f, j, d4, M, l, acc);
+    for (uint32_t i = tid; i < per && rank * per + i < total; i += THREADS) {
+        const uint32_t idx = rank * per + i;
+        float M, l;
+        float4 acc;
+        inboxTake<V4>(inbox, i, per, n, M, l, acc);
+        foldStore<HD>(f, idx / V4, idx % V4, M, l, acc);
     }
-    clusterSync();  // nobody leaves while its shared memory may still be read
 }
+
 // ---- the new token's row ---------------------------------------------------------------------------------
 template <typename KVT>
 __device__ __forceinline__ KVT kvElem(float x) {
@@ -358,39 +359,102 @@ __device__ __forceinline__ KVT kvElem(float x) {
     else return x;
 }
 
-// The new K/V row of one kv head into an f32 / fp16 store by one warp: V verbatim, K rotated NEOX-style when there
-// are tables (x0' = fmaf(x0, c, -(x1 s)), x1' = fmaf(x0, s, x1 c)) -- the arithmetic of kvAppendKernel, bit for bit.  The
-// warp's own copies read the row back afterwards.
-template <int HD, typename KVT>
-__device__ __forceinline__ void appendRow(const NewToken &t, uint32_t kvHead, KVT *kRow, KVT *vRow, uint32_t tableRow,
-                                          uint32_t lane) {
-    constexpr uint32_t H = HD / 2;
-    const float *k = t.k + static_cast<size_t>(kvHead) * HD, *v = t.v + static_cast<size_t>(kvHead) * HD;
-    float k0[H / 32], k1[H / 32], v0[H / 32], v1[H / 32], c[H / 32], s[H / 32];
+// The new token's K and V row of one kv head, by one warp: loaded ahead of the query's preparation, stored behind it -- into
+// the store and, when the warp's tile with that row is among the first ones (`tileK` / `tileV`, row r of them), into that
+// tile: the row does not go through memory on its way there.  A later tile's copies read it back.
+//
+// f32 / fp16 stores: V verbatim, K rotated NEOX-style when there are tables (x0' = fmaf(x0, c, -(x1 s)), x1' = fmaf(x0, s, x1
+// c)): the arithmetic of kvAppendKernel, bit for bit.
+template <int HD>
+struct NewRow {
+    static constexpr int N = HD / 64;
+    float k0[N], k1[N], v0[N], v1[N], c[N], s[N];
+    __device__ __forceinline__ void load(const NewToken &t, uint32_t kvHead, uint32_t tableRow, uint32_t lane) {
+        const float *k = t.k + static_cast<size_t>(kvHead) * HD, *v = t.v + static_cast<size_t>(kvHead) * HD;
 #pragma unroll
-    for (uint32_t i = 0; i < H / 32; ++i) {
-        const uint32_t j = lane + 32 * i;
-        k0[i] = k[j], k1[i] = k[j + H], v0[i] = v[j], v1[i] = v[j + H];
-        if (t.cosT != nullptr) {
-            c[i] = __ldg(t.cosT + static_cast<size_t>(tableRow) * H + j);
-            s[i] = __ldg(t.sinT + static_cast<size_t>(tableRow) * H + j);
+        for (uint32_t i = 0; i < N; ++i) {
+            const uint32_t j = lane + 32 * i;
+            k0[i] = k[j], k1[i] = k[j + HD / 2], v0[i] = v[j], v1[i] = v[j + HD / 2];
+            if (t.cosT != nullptr) {
+                c[i] = __ldg(t.cosT + static_cast<size_t>(tableRow) * (HD / 2) + j);
+                s[i] = __ldg(t.sinT + static_cast<size_t>(tableRow) * (HD / 2) + j);
+            }
         }
     }
+    template <typename KVT>
+    __device__ __forceinline__ void store(bool rotate, KVT *kRow, KVT *vRow, uint8_t *tileK, uint8_t *tileV, uint32_t r,
+                                          uint32_t lane) const {
 #pragma unroll
-    for (uint32_t i = 0; i < H / 32; ++i) {
-        const uint32_t j = lane + 32 * i;
-        float a = k0[i], b = k1[i];
-        if (t.cosT != nullptr) {
-            a = fmaf(k0[i], c[i], -__fmul_rn(k1[i], s[i]));
-            b = fmaf(k0[i], s[i], __fmul_rn(k1[i], c[i]));
+        for (uint32_t i = 0; i < N; ++i) {
+            const uint32_t j = lane + 32 * i, j2 = j + HD / 2;
+            float a = k0[i], b = k1[i];
+            if (rotate) {
+                a = fmaf(k0[i], c[i], -__fmul_rn(k1[i], s[i]));
+                b = fmaf(k0[i], s[i], __fmul_rn(k1[i], c[i]));
+            }
+            const KVT ka = kvElem<KVT>(a), kb = kvElem<KVT>(b), va = kvElem<KVT>(v0[i]), vb = kvElem<KVT>(v1[i]);
+            kRow[j] = ka, kRow[j2] = kb;
+            vRow[j] = va, vRow[j2] = vb;
+            if (tileK != nullptr) {
+                const uint32_t o = tileOffset<16>(r, j * sizeof(KVT)), o2 = tileOffset<16>(r, j2 * sizeof(KVT));
+                *reinterpret_cast<KVT *>(tileK + o) = ka, *reinterpret_cast<KVT *>(tileK + o2) = kb;
+                *reinterpret_cast<KVT *>(tileV + o) = va, *reinterpret_cast<KVT *>(tileV + o2) = vb;
+            }
         }
-        kRow[j] = kvElem<KVT>(a);
-        kRow[j + H] = kvElem<KVT>(b);
-        vRow[j] = kvElem<KVT>(v0[i]);
-        vRow[j + H] = kvElem<KVT>(v1[i]);
     }
-    __syncwarp();
-}
+};
+
+// int8 pools: quantised (the arithmetic of kvQuantKernel), with its scale; mirK / mirV (nullable): an f32 store's rows that
+// get it verbatim.
+template <int HD, int T>
+struct NewQuantRow {
+    static constexpr int N = HD / 128;
+    float4 kx[N], vx[N];
+    __device__ __forceinline__ void load(const float *k, const float *v, uint32_t lane) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            kx[i] = __ldg(reinterpret_cast<const float4 *>(k) + lane + 32 * i);
+            vx[i] = __ldg(reinterpret_cast<const float4 *>(v) + lane + 32 * i);
+        }
+    }
+    __device__ __forceinline__ void store(uint32_t *kRow, uint32_t *vRow, float *ksp, float *vsp, float4 *mirK, float4 *mirV,
+                                          uint8_t *tileK, uint8_t *tileV, float *scaleK, float *scaleV, uint32_t r,
+                                          uint32_t lane) const {
+        float mk = 0.0f, mv = 0.0f;
+        auto amax4 = [](const float4 &x) { return fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))); };
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            mk = fmaxf(mk, amax4(kx[i]));
+            mv = fmaxf(mv, amax4(vx[i]));
+            if (mirK != nullptr) mirK[lane + 32 * i] = kx[i], mirV[lane + 32 * i] = vx[i];
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            mk = fmaxf(mk, __shfl_xor_sync(0xffffffffu, mk, o));
+            mv = fmaxf(mv, __shfl_xor_sync(0xffffffffu, mv, o));
+        }
+        const float sk = mk > 0.0f ? __fdiv_rn(mk, 127.0f) : 1.0f, sv = mv > 0.0f ? __fdiv_rn(mv, 127.0f) : 1.0f;
+        if (lane == 0) {
+            *ksp = sk, *vsp = sv;
+            if (tileK != nullptr) scaleK[r] = sk, scaleV[r] = sv;
+        }
+        auto q8 = [](float x, float sc) -> uint32_t {
+            int qv = __float2int_rn(__fdiv_rn(x, sc));
+            qv = qv < -128 ? -128 : (qv > 127 ? 127 : qv);
+            return static_cast<uint32_t>(qv) & 0xffu;
+        };
+        auto pack = [&](const float4 &x, float sc) {
+            return q8(x.x, sc) | (q8(x.y, sc) << 8) | (q8(x.z, sc) << 16) | (q8(x.w, sc) << 24);
+        };
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const uint32_t w = pack(kx[i], sk), w2 = pack(vx[i], sv), o = tileOffset<T>(r, 4 * (lane + 32 * i));
+            kRow[lane + 32 * i] = w;
+            vRow[lane + 32 * i] = w2;
+            if (tileK != nullptr) *reinterpret_cast<uint32_t *>(tileK + o) = w, *reinterpret_cast<uint32_t *>(tileV + o) = w2;
+        }
+    }
+};
 
 // A kernel's shared-memory and cluster attributes, set once per device, and how many clusters of each size are
 // resident at once (the answer depends on its shared memory).

@@ -39,7 +39,7 @@ struct DecodeI8Smem {
     static constexpr int kHalfBytes = T * 128;            // one half-tile
     static constexpr int kTileBytes = T * HD;             // K (or V) bytes of a tile
     static constexpr int kScales = NW * NS * 2 * kTileBytes;   // [warp][slot][K, V][T] floats
-    static constexpr int kSlots = kScales + NW * NS * 2 * T * 4, kScratch = (NW + 1) * (8 * HD + 16) * 4;  // (the fold reuses the slots)
+    static constexpr int kSlots = kScales + NW * NS * 2 * T * 4, kScratch = NW * (8 * HD + 16) * 4;  // (the fold reuses the slots)
     static constexpr int kTotal = (kSlots > kScratch ? kSlots : kScratch) + 128;
     static_assert(kTotal <= 227 * 1024, "shared memory of an SM");
 };
@@ -87,6 +87,7 @@ decodeI8Kernel(const __grid_constant__ DecodeI8Params p) {
         if ((chunk - clusterRank()) * p.chunkTokens >= len) return;
     }
     const uint32_t t0 = ROWS ? 0u : chunk * p.chunkTokens;
+    if (!ROWS && clusterSize() > 1) clusterHello();
     const uint32_t t1 = ROWS ? len : min(len, t0 + p.chunkTokens);
     const uint32_t nTiles = t0 < t1 ? (t1 - t0 + T - 1) / T : 0u;
     const uint64_t rowBase = ROWS ? 0ull : (p.devRowBase ? p.devRowBase[b] : static_cast<uint64_t>(b) * p.rowsPerSeq);
@@ -99,48 +100,34 @@ decodeI8Kernel(const __grid_constant__ DecodeI8Params p) {
     const uint32_t stride = p.nKV * HD;
     const uint8_t *storeK = reinterpret_cast<const uint8_t *>(p.k8w) + static_cast<size_t>(kvHead) * HD;
     const uint8_t *storeV = reinterpret_cast<const uint8_t *>(p.v8w) + static_cast<size_t>(kvHead) * HD;
-    auto copyScales = [&](float *dst, const float *src, uint64_t row) {
-        if (lane < T) cpAsync4(dst + lane, src + min(row + lane, p.totalRows - 1) * p.nKV + kvHead);
-    };
-    auto requestK = [&](uint32_t i) {
-        const uint32_t j = warp + i * NW;
-        if (j < nTiles) {
-            if (!ROWS && p.appendK != nullptr && j + 1 == nTiles && t1 == len) {
-                // the tile that holds the new token's row: the row goes in first
-                const uint64_t row = rowBase + (p.devLens ? p.devLens[b] + p.lenAdd : len) - 1u;
-                if (row >= p.totalRows) {  // a device length outside the pool: no row written, and said so
-                    if (lane == 0) atomicOr(p.err, kDevErrRowBound);
-                } else {
-                    const size_t src = (static_cast<size_t>(b) * p.nKV + kvHead) * (HD / 4);
-                    const uint64_t dst = row * p.nKV + kvHead;
-                    float4 *mk = nullptr, *mv = nullptr;
-                    if (p.mir.k != nullptr)
-                        mk = reinterpret_cast<float4 *>(p.mir.k) + dst * (HD / 4), mv = reinterpret_cast<float4 *>(p.mir.v) + dst * (HD / 4);
-                    appendQuantRow<HD>(reinterpret_cast<const float4 *>(p.appendK) + src,
-                                       reinterpret_cast<const float4 *>(p.appendV) + src, p.k8w, p.v8w,
-                                       const_cast<float *>(p.ks), const_cast<float *>(p.vs), dst, mk, mv, lane);
-                }
-            }
-            const uint64_t row = rowBase + t0 + j * T;
-            copyTile<T, HD>(smemAddr(slotK(i)), storeK, stride, row, p.totalRows - 1, lane);
-            copyScales(scaleK(i), p.ks, row);
-        }
-        cpAsyncCommit();
-    };
-    auto requestV = [&](uint32_t i) {
+    // the warp that takes the last tile stores the token's row; into the tile itself when that is among its first ones
+    const bool append = !ROWS && p.appendK != nullptr && t1 == len && nTiles != 0;
+    const uint64_t newRow = rowBase + (!ROWS && p.devLens ? p.devLens[b] + p.lenAdd : len) - 1u;
+    const bool outside = append && newRow >= p.totalRows;  // a device length outside the pool: no row written
+    if (outside && threadIdx.x == 0) atomicOr(p.err, kDevErrRowBound);
+    const bool mine = append && !outside && (nTiles - 1u) % NW == warp;
+    const bool intoTile = mine && (nTiles - 1u) / NW < NS;
+    const uint64_t have = intoTile ? rowBase + len - 1u : min(rowBase + len, p.totalRows);
+    auto request = [&](uint32_t i, bool isV) {
         const uint32_t j = warp + i * NW;
         if (j < nTiles) {
             const uint64_t row = rowBase + t0 + j * T;
-            copyTile<T, HD>(smemAddr(slotK(i) + L::kTileBytes), storeV, stride, row, p.totalRows - 1, lane);
-            copyScales(scaleK(i) + T, p.vs, row);
+            const uint32_t count = have > row ? static_cast<uint32_t>(min(have - row, static_cast<uint64_t>(T))) : 0u;
+            copyTile<T, HD>(smemAddr(slotK(i) + (isV ? L::kTileBytes : 0)), isV ? storeV : storeK, stride, row, count, lane);
+            if (lane < count) cpAsync4(scaleK(i) + (isV ? T : 0) + lane, (isV ? p.vs : p.ks) + (row + lane) * p.nKV + kvHead);
         }
         cpAsyncCommit();
     };
+    auto requestK = [&](uint32_t i) { request(i, false); };
+    auto requestV = [&](uint32_t i) { request(i, true); };
 #pragma unroll
     for (uint32_t i = 0; i < NS; ++i) {
         requestK(i);
         requestV(i);
     }
+    NewQuantRow<HD, T> fresh;
+    const size_t newSrc = (static_cast<size_t>(b) * p.nKV + kvHead) * HD;
+    if (mine) fresh.load(p.appendK + newSrc, p.appendV + newSrc, lane);
 
     const uint32_t g = lane >> 2, t = lane & 3u;
     // What MMA column j (0..7) of this warp stands for.
@@ -154,6 +141,17 @@ decodeI8Kernel(const __grid_constant__ DecodeI8Params p) {
 
     I8Query<HD> qf;
     i8LoadQuery<HD>(qf, p.q + colIndex(colValid(g) ? g : 0) * HD, colValid(g), p.invSqrt, lane);
+    if (mine) {
+        const size_t dst = newRow * p.nKV + kvHead;
+        const uint32_t i = (nTiles - 1u) / NW;
+        float4 *mk = nullptr, *mv = nullptr;
+        if (p.mir.k != nullptr)
+            mk = reinterpret_cast<float4 *>(p.mir.k) + dst * (HD / 4), mv = reinterpret_cast<float4 *>(p.mir.v) + dst * (HD / 4);
+        uint8_t *tile = intoTile ? slotK(i) : nullptr;
+        fresh.store(p.k8w + dst * (HD / 4), p.v8w + dst * (HD / 4), const_cast<float *>(p.ks) + dst, const_cast<float *>(p.vs) + dst,
+                    mk, mv, tile, tile + L::kTileBytes, scaleK(i), scaleK(i) + T, len - 1u - (t0 + (nTiles - 1u) * T), lane);
+        __syncwarp();
+    }
     const uint32_t len0 = colLen(2 * t), len1 = colLen(2 * t + 1);
 
     float m0 = kNegBig, m1 = kNegBig, l0 = 0.0f, l1 = 0.0f;

@@ -36,7 +36,7 @@ struct I8StreamSmem {
     static constexpr int kEnd = kMax + 2 * kScoreWarps * 12 * 4;   // m[8], E, then l[8], sums of P x scale [8]
     static constexpr int kBars = kEnd + 32 * 4;                    // full, empty per slot
     static constexpr int kTotal = kBars + 2 * kSlots * 8 + 128;
-    static_assert(2 * (8 * HD + 16) * 4 <= kV, "the fold reuses the K tiles");
+    static_assert((8 * HD + 16) * 4 <= kV, "the fold reuses the K tiles");
     static_assert(kTotal <= 227 * 1024, "shared memory of an SM");
 };
 
@@ -61,6 +61,7 @@ decodeI8StreamsKernel(const __grid_constant__ DecodeI8Params p) {
         fenceBarrierInit();
     }
     __syncthreads();
+    clusterHello();
     gridDepWait();
     gridDepLaunch();
 
@@ -86,29 +87,23 @@ decodeI8StreamsKernel(const __grid_constant__ DecodeI8Params p) {
         const uint8_t *storeV = reinterpret_cast<const uint8_t *>(p.v8w) + static_cast<size_t>(kvHead) * HD;
         auto slotK = [&](uint32_t i) { return smem + L::kK + (warp * 2 + (i / SW) % 2) * L::kTileBytes; };
         auto scales = [&](uint32_t i) { return reinterpret_cast<float *>(smem + L::kScales) + (warp * 2 + (i / SW) % 2) * 2 * T; };
-        auto copyScales = [&](float *dst, const float *src, uint64_t row) {
-            if (lane < T) cpAsync4(dst + lane, src + min(row + lane, p.totalRows - 1) * p.nKV + kvHead);
+        // the warp that takes the last tile stores the token's row; into the tile itself when it is the warp's first one
+        const bool outside = p.appendK != nullptr && want > p.totalRows;  // a device position outside the pool: no row written
+        if (outside && stream == 0 && threadIdx.x == 0) atomicOr(p.err, kDevErrRowBound);
+        const uint32_t iLast = (nTiles - 1u) / 8u;
+        const bool mine = p.appendK != nullptr && !outside && (nTiles - 1u) % 8u == stream && iLast % SW == warp;
+        const bool intoTile = mine && iLast < SW;
+        const uint32_t have = intoTile ? len - 1u : static_cast<uint32_t>(min(static_cast<uint64_t>(len), p.totalRows));
+        auto request = [&](uint32_t i, bool isV) {
+            const uint32_t row = (stream + 8u * i) * T;
+            uint8_t *tile = isV ? smem + L::kV + (i % NSLOT) * L::kTileBytes : slotK(i);
+            const uint32_t count = have > row ? min(have - row, static_cast<uint32_t>(T)) : 0u;
+            copyTile<T, HD>(smemAddr(tile), isV ? storeV : storeK, stride, row, count, lane);
+            if (lane < count)
+                cpAsync4(scales(i) + (isV ? T : 0) + lane, (isV ? p.vs : p.ks) + static_cast<size_t>(row + lane) * p.nKV + kvHead);
         };
         auto requestK = [&](uint32_t i) {
-            if (i < n) {
-                const uint32_t j = stream + 8u * i;
-                if (p.appendK != nullptr && j + 1 == nTiles) {
-                    // the tile that holds the new token's row: the row goes in first
-                    const uint64_t row = static_cast<uint64_t>(want) - 1u;
-                    if (row >= p.totalRows) {  // a device position outside the pool: no row written, and said so
-                        if (lane == 0) atomicOr(p.err, kDevErrRowBound);
-                    } else {
-                        const size_t src = static_cast<size_t>(kvHead) * (HD / 4);
-                        appendQuantRow<HD>(reinterpret_cast<const float4 *>(p.appendK) + src,
-                                           reinterpret_cast<const float4 *>(p.appendV) + src, p.k8w, p.v8w,
-                                           const_cast<float *>(p.ks), const_cast<float *>(p.vs), row * p.nKV + kvHead, nullptr,
-                                           nullptr, lane);
-                    }
-                }
-                const uint64_t row = static_cast<uint64_t>(j) * T;
-                copyTile<T, HD>(smemAddr(slotK(i)), storeK, stride, row, p.totalRows - 1, lane);
-                copyScales(scales(i), p.ks, row);
-            }
+            if (i < n) request(i, false);
             cpAsyncCommit();
         };
         bool ok = true;
@@ -116,17 +111,28 @@ decodeI8StreamsKernel(const __grid_constant__ DecodeI8Params p) {
             if (ok && i < n) {
                 // the slot's tile of a round before has been folded by everybody
                 if (i >= NSLOT) ok = mbarWaitClock(&emptyBar[i % NSLOT], (i / NSLOT - 1u) & 1u, p.err, kDevErrEmptyWait);
-                const uint64_t row = static_cast<uint64_t>(stream + 8u * i) * T;
-                copyTile<T, HD>(smemAddr(smem + L::kV + (i % NSLOT) * L::kTileBytes), storeV, stride, row, p.totalRows - 1, lane);
-                copyScales(scales(i) + T, p.vs, row);
+                request(i, true);
             }
             cpAsyncCommit();
         };
         requestK(warp);
         requestV(warp);
-        requestK(warp + SW);
+        // (the tile after that one is requested behind the row's store when it holds the row)
+        NewQuantRow<HD, T> fresh;
+        const size_t newSrc = static_cast<size_t>(kvHead) * HD;
+        if (mine) fresh.load(p.appendK + newSrc, p.appendV + newSrc, lane);
+        else requestK(warp + SW);
         I8Query<HD> qf;
         i8LoadQuery<HD>(qf, p.q + static_cast<size_t>(head0 + (g < nValid ? g : 0u)) * HD, g < nValid, p.invSqrt, lane);
+        if (mine) {
+            const size_t dst = static_cast<size_t>(len - 1u) * p.nKV + kvHead;
+            uint8_t *tile = intoTile ? slotK(iLast) : nullptr;
+            fresh.store(p.k8w + dst * (HD / 4), p.v8w + dst * (HD / 4), const_cast<float *>(p.ks) + dst,
+                        const_cast<float *>(p.vs) + dst, nullptr, nullptr, tile, smem + L::kV + (iLast % NSLOT) * L::kTileBytes,
+                        scales(iLast), scales(iLast) + T, len - 1u - (nTiles - 1u) * T, lane);
+            __syncwarp();
+            requestK(warp + SW);
+        }
         float *sMax = reinterpret_cast<float *>(smem + L::kMax);
         float m0 = kNegBig, m1 = kNegBig;  // at the start of the round
         uint32_t Ebits = 0;                // running power-of-two scale of the V row scales (0 = unset)

@@ -234,6 +234,11 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     if (FOLD != TcFold::kCluster && t0 >= len) return;
     const uint32_t t1 = min(len, t0 + share);
     const uint32_t nTiles = t0 >= len ? 0u : (t1 - t0 + T - 1) / T;
+    constexpr bool CLUSTER = FOLD == TcFold::kCluster;
+    __shared__ FoldInbox<CLUSTER ? 32 : 1> inbox;
+    const uint32_t foldTotal = min(8u, p.group - p.colBase) * 32u;  // float4s of the outputs, and a block's share of them
+    const uint32_t foldPer = CLUSTER ? (foldTotal + clusterSize() - 1u) / clusterSize() : 0u;
+    if constexpr (CLUSTER) clusterHello();
     const uint64_t rowBase = p.devRowBase ? p.devRowBase[b] : static_cast<uint64_t>(b) * p.rowsPerSeq;
 
     if (warp == 0) {
@@ -618,7 +623,6 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         float *mF = scr + 8 * 128;
         float *mS = mF + 8;                       // [NWG][8]
         float *lS = mS + NWG * 8;                 // [4 NWG warps][8]
-        float *clusterL = lS + 4 * NWG * 8;       // [8]: row sums against mF (cluster fold)
         namedBarSync(kEndBar, kEndThreads);       // the fold warpgroup is through: every P tile has been consumed
         if (lane == 0) {
 #pragma unroll
@@ -629,6 +633,7 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         }
         namedBarSync(kEndBar, kEndThreads);
         if (threadIdx.x == 0) TC_STAMP(11);
+        if constexpr (CLUSTER) clusterHelloWait();
         if (warp < 8u) {
             const uint32_t tid = threadIdx.x;  // 0..255: head tid / 32, dims 4 (tid % 32) ..
             const uint32_t h = tid >> 5, d4 = tid & 31u;
@@ -646,8 +651,8 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
                     lsum = fmaf(a, lg, lsum);
                 }
                 const size_t oidx = static_cast<size_t>(b) * p.nHeads + kvHead * p.group + p.colBase + h;
-                if (FOLD == TcFold::kCluster) {
-                    if (d4 == 0) clusterL[h] = lsum;  // (the accumulators stay where they are, in oS)
+                if constexpr (CLUSTER) {
+                    inboxPush<32>(inbox, tid, foldPer, clusterRank(), M, lsum, acc);
                 } else if (p.directOut) {
                     const float inv = lsum > 0.0f ? 1.0f / lsum : 0.0f;
                     *reinterpret_cast<float4 *>(p.out + oidx * 128u + 4u * d4) =
@@ -722,46 +727,20 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     }
     if (threadIdx.x == 0) TC_STAMP(12);
     tcFenceBefore();
-    if (FOLD == TcFold::kCluster) {
-        // every block of the cluster has its accumulators, reference points and row sums in place: rank r puts together and
-        // stores the r-th share of the 8 x 128 outputs
+    if constexpr (CLUSTER) {
+        // every block's results are in the inboxes of the blocks that put them together
+        if (warp >= kFoldWarp0) clusterHelloWait();
         clusterSync();
-        const uint32_t n = clusterSize(), per = 256u / n, base = smemAddr(smem + L::kP);
-        if (threadIdx.x < per) {
-            const uint32_t idx = clusterRank() * per + threadIdx.x, h = idx >> 5, d4 = idx & 31u;
-            if (p.colBase + h < p.group) {
-                float m[16], ls[16];
-                float4 a[16];
-#pragma unroll
-                for (uint32_t r = 0; r < 16; ++r) {
-                    m[r] = kNegBig, ls[r] = 0.0f, a[r] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (r < n) {
-                        const uint32_t q = mapRank(base, r);
-                        m[r] = ldCluster(q + (8 * 128 + h) * 4);
-                        ls[r] = ldCluster(q + (8 * 128 + 8 + 8 * NWG + 32 * NWG + h) * 4);
-                        a[r] = ldCluster4(q + (h * 128 + 4 * d4) * 4);
-                    }
-                }
-                float M = m[0], lsum = 0.0f;
-#pragma unroll
-                for (uint32_t r = 1; r < 16; ++r) M = fmaxf(M, m[r]);
-                float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-                for (uint32_t r = 0; r < 16; ++r) {
-                    const float w = fastExp2(m[r] - M);
-                    lsum = fmaf(w, ls[r], lsum);
-                    acc.x = fmaf(w, a[r].x, acc.x);
-                    acc.y = fmaf(w, a[r].y, acc.y);
-                    acc.z = fmaf(w, a[r].z, acc.z);
-                    acc.w = fmaf(w, a[r].w, acc.w);
-                }
-                const float inv = lsum > 0.0f ? 1.0f / lsum : 0.0f;
-                const size_t oidx = static_cast<size_t>(b) * p.nHeads + kvHead * p.group + p.colBase + h;
-                *reinterpret_cast<float4 *>(p.out + oidx * 128u + 4u * d4) =
-                        make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
-            }
+        const uint32_t idx = clusterRank() * foldPer + threadIdx.x;
+        if (threadIdx.x < foldPer && idx < foldTotal) {
+            float M, l;
+            float4 acc;
+            inboxTake<32>(inbox, threadIdx.x, foldPer, clusterSize(), M, l, acc);
+            const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+            const size_t oidx = static_cast<size_t>(b) * p.nHeads + kvHead * p.group + p.colBase + (idx >> 5);
+            *reinterpret_cast<float4 *>(p.out + oidx * 128u + 4u * (idx & 31u)) =
+                    make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
         }
-        clusterSync();  // nobody leaves while its shared memory may still be read
     }
     __syncthreads();
     if (warp == 0) {

@@ -24,7 +24,7 @@ template <int HD, int NW, int SLOTS>
 struct DecodeKv16Smem {
     static constexpr int kAtomBytes = 16 * 128;      // one half-tile
     static constexpr int kTileBytes = 16 * HD * 2;
-    static constexpr int kSlots = NW * SLOTS * 2 * kTileBytes, kScratch = (NW + 1) * (8 * HD + 16) * 4;  // (the fold reuses the slots)
+    static constexpr int kSlots = NW * SLOTS * 2 * kTileBytes, kScratch = NW * (8 * HD + 16) * 4;  // (the fold reuses the slots)
     static constexpr int kTotal = (kSlots > kScratch ? kSlots : kScratch) + 128;
     static_assert(kTotal <= 227 * 1024, "shared memory of an SM");
 };
@@ -69,6 +69,7 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKv16Kernel(const __grid_co
     const uint32_t share = ROWS ? len : (p.devPos ? tokensPerBlock(len, gridDim.x) : p.chunkTokens);
     const uint32_t t0 = ROWS ? 0u : chunk * share;
     if (!ROWS && t0 >= len && clusterSize() == 1) return;
+    if (!ROWS && clusterSize() > 1) clusterHello();
     const uint32_t t1 = min(len, t0 + share);
     const uint32_t nTiles = t0 < t1 ? (t1 - t0 + T - 1) / T : 0u;
     const uint32_t kvHead = ROWS ? hg / p.group : hg;
@@ -79,33 +80,29 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKv16Kernel(const __grid_co
     const uint32_t stride = p.nKV * HD * 2;
     const uint8_t *storeK = static_cast<const uint8_t *>(p.kvK) + static_cast<size_t>(kvHead) * HD * 2;
     const uint8_t *storeV = static_cast<const uint8_t *>(p.kvV) + static_cast<size_t>(kvHead) * HD * 2;
-    auto requestK = [&](uint32_t i) {
-        const uint32_t j = warp + i * NW;
-        if (j < nTiles) {
-            if (!ROWS && p.tok.k != nullptr && j + 1 == nTiles && t1 == len) {
-                // the tile that holds the new token's row: the row goes in first
-                if (p.devPos && pos >= p.totalRows) {  // a device position outside the store: no row written, and said so
-                    if (lane == 0) atomicOr(p.err, kDevErrRowBound);
-                } else {
-                    const size_t at = (static_cast<size_t>(len - 1u) * p.nKV + kvHead) * HD;
-                    appendRow<HD, __half>(p.tok, kvHead, static_cast<__half *>(p.kvK) + at, static_cast<__half *>(p.kvV) + at,
-                                          len - 1u, lane);
-                }
-            }
-            copyTile<T, HD * 2>(smemAddr(slotK(i)), storeK, stride, t0 + j * T, p.totalRows - 1, lane);
-        }
+    // the warp that takes the last tile stores the token's row; into the tile itself when that is among its first ones
+    const bool append = !ROWS && p.tok.k != nullptr && t1 == len && nTiles != 0;
+    const bool outside = append && p.devPos && pos >= p.totalRows;  // a device position outside the store: no row written
+    if (outside && threadIdx.x == 0) atomicOr(p.err, kDevErrRowBound);
+    const bool mine = append && !outside && (nTiles - 1u) % NW == warp;
+    const bool intoTile = mine && (nTiles - 1u) / NW < SLOTS;
+    const uint32_t have = intoTile ? len - 1u : static_cast<uint32_t>(min(static_cast<uint64_t>(len), p.totalRows));
+    auto request = [&](uint32_t i, bool isV) {
+        const uint32_t j = warp + i * NW, row = t0 + j * T;
+        if (j < nTiles)
+            copyTile<T, HD * 2>(smemAddr(slotK(i) + (isV ? L::kTileBytes : 0)), isV ? storeV : storeK, stride, row,
+                                have > row ? have - row : 0u, lane);
         cpAsyncCommit();
     };
-    auto requestV = [&](uint32_t i) {
-        const uint32_t j = warp + i * NW;
-        if (j < nTiles) copyTile<T, HD * 2>(smemAddr(slotK(i) + L::kTileBytes), storeV, stride, t0 + j * T, p.totalRows - 1, lane);
-        cpAsyncCommit();
-    };
+    auto requestK = [&](uint32_t i) { request(i, false); };
+    auto requestV = [&](uint32_t i) { request(i, true); };
 #pragma unroll
     for (uint32_t i = 0; i < SLOTS; ++i) {
         requestK(i);
         requestV(i);
     }
+    NewRow<HD> fresh;
+    if (mine) fresh.load(p.tok, kvHead, len - 1u, lane);
 
     const uint32_t g = lane >> 2, t = lane & 3u;
     auto colValid = [&](uint32_t j) { return ROWS ? (b * 8u + j < p.qRows) : (p.colBase + j < p.group); };
@@ -173,6 +170,14 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKv16Kernel(const __grid_co
     const float cs0 = __shfl_sync(0xffffffffu, headScale, (2 * t) * 4);
     const float cs1 = __shfl_sync(0xffffffffu, headScale, (2 * t + 1) * 4);
     const uint32_t len0 = colLen(2 * t), len1 = colLen(2 * t + 1);
+
+    if (mine) {
+        const size_t at = (static_cast<size_t>(len - 1u) * p.nKV + kvHead) * HD;
+        uint8_t *tile = intoTile ? slotK((nTiles - 1u) / NW) : nullptr;
+        fresh.store(p.tok.cosT != nullptr, static_cast<__half *>(p.kvK) + at, static_cast<__half *>(p.kvV) + at, tile,
+                    tile + L::kTileBytes, len - 1u - (t0 + (nTiles - 1u) * T), lane);
+        __syncwarp();
+    }
 
     float m0 = kNegBig, m1 = kNegBig, l0 = 0.0f, l1 = 0.0f;
     float o[NS][4];
