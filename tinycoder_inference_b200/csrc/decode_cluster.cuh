@@ -131,6 +131,12 @@ int decodeKvToken(const float *q, const void *kvK, const void *kvV, float *attnO
                   uint32_t numChunks, float invSqrt, int kvHalf, uint8_t *q81Out, const NewToken &tok, cudaStream_t st);
 int decodeKv16(const DecodeKvParams &prm, uint32_t hd, uint8_t *q81Out, cudaStream_t st);
 int prefillKv16(DecodeKvParams prm, uint32_t hd, cudaStream_t st);
+// causal rows over either store in blocks of 32 (prefill_exact.cu), and whether they beat the 8-row form; arguments
+// already validated
+bool prefillExactWins(uint32_t rows, uint64_t before, uint32_t nHeads, uint32_t hd, int kvHalf);
+int prefillExact(const float *q, const void *kvK, const void *kvV, float *out, uint32_t seqLen, uint32_t nHeads,
+                 uint32_t nKV, uint32_t hd, uint32_t cachePos, const uint32_t *devPos, uint64_t totalRows, float invSqrt,
+                 int kvHalf, cudaStream_t st);
 
 #ifdef __CUDACC__
 
