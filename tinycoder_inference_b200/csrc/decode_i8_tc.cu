@@ -29,9 +29,7 @@
 // warps 8-11 the fold warpgroup (thread = head dimension: every tile's integer P.V out of TMEM into
 // one f32 accumulator per head, so a softmax warpgroup's next tile does not wait for the previous
 // one's fold), warp 12 TMA producer (six-stage ring of K, V and their scales), warps 13-16 issue the
-// MMAs (score / P.V products of even / odd tiles: a tcgen05.mma costs its issuing thread about a
-// hundred cycles whatever its shape, threads of different warps issue concurrently).  Partials
-// leave in the reference's layout for the merge kernel (merge.cu).
+// MMAs (score / P.V products of even / odd tiles; one elected thread of each).  Partials leave in the reference's layout for the merge kernel (merge.cu).
 #include <cstdlib>
 
 #include "tc_tcgen05.cuh"
@@ -121,14 +119,12 @@ __host__ __device__ constexpr uint32_t tcIdescI8(uint32_t M, uint32_t N, uint32_
                                                  uint32_t bSigned) {
     return (2u << 4) | (aSigned << 7) | (bSigned << 10) | (aMN << 15) | (bMN << 16) | ((N >> 3) << 17) | ((M >> 4) << 24);
 }
-__device__ __forceinline__ void tcMmaI8If(uint32_t issue, uint32_t dTmem, uint64_t aDesc, uint64_t bDesc, uint32_t idesc,
-                                          uint32_t accumulate) {
+__device__ __forceinline__ void tcMmaI8(uint32_t dTmem, uint64_t aDesc, uint64_t bDesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-            "{\n\t.reg .pred p, q;\n\t"
+            "{\n\t.reg .pred p;\n\t"
             "setp.ne.b32 p, %4, 0;\n\t"
-            "setp.ne.b32 q, %5, 0;\n\t"
-            "@q tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(dTmem),
-            "l"(aDesc), "l"(bDesc), "r"(idesc), "r"(accumulate), "r"(issue)
+            "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(dTmem),
+            "l"(aDesc), "l"(bDesc), "r"(idesc), "r"(accumulate)
             : "memory");
 }
 __device__ __forceinline__ void tmemLd16(uint32_t taddr, uint32_t (&r)[16]) {
@@ -177,7 +173,7 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     constexpr uint32_t kEndThreads = 32u * kProducerWarp;   // softmax + fold threads
     constexpr uint32_t T = kTcTile;
     const uint32_t chunk = blockIdx.x, kvHead = blockIdx.y, b = blockIdx.z;
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31u;
 
     extern __shared__ uint8_t smemRaw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
@@ -344,11 +340,9 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         if (p.prefetchNext && lane == 0) prefetchNextPools();
     } else if (warp > kProducerWarp) {
         // -------------------------------- MMA issuers --------------------------------
-        // One tcgen05.mma costs its issuing thread about a hundred cycles whatever its shape, and
-        // threads of different warps issue concurrently: four issuing warps -- score products and
-        // P.V products of the even (warpgroup 0) and of the odd (warpgroup 1) tiles.  Warp-uniform
-        // control flow; lane 0 executes the tcgen05 instructions.
-        const uint32_t issue = lane == 0 ? 1u : 0u;
+        // Four issuing warps, so that no wait stands in front of another tile's products: score products and P.V products of
+        // the even (warpgroup 0) and of the odd (warpgroup 1) tiles.  Warp-uniform control flow; the elected thread
+        // executes the tcgen05 instructions.
         const uint32_t par = (warp - kMmaWarp0) & 1u;       // which tiles: j = par, par + 2, ...
         const bool pvRole = warp >= kMmaWarp0 + 2u;
         if (!pvRole) {
@@ -367,10 +361,13 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
                 tcFenceAfter();
                 const uint64_t dK = tcDesc(smemAddr(smem + s * L::kStageBytes), 16, 1024, 2);
                 const uint32_t tS = tmemBase + 32u * (2u * w + bb);
+                if (electOne()) {
 #pragma unroll
-                for (uint32_t k = 0; k < 4; ++k)  // 32 dims per instruction = 32 bytes inside the swizzle span
-                    tcMmaI8If(issue, tS, dK + ((k * 32u) >> 4), dQd + ((k * 32u) >> 4), idQK, k > 0 ? 1u : 0u);
-                umaCommitIf(issue, &sFull[2u * w + bb]);
+                    for (uint32_t k = 0; k < 4; ++k)  // 32 dims per instruction = 32 bytes inside the swizzle span
+                        tcMmaI8(tS, dK + ((k * 32u) >> 4), dQd + ((k * 32u) >> 4), idQK, k > 0 ? 1u : 0u);
+                    umaCommit(&sFull[2u * w + bb]);
+                }
+                __syncwarp();
             }
         } else {
             constexpr uint32_t idPV = tcIdescI8(128, 32, 1, 1, 1, 0);   // MN-major A (V tile), MN-major unsigned B (p digits)
@@ -387,13 +384,16 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
                 const uint64_t dV = tcDesc(smemAddr(smem + s * L::kStageBytes + L::kTileBytes), 16, 1024, 2);
                 const uint64_t dP = tcDesc(smemAddr(smem + L::kP + (2u * w + bb) * 4096u), 16, 256, 6);
                 const uint32_t tO = tmemBase + 64u * kWG + 32u * (2u * w + bb);
+                if (electOne()) {
 #pragma unroll
-                for (uint32_t k = 0; k < 4; ++k)  // 32 tokens per instruction: 4096 B of V, 1024 B of P
-                    tcMmaI8If(issue, tO, dV + ((k * 4096u) >> 4), dP + ((k * 1024u) >> 4), idPV, k > 0 ? 1u : 0u);
-                umaCommitIf(issue, &oFull[2u * w + bb]);
-                // K and V of the stage are consumed once these products are done (the score product
-                // of the tile completed before its P could be written)
-                umaCommitIf(issue, &emptyBar[s]);
+                    for (uint32_t k = 0; k < 4; ++k)  // 32 tokens per instruction: 4096 B of V, 1024 B of P
+                        tcMmaI8(tO, dV + ((k * 4096u) >> 4), dP + ((k * 1024u) >> 4), idPV, k > 0 ? 1u : 0u);
+                    umaCommit(&oFull[2u * w + bb]);
+                    // K and V of the stage are consumed once these products are done (the score product
+                    // of the tile completed before its P could be written)
+                    umaCommit(&emptyBar[s]);
+                }
+                __syncwarp();
                 if (lane == 0) TC_STAMP(16);
             }
         }

@@ -31,8 +31,7 @@
 //   warps 9, 10  issue the score products of tile A / B: S_X(t) = Q_X K^T (M128 N64 K16 per
 //              instruction), tcgen05.commit onto the softmax warps' barrier;
 //   warps 11, 12  issue the P.V products of tile A / B: O_X += P_X(t) V (A from TMEM, B = V
-//              MN-major from shared memory).  Issuing an instruction costs its thread about a
-//              hundred cycles and threads of different warps issue concurrently, hence four warps.
+//              MN-major from shared memory).  One elected thread of each issues (tc_tcgen05.cuh).
 // S is DOUBLE-BUFFERED per query tile: S_X(t+2) goes into the buffer P_X(t) leaves once its P.V
 // product is complete, so S_X(t+1) is there when the softmax of tile t finishes.  TMEM (512
 // columns): O_A, O_B (128 each, f32; one O of 256 at head_dim 256), S_{A,0}, S_{A,1}, S_{B,0},
@@ -387,7 +386,7 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
              *exFull = itemFull + 4, *exRead = exFull + 1;
     uint32_t *tmemSlot = reinterpret_cast<uint32_t *>(smem + L::kTmemSlot);
     volatile uint32_t *itemSlots = reinterpret_cast<volatile uint32_t *>(smem + L::kItemSlots);  // [4]
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31u;
     const bool split = !kOne && p.split != 0;
 
     if (threadIdx.x == 0) {
@@ -519,17 +518,15 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         }
     } else if (warp >= 9) {
         // ------------------------------- MMA issuers -------------------------------
-        // Issuing one tcgen05.mma costs its thread about a hundred cycles whatever the shape, and
-        // threads of different warps issue concurrently.  So the score products and the P.V products
-        // of a query tile have an issuing warp each: warp 9 + X issues S_X(t) = Q_X K^T (M128 N64
+        // The score products and the P.V products of a query tile have an issuing warp each, so that no wait stands in front
+        // of the other tile's products: warp 9 + X issues S_X(t) = Q_X K^T (M128 N64
         // K16 x8), warp 11 + X issues O_X += P_X(t) V (A from TMEM, B = V MN-major from shared
         // memory, K16 x4).  t counts the tiles of X over all items; tile t uses score buffer t % 2,
         // and S_X(t+2) goes into the buffer P_X(t) occupies: the score warp waits for the commit of
         // that P.V product (pvBuf) before it issues.
-        // All 32 lanes run this warp-uniform code; only lane 0 executes the tcgen05 instructions.
+        // All 32 lanes run this warp-uniform code; the elected one executes the tcgen05 instructions.
         const uint32_t x = (warp - 9u) & 1u;
         const bool pvRole = warp >= 11u;
-        const uint32_t issue = lane == 0 ? 1u : 0u;
         constexpr uint32_t idQK = umaInstrDescF16(kPfBM, BN, 0, 0);
         constexpr uint32_t idPV = umaInstrDescF16(kPfBM, HD, 0, 1);
         const uint64_t dQ = umaSmemDesc(smemAddr(smem + L::kQ + (split ? 0u : x) * L::kQTile), 16, 1024);
@@ -560,18 +557,23 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                         if (!ok) break;
                         tcFenceAfter();
                         const uint64_t dK = descAdvance(dK0, s * L::kKvTile);
+                        if (electOne()) {
 #pragma unroll
-                        for (uint32_t ks = 0; ks < HD / 16; ++ks) {
-                            // k step ks: dims 16 ks .. +15 = 32 bytes inside the (ks >> 2)-th 64-dim half
-                            umaMmaSSIf(issue, tS0 + 64u * (tt & 1u), descAdvance(dQ, (ks >> 2) * L::kQHalf + (ks & 3u) * 32u),
-                                       descAdvance(dK, (ks >> 2) * L::kKvHalf + (ks & 3u) * 32u), idQK, ks > 0 ? 1u : 0u);
+                            for (uint32_t ks = 0; ks < HD / 16; ++ks) {
+                                // k step ks: dims 16 ks .. +15 = 32 bytes inside the (ks >> 2)-th 64-dim half
+                                umaMmaSS(tS0 + 64u * (tt & 1u), descAdvance(dQ, (ks >> 2) * L::kQHalf + (ks & 3u) * 32u),
+                                         descAdvance(dK, (ks >> 2) * L::kKvHalf + (ks & 3u) * 32u), idQK, ks > 0 ? 1u : 0u);
+                            }
+                            umaCommit(&sFull[2u * x + (tt & 1u)]);
+                            // the item's last score product: the query tiles may be replaced once it is complete
+                            if (tt + 1u == t + myTiles) umaCommit(&qFree[x]);
+                            umaCommit(&kEmpty[s]);
+                            PF_STAMP(2u + x, j, 2);
                         }
-                        umaCommitIf(issue, &sFull[2u * x + (tt & 1u)]);
-                        if (lane == 0) PF_STAMP(2u + x, j, 2);
-                        // the item's last score product: the query tiles may be replaced once it is complete
-                        if (tt + 1u == t + myTiles) umaCommitIf(issue, &qFree[x]);
+                    } else if (ok && electOne()) {
+                        umaCommit(&kEmpty[s]);
                     }
-                    if (ok) umaCommitIf(issue, &kEmpty[s]);
+                    __syncwarp();
                 } else {
                     const uint32_t s = gg % NV;
                     ok = pfWait(&vFull[s], (gg / NV) & 1u, p.err, kDevErrFullWait);
@@ -583,14 +585,19 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                         tcFenceAfter();
                         const uint64_t dV = descAdvance(dV0, s * L::kKvTile);
                         const uint32_t tP = tS0 + 64u * (tt & 1u);
+                        if (electOne()) {
 #pragma unroll
-                        for (uint32_t ks = 0; ks < BN / 16; ++ks)  // 16 tokens per step: 8 columns of fp16 P, 2 KB of V
-                            umaMmaTSIf(issue, tO, tP + ks * 8u, descAdvance(dV, ks * 2048u), idPV, (tt > t || ks > 0) ? 1u : 0u);
-                        umaCommitIf(issue, &pvDone[x]);
-                        umaCommitIf(issue, &pvBuf[2u * x + (tt & 1u)]);
-                        if (lane == 0) PF_STAMP(4u + x, j, 2);
+                            for (uint32_t ks = 0; ks < BN / 16; ++ks)  // 16 tokens per step: 8 columns of fp16 P, 2 KB of V
+                                umaMmaTS(tO, tP + ks * 8u, descAdvance(dV, ks * 2048u), idPV, (tt > t || ks > 0) ? 1u : 0u);
+                            umaCommit(&pvBuf[2u * x + (tt & 1u)]);
+                            umaCommit(&pvDone[x]);
+                            umaCommit(&vEmpty[s]);
+                            PF_STAMP(4u + x, j, 2);
+                        }
+                    } else if (ok && electOne()) {
+                        umaCommit(&vEmpty[s]);
                     }
-                    if (ok) umaCommitIf(issue, &vEmpty[s]);
+                    __syncwarp();
                 }
             }
             // A half without tiles still hands in its phase of qFree, one per item -- but only behind the item's last
@@ -599,7 +606,8 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             // (A split item without odd tiles has one tile: its own full barrier stands for the last K tile.)
             if (!pvRole && myTiles == 0u && ok) {
                 if (split) ok = pfWait(&kFull[g % NK], (g / NK) & 1u, p.err, kDevErrFullWait);
-                if (ok) umaCommitIf(issue, &qFree[x]);
+                if (ok && electOne()) umaCommit(&qFree[x]);
+                __syncwarp();
             }
             t += myTiles;
             g += it.nTiles;
