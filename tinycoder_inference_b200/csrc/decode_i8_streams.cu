@@ -110,7 +110,7 @@ decodeI8StreamsKernel(const __grid_constant__ DecodeI8Params p) {
         auto requestV = [&](uint32_t i) {
             if (ok && i < n) {
                 // the slot's tile of a round before has been folded by everybody
-                if (i >= NSLOT) ok = mbarWaitClock(&emptyBar[i % NSLOT], (i / NSLOT - 1u) & 1u, p.err, kDevErrEmptyWait);
+                if (i >= NSLOT) ok = mbarWait(&emptyBar[i % NSLOT], (i / NSLOT - 1u) & 1u, p.err, kDevErrEmptyWait);
                 request(i, true);
             }
             cpAsyncCommit();
@@ -233,7 +233,7 @@ decodeI8StreamsKernel(const __grid_constant__ DecodeI8Params p) {
         // ---------------------------------- accumulators ----------------------------------
         const uint32_t cp0 = (warp - SW) * CP;  // dims 32 cp0 .. 32 (cp0 + CP) - 1
         for (uint32_t i = 0; i < n; ++i) {
-            if (!mbarWaitClock(&fullBar[i % NSLOT], (i / NSLOT) & 1u, p.err, kDevErrFullWait)) break;
+            if (!mbarWait(&fullBar[i % NSLOT], (i / NSLOT) & 1u, p.err, kDevErrFullWait)) break;
             const uint8_t *rec = record(i);
             const float *fac = reinterpret_cast<const float *>(rec + kRecF);
             uint4 b[MT];
@@ -276,7 +276,7 @@ decodeI8StreamsKernel(const __grid_constant__ DecodeI8Params p) {
         // ---------------------------------- row sums ----------------------------------
         float l0 = 0.0f, l1 = 0.0f, ps0 = 0.0f, ps1 = 0.0f;
         for (uint32_t i = 0; i < n; ++i) {
-            if (!mbarWaitClock(&fullBar[i % NSLOT], (i / NSLOT) & 1u, p.err, kDevErrFullWait)) break;
+            if (!mbarWait(&fullBar[i % NSLOT], (i / NSLOT) & 1u, p.err, kDevErrFullWait)) break;
             const uint8_t *rec = record(i);
             const float *fac = reinterpret_cast<const float *>(rec + kRecF);
             const float *recP = reinterpret_cast<const float *>(rec + kRecP) + lane;

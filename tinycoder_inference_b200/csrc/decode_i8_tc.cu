@@ -278,7 +278,7 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         bool waited = !earlyOk;
         auto requestTile = [&](uint32_t it) -> bool {
             const uint32_t s = it % NS;
-            if (it >= NS && !mbarWaitClock(&emptyBar[s], ((it / NS) - 1u) & 1u, p.err, kDevErrEmptyWait)) return false;
+            if (it >= NS && !mbarWait(&emptyBar[s], ((it / NS) - 1u) & 1u, p.err, kDevErrEmptyWait)) return false;
             const uint32_t tok = t0 + it * T;
             if (!waited && (tok + T > p.prefetchRows || it >= p.earlyStages)) {
                 // rows the kernel in front may still be writing, or further ahead of the dependency
@@ -353,14 +353,14 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         if (!pvRole) {
             constexpr uint32_t idQK = tcIdescI8(128, 32, 0, 0, 1, 1);   // K-major A (K tile), K-major B (q digits)
             const uint64_t dQd = tcDesc(smemAddr(smem + L::kQd), 16, 1024, 2);
-            bool ok = mbarWaitClock(qFull, 0, p.err, kDevErrFullWait);
+            bool ok = mbarWait(qFull, 0, p.err, kDevErrFullWait);
             if (lane == 0 && par == 0) TC_STAMP(15);
             for (uint32_t j = par; ok && j < nTiles; j += 2u) {
                 const uint32_t s = j % NS, w = j % kWG, bb = (j / kWG) & 1u;
                 // the S buffer's previous contents (tile j - 2 NWG) have been read once that tile's P is out
                 if (j >= 2u * kWG)
-                    ok = mbarWaitClock(&pFull[2u * w + bb], ((j - 2u * kWG) / (2u * kWG)) & 1u, p.err, kDevErrMmaWait);
-                ok = ok && mbarWaitClock(&fullBar[s], (j / NS) & 1u, p.err, kDevErrFullWait);
+                    ok = mbarWait(&pFull[2u * w + bb], ((j - 2u * kWG) / (2u * kWG)) & 1u, p.err, kDevErrMmaWait);
+                ok = ok && mbarWait(&fullBar[s], (j / NS) & 1u, p.err, kDevErrFullWait);
                 if (lane == 0 && j < 8u) TC_STAMP(20 + j);
                 if (!ok) break;
                 tcFenceAfter();
@@ -380,10 +380,10 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
             for (uint32_t j = par; ok && j < nTiles; j += 2u) {
                 const uint32_t s = j % NS, w = j % kWG, bb = (j / kWG) & 1u;
                 // P of tile j published
-                ok = mbarWaitClock(&pFull[2u * w + bb], (j / (2u * kWG)) & 1u, p.err, kDevErrMmaWait);
+                ok = mbarWait(&pFull[2u * w + bb], (j / (2u * kWG)) & 1u, p.err, kDevErrMmaWait);
                 // and the fold warpgroup has read the O buffer's previous contents (tile j - 2 NWG)
                 if (ok && j >= 2u * kWG)
-                    ok = mbarWaitClock(&oFree[2u * w + bb], ((j - 2u * kWG) / (2u * kWG)) & 1u, p.err, kDevErrMmaWait);
+                    ok = mbarWait(&oFree[2u * w + bb], ((j - 2u * kWG) / (2u * kWG)) & 1u, p.err, kDevErrMmaWait);
                 if (!ok) break;
                 tcFenceAfter();
                 const uint64_t dV = tcDesc(smemAddr(smem + s * L::kStageBytes + L::kTileBytes), 16, 1024, 2);
@@ -418,7 +418,7 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         bool ok = true;
         for (uint32_t j = 0; ok && j < nTiles; ++j) {
             const uint32_t w = j % kWG, bb = (j / kWG) & 1u, par = (j / (2u * kWG)) & 1u;
-            ok = mbarWaitClock(&oFull[2u * w + bb], par, p.err, kDevErrMmaWait);
+            ok = mbarWait(&oFull[2u * w + bb], par, p.err, kDevErrMmaWait);
             if (!ok) break;
             tcFenceAfter();
             uint32_t r[32];
@@ -528,7 +528,7 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         for (uint32_t j = w; j < nTiles; j += kWG) {
             const uint32_t s = j % NS, bb = (j / kWG) & 1u;
             // ---- this thread's token against the 8 heads ----
-            if (!mbarWaitClock(&sFull[2u * w + bb], (j / (2u * kWG)) & 1u, p.err, kDevErrMmaWait)) {
+            if (!mbarWait(&sFull[2u * w + bb], (j / (2u * kWG)) & 1u, p.err, kDevErrMmaWait)) {
                 ok = false;
                 break;
             }
@@ -596,7 +596,7 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
             // P.V product is complete and folded once the fold warpgroup has said so on oFree (long
             // ago, as a rule: two tiles of this warpgroup lie in between).
             if (j >= 2u * kWG &&
-                !mbarWaitClock(&oFree[2u * w + bb], ((j - 2u * kWG) / (2u * kWG)) & 1u, p.err, kDevErrMmaWait)) {
+                !mbarWait(&oFree[2u * w + bb], ((j - 2u * kWG) / (2u * kWG)) & 1u, p.err, kDevErrMmaWait)) {
                 ok = false;
                 break;
             }

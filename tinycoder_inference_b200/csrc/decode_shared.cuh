@@ -41,16 +41,14 @@ int decodeI8Streams(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenA
 int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, const F32Mirror &mir, cudaStream_t st);
 
 #ifdef __CUDACC__
-__device__ __forceinline__ bool mbarWaitClock(uint64_t *bar, uint32_t parity, unsigned int *err,
-                                              uint32_t errBit) {
-    // ~2^31 cycles (about a second) before giving up.
-    const long long t0 = clock64();
-    for (;;) {
+// Bounded wait: the first poll, which most waits need alone, in front of a loop of up to 2^18 more, each parked for up to
+// 20 us by the hardware.  (A loop that reads the clock: captured int8 step of 28 / 4 / 128 at 12000 rows 23.6 us per layer
+// against 23.0, 8 sequences of 4098 rows 9.95 against 9.83.)
+__device__ __forceinline__ bool mbarWait(uint64_t *bar, uint32_t parity, unsigned int *err, uint32_t errBit) {
+    if (mbarTryWait(bar, parity)) return true;
 #pragma unroll 1
-        for (int i = 0; i < 256; ++i)
-            if (mbarTryWait(bar, parity)) return true;
-        if (clock64() - t0 > (1ll << 31)) break;
-    }
+    for (uint32_t i = 0; i < (1u << 18); ++i)
+        if (mbarTryWait(bar, parity)) return true;
     atomicOr(err, errBit);
     return false;
 }

@@ -298,19 +298,29 @@ struct PrefillF16Smem {
     static_assert(kTotal <= 227 * 1024, "shared memory of an SM");
 };
 
-__device__ __forceinline__ bool pfWait(uint64_t *bar, uint32_t parity, unsigned int *err, uint32_t bit) {
-    const long long t0 = clock64();
-    for (;;) {
+// Bounded wait: 2^18 polls, each parked for up to 20 us by the hardware.
+__device__ __forceinline__ bool pfPoll(uint64_t *bar, uint32_t parity, unsigned int *err, uint32_t bit) {
 #pragma unroll 1
-        for (int i = 0; i < 128; ++i)
-            if (mbarTryWait(bar, parity)) return true;
+    for (uint32_t i = 0; i < (1u << 18); ++i) {
+        if (mbarTryWait(bar, parity)) return true;
         // somebody has already given up: what this thread waits for will not come either
-        if ((*reinterpret_cast<volatile unsigned int *>(err) & (kDevErrFullWait | kDevErrEmptyWait | kDevErrMmaWait)) != 0u)
+        if ((i & 63u) == 63u &&
+            (*reinterpret_cast<volatile unsigned int *>(err) & (kDevErrFullWait | kDevErrEmptyWait | kDevErrMmaWait)) != 0u)
             return false;
-        if (clock64() - t0 > (1ll << 31)) break;
     }
     atomicOr(err, bit);
     return false;
+}
+static __device__ __noinline__ bool pfPollCall(uint64_t *bar, uint32_t parity, unsigned int *err, uint32_t bit) {
+    return pfPoll(bar, parity, err, bit);
+}
+// Most waits find their phase complete, a step's chain goes through five of them, and their code sits in the middle of long
+// unrolled loops: the first poll stands alone and the loop behind it is a call.  Launch of 4096 rows of 28 / 4 / 128 (rows
+// launch included) 139.6 us with a loop that reads the clock, 135.3 with the first poll in front of a short loop,
+// 130.0 with that loop as a call; 512 rows behind 3584 49.7, 43.7 and 43.4.
+template <bool CALL>
+__device__ __forceinline__ bool pfWait(uint64_t *bar, uint32_t parity, unsigned int *err, uint32_t bit) {
+    return mbarTryWait(bar, parity) || (CALL ? pfPollCall(bar, parity, err, bit) : pfPoll(bar, parity, err, bit));
 }
 
 // one 32-byte store (the address has to be 32-byte aligned)
@@ -376,6 +386,7 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     constexpr int BN = kPfBN;
     constexpr int NC = BN / 32;  // 32-column chunks of a score row
     constexpr uint32_t NK = L::NK, NV = L::NV;
+    constexpr bool kCall = HD < 256;     // (a call costs the softmax threads of head_dim 256 spills: 68 -> 79 us)
     constexpr bool kOne = L::kQTiles == 1;  // the second half of the block has nothing to do
     extern __shared__ uint8_t smemRaw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
@@ -432,7 +443,7 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     // The n-th item of this block: the producer publishes it in slot n % 4 (the end of the list as
     // an index past the last item); the other roles pick it up there.
     auto takeItem = [&](uint32_t n, uint32_t &item) -> bool {
-        if (!pfWait(&itemFull[n & 3u], (n >> 2) & 1u, p.err, kDevErrFullWait)) return false;
+        if (!pfWait<kCall>(&itemFull[n & 3u], (n >> 2) & 1u, p.err, kDevErrFullWait)) return false;
         item = itemSlots[n & 3u];
         return item < p.totalItems;
     };
@@ -448,7 +459,7 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             bool ok = true;
             auto requestK = [&](uint32_t kvHead, uint32_t j) {
                 const uint32_t s = gk % NK;
-                if (gk >= NK && !pfWait(&kEmpty[s], ((gk / NK) - 1u) & 1u, p.err, kDevErrEmptyWait)) return false;
+                if (gk >= NK && !pfWait<kCall>(&kEmpty[s], ((gk / NK) - 1u) & 1u, p.err, kDevErrEmptyWait)) return false;
                 mbarExpectTx(&kFull[s], L::kKvTile);
 #pragma unroll
                 for (int h = 0; h < L::kHalves; ++h)
@@ -458,7 +469,7 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             };
             auto requestV = [&](uint32_t kvHead, uint32_t j) {
                 const uint32_t s = gv % NV;
-                if (gv >= NV && !pfWait(&vEmpty[s], ((gv / NV) - 1u) & 1u, p.err, kDevErrEmptyWait)) return false;
+                if (gv >= NV && !pfWait<kCall>(&vEmpty[s], ((gv / NV) - 1u) & 1u, p.err, kDevErrEmptyWait)) return false;
                 mbarExpectTx(&vFull[s], L::kKvTile);
 #pragma unroll
                 for (int h = 0; h < L::kHalves; ++h)
@@ -475,8 +486,8 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 // the query tiles are free once the score warps have issued the last product of the previous item and
                 // those products are complete
                 if (n > 0)
-                    ok = pfWait(&qFree[0], (n - 1u) & 1u, p.err, kDevErrEmptyWait) &&
-                         (kOne || pfWait(&qFree[1], (n - 1u) & 1u, p.err, kDevErrEmptyWait));
+                    ok = pfWait<kCall>(&qFree[0], (n - 1u) & 1u, p.err, kDevErrEmptyWait) &&
+                         (kOne || pfWait<kCall>(&qFree[1], (n - 1u) & 1u, p.err, kDevErrEmptyWait));
                 if (!ok) break;
                 const int qTiles = kOne || split ? 1 : 2;
                 mbarExpectTx(qFull, qTiles * L::kQTile);
@@ -509,11 +520,11 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             // the last release of every slot has to have arrived before the block leaves
             for (uint32_t back = 0; ok && back < NK && back < gk; ++back) {
                 const uint32_t g = gk - 1u - back;
-                ok = pfWait(&kEmpty[g % NK], (g / NK) & 1u, p.err, kDevErrEmptyWait);
+                ok = pfWait<kCall>(&kEmpty[g % NK], (g / NK) & 1u, p.err, kDevErrEmptyWait);
             }
             for (uint32_t back = 0; ok && back < NV && back < gv; ++back) {
                 const uint32_t g = gv - 1u - back;
-                ok = pfWait(&vEmpty[g % NV], (g / NV) & 1u, p.err, kDevErrEmptyWait);
+                ok = pfWait<kCall>(&vEmpty[g % NV], (g / NV) & 1u, p.err, kDevErrEmptyWait);
             }
         }
     } else if (warp >= 9) {
@@ -549,11 +560,11 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 const bool mine = split || j < myTiles;
                 if (!pvRole) {
                     const uint32_t s = gg % NK;
-                    if (mine && j == j0) ok = pfWait(qFull, n & 1u, p.err, kDevErrFullWait);
+                    if (mine && j == j0) ok = pfWait<kCall>(qFull, n & 1u, p.err, kDevErrFullWait);
                     if (lane == 0) PF_STAMP(2u + x, j, 0);
-                    ok = ok && pfWait(&kFull[s], (gg / NK) & 1u, p.err, kDevErrFullWait);
+                    ok = ok && pfWait<kCall>(&kFull[s], (gg / NK) & 1u, p.err, kDevErrFullWait);
                     if (mine) {
-                        if (ok && tt >= 2u) ok = pfWait(&pvBuf[2u * x + (tt & 1u)], ((tt - 2u) >> 1) & 1u, p.err, kDevErrMmaWait);
+                        if (ok && tt >= 2u) ok = pfWait<kCall>(&pvBuf[2u * x + (tt & 1u)], ((tt - 2u) >> 1) & 1u, p.err, kDevErrMmaWait);
                         if (!ok) break;
                         tcFenceAfter();
                         const uint64_t dK = descAdvance(dK0, s * L::kKvTile);
@@ -576,10 +587,10 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                     __syncwarp();
                 } else {
                     const uint32_t s = gg % NV;
-                    ok = pfWait(&vFull[s], (gg / NV) & 1u, p.err, kDevErrFullWait);
+                    ok = pfWait<kCall>(&vFull[s], (gg / NV) & 1u, p.err, kDevErrFullWait);
                     if (mine) {
                         if (lane == 0) PF_STAMP(4u + x, j, 0);
-                        ok = ok && pfWait(&pFull[2u * x + (tt & 1u)], (tt >> 1) & 1u, p.err, kDevErrMmaWait);
+                        ok = ok && pfWait<kCall>(&pFull[2u * x + (tt & 1u)], (tt >> 1) & 1u, p.err, kDevErrMmaWait);
                         if (lane == 0) PF_STAMP(4u + x, j, 1);
                         if (!ok) break;
                         tcFenceAfter();
@@ -605,7 +616,7 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             // complete two phases before the producer has seen the first (a parity wait cannot tell those apart).
             // (A split item without odd tiles has one tile: its own full barrier stands for the last K tile.)
             if (!pvRole && myTiles == 0u && ok) {
-                if (split) ok = pfWait(&kFull[g % NK], (g / NK) & 1u, p.err, kDevErrFullWait);
+                if (split) ok = pfWait<kCall>(&kFull[g % NK], (g / NK) & 1u, p.err, kDevErrFullWait);
                 if (ok && electOne()) umaCommit(&qFree[x]);
                 __syncwarp();
             }
@@ -615,7 +626,7 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         if (pvRole && ok) {
             // nobody waits for the last two buffer commits; they have to land before the block leaves
             for (uint32_t tt = t >= 2u ? t - 2u : 0u; tt < t; ++tt)
-                if (!pfWait(&pvBuf[2u * x + (tt & 1u)], (tt >> 1) & 1u, p.err, kDevErrMmaWait)) break;
+                if (!pfWait<kCall>(&pvBuf[2u * x + (tt & 1u)], (tt >> 1) & 1u, p.err, kDevErrMmaWait)) break;
         }
     } else {
         // --------------------------------- softmax ---------------------------------
@@ -641,7 +652,7 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 const uint32_t kt = split ? 2u * j + x : j;  // KV tile
                 const uint32_t tS = tmemBase + 256u + 128u * x + 64u * b;
                 if (row == 0) PF_STAMP(x, j, 0);
-                if (!pfWait(&sFull[2u * x + b], (tt >> 1) & 1u, p.err, kDevErrMmaWait)) {
+                if (!pfWait<kCall>(&sFull[2u * x + b], (tt >> 1) & 1u, p.err, kDevErrMmaWait)) {
                     ok = false;
                     break;
                 }
@@ -664,18 +675,18 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                         for (int i = 0; i < 32; ++i)
                             if (first + c * 32 + i > static_cast<int32_t>(rowInBlock)) r[c][i] = 0xff800000u;  // -inf
                 }
-                float mxa = -INFINITY, mxb = -INFINITY;
+                float mxs[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
                 for (int c = 0; c < NC; ++c)
 #pragma unroll
-                    for (int i = 0; i < 32; i += 4) {
-                        mxa = max3(mxa, __uint_as_float(r[c][i]), __uint_as_float(r[c][i + 1]));
-                        mxb = max3(mxb, __uint_as_float(r[c][i + 2]), __uint_as_float(r[c][i + 3]));
-                    }
-                const float mx = fmaxf(mxa, mxb) * p.scaleLog2;  // scale > 0: max commutes with it
+                    for (int i = 0; i < 32; i += 8)
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            mxs[u] = max3(mxs[u], __uint_as_float(r[c][i + 2 * u]), __uint_as_float(r[c][i + 2 * u + 1]));
+                const float mx = fmaxf(fmaxf(mxs[0], mxs[1]), fmaxf(mxs[2], mxs[3])) * p.scaleLog2;  // scale > 0: max commutes with it
                 const float mNew = mx > m + kPfLazyLog2 ? mx : m;
-                const float alpha = fastExp2(m - mNew);
                 const bool rescale = j > 0 && __any_sync(0xffffffffu, mNew != m);
+                float alpha = 1.0f;  // (without a rescale m stays: l is 0 in the first step)
                 if (row == 0 && x == 0) PF_STAMP(6u, j, 1);
                 // O may only be touched between two of its PV products: the previous one has to be
                 // complete (the next one cannot start before this thread publishes P).  The last
@@ -683,13 +694,14 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 // the one before it, and the final wait below must not find the barrier two behind.
                 // (pvDone completes one phase per tile, so its parity follows the running count.)
                 if (j > 0 && (rescale || j + 1u == myTiles)) {
-                    if (!pfWait(&pvDone[x], (tt - 1u) & 1u, p.err, kDevErrMmaWait)) {
+                    if (!pfWait<kCall>(&pvDone[x], (tt - 1u) & 1u, p.err, kDevErrMmaWait)) {
                         ok = false;
                         break;
                     }
                     tcFenceAfter();
                 }
                 if (rescale) {
+                    alpha = fastExp2(m - mNew);
 #pragma unroll 1
                     for (uint32_t c = 0; c < HD / 32; ++c) {
                         uint32_t o[32];
@@ -742,7 +754,7 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 if (row == 0) PF_STAMP(x, j, 2);
                 if (row == 0 && j + 1u == myTiles) PF_BLK(3u + x);
             }
-            ok = ok && (myTiles == 0 || pfWait(&pvDone[x], (t + myTiles - 1u) & 1u, p.err, kDevErrMmaWait));
+            ok = ok && (myTiles == 0 || pfWait<kCall>(&pvDone[x], (t + myTiles - 1u) & 1u, p.err, kDevErrMmaWait));
             if (!ok) break;
             // Split items: each half leaves (m, l) of its rows for the other one and stores half of the dims, out of both
             // accumulators (they lie in the same TMEM lanes).
@@ -752,7 +764,7 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 exch[x * kPfBM + row] = make_float2(m, l);
                 tcFenceBefore();
                 mbarArrive(exFull);
-                ok = pfWait(exFull, n & 1u, p.err, kDevErrMmaWait);
+                ok = pfWait<kCall>(exFull, n & 1u, p.err, kDevErrMmaWait);
                 if (!ok) break;
                 tcFenceAfter();
                 const float2 o = exch[(x ^ 1u) * kPfBM + row];
@@ -816,7 +828,7 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 // the next item's first P.V product may overwrite an accumulator once both halves have read it
                 tcFenceBefore();
                 mbarArrive(exRead);
-                ok = pfWait(exRead, n & 1u, p.err, kDevErrMmaWait);
+                ok = pfWait<kCall>(exRead, n & 1u, p.err, kDevErrMmaWait);
             }
             if (threadIdx.x == 0) PF_BLK(5);
             t += myTiles;

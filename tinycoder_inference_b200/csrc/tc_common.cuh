@@ -117,17 +117,6 @@ __device__ __forceinline__ bool mbarTryWait(uint64_t *bar, uint32_t parity) {
             : "memory");
     return ok != 0;
 }
-// Bounded wait: returns false (and records `errBit`) after ~2^26 failed polls
-// (each poll may itself suspend for a hardware-chosen time), so a lost arrival
-// never turns into an endless spin on a shared GPU.
-__device__ __forceinline__ bool mbarWait(uint64_t *bar, uint32_t parity, unsigned int *err,
-                                         uint32_t errBit) {
-    for (uint32_t i = 0; i < (1u << 26); ++i) {
-        if (mbarTryWait(bar, parity)) return true;
-    }
-    atomicOr(err, errBit);
-    return false;
-}
 __device__ __forceinline__ void fenceBarrierInit() {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
