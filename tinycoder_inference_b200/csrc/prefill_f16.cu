@@ -32,7 +32,7 @@
 //              instruction), tcgen05.commit onto the softmax warps' barrier;
 //   warps 11, 12  issue the P.V products of tile A / B: O_X += P_X(t) V (A from TMEM, B = V
 //              MN-major from shared memory).  One elected thread of each issues (tc_tcgen05.cuh).
-// S is DOUBLE-BUFFERED per query tile: S_X(t+2) goes into the buffer P_X(t) leaves once its P.V
+// S is DOUBLE-BUFFERED per query tile (head_dim 256: kAhead below): S_X(t+2) goes into the buffer P_X(t) leaves once its P.V
 // product is complete, so S_X(t+1) is there when the softmax of tile t finishes.  TMEM (512
 // columns): O_A, O_B (128 each, f32; one O of 256 at head_dim 256), S_{A,0}, S_{A,1}, S_{B,0},
 // S_{B,1} (64 each).  Causality: a query tile only visits KV tiles up to its diagonal, the last
@@ -290,8 +290,8 @@ struct PrefillF16Smem {
     static constexpr int kV = kK + NK * kKvTile;
     static constexpr int kBars = kV + NV * kKvTile;
     // qFull, kFull + kEmpty, vFull + vEmpty, sFull[2][2], pFull[2][2], pvDone[2], pvBuf[2][2], qFree[2], itemFull[4],
-    // exFull, exRead
-    static constexpr int kNumBars = 1 + 2 * NK + 2 * NV + 4 + 4 + 2 + 4 + 2 + 4 + 2;
+    // exFull, exRead, sFree[2]
+    static constexpr int kNumBars = 1 + 2 * NK + 2 * NV + 4 + 4 + 2 + 4 + 2 + 4 + 2 + 2;
     static constexpr int kTmemSlot = kBars + kNumBars * 8;
     static constexpr int kItemSlots = kTmemSlot + 16;  // four work item indices
     static constexpr int kTotal = kItemSlots + 16 + 1024;
@@ -388,13 +388,19 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     constexpr uint32_t NK = L::NK, NV = L::NV;
     constexpr bool kCall = HD < 256;     // (a call costs the softmax threads of head_dim 256 spills: 68 -> 79 us)
     constexpr bool kOne = L::kQTiles == 1;  // the second half of the block has nothing to do
+    // One query tile is a chain of steps; nothing else fills the tensor pipe while it waits.  Its scores take one buffer, free
+    // once they are in the softmax threads' registers, and its probabilities two, so that S(t+1) is computed under the
+    // exponentials of tile t and waits for no P.V product: 512 rows behind 3000 of 16 / 2 / 256 67.7 -> 58.6 us, 2000 rows of
+    // 16 / 4 / 256 55.3 -> 51.0.  With two query tiles the chains fill each other's gaps, and the two waits more per
+    // step cost more than that (4096 rows of 28 / 4 / 128 130 -> 137).
+    constexpr bool kAhead = kOne;
     extern __shared__ uint8_t smemRaw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L::kBars);
     uint64_t *qFull = bars, *kFull = bars + 1, *kEmpty = kFull + NK, *vFull = kEmpty + NK, *vEmpty = vFull + NV,
              *sFull = vEmpty + NV /* [x][b] */, *pFull = sFull + 4 /* [x][b] */, *pvDone = pFull + 4 /* [x] */,
              *pvBuf = pvDone + 2 /* [x][b] */, *qFree = pvBuf + 4 /* [x] */, *itemFull = qFree + 2 /* [4] */,
-             *exFull = itemFull + 4, *exRead = exFull + 1;
+             *exFull = itemFull + 4, *exRead = exFull + 1, *sFree = exRead + 1 /* [x] */;
     uint32_t *tmemSlot = reinterpret_cast<uint32_t *>(smem + L::kTmemSlot);
     volatile uint32_t *itemSlots = reinterpret_cast<volatile uint32_t *>(smem + L::kItemSlots);  // [4]
     const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31u;
@@ -418,8 +424,10 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             mbarInit(&pvBuf[i], 1);
             mbarInit(&itemFull[i], 1);
         }
-        mbarInit(&pvDone[0], 1);
-        mbarInit(&pvDone[1], 1);
+        for (int x = 0; x < 2; ++x) {
+            mbarInit(&sFree[x], 4);  // one arrival per warp
+            mbarInit(&pvDone[x], 1);
+        }
         mbarInit(&qFree[0], 1);  // score warp X is done with the query tiles
         mbarInit(&qFree[1], 1);
         mbarInit(exFull, 2 * kPfBM);  // split items: every softmax thread has left its (m, l) / has read the accumulators
@@ -437,8 +445,8 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     __syncthreads();
     tcFenceAfter();
     const uint32_t tmemBase = *reinterpret_cast<volatile uint32_t *>(tmemSlot);
-    // O of tile X at columns 128 X; S buffer b of tile X at 256 + 128 X + 64 b (its fp16
-    // probabilities overwrite the first 32 of those columns)
+    // O of tile X at columns 128 X; S buffer b of tile X at 256 + 128 X + 64 b, its fp16 probabilities over the first 32 of
+    // those columns.  kAhead: S at 256, the probabilities behind it in two buffers of 32 columns.
 
     // The n-th item of this block: the producer publishes it in slot n % 4 (the end of the list as
     // an index past the last item); the other roles pick it up there.
@@ -534,7 +542,7 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         // K16 x8), warp 11 + X issues O_X += P_X(t) V (A from TMEM, B = V MN-major from shared
         // memory, K16 x4).  t counts the tiles of X over all items; tile t uses score buffer t % 2,
         // and S_X(t+2) goes into the buffer P_X(t) occupies: the score warp waits for the commit of
-        // that P.V product (pvBuf) before it issues.
+        // that P.V product (pvBuf) before it issues.  kAhead: for the softmax threads to have read S(t-1) (sFree).
         // All 32 lanes run this warp-uniform code; the elected one executes the tcgen05 instructions.
         const uint32_t x = (warp - 9u) & 1u;
         const bool pvRole = warp >= 11u;
@@ -564,7 +572,11 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                     if (lane == 0) PF_STAMP(2u + x, j, 0);
                     ok = ok && pfWait<kCall>(&kFull[s], (gg / NK) & 1u, p.err, kDevErrFullWait);
                     if (mine) {
-                        if (ok && tt >= 2u) ok = pfWait<kCall>(&pvBuf[2u * x + (tt & 1u)], ((tt - 2u) >> 1) & 1u, p.err, kDevErrMmaWait);
+                        if (kAhead) {
+                            if (ok && tt >= 1u) ok = pfWait<kCall>(&sFree[x], (tt - 1u) & 1u, p.err, kDevErrMmaWait);
+                        } else if (ok && tt >= 2u) {
+                            ok = pfWait<kCall>(&pvBuf[2u * x + (tt & 1u)], ((tt - 2u) >> 1) & 1u, p.err, kDevErrMmaWait);
+                        }
                         if (!ok) break;
                         tcFenceAfter();
                         const uint64_t dK = descAdvance(dK0, s * L::kKvTile);
@@ -572,10 +584,10 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll
                             for (uint32_t ks = 0; ks < HD / 16; ++ks) {
                                 // k step ks: dims 16 ks .. +15 = 32 bytes inside the (ks >> 2)-th 64-dim half
-                                umaMmaSS(tS0 + 64u * (tt & 1u), descAdvance(dQ, (ks >> 2) * L::kQHalf + (ks & 3u) * 32u),
+                                umaMmaSS(tS0 + (kAhead ? 0u : 64u * (tt & 1u)), descAdvance(dQ, (ks >> 2) * L::kQHalf + (ks & 3u) * 32u),
                                          descAdvance(dK, (ks >> 2) * L::kKvHalf + (ks & 3u) * 32u), idQK, ks > 0 ? 1u : 0u);
                             }
-                            umaCommit(&sFull[2u * x + (tt & 1u)]);
+                            umaCommit(&sFull[kAhead ? x : 2u * x + (tt & 1u)]);
                             // the item's last score product: the query tiles may be replaced once it is complete
                             if (tt + 1u == t + myTiles) umaCommit(&qFree[x]);
                             umaCommit(&kEmpty[s]);
@@ -595,7 +607,7 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                         if (!ok) break;
                         tcFenceAfter();
                         const uint64_t dV = descAdvance(dV0, s * L::kKvTile);
-                        const uint32_t tP = tS0 + 64u * (tt & 1u);
+                        const uint32_t tP = tS0 + (kAhead ? 64u + 32u * (tt & 1u) : 64u * (tt & 1u));
                         if (electOne()) {
 #pragma unroll
                             for (uint32_t ks = 0; ks < BN / 16; ++ks)  // 16 tokens per step: 8 columns of fp16 P, 2 KB of V
@@ -650,9 +662,9 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             for (uint32_t j = 0; j < myTiles; ++j) {
                 const uint32_t tt = t + j, b = tt & 1u;
                 const uint32_t kt = split ? 2u * j + x : j;  // KV tile
-                const uint32_t tS = tmemBase + 256u + 128u * x + 64u * b;
+                const uint32_t tS = tmemBase + 256u + 128u * x + (kAhead ? 0u : 64u * b), tP = kAhead ? tS + 64u + 32u * b : tS;
                 if (row == 0) PF_STAMP(x, j, 0);
-                if (!pfWait<kCall>(&sFull[2u * x + b], (tt >> 1) & 1u, p.err, kDevErrMmaWait)) {
+                if (!pfWait<kCall>(&sFull[kAhead ? x : 2u * x + b], (kAhead ? tt : tt >> 1) & 1u, p.err, kDevErrMmaWait)) {
                     ok = false;
                     break;
                 }
@@ -663,6 +675,11 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll
                 for (int c = 0; c < NC; ++c) tmemLd32(tS + laneBase + 32u * c, r[c]);
                 tmemLdWait();
+                if (kAhead) {
+                    tcFenceBefore();
+                    __syncwarp();
+                    if (lane == 0) mbarArrive(&sFree[x]);  // the next tile's scores may be written
+                }
                 if (row == 0 && x == 0) PF_STAMP(6u, j, 0);
                 if (BN * kt + (BN - 1u) > p.cachePos + m0 + tileRow0) {
                     // causal edge (the tile reaches past the position of this tile's first row): token
@@ -714,8 +731,16 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                     tmemStWait();
                 }
                 m = mNew;
-                // probabilities as fp16 pairs over the first 32 columns of this S buffer: the A
-                // operand of the PV product (every score of the row is already in registers)
+                if (kAhead) {
+                    // the buffer's last probabilities, those of tile t - 2, have been multiplied (long ago as a rule)
+                    if (tt >= 2u && !pfWait<kCall>(&pvBuf[2u * x + b], ((tt - 2u) >> 1) & 1u, p.err, kDevErrMmaWait)) {
+                        ok = false;
+                        break;
+                    }
+                    tcFenceAfter();
+                }
+                // probabilities as fp16 pairs: the A operand of the PV product
+                // (every score of the row is already in registers)
                 // Pairs of elements with packed f32x2 arithmetic (scale-and-shift, row sum).  Evaluating
                 // part of the exponentials on the FMA pipe (round-to-integer trick + cubic) was measured
                 // at 25 / 50 / 75 % of the pairs: 716 / 699 / 694 TFLOP/s against 732 with all of them on
@@ -743,7 +768,7 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                         }
                         psum += sum2.x + sum2.y;
                     }
-                    tmemSt16(tS + laneBase + c * 16u, h);
+                    tmemSt16(tP + laneBase + c * 16u, h);
                     if (row == 0 && x == 0) PF_STAMP(6u, j, 2 + c);
                 }
                 l = l * alpha + psum;
