@@ -350,10 +350,13 @@ static int decodeKv16Hd(const DecodeKvParams &prm, uint8_t *q81Out, cudaStream_t
 // Both are called from decode_kv.cu when kvHalf is set; arguments were validated there.
 // Warps of a block, slots of a warp, blocks per SM: rows beyond what a 16-block cluster covers with one tile per warp
 // (2048) want two tiles of a warp in flight (head_dim 128, per layer: 20000 rows 14.3 against 15.8 us, 47000 rows 24.2
-// against 28.3; 2047 rows 6.0 against 5.9).
+// against 28.3; 2047 rows 6.0 against 5.9).  Half as wide rows beyond what a cluster covers alone want four of them
+// (14 / 2 / 64: 20000 rows 8.2 -> 7.8 us, 47000 10.7 -> 10.1; 12000 rows 6.8 -> 6.9).
 int decodeKv16(const DecodeKvParams &prm, uint32_t hd, uint8_t *q81Out, cudaStream_t st) {
     if (hd == 64)
-        return prm.lenHost <= 2048u ? decodeKv16Hd<64, 8, 1, 2>(prm, q81Out, st) : decodeKv16Hd<64, 8, 2, 1>(prm, q81Out, st);
+        return prm.lenHost <= 2048u    ? decodeKv16Hd<64, 8, 1, 2>(prm, q81Out, st)
+               : prm.lenHost <= 16384u ? decodeKv16Hd<64, 8, 2, 1>(prm, q81Out, st)
+                                       : decodeKv16Hd<64, 8, 4, 1>(prm, q81Out, st);
     return prm.lenHost <= 2048u ? decodeKv16Hd<128, 8, 1, 2>(prm, q81Out, st) : decodeKv16Hd<128, 8, 2, 1>(prm, q81Out, st);
 }
 
