@@ -54,7 +54,7 @@ decodeI8Kernel(const __grid_constant__ DecodeI8Params p) {
     constexpr int NR = 2 * MT;  // 8-token row groups of a warp's tile
     constexpr float k2p24 = kI8Unscale;
 
-    const uint32_t chunk = blockIdx.x, hg = blockIdx.y, b = blockIdx.z;
+    const uint32_t chunk = blockIdx.x, hg = blockIdx.y, b = ROWS ? gridDim.z - 1u - blockIdx.z : blockIdx.z;  // (late rows first)
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
 
     extern __shared__ uint8_t smemRaw[];

@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKvKernel(const __grid_cons
     constexpr int KS = HD / 8;   // tf32 k-steps of the QK product
     constexpr int MTO = HD / 16;  // 16-dim output tiles
 
-    const uint32_t chunk = blockIdx.x, hg = blockIdx.y, b = blockIdx.z;
+    const uint32_t chunk = blockIdx.x, hg = blockIdx.y, b = ROWS ? gridDim.z - 1u - blockIdx.z : blockIdx.z;  // (late rows first)
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
 
     extern __shared__ uint8_t smemRaw[];

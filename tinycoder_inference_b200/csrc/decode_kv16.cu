@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKv16Kernel(const __grid_co
     constexpr int T = 16;
     constexpr int NS = HD / 16;     // k16 steps of QK^T = 16-dim output tiles of PV
 
-    const uint32_t chunk = blockIdx.x, hg = blockIdx.y, b = blockIdx.z;
+    const uint32_t chunk = blockIdx.x, hg = blockIdx.y, b = ROWS ? gridDim.z - 1u - blockIdx.z : blockIdx.z;  // (late rows first)
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
 
     extern __shared__ uint8_t smemRaw[];

@@ -13,10 +13,11 @@
 // instructions it spends on a 16-token tile.  Here a block of 32 query rows of one q head splits a stage of K and V once
 // into planes in shared memory, and a warp works on 16 rows x TG tokens: ldmatrix operands, three products each.  The
 // four token groups of a block take their share of every stage (a short prompt is a chain of stages, not a matter of
-// bytes) and are put together at the end.  Blocks of 64 rows and two token groups leave fewer and longer chains: 512
-// rows of 28 / 4 / 128 83 us against 79.  Measured (8-row form -> this one): f32 512 rows of 14 / 2 / 64 39.7 -> 26.9 us,
-// of 28 / 4 / 128 120 -> 79, 333 of 16 / 2 / 256 77 -> 63; fp16 100 rows of 28 / 4 / 128 15.0 -> 6.4 us, 512 behind 512
-// 107 -> 67, 512 behind 1000 of 14 / 2 / 64 45 -> 31.
+// bytes) and are put together at the end.  (Blocks of 64 rows and two token groups leave fewer and longer chains: 512
+// rows of 28 / 4 / 128 83 us against 79.)  The late rows of all heads come first, so that what starts last is short: that
+// form head by head took 79 us, 62 now.  Measured (8-row form -> this one): f32 512 rows of 14 / 2 / 64 39.7 -> 18.7 us,
+// of 28 / 4 / 128 120 -> 62, 333 of 16 / 2 / 256 77 -> 52; fp16 100 rows of 28 / 4 / 128 15.0 -> 6.4 us, 512 behind 512
+// 107 -> 71, 2000 rows of 8 / 4 / 64 81 -> 40.
 #include "decode_cluster.cuh"
 
 namespace tc {
@@ -114,7 +115,7 @@ __global__ void __launch_bounds__(kExactWarps * 32, 1) prefillExactKernel(const 
 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, g = lane >> 2, t = lane & 3u;
     const uint32_t rt = warp % RT, nh = warp / RT;
-    const uint32_t blk = gridDim.x - 1u - blockIdx.x, head = blockIdx.y;  // late rows (long prefixes) first
+    const uint32_t blk = gridDim.y - 1u - blockIdx.y, head = blockIdx.x;  // late rows (long prefixes) of all heads first
     const uint32_t row0 = blk * S::kRows, rows = min(static_cast<uint32_t>(S::kRows), p.qRows - row0);
     const uint32_t pos0 = p.devPos ? p.devPos[0] : p.cachePos;
     const uint64_t wanted = static_cast<uint64_t>(pos0) + row0 + rows;
@@ -319,7 +320,7 @@ prefillExactHalfKernel(const __grid_constant__ PrefillExactParams p) {
 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, g = lane >> 2, t = lane & 3u;
     const uint32_t rt = warp % RT, nh = warp / RT;
-    const uint32_t blk = gridDim.x - 1u - blockIdx.x, head = blockIdx.y;  // late rows (long prefixes) first
+    const uint32_t blk = gridDim.y - 1u - blockIdx.y, head = blockIdx.x;  // late rows (long prefixes) of all heads first
     const uint32_t row0 = blk * S::kRows, rows = min(static_cast<uint32_t>(S::kRows), p.qRows - row0);
     const uint32_t pos0 = p.devPos ? p.devPos[0] : p.cachePos;
     const uint64_t wanted = static_cast<uint64_t>(pos0) + row0 + rows;
@@ -489,7 +490,7 @@ static int launchExact(K kern, bool (&attrDone)[64], const PrefillExactParams &p
         TC_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(S::kBytes)));
         attrDone[dev] = true;
     }
-    return launchDependent(kern, dim3((prm.qRows + kExactRows - 1) / kExactRows, prm.nHeads), kExactWarps * 32, S::kBytes, st, 1,
+    return launchDependent(kern, dim3(prm.nHeads, (prm.qRows + kExactRows - 1) / kExactRows), kExactWarps * 32, S::kBytes, st, 1,
                            prm);
 }
 template <int HD>
