@@ -194,8 +194,9 @@ typedef struct tc_decode_i8_batch {
     uint32_t prefetchRows;
     /* Optional hint (NULL = none): the int8 pools the NEXT decode call on this stream
      * will read with the same geometry and lengths -- the next layer's slot.  Once a
-     * block has requested its own last tile it asks the memory system to pull the
-     * same rows of these pools into L2 (cp.async.bulk.prefetch.tensor), so DRAM keeps
+     * block has requested its own last tile it asks the memory system to pull rows of
+     * these pools into L2 (cp.async.bulk.prefetch.tensor) -- the tiles of its share that
+     * the next call's block cannot request by itself while it waits -- so DRAM keeps
      * streaming while this call's blocks fold their partials and the merge runs,
      * instead of idling until the next call's blocks start.  Nothing is read or
      * written through these pointers by the SMs.  Ignored when a call's rows
