@@ -95,3 +95,26 @@ def test_decode_batch_descriptor_is_checked_on_the_host():
     # the rows of a new token come as a pair
     assert call(desc(appendK=p)) == capi.TC_EINVAL and b"come together" in lib.tc_last_error()
     assert call(desc(appendV=p)) == capi.TC_EINVAL
+    # ... 16-byte aligned, at either head_dim
+    for hd in (128, 256):
+        for rows in ({"appendK": p + 4, "appendV": p}, {"appendK": p, "appendV": p + 8}):
+            assert call(desc(hd=hd, **rows)) == capi.TC_EINVAL and b"alignment" in lib.tc_last_error()
+
+
+def test_a_session_refuses_a_misaligned_row_for_its_int8_pool():
+    """Before anything is launched: the pool rows are quantised 16 bytes at a time."""
+    lib = capi.lib
+    p = 1 << 20
+    for mirror in (0, 1):
+        cfg = capi.KvSessionConfig()
+        cfg.nHeads, cfg.nKV, cfg.hd, cfg.maxSeqLen, cfg.slots = 16, 2, 256, 64, 1
+        cfg.kvStoreI8, cfg.kvMirror = 1 - mirror, mirror
+        for f in ("kvK8", "kvV8", "kvK8Scale", "kvV8Scale", "pAcc", "pM", "pL") + (("kvK", "kvV") if mirror else ()):
+            setattr(cfg, f, p)
+        cfg.numChunks = 4
+        h = C.c_void_p()
+        assert lib.tc_kv_session_create(C.byref(cfg), C.byref(h)) == 0
+        for k, v in ((p + 4, p), (p, p + 8)):
+            assert lib.tc_kv_session_attend(h, 0, p, k, v, p, 1, 0, None, 0, None) == capi.TC_EINVAL
+            assert b"alignment" in lib.tc_last_error()
+        lib.tc_kv_session_destroy(h)

@@ -454,6 +454,10 @@ int decodeI8Common(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAd
                TC_EINVAL, "decode_i8: q/out/k8/v8 need 16-byte alignment");
     TC_REQUIRE(d->numChunks >= 1, TC_EWORKSPACE, "decode_i8: no chunk slots");
     TC_REQUIRE((d->appendK == nullptr) == (d->appendV == nullptr), TC_EINVAL, "decode_i8: appendK and appendV come together");
+    // (the launch moves the new row, and its f32 copy, 16 bytes at a time)
+    TC_REQUIRE(((reinterpret_cast<uintptr_t>(d->appendK) | reinterpret_cast<uintptr_t>(d->appendV) |
+                 reinterpret_cast<uintptr_t>(mir.k) | reinterpret_cast<uintptr_t>(mir.v)) & 15u) == 0,
+               TC_EINVAL, "decode_i8: the new row needs 16-byte alignment");
     // head_dim 128 runs on the tcgen05 integer path
     if (d->hd == 128) return decodeI8Tc(d, lenHost, lenAdd, mir, st);
 

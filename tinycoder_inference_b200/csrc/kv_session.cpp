@@ -145,8 +145,8 @@ int tc_kv_session_attend(tc_kv_session *s, uint32_t slot, float *q, const float 
         kvV = slotPtr(c.kvV, s->g.kvLayerStride, slot);
     }
     int rc;
-    // the launches that take the new rows along move them (and the tables) 16 bytes at a time; rows at any other
-    // address go in with a launch of their own
+    // the launches that take the new rows along move them (and the tables) 16 bytes at a time; for an f32 / fp16 store rows
+    // at any other address go in with a launch of their own (the quantising launches take aligned rows only)
     const bool aligned = ((reinterpret_cast<uintptr_t>(kSrc) | reinterpret_cast<uintptr_t>(vSrc) |
                            reinterpret_cast<uintptr_t>(c.ropeCos) | reinterpret_cast<uintptr_t>(c.ropeSin) |
                            reinterpret_cast<uintptr_t>(kvK) | reinterpret_cast<uintptr_t>(kvV)) & 15u) == 0;
@@ -176,6 +176,9 @@ int tc_kv_session_attend(tc_kv_session *s, uint32_t slot, float *q, const float 
     // One row, not under graph capture (the row counts below are host state the replay could
     // not update), position known on the host.
     if (int8Pool && seqLen == 1 && !graphCapture && devPos == nullptr) {
+        // (refused by the decode launch as well, but the f32 row must not be written by then)
+        TC_REQUIRE(((reinterpret_cast<uintptr_t>(kSrc) | reinterpret_cast<uintptr_t>(vSrc)) & 15u) == 0, TC_EINVAL,
+                   "tc_kv_session_attend: the new row needs 16-byte alignment");
         uint32_t &rows8 = s->rows8[slot];
         if (!c.kvStoreI8) {
             if (rows8 < pos) {
