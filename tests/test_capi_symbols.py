@@ -99,6 +99,10 @@ def test_decode_batch_descriptor_is_checked_on_the_host():
     for hd in (128, 256):
         for rows in ({"appendK": p + 4, "appendV": p}, {"appendK": p, "appendV": p + 8}):
             assert call(desc(hd=hd, **rows)) == capi.TC_EINVAL and b"alignment" in lib.tc_last_error()
+    # head_dim 256: a host length whose new row lies outside the pool
+    for batch, length in ((1, 4097), (3, 2000)):
+        d = desc(hd=256, nKV=2, nHeads=16, appendK=p, appendV=p, batch=batch, maxLen=length, rowsPerSeq=1100)
+        assert call(d) == capi.TC_ECONTEXT_FULL and b"pool" in lib.tc_last_error()
 
 
 def test_a_session_refuses_a_misaligned_row_for_its_int8_pool():

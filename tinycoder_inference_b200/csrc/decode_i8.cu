@@ -461,6 +461,11 @@ int decodeI8Common(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAd
     // head_dim 128 runs on the tcgen05 integer path
     if (d->hd == 128) return decodeI8Tc(d, lenHost, lenAdd, mir, st);
 
+    // a new row that the host can tell to lie outside the pool (the quantise launch's check; head_dim 128 leaves it to the device)
+    const uint64_t lastRow = static_cast<uint64_t>(d->batch - 1) * d->rowsPerSeq + lenHost - 1;
+    TC_REQUIRE(d->appendK == nullptr || d->lens != nullptr || d->rowBase != nullptr || lastRow < d->totalRows, TC_ECONTEXT_FULL,
+               "decode_i8: row %u of sequence %u passes the pool's %llu rows", lenHost - 1, d->batch - 1,
+               (unsigned long long) d->totalRows);
     DecodeI8Params prm;
     const int rc = i8Params(d, lenHost, lenAdd, mir, &prm);
     if (rc != TC_OK) return rc;
