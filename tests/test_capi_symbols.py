@@ -61,6 +61,10 @@ def test_prefill_entry_points_check_their_arguments_on_the_host():
                                    None) == capi.TC_EINVAL                       # misaligned scratch
     assert lib.tc_attn_prefill_f16(p, p, p, p, p, 4096, 512, 0, 28, 4, 128, 0.088, None) == capi.TC_EWORKSPACE
     assert lib.tc_attn_prefill_f16(p, p, p, p, p, 1 << 30, 0, 0, 28, 4, 128, 0.088, None) == 0   # no rows: nothing to do
+    # exact causal rows: as many blocks of rows as a grid holds, whichever form the launch would take
+    for half in (0, 1):
+        assert lib.tc_attn_prefill_kv(p, p, p, p, 8 * 65535 + 1, 28, 4, 128, 0, None, 1 << 20, 0.088, half,
+                                      None) == capi.TC_EUNSUPPORTED
     # the int8 store needs its scales, the mirror its pool, and the mirror's rows have to fit the pool
     assert lib.tc_attn_prefill_f16_i8(p, p, p, None, None, p, p, 1 << 30, 512, 0, 28, 4, 128, 0.088,
                                       None) == capi.TC_EINVAL

@@ -424,12 +424,12 @@ static int prefillKv(const float *q, const void *kvK, const void *kvV, float *ou
                  (unsigned long long) cachePos + seqLen, (unsigned long long) totalRows);
         return TC_ECONTEXT_FULL;
     }
+    const uint32_t rowBlocks = (seqLen + 7) / 8;
+    TC_REQUIRE(rowBlocks <= 65535 && nHeads <= 65535, TC_EUNSUPPORTED, "prefill_kv: %u rows x %u heads", seqLen, nHeads);
     // (a position on the device: somewhere in the store)
     const uint64_t before = devPos == nullptr ? cachePos : (totalRows > seqLen ? (totalRows - seqLen) / 2 : 0);
     if (prefillExactWins(seqLen, before, nHeads, hd, kvHalf))
         return prefillExact(q, kvK, kvV, out, seqLen, nHeads, nKV, hd, cachePos, devPos, totalRows, invSqrt, kvHalf, st);
-    const uint32_t rowBlocks = (seqLen + 7) / 8;
-    TC_REQUIRE(rowBlocks <= 65535 && nHeads <= 65535, TC_EUNSUPPORTED, "prefill_kv: %u rows x %u heads", seqLen, nHeads);
     DecodeKvParams prm;
     memset(&prm, 0, sizeof(prm));
     prm.q = q;
