@@ -8,7 +8,8 @@
 //
 // Every wrapper returns the C function's code as an int; ops.py turns a non-zero one into an exception.
 // Integers wrap like ctypes' unsigned types do, None is a null pointer, a tensor has to be
-// contiguous and on a CUDA device.
+// contiguous and on a CUDA device.  What torch throws on the way (a tensor without storage, no device) becomes the
+// Python exception that torch itself would raise.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -17,6 +18,7 @@
 #include <utility>
 
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "../../../include/tc_attn.h"
@@ -84,11 +86,13 @@ struct Wrap<Fn> {
         return PyLong_FromLong(std::apply(Fn, v));
     }
     static PyObject *py(PyObject *, PyObject *const *args, Py_ssize_t n) {
+        HANDLE_TH_ERRORS
         if (static_cast<size_t>(n) != kArgs) {
             PyErr_Format(PyExc_TypeError, "%zu arguments expected, got %zd", kArgs, n);
             return nullptr;
         }
         return call(args, std::make_index_sequence<kArgs>());
+        END_HANDLE_TH_ERRORS
     }
 };
 
@@ -96,6 +100,7 @@ struct Wrap<Fn> {
 
 // attend(session, slot, q, k, v, out, pos, dev_pos, graph_capture): the rows of the call are q's
 PyObject *attend(PyObject *, PyObject *const *a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
     if (n != 9) {
         PyErr_SetString(PyExc_TypeError, "attend: 9 arguments expected");
         return nullptr;
@@ -117,6 +122,7 @@ PyObject *attend(PyObject *, PyObject *const *a, Py_ssize_t n) {
     }
     const uint32_t rows = static_cast<uint32_t>(THPVariable_Unpack(a[2]).size(0));
     return PyLong_FromLong(tc_kv_session_attend(s, slot, q, k, v, out, rows, pos, dev, graph, currentStream()));
+    END_HANDLE_TH_ERRORS
 }
 
 // begin(session, n) -> position, or -code
@@ -136,6 +142,7 @@ PyObject *begin(PyObject *, PyObject *const *a, Py_ssize_t n) {
 //                 appendV, rowsPerSeq, totalRows, batch, nHeads, nKV, hd, maxLen, numChunks, invSqrt,
 //                 partialsOnly, flags, prefetchRows) -> chunk slots used, or -code
 PyObject *decodeI8Batch(PyObject *, PyObject *const *a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
     if (n != 28) {
         PyErr_SetString(PyExc_TypeError, "decode_i8_batch: 28 arguments expected");
         return nullptr;
@@ -165,6 +172,7 @@ PyObject *decodeI8Batch(PyObject *, PyObject *const *a, Py_ssize_t n) {
     d.chunksUsed = &used;
     const int rc = tc_attn_decode_i8_batch(&d, currentStream());
     return PyLong_FromLongLong(rc == TC_OK ? static_cast<long long>(used) : -static_cast<long long>(rc));
+    END_HANDLE_TH_ERRORS
 }
 
 #define TC_FAST(name, fn) {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(fn)), METH_FASTCALL, nullptr}
