@@ -41,3 +41,36 @@ def test_attend_refuses_a_q_without_dimensions():
     kv = torch.zeros((1, 2, 128), device="cuda")
     with pytest.raises(IndexError):
         s.attend(0, torch.zeros((), device="cuda"), kv, kv, torch.zeros((1, 8, 128), device="cuda"), 0)
+
+
+@pytest.mark.gpu
+def test_other_threads_run_while_clear_waits_for_the_stream():
+    import threading
+    import time
+
+    import torch
+
+    from tinycoder_inference_b200 import ops
+
+    s = ops.KvSession(8, 2, 128, 64, 1, mode="f32")
+    s.clear()
+    torch.cuda._sleep(1000)
+    torch.cuda.synchronize()
+    stamps, stop = [], threading.Event()
+
+    def tick():
+        while not stop.is_set():
+            stamps.append(time.perf_counter())
+            time.sleep(0.002)
+
+    t = threading.Thread(target=tick)
+    t.start()
+    torch.cuda._sleep(800_000_000)      # about 0.4 s of the stream ahead of the synchronise in clear()
+    a = time.perf_counter()
+    s.clear()
+    b = time.perf_counter()
+    stop.set()
+    t.join()
+    assert b - a > 0.1, "the stream was not busy"
+    inside = [x for x in stamps if a + 0.02 < x < b - 0.02]
+    assert len(inside) > 5, f"{len(inside)} ticks of another thread in {b - a:.2f} s"

@@ -8,7 +8,9 @@
 //
 // Every wrapper returns the C function's code as an int; ops.py turns a non-zero one into an exception.
 // Integers wrap like ctypes' unsigned types do, None is a null pointer, a tensor has to be
-// contiguous and on a CUDA device.  What torch throws on the way (a tensor without storage, no device) becomes the
+// contiguous and on a CUDA device.  The interpreter lock is not held during a call that may block (a launch into a full
+// queue, the synchronise at the end of `clear`): other Python threads go on, and a stream that waits for one of them
+// gets there.  What torch throws on the way (a tensor without storage, no device) becomes the
 // Python exception that torch itself would raise.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
@@ -72,6 +74,15 @@ bool toArg(PyObject *o, T *out) {
     return PyErr_Occurred() == nullptr;
 }
 
+// The C call itself, without the interpreter lock.
+template <typename F>
+auto unlocked(F &&call) {
+    PyThreadState *const state = PyEval_SaveThread();
+    const auto rc = call();
+    PyEval_RestoreThread(state);
+    return rc;
+}
+
 // ---- a C function int f(args..., tc_stream) as a Python function f(args...) -------------------
 template <auto Fn>
 struct Wrap;
@@ -83,7 +94,7 @@ struct Wrap<Fn> {
         std::tuple<A...> v;
         if (!(toArg(args[I], &std::get<I>(v)) && ...)) return nullptr;
         std::get<kArgs>(v) = currentStream();
-        return PyLong_FromLong(std::apply(Fn, v));
+        return PyLong_FromLong(unlocked([&] { return std::apply(Fn, v); }));
     }
     static PyObject *py(PyObject *, PyObject *const *args, Py_ssize_t n) {
         HANDLE_TH_ERRORS
@@ -121,7 +132,8 @@ PyObject *attend(PyObject *, PyObject *const *a, Py_ssize_t n) {
         return nullptr;
     }
     const uint32_t rows = static_cast<uint32_t>(THPVariable_Unpack(a[2]).size(0));
-    return PyLong_FromLong(tc_kv_session_attend(s, slot, q, k, v, out, rows, pos, dev, graph, currentStream()));
+    const tc_stream st = currentStream();
+    return PyLong_FromLong(unlocked([&] { return tc_kv_session_attend(s, slot, q, k, v, out, rows, pos, dev, graph, st); }));
     END_HANDLE_TH_ERRORS
 }
 
@@ -170,7 +182,8 @@ PyObject *decodeI8Batch(PyObject *, PyObject *const *a, Py_ssize_t n) {
         !toArg(a[26], &d.flags) || !toArg(a[27], &d.prefetchRows))
         return nullptr;
     d.chunksUsed = &used;
-    const int rc = tc_attn_decode_i8_batch(&d, currentStream());
+    const tc_stream st = currentStream();
+    const int rc = unlocked([&] { return tc_attn_decode_i8_batch(&d, st); });
     return PyLong_FromLongLong(rc == TC_OK ? static_cast<long long>(used) : -static_cast<long long>(rc));
     END_HANDLE_TH_ERRORS
 }
