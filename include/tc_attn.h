@@ -189,7 +189,11 @@ typedef struct tc_decode_i8_batch {
      * Rows [0, prefetchRows) of each sequence -- rows no kernel in flight writes,
      * e.g. everything before the token being appended -- are streamed in early,
      * but only with host lengths (lens == NULL: every sequence is maxLen rows
-     * long) and rowBase == NULL.  flags == 0 keeps plain stream order. */
+     * long) and rowBase == NULL.  Rows written by a call without this flag -- a KV
+     * writer, a prompt, a decode that takes the new row along -- are in memory before
+     * the next call on the stream can read anything, so they may lie below
+     * prefetchRows; a row that a call WITH the flag appends may not, as long as only
+     * such calls lie in between.  flags == 0 keeps plain stream order. */
     uint32_t flags;
     uint32_t prefetchRows;
     /* Optional hint (NULL = none): the int8 pools the NEXT decode call on this stream

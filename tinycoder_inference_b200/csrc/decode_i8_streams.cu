@@ -63,12 +63,14 @@ decodeI8StreamsKernel(const __grid_constant__ DecodeI8Params p) {
     __syncthreads();
     clusterHello();
     gridDepWait();
-    gridDepLaunch();
 
     const uint32_t want = p.devLens ? p.devLens[0] + p.lenAdd : p.lenHost;
     const uint32_t len = min(want, p.lenHost);  // (the host's length is the upper bound of a device length)
     const uint32_t nTiles = (len + T - 1) / T;
     const uint32_t n = nTiles > stream ? (nTiles - stream + 7u) / 8u : 0u;  // tiles of this stream: stream + 8 i
+    // the block that stores the token's row lets the next grid start behind that store: it may request the row early
+    const bool storesRow = p.appendK != nullptr && want <= p.totalRows && (nTiles - 1u) % 8u == stream;
+    if (!storesRow) gridDepLaunch();
     const uint32_t head0 = kvHead * p.group + p.colBase, nValid = min(8u, p.group - p.colBase);
     // record of a slot: P operands [MT][32 lanes] uint4, P [2 NR][32], P x scale [2 NR][32], then al[8], as[8], flag
     auto record = [&](uint32_t i) { return smem + L::kRec + (i % NSLOT) * L::kRecord; };
@@ -91,8 +93,8 @@ decodeI8StreamsKernel(const __grid_constant__ DecodeI8Params p) {
         const bool outside = p.appendK != nullptr && want > p.totalRows;  // a device position outside the pool: no row written
         if (outside && stream == 0 && threadIdx.x == 0) atomicOr(p.err, kDevErrRowBound);
         const uint32_t iLast = (nTiles - 1u) / 8u;
-        const bool mine = p.appendK != nullptr && !outside && (nTiles - 1u) % 8u == stream && iLast % SW == warp;
-        const bool intoTile = mine && iLast < SW;
+        const bool hasRow = storesRow && iLast % SW == warp;
+        const bool intoTile = hasRow && iLast < SW;
         const uint32_t have = intoTile ? len - 1u : static_cast<uint32_t>(min(static_cast<uint64_t>(len), p.totalRows));
         auto request = [&](uint32_t i, bool isV) {
             const uint32_t row = (stream + 8u * i) * T;
@@ -120,11 +122,11 @@ decodeI8StreamsKernel(const __grid_constant__ DecodeI8Params p) {
         // (the tile after that one is requested behind the row's store when it holds the row)
         NewQuantRow<HD, T> fresh;
         const size_t newSrc = static_cast<size_t>(kvHead) * HD;
-        if (mine) fresh.load(p.appendK + newSrc, p.appendV + newSrc, lane);
+        if (hasRow) fresh.load(p.appendK + newSrc, p.appendV + newSrc, lane);
         else requestK(warp + SW);
         I8Query<HD> qf;
         i8LoadQuery<HD>(qf, p.q + static_cast<size_t>(head0 + (g < nValid ? g : 0u)) * HD, g < nValid, p.invSqrt, lane);
-        if (mine) {
+        if (hasRow) {
             const size_t dst = static_cast<size_t>(len - 1u) * p.nKV + kvHead;
             uint8_t *tile = intoTile ? slotK(iLast) : nullptr;
             fresh.store(p.k8w + dst * (HD / 4), p.v8w + dst * (HD / 4), const_cast<float *>(p.ks) + dst,
@@ -223,6 +225,12 @@ decodeI8StreamsKernel(const __grid_constant__ DecodeI8Params p) {
             if (lane == 0) *reinterpret_cast<uint32_t *>(fac + 16) = any ? 1u : 0u;
             // (a warp whose wait ran out stays with the others' barrier and hands nothing on: their waits end too)
             if (ok) mbarArrive(&fullBar[i % NSLOT]);
+            if (hasRow && round == 0) {
+                // (here the row's stores are long done: right behind them the fence cost 0.5 us of the step)
+                __threadfence();
+                __syncwarp();
+                gridDepLaunch();
+            }
         }
         if (warp == 0) {
             if (g == 0) sEnd[2 * t] = m0, sEnd[2 * t + 1] = m1;

@@ -56,6 +56,7 @@ struct DecodeTcParams {
     uint32_t prefetchRows;
     float invSqrt;
     int directOut;
+    int dependent;          // TC_DECODE_PDL: the next grid may start ahead of this one's wait
     int prefetchNext;
     uint32_t earlyStages;   // tiles the producer may request before the dependency wait
     int l2Hints;            // bit 0: own tiles evict_first, bit 1: next pools evict_last
@@ -201,7 +202,7 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         tmaPrefetchDesc(&tmV);
     }
     __syncthreads();
-    gridDepLaunch();  // the dependent grid (the merge) may be scheduled as soon as room frees up
+    if (p.dependent) gridDepLaunch();  // the next grid (the merge) may be scheduled as soon as room frees up
 
     // The length may live in device memory written by an earlier kernel; only a host-known
     // length lets the producer start before the dependency wait.
@@ -230,6 +231,10 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     if (FOLD != TcFold::kCluster && t0 >= len) return;
     const uint32_t t1 = min(len, t0 + share);
     const uint32_t nTiles = t0 >= len ? 0u : (t1 - t0 + T - 1) / T;
+    // Plain stream order: the kernels ahead are complete by now, and the block that stores a token's row lets the next grid
+    // start behind that store (a call with TC_DECODE_PDL may request the row early).
+    const bool storesRow = APPEND && p.appendK != nullptr && t1 == len && nTiles != 0u;
+    if (!p.dependent && !storesRow) gridDepLaunch();
     constexpr bool CLUSTER = FOLD == TcFold::kCluster;
     __shared__ FoldInbox<CLUSTER ? 32 : 1> inbox;
     const uint32_t foldTotal = min(8u, p.group - p.colBase) * 32u;  // float4s of the outputs, and a block's share of them
@@ -269,7 +274,7 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
                 }
             }
         };
-        if (APPEND && p.appendK != nullptr && t1 == len && nTiles != 0u && lane < 8u) {
+        if (APPEND && storesRow && lane < 8u) {
             // the rows this block will append, towards L2 (their final contents arrive there too)
             const char *src = reinterpret_cast<const char *>((lane < 4u ? p.appendK : p.appendV) +
                                                              (static_cast<size_t>(b) * p.nKV + kvHead) * 128u) + (lane & 3u) * 128u;
@@ -314,11 +319,10 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         // The tile that holds the row of a token being appended (the last tile of the sequence's last
         // chunk) is requested apart from the loop: the row goes into the pool first, once the kernels
         // ahead have completed.
-        const bool appendHere = APPEND && p.appendK != nullptr && t1 == len && nTiles != 0u;
-        const uint32_t nLoop = appendHere ? nTiles - 1u : nTiles;
+        const uint32_t nLoop = storesRow ? nTiles - 1u : nTiles;
         bool okP = true;
         for (uint32_t it = 0; okP && it < nLoop; ++it) okP = requestTile(it);
-        if (appendHere && okP) {
+        if (APPEND && storesRow && okP) {
             if (!waited) {
                 gridDepWait();
                 waited = true;
@@ -339,6 +343,11 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
                                     mk, mv, lane);
             }
             requestTile(nTiles - 1u);
+            if (!p.dependent) {
+                __threadfence();
+                __syncwarp();
+                gridDepLaunch();
+            }
         }
         // all tiles of this block are requested: the next call's rows follow them into L2 (requested
         // earlier they sit in front of this block's own tiles in the queue: 10.2 against 9.1 us)
@@ -856,6 +865,7 @@ int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, c
     prm.prefetchRows = pdl ? d->prefetchRows : 0;
     prm.invSqrt = d->invSqrt;
     prm.directOut = direct ? 1 : 0;
+    prm.dependent = pdl ? 1 : 0;
     prm.prefetchNext = prefetchNext ? 1 : 0;
     // Under programmatic dependent launch the producer requests a whole ring of old rows while the
     // kernels ahead drain (7B shape, 32768 rows, batch 1: 12.4 us per layer against 13.5 with one

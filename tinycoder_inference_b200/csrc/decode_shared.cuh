@@ -22,9 +22,12 @@ struct QRotation {
 
 // devLens (nullable): the merge works out on the device how many of the activeHost partials were written, from the
 // length devLens[s] + lenAdd and chunkTokens per partial (0: tokensPerBlock of the length, at most rot.maxLen).
+// early: the grid behind the merge may start while the one that writes the partials still runs.  For an int8 decode at
+// head_dim 128 that is the caller's word (TC_DECODE_PDL); the others write no row that any launch reads ahead of its
+// wait, and are past their own wait before the merge can start.
 int launchMerge(const float *pAcc, const float *pM, const float *pL, float *out, uint32_t seqLen,
                 uint32_t nHeads, uint32_t numChunks, uint32_t activeHost, uint32_t hd, const uint32_t *devLens,
-                uint32_t lenAdd, uint32_t chunkTokens, uint8_t *q81, bool pdl, cudaStream_t st,
+                uint32_t lenAdd, uint32_t chunkTokens, uint8_t *q81, bool early, cudaStream_t st,
                 uint32_t chunksPerRank = 0, uint64_t rankStride = 0, QRotation rot = {nullptr, nullptr, nullptr, 0});
 
 // An f32 store kept beside an int8 pool: where the appended row of a decode call also goes, verbatim (one

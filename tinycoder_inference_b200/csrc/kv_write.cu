@@ -26,8 +26,7 @@ kvQuantKernel(const float *__restrict__ k, const float *__restrict__ v, int8_t *
               const uint32_t *__restrict__ devDstBase, uint32_t batchMode, uint64_t rowsPerSeq,
               const uint64_t *__restrict__ rowBase, const uint32_t *__restrict__ devLens, int32_t lenAdd,
               uint64_t maxRows, unsigned int *__restrict__ err) {
-    gridDepWait();
-    gridDepLaunch();
+    gridDepWait();  // (no gridDepLaunch: the next grid may request these rows ahead of its own wait)
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t row = static_cast<uint64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= static_cast<uint64_t>(tokens) * nKV) return;
@@ -89,6 +88,7 @@ kvQuantKernel(const float *__restrict__ k, const float *__restrict__ v, int8_t *
             reinterpret_cast<uint32_t *>(v8 + dst * hd)[i] = pv;
         }
     }
+    __threadfence();  // in memory before the block's exit lets the next grid start
 }
 
 // ---------------------------------------------------------------------------

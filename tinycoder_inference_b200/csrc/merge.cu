@@ -64,8 +64,8 @@ mergePartialsKernel(const float *__restrict__ pAcc, const float *__restrict__ pM
         const uint32_t r = c / chunksPerRank;
         return static_cast<uint64_t>(r) * rankStride + (headRow * chunksPerRank + (c - r * chunksPerRank)) * hd;
     };
-    // let the next grid start its prologue -- ahead of the grid that wrote the partials only when that one's caller works
-    // under programmatic dependent launch itself -- and wait until the partials are complete
+    // let the next grid start its prologue -- ahead of the grid that wrote the partials only when that is allowed (see
+    // launchMerge) -- and wait until the partials are complete
     if (early) gridDepLaunch();
     gridDepWait();
     if (!early) gridDepLaunch();
@@ -474,11 +474,11 @@ mergeWarpKernel(const float *__restrict__ pAcc, const float *__restrict__ pM, co
 
 int launchMerge(const float *pAcc, const float *pM, const float *pL, float *out, uint32_t seqLen,
                 uint32_t nHeads, uint32_t numChunks, uint32_t activeHost, uint32_t hd, const uint32_t *devLens,
-                uint32_t lenAdd, uint32_t chunkTokens, uint8_t *q81, bool pdl, cudaStream_t st,
+                uint32_t lenAdd, uint32_t chunkTokens, uint8_t *q81, bool earlyNext, cudaStream_t st,
                 uint32_t chunksPerRank, uint64_t rankStride, QRotation rot) {
     if (chunksPerRank == 0) chunksPerRank = numChunks;
     const uint64_t units = static_cast<uint64_t>(nHeads) * seqLen;
-    const uint32_t early = pdl ? 1u : 0u;
+    const uint32_t early = earlyNext ? 1u : 0u;
     // (under dependent launch the blocks of a merge are resident next to the blocks they wait for: few and small)
     if (q81 == nullptr && units <= 64u) {
         // one sequence: 16-dim slices (7B shape at 32768 rows: 11.36 us per layer against 11.67 with 32-dim slices, 11.38

@@ -75,7 +75,7 @@ struct PrefillRowsParams {
 template <int HD>
 __global__ void __launch_bounds__(256) prefillRowsKernel(const __grid_constant__ PrefillRowsParams p) {
     gridDepWait();
-    gridDepLaunch();  // the attention launch may set itself up while this one drains
+    gridDepLaunch();  // the attention launch may set itself up while this one drains (it waits before it lets anything else in)
     // the attention launch that follows in the stream hands out its work items through this counter
     if (blockIdx.x == 0 && threadIdx.x == 0) *p.workCounter = 0u;
     const size_t tid = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;

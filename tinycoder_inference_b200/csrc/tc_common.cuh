@@ -63,9 +63,14 @@ int getTensorMap(const TensorMapKey &key, CUtensorMap *out);
 
 // Launch under programmatic dependent launch: the grid may be scheduled while the one in front of it drains, so
 // the kernel has to call gridDepWait() before it touches anything that grid may have written or may still read --
-// every kernel launched through here does so first thing.  Kernels that write K/V rows call gridDepLaunch() after
-// that wait: a decode launch that requests old rows early (TC_DECODE_PDL) then has at most the kernel right in front of
-// it in flight, as it had when these were plain launches.  (In stream order a dependent launch takes 3.1 - 3.7 us on
+// every kernel launched through here does so first thing, but for the int8 decode at head_dim 128 under
+// TC_DECODE_PDL, which requests rows of its pool that the caller calls old (prefetchRows) ahead of it.  Where the others
+// call gridDepLaunch() decides what such a launch may find unfinished:
+//   * after the wait, so that the kernels ahead of theirs are complete;
+//   * a kernel that writes int8 rows of head_dim 128 (nothing else is read ahead of a wait), not before those are in
+//     memory: kvQuantKernel by its exit, a decode kernel that takes the new row along behind that row's store.  The rows
+//     launch of a prompt may let the next grid in sooner: that is the attention launch, which waits before it does.
+// So a row written by any call without TC_DECODE_PDL is in memory before a call behind it can look.  (In stream order a dependent launch takes 3.1 - 3.7 us on
 // B200, like this 2.0; as nodes of a graph 1.2 and 0.8.)  cluster: blocks per cluster along x.
 template <typename... P, typename... A>
 int launchDependent(void (*kern)(P...), dim3 grid, uint32_t threads, size_t smem, cudaStream_t st, uint32_t cluster,
