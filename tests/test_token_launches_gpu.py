@@ -103,3 +103,22 @@ def test_rotating_step_on_an_f32_or_fp16_store(mode, nH, nKV, hd, ctx, dev_pos):
     assert np.array_equal(host(dq), qr)
     assert np.array_equal(host(s.kvK[0]), kk) and np.array_equal(host(s.kvV[0]), vv)
     assert_close(host(out), oracle.attention_kv(qr, kk, vv, 1, nH, nKV, hd, ctx, 1.0 / math.sqrt(hd)), what=f"{mode} step")
+
+
+# (window 40000: several blocks per kv head and a merge, which rotates q by the position as well)
+@pytest.mark.parametrize("mode,nH,nKV,hd,window", [("i8", 28, 4, 128, 64), ("i8", 16, 2, 256, 64), ("f32", 14, 2, 64, 64),
+                                                   ("f16", 28, 4, 128, 64), ("f16", 28, 4, 128, 40000)])
+@pytest.mark.parametrize("at", [0xffffffff, 0x80000000, 50000])
+def test_a_device_position_outside_the_store_writes_no_row(mode, nH, nKV, hd, window, at):
+    """(0xffffffff: position + 1 wraps to a length of 0)"""
+    q, k, v = _rows(hd, nH, nKV, hd, 1)
+    rope = tuple(dev(t) for t in oracle.rope_tables(window, hd, 1e6)) if mode[0] == "f" else None
+    s = ops.KvSession(nH, nKV, hd, window, 2, mode=mode, rope=rope)
+    stores = [t for t in (getattr(s, n, None) for n in ("kvK", "kvV", "k8", "v8", "ks", "vs")) if t is not None]
+    before = [t.clone() for t in stores]
+    pos = torch.from_numpy(np.array([at], np.uint32).view(np.int32)).cuda()
+    s.attend(1, dev(q), dev(k), dev(v), torch.zeros((1, nH, hd), device="cuda"), 3, dev_pos=pos, graph_capture=True)
+    torch.cuda.synchronize()
+    assert ops.device_status(raise_on_flags=False) == 32
+    for have, want in zip(stores, before):
+        assert torch.equal(torch.nan_to_num(have.float()), torch.nan_to_num(want.float()))

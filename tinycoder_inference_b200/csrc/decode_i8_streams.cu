@@ -69,7 +69,9 @@ decodeI8StreamsKernel(const __grid_constant__ DecodeI8Params p) {
     const uint32_t nTiles = (len + T - 1) / T;
     const uint32_t n = nTiles > stream ? (nTiles - stream + 7u) / 8u : 0u;  // tiles of this stream: stream + 8 i
     // the block that stores the token's row lets the next grid start behind that store: it may request the row early
-    const bool storesRow = p.appendK != nullptr && want <= p.totalRows && (nTiles - 1u) % 8u == stream;
+    // (a device position outside the pool, the one whose length wraps to 0 among them, stores none)
+    const bool outside = p.appendK != nullptr && want - 1u >= p.totalRows;
+    const bool storesRow = p.appendK != nullptr && !outside && (nTiles - 1u) % 8u == stream;
     if (!storesRow) gridDepLaunch();
     const uint32_t head0 = kvHead * p.group + p.colBase, nValid = min(8u, p.group - p.colBase);
     // record of a slot: P operands [MT][32 lanes] uint4, P [2 NR][32], P x scale [2 NR][32], then al[8], as[8], flag
@@ -90,7 +92,6 @@ decodeI8StreamsKernel(const __grid_constant__ DecodeI8Params p) {
         auto slotK = [&](uint32_t i) { return smem + L::kK + (warp * 2 + (i / SW) % 2) * L::kTileBytes; };
         auto scales = [&](uint32_t i) { return reinterpret_cast<float *>(smem + L::kScales) + (warp * 2 + (i / SW) % 2) * 2 * T; };
         // the warp that takes the last tile stores the token's row; into the tile itself when it is the warp's first one
-        const bool outside = p.appendK != nullptr && want > p.totalRows;  // a device position outside the pool: no row written
         if (outside && stream == 0 && threadIdx.x == 0) atomicOr(p.err, kDevErrRowBound);
         const uint32_t iLast = (nTiles - 1u) / 8u;
         const bool hasRow = storesRow && iLast % SW == warp;

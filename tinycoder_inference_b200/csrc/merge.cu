@@ -18,11 +18,17 @@ namespace tc {
 
 constexpr int kMergeMaxChunks = 1024;
 
+// Attended rows of a token whose position is on the device, as its decode launch counts them: the host's bound stands for
+// every position beyond it, 0xffffffff (which + 1 would be 0) included.
+__device__ __forceinline__ uint32_t tokenLen(uint32_t pos, uint32_t lenAdd, uint32_t maxLen) {
+    return min(pos, maxLen - lenAdd) + lenAdd;
+}
+
 // The rotation of q in place (see QRotation), block `part` of `parts` of a head.
 __device__ __forceinline__ void rotateHead(const QRotation &rot, uint32_t head, uint32_t hd, const uint32_t *devLens,
                                            uint32_t lenAdd, uint32_t part, uint32_t parts) {
     const uint32_t H = hd >> 1;
-    const uint32_t len = devLens != nullptr ? min(devLens[0] + lenAdd, rot.maxLen) : rot.maxLen;
+    const uint32_t len = devLens != nullptr ? tokenLen(devLens[0], lenAdd, rot.maxLen) : rot.maxLen;
     const float *c = rot.cosT + static_cast<size_t>(len - 1u) * H, *s = rot.sinT + static_cast<size_t>(len - 1u) * H;
     float *x = rot.q + static_cast<size_t>(head) * hd;
     for (uint32_t j = part * blockDim.x + threadIdx.x; j < H; j += parts * blockDim.x) {
@@ -73,7 +79,7 @@ mergePartialsKernel(const float *__restrict__ pAcc, const float *__restrict__ pM
     uint32_t active = activeHost < numChunks ? activeHost : numChunks;
     if (devLens != nullptr) {
         uint32_t len = devLens[s] + lenAdd, per = chunkTokens;
-        if (per == 0) len = min(len, rot.maxLen), per = tokensPerBlock(len, activeHost);
+        if (per == 0) len = tokenLen(devLens[s], lenAdd, rot.maxLen), per = tokensPerBlock(len, activeHost);
         const uint32_t need = (len + per - 1) / per;
         // never past the slots the launch that wrote the partials covered (activeHost): a device
         // length beyond the host bound the plan was built from must not pull in stale slots
@@ -247,7 +253,7 @@ mergeSliceKernel(const float *__restrict__ pAcc, const float *__restrict__ pM, c
     uint32_t active = activeHost < numChunks ? activeHost : numChunks;
     if (devLens != nullptr) {
         uint32_t len = devLens[s] + lenAdd, per = chunkTokens;
-        if (TOKEN && per == 0) len = min(len, rot.maxLen), per = tokensPerBlock(len, activeHost);
+        if (TOKEN && per == 0) len = tokenLen(devLens[s], lenAdd, rot.maxLen), per = tokensPerBlock(len, activeHost);
         const uint32_t need = (len + per - 1) / per;
         // never past the slots the launch that wrote the partials covered (activeHost): a device
         // length beyond the host bound the plan was built from must not pull in stale slots
