@@ -32,7 +32,8 @@ def _int8_session(nH, nKV, hd, ctx, window, seed):
 @pytest.mark.parametrize("nH,nKV,hd,ctx", [(28, 4, 128, 0), (28, 4, 128, 31), (28, 4, 128, 32), (8, 2, 128, 255),
                                            (12, 2, 128, 256), (28, 4, 128, 2047), (28, 4, 128, 4096), (9, 1, 128, 4129),
                                            (28, 4, 128, 9000), (16, 2, 256, 0), (16, 2, 256, 15), (16, 4, 256, 128),
-                                           (8, 4, 256, 2049), (20, 2, 256, 4500)])
+                                           (8, 4, 256, 2049), (20, 2, 256, 4500),
+                                           (72, 1, 128, 300)])
 def test_captured_step_on_the_int8_store(nH, nKV, hd, ctx):
     """The device-position step stores the row itself and keeps the causal kernel's accumulation order."""
     s, q, k, v, quant = _int8_session(nH, nKV, hd, ctx, ctx + 300, seed=ctx + hd + nH)

@@ -424,8 +424,6 @@ static int i8Params(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenA
 
 int decodeI8Streams(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, cudaStream_t st) {
     TC_REQUIRE(d->hd == 128 || d->hd == 256, TC_EUNSUPPORTED, "decode_i8: head_dim %u (built for 128 and 256)", d->hd);
-    TC_REQUIRE(d->nHeads / d->nKV <= 64, TC_EUNSUPPORTED, "decode_i8: %u q heads per kv head (built for <= 64)",
-               d->nHeads / d->nKV);
     TC_REQUIRE(((reinterpret_cast<uintptr_t>(d->k8) | reinterpret_cast<uintptr_t>(d->v8) |
                  reinterpret_cast<uintptr_t>(d->q) | reinterpret_cast<uintptr_t>(d->out) |
                  reinterpret_cast<uintptr_t>(d->appendK) | reinterpret_cast<uintptr_t>(d->appendV)) & 15u) == 0,
