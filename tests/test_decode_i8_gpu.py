@@ -477,3 +477,46 @@ def test_merge_inside_the_kernel_equals_the_merge_launch():
         assert torch.allclose(a, b, rtol=1e-5, atol=1e-6)
         assert int(tickets.abs().sum().item()) == 0
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("hd", [128, 256])
+@pytest.mark.parametrize("longest", [130, 700, 6000])
+def test_a_sequence_without_rows_gives_zeros(hd, longest):
+    """A device length of 0 next to others, in every form that brings a sequence's blocks together (at 130 rows of head_dim
+    256 one block, then a cluster, then blocks and a merge)."""
+    nH, nKV, B, chunks = 16, 4, 3, 64
+    g = torch.Generator(device="cuda").manual_seed(longest + hd)
+    k8 = torch.randint(-128, 128, (B * longest, nKV, hd), dtype=torch.int8, device="cuda", generator=g)
+    v8 = torch.randint(-128, 128, (B * longest, nKV, hd), dtype=torch.int8, device="cuda", generator=g)
+    ks, vs = (torch.rand((B * longest, nKV), device="cuda", generator=g) / 64 for _ in range(2))
+    q = torch.randn((B, nH, hd), device="cuda", generator=g)
+    lens = torch.tensor([longest, 0, longest // 2], dtype=torch.int32, device="cuda")
+    out = torch.full((B, nH, hd), float("nan"), device="cuda")
+    ops.decode_i8_batch(q, k8, v8, ks, vs, out, ops.workspace(B, nH, hd, chunks), lens, B, nH, nKV, hd, longest, chunks,
+                        rows_per_seq=longest)
+    torch.cuda.synchronize()
+    assert ops.device_status() == 0
+    assert (out[1] == 0).all()
+    for b in (0, 2):
+        n, at = int(lens[b]), b * longest
+        want = oracle.attention_i8(host(q[b:b + 1]), *(host(t[at:at + n]) for t in (k8, v8, ks, vs)), 1, nH, nKV, hd, n - 1,
+                                   1.0 / math.sqrt(hd))
+        assert_close(host(out[b]), want[0], what=f"sequence {b}")
+
+
+def test_a_new_row_of_a_sequence_without_rows_is_flagged():
+    """head_dim 256, device length 0: there is no row len - 1."""
+    nH, nKV, hd, rows = 8, 2, 256, 64
+    k8 = torch.full((rows, nKV, hd), 5, dtype=torch.int8, device="cuda")
+    pool = [k8, k8.clone(), torch.ones((rows, nKV), device="cuda"), torch.ones((rows, nKV), device="cuda")]
+    before = [t.clone() for t in pool]
+    new = torch.randn((1, nKV, hd), device="cuda")
+    out = torch.full((1, nH, hd), float("nan"), device="cuda")
+    ops.decode_i8_batch(torch.randn((1, nH, hd), device="cuda"), *pool, out, ops.workspace(1, nH, hd, 4),
+                        torch.zeros(1, dtype=torch.int32, device="cuda"), 1, nH, nKV, hd, rows, 4, rows_per_seq=rows,
+                        append=(new, new))
+    torch.cuda.synchronize()
+    assert ops.device_status(raise_on_flags=False) == 32
+    assert (out == 0).all()
+    for a, b in zip(pool, before):
+        assert torch.equal(a, b)

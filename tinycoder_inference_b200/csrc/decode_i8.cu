@@ -83,8 +83,9 @@ decodeI8Kernel(const __grid_constant__ DecodeI8Params p) {
     } else {
         // (the host's length is the upper bound of a device length)
         len = p.devLens ? min(p.devLens[b] + p.lenAdd, p.lenHost) : p.lenHost;
-        // a cluster behind the last row leaves as a whole: the merge derives the active count from len
-        if ((chunk - clusterRank()) * p.chunkTokens >= len) return;
+        // a cluster behind the last row leaves as a whole: the merge derives the active count from len.  The first one stays: it
+        // writes the zeros of a sequence without rows
+        if ((chunk - clusterRank()) * p.chunkTokens >= len && chunk != clusterRank()) return;
     }
     const uint32_t t0 = ROWS ? 0u : chunk * p.chunkTokens;
     if (!ROWS && clusterSize() > 1) clusterHello();
@@ -103,7 +104,8 @@ decodeI8Kernel(const __grid_constant__ DecodeI8Params p) {
     // the warp that takes the last tile stores the token's row; into the tile itself when that is among its first ones
     const bool append = !ROWS && p.appendK != nullptr && t1 == len && nTiles != 0;
     const uint64_t newRow = rowBase + (!ROWS && p.devLens ? p.devLens[b] + p.lenAdd : len) - 1u;
-    const bool outside = append && newRow >= p.totalRows;  // a device length outside the pool: no row written
+    // a device length outside the pool (or no length at all): no row written
+    const bool outside = (append && newRow >= p.totalRows) || (!ROWS && p.appendK != nullptr && len == 0u);
     if (outside && threadIdx.x == 0) atomicOr(p.err, kDevErrRowBound);
     const bool mine = append && !outside && (nTiles - 1u) % NW == warp;
     const bool intoTile = mine && (nTiles - 1u) / NW < NS;

@@ -227,8 +227,9 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     }
     const uint32_t share = tokensOfBlock();
     const uint32_t t0 = chunk * share;
-    // inactive chunk (block-uniform): the merge derives the active count from len
-    if (FOLD != TcFold::kCluster && t0 >= len) return;
+    // inactive chunk (block-uniform): the merge derives the active count from len.  (The block that writes the output by
+    // itself stays: a sequence without rows gets zeros.)
+    if (FOLD != TcFold::kCluster && t0 >= len && (chunk != 0u || !p.directOut)) return;
     const uint32_t t1 = min(len, t0 + share);
     const uint32_t nTiles = t0 >= len ? 0u : (t1 - t0 + T - 1) / T;
     // Plain stream order: the kernels ahead are complete by now, and the block that stores a token's row lets the next grid
