@@ -520,3 +520,16 @@ def test_a_new_row_of_a_sequence_without_rows_is_flagged():
     assert (out == 0).all()
     for a, b in zip(pool, before):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("hd", [128, 256])
+def test_the_reported_chunk_slots_are_within_the_callers(hd):
+    nH, nKV, ctx = 8, 2, 8192
+    k8 = torch.zeros((ctx, nKV, hd), dtype=torch.int8, device="cuda")
+    s = torch.ones((ctx, nKV), device="cuda")
+    q = torch.randn((1, nH, hd), device="cuda")
+    for chunks in (1, 2, 40):
+        used = ops.decode_i8_batch(q, k8, k8, s, s, torch.empty_like(q), ops.workspace(1, nH, hd, chunks), None, 1, nH, nKV, hd,
+                                   ctx, chunks)
+        assert 1 <= used <= chunks
+    torch.cuda.synchronize()

@@ -794,7 +794,7 @@ int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, c
     const bool pdl = (d->flags & TC_DECODE_PDL) != 0;
     const bool direct = (pl.chunksPerSeq == 1 || cluster > 1) && !d->partialsOnly;
     if (!direct) TC_REQUIRE(d->pAcc && d->pM && d->pL, TC_EWORKSPACE, "decode_i8: partial buffers are required");
-    if (d->chunksUsed) *d->chunksUsed = pl.chunksPerSeq;
+    if (d->chunksUsed) *d->chunksUsed = cluster > 1 ? 1u : pl.chunksPerSeq;  // (a cluster's blocks write no slots)
     TC_REQUIRE(d->nKV <= 65535, TC_EUNSUPPORTED, "decode_i8: %u kv heads", d->nKV);
 
     TensorMapKey key;
