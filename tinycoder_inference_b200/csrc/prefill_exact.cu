@@ -18,6 +18,13 @@
 // form head by head took 79 us, 62 now.  Measured (8-row form -> this one): f32 512 rows of 14 / 2 / 64 39.7 -> 18.7 us,
 // of 28 / 4 / 128 120 -> 62, 333 of 16 / 2 / 256 77 -> 52; fp16 100 rows of 28 / 4 / 128 15.0 -> 6.4 us, 512 behind 512
 // 107 -> 71, 2000 rows of 8 / 4 / 64 81 -> 40.
+//
+// What keeps it exact: a tensor-core product drops the bits of a running sum that do not fit, and those losses add up
+// along a chain.  The 8-row form has up to sixteen warps and so as many sums per output; four token groups with one
+// running sum each were further from a 64-bit evaluation (head_dim 64, 200 rows behind 6000: f32 5.6e-6 -> 1.1e-5 of the
+// result's norm, fp16 512 behind 1000 5.5e-7 -> 9.1e-7).  So where it is needed (kOwnSums, and the fp16 form) a stage's
+// products are summed by themselves, the small terms apart (f32) or first (fp16), and added to O in f32: 4.0e-7 and 2.9e-7,
+// for 1 - 3 % more time.  At head_dim 128 and 256 the f32 form's short stages are no further off than the 8-row form was, and keep one sum.
 #include "decode_cluster.cuh"
 
 namespace tc {
@@ -39,6 +46,7 @@ static constexpr int kExactRT = 2, kExactNH = 4, kExactWarps = kExactRT * kExact
 template <int HD>
 struct ExactShape {
     static constexpr int TG = 2048 / HD, kRows = kExactRows, kStage = kExactNH * TG;
+    static constexpr bool kOwnSums = HD == 64;  // see the head of the file
     static constexpr int kLd = HD + 4;  // floats per row of a plane: eight rows hit different banks
     static constexpr int kQ = 0;                                  // planes (hi, lo): q [kRows][kLd],
     static constexpr int kK = kQ + 2 * kRows * kLd;               // K [kStage][kLd],
@@ -251,6 +259,15 @@ __global__ void __launch_bounds__(kExactWarps * 32, 1) prefillExactKernel(const 
         }
         // ---- O += P V.  The k slots t / t + 4 of an 8-token step stand for tokens 2t / 2t + 1: the accumulator layout
         // of the scores is the A operand then, and V is read with rows 2t, 2t + 1 ----
+        float own[S::kOwnSums ? HD / 8 : 1][4], ownCross[S::kOwnSums ? HD / 8 : 1][4];  // this stage's hi*hi, and the cross terms
+        auto sum = [&](int d) -> float (&)[4] { return S::kOwnSums ? own[S::kOwnSums ? d : 0] : o[d]; };
+        auto cross = [&](int d) -> float (&)[4] { return S::kOwnSums ? ownCross[S::kOwnSums ? d : 0] : o[d]; };
+        if (S::kOwnSums) {
+#pragma unroll
+            for (int d = 0; d < HD / 8; ++d)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) sum(d)[i] = cross(d)[i] = 0.0f;
+        }
 #pragma unroll
         for (int n = 0; n < NT; ++n) {
             float ph[4], pl[4];
@@ -277,12 +294,18 @@ __global__ void __launch_bounds__(kExactWarps * 32, 1) prefillExactKernel(const 
                     b[d][2] = u(a0[S::kStage * LD]), b[d][3] = u(a1[S::kStage * LD]);
                 }
 #pragma unroll
-                for (int d = 0; d < DB; ++d) mmaTf32(o[d0 + d], u(ph[0]), u(ph[1]), u(ph[2]), u(ph[3]), b[d][0], b[d][1]);
+                for (int d = 0; d < DB; ++d) mmaTf32(sum(d0 + d), u(ph[0]), u(ph[1]), u(ph[2]), u(ph[3]), b[d][0], b[d][1]);
 #pragma unroll
-                for (int d = 0; d < DB; ++d) mmaTf32(o[d0 + d], u(pl[0]), u(pl[1]), u(pl[2]), u(pl[3]), b[d][0], b[d][1]);
+                for (int d = 0; d < DB; ++d) mmaTf32(cross(d0 + d), u(pl[0]), u(pl[1]), u(pl[2]), u(pl[3]), b[d][0], b[d][1]);
 #pragma unroll
-                for (int d = 0; d < DB; ++d) mmaTf32(o[d0 + d], u(ph[0]), u(ph[1]), u(ph[2]), u(ph[3]), b[d][2], b[d][3]);
+                for (int d = 0; d < DB; ++d) mmaTf32(cross(d0 + d), u(ph[0]), u(ph[1]), u(ph[2]), u(ph[3]), b[d][2], b[d][3]);
             }
+        }
+        if (S::kOwnSums) {
+#pragma unroll
+            for (int d = 0; d < HD / 8; ++d)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) o[d][i] += sum(d)[i] + cross(d)[i];
         }
     }
     exactFold<HD>(sm, o, m0, m1, l0, l1, nh, rt, rows,
@@ -440,37 +463,44 @@ prefillExactHalfKernel(const __grid_constant__ PrefillExactParams p) {
                 m0 = mn0;
                 m1 = mn1;
             }
+            // 16 tokens at a time: the accumulator layout of the scores is the A operand's
+            uint32_t ph[NT / 2][4], pl[NT / 2][4];
 #pragma unroll
-            for (int n = 0; n < NT; n += 2) {  // 16 tokens: the accumulator layout of the scores is the A operand's
-                uint32_t ph[4], pl[4];
+            for (int n = 0; n < NT; ++n) {
+                float h[4], l[4];
+                const float p0 = fastExp2(s[n][0] - m0), p1 = fastExp2(s[n][1] - m0);
+                const float p2 = fastExp2(s[n][2] - m1), p3 = fastExp2(s[n][3] - m1);
+                l0 += p0 + p1;
+                l1 += p2 + p3;
+                splitHalf(p0, h[0], l[0]);
+                splitHalf(p1, h[1], l[1]);
+                splitHalf(p2, h[2], l[2]);
+                splitHalf(p3, h[3], l[3]);
+                const int k = n % 2;
+                ph[n / 2][2 * k] = packHalf2(h[0], h[1]), ph[n / 2][2 * k + 1] = packHalf2(h[2], h[3]);
+                pl[n / 2][2 * k] = packHalf2(l[0], l[1]), pl[n / 2][2 * k + 1] = packHalf2(l[2], l[3]);
+            }
+            constexpr int DB = HD == 64 ? 2 : 4;  // pairs of dim tiles at a time, their chains alternating
 #pragma unroll
-                for (int k = 0; k < 2; ++k) {
-                    float h[4], l[4];
-                    const float p0 = fastExp2(s[n + k][0] - m0), p1 = fastExp2(s[n + k][1] - m0);
-                    const float p2 = fastExp2(s[n + k][2] - m1), p3 = fastExp2(s[n + k][3] - m1);
-                    l0 += p0 + p1;
-                    l1 += p2 + p3;
-                    splitHalf(p0, h[0], l[0]);
-                    splitHalf(p1, h[1], l[1]);
-                    splitHalf(p2, h[2], l[2]);
-                    splitHalf(p3, h[3], l[3]);
-                    ph[2 * k] = packHalf2(h[0], h[1]), ph[2 * k + 1] = packHalf2(h[2], h[3]);
-                    pl[2 * k] = packHalf2(l[0], l[1]), pl[2 * k + 1] = packHalf2(l[2], l[3]);
-                }
-                constexpr int DB = 4;  // pairs of dim tiles at a time, their chains alternating
+            for (int d0 = 0; d0 < HD / 16; d0 += DB) {
+                float sum[2 * DB][4] = {};  // a stage's products by themselves (see the head of the file)
 #pragma unroll
-                for (int d0 = 0; d0 < HD / 16; d0 += DB) {
+                for (int n = 0; n < NT / 2; ++n) {
                     uint32_t b[DB][4];
 #pragma unroll
                     for (int d = 0; d < DB; ++d)
-                        ldmatrixX4Trans(b[d][0], b[d][1], b[d][2], b[d][3], base + vOff + n * (8 * LD * 2) + (d0 + d) * 32);
+                        ldmatrixX4Trans(b[d][0], b[d][1], b[d][2], b[d][3], base + vOff + n * (16 * LD * 2) + (d0 + d) * 32);
 #pragma unroll
                     for (int d = 0; d < 2 * DB; ++d)
-                        mmaF16(o[2 * d0 + d], ph[0], ph[1], ph[2], ph[3], b[d / 2][d % 2 * 2], b[d / 2][d % 2 * 2 + 1]);
+                        mmaF16(sum[d], pl[n][0], pl[n][1], pl[n][2], pl[n][3], b[d / 2][d % 2 * 2], b[d / 2][d % 2 * 2 + 1]);
 #pragma unroll
                     for (int d = 0; d < 2 * DB; ++d)
-                        mmaF16(o[2 * d0 + d], pl[0], pl[1], pl[2], pl[3], b[d / 2][d % 2 * 2], b[d / 2][d % 2 * 2 + 1]);
+                        mmaF16(sum[d], ph[n][0], ph[n][1], ph[n][2], ph[n][3], b[d / 2][d % 2 * 2], b[d / 2][d % 2 * 2 + 1]);
                 }
+#pragma unroll
+                for (int d = 0; d < 2 * DB; ++d)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) o[2 * d0 + d][i] += sum[d][i];
             }
         }
         __syncthreads();  // everybody is through with the stage
