@@ -10,10 +10,13 @@
 // Same skeleton as the f32 kernel (decode_kv.cu) -- a block streams a token range of one kv head,
 // its warps take 16-token tiles in turn and serve every q head of the kv head, decode_cluster.cuh
 // around it -- with the natural operands: fp16 K and V go into mma.sync.m16n8k16 as they are (ldmatrix for K,
-// ldmatrix.trans for V, both straight from the 128-byte-swizzled TMA tiles), q and p are
+// ldmatrix.trans for V, both straight from the tiles that each warp copies for itself, 128-byte swizzled), q and p are
 // carried as fp16 hi + lo pairs (two MMAs, ~22 mantissa bits) after a power-of-two
 // normalisation of q, accumulation is f32.  Nothing is rounded that the reference does not
-// round: float(k) and float(v) are exact.
+// round: float(k) and float(v) are exact.  (A tensor-core product drops the bits of its running sum that do not fit, and
+// those losses add up over a warp's tiles, hence the sums per tile; the small terms go first.  28 / 4 / 128, distance from
+// a 64-bit evaluation with one sum throughout -> like this: 8191 rows 4.2e-7 -> 3.2e-7, 40000 rows 7.9e-7 -> 3.4e-7, for
+// 7.71 -> 7.87 and 20.8 -> 21.0 us; the additions put off until the next tile's scores are under way: 7.93.)
 #include "decode_cluster.cuh"
 
 namespace tc {
@@ -183,6 +186,8 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKv16Kernel(const __grid_co
     float o[NS][4];
 #pragma unroll
     for (int i = 0; i < NS; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
+    // Where a warp takes several tiles (SLOTS > 1), a tile's products have sums of their own: see the head of the file.
+    constexpr bool kOwnSums = SLOTS > 1;
 
     const uint32_t lr = (lane & 7u) + ((lane >> 3) & 1u) * 8u;  // ldmatrix row this lane addresses
     const uint32_t lco = lane >> 4;                             // and which 16-byte chunk of the pair
@@ -270,8 +275,14 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKv16Kernel(const __grid_co
             r1 &= mk1;
             r3 &= mk1;
             // A rows g / g+8 = dims 16ks + g / + 8 + g; k = tokens
-            mmaF16(o[ks], r0, r2, r1, r3, bh[0], bh[1]);
-            mmaF16(o[ks], r0, r2, r1, r3, bl[0], bl[1]);
+            float own[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            float(&sum)[4] = kOwnSums ? own : o[ks];
+            mmaF16(sum, r0, r2, r1, r3, bl[0], bl[1]);
+            mmaF16(sum, r0, r2, r1, r3, bh[0], bh[1]);
+            if (kOwnSums) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) o[ks][i] += own[i];
+            }
         }
         __syncwarp();
         requestV(i + SLOTS);
