@@ -532,8 +532,6 @@ static int prefillI8(const float *q, const int8_t *k8, const int8_t *v8, const f
     prm.directOut = 1;
     prm.err = devErrorWord();
     TC_REQUIRE(prm.err != nullptr, TC_ECUDA, "prefill_i8: no device error word");
-    // heaviest row blocks first would need a reversed grid; the hardware scheduler
-    // hands out blocks in z-major order, so late (long) blocks start last -- acceptable here
     if (hd == 256) return launchRowsI8<256, 1>(prm, st);
     return launchRowsI8<128, 2>(prm, st);
 }

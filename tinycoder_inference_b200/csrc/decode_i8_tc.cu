@@ -774,7 +774,9 @@ int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, c
     // cost more than the launch: a tile more per block takes 0.3 us while latency is what bounds it.  7B shape, per layer in
     // a graph: 8192 rows 8.4 -> 7.1 us, 8 sequences of 2048 / 8192 rows 10.7 -> 8.3 / 18.1 -> 16.1, 16384 rows 9.0 in
     // either form.  With ragged device lengths the cluster also shares every sequence evenly among its blocks, where the
-    // merge form cuts chunks by the longest one.
+    // merge form cuts chunks by the longest one.  There the line is 20 tiles per block of the longest sequence: cluster
+    // against merge, 2 / 3 / 4 / 8 sequences of up to 6000 rows (6 - 12 tiles) 0.44 / 0.48 / 0.66 / 0.67 of the time, up to 20000
+    // (20 tiles, 2 and 3 sequences) 0.83 and 0.87, up to 12000 (24 tiles, 4 and 8) 0.93 and 0.98, up to 32768 (32, 2 and 3) 1.15.
     static ClusterSetup setup;
     const uint32_t *limits = nullptr;
     int rc = setupCluster(setup, decodeI8TcKernel<2, 6, true, TcFold::kCluster>, Smem::kThreads, Smem::kTotal, &limits);
@@ -818,8 +820,10 @@ int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, c
     rc = getTensorMap(key, &tmV);
     if (rc != TC_OK) return rc;
     CUtensorMap tmKn = tmK, tmVn = tmV;
-    // the next call's pools, pulled into L2 behind this call's rows; larger calls keep HBM busy by themselves (50000 rows,
-    // 53 MB: 14.4 us per layer without, 14.7 with)
+    // the next call's pools, pulled into L2 behind this call's rows; larger calls keep HBM busy by themselves.  (With the hint
+    // against without it, per layer of pools that do not fit L2 together: 20000 rows 8.70 / 9.25 us, 32768 rows 10.90 /
+    // 10.98, 47000 rows (46 MiB) 14.04 / 13.55, 50000 rows 14.25 / 14.02, 80000 rows 18.13 / 18.46; 4 sequences of 8192 rows
+    // 12.2 / 11.7, 8 of 8192 14.24 / 14.60.  It pays where a call is short; from some 30 MB on it is within 4 % either way.)
     const uint64_t callBytes = static_cast<uint64_t>(d->batch) * d->maxLen * d->nKV * hd * 2ull;
     const bool prefetchNext = d->nextK8 != nullptr && d->nextV8 != nullptr && callBytes <= (48ull << 20);
     if (prefetchNext) {

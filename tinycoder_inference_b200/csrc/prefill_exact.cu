@@ -9,13 +9,13 @@
 // lo*hi + hi*lo keeps about 21 mantissa bits and the full exponent range, f32 accumulation).
 //
 // What bounds it: the issue slots.  With 8 query rows at a time (the causal form of the decode kernels, which stays for
-// few rows behind a long prefix: prefillForm below) every warp splits K and V into hi and lo for itself, half of the 370
+// few rows behind a long prefix: prefillExactWins below) every warp splits K and V into hi and lo for itself, half of the 370
 // instructions it spends on a 16-token tile.  Here a block of 32 query rows of one q head splits a stage of K and V once
 // into planes in shared memory, and a warp works on 16 rows x TG tokens: ldmatrix operands, three products each.  The
 // four token groups of a block take their share of every stage (a short prompt is a chain of stages, not a matter of
 // bytes) and are put together at the end.  (Blocks of 64 rows and two token groups leave fewer and longer chains: 512
 // rows of 28 / 4 / 128 83 us against 79.)  The late rows of all heads come first, so that what starts last is short: that
-// form head by head took 79 us, 62 now.  Measured (8-row form -> this one): f32 512 rows of 14 / 2 / 64 39.7 -> 18.7 us,
+// form head by head took 79 us, 62 now (fp16, 512 behind 512 of 28 / 4 / 128, is the one that lost: 67.6 -> 70.7).  Measured (8-row form -> this one): f32 512 rows of 14 / 2 / 64 39.7 -> 18.7 us,
 // of 28 / 4 / 128 120 -> 62, 333 of 16 / 2 / 256 77 -> 52; fp16 100 rows of 28 / 4 / 128 15.0 -> 6.4 us, 512 behind 512
 // 107 -> 71, 2000 rows of 8 / 4 / 64 81 -> 40.
 //

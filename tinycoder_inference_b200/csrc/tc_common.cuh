@@ -243,24 +243,10 @@ __device__ __forceinline__ uint32_t toTf32(float x) {
 }
 
 // ---- exact int8 -> fp16 ----------------------------------------------------------
-// w holds four int8 already xor-ed with 0x80 (i.e. x + 128 as unsigned bytes).
-// Bytes (b0, b1) become the fp16 pair (x0, x1): 0x6400 | u is 1024 + u exactly,
-// minus 1152 gives x.  Two instructions per pair, no rounding anywhere.
-__device__ __forceinline__ uint32_t biasedPairLo(uint32_t w) {
-    uint32_t h = __byte_perm(w, 0x64646464u, 0x4140);
-    __half2 r = __hsub2(*reinterpret_cast<__half2 *>(&h), __half2half2(__ushort_as_half(0x6480)));
-    return *reinterpret_cast<uint32_t *>(&r);
-}
-__device__ __forceinline__ uint32_t biasedPairHi(uint32_t w) {
-    uint32_t h = __byte_perm(w, 0x64646464u, 0x4342);
-    __half2 r = __hsub2(*reinterpret_cast<__half2 *>(&h), __half2half2(__ushort_as_half(0x6480)));
-    return *reinterpret_cast<uint32_t *>(&r);
-}
-
-// Cheaper exact form used by the decode kernel: a byte u placed in the low mantissa
-// bits of an fp16 with zero exponent IS the subnormal u * 2^-24, exactly.  With
-// u = x + 128 (w already xor-ed with 0x80) the operand carries a +128 offset that
-// the caller removes after the MMA with a per-column sum; one prmt per pair.
+// A byte u placed in the low mantissa bits of an fp16 with zero exponent IS the
+// subnormal u * 2^-24, exactly.  With u = x + 128 (w holds four int8 already xor-ed with
+// 0x80) the operand carries a +128 offset that the caller removes after the MMA with a
+// per-column sum; one prmt per pair.
 template <uint32_t SEL>
 __device__ __forceinline__ uint32_t subnormalPair(uint32_t w) {
     return __byte_perm(w, 0u, SEL);
