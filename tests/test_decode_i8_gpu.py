@@ -533,3 +533,36 @@ def test_the_reported_chunk_slots_are_within_the_callers(hd):
                                    ctx, chunks)
         assert 1 <= used <= chunks
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("nH,nKV", [(4, 1), (10, 2), (12, 2), (7, 1), (8, 1)])
+@pytest.mark.parametrize("ctx", [1, 128, 129, 768, 769, 897, 1700])
+@pytest.mark.parametrize("chunks", [1, 64])
+def test_appended_row_in_its_tile(nH, nKV, ctx, chunks):
+    """The appended row at the edges of a tile, in and behind the first ring of tiles (one block per sequence, or a cluster),
+    for every width of the score loop.  The pool's row holds NaN scales before the call: neither they nor the stale bytes
+    may reach the result."""
+    hd, B = 128, 2
+    rng = np.random.default_rng(1000 * chunks + 10 * ctx + nH)
+    q = rng.standard_normal((B, nH, hd), dtype=np.float32)
+    k = rng.standard_normal((B, ctx, nKV, hd), dtype=np.float32)
+    v = rng.standard_normal((B, ctx, nKV, hd), dtype=np.float32)
+    stores = [make_i8_store(k[b], v[b], nKV, hd) for b in range(B)]
+    pool = [np.concatenate([s[i] for s in stores]) for i in range(4)]
+    stale = [x.copy() for x in pool]
+    for b in range(B):
+        row = b * ctx + ctx - 1
+        stale[0][row], stale[1][row] = 127, -128
+        stale[2][row] = stale[3][row] = np.nan
+    d = [dev(x) for x in stale]
+    out = torch.full((B, nH, hd), float("nan"), device="cuda")
+    ops.decode_i8_batch(dev(q), *d, out, ops.workspace(B, nH, hd, chunks), None, B, nH, nKV, hd, ctx, chunks, rows_per_seq=ctx,
+                        append=(dev(np.ascontiguousarray(k[:, -1])), dev(np.ascontiguousarray(v[:, -1]))))
+    torch.cuda.synchronize()
+    assert ops.device_status() == 0
+    for got, want in zip(d, pool):
+        assert np.array_equal(host(got)[:B * ctx], want[:B * ctx])
+    inv = 1.0 / math.sqrt(hd)
+    for b in range(B):
+        want = oracle.attention_i8(q[b:b + 1], *[x[b * ctx:(b + 1) * ctx] for x in pool], 1, nH, nKV, hd, ctx - 1, inv)
+        assert_close(host(out)[b:b + 1], want, what=f"sequence {b}")

@@ -27,9 +27,17 @@
 // CTA = one kv head x one token range (grid: chunks, kv heads, sequences), 17 warps:
 // warps 0-3 / 4-7 two softmax warpgroups taking alternate tiles (scores -> probabilities only),
 // warps 8-11 the fold warpgroup (thread = head dimension: every tile's integer P.V out of TMEM into
-// one f32 accumulator per head, so a softmax warpgroup's next tile does not wait for the previous
+// f32 accumulators, so a softmax warpgroup's next tile does not wait for the previous
 // one's fold), warp 12 TMA producer (six-stage ring of K, V and their scales), warps 13-16 issue the
 // MMAs (score / P.V products of even / odd tiles; one elected thread of each).  Partials leave in the reference's layout for the merge kernel (merge.cu).
+//
+// What bounds it up to some ten megabytes of rows is a chain of latencies: a softmax warp issues an instruction of its tile every
+// five cycles or so, alone on its scheduler or not.  So the loops carry as few as they can: digit planes combine two at a time in
+// integers before the conversions, only the q heads there are (NH) are worked on, the fold keeps accumulators per softmax
+// warpgroup and rescales them when the reference point moved, one arrival per warp, one barrier wait per tile of a softmax
+// thread.  A steady tile takes it 970 cycles (1280 before); the first one, whose reference point has to be agreed on, 0.5 us
+// (0.8 with shuffles in place of redux.max).  28 / 4 heads, per layer: 32768 rows 10.95 -> 10.15 us, 4098 rows with an f32 mirror
+// 7.2 -> 6.65, 8 sequences of 8192 15.0 -> 14.3, 64 of 512 - 32768 rows 197 -> 190.
 #include <cstdlib>
 
 #include "tc_tcgen05.cuh"
@@ -92,10 +100,12 @@ struct DecodeTcSmem {
     static constexpr int kP = kQd + 4096;                         // 2 NWG probability tiles of 128 x 32 B
     static constexpr int kRed = kP + 2 * NWG * 4096;              // [NWG warpgroups][4 warps][12] floats
     static constexpr int kHs = kRed + NWG * 4 * 12 * 4;           // head scales [8]
-    static constexpr int kMeta = kHs + 64;                        // per (warpgroup, buffer): reference points [8], tile scale
-    static constexpr int kBars = kMeta + 2 * NWG * 12 * 4;
-    // full[NS], empty[NS], sFull[2 NWG], pFull[2 NWG], oFull[2 NWG], oFree[2 NWG], qFull
-    static constexpr int kNumBars = 2 * NS + 8 * NWG + 1;
+    // per (warpgroup, tile of the warpgroup % 4): reference points [8], tile scale, whether they moved.  Four, not two, slots:
+    // scores of tile j wait for the P.V product of tile j - 2 NWG, which waits for the fold of tile j - 4 NWG.
+    static constexpr int kMeta = kHs + 64;
+    static constexpr int kBars = kMeta + 4 * NWG * 12 * 4;
+    // full[NS], empty[NS], sFull[2 NWG], pFull[2 NWG], oFull[2 NWG], oFree[2 NWG], qFull, rowFull
+    static constexpr int kNumBars = 2 * NS + 8 * NWG + 2;
     static constexpr int kTmemCols = 128 * NWG;                   // S and O buffers of 32 columns each
     static constexpr int kTmemSlot = kBars + kNumBars * 8;
     static constexpr int kTotal = kTmemSlot + 16 + 1024;
@@ -155,6 +165,12 @@ __device__ __forceinline__ bool barOr(uint32_t id, uint32_t threads, bool pred) 
             : "memory");
     return r != 0;
 }
+// maximum over the warp (NaN is ignored, as in fmaxf)
+__device__ __forceinline__ float warpMax(float x) {
+    float r;
+    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+    return r;
+}
 __device__ __forceinline__ float i2f(uint32_t x) { return __int2float_rn(static_cast<int>(x)); }
 
 // APPEND: the instantiation for calls that hand in the new token's rows.  It is a kernel of its own
@@ -163,7 +179,9 @@ __device__ __forceinline__ float i2f(uint32_t x) { return __int2float_rn(static_
 // FOLD: how a sequence's blocks come together: a merge launch (or one block per sequence, which writes the output), the
 // last block to arrive (tickets), or a cluster that holds them all and folds through distributed shared memory.
 enum class TcFold { kLaunch, kTickets, kCluster };
-template <int NWG, int NS, bool APPEND, TcFold FOLD>
+// NH: columns the softmax and fold threads work on, the q heads of a kv head (at most 8 per launch) -- not a runtime bound,
+// which would put a branch in front of every column of the unrolled loops.
+template <int NWG, int NS, int NH, bool APPEND, TcFold FOLD>
 __global__ void __launch_bounds__((4 * NWG + 9) * 32, 1)
 decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                  const __grid_constant__ CUtensorMap tmKn, const __grid_constant__ CUtensorMap tmVn,
@@ -180,7 +198,7 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L::kBars);
     uint64_t *fullBar = bars, *emptyBar = bars + NS, *sFull = bars + 2 * NS, *pFull = sFull + 2 * NWG,
-             *oFull = pFull + 2 * NWG, *oFree = oFull + 2 * NWG, *qFull = oFree + 2 * NWG;
+             *oFull = pFull + 2 * NWG, *oFree = oFull + 2 * NWG, *qFull = oFree + 2 * NWG, *rowFull = qFull + 1;
     uint32_t *tmemSlot = reinterpret_cast<uint32_t *>(smem + L::kTmemSlot);
     float *sHs = reinterpret_cast<float *>(smem + L::kHs);
 
@@ -192,18 +210,16 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         }
         for (int i = 0; i < 2 * NWG; ++i) {
             mbarInit(&sFull[i], 1);
-            mbarInit(&pFull[i], 128);
+            mbarInit(&pFull[i], 4);  // (an arrival per warp: 128 of them serialise on the barrier)
             mbarInit(&oFull[i], 1);
-            mbarInit(&oFree[i], 128);
+            mbarInit(&oFree[i], 4);
         }
-        mbarInit(qFull, 256);
+        mbarInit(qFull, 8);
+        mbarInit(rowFull, 1);
         fenceBarrierInit();
         tmaPrefetchDesc(&tmK);
         tmaPrefetchDesc(&tmV);
     }
-    __syncthreads();
-    if (p.dependent) gridDepLaunch();  // the next grid (the merge) may be scheduled as soon as room frees up
-
     // The length may live in device memory written by an earlier kernel; only a host-known
     // length lets the producer start before the dependency wait.
     uint32_t len = p.lenHost;
@@ -212,6 +228,22 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     auto tokensOfBlock = [&]() {
         return FOLD == TcFold::kCluster ? ((len + T - 1u) / T + gridDim.x - 1u) / gridDim.x * T : p.chunkTokens;
     };
+    // inactive chunk (block-uniform): the merge derives the active count from len.  (The block that writes the output by
+    // itself stays: a sequence without rows gets zeros.)
+    auto inactive = [&]() { return FOLD != TcFold::kCluster && chunk * tokensOfBlock() >= len && (chunk != 0u || !p.directOut); };
+    auto allocTmem = [&]() {
+        if (warp != 0) return;
+        __syncwarp();
+        tmemAlloc(tmemSlot, L::kTmemCols);
+        tmemRelinquish();
+        tcFenceBefore();
+    };
+    // Tensor memory ahead of the dependency wait, where the length already says that the block will need it.
+    const bool allocEarly = p.devLens == nullptr && !inactive();
+    if (allocEarly) allocTmem();
+    __syncthreads();
+    if (p.dependent) gridDepLaunch();  // the next grid (the merge) may be scheduled as soon as room frees up
+
     if (!earlyOk) {
         // pulling this block's rows into L2 is right at any time: a row that a kernel in flight writes is read after the wait
         if (p.devLens == nullptr && p.devRowBase == nullptr && warp == kProducerWarp && lane < NS) {
@@ -227,9 +259,7 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     }
     const uint32_t share = tokensOfBlock();
     const uint32_t t0 = chunk * share;
-    // inactive chunk (block-uniform): the merge derives the active count from len.  (The block that writes the output by
-    // itself stays: a sequence without rows gets zeros.)
-    if (FOLD != TcFold::kCluster && t0 >= len && (chunk != 0u || !p.directOut)) return;
+    if (inactive()) return;
     const uint32_t t1 = min(len, t0 + share);
     const uint32_t nTiles = t0 >= len ? 0u : (t1 - t0 + T - 1) / T;
     // Plain stream order: the kernels ahead are complete by now, and the block that stores a token's row lets the next grid
@@ -242,13 +272,10 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     const uint32_t foldPer = CLUSTER ? (foldTotal + clusterSize() - 1u) / clusterSize() : 0u;
     if constexpr (CLUSTER) clusterHello();
     const uint64_t rowBase = p.devRowBase ? p.devRowBase[b] : static_cast<uint64_t>(b) * p.rowsPerSeq;
-
-    if (warp == 0) {
-        tmemAlloc(tmemSlot, L::kTmemCols);
-        tmemRelinquish();
-        tcFenceBefore();
+    if (!allocEarly) {
+        allocTmem();
+        __syncthreads();
     }
-    __syncthreads();
     tcFenceAfter();
     const uint32_t tmemBase = *reinterpret_cast<volatile uint32_t *>(tmemSlot);
     if (threadIdx.x == 0) TC_STAMP(1);
@@ -282,7 +309,8 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
             asm volatile("prefetch.global.L2 [%0];" ::"l"(src));
         }
         bool waited = !earlyOk;
-        auto requestTile = [&](uint32_t it) -> bool {
+        // K and V of tile `it`, completion on `bar` (its stage's fullBar, but for the tile with the appended row)
+        auto requestRows = [&](uint32_t it, uint64_t *bar) -> bool {
             const uint32_t s = it % NS;
             if (it >= NS && !mbarWait(&emptyBar[s], ((it / NS) - 1u) & 1u, p.err, kDevErrEmptyWait)) return false;
             const uint32_t tok = t0 + it * T;
@@ -295,55 +323,79 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
             uint8_t *st = smem + s * L::kStageBytes;
             const uint64_t row = rowBase + tok;
             if (lane == 0) {
-                mbarExpectTx(&fullBar[s], 2 * L::kTileBytes);
+                mbarExpectTx(bar, 2 * L::kTileBytes);
                 if (p.l2Hints & 1) {
-                    tmaLoad3DHint(st, &tmK, &fullBar[s], 0, kvHead, static_cast<int>(row), polFirst);
-                    tmaLoad3DHint(st + L::kTileBytes, &tmV, &fullBar[s], 0, kvHead, static_cast<int>(row), polFirst);
+                    tmaLoad3DHint(st, &tmK, bar, 0, kvHead, static_cast<int>(row), polFirst);
+                    tmaLoad3DHint(st + L::kTileBytes, &tmV, bar, 0, kvHead, static_cast<int>(row), polFirst);
                 } else {
-                    tmaLoad3D(st, &tmK, &fullBar[s], 0, kvHead, static_cast<int>(row));
-                    tmaLoad3D(st + L::kTileBytes, &tmV, &fullBar[s], 0, kvHead, static_cast<int>(row));
+                    tmaLoad3D(st, &tmK, bar, 0, kvHead, static_cast<int>(row));
+                    tmaLoad3D(st + L::kTileBytes, &tmV, bar, 0, kvHead, static_cast<int>(row));
                 }
+                if (it == 0) TC_STAMP(13);
+                TC_STAMP(14);
             }
-            float *sK = reinterpret_cast<float *>(st + 2 * L::kTileBytes);
+            return true;
+        };
+        // its row scales but that of row `skip` of the tile (T: all of them)
+        auto requestScales = [&](uint32_t it, uint32_t skip) {
+            const uint32_t s = it % NS;
+            const uint64_t row = rowBase + t0 + it * T;
+            float *sK = reinterpret_cast<float *>(smem + s * L::kStageBytes + 2 * L::kTileBytes);
             float *sV = sK + T;
 #pragma unroll
             for (uint32_t idx = lane; idx < T; idx += 32) {
                 uint64_t r = row + idx;
                 r = r < p.totalRows ? r : p.totalRows - 1;
+                if (APPEND && idx == skip) continue;
                 cpAsync4(&sK[idx], p.ks + r * p.nKV + kvHead);
                 cpAsync4(&sV[idx], p.vs + r * p.nKV + kvHead);
             }
             cpAsyncMbarArriveNoinc(&fullBar[s]);
-            if (lane == 0) { if (it == 0) TC_STAMP(13); TC_STAMP(14); }
-            return true;
         };
-        // The tile that holds the row of a token being appended (the last tile of the sequence's last
-        // chunk) is requested apart from the loop: the row goes into the pool first, once the kernels
-        // ahead have completed.
+        // The tile that holds the row of a token being appended (the last tile of the sequence's last chunk) is requested apart
+        // from the others.  The row goes into the tile itself behind the tile's copies, and into the pool: read back from
+        // there, the tile came 1 us behind the other blocks' (28 / 4 heads, 4098 rows, f32 + int8: 6.75 us a layer, 6.5 like
+        // this).  (All rows of the ring ahead of the first scales: these arrive behind 200 KB, 32768 rows 10.0 -> 11.6 us.)
         const uint32_t nLoop = storesRow ? nTiles - 1u : nTiles;
         bool okP = true;
-        for (uint32_t it = 0; okP && it < nLoop; ++it) okP = requestTile(it);
+        for (uint32_t it = 0; okP && it < nLoop; ++it) {
+            okP = requestRows(it, &fullBar[it % NS]);
+            if (okP) requestScales(it, T);
+        }
         if (APPEND && storesRow && okP) {
             if (!waited) {
                 gridDepWait();
                 waited = true;
             }
-            const size_t srcRow = (static_cast<size_t>(b) * p.nKV + kvHead) * 32u;
             const uint64_t row = rowBase + (p.devLens ? p.devLens[b] + p.lenAdd : len) - 1u;
-            const uint64_t dst = row * p.nKV + kvHead;
             // a length read from device memory is checked where it is known: outside the pool the
             // store is skipped and the error word says so
-            if (row >= p.totalRows) {
-                if (lane == 0) atomicOr(p.err, kDevErrRowBound);
-            } else {
+            const bool outside = row >= p.totalRows;
+            if (outside && lane == 0) atomicOr(p.err, kDevErrRowBound);
+            // (a device length above the host's bound: the row is stored, and lies behind the attended ones)
+            const bool intoTile = !outside && row == rowBase + len - 1u;
+            const uint32_t it = nTiles - 1u, inTile = len - 1u - (t0 + it * T);
+            NewQuantRow<128, 128> fresh;
+            const size_t src = (static_cast<size_t>(b) * p.nKV + kvHead) * 128u;
+            fresh.load(p.appendK + src, p.appendV + src, lane);
+            okP = requestRows(it, rowFull);
+            if (okP) requestScales(it, intoTile ? inTile : T);
+            okP = okP && mbarWait(rowFull, 0, p.err, kDevErrFullWait);
+            if (okP && !outside) {
+                const uint64_t dst = row * p.nKV + kvHead;
                 float4 *mk = nullptr, *mv = nullptr;
                 if (p.mirK != nullptr) mk = reinterpret_cast<float4 *>(p.mirK) + dst * 32u, mv = reinterpret_cast<float4 *>(p.mirV) + dst * 32u;
-                appendQuantRow<128>(reinterpret_cast<const float4 *>(p.appendK) + srcRow,
-                                    reinterpret_cast<const float4 *>(p.appendV) + srcRow, reinterpret_cast<uint32_t *>(p.k8w),
-                                    reinterpret_cast<uint32_t *>(p.v8w), const_cast<float *>(p.ks), const_cast<float *>(p.vs), dst,
-                                    mk, mv, lane);
+                uint8_t *st = smem + (it % NS) * L::kStageBytes;
+                float *sc = reinterpret_cast<float *>(st + 2 * L::kTileBytes);
+                fresh.store(reinterpret_cast<uint32_t *>(p.k8w) + dst * 32u, reinterpret_cast<uint32_t *>(p.v8w) + dst * 32u,
+                            const_cast<float *>(p.ks) + dst, const_cast<float *>(p.vs) + dst, mk, mv, intoTile ? st : nullptr,
+                            st + L::kTileBytes, sc, sc + T, inTile, lane);
             }
-            requestTile(nTiles - 1u);
+            fenceProxyAsync();
+            __syncwarp();
+            if (okP && lane == 0) mbarArrive(&fullBar[it % NS]);
+            // (the pool's row is next read by another launch's copies)
+            asm volatile("fence.proxy.async.global;" ::: "memory");
             if (!p.dependent) {
                 __threadfence();
                 __syncwarp();
@@ -367,9 +419,10 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
             if (lane == 0 && par == 0) TC_STAMP(15);
             for (uint32_t j = par; ok && j < nTiles; j += 2u) {
                 const uint32_t s = j % NS, w = j % kWG, bb = (j / kWG) & 1u;
-                // the S buffer's previous contents (tile j - 2 NWG) have been read once that tile's P is out
+                // the P.V product of the buffers' previous tile (j - 2 NWG) is done: its scores have been read and its P tile
+                // is free -- the softmax threads need not wait for that once more
                 if (j >= 2u * kWG)
-                    ok = mbarWait(&pFull[2u * w + bb], ((j - 2u * kWG) / (2u * kWG)) & 1u, p.err, kDevErrMmaWait);
+                    ok = mbarWait(&oFull[2u * w + bb], ((j - 2u * kWG) / (2u * kWG)) & 1u, p.err, kDevErrMmaWait);
                 ok = ok && mbarWait(&fullBar[s], (j / NS) & 1u, p.err, kDevErrFullWait);
                 if (lane == 0 && j < 8u) TC_STAMP(20 + j);
                 if (!ok) break;
@@ -415,42 +468,66 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     } else if (warp >= kFoldWarp0) {
         // ------------------------------ fold warpgroup ------------------------------
         // thread = one head dimension: takes every tile's integer P.V out of TMEM in tile order and
-        // folds it into ONE f32 accumulator per head, against a running reference point of its own
-        // (the two softmax warpgroups keep separate ones; a tile arrives with the reference it was
-        // exponentiated against and with its fixed-point scale)
+        // folds it into one f32 accumulator per head and softmax warpgroup, against that warpgroup's reference point
+        // (a tile arrives with its fixed-point scale and, when it moved, the reference it was exponentiated against)
         const uint32_t wq = warp & 3u;
         const uint32_t row = wq * 32u + lane;
         const uint32_t laneBase = (wq * 32u) << 16;
         const float *meta = reinterpret_cast<const float *>(smem + L::kMeta);
-        float o[8], M[8];
+        // accumulators and their reference points by softmax warpgroup: within one, the reference moves with a tile or two
+        // of a call, and only then the accumulators are rescaled
+        float oW[NWG][NH], M[NWG][NH];
 #pragma unroll
-        for (int h = 0; h < 8; ++h) o[h] = 0.0f, M[h] = kNegBig;
+        for (int w = 0; w < NWG; ++w)
+#pragma unroll
+            for (int h = 0; h < NH; ++h) oW[w][h] = 0.0f, M[w][h] = kNegBig;
         bool ok = true;
-        for (uint32_t j = 0; ok && j < nTiles; ++j) {
-            const uint32_t w = j % kWG, bb = (j / kWG) & 1u, par = (j / (2u * kWG)) & 1u;
-            ok = mbarWait(&oFull[2u * w + bb], par, p.err, kDevErrMmaWait);
-            if (!ok) break;
-            tcFenceAfter();
-            uint32_t r[32];
-            tmemLd32(tmemBase + 64u * kWG + 32u * (2u * w + bb) + laneBase, r);
-            const float *mt = meta + (2u * w + bb) * 12u;
-            float tmr[8];
+        for (uint32_t j0 = 0; ok && j0 < nTiles; j0 += kWG) {
 #pragma unroll
-            for (int h = 0; h < 8; ++h) tmr[h] = mt[h];
-            const float esc = mt[8];
-            tmemLdWait();
-            tcFenceBefore();
-            mbarArrive(&oFree[2u * w + bb]);   // the buffer and its meta slot may be reused
+            for (uint32_t w = 0; w < kWG; ++w) {
+                const uint32_t j = j0 + w, bb = (j / kWG) & 1u, par = (j / (2u * kWG)) & 1u;
+                if (j >= nTiles) break;
+                ok = mbarWait(&oFull[2u * w + bb], par, p.err, kDevErrMmaWait);
+                if (!ok) break;
+                tcFenceAfter();
+                uint32_t r[32];
+                tmemLd32(tmemBase + 64u * kWG + 32u * (2u * w + bb) + laneBase, r);
+                const float *mt = meta + (4u * w + ((j / kWG) & 3u)) * 12u;
+                const float2 em = *reinterpret_cast<const float2 *>(mt + 8);  // scale of the tile, whether the reference moved
+                if (em.y != 0.0f) {
 #pragma unroll
-            for (int h = 0; h < 8; ++h) {
-                // column 4h + i carries byte i of the fixed-point probability: weight 256^i
-                const float c = fmaf(fmaf(fmaf(i2f(r[4 * h + 3]), 256.0f, i2f(r[4 * h + 2])), 256.0f, i2f(r[4 * h + 1])),
-                                     256.0f, i2f(r[4 * h]));
-                const float mn = fmaxf(M[h], tmr[h]);
-                o[h] = fmaf(c, esc * fastExp2(tmr[h] - mn), o[h] * fastExp2(M[h] - mn));
-                M[h] = mn;
+                    for (int h = 0; h < NH; ++h) {
+                        const float mn = mt[h];  // (a reference only ever grows)
+                        oW[w][h] *= fastExp2(M[w][h] - mn);
+                        M[w][h] = mn;
+                    }
+                }
+                tmemLdWait();
+                tcFenceBefore();
+                __syncwarp();
+                if (lane == 0) mbarArrive(&oFree[2u * w + bb]);   // the buffer and its meta slot may be reused
+#pragma unroll
+                for (int h = 0; h < NH; ++h) {
+                    // column 4h + i carries byte i of the fixed-point probability: weight 256^i; a sum is below 2^22, so
+                    // two of them combine exactly in 32 bits
+                    const int lo = static_cast<int>(r[4 * h + 1]) * 256 + static_cast<int>(r[4 * h]);
+                    const int hi = static_cast<int>(r[4 * h + 3]) * 256 + static_cast<int>(r[4 * h + 2]);
+                    const float c = fmaf(__int2float_rn(hi), 65536.0f, __int2float_rn(lo));
+                    oW[w][h] = fmaf(c, em.x, oW[w][h]);
+                }
+                if (threadIdx.x == kFoldWarp0 * 32u && j + 1u == nTiles) TC_STAMP(10);
             }
-            if (threadIdx.x == kFoldWarp0 * 32u && j + 1u == nTiles) TC_STAMP(10);
+        }
+        float o[8], Mx[8];
+#pragma unroll
+        for (int h = 0; h < 8; ++h) {
+            o[h] = 0.0f, Mx[h] = kNegBig;
+            if (h < NH) {
+#pragma unroll
+                for (int w = 0; w < NWG; ++w) Mx[h] = fmaxf(Mx[h], M[w][h]);
+#pragma unroll
+                for (int w = 0; w < NWG; ++w) o[h] = fmaf(oW[w][h], fastExp2(M[w][h] - Mx[h]), o[h]);
+            }
         }
         // every P tile has been consumed (its O was waited for above): their space is the scratch
         float *scr = reinterpret_cast<float *>(smem + L::kP);
@@ -459,7 +536,7 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         for (int h = 0; h < 8; ++h) scr[h * 128u + row] = o[h];
         if (threadIdx.x == kFoldWarp0 * 32u) {
 #pragma unroll
-            for (int h = 0; h < 8; ++h) scr[8 * 128 + h] = M[h];
+            for (int h = 0; h < 8; ++h) scr[8 * 128 + h] = Mx[h];
         }
         namedBarSync(kEndBar, kEndThreads);
     } else {
@@ -521,17 +598,18 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
             if (lane == 0)
                 sHs[h] = valid ? p.invSqrt * kLog2e * __uint_as_float(static_cast<uint32_t>(127 + e - 20) << 23) : 0.0f;
             fenceProxyAsync();
-            mbarArrive(qFull);
+            __syncwarp();
+            if (lane == 0) mbarArrive(qFull);
         }
         if (threadIdx.x == 0) TC_STAMP(3);
         namedBarSync(kAllBar, kSoftThreads);  // head scales visible to every warpgroup
-        float hs[8];
+        float hs[NH];
 #pragma unroll
-        for (int h = 0; h < 8; ++h) hs[h] = sHs[h];
+        for (int h = 0; h < NH; ++h) hs[h] = sHs[h];
 
-        float mref[8], l[8];
+        float mref[NH], l[NH];
 #pragma unroll
-        for (int h = 0; h < 8; ++h) mref[h] = kNegBig, l[h] = 0.0f;
+        for (int h = 0; h < NH; ++h) mref[h] = kNegBig, l[h] = 0.0f;
         float Eref = 0.0f, invW = 0.0f;  // power of two above every V scale seen; 2^24 / Eref
         bool ok = true;
 
@@ -553,41 +631,49 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
             const float skr = sK[row];
             const float svr = valid ? sK[T + row] : 0.0f;
             tmemLdWait();
-            float sc[8];
-            bool need = svr >= Eref;
+            // x = score - reference point (log2 units)
+            float f[NH], x[NH];
 #pragma unroll
-            for (int h = 0; h < 8; ++h) {
-                const float f = fmaf(fmaf(i2f(ra[h]), 128.0f, i2f(ra[8 + h])), 128.0f, i2f(rb[h]));
-                sc[h] = valid ? f * (skr * hs[h]) : -INFINITY;
-                need = need || sc[h] > mref[h] + kTcLazyLog2;
+            for (int h = 0; h < NH; ++h) {
+                // digit planes 1 and 2 combine exactly in 32 bits (below 2^20 each)
+                const int lo = static_cast<int>(ra[8 + h]) * 128 + static_cast<int>(rb[h]);
+                f[h] = fmaf(i2f(ra[h]), 16384.0f, __int2float_rn(lo));
+                x[h] = fmaf(f[h], skr * hs[h], -mref[h]);
             }
-            if (barOr(wgBar, 128, need)) {
+            if (t0 + (j + 1u) * T > t1) {  // the last tile: rows behind the range (whatever their scales hold)
+#pragma unroll
+                for (int h = 0; h < NH; ++h) x[h] = valid ? x[h] : -INFINITY;
+            }
+            float top = x[0];
+#pragma unroll
+            for (int h = 1; h < NH; ++h) top = fmaxf(top, x[h]);
+            // (the first tile of a warpgroup always moves it)
+            const bool moved = j == w || barOr(wgBar, 128, svr >= Eref || top > kTcLazyLog2);
+            if (moved) {
                 // rare: the reference point of a head (or the bound of the V scales) has to move --
                 // tile maxima over the warpgroup, then every thread applies the same update
-                float tm[9];
+                float tm[NH + 1];
 #pragma unroll
-                for (int h = 0; h < 8; ++h) tm[h] = sc[h];
-                tm[8] = svr;
+                for (int h = 0; h < NH; ++h) x[h] = tm[h] = valid ? f[h] * (skr * hs[h]) : -INFINITY;
+                tm[NH] = svr;
 #pragma unroll
-                for (int i = 0; i < 9; ++i)
-#pragma unroll
-                    for (int off = 16; off; off >>= 1) tm[i] = fmaxf(tm[i], __shfl_xor_sync(0xffffffffu, tm[i], off));
+                for (int i = 0; i <= NH; ++i) tm[i] = warpMax(tm[i]);
                 if (lane == 0) {
 #pragma unroll
-                    for (int i = 0; i < 9; ++i) red[wq * 12u + i] = tm[i];
+                    for (int i = 0; i <= NH; ++i) red[wq * 12u + i] = tm[i];
                 }
-                namedBarSync(wgBar, 128);
+                namedBarSync(wgBar, 128);  // (the next vote lies between these reads and the next rare pass's writes)
 #pragma unroll
-                for (int i = 0; i < 9; ++i) tm[i] = fmaxf(fmaxf(red[i], red[12 + i]), fmaxf(red[24 + i], red[36 + i]));
-                namedBarSync(wgBar, 128);  // red may be rewritten by the next rare pass
+                for (int i = 0; i <= NH; ++i) tm[i] = fmaxf(fmaxf(red[i], red[12 + i]), fmaxf(red[24 + i], red[36 + i]));
 #pragma unroll
-                for (int h = 0; h < 8; ++h) {
+                for (int h = 0; h < NH; ++h) {
                     const float mn = fmaxf(mref[h], tm[h]);
                     l[h] *= fastExp2(mref[h] - mn);
                     mref[h] = mn;
+                    x[h] -= mn;
                 }
-                if (tm[8] >= Eref) {
-                    uint32_t eb = (__float_as_uint(tm[8]) & 0x7f800000u) + 0x00800000u;  // 2^(floor(log2) + 1)
+                if (tm[NH] >= Eref) {
+                    uint32_t eb = (__float_as_uint(tm[NH]) & 0x7f800000u) + 0x00800000u;  // 2^(floor(log2) + 1)
                     eb = min(max(eb, 24u << 23), 253u << 23);
                     Eref = __uint_as_float(eb);
                     invW = __uint_as_float((127u + 24u + 127u) * (1u << 23) - eb);  // 2^24 / Eref
@@ -598,39 +684,37 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
             uint32_t X[8];
 #pragma unroll
             for (int h = 0; h < 8; ++h) {
-                const float pr = fastExp2(sc[h] - mref[h]);
-                l[h] += pr;
-                X[h] = __float2uint_rn(pr * wv);
-            }
-            // The P tile and the meta slot of this buffer were last used by tile j - 2 NWG: that tile's
-            // P.V product is complete and folded once the fold warpgroup has said so on oFree (long
-            // ago, as a rule: two tiles of this warpgroup lie in between).
-            if (j >= 2u * kWG &&
-                !mbarWait(&oFree[2u * w + bb], ((j - 2u * kWG) / (2u * kWG)) & 1u, p.err, kDevErrMmaWait)) {
-                ok = false;
-                break;
+                X[h] = 0u;
+                if (h < NH) {
+                    const float pr = fastExp2(x[h < NH ? h : 0]);
+                    l[h < NH ? h : 0] += pr;
+                    X[h] = __float2uint_rn(pr * wv);
+                }
             }
             uint8_t *pt = smem + L::kP + (2u * w + bb) * 4096u + row * 32u;
             const uint32_t sw = (row >> 2) & 1u;  // 32-byte swizzle: 16-byte halves swap on rows 4..7 of every 8
             *reinterpret_cast<uint4 *>(pt + ((0u ^ sw) << 4)) = make_uint4(X[0], X[1], X[2], X[3]);
             *reinterpret_cast<uint4 *>(pt + ((1u ^ sw) << 4)) = make_uint4(X[4], X[5], X[6], X[7]);
             if (row == 0) {
-                // what the fold warpgroup needs with this tile: the reference points its probabilities
-                // were taken against and the scale of their fixed-point form
-                float *mt = meta + (2u * w + bb) * 12u;
+                // what the fold warpgroup needs with this tile: the scale of its fixed-point probabilities and, when they
+                // moved, the reference points these were taken against
+                float *mt = meta + (4u * w + ((j / kWG) & 3u)) * 12u;
+                if (moved) {
 #pragma unroll
-                for (int h = 0; h < 8; ++h) mt[h] = mref[h];
-                mt[8] = Eref * 5.9604644775390625e-8f;  // Eref * 2^-24
+                    for (int h = 0; h < NH; ++h) mt[h] = mref[h];
+                }
+                *reinterpret_cast<float2 *>(mt + 8) = make_float2(Eref * 5.9604644775390625e-8f, moved ? 1.0f : 0.0f);  // Eref * 2^-24
             }
             fenceProxyAsync();
             tcFenceBefore();
-            mbarArrive(&pFull[2u * w + bb]);
+            __syncwarp();
+            if (lane == 0) mbarArrive(&pFull[2u * w + bb]);
             if (threadIdx.x == 0 && j / kWG < 4u) TC_STAMP(5 + j / kWG);
         }
 
         // ---- row sums of this warpgroup, then the end of the block ----
 #pragma unroll
-        for (int h = 0; h < 8; ++h)
+        for (int h = 0; h < NH; ++h)
 #pragma unroll
             for (int off = 16; off; off >>= 1) l[h] += __shfl_xor_sync(0xffffffffu, l[h], off);
         float *scr = reinterpret_cast<float *>(smem + L::kP);
@@ -641,7 +725,7 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         namedBarSync(kEndBar, kEndThreads);       // the fold warpgroup is through: every P tile has been consumed
         if (lane == 0) {
 #pragma unroll
-            for (int h = 0; h < 8; ++h) {
+            for (int h = 0; h < NH; ++h) {
                 lS[warp * 8u + h] = l[h];
                 if (wq == 0) mS[w * 8u + h] = mref[h];
             }
@@ -741,7 +825,12 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         }
     }
     if (threadIdx.x == 0) TC_STAMP(12);
-    tcFenceBefore();
+    // (every product was waited for by the fold warps, every read of tensor memory lies in front of the barrier that they
+    // and the softmax warps met at)
+    if (warp == 0) {
+        tcFenceAfter();
+        tmemDealloc(tmemBase, L::kTmemCols);
+    }
     if constexpr (CLUSTER) {
         // every block's results are in the inboxes of the blocks that put them together
         if (warp >= kFoldWarp0) clusterHelloWait();
@@ -756,11 +845,6 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
             *reinterpret_cast<float4 *>(p.out + oidx * 128u + 4u * (idx & 31u)) =
                     make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
         }
-    }
-    __syncthreads();
-    if (warp == 0) {
-        tcFenceAfter();
-        tmemDealloc(tmemBase, L::kTmemCols);
     }
 }
 
@@ -779,7 +863,7 @@ int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, c
     // (20 tiles, 2 and 3 sequences) 0.83 and 0.87, up to 12000 (24 tiles, 4 and 8) 0.93 and 0.98, up to 32768 (32, 2 and 3) 1.15.
     static ClusterSetup setup;
     const uint32_t *limits = nullptr;
-    int rc = setupCluster(setup, decodeI8TcKernel<2, 6, true, TcFold::kCluster>, Smem::kThreads, Smem::kTotal, &limits);
+    int rc = setupCluster(setup, decodeI8TcKernel<2, 6, 8, true, TcFold::kCluster>, Smem::kThreads, Smem::kTotal, &limits);
     if (rc != TC_OK) return rc;
     DecodePlan pl = planDecode(d->batch, d->nKV, d->maxLen, d->numChunks, kTcTile, d->lens == nullptr, 1u);
     uint32_t cluster = 1;
@@ -891,24 +975,34 @@ int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, c
     // (Four softmax warpgroups with a five-stage ring were measured and dropped: 11.5 against 8.3 us
     // per layer for the split launch alone at 32768 rows, 53.9 against 47.0 us at batch 8.)
     // (each way of coming together is an instantiation of its own for the same reason as the append)
-    using Kern = decltype(&decodeI8TcKernel<2, 6, true, TcFold::kLaunch>);
-    static const Kern kerns[2][3] = {
-            {decodeI8TcKernel<2, 6, false, TcFold::kLaunch>, decodeI8TcKernel<2, 6, false, TcFold::kTickets>,
-             decodeI8TcKernel<2, 6, false, TcFold::kCluster>},
-            {decodeI8TcKernel<2, 6, true, TcFold::kLaunch>, decodeI8TcKernel<2, 6, true, TcFold::kTickets>,
-             decodeI8TcKernel<2, 6, true, TcFold::kCluster>}};
+    using Kern = decltype(&decodeI8TcKernel<2, 6, 8, true, TcFold::kLaunch>);
+#define TC_KERNS(NH, APPEND) {decodeI8TcKernel<2, 6, NH, APPEND, TcFold::kLaunch>, decodeI8TcKernel<2, 6, NH, APPEND, TcFold::kCluster>}
+    static const Kern kerns[4][2][2] = {{TC_KERNS(4, false), TC_KERNS(4, true)},
+                                        {TC_KERNS(6, false), TC_KERNS(6, true)},
+                                        {TC_KERNS(7, false), TC_KERNS(7, true)},
+                                        {TC_KERNS(8, false), TC_KERNS(8, true)}};
+#undef TC_KERNS
+    static const Kern ticketKerns[2] = {decodeI8TcKernel<2, 6, 8, false, TcFold::kTickets>,
+                                        decodeI8TcKernel<2, 6, 8, true, TcFold::kTickets>};
     static bool attrDone[64] = {false};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !attrDone[dev]) {
-        for (auto &row : kerns)
-            for (Kern k : row) {
-                TC_CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem::kTotal));
-                TC_CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-            }
+        auto attributes = [](Kern k) {
+            TC_CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem::kTotal));
+            TC_CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            return static_cast<int>(TC_OK);
+        };
+        for (auto &byHeads : kerns)
+            for (auto &byAppend : byHeads)
+                for (Kern k : byAppend)
+                    if ((rc = attributes(k)) != TC_OK) return rc;
+        for (Kern k : ticketKerns)
+            if ((rc = attributes(k)) != TC_OK) return rc;
         attrDone[dev] = true;
     }
-    const Kern kern = kerns[d->appendK != nullptr ? 1 : 0][cluster > 1 ? 2 : (fused ? 1 : 0)];
+    const uint32_t append = d->appendK != nullptr ? 1 : 0, heads = group <= 4 ? 0 : group <= 6 ? 1 : group == 7 ? 2 : 3;
+    const Kern kern = fused ? ticketKerns[append] : kerns[heads][append][cluster > 1 ? 1 : 0];
     // (without TC_DECODE_PDL prefetchRows is 0 and every block waits for the kernels ahead first thing)
     // a launch serves 8 q heads per kv head (the MMA columns); wider groups take one launch per
     // block of 8 and stream the rows again

@@ -48,64 +48,12 @@ int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, c
 // 20 us by the hardware.  (A loop that reads the clock: captured int8 step of 28 / 4 / 128 at 12000 rows 23.6 us per layer
 // against 23.0, 8 sequences of 4098 rows 9.95 against 9.83.)
 __device__ __forceinline__ bool mbarWait(uint64_t *bar, uint32_t parity, unsigned int *err, uint32_t errBit) {
-    if (mbarTryWait(bar, parity)) return true;
+    if (mbarTestWait(bar, parity)) return true;
 #pragma unroll 1
     for (uint32_t i = 0; i < (1u << 18); ++i)
         if (mbarTryWait(bar, parity)) return true;
     atomicOr(err, errBit);
     return false;
-}
-
-// The new token's K and V row of one kv head into an int8 pool, by one warp (the arithmetic of kvQuantKernel: amax / 127,
-// IEEE divide, round-half-even; lane i owns float4 i, i + 32 of the row).  Blocks that share the kv head write the same
-// bytes.  Both rows are loaded at once; the block's own TMA load and scale copies read the row back, so the stores are
-// ordered before the async proxy and nothing wider.  srcK / srcV: the rows; dst: row x nKV + kv head of the pool.
-// mirK / mirV (nullable): the same row of an f32 store beside the pool, written verbatim.
-template <int HD>
-__device__ __forceinline__ void appendQuantRow(const float4 *srcK, const float4 *srcV, uint32_t *k8w, uint32_t *v8w,
-                                               float *ksw, float *vsw, uint64_t dst, float4 *mirK, float4 *mirV,
-                                               uint32_t lane) {
-    constexpr int N = HD / 128;
-    float4 kx[N], vx[N];
-    float mk = 0.0f, mv = 0.0f;
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-        kx[i] = __ldg(srcK + lane + 32 * i);
-        vx[i] = __ldg(srcV + lane + 32 * i);
-    }
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-        mk = fmaxf(mk, fmaxf(fmaxf(fabsf(kx[i].x), fabsf(kx[i].y)), fmaxf(fabsf(kx[i].z), fabsf(kx[i].w))));
-        mv = fmaxf(mv, fmaxf(fmaxf(fabsf(vx[i].x), fabsf(vx[i].y)), fmaxf(fabsf(vx[i].z), fabsf(vx[i].w))));
-        if (mirK != nullptr) {
-            mirK[lane + 32 * i] = kx[i];
-            mirV[lane + 32 * i] = vx[i];
-        }
-    }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-        mk = fmaxf(mk, __shfl_xor_sync(0xffffffffu, mk, o));
-        mv = fmaxf(mv, __shfl_xor_sync(0xffffffffu, mv, o));
-    }
-    const float sk = mk > 0.0f ? __fdiv_rn(mk, 127.0f) : 1.0f;
-    const float sv = mv > 0.0f ? __fdiv_rn(mv, 127.0f) : 1.0f;
-    if (lane == 0) {
-        ksw[dst] = sk;
-        vsw[dst] = sv;
-    }
-    auto q8 = [](float x, float sc) -> uint32_t {
-        int qv = __float2int_rn(__fdiv_rn(x, sc));
-        qv = qv < -128 ? -128 : (qv > 127 ? 127 : qv);
-        return static_cast<uint32_t>(qv) & 0xffu;
-    };
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-        const uint64_t at = dst * (HD / 4) + lane + 32 * i;
-        k8w[at] = q8(kx[i].x, sk) | (q8(kx[i].y, sk) << 8) | (q8(kx[i].z, sk) << 16) | (q8(kx[i].w, sk) << 24);
-        v8w[at] = q8(vx[i].x, sv) | (q8(vx[i].y, sv) << 8) | (q8(vx[i].z, sv) << 16) | (q8(vx[i].w, sv) << 24);
-    }
-    asm volatile("fence.proxy.async.global;" ::: "memory");
-    __syncwarp();
 }
 
 #endif

@@ -122,6 +122,18 @@ __device__ __forceinline__ bool mbarTryWait(uint64_t *bar, uint32_t parity) {
             : "memory");
     return ok != 0;
 }
+// Whether a phase is complete, without parking the thread.
+__device__ __forceinline__ bool mbarTestWait(uint64_t *bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.b32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(smemAddr(bar)), "r"(parity)
+            : "memory");
+    return ok != 0;
+}
 __device__ __forceinline__ void fenceBarrierInit() {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
