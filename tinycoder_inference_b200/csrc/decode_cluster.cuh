@@ -313,12 +313,20 @@ __device__ __forceinline__ void inboxTake(const FoldInbox<V4> &in, uint32_t i, u
     }
 }
 
-// Every warp has left [8 columns][HD] accumulators, m[8] (log2 units) and l[8] in its part of
-// scr ([NW][8 HD + 16]).  Called by all THREADS threads of the block (tid) with the warps' parts complete; in a cluster
-// every thread has said clusterHello() before.
+// A warp's results in shared memory: [8 columns][kRow] accumulators, m[8] (log2 units), l[8].  The row stride keeps the four
+// columns that a warp stores at a time in different banks (rows of HD floats put them into the same ones: a four-way
+// conflict: 0.15 - 0.6 us of a decode call, the most at head_dim 256).
+template <int HD>
+struct FoldScratch {
+    static constexpr int kRow = HD + 4, kM = 8 * kRow, kL = kM + 8, kWarp = kL + 8;
+};
+
+// Every warp has left its results in its part of scr ([NW][FoldScratch::kWarp]).  Called by all THREADS threads of the block
+// (tid) with the warps' parts complete; in a cluster every thread has said clusterHello() before.
 template <int HD, int NW, int THREADS = NW * 32>
 __device__ __forceinline__ void clusterFold(const float *scr, const FoldTarget &f, uint32_t tid) {
-    constexpr uint32_t kWarpScr = 8 * HD + 16, V4 = HD / 4;
+    using F = FoldScratch<HD>;
+    constexpr uint32_t kWarpScr = F::kWarp, V4 = HD / 4;
     __shared__ FoldInbox<V4> inbox;
     const uint32_t n = clusterSize(), rank = clusterRank();
     const uint32_t total = f.nValid * V4, per = (total + n - 1) / n;
@@ -327,15 +335,15 @@ __device__ __forceinline__ void clusterFold(const float *scr, const FoldTarget &
         const uint32_t d4 = idx % V4, j = idx / V4;
         float M = kNegBig;
 #pragma unroll
-        for (int w = 0; w < NW; ++w) M = fmaxf(M, scr[w * kWarpScr + 8 * HD + j]);
+        for (int w = 0; w < NW; ++w) M = fmaxf(M, scr[w * kWarpScr + F::kM + j]);
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
         float l = 0.0f;
 #pragma unroll
         for (int w = 0; w < NW; ++w) {
             const float *s = scr + w * kWarpScr;
-            const float wgt = fastExp2(s[8 * HD + j] - M);
-            l = fmaf(wgt, s[8 * HD + 8 + j], l);
-            const float4 a = *reinterpret_cast<const float4 *>(s + j * HD + 4 * d4);
+            const float wgt = fastExp2(s[F::kM + j] - M);
+            l = fmaf(wgt, s[F::kL + j], l);
+            const float4 a = *reinterpret_cast<const float4 *>(s + j * F::kRow + 4 * d4);
             acc.x = fmaf(wgt, a.x, acc.x);
             acc.y = fmaf(wgt, a.y, acc.y);
             acc.z = fmaf(wgt, a.z, acc.z);

@@ -33,29 +33,34 @@ constexpr int kHD = 128;
 //
 // Every warp has NS slots for tiles of 16 MT tokens of K and as many of V, each as HD/128 half-tiles of [rows][128 bytes],
 // half-tile h covering dims [128h, 128h + 128); the rows' scales lie behind all slots.
-template <int HD, int NW, int NS, int MT>
+template <int HD, int NW, int NS, int MT, bool ROWS>
 struct DecodeI8Smem {
     static constexpr int T = 16 * MT;
     static constexpr int kHalfBytes = T * 128;            // one half-tile
     static constexpr int kTileBytes = T * HD;             // K (or V) bytes of a tile
     static constexpr int kScales = NW * NS * 2 * kTileBytes;   // [warp][slot][K, V][T] floats
-    static constexpr int kSlots = kScales + NW * NS * 2 * T * 4, kScratch = NW * (8 * HD + 16) * 4;  // (the fold reuses the slots)
-    static constexpr int kTotal = (kSlots > kScratch ? kSlots : kScratch) + 128;
+    static constexpr int kSlots = kScales + NW * NS * 2 * T * 4, kScratch = NW * FoldScratch<HD>::kWarp * 4;  // (the fold reuses the slots)
+    static constexpr int kQuery = kSlots > kScratch ? kSlots : kScratch;   // decode: the block's query fragments
+    static constexpr int kTotal = kQuery + (ROWS ? 0 : I8QueryShare<HD, NW>::kBytes) + 128;
     static_assert(kTotal <= 227 * 1024, "shared memory of an SM");
 };
 
-// ROWS: causal query rows; otherwise a token's q heads over chunks of the store.
-template <int HD, int NW, int NS, int MT, bool ROWS>
-__global__ void __launch_bounds__(NW * 32, !ROWS && NW <= 4 ? 2 : 1)
+// ROWS: causal query rows; otherwise a token's q heads over chunks of the store: SW warps share a chunk, a block holds NW / SW
+// neighbouring chunks.
+template <int HD, int NW, int SW, int NS, int MT, bool ROWS>
+__global__ void __launch_bounds__(NW * 32, 1)
 decodeI8Kernel(const __grid_constant__ DecodeI8Params p) {
-    using L = DecodeI8Smem<HD, NW, NS, MT>;
+    using L = DecodeI8Smem<HD, NW, NS, MT, ROWS>;
+    static_assert(!ROWS || SW == NW, "rows share all tiles");
     constexpr int T = L::T;
     constexpr int NC = HD / 16;  // 16-dim groups of a head vector
     constexpr int NR = 2 * MT;  // 8-token row groups of a warp's tile
     constexpr float k2p24 = kI8Unscale;
 
-    const uint32_t chunk = blockIdx.x, hg = blockIdx.y, b = ROWS ? gridDim.z - 1u - blockIdx.z : blockIdx.z;  // (late rows first)
+    constexpr uint32_t G = NW / SW;  // chunks of a block
+    const uint32_t hg = blockIdx.y, b = ROWS ? gridDim.z - 1u - blockIdx.z : blockIdx.z;  // (late rows first)
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const uint32_t chunk = blockIdx.x * G + warp / SW, sw = warp % SW;
 
     extern __shared__ uint8_t smemRaw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smemRaw) + 127) & ~uintptr_t(127));
@@ -65,7 +70,7 @@ decodeI8Kernel(const __grid_constant__ DecodeI8Params p) {
         const uint32_t t0 = chunk * p.chunkTokens, t1 = min(p.lenHost, t0 + p.chunkTokens);
         const uint8_t *k = reinterpret_cast<const uint8_t *>(p.k8w) + static_cast<size_t>(hg) * HD;
         const uint8_t *v = reinterpret_cast<const uint8_t *>(p.v8w) + static_cast<size_t>(hg) * HD;
-        for (uint32_t i = 0, tok = t0 + warp * T; i < kPrefetchTiles && tok < t1; ++i, tok += NW * T) {
+        for (uint32_t i = 0, tok = t0 + sw * T; i < kPrefetchTiles && tok < t1; ++i, tok += SW * T) {
             prefetchTile<HD>(k, v, static_cast<size_t>(p.nKV) * HD, base + tok, p.totalRows - 1, lane);
             if (lane < 2u) {
                 const float *s = (lane ? p.vs : p.ks) + min(base + tok, p.totalRows - 1) * p.nKV + hg;
@@ -85,7 +90,7 @@ decodeI8Kernel(const __grid_constant__ DecodeI8Params p) {
         len = p.devLens ? min(p.devLens[b] + p.lenAdd, p.lenHost) : p.lenHost;
         // a cluster behind the last row leaves as a whole: the merge derives the active count from len.  The first one stays: it
         // writes the zeros of a sequence without rows
-        if ((chunk - clusterRank()) * p.chunkTokens >= len && chunk != clusterRank()) return;
+        if ((blockIdx.x - clusterRank()) * G * p.chunkTokens >= len && blockIdx.x != clusterRank()) return;
     }
     const uint32_t t0 = ROWS ? 0u : chunk * p.chunkTokens;
     if (!ROWS && clusterSize() > 1) clusterHello();
@@ -94,7 +99,7 @@ decodeI8Kernel(const __grid_constant__ DecodeI8Params p) {
     const uint64_t rowBase = ROWS ? 0ull : (p.devRowBase ? p.devRowBase[b] : static_cast<uint64_t>(b) * p.rowsPerSeq);
     const uint32_t kvHead = ROWS ? hg / p.group : hg;
 
-    // Tile j belongs to warp j % NW, its slot (j / NW) % NS.  A warp copies its own tiles: with one slot the next
+    // Tile j of a chunk belongs to its warp j % SW, slot (j / SW) % NS.  A warp copies its own tiles: with one slot the next
     // tile's K while it works on this one's V and the next V while it works on K.
     auto slotK = [&](uint32_t i) { return smem + (warp * NS + i % NS) * 2 * L::kTileBytes; };
     auto scaleK = [&](uint32_t i) { return reinterpret_cast<float *>(smem + L::kScales) + (warp * NS + i % NS) * 2 * T; };
@@ -106,12 +111,12 @@ decodeI8Kernel(const __grid_constant__ DecodeI8Params p) {
     const uint64_t newRow = rowBase + (!ROWS && p.devLens ? p.devLens[b] + p.lenAdd : len) - 1u;
     // a device length outside the pool (or no length at all): no row written
     const bool outside = (append && newRow >= p.totalRows) || (!ROWS && p.appendK != nullptr && len == 0u);
-    if (outside && threadIdx.x == 0) atomicOr(p.err, kDevErrRowBound);
-    const bool mine = append && !outside && (nTiles - 1u) % NW == warp;
-    const bool intoTile = mine && (nTiles - 1u) / NW < NS;
+    if (outside && lane == 0) atomicOr(p.err, kDevErrRowBound);
+    const bool mine = append && !outside && (nTiles - 1u) % SW == sw;
+    const bool intoTile = mine && (nTiles - 1u) / SW < NS;
     const uint64_t have = intoTile ? rowBase + len - 1u : min(rowBase + len, p.totalRows);
     auto request = [&](uint32_t i, bool isV) {
-        const uint32_t j = warp + i * NW;
+        const uint32_t j = sw + i * SW;
         if (j < nTiles) {
             const uint64_t row = rowBase + t0 + j * T;
             const uint32_t count = have > row ? static_cast<uint32_t>(min(have - row, static_cast<uint64_t>(T))) : 0u;
@@ -142,10 +147,12 @@ decodeI8Kernel(const __grid_constant__ DecodeI8Params p) {
     auto colLen = [&](uint32_t j) { return ROWS ? min(t1, rowsPos + b * 8u + j + 1u) : t1; };
 
     I8Query<HD> qf;
-    i8LoadQuery<HD>(qf, p.q + colIndex(colValid(g) ? g : 0) * HD, colValid(g), p.invSqrt, lane);
+    const float *qp = p.q + colIndex(colValid(g) ? g : 0) * HD;
+    if constexpr (ROWS) i8LoadQuery<HD>(qf, qp, colValid(g), p.invSqrt, lane);
+    else i8LoadQueryShared<HD, NW>(qf, smem + L::kQuery, qp, colValid(g), p.invSqrt, warp, lane);
     if (mine) {
         const size_t dst = newRow * p.nKV + kvHead;
-        const uint32_t i = (nTiles - 1u) / NW;
+        const uint32_t i = (nTiles - 1u) / SW;
         float4 *mk = nullptr, *mv = nullptr;
         if (p.mir.k != nullptr)
             mk = reinterpret_cast<float4 *>(p.mir.k) + dst * (HD / 4), mv = reinterpret_cast<float4 *>(p.mir.v) + dst * (HD / 4);
@@ -168,7 +175,7 @@ decodeI8Kernel(const __grid_constant__ DecodeI8Params p) {
     const uint32_t lco = lane >> 4;                             // and which chunk of the pair
     const uint32_t lmOff = lr * 128;
 
-    for (uint32_t i = 0, tile = warp; tile < nTiles; ++i, tile += NW) {
+    for (uint32_t i = 0, tile = sw; tile < nTiles; ++i, tile += SW) {
         cpAsyncWait<2 * NS - 1>();  // K of this tile is in, what was requested behind it may still be on its way
         const float *sK = scaleK(i), *sV = sK + T;
         const uint32_t tokBase = t0 + tile * T + g;
@@ -249,11 +256,11 @@ decodeI8Kernel(const __grid_constant__ DecodeI8Params p) {
         const uint32_t vTile = smemAddr(slotK(i) + L::kTileBytes);
 #pragma unroll
         for (int cp = 0; cp < NC / 2; ++cp) {
-            const uint32_t sw = (((2 * (cp & 3) + lco) ^ (lr & 7u)) << 4) + (cp >> 2) * L::kHalfBytes;
+            const uint32_t at = (((2 * (cp & 3) + lco) ^ (lr & 7u)) << 4) + (cp >> 2) * L::kHalfBytes;
 #pragma unroll
             for (int mt = 0; mt < MT; ++mt) {
                 uint32_t r0, r1, r2, r3;
-                ldmatrixX4Trans(r0, r1, r2, r3, vTile + mt * 2048 + lmOff + sw);
+                ldmatrixX4Trans(r0, r1, r2, r3, vTile + mt * 2048 + lmOff + at);
                 r0 ^= 0x80808080u;
                 r1 ^= 0x80808080u;
                 r2 ^= 0x80808080u;
@@ -287,8 +294,9 @@ decodeI8Kernel(const __grid_constant__ DecodeI8Params p) {
     }
     namedBarSync(1, NW * 32);  // every consumer is done reading the ring
     float *scr = reinterpret_cast<float *>(smem);
-    constexpr int kWarpScr = 8 * HD + 16;
-    float *wO = scr + warp * kWarpScr;  // [8 heads][HD], then m[8], l[8]
+    using F = FoldScratch<HD>;
+    constexpr int kWarpScr = F::kWarp;
+    float *wO = scr + warp * kWarpScr;  // [8 heads][FoldScratch::kRow], then m[8], l[8]
     {
         // true accumulator = 2^24 * raw - 128 * sum(p*sv), then back from the E-scaled domain
         const float E = __uint_as_float(Ebits);
@@ -296,23 +304,23 @@ decodeI8Kernel(const __grid_constant__ DecodeI8Params p) {
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
             const int d = 16 * c + 2 * g;
-            *reinterpret_cast<float2 *>(wO + (2 * t) * HD + d) =
+            *reinterpret_cast<float2 *>(wO + (2 * t) * F::kRow + d) =
                     make_float2(fmaf(o[c][0], k2p24, -c0) * E, fmaf(o[c][2], k2p24, -c0) * E);
-            *reinterpret_cast<float2 *>(wO + (2 * t + 1) * HD + d) =
+            *reinterpret_cast<float2 *>(wO + (2 * t + 1) * F::kRow + d) =
                     make_float2(fmaf(o[c][1], k2p24, -c1) * E, fmaf(o[c][3], k2p24, -c1) * E);
         }
     }
     if (g == 0) {
-        wO[8 * HD + 2 * t] = m0;
-        wO[8 * HD + 2 * t + 1] = m1;
-        wO[8 * HD + 8 + 2 * t] = l0;
-        wO[8 * HD + 8 + 2 * t + 1] = l1;
+        wO[F::kM + 2 * t] = m0;
+        wO[F::kM + 2 * t + 1] = m1;
+        wO[F::kL + 2 * t] = l0;
+        wO[F::kL + 2 * t + 1] = l1;
     }
     namedBarSync(1, NW * 32);
     if (!ROWS) {
         FoldTarget f;
         f.out = p.out, f.pAcc = p.pAcc, f.pM = p.pM, f.pL = p.pL;
-        f.numChunks = p.numChunks, f.slot = chunk / clusterSize();
+        f.numChunks = p.numChunks, f.slot = blockIdx.x / clusterSize();
         f.firstHead = static_cast<uint32_t>(colIndex(0)), f.nValid = min(8u, p.group - p.colBase);
         f.direct = p.directOut;
         f.qRot = nullptr, f.cosT = nullptr, f.sinT = nullptr, f.tableRow = 0;
@@ -325,15 +333,15 @@ decodeI8Kernel(const __grid_constant__ DecodeI8Params p) {
         if (!colValid(j)) continue;
         float M = kNegBig;
 #pragma unroll
-        for (int w = 0; w < NW; ++w) M = fmaxf(M, scr[w * kWarpScr + 8 * HD + j]);
+        for (int w = 0; w < NW; ++w) M = fmaxf(M, scr[w * kWarpScr + F::kM + j]);
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
         float lsum = 0.0f;
 #pragma unroll
         for (int w = 0; w < NW; ++w) {
             const float *s = scr + w * kWarpScr;
-            const float wgt = fastExp2(s[8 * HD + j] - M);
-            lsum += wgt * s[8 * HD + 8 + j];
-            const float4 a = *reinterpret_cast<const float4 *>(s + j * HD + 4 * d4);
+            const float wgt = fastExp2(s[F::kM + j] - M);
+            lsum += wgt * s[F::kL + j];
+            const float4 a = *reinterpret_cast<const float4 *>(s + j * F::kRow + 4 * d4);
             acc.x = fmaf(wgt, a.x, acc.x);
             acc.y = fmaf(wgt, a.y, acc.y);
             acc.z = fmaf(wgt, a.z, acc.z);
@@ -347,31 +355,34 @@ decodeI8Kernel(const __grid_constant__ DecodeI8Params p) {
 
 // The split at head_dim 256.  Which tokens one warp accumulates in a row decides the roundings of the result: the V
 // bytes enter the products with an offset of 128 that is taken out at the end, so the running sums are large next to the
-// result.  Short runs keep that small, and the runs stay what they are whatever the clusters look like: chunks of
-// planDecode (one wave of blocks that stream up to four kv heads), a chunk's tokens dealt to 8 / hpc warps.  A chunk is a
-// block here; the cluster only decides how the blocks' results come together.
-static ClusterPlan decodeI8Plan(const tc_decode_i8_batch *d, const uint32_t *maxClusters) {
+// result.  Short runs keep that small, and the runs stay what they are whatever the blocks look like: chunks of
+// planDecode (one wave of blocks that stream up to four kv heads), a chunk's tokens dealt to 8 / hpc warps.  A block of eight
+// warps takes as many neighbouring chunks as fill it: it prepares the query once, and leaves one partial.
+// (16 / 2 heads, norm, decode and gate of a layer: a block per chunk with one slot per warp -> this: 2000 rows 12.05 -> 10.05 us, now
+// one cluster, 16383 rows 17.1 -> 16.05; 16 / 4: 2000 rows 12.6 -> 9.9, 60000 rows 35.2 -> 31.6; 20 rows of 16 / 2 9.48 -> 9.6.)
+static ClusterPlan decodeI8Plan(const tc_decode_i8_batch *d, uint32_t chunksPerBlock, const uint32_t *maxClusters) {
     const DecodePlan dp = planDecode(d->batch, d->nKV, d->maxLen, d->numChunks, 8u * 16u, d->lens == nullptr);
-    ClusterPlan best = {1, dp.chunksPerSeq, dp.chunkTokens};
-    // up to 16 chunks one cluster per kv head folds them all; more take the merge
+    const uint32_t blocks = (dp.chunksPerSeq + chunksPerBlock - 1u) / chunksPerBlock;
+    ClusterPlan best = {1, blocks, dp.chunkTokens};
+    // up to 16 blocks one cluster per kv head folds them all; more take the merge
     for (uint32_t lg = 1; lg < 5; ++lg)
-        if (dp.chunksPerSeq > 1 && dp.chunksPerSeq <= (1u << lg) && maxClusters[lg] >= d->nKV * d->batch) {
+        if (blocks > 1 && blocks <= (1u << lg) && maxClusters[lg] >= d->nKV * d->batch) {
             best.cluster = 1u << lg, best.clusters = 1;
             break;
         }
     return best;
 }
 
-template <int NW>
+template <int SW>
 static int decodeI8Hd256(const tc_decode_i8_batch *d, DecodeI8Params prm, cudaStream_t st) {
-    constexpr int HD = 256;
-    using L = DecodeI8Smem<HD, NW, 1, 1>;
-    auto kern = decodeI8Kernel<HD, NW, 1, 1, false>;
+    constexpr int HD = 256, NW = 8, NS = 2;
+    using L = DecodeI8Smem<HD, NW, NS, 1, false>;
+    auto kern = decodeI8Kernel<HD, NW, SW, NS, 1, false>;
     static ClusterSetup setup;
     const uint32_t *limits = nullptr;
     int rc = setupCluster(setup, kern, NW * 32, L::kTotal, &limits);
     if (rc != TC_OK) return rc;
-    const ClusterPlan pl = decodeI8Plan(d, limits);
+    const ClusterPlan pl = decodeI8Plan(d, NW / SW, limits);
     const bool direct = pl.clusters == 1 && !d->partialsOnly;
     if (!direct)
         TC_REQUIRE(d->pAcc && d->pM && d->pL, TC_EWORKSPACE, "decode_i8: partial buffers are required");
@@ -391,7 +402,7 @@ static int decodeI8Hd256(const tc_decode_i8_batch *d, DecodeI8Params prm, cudaSt
     // merge: the active partial count of a sequence follows from its length (read on
     // the device when the length lives there); slots past it were never written.
     return launchMerge(d->pAcc, d->pM, d->pL, d->out, d->batch, d->nHeads, d->numChunks, pl.clusters, HD, d->lens, prm.lenAdd,
-                       pl.chunkTokens * pl.cluster, nullptr, true, st);
+                       pl.chunkTokens * (NW / SW) * pl.cluster, nullptr, true, st);
 }
 
 static int i8Params(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, const F32Mirror &mir, DecodeI8Params *o) {
@@ -478,8 +489,8 @@ int decodeI8Common(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAd
 template <int HD, int MT>
 static int launchRowsI8(const DecodeI8Params &prm, cudaStream_t st) {
     constexpr int NW = 8, NS = 3;
-    using L = DecodeI8Smem<HD, NW, NS, MT>;
-    auto kern = decodeI8Kernel<HD, NW, NS, MT, true>;
+    using L = DecodeI8Smem<HD, NW, NS, MT, true>;
+    auto kern = decodeI8Kernel<HD, NW, NW, NS, MT, true>;
     static bool attrDone[64] = {false};
     int dev = 0;
     cudaGetDevice(&dev);

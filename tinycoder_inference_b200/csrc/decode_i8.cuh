@@ -104,6 +104,76 @@ __device__ __forceinline__ void i8LoadQuery(I8Query<HD> &f, const float *qp, boo
     f.off1 = __shfl_sync(0xffffffffu, headOff, (2 * t + 1) * 4);
 }
 
+// The same by all NW warps of a block together, through `share` in its shared memory: a warp takes HD / (16 NW) of the 16-dim
+// groups, then everybody reads all fragments.  (One warp alone spends 700 instructions on the 64 dims of a lane at head_dim
+// 256, and eight warps of an SM doing that for themselves 1.2 us of a decode call.)  Bit for bit what i8LoadQuery gives: the
+// sums keep its order.  Called by all threads of the block.
+template <int HD, int NW>
+struct I8QueryShare {
+    static constexpr int NC = HD / 16;
+    static constexpr int kFrag = 0;                     // [NC][32 lanes] uint4: hi, lo
+    static constexpr int kSum = kFrag + NC * 512;       // [NC][32] sums of the rounded parts
+    static constexpr int kMax = kSum + NC * 128;        // [NW][32] maxima
+    static constexpr int kBytes = kMax + NW * 128;
+    static_assert(NC % NW == 0, "whole groups per warp");
+};
+template <int HD, int NW>
+__device__ __forceinline__ void i8LoadQueryShared(I8Query<HD> &f, uint8_t *share, const float *qp, bool valid, float invSqrt,
+                                                  uint32_t warp, uint32_t lane) {
+    using S = I8QueryShare<HD, NW>;
+    constexpr int NC = S::NC, N = NC / NW;
+    const uint32_t t = lane & 3u;
+    uint4 *frag = reinterpret_cast<uint4 *>(share + S::kFrag) + lane;
+    float *sum = reinterpret_cast<float *>(share + S::kSum) + lane, *top = reinterpret_cast<float *>(share + S::kMax) + lane;
+    float4 qv[N];
+    float amax = 0.0f;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const int c = warp * N + i;
+        qv[i] = valid ? __ldg(reinterpret_cast<const float4 *>(qp + 16 * c + 4 * t)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        amax = fmaxf(amax, fmaxf(fmaxf(fabsf(qv[i].x), fabsf(qv[i].y)), fmaxf(fabsf(qv[i].z), fabsf(qv[i].w))));
+    }
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+    top[warp * 32] = amax;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < NW; ++w) amax = fmaxf(amax, top[w * 32]);
+    int e = static_cast<int>((__float_as_uint(amax) >> 23) & 0xffu) - 127;  // floor(log2 amax)
+    e = amax > 0.0f ? max(-100, min(100, e)) : 0;
+    const float down = __uint_as_float(static_cast<uint32_t>(127 - e) << 23);  // 2^-e
+    const float up = __uint_as_float(static_cast<uint32_t>(127 + e) << 23);    // 2^e
+    const float headScale = invSqrt * up * kLog2e;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const int c = warp * N + i;
+        float h0, l0, h1, l1, h2, l2, h3, l3;
+        splitHalf(qv[i].x * down, h0, l0);
+        splitHalf(qv[i].y * down, h1, l1);
+        splitHalf(qv[i].z * down, h2, l2);
+        splitHalf(qv[i].w * down, h3, l3);
+        uint4 x = make_uint4(packHalf2(h0, h1), packHalf2(h2, h3), packHalf2(l0, l1), packHalf2(l2, l3));
+        frag[c * 32] = x;
+        const __half2 a = *reinterpret_cast<__half2 *>(&x.z), bb = *reinterpret_cast<__half2 *>(&x.w);
+        sum[c * 32] = (h0 + __low2float(a)) + (h1 + __high2float(a)) + (h2 + __low2float(bb)) + (h3 + __high2float(bb));
+    }
+    __syncthreads();
+    float qsum = 0.0f;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+        const uint4 x = frag[c * 32];
+        f.hi[c][0] = x.x, f.hi[c][1] = x.y, f.lo[c][0] = x.z, f.lo[c][1] = x.w;
+        qsum += sum[c * 32];
+    }
+    qsum += __shfl_xor_sync(0xffffffffu, qsum, 1);
+    qsum += __shfl_xor_sync(0xffffffffu, qsum, 2);
+    const float headOff = 128.0f * qsum;
+    f.cs0 = __shfl_sync(0xffffffffu, headScale, (2 * t) * 4);
+    f.cs1 = __shfl_sync(0xffffffffu, headScale, (2 * t + 1) * 4);
+    f.off0 = __shfl_sync(0xffffffffu, headOff, (2 * t) * 4);
+    f.off1 = __shfl_sync(0xffffffffu, headOff, (2 * t + 1) * 4);
+}
+
 // log2-domain scores of a tile (16 MT tokens at kTile, their K scales at sK) against the eight columns: sc[r][0 / 1] is
 // token g + 8 r against column 2t / 2t + 1; tokens tokBase + 8 r >= len0 / len1 are masked out.
 template <int HD, int MT>

@@ -36,7 +36,7 @@ struct I8StreamSmem {
     static constexpr int kEnd = kMax + 2 * kScoreWarps * 12 * 4;   // m[8], E, then l[8], sums of P x scale [8]
     static constexpr int kBars = kEnd + 32 * 4;                    // full, empty per slot
     static constexpr int kTotal = kBars + 2 * kSlots * 8 + 128;
-    static_assert((8 * HD + 16) * 4 <= kV, "the fold reuses the K tiles");
+    static_assert(FoldScratch<HD>::kWarp * 4 <= kV, "the fold reuses the K tiles");
     static_assert(kTotal <= 227 * 1024, "shared memory of an SM");
 };
 
@@ -320,21 +320,21 @@ decodeI8StreamsKernel(const __grid_constant__ DecodeI8Params p) {
         }
     }
     __syncthreads();
-    float *scr = reinterpret_cast<float *>(smem);  // [8 heads][HD], then m[8], l[8]
+    float *scr = reinterpret_cast<float *>(smem);  // [8 heads][FoldScratch::kRow], then m[8], l[8]
     if (warp >= SW && warp < SW + VW) {
         // true accumulator = 2^24 * raw - 128 * sum(p*sv), then back from the E-scaled domain
         const float E = sEnd[8], c0 = 128.0f * sEnd[24 + 2 * t], c1 = 128.0f * sEnd[25 + 2 * t];
 #pragma unroll
         for (int c = 0; c < 2 * CP; ++c) {
             const uint32_t d = (warp - SW) * (HD / 4) + 16 * c + 2 * g;
-            *reinterpret_cast<float2 *>(scr + (2 * t) * HD + d) =
+            *reinterpret_cast<float2 *>(scr + (2 * t) * FoldScratch<HD>::kRow + d) =
                     make_float2(fmaf(o[c][0], kI8Unscale, -c0) * E, fmaf(o[c][2], kI8Unscale, -c0) * E);
-            *reinterpret_cast<float2 *>(scr + (2 * t + 1) * HD + d) =
+            *reinterpret_cast<float2 *>(scr + (2 * t + 1) * FoldScratch<HD>::kRow + d) =
                     make_float2(fmaf(o[c][1], kI8Unscale, -c1) * E, fmaf(o[c][3], kI8Unscale, -c1) * E);
         }
     } else if (warp == 0 && lane < 8u) {
-        scr[8 * HD + lane] = sEnd[lane];
-        scr[8 * HD + 8 + lane] = sEnd[16 + lane];
+        scr[FoldScratch<HD>::kM + lane] = sEnd[lane];
+        scr[FoldScratch<HD>::kL + lane] = sEnd[16 + lane];
     }
     __syncthreads();
     FoldTarget f;

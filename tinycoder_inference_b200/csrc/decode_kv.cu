@@ -27,7 +27,7 @@ template <int HD, int NW, int SLOTS>
 struct DecodeKvSmem {
     static constexpr int NB = HD / 32;             // 32-float boxes per row
     static constexpr int kTileBytes = 16 * HD * 4; // K (or V) bytes of a tile
-    static constexpr int kSlots = NW * SLOTS * 2 * kTileBytes, kScratch = NW * (8 * HD + 16) * 4;  // (the fold reuses the slots)
+    static constexpr int kSlots = NW * SLOTS * 2 * kTileBytes, kScratch = NW * FoldScratch<HD>::kWarp * 4;  // (the fold reuses the slots)
     static constexpr int kTotal = (kSlots > kScratch ? kSlots : kScratch) + 128;
     static_assert(kTotal <= 227 * 1024, "shared memory of an SM");
 };
@@ -322,21 +322,22 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKvKernel(const __grid_cons
     }
     namedBarSync(1, NW * 32);
     float *scr = reinterpret_cast<float *>(smem);
-    constexpr int kWarpScr = 8 * HD + 16;
+    using F = FoldScratch<HD>;
+    constexpr int kWarpScr = F::kWarp;
     float *wO = scr + warp * kWarpScr;
 #pragma unroll
     for (int bx = 0; bx < NB; ++bx) {
         const int d = 32 * bx + 4 * g;
-        *reinterpret_cast<float4 *>(wO + (2 * t) * HD + d) =
+        *reinterpret_cast<float4 *>(wO + (2 * t) * F::kRow + d) =
                 make_float4(o[2 * bx][0], o[2 * bx][2], o[2 * bx + 1][0], o[2 * bx + 1][2]);
-        *reinterpret_cast<float4 *>(wO + (2 * t + 1) * HD + d) =
+        *reinterpret_cast<float4 *>(wO + (2 * t + 1) * F::kRow + d) =
                 make_float4(o[2 * bx][1], o[2 * bx][3], o[2 * bx + 1][1], o[2 * bx + 1][3]);
     }
     if (g == 0) {
-        wO[8 * HD + 2 * t] = m0;
-        wO[8 * HD + 2 * t + 1] = m1;
-        wO[8 * HD + 8 + 2 * t] = l0;
-        wO[8 * HD + 8 + 2 * t + 1] = l1;
+        wO[F::kM + 2 * t] = m0;
+        wO[F::kM + 2 * t + 1] = m1;
+        wO[F::kL + 2 * t] = l0;
+        wO[F::kL + 2 * t + 1] = l1;
     }
     namedBarSync(1, NW * 32);
     if (!ROWS) {
@@ -356,15 +357,15 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKvKernel(const __grid_cons
         if (!colValid(j)) continue;
         float M = kNegBig;
 #pragma unroll
-        for (int w = 0; w < NW; ++w) M = fmaxf(M, scr[w * kWarpScr + 8 * HD + j]);
+        for (int w = 0; w < NW; ++w) M = fmaxf(M, scr[w * kWarpScr + F::kM + j]);
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
         float lsum = 0.0f;
 #pragma unroll
         for (int w = 0; w < NW; ++w) {
             const float *s = scr + w * kWarpScr;
-            const float wgt = fastExp2(s[8 * HD + j] - M);
-            lsum += wgt * s[8 * HD + 8 + j];
-            const float4 a = *reinterpret_cast<const float4 *>(s + j * HD + 4 * d4);
+            const float wgt = fastExp2(s[F::kM + j] - M);
+            lsum += wgt * s[F::kL + j];
+            const float4 a = *reinterpret_cast<const float4 *>(s + j * F::kRow + 4 * d4);
             acc.x = fmaf(wgt, a.x, acc.x);
             acc.y = fmaf(wgt, a.y, acc.y);
             acc.z = fmaf(wgt, a.z, acc.z);

@@ -27,7 +27,7 @@ template <int HD, int NW, int SLOTS>
 struct DecodeKv16Smem {
     static constexpr int kAtomBytes = 16 * 128;      // one half-tile
     static constexpr int kTileBytes = 16 * HD * 2;
-    static constexpr int kSlots = NW * SLOTS * 2 * kTileBytes, kScratch = NW * (8 * HD + 16) * 4;  // (the fold reuses the slots)
+    static constexpr int kSlots = NW * SLOTS * 2 * kTileBytes, kScratch = NW * FoldScratch<HD>::kWarp * 4;  // (the fold reuses the slots)
     static constexpr int kTotal = (kSlots > kScratch ? kSlots : kScratch) + 128;
     static_assert(kTotal <= 227 * 1024, "shared memory of an SM");
 };
@@ -296,21 +296,22 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKv16Kernel(const __grid_co
     }
     namedBarSync(1, NW * 32);  // every consumer is done reading the ring
     float *scr = reinterpret_cast<float *>(smem);
-    constexpr int kWarpScr = 8 * HD + 16;
-    float *wO = scr + warp * kWarpScr;  // [8 columns][HD], then m[8], l[8]
+    using F = FoldScratch<HD>;
+    constexpr int kWarpScr = F::kWarp;
+    float *wO = scr + warp * kWarpScr;  // [8 columns][FoldScratch::kRow], then m[8], l[8]
 #pragma unroll
     for (int c = 0; c < NS; ++c) {
         const int d = 16 * c + g;
-        wO[(2 * t) * HD + d] = o[c][0];
-        wO[(2 * t + 1) * HD + d] = o[c][1];
-        wO[(2 * t) * HD + d + 8] = o[c][2];
-        wO[(2 * t + 1) * HD + d + 8] = o[c][3];
+        wO[(2 * t) * F::kRow + d] = o[c][0];
+        wO[(2 * t + 1) * F::kRow + d] = o[c][1];
+        wO[(2 * t) * F::kRow + d + 8] = o[c][2];
+        wO[(2 * t + 1) * F::kRow + d + 8] = o[c][3];
     }
     if (g == 0) {
-        wO[8 * HD + 2 * t] = m0;
-        wO[8 * HD + 2 * t + 1] = m1;
-        wO[8 * HD + 8 + 2 * t] = l0;
-        wO[8 * HD + 8 + 2 * t + 1] = l1;
+        wO[F::kM + 2 * t] = m0;
+        wO[F::kM + 2 * t + 1] = m1;
+        wO[F::kL + 2 * t] = l0;
+        wO[F::kL + 2 * t + 1] = l1;
     }
     namedBarSync(1, NW * 32);
     if (!ROWS) {
@@ -330,15 +331,15 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKv16Kernel(const __grid_co
         if (!colValid(j)) continue;
         float M = kNegBig;
 #pragma unroll
-        for (int w = 0; w < NW; ++w) M = fmaxf(M, scr[w * kWarpScr + 8 * HD + j]);
+        for (int w = 0; w < NW; ++w) M = fmaxf(M, scr[w * kWarpScr + F::kM + j]);
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
         float lsum = 0.0f;
 #pragma unroll
         for (int w = 0; w < NW; ++w) {
             const float *s = scr + w * kWarpScr;
-            const float wgt = fastExp2(s[8 * HD + j] - M);
-            lsum += wgt * s[8 * HD + 8 + j];
-            const float4 a = *reinterpret_cast<const float4 *>(s + j * HD + 4 * d4);
+            const float wgt = fastExp2(s[F::kM + j] - M);
+            lsum += wgt * s[F::kL + j];
+            const float4 a = *reinterpret_cast<const float4 *>(s + j * F::kRow + 4 * d4);
             acc.x = fmaf(wgt, a.x, acc.x);
             acc.y = fmaf(wgt, a.y, acc.y);
             acc.z = fmaf(wgt, a.z, acc.z);
