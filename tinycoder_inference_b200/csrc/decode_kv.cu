@@ -23,14 +23,17 @@
 namespace tc {
 
 // Every warp has SLOTS slots for 16-token tiles of K and as many of V, each as HD / 32 boxes of [16 rows][32 floats].
-template <int HD, int NW, int SLOTS>
+template <int HD, int NW, int SLOTS, bool SHAREQ>
 struct DecodeKvSmem {
     static constexpr int NB = HD / 32;             // 32-float boxes per row
     static constexpr int kTileBytes = 16 * HD * 4; // K (or V) bytes of a tile
     static constexpr int kSlots = NW * SLOTS * 2 * kTileBytes, kScratch = NW * FoldScratch<HD>::kWarp * 4;  // (the fold reuses the slots)
-    static constexpr int kTotal = (kSlots > kScratch ? kSlots : kScratch) + 128;
+    static constexpr int kQuery = kSlots > kScratch ? kSlots : kScratch;   // decode: the block's query operands
+    static constexpr int kTotal = kQuery + (SHAREQ ? HD * 64 : 0) + 128;
     static_assert(kTotal <= 227 * 1024, "shared memory of an SM");
 };
+
+constexpr bool kvSharesQuery(int hd, int blocksPerSm, bool rows) { return !rows && hd >= 128 && blocksPerSm == 1; }
 
 __device__ __forceinline__ void splitTf32(float x, uint32_t &hi, uint32_t &lo) {
     hi = toTf32(x);
@@ -47,7 +50,12 @@ __device__ __forceinline__ void splitTf32(float x, uint32_t &hi, uint32_t &lo) {
 // too few of them (17 us; this form 15).  192 MB of one layer (28 / 4 / 128 at 47000 rows): 42 us.
 template <int HD, int NW, int SLOTS, int BPS, bool ROWS>
 __global__ void __launch_bounds__(NW * 32, BPS) decodeKvKernel(const __grid_constant__ DecodeKvParams p) {
-    using L = DecodeKvSmem<HD, NW, SLOTS>;
+    // The block's warps prepare the query together, but where it is cheap (head_dim 64) or registers and shared memory are short
+    // (two blocks per SM).  One of head_dim 256 stays in shared memory: 128 registers, and the spills that came with them.
+    // 28 / 4 / 128, per layer: 2047 rows 7.85 -> 7.65 us, 8191 rows 14.85 -> 14.6; 16 / 4 / 256 (norm and gate included) 14000
+    // rows 40.9 -> 35.8, 20000 rows 54.6 -> 45.0.
+    constexpr bool kShareQuery = kvSharesQuery(HD, BPS, ROWS), kQueryInRegs = HD <= 128 || !kShareQuery;
+    using L = DecodeKvSmem<HD, NW, SLOTS, kShareQuery>;
     constexpr int T = 16, NB = L::NB;
     constexpr int KS = HD / 8;   // tf32 k-steps of the QK product
     constexpr int MTO = HD / 16;  // 16-dim output tiles
@@ -57,7 +65,8 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKvKernel(const __grid_cons
 
     extern __shared__ uint8_t smemRaw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smemRaw) + 127) & ~uintptr_t(127));
-    __shared__ float pScratch[NW][16 * 8];
+    constexpr bool kOwnScratch = !kShareQuery || !kQueryInRegs;  // else where the query operands were
+    __shared__ float pScratch[kOwnScratch ? NW : 1][16 * 8];
 
     if (!ROWS) {
         // (a device position read here may be a step old: good enough to know which rows to pull)
@@ -128,8 +137,9 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKvKernel(const __grid_cons
 
     // q of column n = g as the B operand: k slot t / t+4 of step (bx, h, e) is
     // dim 32bx + 8t + 4h + 2e / +1 -- the order the swizzled 16-byte loads deliver.
-    uint32_t qhi[KS][2], qlo[KS][2];
-    {
+    uint32_t qhi[kQueryInRegs ? KS : 1][2], qlo[kQueryInRegs ? KS : 1][2];
+    const uint4 *frag = reinterpret_cast<const uint4 *>(smem + L::kQuery) + lane;  // [32-dim box][half][hi, lo][lane]
+    if constexpr (!kShareQuery) {
         const bool valid = colValid(g);
         const float *qp = p.q + colIndex(valid ? g : 0) * HD;
         float4 qv[NB][2];
@@ -173,6 +183,50 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKvKernel(const __grid_cons
                 splitTf32(v.z, qhi[ks + 1][0], qlo[ks + 1][0]);
                 splitTf32(v.w, qhi[ks + 1][1], qlo[ks + 1][1]);
             }
+    } else {
+        // a column at a time each, four dims to a lane, the operands left where they are read
+        uint4 *to = reinterpret_cast<uint4 *>(smem + L::kQuery);
+        for (uint32_t j = warp; j < 8; j += NW) {
+            const bool valid = colValid(j);
+            const float *qp = p.q + colIndex(valid ? j : 0) * HD;
+#pragma unroll
+            for (uint32_t i = lane; i < HD / 4; i += 32) {
+                // (plain loads: with a rotation q is written in place at the end of the launch)
+                float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (valid) x = *reinterpret_cast<const float4 *>(qp + 4 * i);
+                if (valid && p.tok.cosT != nullptr) {
+                    // NEOX rotation: the partner of dim d is d + HD / 2
+                    const bool upper = i >= HD / 8;
+                    const float4 y = *reinterpret_cast<const float4 *>(qp + 4 * (upper ? i - HD / 8 : i + HD / 8));
+                    const size_t at = static_cast<size_t>(len - 1u) * (HD / 2) + 4 * (upper ? i - HD / 8 : i);
+                    const float4 c = __ldg(reinterpret_cast<const float4 *>(p.tok.cosT + at));
+                    const float4 sn = __ldg(reinterpret_cast<const float4 *>(p.tok.sinT + at));
+                    auto rot = [upper](float own, float other, float cc, float ss) {
+                        return upper ? fmaf(other, ss, __fmul_rn(own, cc)) : fmaf(own, cc, -__fmul_rn(other, ss));
+                    };
+                    x = make_float4(rot(x.x, y.x, c.x, sn.x), rot(x.y, y.y, c.y, sn.y), rot(x.z, y.z, c.z, sn.z),
+                                    rot(x.w, y.w, c.w, sn.w));
+                }
+                uint4 hi, lo;
+                splitTf32(x.x, hi.x, lo.x);
+                splitTf32(x.y, hi.y, lo.y);
+                splitTf32(x.z, hi.z, lo.z);
+                splitTf32(x.w, hi.w, lo.w);
+                // dims 4i ..: box i / 8, k slot (i % 8) / 2 of column j, half i % 2
+                const uint32_t at = ((i / 8) * 4 + (i & 1u) * 2) * 32 + j * 4 + (i % 8) / 2;
+                to[at] = hi, to[at + 32] = lo;
+            }
+        }
+        __syncthreads();
+        if constexpr (kQueryInRegs) {
+#pragma unroll
+            for (int k = 0; k < KS; k += 2) {
+                const uint4 hi = frag[k * 32], lo = frag[(k + 1) * 32];
+                qhi[k][0] = hi.x, qhi[k][1] = hi.y, qhi[k + 1][0] = hi.z, qhi[k + 1][1] = hi.w;
+                qlo[k][0] = lo.x, qlo[k][1] = lo.y, qlo[k + 1][0] = lo.z, qlo[k + 1][1] = lo.w;
+            }
+            __syncthreads();  // (the warps' scratch for probabilities takes their place)
+        }
     }
     const float cs = p.invSqrt * kLog2e;
     const uint32_t len0 = colLen(2 * t), len1 = colLen(2 * t + 1);
@@ -189,7 +243,8 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKvKernel(const __grid_cons
     float o[MTO][4];
 #pragma unroll
     for (int i = 0; i < MTO; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
-    float *pS = pScratch[warp];
+    static_assert(kOwnScratch || NW * 128 * 4 <= HD * 64, "scratch in place of the query operands");
+    float *pS = kOwnScratch ? pScratch[kOwnScratch ? warp : 0] : reinterpret_cast<float *>(smem + L::kQuery) + warp * 128;
 
     for (uint32_t i = 0, tile = warp; tile < nTiles; ++i, tile += NW) {
         cpAsyncWait<2 * SLOTS - 1>();  // K of this tile is in, V may still be on its way
@@ -208,15 +263,22 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKvKernel(const __grid_cons
                 const float4 xa = *reinterpret_cast<const float4 *>(kT + g * 128 + off);
                 const float4 xb = *reinterpret_cast<const float4 *>(kT + (g + 8) * 128 + off);
                 const int ks = (bx * 2 + h) * 2;
+                uint4 qh, ql;
+                if constexpr (kQueryInRegs) {
+                    qh = make_uint4(qhi[ks][0], qhi[ks][1], qhi[ks + 1][0], qhi[ks + 1][1]);
+                    ql = make_uint4(qlo[ks][0], qlo[ks][1], qlo[ks + 1][0], qlo[ks + 1][1]);
+                } else {
+                    qh = frag[ks * 32], ql = frag[(ks + 1) * 32];
+                }
                 {
                     uint32_t h0, l0_, h1, l1_, h2, l2_, h3, l3_;
                     splitTf32(xa.x, h0, l0_);
                     splitTf32(xb.x, h1, l1_);
                     splitTf32(xa.y, h2, l2_);
                     splitTf32(xb.y, h3, l3_);
-                    mmaTf32(sa[0], h0, h1, h2, h3, qhi[ks][0], qhi[ks][1]);
-                    mmaTf32(sb[0], l0_, l1_, l2_, l3_, qhi[ks][0], qhi[ks][1]);
-                    mmaTf32(sc[0], h0, h1, h2, h3, qlo[ks][0], qlo[ks][1]);
+                    mmaTf32(sa[0], h0, h1, h2, h3, qh.x, qh.y);
+                    mmaTf32(sb[0], l0_, l1_, l2_, l3_, qh.x, qh.y);
+                    mmaTf32(sc[0], h0, h1, h2, h3, ql.x, ql.y);
                 }
                 {
                     uint32_t h0, l0_, h1, l1_, h2, l2_, h3, l3_;
@@ -224,9 +286,9 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKvKernel(const __grid_cons
                     splitTf32(xb.z, h1, l1_);
                     splitTf32(xa.w, h2, l2_);
                     splitTf32(xb.w, h3, l3_);
-                    mmaTf32(sa[1], h0, h1, h2, h3, qhi[ks + 1][0], qhi[ks + 1][1]);
-                    mmaTf32(sb[1], l0_, l1_, l2_, l3_, qhi[ks + 1][0], qhi[ks + 1][1]);
-                    mmaTf32(sc[1], h0, h1, h2, h3, qlo[ks + 1][0], qlo[ks + 1][1]);
+                    mmaTf32(sa[1], h0, h1, h2, h3, qh.z, qh.w);
+                    mmaTf32(sb[1], l0_, l1_, l2_, l3_, qh.z, qh.w);
+                    mmaTf32(sc[1], h0, h1, h2, h3, ql.z, ql.w);
                 }
             }
         }
@@ -386,7 +448,7 @@ struct KvShape {
 template <int HD>
 static int launchRows(const DecodeKvParams &prm, cudaStream_t st) {
     constexpr int NW = KvShape<HD>::kRowsWarps;
-    using L = DecodeKvSmem<HD, NW, 1>;
+    using L = DecodeKvSmem<HD, NW, 1, false>;
     auto kern = decodeKvKernel<HD, NW, 1, 1, true>;
     static bool attrDone[64] = {false};
     int dev = 0;
@@ -456,10 +518,10 @@ static int prefillKv(const float *q, const void *kvK, const void *kvV, float *ou
 
 template <int HD, int NW, int SLOTS, int BPS>
 static int decodeKv32(const DecodeKvParams &prm, uint8_t *q81Out, cudaStream_t st) {
-    using L = DecodeKvSmem<HD, NW, SLOTS>;
+    using L = DecodeKvSmem<HD, NW, SLOTS, kvSharesQuery(HD, BPS, false)>;
     static ClusterSetup setup;
     return launchKvDecode(setup, decodeKvKernel<HD, NW, SLOTS, BPS, false>, NW * 32, L::kTotal, HD, NW, 2 * L::kTileBytes,
-                          HD == 256 ? 4.2f : (HD == 128 ? 2.85f : 1.7f), HD == 256 ? 1.2f : (HD == 128 ? 0.38f : 0.2f), prm,
+                          HD == 256 ? 3.4f : (HD == 128 ? 2.85f : 1.7f), HD == 256 ? 0.8f : (HD == 128 ? 0.38f : 0.2f), prm,
                           q81Out, st);
 }
 
@@ -495,12 +557,12 @@ int decodeKvToken(const float *q, const void *kvK, const void *kvV, float *attnO
     if (kvHalf) return decodeKv16(prm, hd, q81Out, st);
     // Warps of a block, slots of a warp, blocks per SM.  Rows that a 16-block cluster covers with one tile per warp (head_dim
     // 128: 1536) want small blocks; longer ones as many warps per SM as fit (head_dim 128, per layer: 2048 rows 8.6 against
-    // 9.5 us, 20000 rows 23.8 against 26.4, 200 rows 7.2 against 6.5; head_dim 256: 8191 / 20000 rows 19.5 / 36.2 us with
-    // four warps per SM, 21.5 / 29.8 with six).
+    // 9.5 us, 20000 rows 23.8 against 26.4, 200 rows 7.2 against 6.5; head_dim 256, 16 / 4 heads with norm and gate: four warps 12.4 /
+    // 32.4 / 43.1 us at 500 / 8191 / 12000 rows, six 11.9 / 29.0 / 34.6).
     if (hd == 64) return decodeKv32<64, 8, 2, 1>(prm, q81Out, st);
     if (hd == 128)
         return prm.lenHost <= 1536u ? decodeKv32<128, 6, 1, 2>(prm, q81Out, st) : decodeKv32<128, 8, 1, 1>(prm, q81Out, st);
-    return prm.lenHost <= 12288u ? decodeKv32<256, 4, 1, 1>(prm, q81Out, st) : decodeKv32<256, 6, 1, 1>(prm, q81Out, st);
+    return decodeKv32<256, 6, 1, 1>(prm, q81Out, st);
 }
 
 }  // namespace tc

@@ -23,12 +23,13 @@ namespace tc {
 
 // Every warp has SLOTS slots for 16-token tiles of K and as many of V, each as HD / 64 half-tiles of [16 rows][64 halves =
 // 128 bytes], half-tile a covering dims [64a, 64a + 64).
-template <int HD, int NW, int SLOTS>
+template <int HD, int NW, int SLOTS, bool ROWS>
 struct DecodeKv16Smem {
     static constexpr int kAtomBytes = 16 * 128;      // one half-tile
     static constexpr int kTileBytes = 16 * HD * 2;
     static constexpr int kSlots = NW * SLOTS * 2 * kTileBytes, kScratch = NW * FoldScratch<HD>::kWarp * 4;  // (the fold reuses the slots)
-    static constexpr int kTotal = (kSlots > kScratch ? kSlots : kScratch) + 128;
+    static constexpr int kQuery = kSlots > kScratch ? kSlots : kScratch;   // decode: the block's query operands
+    static constexpr int kTotal = kQuery + (ROWS ? 0 : HD * 32 + 32) + 128;
     static_assert(kTotal <= 227 * 1024, "shared memory of an SM");
 };
 
@@ -38,7 +39,7 @@ constexpr float kLazyLog2Kv16 = 8.0f;  // see decode_i8.cu: p stays <= 2^8, exac
 // share a kv head's tokens.
 template <int HD, int NW, int SLOTS, int BPS, bool ROWS>
 __global__ void __launch_bounds__(NW * 32, BPS) decodeKv16Kernel(const __grid_constant__ DecodeKvParams p) {
-    using L = DecodeKv16Smem<HD, NW, SLOTS>;
+    using L = DecodeKv16Smem<HD, NW, SLOTS, ROWS>;
     constexpr int T = 16;
     constexpr int NS = HD / 16;     // k16 steps of QK^T = 16-dim output tiles of PV
 
@@ -118,8 +119,12 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKv16Kernel(const __grid_co
     // q of column n = g as the B operand of k16 step s: b0 = dims 16s + 2t, +1; b1 = dims
     // 16s + 8 + 2t, +1.  Power-of-two normalised, split into fp16 hi + lo.
     uint32_t qhi[NS][2], qlo[NS][2];
-    float headScale;
-    {
+    float cs0, cs1;
+    auto exponent = [](float amax) {
+        const int e = static_cast<int>((__float_as_uint(amax) >> 23) & 0xffu) - 127;  // floor(log2 amax)
+        return amax > 0.0f ? max(-100, min(100, e)) : 0;
+    };
+    if constexpr (ROWS) {
         const bool valid = colValid(g);
         const float *qp = p.q + colIndex(valid ? g : 0) * HD;
         float2 qv[NS][2];
@@ -128,37 +133,16 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKv16Kernel(const __grid_co
         for (int s = 0; s < NS; ++s)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                // (a plain load: with a rotation q is written in place at the end of the launch)
                 qv[s][h] = valid ? *reinterpret_cast<const float2 *>(qp + 16 * s + 8 * h + 2 * t)
                                  : make_float2(0.f, 0.f);
+                amax = fmaxf(amax, fmaxf(fabsf(qv[s][h].x), fabsf(qv[s][h].y)));
             }
-        if (!ROWS && p.tok.cosT != nullptr) {
-            // NEOX rotation: the partner of dim d is d + HD / 2, NS / 2 steps further on
-            const size_t row = static_cast<size_t>(len - 1u) * (HD / 2);
-#pragma unroll
-            for (int s = 0; s < NS / 2; ++s)
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int d = 16 * s + 8 * h + 2 * t;
-                    const float2 c = __ldg(reinterpret_cast<const float2 *>(p.tok.cosT + row + d));
-                    const float2 sn = __ldg(reinterpret_cast<const float2 *>(p.tok.sinT + row + d));
-                    float2 &x = qv[s][h], &y = qv[s + NS / 2][h];
-                    const float2 x0 = x, x1 = y;
-                    x = make_float2(fmaf(x0.x, c.x, -__fmul_rn(x1.x, sn.x)), fmaf(x0.y, c.y, -__fmul_rn(x1.y, sn.y)));
-                    y = make_float2(fmaf(x0.x, sn.x, __fmul_rn(x1.x, c.x)), fmaf(x0.y, sn.y, __fmul_rn(x1.y, c.y)));
-                }
-        }
-#pragma unroll
-        for (int s = 0; s < NS; ++s)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) amax = fmaxf(amax, fmaxf(fabsf(qv[s][h].x), fabsf(qv[s][h].y)));
         amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
         amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-        int e = static_cast<int>((__float_as_uint(amax) >> 23) & 0xffu) - 127;  // floor(log2 amax)
-        e = amax > 0.0f ? max(-100, min(100, e)) : 0;
+        const int e = exponent(amax);
         const float down = __uint_as_float(static_cast<uint32_t>(127 - e) << 23);  // 2^-e
         const float up = __uint_as_float(static_cast<uint32_t>(127 + e) << 23);    // 2^e
-        headScale = p.invSqrt * up * kLog2e;
+        const float headScale = p.invSqrt * up * kLog2e;
 #pragma unroll
         for (int s = 0; s < NS; ++s)
 #pragma unroll
@@ -169,9 +153,58 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKv16Kernel(const __grid_co
                 qhi[s][h] = packHalf2(h0, h1);
                 qlo[s][h] = packHalf2(l0, l1);
             }
+        cs0 = __shfl_sync(0xffffffffu, headScale, (2 * t) * 4);
+        cs1 = __shfl_sync(0xffffffffu, headScale, (2 * t + 1) * 4);
+    } else {
+        // The block's warps share the work, a column at a time each: a lane takes dims 2 lane, + 1 of both halves of the
+        // vector (partners of the NEOX rotation) and leaves them where the operands are read.  (Every warp for itself took 350
+        // instructions.  Per layer, before -> with this: 28 / 4 / 128 at 500 / 2000 / 8191 rows 5.05 / 5.9 / 9.45 -> 4.45 / 5.2 / 8.55
+        // us, 14 / 2 / 64 at 2000 rows 4.7 -> 4.5; 8 / 4 / 64 at 20 rows 3.3 -> 3.4.)
+        uint32_t *frag = reinterpret_cast<uint32_t *>(smem + L::kQuery);  // [step][lane]: hi 0, hi 1, lo 0, lo 1
+        float *scale = reinterpret_cast<float *>(smem + L::kQuery + HD * 32);
+        for (uint32_t j = warp; j < 8; j += NW) {
+            const bool valid = colValid(j) && 2 * lane < HD / 2;
+            // (plain loads: with a rotation q is written in place at the end of the launch)
+            float2 x = make_float2(0.f, 0.f), y = x;
+            if (valid) {
+                const float *qp = p.q + colIndex(j) * HD + 2 * lane;
+                x = *reinterpret_cast<const float2 *>(qp), y = *reinterpret_cast<const float2 *>(qp + HD / 2);
+                if (p.tok.cosT != nullptr) {
+                    const size_t at = static_cast<size_t>(len - 1u) * (HD / 2) + 2 * lane;
+                    const float2 c = __ldg(reinterpret_cast<const float2 *>(p.tok.cosT + at));
+                    const float2 sn = __ldg(reinterpret_cast<const float2 *>(p.tok.sinT + at));
+                    const float2 x0 = x, x1 = y;
+                    x = make_float2(fmaf(x0.x, c.x, -__fmul_rn(x1.x, sn.x)), fmaf(x0.y, c.y, -__fmul_rn(x1.y, sn.y)));
+                    y = make_float2(fmaf(x0.x, sn.x, __fmul_rn(x1.x, c.x)), fmaf(x0.y, sn.y, __fmul_rn(x1.y, c.y)));
+                }
+            }
+            const float top = fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(y.x), fabsf(y.y)));
+            // (maxima of non-negative floats, by their bits)
+            const int e = exponent(__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(top))));
+            const float down = __uint_as_float(static_cast<uint32_t>(127 - e) << 23);  // 2^-e
+            if (lane == 0) scale[j] = p.invSqrt * __uint_as_float(static_cast<uint32_t>(127 + e) << 23) * kLog2e;
+            if (2 * lane < HD / 2) {
+#pragma unroll
+                for (uint32_t half = 0; half < 2; ++half) {
+                    const float2 v = half ? y : x;
+                    const uint32_t dim = half * (HD / 2) + 2 * lane;
+                    uint32_t *to = frag + ((dim / 16) * 32 + j * 4 + (dim % 8) / 2) * 4 + (dim % 16) / 8;
+                    float h0, l0, h1, l1;
+                    splitHalf(v.x * down, h0, l0);
+                    splitHalf(v.y * down, h1, l1);
+                    to[0] = packHalf2(h0, h1);
+                    to[2] = packHalf2(l0, l1);
+                }
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+            const uint4 f = *reinterpret_cast<const uint4 *>(frag + (s * 32 + lane) * 4);
+            qhi[s][0] = f.x, qhi[s][1] = f.y, qlo[s][0] = f.z, qlo[s][1] = f.w;
+        }
+        cs0 = scale[2 * t], cs1 = scale[2 * t + 1];
     }
-    const float cs0 = __shfl_sync(0xffffffffu, headScale, (2 * t) * 4);
-    const float cs1 = __shfl_sync(0xffffffffu, headScale, (2 * t + 1) * 4);
     const uint32_t len0 = colLen(2 * t), len1 = colLen(2 * t + 1);
 
     if (mine) {
@@ -353,7 +386,7 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKv16Kernel(const __grid_co
 
 template <int HD, int NW, int SLOTS, int BPS>
 static int decodeKv16Hd(const DecodeKvParams &prm, uint8_t *q81Out, cudaStream_t st) {
-    using L = DecodeKv16Smem<HD, NW, SLOTS>;
+    using L = DecodeKv16Smem<HD, NW, SLOTS, false>;
     static ClusterSetup setup;
     return launchKvDecode(setup, decodeKv16Kernel<HD, NW, SLOTS, BPS, false>, NW * 32, L::kTotal, HD, NW, 2 * L::kTileBytes,
                           HD == 128 ? 0.87f : 0.73f, HD == 128 ? 0.12f : 0.08f, prm, q81Out, st);
@@ -375,7 +408,7 @@ int decodeKv16(const DecodeKvParams &prm, uint32_t hd, uint8_t *q81Out, cudaStre
 template <int HD>
 static int rowsKv16Hd(const DecodeKvParams &prm, cudaStream_t st) {
     constexpr int NW = 16;
-    using L = DecodeKv16Smem<HD, NW, 1>;
+    using L = DecodeKv16Smem<HD, NW, 1, true>;
     auto kern = decodeKv16Kernel<HD, NW, 1, 1, true>;
     static bool attrDone[64] = {false};
     int dev = 0;
