@@ -13,9 +13,7 @@ from tests.util import assert_close, dev, host
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("S,pos", [(1, 0), (63, 0), (64, 0), (65, 0), (2, 127), (128, 64), (129, 63), (257, 190)])
-@pytest.mark.parametrize("nH,nKV,hd", [(7, 1, 64), (6, 2, 128), (4, 2, 256)])
-def test_tile_edges(S, pos, nH, nKV, hd):
+def _check(S, pos, nH, nKV, hd):
     r = np.random.default_rng(S + pos + hd)
     q, k, v = (r.standard_normal((n, h, hd), dtype=np.float32) for n, h in ((S, nH), (pos + S, nKV), (pos + S, nKV)))
     out = torch.full((S + 1, nH, hd), float("nan"), device="cuda")
@@ -30,3 +28,19 @@ def test_tile_edges(S, pos, nH, nKV, hd):
     # probabilities are rounded to fp16 (2^-11 each, both in the sums): 2^-10 of the largest |v| of N(0, 1) rows (4.5)
     assert_close(host(out[:S]), want, rtol=0.0, atol=4.5e-3, what=f"{S} rows behind {pos}")
     assert torch.isnan(out[S]).all()
+
+
+@pytest.mark.parametrize("S,pos", [(1, 0), (63, 0), (64, 0), (65, 0), (2, 127), (128, 64), (129, 63), (257, 190)])
+@pytest.mark.parametrize("nH,nKV,hd", [(7, 1, 64), (6, 2, 128), (4, 2, 256)])
+def test_tile_edges(S, pos, nH, nKV, hd):
+    _check(S, pos, nH, nKV, hd)
+
+
+# few items: clusters of 8, 4 and 2 blocks share an item's KV tiles; ragged rows, KV tiles that do not divide evenly, rows
+# whose blocks have no tile at all (no prefix, long calls) or only tiles behind their diagonal
+@pytest.mark.parametrize("S,pos,nH,nKV,hd", [(1, 3000, 14, 2, 64), (100, 1500, 8, 4, 64), (385, 1900, 8, 4, 64), (512, 1600, 14, 2, 64),
+                                             (77, 1217, 12, 2, 128), (1100, 0, 3, 1, 128), (512, 777, 8, 2, 128),
+                                             (130, 2500, 28, 4, 128), (77, 1500, 2, 1, 256), (1000, 0, 4, 2, 256),
+                                             (300, 601, 16, 2, 256)])
+def test_items_shared_by_a_cluster(S, pos, nH, nKV, hd):
+    _check(S, pos, nH, nKV, hd)

@@ -15,6 +15,8 @@
 // tile whose KV tiles the two halves of the block share (even / odd) and put together at the end: 512 rows
 // behind 3584 of 28 q heads of 128 take 48.6 us, with one half idle 55.5.  At head_dim 256 a block
 // holds one query tile (2000 rows of 16 heads: 55.9 us, with 32-token KV tiles 79.0).
+// Calls of so few one-tile items that blocks would be left without give each item to a cluster of 2 - 8 blocks, which share its KV
+// tiles and put their results together through distributed shared memory (SHARED below).
 // The first item of a block is its index, the following ones come from a
 // counter, heavy (late) query blocks first; the mbarriers are initialised once, every ring index
 // counts on from item to item, so the next item's loads and first score products run under the
@@ -44,6 +46,7 @@
 #include <algorithm>
 #include <cstring>
 
+#include "decode_cluster.cuh"
 #include "prefill_rows.cuh"
 #include "tc_tcgen05.cuh"
 
@@ -347,9 +350,12 @@ __device__ __forceinline__ uint64_t descAdvance(uint64_t d, uint32_t bytes) { re
 // may lie wholly past the sequence.  Split items (128 query rows): both halves of the block work on the same query
 // tile, A on the even KV tiles, B on the odd ones, and put their results together at the end -- a call too short to give
 // every SM a two-tile item is bound by the chain of one tile's steps, not by the tensor pipe.
+// SHARED: block r of a cluster of C takes KV tiles r, r + C, ... of the item (none, if there are fewer than r + 1); nA, nB and
+// nTiles count those.
 struct PfItem {
     uint32_t head, kvHead, m0, nA, nB, nTiles;
 };
+template <bool SHARED>
 __device__ __forceinline__ PfItem pfItem(const PrefillF16Params &p, uint32_t item) {
     PfItem it;
     const uint32_t qb = p.nQTiles - 1u - item / p.nHeads;  // heavy query blocks (long causal prefixes) first
@@ -362,6 +368,10 @@ __device__ __forceinline__ PfItem pfItem(const PrefillF16Params &p, uint32_t ite
     it.nA = tilesOf(it.m0);
     it.nB = p.itemRows > kPfBM && it.m0 + kPfBM < p.seqLen ? tilesOf(it.m0 + kPfBM) : 0u;
     it.nTiles = max(it.nA, it.nB);
+    if constexpr (SHARED) {
+        const uint32_t r = clusterRank(), c = clusterSize();
+        it.nA = it.nTiles = it.nTiles > r ? (it.nTiles - r + c - 1u) / c : 0u, it.nB = 0u;
+    }
     if (p.split) it.nB = it.nTiles / 2u, it.nA = it.nTiles - it.nB;
     return it;
 }
@@ -378,7 +388,12 @@ __device__ __forceinline__ PfItem pfItem(const PrefillF16Params &p, uint32_t ite
 // product has been issued, its first scores are in TMEM while the softmax threads still write this
 // item's output, and tile A moves on while tile B finishes its two extra diagonal tiles.
 constexpr int kPfThreads = 416;
-template <int HD>
+//
+// SHARED: a cluster works on ONE item and leaves.  What bounds an item alone is the chain of its KV tiles' steps (0.9 us
+// each), while SMs stand idle.  Per call, one block -> the cluster that prefillShare picks, rows @ rows in front: 8 / 2 / 128 512 @ 512 /
+// 1536 / 3584 17.5 / 25.3 / 41.3 -> 16.4 / 17.7 / 22.6 us, 16 / 2 / 256 25.6 / 39.6 / 67.8 -> 20.9 / 28.3 / 43.4, 14 / 2 / 64 512 @ 3584
+// 36.7 -> 24.8, 28 / 4 / 128 100 @ 3000 34.3 -> 20.8.  Putting the results together is what limits it: 3 - 8 us.
+template <int HD, bool SHARED>
 __global__ void __launch_bounds__(kPfThreads, 1)
 prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const PrefillF16Params p) {
@@ -405,6 +420,11 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     volatile uint32_t *itemSlots = reinterpret_cast<volatile uint32_t *>(smem + L::kItemSlots);  // [4]
     const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31u;
     const bool split = !kOne && p.split != 0;
+    const uint32_t rank = SHARED ? clusterRank() : 0u, share = SHARED ? clusterSize() : 1u;  // KV tile j of the block: share j + rank
+    // what a softmax thread hands to the cluster: its row's maximum and sum over the block's tiles, the weights of the halves'
+    // accumulators
+    float rowM = kNegBig, rowL = 0.0f, rowW = 1.0f, rowW2 = 0.0f;
+    bool rowBoth = false, rowAny = false;
 
     if (threadIdx.x == 0) {
         mbarInit(qFull, 1);
@@ -459,7 +479,7 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     if (warp == 8) {
         // ------------------------ TMA producer and scheduler ------------------------
         if (lane == 0) {
-            uint32_t item = blockIdx.x, gk = 0, gv = 0;  // gk / gv: K / V tiles requested so far, over all items
+            uint32_t item = SHARED ? blockIdx.x / share : blockIdx.x, gk = 0, gv = 0;  // gk / gv: K / V tiles requested so far, over all items
             gridDepWait();  // the twins and the work counter come from the launch in front
             gridDepLaunch();
             itemSlots[0] = item;
@@ -471,7 +491,7 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 mbarExpectTx(&kFull[s], L::kKvTile);
 #pragma unroll
                 for (int h = 0; h < L::kHalves; ++h)
-                    tmaLoad3D(smem + L::kK + s * L::kKvTile + h * L::kKvHalf, &tmK, &kFull[s], 64 * h, kvHead, j * BN);
+                    tmaLoad3D(smem + L::kK + s * L::kKvTile + h * L::kKvHalf, &tmK, &kFull[s], 64 * h, kvHead, (share * j + rank) * BN);
                 ++gk;
                 return true;
             };
@@ -481,12 +501,13 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 mbarExpectTx(&vFull[s], L::kKvTile);
 #pragma unroll
                 for (int h = 0; h < L::kHalves; ++h)
-                    tmaLoad3D(smem + L::kV + s * L::kKvTile + h * L::kKvHalf, &tmV, &vFull[s], 64 * h, kvHead, j * BN);
+                    tmaLoad3D(smem + L::kV + s * L::kKvTile + h * L::kKvHalf, &tmV, &vFull[s], 64 * h, kvHead, (share * j + rank) * BN);
                 ++gv;
                 return true;
             };
             for (uint32_t n = 0; ok && item < p.totalItems; ++n) {
-                const PfItem it = pfItem(p, item);
+                const PfItem it = pfItem<SHARED>(p, item);
+                if (SHARED && it.nTiles == 0u) break;  // (nothing is loaded: the block's part of the cluster's end is all there is)
                 PF_BLK(0);
 #ifdef TC_TRACE
                 if (p.trace) { unsigned sm; asm("mov.u32 %0, %%smid;" : "=r"(sm)); p.trace[8u * 64u * 4u + item * 8u + 6] = sm; }
@@ -511,7 +532,7 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 const uint32_t drawAt = it.nTiles >= 3u ? it.nTiles - 3u : 0u;
                 uint32_t drawn = 0, flags = 0;
                 for (uint32_t j = 0; ok && j < it.nTiles; ++j) {
-                    if (j == drawAt) {
+                    if (!SHARED && j == drawAt) {
                         flags = *reinterpret_cast<volatile unsigned int *>(p.err);
                         drawn = gridDim.x + atomicAdd(p.workCounter, 1u);
                     }
@@ -520,7 +541,7 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 if (!ok) break;
                 // a wait that ran out anywhere ends the launch: the flag is the caller's to read
                 constexpr unsigned int kWaitBits = kDevErrFullWait | kDevErrEmptyWait | kDevErrMmaWait;
-                const uint32_t next = (flags & kWaitBits) != 0u ? p.totalItems : drawn;
+                const uint32_t next = SHARED || (flags & kWaitBits) != 0u ? p.totalItems : drawn;
                 itemSlots[(n + 1u) & 3u] = next;
                 mbarArrive(&itemFull[(n + 1u) & 3u]);
                 item = next;
@@ -555,7 +576,8 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         uint32_t g = 0, t = 0, item = 0;  // K (V) tiles of the items done, tiles of X done, over all items
         bool ok = !(kOne && x == 1u);
         for (uint32_t n = 0; ok && takeItem(n, item); ++n) {
-            const PfItem it = pfItem(p, item);
+            const PfItem it = pfItem<SHARED>(p, item);
+            if (SHARED && it.nTiles == 0u) break;
             const uint32_t myTiles = x == 0 ? it.nA : it.nB;
             // A split item's warps look at their own KV tiles only.  In a two-tile item every tile is released by both
             // query tiles' warps, also the ones past a tile's diagonal -- but only after it has been filled: a warp with
@@ -653,15 +675,16 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         uint32_t t = 0, item = 0;  // tiles of X done over all items
         bool ok = true;
         for (uint32_t n = 0; ok && takeItem(n, item); ++n) {
-            const PfItem it = pfItem(p, item);
+            const PfItem it = pfItem<SHARED>(p, item);
             const uint32_t m0 = it.m0, head = it.head;
             const uint32_t rq = m0 + rowInBlock;  // query position
             const uint32_t myTiles = x == 0 ? it.nA : it.nB;
+            if (SHARED && it.nTiles == 0u) break;
             if (myTiles == 0 && !split) continue;
             float m = kNegBig, l = 0.0f;
             for (uint32_t j = 0; j < myTiles; ++j) {
                 const uint32_t tt = t + j, b = tt & 1u;
-                const uint32_t kt = split ? 2u * j + x : j;  // KV tile
+                const uint32_t kt = share * (split ? 2u * j + x : j) + rank;  // KV tile
                 const uint32_t tS = tmemBase + 256u + 128u * x + (kAhead ? 0u : 64u * b), tP = kAhead ? tS + 64u + 32u * b : tS;
                 if (row == 0) PF_STAMP(x, j, 0);
                 if (!pfWait<kCall>(&sFull[kAhead ? x : 2u * x + b], (kAhead ? tt : tt >> 1) & 1u, p.err, kDevErrMmaWait)) {
@@ -796,12 +819,23 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 const float M = fmaxf(m, o.x), wMine = fastExp2(m - M);
                 wOther = fastExp2(o.x - M);
                 const float lAll = fmaf(wMine, l, wOther * o.y);
+                if constexpr (SHARED) {
+                    rowM = M, rowL = lAll, rowW = wMine, rowW2 = wOther;
+                    rowBoth = it.nB != 0u, rowAny = true;
+                    t += myTiles;
+                    continue;
+                }
                 inv = lAll > 0.0f ? 1.0f / lAll : 0.0f;
                 wOther *= inv;
                 inv *= wMine;
                 both = it.nB != 0u;
             } else {
                 tcFenceAfter();
+                if constexpr (SHARED) {
+                    rowM = m, rowL = l, rowAny = true;
+                    t += myTiles;
+                    continue;
+                }
                 inv = l > 0.0f ? 1.0f / l : 0.0f;
             }
             float *orow = p.out + (static_cast<size_t>(rq) * p.nHeads + head) * HD;
@@ -859,6 +893,112 @@ prefillF16Kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             t += myTiles;
         }
     }
+    if constexpr (SHARED) {
+        // Every block leaves its accumulators (relative to its own maximum), maxima and sums where its tiles were, and block o of the
+        // cluster puts the o-th share of the rows together, reading the others' memory row by row.  (Written into the owner's
+        // memory instead, a thread its row, 16 bytes at a time: 3 / 6 / 11 us at head_dim 64 / 128 / 256.)  Every thread takes
+        // part in the two barriers, whatever became of its waits.
+        constexpr uint32_t kRowBytes = HD * 4 + 16;  // (threads of a warp store different rows)
+        constexpr uint32_t kAt = kOne ? 0 : L::kK;   // (in split items the halves exchange through the second query tile's room)
+        static_assert(kAt + kPfBM * (kRowBytes + 12) <= L::kBars, "the tiles' room");
+        const uint32_t stage = smemAddr(smem + kAt), stageMl = stage + kPfBM * kRowBytes;
+        float *weights = reinterpret_cast<float *>(smem + kAt + kPfBM * (kRowBytes + 8));  // [block][row of this block's share]
+        const uint32_t x = warp >> 2, row = (warp & 3u) * 32u + lane;
+        if (warp < (kOne ? 4u : 8u)) {
+            const uint32_t laneBase = ((warp & 3u) * 32u) << 16;
+            if (x == 0u) asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(stageMl + row * 8u), "f"(rowM), "f"(rowL) : "memory");
+            constexpr uint32_t kChunks = HD / 32;
+            const uint32_t c0 = split ? x * (kChunks / 2) : 0u, c1 = split ? c0 + kChunks / 2 : kChunks;
+            const uint32_t tMine = tmemBase + 128u * x, tOther = tmemBase + 128u * (x ^ 1u);
+            // (block-uniform: a block without tiles has nothing in its accumulators; without odd tiles everything is in A)
+            const bool onlyOther = split && x == 1u && !rowBoth;
+            if (__all_sync(0xffffffffu, rowAny)) {
+#pragma unroll 1
+                for (uint32_t c = c0; c < c1; ++c) {
+                    uint32_t o[32];
+                    tmemLd32((onlyOther ? tOther : tMine) + laneBase + c * 32u, o);
+                    if (rowBoth) {
+                        uint32_t o2[32];
+                        tmemLd32(tOther + laneBase + c * 32u, o2);
+                        tmemLdWait();
+#pragma unroll
+                        for (int i = 0; i < 32; ++i)
+                            o[i] = __float_as_uint(fmaf(__uint_as_float(o2[i]), rowW2, __uint_as_float(o[i]) * rowW));
+                    } else {
+                        tmemLdWait();
+                        const float w = onlyOther ? rowW2 : rowW;
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * w);
+                    }
+#pragma unroll
+                    for (int i = 0; i < 32; i += 4)
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stage + row * kRowBytes + (c * 32u + i) * 4u),
+                                     "r"(o[i]), "r"(o[i + 1]), "r"(o[i + 2]), "r"(o[i + 3])
+                                     : "memory");
+                }
+            }
+        }
+        clusterSync();
+        const uint32_t rows = kPfBM / share, item = blockIdx.x / share;
+        const uint32_t head = item % p.nHeads, first = (p.nQTiles - 1u - item / p.nHeads) * p.itemRows;
+        constexpr uint32_t V4 = HD / 4;
+        // Every lane's access to another block's memory is a request of its own, one per cycle and SM (with the maxima and sums
+        // read beside each value, and this block's own results the same way, this took 8.4 us at head_dim 256): the weights of
+        // the blocks come first, once per row.
+        if (threadIdx.x < rows) {
+            float2 ml[8];
+            float M = kNegBig, l = 0.0f;
+#pragma unroll
+            for (uint32_t b = 0; b < 8u; ++b) {
+                ml[b] = make_float2(kNegBig, 0.0f);
+                if (b < share)
+                    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];"
+                                 : "=f"(ml[b].x), "=f"(ml[b].y) : "r"(mapRank(stageMl + (rank * rows + threadIdx.x) * 8u, b)));
+            }
+#pragma unroll
+            for (uint32_t b = 0; b < 8u; ++b) M = fmaxf(M, ml[b].x);
+#pragma unroll
+            for (uint32_t b = 0; b < 8u; ++b) l = fmaf(fastExp2(ml[b].x - M), ml[b].y, l);
+            const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+#pragma unroll
+            for (uint32_t b = 0; b < 8u; ++b)  // (0: no tile of that block has tokens for the row, or it has no tiles at all)
+                if (b < share) weights[b * rows + threadIdx.x] = ml[b].y != 0.0f ? fastExp2(ml[b].x - M) * inv : 0.0f;
+        }
+        __syncthreads();
+        constexpr uint32_t U = 4;  // outputs of a thread on the way together
+        const uint32_t total = min(rows, p.seqLen > first + rank * rows ? p.seqLen - first - rank * rows : 0u) * V4;
+        for (uint32_t i0 = threadIdx.x; i0 < total; i0 += U * kPfThreads) {
+            float4 acc[U];
+#pragma unroll
+            for (uint32_t u = 0; u < U; ++u) acc[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (uint32_t b = 0; b < share; ++b) {
+                const uint32_t from = mapRank(stage, b);
+                float4 a[U];
+#pragma unroll
+                for (uint32_t u = 0; u < U; ++u) {
+                    const uint32_t i = min(i0 + u * kPfThreads, total - 1u), at = (rank * rows + i / V4) * kRowBytes + i % V4 * 16u;
+                    if (b == rank) a[u] = *reinterpret_cast<const float4 *>(smem + kAt + at);
+                    else
+                        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                     : "=f"(a[u].x), "=f"(a[u].y), "=f"(a[u].z), "=f"(a[u].w) : "r"(from + at));
+                }
+#pragma unroll
+                for (uint32_t u = 0; u < U; ++u) {
+                    const float w = weights[b * rows + min(i0 + u * kPfThreads, total - 1u) / V4];
+                    if (w == 0.0f) continue;
+                    acc[u].x = fmaf(w, a[u].x, acc[u].x), acc[u].y = fmaf(w, a[u].y, acc[u].y);
+                    acc[u].z = fmaf(w, a[u].z, acc[u].z), acc[u].w = fmaf(w, a[u].w, acc[u].w);
+                }
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < U; ++u) {
+                const uint32_t i = i0 + u * kPfThreads;
+                if (i >= total) break;
+                *reinterpret_cast<float4 *>(p.out + (static_cast<size_t>(first + rank * rows + i / V4) * p.nHeads + head) * HD + i % V4 * 4u) = acc[u];
+            }
+        }
+        clusterSync();  // (nobody reads this block's memory any more)
+    }
     tcFenceBefore();
     __syncthreads();
     if (warp == 0) {
@@ -912,6 +1052,35 @@ int tc_attn_prefill_f16_scratch_bytes(uint32_t seqLen, uint32_t cachePos, uint32
 }  // extern "C"
 
 namespace tc {
+
+// How many blocks share an item's KV tiles.  All clusters have to be resident at once (2 blocks: 74 clusters, 4: 33, 8: 15).  In 0.1
+// us: a step of a block's halves takes 9; putting the blocks' results together takes 20 more than an item's own end, and
+// what the rows of a block cost to fetch from the others.
+static uint32_t prefillShare(uint32_t items, uint32_t tiles, uint32_t halves, uint32_t hd, const uint32_t *maxClusters) {
+    auto cost = [&](uint32_t c) { return (tiles + halves * c - 1u) / (halves * c) * 9u + (c > 1u ? 20u + hd * (c - 1u) / (4u * c) : 0u); };
+    uint32_t best = 1;
+    for (uint32_t lg = 1; lg <= 3; ++lg)
+        if (items <= maxClusters[lg] && cost(1u << lg) < cost(best)) best = 1u << lg;
+    return best;
+}
+
+template <int HD>
+static int launchPrefill(const PrefillF16Params &prm, uint32_t tiles, const CUtensorMap &tmQ, const CUtensorMap &tmK,
+                         const CUtensorMap &tmV, cudaStream_t st) {
+    constexpr size_t smem = PrefillF16Smem<HD>::kTotal;
+    static ClusterSetup setup, setupShared;
+    const uint32_t *limits = nullptr;
+    int rc = setupCluster(setup, prefillF16Kernel<HD, false>, kPfThreads, smem, &limits);
+    if (rc == TC_OK) rc = setupCluster(setupShared, prefillF16Kernel<HD, true>, kPfThreads, smem, &limits);
+    if (rc != TC_OK) return rc;
+    // (the blocks allocate TMEM and set up their barriers while the rows launch drains; the producer waits for it before its
+    // first load, nothing else reads its outputs)
+    const uint32_t share = prm.itemRows == kPfBM ? prefillShare(prm.totalItems, tiles, prm.split ? 2u : 1u, HD, limits) : 1u;
+    if (share > 1u)
+        return launchDependent(prefillF16Kernel<HD, true>, dim3(prm.totalItems * share), kPfThreads, smem, st, share, tmQ, tmK, tmV, prm);
+    const uint32_t grid = std::min<uint32_t>(prm.totalItems, static_cast<uint32_t>(numSMs()));  // one block per SM
+    return launchDependent(prefillF16Kernel<HD, false>, dim3(grid), kPfThreads, smem, st, 1, tmQ, tmK, tmV, prm);
+}
 
 int prefillF16(float *q, const PrefillKvStore &src, float *out, void *scratch, size_t scratchBytes, uint32_t seqLen,
                uint32_t cachePos, uint32_t nHeads, uint32_t nKV, uint32_t hd, float invSqrt, const PrefillMirror &mir,
@@ -1004,26 +1173,10 @@ int prefillF16(float *q, const PrefillKvStore &src, float *out, void *scratch, s
 #ifdef TC_TRACE
     prm.trace = tc::g_pfTrace;
 #endif
-    static bool attrDone[64] = {false};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 64 && !attrDone[dev]) {
-        TC_CUDA_OK(cudaFuncSetAttribute(prefillF16Kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        PrefillF16Smem<64>::kTotal));
-        TC_CUDA_OK(cudaFuncSetAttribute(prefillF16Kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        PrefillF16Smem<128>::kTotal));
-        TC_CUDA_OK(cudaFuncSetAttribute(prefillF16Kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        PrefillF16Smem<256>::kTotal));
-        attrDone[dev] = true;
-    }
-    const uint32_t grid = std::min<uint32_t>(prm.totalItems, static_cast<uint32_t>(sms));  // one block per SM
-    // (the blocks allocate TMEM and set up their barriers while the rows launch drains; the producer waits for it before its
-    // first load, nothing else reads its outputs)
-    if (hd == 64)
-        return launchDependent(prefillF16Kernel<64>, dim3(grid), kPfThreads, PrefillF16Smem<64>::kTotal, st, 1, tmQ, tmK, tmV, prm);
-    if (hd == 128)
-        return launchDependent(prefillF16Kernel<128>, dim3(grid), kPfThreads, PrefillF16Smem<128>::kTotal, st, 1, tmQ, tmK, tmV, prm);
-    return launchDependent(prefillF16Kernel<256>, dim3(grid), kPfThreads, PrefillF16Smem<256>::kTotal, st, 1, tmQ, tmK, tmV, prm);
+    const uint32_t tiles = (kvRows + kPfBN - 1u) / kPfBN;  // of the heaviest item
+    if (hd == 64) return launchPrefill<64>(prm, tiles, tmQ, tmK, tmV, st);
+    if (hd == 128) return launchPrefill<128>(prm, tiles, tmQ, tmK, tmV, st);
+    return launchPrefill<256>(prm, tiles, tmQ, tmK, tmV, st);
 }
 
 static int prefillStore(const float *q, const PrefillKvStore &src, float *out, void *scratch, size_t scratchBytes,
