@@ -305,3 +305,13 @@ def test_split_decode_replayed_at_a_growing_device_position(mode):
             want = oracle.attention_kv(q, K, V, 1, NH, NKV, HD, pos, inv)
             assert_close(host(douts[slot]), want, what=f"{mode}: graph replay {t} (position {pos}), slot {slot}")
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("mode,nH,nKV,hd,window,slots", [("f32", 2, 1, 64, 1, 1), ("f32", 14, 2, 64, 37, 3), ("f16", 12, 2, 128, 4099, 2),
+                                                         ("f16", 2, 1, 64, 3, 1), ("f32+i8", 16, 4, 256, 3001, 5)])
+def test_clear_zeroes_the_whole_store(mode, nH, nKV, hd, window, slots):
+    s = ops.KvSession(nH, nKV, hd, window, slots, mode=mode)
+    s.kvK.fill_(1.0)
+    s.kvV.fill_(float("nan"))
+    s.clear()
+    assert int(torch.count_nonzero(s.kvK)) == 0 and int(torch.count_nonzero(s.kvV)) == 0

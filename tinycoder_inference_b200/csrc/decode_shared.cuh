@@ -36,6 +36,9 @@ struct F32Mirror {
     float *k, *v;  // nullable: [rows][nKV][hd]
 };
 
+// `bytes` of K and of V zeroed (kv_write.cu)
+int kvClear(void *k, void *v, size_t bytes, cudaStream_t st);
+
 // int8 decode (decode_i8.cu): tc_attn_decode_i8_batch plus the mirror; lens[b] + lenAdd is the length on the device
 int decodeI8Common(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, const F32Mirror &mir, cudaStream_t st);
 // one sequence whose length the launch need not know (captured decode steps): no partials, one launch
@@ -45,10 +48,13 @@ int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, c
 
 #ifdef __CUDACC__
 // Bounded wait: the first poll, which most waits need alone, in front of a loop of up to 2^18 more, each parked for up to
-// 20 us by the hardware.  (A loop that reads the clock: captured int8 step of 28 / 4 / 128 at 12000 rows 23.6 us per layer
-// against 23.0, 8 sequences of 4098 rows 9.95 against 9.83.)
+// 20 us by the hardware.  (A loop that reads the clock: captured int8 step of 28 / 4 / 128 at 12000 rows 23.0 -> 23.6 us per layer,
+// 8 sequences of 4098 rows 9.83 -> 9.95.)  TEST: a first poll that does not park.  It is the better one where the phase is nearly
+// always complete (tcgen05 decode: 64 ragged sequences 185.8 -> 185.3 us, 5 of up to 9000 rows 13.1 -> 12.95 a layer) and
+// the worse one where warps do wait (captured step, 5000 rows, 11.95 -> 12.05).
+template <bool TEST = false>
 __device__ __forceinline__ bool mbarWait(uint64_t *bar, uint32_t parity, unsigned int *err, uint32_t errBit) {
-    if (mbarTestWait(bar, parity)) return true;
+    if (TEST ? mbarTestWait(bar, parity) : mbarTryWait(bar, parity)) return true;
 #pragma unroll 1
     for (uint32_t i = 0; i < (1u << 18); ++i)
         if (mbarTryWait(bar, parity)) return true;

@@ -83,8 +83,7 @@ int tc_kv_session_clear(tc_kv_session *s, tc_stream stream) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (!s->c.kvStoreI8) {
         const size_t bytes = static_cast<size_t>(s->g.kvLayerStride) * s->c.slots;
-        if (cudaMemsetAsync(s->c.kvK, 0, bytes, st) != cudaSuccess) return TC_ECUDA;
-        if (cudaMemsetAsync(s->c.kvV, 0, bytes, st) != cudaSuccess) return TC_ECUDA;
+        if (tc::kvClear(s->c.kvK, s->c.kvV, bytes, st) != TC_OK) return TC_ECUDA;
     }
     s->kvPos = 0;
     // the pool itself needs no memset: the next decode rebuilds exactly rows [0, pos)
