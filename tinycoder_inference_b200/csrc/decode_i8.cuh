@@ -107,7 +107,7 @@ __device__ __forceinline__ void i8LoadQuery(I8Query<HD> &f, const float *qp, boo
 // The same by all NW warps of a block together, through `share` in its shared memory: a warp takes HD / (16 NW) of the 16-dim
 // groups, then everybody reads all fragments.  (One warp alone spends 700 instructions on the 64 dims of a lane at head_dim
 // 256, and eight warps of an SM doing that for themselves 1.2 us of a decode call.)  Bit for bit what i8LoadQuery gives: the
-// sums keep its order.  Called by all threads of the block.
+// sums keep its order.  Called by all threads of those warps; BAR: a named barrier for them (0: they are the block).
 template <int HD, int NW>
 struct I8QueryShare {
     static constexpr int NC = HD / 16;
@@ -117,7 +117,7 @@ struct I8QueryShare {
     static constexpr int kBytes = kMax + NW * 128;
     static_assert(NC % NW == 0, "whole groups per warp");
 };
-template <int HD, int NW>
+template <int HD, int NW, int BAR = 0>
 __device__ __forceinline__ void i8LoadQueryShared(I8Query<HD> &f, uint8_t *share, const float *qp, bool valid, float invSqrt,
                                                   uint32_t warp, uint32_t lane) {
     using S = I8QueryShare<HD, NW>;
@@ -136,7 +136,11 @@ __device__ __forceinline__ void i8LoadQueryShared(I8Query<HD> &f, uint8_t *share
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
     top[warp * 32] = amax;
-    __syncthreads();
+    auto sync = [] {
+        if (BAR == 0) __syncthreads();
+        else namedBarSync(BAR, NW * 32);
+    };
+    sync();
 #pragma unroll
     for (int w = 0; w < NW; ++w) amax = fmaxf(amax, top[w * 32]);
     int e = static_cast<int>((__float_as_uint(amax) >> 23) & 0xffu) - 127;  // floor(log2 amax)
@@ -157,7 +161,7 @@ __device__ __forceinline__ void i8LoadQueryShared(I8Query<HD> &f, uint8_t *share
         const __half2 a = *reinterpret_cast<__half2 *>(&x.z), bb = *reinterpret_cast<__half2 *>(&x.w);
         sum[c * 32] = (h0 + __low2float(a)) + (h1 + __high2float(a)) + (h2 + __low2float(bb)) + (h3 + __high2float(bb));
     }
-    __syncthreads();
+    sync();
     float qsum = 0.0f;
 #pragma unroll
     for (int c = 0; c < NC; ++c) {

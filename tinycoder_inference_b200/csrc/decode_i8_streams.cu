@@ -35,7 +35,12 @@ struct I8StreamSmem {
     static constexpr int kMax = kScales + kScoreWarps * 4 * T * 4; // [2][score warp][12]: column maxima, V scale bits
     static constexpr int kEnd = kMax + 2 * kScoreWarps * 12 * 4;   // m[8], E, then l[8], sums of P x scale [8]
     static constexpr int kBars = kEnd + 32 * 4;                    // full, empty per slot
-    static constexpr int kTotal = kBars + 2 * kSlots * 8 + 128;
+    // The score warps prepare the query together where it is long (16 / 2 / 256, norm and gate included: 20 / 500 / 2000 / 5000 rows
+    // 10.0 / 10.5 / 14.2 / 25.3 -> 9.75 / 10.0 / 13.85 / 24.9 us a layer; 8 / 2 / 128 at 20 rows 5.65 -> 5.9).
+    static constexpr bool kShareQuery = HD > 128;
+    static constexpr int kQuery = kBars + 2 * kSlots * 8;          // the query operands
+    static constexpr int kTotal = kQuery + (kShareQuery ? I8QueryShare<HD, kScoreWarps>::kBytes : 0) + 128;
+    static_assert(kQuery % 16 == 0, "16-byte accesses");
     static_assert(FoldScratch<HD>::kWarp * 4 <= kV, "the fold reuses the K tiles");
     static_assert(kTotal <= 227 * 1024, "shared memory of an SM");
 };
@@ -126,7 +131,9 @@ decodeI8StreamsKernel(const __grid_constant__ DecodeI8Params p) {
         if (hasRow) fresh.load(p.appendK + newSrc, p.appendV + newSrc, lane);
         else requestK(warp + SW);
         I8Query<HD> qf;
-        i8LoadQuery<HD>(qf, p.q + static_cast<size_t>(head0 + (g < nValid ? g : 0u)) * HD, g < nValid, p.invSqrt, lane);
+        const float *qp = p.q + static_cast<size_t>(head0 + (g < nValid ? g : 0u)) * HD;
+        if constexpr (L::kShareQuery) i8LoadQueryShared<HD, SW, 1>(qf, smem + L::kQuery, qp, g < nValid, p.invSqrt, warp, lane);
+        else i8LoadQuery<HD>(qf, qp, g < nValid, p.invSqrt, lane);
         if (hasRow) {
             const size_t dst = static_cast<size_t>(len - 1u) * p.nKV + kvHead;
             uint8_t *tile = intoTile ? slotK(iLast) : nullptr;

@@ -312,7 +312,7 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         // K and V of tile `it`, completion on `bar` (its stage's fullBar, but for the tile with the appended row)
         auto requestRows = [&](uint32_t it, uint64_t *bar) -> bool {
             const uint32_t s = it % NS;
-            if (it >= NS && !mbarWait(&emptyBar[s], ((it / NS) - 1u) & 1u, p.err, kDevErrEmptyWait)) return false;
+            if (it >= NS && !mbarWait<true>(&emptyBar[s], ((it / NS) - 1u) & 1u, p.err, kDevErrEmptyWait)) return false;
             const uint32_t tok = t0 + it * T;
             if (!waited && (tok + T > p.prefetchRows || it >= p.earlyStages)) {
                 // rows the kernel in front may still be writing, or further ahead of the dependency
@@ -380,7 +380,7 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
             fresh.load(p.appendK + src, p.appendV + src, lane);
             okP = requestRows(it, rowFull);
             if (okP) requestScales(it, intoTile ? inTile : T);
-            okP = okP && mbarWait(rowFull, 0, p.err, kDevErrFullWait);
+            okP = okP && mbarWait<true>(rowFull, 0, p.err, kDevErrFullWait);
             if (okP && !outside) {
                 const uint64_t dst = row * p.nKV + kvHead;
                 float4 *mk = nullptr, *mv = nullptr;
@@ -415,15 +415,15 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         if (!pvRole) {
             constexpr uint32_t idQK = tcIdescI8(128, 32, 0, 0, 1, 1);   // K-major A (K tile), K-major B (q digits)
             const uint64_t dQd = tcDesc(smemAddr(smem + L::kQd), 16, 1024, 2);
-            bool ok = mbarWait(qFull, 0, p.err, kDevErrFullWait);
+            bool ok = mbarWait<true>(qFull, 0, p.err, kDevErrFullWait);
             if (lane == 0 && par == 0) TC_STAMP(15);
             for (uint32_t j = par; ok && j < nTiles; j += 2u) {
                 const uint32_t s = j % NS, w = j % kWG, bb = (j / kWG) & 1u;
                 // the P.V product of the buffers' previous tile (j - 2 NWG) is done: its scores have been read and its P tile
                 // is free -- the softmax threads need not wait for that once more
                 if (j >= 2u * kWG)
-                    ok = mbarWait(&oFull[2u * w + bb], ((j - 2u * kWG) / (2u * kWG)) & 1u, p.err, kDevErrMmaWait);
-                ok = ok && mbarWait(&fullBar[s], (j / NS) & 1u, p.err, kDevErrFullWait);
+                    ok = mbarWait<true>(&oFull[2u * w + bb], ((j - 2u * kWG) / (2u * kWG)) & 1u, p.err, kDevErrMmaWait);
+                ok = ok && mbarWait<true>(&fullBar[s], (j / NS) & 1u, p.err, kDevErrFullWait);
                 if (lane == 0 && j < 8u) TC_STAMP(20 + j);
                 if (!ok) break;
                 tcFenceAfter();
@@ -443,10 +443,10 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
             for (uint32_t j = par; ok && j < nTiles; j += 2u) {
                 const uint32_t s = j % NS, w = j % kWG, bb = (j / kWG) & 1u;
                 // P of tile j published
-                ok = mbarWait(&pFull[2u * w + bb], (j / (2u * kWG)) & 1u, p.err, kDevErrMmaWait);
+                ok = mbarWait<true>(&pFull[2u * w + bb], (j / (2u * kWG)) & 1u, p.err, kDevErrMmaWait);
                 // and the fold warpgroup has read the O buffer's previous contents (tile j - 2 NWG)
                 if (ok && j >= 2u * kWG)
-                    ok = mbarWait(&oFree[2u * w + bb], ((j - 2u * kWG) / (2u * kWG)) & 1u, p.err, kDevErrMmaWait);
+                    ok = mbarWait<true>(&oFree[2u * w + bb], ((j - 2u * kWG) / (2u * kWG)) & 1u, p.err, kDevErrMmaWait);
                 if (!ok) break;
                 tcFenceAfter();
                 const uint64_t dV = tcDesc(smemAddr(smem + s * L::kStageBytes + L::kTileBytes), 16, 1024, 2);
@@ -487,7 +487,7 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
             for (uint32_t w = 0; w < kWG; ++w) {
                 const uint32_t j = j0 + w, bb = (j / kWG) & 1u, par = (j / (2u * kWG)) & 1u;
                 if (j >= nTiles) break;
-                ok = mbarWait(&oFull[2u * w + bb], par, p.err, kDevErrMmaWait);
+                ok = mbarWait<true>(&oFull[2u * w + bb], par, p.err, kDevErrMmaWait);
                 if (!ok) break;
                 tcFenceAfter();
                 uint32_t r[32];
@@ -616,7 +616,7 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         for (uint32_t j = w; j < nTiles; j += kWG) {
             const uint32_t s = j % NS, bb = (j / kWG) & 1u;
             // ---- this thread's token against the 8 heads ----
-            if (!mbarWait(&sFull[2u * w + bb], (j / (2u * kWG)) & 1u, p.err, kDevErrMmaWait)) {
+            if (!mbarWait<true>(&sFull[2u * w + bb], (j / (2u * kWG)) & 1u, p.err, kDevErrMmaWait)) {
                 ok = false;
                 break;
             }
