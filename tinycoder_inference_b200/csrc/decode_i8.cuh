@@ -56,8 +56,9 @@ struct I8Query {
 // q fragments for head column n = g of this kv head's group: power-of-two
 // normalised, split into fp16 hi + lo, laid out as the B operand whose k
 // slots follow the byte order ldmatrix hands out (dims 16c + 4t + {0..3}).
-template <int HD>
-__device__ __forceinline__ void i8LoadQuery(I8Query<HD> &f, const float *qp, bool valid, float invSqrt, uint32_t lane) {
+// behind() is called once the loads are on their way.
+template <int HD, typename Behind>
+__device__ __forceinline__ void i8LoadQuery(I8Query<HD> &f, const float *qp, bool valid, float invSqrt, uint32_t lane, Behind behind) {
     constexpr int NC = HD / 16;
     const uint32_t t = lane & 3u;
     float headScale, headOff;
@@ -65,9 +66,11 @@ __device__ __forceinline__ void i8LoadQuery(I8Query<HD> &f, const float *qp, boo
         float4 qv[NC];
         float amax = 0.0f;
 #pragma unroll
+        for (int c = 0; c < NC; ++c)
+            qv[c] = valid ? *reinterpret_cast<const float4 *>(qp + 16 * c + 4 * t) : make_float4(0.f, 0.f, 0.f, 0.f);
+        behind();
+#pragma unroll
         for (int c = 0; c < NC; ++c) {
-            qv[c] = valid ? __ldg(reinterpret_cast<const float4 *>(qp + 16 * c + 4 * t))
-                          : make_float4(0.f, 0.f, 0.f, 0.f);
             amax = fmaxf(amax, fmaxf(fmaxf(fabsf(qv[c].x), fabsf(qv[c].y)), fmaxf(fabsf(qv[c].z), fabsf(qv[c].w))));
         }
         amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
@@ -117,9 +120,9 @@ struct I8QueryShare {
     static constexpr int kBytes = kMax + NW * 128;
     static_assert(NC % NW == 0, "whole groups per warp");
 };
-template <int HD, int NW, int BAR = 0>
+template <int HD, int NW, int BAR, typename Behind>
 __device__ __forceinline__ void i8LoadQueryShared(I8Query<HD> &f, uint8_t *share, const float *qp, bool valid, float invSqrt,
-                                                  uint32_t warp, uint32_t lane) {
+                                                  uint32_t warp, uint32_t lane, Behind behind) {
     using S = I8QueryShare<HD, NW>;
     constexpr int NC = S::NC, N = NC / NW;
     const uint32_t t = lane & 3u;
@@ -130,9 +133,12 @@ __device__ __forceinline__ void i8LoadQueryShared(I8Query<HD> &f, uint8_t *share
 #pragma unroll
     for (int i = 0; i < N; ++i) {
         const int c = warp * N + i;
-        qv[i] = valid ? __ldg(reinterpret_cast<const float4 *>(qp + 16 * c + 4 * t)) : make_float4(0.f, 0.f, 0.f, 0.f);
-        amax = fmaxf(amax, fmaxf(fmaxf(fabsf(qv[i].x), fabsf(qv[i].y)), fmaxf(fabsf(qv[i].z), fabsf(qv[i].w))));
+        qv[i] = valid ? *reinterpret_cast<const float4 *>(qp + 16 * c + 4 * t) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
+    behind();
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+        amax = fmaxf(amax, fmaxf(fmaxf(fabsf(qv[i].x), fabsf(qv[i].y)), fmaxf(fabsf(qv[i].z), fabsf(qv[i].w))));
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
     top[warp * 32] = amax;

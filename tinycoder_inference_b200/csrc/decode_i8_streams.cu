@@ -123,17 +123,20 @@ decodeI8StreamsKernel(const __grid_constant__ DecodeI8Params p) {
             }
             cpAsyncCommit();
         };
-        requestK(warp);
-        requestV(warp);
-        // (the tile after that one is requested behind the row's store when it holds the row)
         NewQuantRow<HD, T> fresh;
         const size_t newSrc = static_cast<size_t>(kvHead) * HD;
-        if (hasRow) fresh.load(p.appendK + newSrc, p.appendV + newSrc, lane);
-        else requestK(warp + SW);
+        // (behind the loads of q, which would queue behind the tiles' otherwise; the tile after the first one is requested behind
+        // the row's store when it holds the row)
+        auto requestFirst = [&]() {
+            if (hasRow) fresh.load(p.appendK + newSrc, p.appendV + newSrc, lane);
+            requestK(warp);
+            requestV(warp);
+            if (!hasRow) requestK(warp + SW);
+        };
         I8Query<HD> qf;
         const float *qp = p.q + static_cast<size_t>(head0 + (g < nValid ? g : 0u)) * HD;
-        if constexpr (L::kShareQuery) i8LoadQueryShared<HD, SW, 1>(qf, smem + L::kQuery, qp, g < nValid, p.invSqrt, warp, lane);
-        else i8LoadQuery<HD>(qf, qp, g < nValid, p.invSqrt, lane);
+        if constexpr (L::kShareQuery) i8LoadQueryShared<HD, SW, 1>(qf, smem + L::kQuery, qp, g < nValid, p.invSqrt, warp, lane, requestFirst);
+        else i8LoadQuery<HD>(qf, qp, g < nValid, p.invSqrt, lane, requestFirst);
         if (hasRow) {
             const size_t dst = static_cast<size_t>(len - 1u) * p.nKV + kvHead;
             uint8_t *tile = intoTile ? slotK(iLast) : nullptr;

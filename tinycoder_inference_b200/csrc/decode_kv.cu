@@ -119,13 +119,17 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKvKernel(const __grid_cons
     };
     auto requestK = [&](uint32_t i) { request(i, false); };
     auto requestV = [&](uint32_t i) { request(i, true); };
-#pragma unroll
-    for (uint32_t i = 0; i < SLOTS; ++i) {
-        requestK(i);
-        requestV(i);
-    }
     NewRow<HD> fresh;
-    if (mine) fresh.load(p.tok, kvHead, len - 1u, lane);
+    // Behind the loads of q, which would queue behind the tiles' otherwise (28 / 4 / 128 at 2047 / 8191 rows 7.6 / 14.6 -> 7.45 / 13.8 us,
+    // 16 / 4 / 256 at 2047 rows, norm and gate included, 16.9 -> 16.0) -- but at head_dim 64, where they are few (5.6 -> 5.7).
+    auto requestFirst = [&]() {
+        if (mine) fresh.load(p.tok, kvHead, len - 1u, lane);
+#pragma unroll
+        for (uint32_t i = 0; i < SLOTS; ++i) {
+            requestK(i);
+            requestV(i);
+        }
+    };
 
     const uint32_t g = lane >> 2, t = lane & 3u;
     auto colValid = [&](uint32_t j) { return ROWS ? (b * 8u + j < p.qRows) : (p.colBase + j < p.group); };
@@ -142,6 +146,7 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKvKernel(const __grid_cons
     if constexpr (!kShareQuery) {
         const bool valid = colValid(g);
         const float *qp = p.q + colIndex(valid ? g : 0) * HD;
+        if constexpr (HD == 64) requestFirst();
         float4 qv[NB][2];
         // (plain loads: with a rotation q is written in place at the end of the launch)
 #pragma unroll
@@ -150,6 +155,7 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKvKernel(const __grid_cons
             for (int h = 0; h < 2; ++h)
                 qv[bx][h] = valid ? *reinterpret_cast<const float4 *>(qp + 32 * bx + 8 * t + 4 * h)
                                   : make_float4(0.f, 0.f, 0.f, 0.f);
+        if constexpr (HD != 64) requestFirst();
         if (!ROWS && p.tok.cosT != nullptr) {
             // NEOX rotation: the partner of dim d is d + HD / 2, NB / 2 boxes further on
             const size_t row = static_cast<size_t>(len - 1u) * (HD / 2);
@@ -186,21 +192,40 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKvKernel(const __grid_cons
     } else {
         // a column at a time each, four dims to a lane, the operands left where they are read
         uint4 *to = reinterpret_cast<uint4 *>(smem + L::kQuery);
-        for (uint32_t j = warp; j < 8; j += NW) {
-            const bool valid = colValid(j);
-            const float *qp = p.q + colIndex(valid ? j : 0) * HD;
+        constexpr int QC = (8 + NW - 1) / NW, QI = (HD + 127) / 128;  // columns of a warp, float4s of a lane
+        float4 qx[QC][QI], qy[QC][QI], qc[QI], qs[QI];
+        const bool rotate = p.tok.cosT != nullptr;
 #pragma unroll
-            for (uint32_t i = lane; i < HD / 4; i += 32) {
+        for (int k = 0; k < QC; ++k)
+#pragma unroll
+            for (int u = 0; u < QI; ++u) {
+                const uint32_t j = warp + k * NW, i = lane + 32u * u;
+                const bool upper = i >= HD / 8;
+                const float *qp = p.q + colIndex(j < 8 && colValid(j) ? j : 0) * HD;
                 // (plain loads: with a rotation q is written in place at the end of the launch)
-                float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (valid) x = *reinterpret_cast<const float4 *>(qp + 4 * i);
-                if (valid && p.tok.cosT != nullptr) {
+                qx[k][u] = qy[k][u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (j < 8 && colValid(j)) {
+                    qx[k][u] = *reinterpret_cast<const float4 *>(qp + 4 * i);
+                    if (rotate) qy[k][u] = *reinterpret_cast<const float4 *>(qp + 4 * (upper ? i - HD / 8 : i + HD / 8));
+                }
+                if (k == 0 && rotate) {
+                    const size_t at = static_cast<size_t>(len - 1u) * (HD / 2) + 4 * (upper ? i - HD / 8 : i);
+                    qc[u] = *reinterpret_cast<const float4 *>(p.tok.cosT + at), qs[u] = *reinterpret_cast<const float4 *>(p.tok.sinT + at);
+                }
+            }
+        requestFirst();
+#pragma unroll
+        for (int k = 0; k < QC; ++k) {
+            const uint32_t j = warp + k * NW;
+            if (j >= 8) break;
+#pragma unroll
+            for (int u = 0; u < QI; ++u) {
+                const uint32_t i = lane + 32u * u;
+                float4 x = qx[k][u];
+                if (rotate) {
                     // NEOX rotation: the partner of dim d is d + HD / 2
                     const bool upper = i >= HD / 8;
-                    const float4 y = *reinterpret_cast<const float4 *>(qp + 4 * (upper ? i - HD / 8 : i + HD / 8));
-                    const size_t at = static_cast<size_t>(len - 1u) * (HD / 2) + 4 * (upper ? i - HD / 8 : i);
-                    const float4 c = __ldg(reinterpret_cast<const float4 *>(p.tok.cosT + at));
-                    const float4 sn = __ldg(reinterpret_cast<const float4 *>(p.tok.sinT + at));
+                    const float4 y = qy[k][u], c = qc[u], sn = qs[u];
                     auto rot = [upper](float own, float other, float cc, float ss) {
                         return upper ? fmaf(other, ss, __fmul_rn(own, cc)) : fmaf(own, cc, -__fmul_rn(other, ss));
                     };

@@ -100,13 +100,17 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKv16Kernel(const __grid_co
     };
     auto requestK = [&](uint32_t i) { request(i, false); };
     auto requestV = [&](uint32_t i) { request(i, true); };
-#pragma unroll
-    for (uint32_t i = 0; i < SLOTS; ++i) {
-        requestK(i);
-        requestV(i);
-    }
     NewRow<HD> fresh;
-    if (mine) fresh.load(p.tok, kvHead, len - 1u, lane);
+    // (behind the loads of q, which would queue behind the tiles' otherwise: 28 / 4 / 128 at 8191 / 20000 rows 8.6 / 13.6 -> 7.5 / 13.0 us
+    // a layer, 8 / 4 / 64 at 2000 / 20000 rows 4.7 / 10.0 -> 4.5 / 9.1)
+    auto requestFirst = [&]() {
+        if (mine) fresh.load(p.tok, kvHead, len - 1u, lane);
+#pragma unroll
+        for (uint32_t i = 0; i < SLOTS; ++i) {
+            requestK(i);
+            requestV(i);
+        }
+    };
 
     const uint32_t g = lane >> 2, t = lane & 3u;
     auto colValid = [&](uint32_t j) { return ROWS ? (b * 8u + j < p.qRows) : (p.colBase + j < p.group); };
@@ -135,8 +139,12 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKv16Kernel(const __grid_co
             for (int h = 0; h < 2; ++h) {
                 qv[s][h] = valid ? *reinterpret_cast<const float2 *>(qp + 16 * s + 8 * h + 2 * t)
                                  : make_float2(0.f, 0.f);
-                amax = fmaxf(amax, fmaxf(fabsf(qv[s][h].x), fabsf(qv[s][h].y)));
             }
+        requestFirst();
+#pragma unroll
+        for (int s = 0; s < NS; ++s)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) amax = fmaxf(amax, fmaxf(fabsf(qv[s][h].x), fabsf(qv[s][h].y)));
         amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
         amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
         const int e = exponent(amax);
@@ -162,21 +170,25 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKv16Kernel(const __grid_co
         // us, 14 / 2 / 64 at 2000 rows 4.7 -> 4.5; 8 / 4 / 64 at 20 rows 3.3 -> 3.4.)
         uint32_t *frag = reinterpret_cast<uint32_t *>(smem + L::kQuery);  // [step][lane]: hi 0, hi 1, lo 0, lo 1
         float *scale = reinterpret_cast<float *>(smem + L::kQuery + HD * 32);
-        for (uint32_t j = warp; j < 8; j += NW) {
-            const bool valid = colValid(j) && 2 * lane < HD / 2;
+        static_assert(ROWS || NW == 8, "a column per warp");
+        {
+            const uint32_t j = warp;
+            const bool valid = colValid(j) && 2 * lane < HD / 2, rotate = valid && p.tok.cosT != nullptr;
             // (plain loads: with a rotation q is written in place at the end of the launch)
-            float2 x = make_float2(0.f, 0.f), y = x;
+            float2 x = make_float2(0.f, 0.f), y = x, c = x, sn = x;
             if (valid) {
                 const float *qp = p.q + colIndex(j) * HD + 2 * lane;
                 x = *reinterpret_cast<const float2 *>(qp), y = *reinterpret_cast<const float2 *>(qp + HD / 2);
-                if (p.tok.cosT != nullptr) {
-                    const size_t at = static_cast<size_t>(len - 1u) * (HD / 2) + 2 * lane;
-                    const float2 c = __ldg(reinterpret_cast<const float2 *>(p.tok.cosT + at));
-                    const float2 sn = __ldg(reinterpret_cast<const float2 *>(p.tok.sinT + at));
-                    const float2 x0 = x, x1 = y;
-                    x = make_float2(fmaf(x0.x, c.x, -__fmul_rn(x1.x, sn.x)), fmaf(x0.y, c.y, -__fmul_rn(x1.y, sn.y)));
-                    y = make_float2(fmaf(x0.x, sn.x, __fmul_rn(x1.x, c.x)), fmaf(x0.y, sn.y, __fmul_rn(x1.y, c.y)));
-                }
+            }
+            if (rotate) {
+                const size_t at = static_cast<size_t>(len - 1u) * (HD / 2) + 2 * lane;
+                c = *reinterpret_cast<const float2 *>(p.tok.cosT + at), sn = *reinterpret_cast<const float2 *>(p.tok.sinT + at);
+            }
+            requestFirst();
+            if (rotate) {
+                const float2 x0 = x, x1 = y;
+                x = make_float2(fmaf(x0.x, c.x, -__fmul_rn(x1.x, sn.x)), fmaf(x0.y, c.y, -__fmul_rn(x1.y, sn.y)));
+                y = make_float2(fmaf(x0.x, sn.x, __fmul_rn(x1.x, c.x)), fmaf(x0.y, sn.y, __fmul_rn(x1.y, c.y)));
             }
             const float top = fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(y.x), fabsf(y.y)));
             // (maxima of non-negative floats, by their bits)

@@ -130,19 +130,15 @@ __global__ void __launch_bounds__(kExactWarps * 32, 1) prefillExactKernel(const 
     const uint32_t len = static_cast<uint32_t>(wanted < p.totalRows ? wanted : p.totalRows);  // (a device position past the store)
     const uint32_t kvHead = head / p.group;
 
-    // q: hi and lo planes
-    for (uint32_t i = threadIdx.x; i < S::kRows * (HD / 4); i += kThreads) {
-        const uint32_t r = i / (HD / 4), c = (i % (HD / 4)) * 4;
-        const float4 x = r < rows ? __ldg(reinterpret_cast<const float4 *>(
-                                            p.q + (static_cast<size_t>(row0 + r) * p.nHeads + head) * HD + c))
-                                  : make_float4(0.f, 0.f, 0.f, 0.f);
-        float4 h, l;
-        splitTf32(x.x, h.x, l.x);
-        splitTf32(x.y, h.y, l.y);
-        splitTf32(x.z, h.z, l.z);
-        splitTf32(x.w, h.w, l.w);
-        *reinterpret_cast<float4 *>(sQ + r * LD + c) = h;
-        *reinterpret_cast<float4 *>(sQ + (S::kRows + r) * LD + c) = l;
+    // (the loads of q first, those of the first stage behind them, then q's planes: one wait for both)
+    constexpr uint32_t kQUnits = S::kRows * (HD / 4), kQPer = kQUnits / kThreads;
+    static_assert(kQUnits % kThreads == 0, "even shares");
+    float4 qv[kQPer];
+#pragma unroll
+    for (uint32_t i = 0; i < kQPer; ++i) {
+        const uint32_t idx = threadIdx.x + i * kThreads, r = idx / (HD / 4), c = (idx % (HD / 4)) * 4;
+        qv[i] = r < rows ? __ldg(reinterpret_cast<const float4 *>(p.q + (static_cast<size_t>(row0 + r) * p.nHeads + head) * HD + c))
+                         : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 
     // A stage's rows pass through registers: requested while the stage before it is worked on, split into the planes
@@ -174,6 +170,20 @@ __global__ void __launch_bounds__(kExactWarps * 32, 1) prefillExactKernel(const 
         *reinterpret_cast<float4 *>(plane + (S::kStage + r) * LD + c) = l;
     };
 
+    request(0);
+    // q: hi and lo planes
+#pragma unroll
+    for (uint32_t i = 0; i < kQPer; ++i) {
+        const uint32_t idx = threadIdx.x + i * kThreads, r = idx / (HD / 4), c = (idx % (HD / 4)) * 4;
+        float4 h, l;
+        splitTf32(qv[i].x, h.x, l.x);
+        splitTf32(qv[i].y, h.y, l.y);
+        splitTf32(qv[i].z, h.z, l.z);
+        splitTf32(qv[i].w, h.w, l.w);
+        *reinterpret_cast<float4 *>(sQ + r * LD + c) = h;
+        *reinterpret_cast<float4 *>(sQ + (S::kRows + r) * LD + c) = l;
+    }
+
     float o[HD / 8][4];
 #pragma unroll
     for (int i = 0; i < HD / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
@@ -189,7 +199,6 @@ __global__ void __launch_bounds__(kExactWarps * 32, 1) prefillExactKernel(const 
     const uint32_t bAddr = smemAddr(sK + bRow * LD + ((lane >> 3) & 1u) * 4u);
 
     const uint32_t nStages = (len + S::kStage - 1) / S::kStage;
-    request(0);
     for (uint32_t st = 0; st < nStages; ++st) {
         __syncthreads();  // the planes are free (and, the first time, q's are complete)
 #pragma unroll
@@ -366,16 +375,23 @@ prefillExactHalfKernel(const __grid_constant__ PrefillExactParams p) {
         cpAsyncCommit();
     };
     const uint32_t nStages = (len + S::kStage - 1) / S::kStage;
-    request(0);
-    if (nStages > 1) request(1);
-    else cpAsyncCommit();
-
-    {   // q: HD / 4 lanes per row
-        constexpr uint32_t W = HD / 4, R = 32 / W;
-        for (uint32_t r = warp * R + lane / W; r < S::kRows; r += kExactWarps * R) {
-            const uint32_t c = lane % W * 4;
-            const float4 x = r < rows ? *reinterpret_cast<const float4 *>(p.q + (static_cast<size_t>(row0 + r) * p.nHeads + head) * HD + c)
-                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+    {   // q: HD / 4 lanes per row; its loads go ahead of the first stages' copies, or they queue behind them
+        constexpr uint32_t W = HD / 4, R = 32 / W, N = S::kRows / (kExactWarps * R);
+        static_assert(S::kRows % (kExactWarps * R) == 0, "even shares");
+        float4 qv[N];
+#pragma unroll
+        for (uint32_t i = 0; i < N; ++i) {
+            const uint32_t r = (i * kExactWarps + warp) * R + lane / W, c = lane % W * 4;
+            qv[i] = r < rows ? *reinterpret_cast<const float4 *>(p.q + (static_cast<size_t>(row0 + r) * p.nHeads + head) * HD + c)
+                             : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        request(0);
+        if (nStages > 1) request(1);
+        else cpAsyncCommit();
+#pragma unroll
+        for (uint32_t i = 0; i < N; ++i) {
+            const uint32_t r = (i * kExactWarps + warp) * R + lane / W, c = lane % W * 4;
+            const float4 x = qv[i];
             float amax = fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w)));
 #pragma unroll
             for (int o = W / 2; o; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
