@@ -72,6 +72,7 @@ struct PrefillRowsParams {
     PrefillNewRows nr;
     PrefillMirror mir;
     uint32_t seqLen, cachePos, nHeads, nKV;
+    uint32_t qBlocks;      // blocks that work on q, the others on K and V (0: every block does both, one after the other)
     unsigned int *err, *workCounter;
 };
 
@@ -81,8 +82,9 @@ __global__ void __launch_bounds__(256) prefillRowsKernel(const __grid_constant__
     gridDepLaunch();  // the attention launch may set itself up while this one drains (it waits before it lets anything else in)
     // the attention launch that follows in the stream hands out its work items through this counter
     if (blockIdx.x == 0 && threadIdx.x == 0) *p.workCounter = 0u;
-    const size_t tid = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
+    const bool both = p.qBlocks == 0u, forQ = both || blockIdx.x < p.qBlocks;
+    const size_t tid = static_cast<size_t>(blockIdx.x - (forQ ? 0u : p.qBlocks)) * blockDim.x + threadIdx.x;
+    const size_t stride = static_cast<size_t>(both ? gridDim.x : forQ ? p.qBlocks : gridDim.x - p.qBlocks) * blockDim.x;
     constexpr uint32_t half = HD / 2, perRow = half / 4, nvec = HD / 4;
     constexpr int MAXV = HD > 128 ? 2 : 1;  // float4 per lane and K/V row
     auto half4 = [](const float4 &x) { return make_uint2(packHalf2(x.x, x.y), packHalf2(x.z, x.w)); };
@@ -97,7 +99,7 @@ __global__ void __launch_bounds__(256) prefillRowsKernel(const __grid_constant__
         rot(a.z, b.z, c.z, s.z);
         rot(a.w, b.w, c.w, s.w);
     };
-    const size_t qUnits = static_cast<size_t>(p.seqLen) * p.nHeads * perRow;
+    const size_t qUnits = forQ ? static_cast<size_t>(p.seqLen) * p.nHeads * perRow : 0;
     constexpr int N = 4;  // units of a thread in flight
     for (size_t i0 = tid; i0 < qUnits; i0 += N * stride) {
         float4 x[N], y[N];
@@ -125,6 +127,7 @@ __global__ void __launch_bounds__(256) prefillRowsKernel(const __grid_constant__
             p.q16[at + perRow] = half4(y[u]);
         }
     }
+    if (forQ && !both) return;
     const uint32_t lane = threadIdx.x & 31u;
     const size_t newFrom = static_cast<size_t>(p.cachePos) * p.nKV;            // first (row, kv head) of the call's rows
     const size_t end = newFrom + static_cast<size_t>(p.seqLen) * p.nKV;
@@ -1143,8 +1146,14 @@ int prefillF16(float *q, const PrefillKvStore &src, float *out, void *scratch, s
         rp.seqLen = seqLen, rp.cachePos = cachePos, rp.nHeads = nHeads, rp.nKV = nKV;
         rp.err = err, rp.workCounter = workCounter;
         const size_t rowHeads = static_cast<size_t>(src.kind == 1 ? (nr.k != nullptr ? seqLen : 0) : kvRows) * nKV;
-        const size_t threads = std::max(qElems / 8, rowHeads * 32);
-        const uint32_t blocks = static_cast<uint32_t>(std::min<size_t>((threads + 255) / 256, static_cast<size_t>(sms) * 16));
+        // A short call is a chain of latencies: q has blocks of its own, so that K and V do not wait behind it.  From some four blocks per
+        // SM on every block does both (8 / 2 / 128: 16 rows 7.3 -> 6.9 us with the attention launch, 512 behind 512 (512 blocks) 16.4 ->
+        // 16.0, 512 behind 1536 (768) 17.7 -> 18.4; 14 / 2 / 64 over fp16, 512 behind 1536 (352) 17.5 -> 16.8; 28 / 4 / 128, 512 rows
+        // (1408) 14.0 -> 14.6).
+        const size_t most = static_cast<size_t>(sms) * 16, qBlocks = (qElems / 8 + 255) / 256, kvBlocks = (rowHeads * 32 + 255) / 256;
+        const bool apart = kvBlocks != 0 && qBlocks + kvBlocks <= static_cast<size_t>(sms) * 4;
+        rp.qBlocks = apart ? static_cast<uint32_t>(qBlocks) : 0u;
+        const uint32_t blocks = static_cast<uint32_t>(std::min(apart ? qBlocks + kvBlocks : std::max(qBlocks, kvBlocks), most));
         const int rc = launchDependent(hd == 64 ? prefillRowsKernel<64> : (hd == 128 ? prefillRowsKernel<128> : prefillRowsKernel<256>), dim3(blocks), 256, 0, st, 1, rp);
         if (rc != TC_OK) return rc;
     }
