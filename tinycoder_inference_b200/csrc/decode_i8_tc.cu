@@ -165,10 +165,10 @@ __device__ __forceinline__ bool barOr(uint32_t id, uint32_t threads, bool pred) 
             : "memory");
     return r != 0;
 }
-// maximum over the warp (NaN is ignored, as in fmaxf)
+// maximum over the warp (NaN is ignored, as in fmaxf); volatile, or it may end up where only lane 0 uses the result
 __device__ __forceinline__ float warpMax(float x) {
     float r;
-    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
     return r;
 }
 __device__ __forceinline__ float i2f(uint32_t x) { return __int2float_rn(static_cast<int>(x)); }
