@@ -44,3 +44,43 @@ def test_tile_edges(S, pos, nH, nKV, hd):
                                              (300, 601, 16, 2, 256)])
 def test_items_shared_by_a_cluster(S, pos, nH, nKV, hd):
     _check(S, pos, nH, nKV, hd)
+
+
+# The launch in front of the attention: q and K / V in blocks of their own (up to two of each per SM, and no more for the
+# rows that the store already has than for q) or one after the other in every block; the sizes lie on both sides of each of the two lines on 148 SMs.
+@pytest.mark.parametrize("mode,nH,nKV,hd,before,rows", [("f32", 28, 4, 128, 0, 169), ("f32", 28, 4, 128, 0, 170), ("f32+i8", 28, 4, 128, 0, 169),
+                                                        ("i8", 28, 4, 128, 3, 170), ("f32", 8, 2, 128, 200, 100), ("i8", 8, 2, 128, 204, 100),
+                                                        ("f16", 14, 2, 64, 5, 676), ("f16", 14, 2, 64, 0, 679), ("f32", 4, 4, 256, 76, 75),
+                                                        ("f32", 4, 4, 256, 80, 75)])
+def test_prompt_rows_in_either_kind_of_launch(mode, nH, nKV, hd, before, rows):
+    n, inv = before + rows, 1.0 / math.sqrt(hd)
+    r = np.random.default_rng(n + hd)
+    q, k, v = (r.standard_normal((n, h, hd), dtype=np.float32) for h in (nH, nKV, nKV))
+    rope = oracle.rope_tables(n, hd, 1e6) if mode in ("f32", "f16") else None
+    s = ops.KvSession(nH, nKV, hd, n, 1, mode=mode, rope=None if rope is None else tuple(dev(t) for t in rope), prefill_scratch_rows=n)
+    for a, b in ((0, before), (before, n)):
+        if a == b:
+            continue
+        dq, out = dev(q[a:b]), torch.full((b - a, nH, hd), float("nan"), device="cuda")
+        s.attend(0, dq, dev(k[a:b]), dev(v[a:b]), out, a)
+    torch.cuda.synchronize()
+    assert ops.device_status() == 0
+    K, V, q = np.zeros_like(k), np.zeros_like(v), q[before:]
+    if rope is not None:
+        q = oracle.rope_q(q, *rope, rows, nH, hd, before)
+        oracle.kv_append(k, v, K, V, n, nKV, hd, 0, ropePos=0, cosT=rope[0], sinT=rope[1])
+    else:
+        K, V = k, v
+    assert np.array_equal(host(dq), q)
+    if mode != "i8":
+        dt = np.float16 if mode == "f16" else np.float32
+        assert np.array_equal(host(s.kvK[0]), K.astype(dt)) and np.array_equal(host(s.kvV[0]), V.astype(dt))
+    if "i8" in mode:
+        quant = oracle.quant_kv8(K, V, nKV, hd)
+        for have, want in zip((s.k8, s.v8, s.ks, s.vs), quant):
+            assert np.array_equal(host(have[0, :n]), want)
+    if mode == "i8":    # the rows as the store holds them
+        K, V = (x8.astype(np.float32) * sc[:, :, None] for x8, sc in ((quant[0], quant[2]), (quant[1], quant[3])))
+    q, K, V = (x.astype(np.float16) for x in (q, K, V))
+    want = oracle.attention_f64(q.astype(np.float32), K, V, None, None, rows, nH, nKV, hd, before, inv)
+    assert_close(host(out), want, rtol=0.0, atol=4.5e-3, what=f"{rows} rows behind {before}")

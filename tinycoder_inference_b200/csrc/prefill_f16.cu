@@ -72,19 +72,20 @@ struct PrefillRowsParams {
     PrefillNewRows nr;
     PrefillMirror mir;
     uint32_t seqLen, cachePos, nHeads, nKV;
-    uint32_t qBlocks;      // blocks that work on q, the others on K and V (0: every block does both, one after the other)
+    uint32_t qBlocks;      // APART: the first blocks, which work on q
     unsigned int *err, *workCounter;
 };
 
-template <int HD>
+// APART: the first qBlocks blocks work on q, the others on K and V; else every block does both, one after the other.
+template <int HD, bool APART>
 __global__ void __launch_bounds__(256) prefillRowsKernel(const __grid_constant__ PrefillRowsParams p) {
     gridDepWait();
     gridDepLaunch();  // the attention launch may set itself up while this one drains (it waits before it lets anything else in)
     // the attention launch that follows in the stream hands out its work items through this counter
     if (blockIdx.x == 0 && threadIdx.x == 0) *p.workCounter = 0u;
-    const bool both = p.qBlocks == 0u, forQ = both || blockIdx.x < p.qBlocks;
-    const size_t tid = static_cast<size_t>(blockIdx.x - (forQ ? 0u : p.qBlocks)) * blockDim.x + threadIdx.x;
-    const size_t stride = static_cast<size_t>(both ? gridDim.x : forQ ? p.qBlocks : gridDim.x - p.qBlocks) * blockDim.x;
+    const bool forQ = !APART || blockIdx.x < p.qBlocks;
+    const size_t tid = static_cast<size_t>(forQ ? blockIdx.x : blockIdx.x - p.qBlocks) * blockDim.x + threadIdx.x;
+    const size_t stride = static_cast<size_t>(!APART ? gridDim.x : forQ ? p.qBlocks : gridDim.x - p.qBlocks) * blockDim.x;
     constexpr uint32_t half = HD / 2, perRow = half / 4, nvec = HD / 4;
     constexpr int MAXV = HD > 128 ? 2 : 1;  // float4 per lane and K/V row
     auto half4 = [](const float4 &x) { return make_uint2(packHalf2(x.x, x.y), packHalf2(x.z, x.w)); };
@@ -127,7 +128,7 @@ __global__ void __launch_bounds__(256) prefillRowsKernel(const __grid_constant__
             p.q16[at + perRow] = half4(y[u]);
         }
     }
-    if (forQ && !both) return;
+    if (APART && forQ) return;
     const uint32_t lane = threadIdx.x & 31u;
     const size_t newFrom = static_cast<size_t>(p.cachePos) * p.nKV;            // first (row, kv head) of the call's rows
     const size_t end = newFrom + static_cast<size_t>(p.seqLen) * p.nKV;
@@ -1146,15 +1147,21 @@ int prefillF16(float *q, const PrefillKvStore &src, float *out, void *scratch, s
         rp.seqLen = seqLen, rp.cachePos = cachePos, rp.nHeads = nHeads, rp.nKV = nKV;
         rp.err = err, rp.workCounter = workCounter;
         const size_t rowHeads = static_cast<size_t>(src.kind == 1 ? (nr.k != nullptr ? seqLen : 0) : kvRows) * nKV;
-        // A short call is a chain of latencies: q has blocks of its own, so that K and V do not wait behind it.  From some four blocks per
-        // SM on every block does both (8 / 2 / 128: 16 rows 7.3 -> 6.9 us with the attention launch, 512 behind 512 (512 blocks) 16.4 ->
-        // 16.0, 512 behind 1536 (768) 17.7 -> 18.4; 14 / 2 / 64 over fp16, 512 behind 1536 (352) 17.5 -> 16.8; 28 / 4 / 128, 512 rows
-        // (1408) 14.0 -> 14.6).
+        // A short call is a chain of latencies: q has blocks of its own, so that K and V do not wait behind it -- while an SM holds
+        // two blocks of each kind (four are resident), and the rows that the store already has are no more than q's.  With the
+        // attention launch, every block does both -> apart: 8 / 2 / 128 int8, 60 rows 7.2 -> 6.85 us, 512 behind 512 (256 and 256
+        // blocks) 15.5 -> 14.95; 14 / 2 / 64 fp16, 512 behind 512 12.8 -> 12.1.  Beyond the line: 12 / 2 / 128, 512 rows (384 and 128)
+        // 12.1 -> 12.5; 28 / 4 / 128, 200 rows (350 and 100) 9.6 -> 9.85; 8 / 2 / 128, 60 behind 500 (30 and 140) 10.7 -> 11.1.  (Two
+        // instantiations: with a choice at run time the calls that do both lost 0.1 - 0.2 us.)
         const size_t most = static_cast<size_t>(sms) * 16, qBlocks = (qElems / 8 + 255) / 256, kvBlocks = (rowHeads * 32 + 255) / 256;
-        const bool apart = kvBlocks != 0 && qBlocks + kvBlocks <= static_cast<size_t>(sms) * 4;
+        const size_t oldBlocks = ((rowHeads - (nr.k != nullptr ? static_cast<size_t>(seqLen) * nKV : 0)) * 32 + 255) / 256;
+        const bool apart = kvBlocks != 0 && std::max(qBlocks, kvBlocks) <= static_cast<size_t>(sms) * 2 && oldBlocks <= qBlocks;
         rp.qBlocks = apart ? static_cast<uint32_t>(qBlocks) : 0u;
         const uint32_t blocks = static_cast<uint32_t>(std::min(apart ? qBlocks + kvBlocks : std::max(qBlocks, kvBlocks), most));
-        const int rc = launchDependent(hd == 64 ? prefillRowsKernel<64> : (hd == 128 ? prefillRowsKernel<128> : prefillRowsKernel<256>), dim3(blocks), 256, 0, st, 1, rp);
+        static constexpr decltype(&prefillRowsKernel<64, false>) kerns[3][2] = {{prefillRowsKernel<64, false>, prefillRowsKernel<64, true>},
+                                                                               {prefillRowsKernel<128, false>, prefillRowsKernel<128, true>},
+                                                                               {prefillRowsKernel<256, false>, prefillRowsKernel<256, true>}};
+        const int rc = launchDependent(kerns[hd == 64 ? 0 : hd == 128 ? 1 : 2][apart ? 1 : 0], dim3(blocks), 256, 0, st, 1, rp);
         if (rc != TC_OK) return rc;
     }
     CUtensorMap tmQ, tmK, tmV;
