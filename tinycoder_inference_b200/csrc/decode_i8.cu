@@ -130,10 +130,13 @@ decodeI8Kernel(const __grid_constant__ DecodeI8Params p) {
     NewQuantRow<HD, T> fresh;
     const size_t newSrc = (static_cast<size_t>(b) * p.nKV + kvHead) * HD;
     // (behind the loads of q: queued behind 128 KB of tiles of the SM, q came 3.7 us after the dependency:
-    // 16 / 2 / 256, norm and gate included, 16383 rows 16.1 -> 15.1 us a layer, 8 / 4 / 256 at 8000 rows 14.8 -> 13.5)
+    // 16 / 2 / 256, norm and gate included, 16383 rows 16.1 -> 15.1 us a layer, 8 / 4 / 256 at 8000 rows 14.8 -> 13.5.  Causal rows, tiles
+    // first -> this: 28 / 4 / 128, 64 rows 7.6 -> 6.55 us, 512 behind 2000 199 -> 188; 16 / 2 / 256, 64 rows 6.15 -> 4.9, 512 behind 2000
+    // 199 -> 194.  There the loop is not unrolled and q goes through the read-only path: without that, 2 rows behind 16000
+    // took 91.4 and 177.6 us, with the tiles first 90.8 and 176.2, like this 88.4 and 175.5.)
     auto requestFirst = [&]() {
         if (mine) fresh.load(p.appendK + newSrc, p.appendV + newSrc, lane);
-#pragma unroll
+#pragma unroll(ROWS ? 1 : NS)
         for (uint32_t i = 0; i < NS; ++i) {
             requestK(i);
             requestV(i);

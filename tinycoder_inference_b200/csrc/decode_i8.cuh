@@ -67,7 +67,7 @@ __device__ __forceinline__ void i8LoadQuery(I8Query<HD> &f, const float *qp, boo
         float amax = 0.0f;
 #pragma unroll
         for (int c = 0; c < NC; ++c)
-            qv[c] = valid ? *reinterpret_cast<const float4 *>(qp + 16 * c + 4 * t) : make_float4(0.f, 0.f, 0.f, 0.f);
+            qv[c] = valid ? __ldg(reinterpret_cast<const float4 *>(qp + 16 * c + 4 * t)) : make_float4(0.f, 0.f, 0.f, 0.f);
         behind();
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
