@@ -2,6 +2,7 @@
 driven the way GPUModel drives its attention block -- prefill, decode, a second session after
 clear, chunked prefill, the window guard -- in all KV modes, against the oracle run on the
 full history."""
+import ctypes as C
 import math
 
 import numpy as np
@@ -315,3 +316,26 @@ def test_clear_zeroes_the_whole_store(mode, nH, nKV, hd, window, slots):
     s.kvV.fill_(float("nan"))
     s.clear()
     assert int(torch.count_nonzero(s.kvK)) == 0 and int(torch.count_nonzero(s.kvV)) == 0
+
+
+# one launch for both stores, or a memset each: stores of no whole 16 bytes' address, memory that is not the current device's own
+@pytest.mark.parametrize("where,half,window,slots", [("device", 0, 1, 1), ("device", 1, 37, 3), ("odd address", 0, 37, 2), ("odd address", 1, 1, 1), ("host", 0, 5, 2)])
+def test_clear_writes_the_store_and_nothing_beside_it(where, half, window, slots):
+    nKV, hd, guard = 1, 64, 4096
+    n = ops.kv_pool_geometry(window, slots, 1, nKV, nKV, hd, bool(half)).kvLayerStride * slots
+    assert n == window * slots * nKV * hd * (2 if half else 4)
+    off = guard + (8 if where == "odd address" else 0)
+    kw = dict(pin_memory=True) if where == "host" else dict(device="cuda")
+    bufs = [torch.full((n + 2 * guard + 16,), 0xa5, dtype=torch.uint8, **kw) for _ in range(2)]
+    cfg = capi.KvSessionConfig()
+    cfg.nHeads = cfg.nKV = nKV
+    cfg.hd, cfg.maxSeqLen, cfg.slots, cfg.kvHalf, cfg.numChunks = hd, window, slots, half, 1
+    cfg.kvK, cfg.kvV = (b.data_ptr() + off for b in bufs)
+    h = C.c_void_p()
+    assert capi.lib.tc_kv_session_create(C.byref(cfg), C.byref(h)) == capi.TC_OK
+    torch.cuda.synchronize()
+    assert capi.lib.tc_kv_session_clear(h, C.c_void_p(torch.cuda.current_stream().cuda_stream)) == capi.TC_OK
+    capi.lib.tc_kv_session_destroy(h)
+    for b in bufs:
+        assert int(torch.count_nonzero(b[off:off + n])) == 0
+        assert bool((b[:off] == 0xa5).all()) and bool((b[off + n:] == 0xa5).all())
