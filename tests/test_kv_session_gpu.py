@@ -318,8 +318,10 @@ def test_clear_zeroes_the_whole_store(mode, nH, nKV, hd, window, slots):
     assert int(torch.count_nonzero(s.kvK)) == 0 and int(torch.count_nonzero(s.kvV)) == 0
 
 
-# one launch for both stores, or a memset each: stores of no whole 16 bytes' address, memory that is not the current device's own
-@pytest.mark.parametrize("where,half,window,slots", [("device", 0, 1, 1), ("device", 1, 37, 3), ("odd address", 0, 37, 2), ("odd address", 1, 1, 1), ("host", 0, 5, 2)])
+# one launch for both stores, or a memset each: stores of no whole 16 bytes' address, longer ones than 64 MB (the sizes lie on both
+# sides), memory that is not the current device's own
+@pytest.mark.parametrize("where,half,window,slots", [("device", 0, 1, 1), ("device", 1, 37, 3), ("device", 0, 262144, 1), ("device", 0, 262145, 1),
+                                                     ("odd address", 0, 37, 2), ("odd address", 1, 1, 1), ("host", 0, 5, 2)])
 def test_clear_writes_the_store_and_nothing_beside_it(where, half, window, slots):
     nKV, hd, guard = 1, 64, 4096
     n = ops.kv_pool_geometry(window, slots, 1, nKV, nKV, hd, bool(half)).kvLayerStride * slots

@@ -231,7 +231,10 @@ static int launchAppend(float *q, const float *kSrc, const float *vSrc, void *kD
 // K and V store of a session zeroed
 // ---------------------------------------------------------------------------
 // One launch for both: what bounds a short call is the host's way to the GPU and back (the caller synchronises), and a memset
-// each puts two launches into it.  clear() alone, memsets -> launch: 1 MB of K 12.2 -> 9.4 us, 16 MB 16.9 -> 14.4, 64 MB 31.1 -> 30.7.
+// each puts two launches into it.  clear() alone, memsets -> launch: 1 MB of K 12.2 -> 9.4 us, 16 MB 16.9 -> 14.4, 48 MB 26.0 -> 24.9,
+// 64 MB 31.1 -> 30.7.  Longer ones are bound by HBM, which the memsets write at 7.2 TB/s and this loop at 6: 96 MB 40.8 -> 42.0,
+// 256 MB 86 -> 97, 2 GB 596 -> 718.
+constexpr size_t kClearLaunchBytes = size_t(64) << 20;  // of K, at most
 __global__ void __launch_bounds__(256) kvClearKernel(uint4 *k, uint4 *v, size_t n) {
     gridDepWait();
     const size_t step = static_cast<size_t>(gridDim.x) * blockDim.x;
@@ -251,7 +254,7 @@ static bool onCurrentDevice(const void *k, const void *v) {
 }
 int kvClear(void *k, void *v, size_t bytes, cudaStream_t st) {
     const size_t n = bytes / 16;
-    if (n != 0 && ((reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | bytes) & 15u) == 0 &&
+    if (n != 0 && bytes <= kClearLaunchBytes && ((reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | bytes) & 15u) == 0 &&
         onCurrentDevice(k, v)) {
         const size_t blocks = (n + 255) / 256, most = static_cast<size_t>(numSMs()) * 8;
         if (launchDependent(kvClearKernel, dim3(static_cast<uint32_t>(blocks < most ? blocks : most)), 256, 0, st, 1,
