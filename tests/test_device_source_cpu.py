@@ -22,3 +22,21 @@ def test_asm_that_synchronises_is_volatile():
                 if not m.group(1):
                     bad.append((name, m.group(2).strip()))
     assert seen > 30 and bad == []
+
+
+def test_tensor_memory_is_given_back_behind_the_warps_that_issue():
+    """A wait that ran out in some warps must not free tensor memory that others still issue products into: in front of each
+    deallocation stands a barrier of the block, or the one that the issuing warps arrive at when they are through."""
+    found = 0
+    for name in SOURCES:
+        lines = _code(name).splitlines()
+        for i, line in enumerate(lines):
+            if "tmemDealloc(" not in line or "__device__" in line:
+                continue
+            found += 1
+            before = "\n".join(x for x in lines[:i] if x.strip()).splitlines()[-5:]
+            barrier = re.search(r"__syncthreads\(\)|namedBarSync\((kIssuedBar), ", "\n".join(before))
+            assert barrier, (name, i + 1)
+            if barrier.group(1):
+                assert "namedBarArrive(kIssuedBar, " in "\n".join(lines[:i]), (name, i + 1)
+    assert found >= 2

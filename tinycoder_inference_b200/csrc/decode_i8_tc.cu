@@ -187,7 +187,7 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
                  const __grid_constant__ CUtensorMap tmKn, const __grid_constant__ CUtensorMap tmVn,
                  const DecodeTcParams p) {
     using L = DecodeTcSmem<NWG, NS>;
-    constexpr uint32_t kWG = NWG, kSoftThreads = 128u * NWG, kAllBar = NWG + 1u, kEndBar = NWG + 2u;
+    constexpr uint32_t kWG = NWG, kSoftThreads = 128u * NWG, kAllBar = NWG + 1u, kEndBar = NWG + 2u, kIssuedBar = NWG + 3u;
     constexpr uint32_t kFoldWarp0 = 4u * NWG, kProducerWarp = 4u * NWG + 4u, kMmaWarp0 = 4u * NWG + 5u;
     constexpr uint32_t kEndThreads = 32u * kProducerWarp;   // softmax + fold threads
     constexpr uint32_t T = kTcTile;
@@ -465,6 +465,8 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
                 if (lane == 0) TC_STAMP(16);
             }
         }
+        // this warp issues nothing into tensor memory any more, whatever waits ran out: its owner may give it back
+        namedBarArrive(kIssuedBar, 160);
     } else if (warp >= kFoldWarp0) {
         // ------------------------------ fold warpgroup ------------------------------
         // thread = one head dimension: takes every tile's integer P.V out of TMEM in tile order and
@@ -825,9 +827,10 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         }
     }
     if (threadIdx.x == 0) TC_STAMP(12);
-    // (every product was waited for by the fold warps, every read of tensor memory lies in front of the barrier that they
-    // and the softmax warps met at)
+    // (every read of tensor memory lies in front of the barrier that the fold and the softmax warps met at, and the issuing
+    // warps are through -- long ago, and with every product waited for by the fold warps, unless a wait ran out)
     if (warp == 0) {
+        namedBarSync(kIssuedBar, 160);
         tcFenceAfter();
         tmemDealloc(tmemBase, L::kTmemCols);
     }

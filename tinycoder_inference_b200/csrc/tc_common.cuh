@@ -288,6 +288,9 @@ __device__ __forceinline__ float fastExp2(float x) {
 __device__ __forceinline__ void namedBarSync(uint32_t id, uint32_t threads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
+__device__ __forceinline__ void namedBarArrive(uint32_t id, uint32_t threads) {
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
 
 #endif  // __CUDACC__
 
