@@ -1072,16 +1072,24 @@ template <int HD>
 static int launchPrefill(const PrefillF16Params &prm, uint32_t tiles, const CUtensorMap &tmQ, const CUtensorMap &tmK,
                          const CUtensorMap &tmV, cudaStream_t st) {
     constexpr size_t smem = PrefillF16Smem<HD>::kTotal;
-    static ClusterSetup setup, setupShared;
-    const uint32_t *limits = nullptr;
-    int rc = setupCluster(setup, prefillF16Kernel<HD, false>, kPfThreads, smem, &limits);
-    if (rc == TC_OK) rc = setupCluster(setupShared, prefillF16Kernel<HD, true>, kPfThreads, smem, &limits);
-    if (rc != TC_OK) return rc;
     // (the blocks allocate TMEM and set up their barriers while the rows launch drains; the producer waits for it before its
     // first load, nothing else reads its outputs)
-    const uint32_t share = prm.itemRows == kPfBM ? prefillShare(prm.totalItems, tiles, prm.split ? 2u : 1u, HD, limits) : 1u;
-    if (share > 1u)
-        return launchDependent(prefillF16Kernel<HD, true>, dim3(prm.totalItems * share), kPfThreads, smem, st, share, tmQ, tmK, tmV, prm);
+    if (prm.itemRows == kPfBM) {
+        static ClusterSetup setup;
+        const uint32_t *limits = nullptr;
+        const int rc = setupCluster(setup, prefillF16Kernel<HD, true>, kPfThreads, smem, &limits);
+        if (rc != TC_OK) return rc;
+        const uint32_t share = prefillShare(prm.totalItems, tiles, prm.split ? 2u : 1u, HD, limits);
+        if (share > 1u)
+            return launchDependent(prefillF16Kernel<HD, true>, dim3(prm.totalItems * share), kPfThreads, smem, st, share, tmQ, tmK, tmV, prm);
+    }
+    static bool attrDone[64] = {false};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 0 && dev < 64 && !attrDone[dev]) {
+        TC_CUDA_OK(cudaFuncSetAttribute(prefillF16Kernel<HD, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        attrDone[dev] = true;
+    }
     const uint32_t grid = std::min<uint32_t>(prm.totalItems, static_cast<uint32_t>(numSMs()));  // one block per SM
     return launchDependent(prefillF16Kernel<HD, false>, dim3(grid), kPfThreads, smem, st, 1, tmQ, tmK, tmV, prm);
 }
