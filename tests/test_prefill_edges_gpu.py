@@ -30,6 +30,30 @@ def _check(S, pos, nH, nKV, hd):
     assert torch.isnan(out[S]).all()
 
 
+def _check_norm(S, pos, nH, nKV, hd, peak=None):
+    """Against the distance that the fp16 probabilities explain: each is off by at most 2^-11 of itself, 2^-11 / sqrt(3) on
+    average and independently of the others, and so is then the output of a row and head -- 2.8e-4 of its norm where the
+    values are N(0, 1).  Four times that.  A weight of a block's results that is off by more than a few thousandths shows."""
+    r = np.random.default_rng(7 * S + pos + hd)
+    q, k, v = (r.standard_normal((n, h, hd), dtype=np.float32) for n, h in ((S, nH), (pos + S, nKV), (pos + S, nKV)))
+    if peak is not None:    # a share of q that all rows have in common, and keys that lie along it
+        log2, rows = peak
+        u = np.where(r.random(hd) < 0.5, -1.0, 1.0).astype(np.float32)
+        q += 0.5 * u
+        k[rows] += np.float32(log2 * math.log(2.0) / math.sqrt(hd) / 0.5) * u
+    q, k, v = (x.astype(np.float16) for x in (q, k, v))
+    out = torch.full((S, nH, hd), float("nan"), device="cuda")
+    n = ops.prefill_f16_scratch_bytes(S, nH, nKV, hd, cachePos=pos)
+    scratch = torch.empty(n + 1024, dtype=torch.uint8, device="cuda")
+    off = (-scratch.data_ptr()) % 1024
+    ops.prefill_f16(*(dev(x.astype(np.float32)) for x in (q, k, v)), out, scratch[off:off + n], S, nH, nKV, hd, cachePos=pos)
+    torch.cuda.synchronize()
+    assert ops.device_status() == 0
+    want = oracle.attention_f64(q.astype(np.float32), k, v, None, None, S, nH, nKV, hd, pos, 1.0 / math.sqrt(hd)).astype(np.float64)
+    err = np.linalg.norm(host(out) - want, axis=2) / np.linalg.norm(want, axis=2)
+    assert err.max() < 4 * 2.0 ** -11 / math.sqrt(3.0), (err.max(), np.unravel_index(err.argmax(), err.shape))
+
+
 @pytest.mark.parametrize("S,pos", [(1, 0), (63, 0), (64, 0), (65, 0), (2, 127), (128, 64), (129, 63), (257, 190)])
 @pytest.mark.parametrize("nH,nKV,hd", [(7, 1, 64), (6, 2, 128), (4, 2, 256)])
 def test_tile_edges(S, pos, nH, nKV, hd):
@@ -44,6 +68,18 @@ def test_tile_edges(S, pos, nH, nKV, hd):
                                              (300, 601, 16, 2, 256)])
 def test_items_shared_by_a_cluster(S, pos, nH, nKV, hd):
     _check(S, pos, nH, nKV, hd)
+    _check_norm(S, pos, nH, nKV, hd)
+
+
+# A few keys in one KV tile outweigh all others, by 2^30 or so far that what the other tiles add vanishes: the maxima of the
+# blocks (and of the even and odd tiles of a block) that share an item are then far apart.  Tile 0 is the first block's, tile 7 the
+# last one's whether 2, 4 or 8 blocks share the tiles.
+@pytest.mark.parametrize("tile", [0, 7])
+@pytest.mark.parametrize("log2", [30, 150])
+@pytest.mark.parametrize("S,pos,nH,nKV,hd", [(16, 3000, 14, 2, 64), (77, 1217, 12, 2, 128), (130, 2500, 28, 4, 128), (300, 601, 16, 2, 256),
+                                             (1000, 0, 4, 2, 256)])
+def test_items_shared_by_a_cluster_with_keys_that_dominate(S, pos, nH, nKV, hd, log2, tile):
+    _check_norm(S, pos, nH, nKV, hd, (log2, [64 * tile + i for i in (3, 17, 60)]))
 
 
 # The launch in front of the attention: q and K / V in blocks of their own (up to two of each per SM, and no more for the

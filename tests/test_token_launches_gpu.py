@@ -82,7 +82,11 @@ def test_eager_step_on_an_int8_pool(mode, nH, nKV, hd, ctx):
 @pytest.mark.parametrize("mode,nH,nKV,hd,ctx", [("f32", 14, 2, 64, 0), ("f32", 14, 2, 64, 15), ("f32", 14, 2, 64, 2047),
                                                 ("f32", 9, 1, 128, 640), ("f32", 28, 4, 128, 5000), ("f16", 14, 2, 64, 16),
                                                 ("f16", 28, 4, 128, 129), ("f16", 28, 4, 128, 2500), ("f16", 40, 2, 128, 9001),
-                                                ("f16", 14, 2, 64, 20000)])
+                                                ("f16", 14, 2, 64, 20000),
+                                                # (head_dim 256: a rotation partner in the lane's other float4, six warps for
+                                                # eight columns; groups of 3, 8 and 20; one tile, a cluster, a merge)
+                                                ("f32", 3, 1, 256, 0), ("f32", 16, 2, 256, 0), ("f32", 6, 2, 256, 700),
+                                                ("f32", 20, 1, 256, 333), ("f32", 16, 2, 256, 15000), ("f32", 20, 1, 256, 9000)])
 def test_rotating_step_on_an_f32_or_fp16_store(mode, nH, nKV, hd, ctx, dev_pos):
     q, k, v = _rows(ctx + hd, nH, nKV, hd, ctx + 1)
     cos, sin = oracle.rope_tables(ctx + 1, hd, 1e6)
