@@ -99,8 +99,8 @@ decodeI8Kernel(const __grid_constant__ DecodeI8Params p) {
     const uint64_t rowBase = ROWS ? 0ull : (p.devRowBase ? p.devRowBase[b] : static_cast<uint64_t>(b) * p.rowsPerSeq);
     const uint32_t kvHead = ROWS ? hg / p.group : hg;
 
-    // Tile j of a chunk belongs to its warp j % SW, slot (j / SW) % NS.  A warp copies its own tiles: with one slot the next
-    // tile's K while it works on this one's V and the next V while it works on K.
+    // Tile j of a chunk belongs to its warp j % SW, slot (j / SW) % NS.  A warp copies its own tiles, NS of them ahead: a slot's
+    // next K is requested once its K has been read, its next V once its V has.
     auto slotK = [&](uint32_t i) { return smem + (warp * NS + i % NS) * 2 * L::kTileBytes; };
     auto scaleK = [&](uint32_t i) { return reinterpret_cast<float *>(smem + L::kScales) + (warp * NS + i % NS) * 2 * T; };
     const uint32_t stride = p.nKV * HD;

@@ -180,7 +180,9 @@ __device__ __forceinline__ float i2f(uint32_t x) { return __int2float_rn(static_
 // last block to arrive (tickets), or a cluster that holds them all and folds through distributed shared memory.
 enum class TcFold { kLaunch, kTickets, kCluster };
 // NH: columns the softmax and fold threads work on, the q heads of a kv head (at most 8 per launch) -- not a runtime bound,
-// which would put a branch in front of every column of the unrolled loops.
+// which would put a branch in front of every column of the unrolled loops.  Instantiated for 4, 6, 7 and 8; other groups take the
+// next wider one.  One kv head with 4 / 5 / 6 / 7 / 8 q heads, us a layer: 4.1 / 4.35 / 4.35 / 4.35 / 4.6 at 60 rows, 5.85 / 6.15 / 5.9 / 6.3 / 6.4
+// at 8000, 6.9 / 7.3 / 7.4 / 7.5 / 7.7 at 32767: a group of 5 loses nothing by its dead column.
 template <int NWG, int NS, int NH, bool APPEND, TcFold FOLD>
 __global__ void __launch_bounds__((4 * NWG + 9) * 32, 1)
 decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
@@ -617,7 +619,7 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
 
         for (uint32_t j = w; j < nTiles; j += kWG) {
             const uint32_t s = j % NS, bb = (j / kWG) & 1u;
-            // ---- this thread's token against the 8 heads ----
+            // ---- this thread's token against the NH columns ----
             if (!mbarWait<true>(&sFull[2u * w + bb], (j / (2u * kWG)) & 1u, p.err, kDevErrMmaWait)) {
                 ok = false;
                 break;
