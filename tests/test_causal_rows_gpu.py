@@ -41,3 +41,59 @@ def test_blocks_of_32_rows(S, nH, nKV, hd, pos, half):
         assert ops.device_status() == 0
         assert_close(host(out[:S]), want, rtol=0.0, atol=ATOL, what=f"{S} rows, {where}")
         assert torch.isnan(out[S]).all()  # a ragged last block writes its own rows only
+
+
+def _rows(r, S, nH, nKV, hd, pos, qScale, kScale, vScale):
+    q = r.standard_normal((S, nH, hd)) * 2.0 ** qScale
+    k = r.standard_normal((pos + S, nKV, hd)) * 2.0 ** (kScale - r.integers(0, 12, (pos + S, 1, 1)))
+    v = r.standard_normal((pos + S, nKV, hd)) * 2.0 ** (vScale - r.integers(0, 16, (pos + S, 1, 1)))
+    return (x.astype(np.float32) for x in (q, k, v))
+
+
+def _want(q, k, v, pos):
+    """The same in 64 bits, [rows][heads][hd]."""
+    S, nH, hd = q.shape
+    out = np.empty(q.shape)
+    mask = np.arange(k.shape[0])[None] > pos + np.arange(S)[:, None]
+    for h in range(nH):
+        s = q[:, h].astype(np.float64) @ k[:, h // (nH // k.shape[1])].astype(np.float64).T / math.sqrt(hd)
+        s[mask] = -np.inf
+        p = np.exp(s - s.max(1, keepdims=True))
+        out[:, h] = (p / p.sum(1, keepdims=True)) @ v[:, h // (nH // k.shape[1])].astype(np.float64)
+    return out
+
+
+@pytest.mark.parametrize("qScale,kScale,vScale", [(0, 0, 0), (40, -40, 60), (-60, 62, -90)])
+@pytest.mark.parametrize("S,nH,nKV,hd,pos", [(33, 64, 8, 64, 95), (200, 14, 2, 64, 1), (65, 48, 8, 128, 63), (47, 64, 4, 256, 17)])
+def test_rows_of_any_magnitude(S, nH, nKV, hd, pos, qScale, kScale, vScale):
+    """The f32 form takes its operands apart relative to a row's largest element: rows of very different size, next to one another and
+    as a whole, keep 21 bits each.  Bound: the scores of `ATOL` (rows smaller than their neighbours only lower them), against the
+    norm of a row's result, of which one |v| is at most 4.5 in 8."""
+    q, k, v = _rows(np.random.default_rng(S + pos), S, nH, nKV, hd, pos, qScale, kScale, vScale)
+    out = torch.full((S, nH, hd), float("nan"), device="cuda")
+    ops.prefill_kv(dev(q), dev(k), dev(v), out, S, nH, nKV, hd, pos)
+    want = _want(q, k, v, pos)
+    err = np.linalg.norm(host(out).astype(np.float64) - want, axis=2) / np.linalg.norm(want, axis=2)
+    assert err.max() < 2e-5
+
+
+@pytest.mark.parametrize("hd,nH,nKV", [(64, 64, 8), (128, 48, 8), (256, 64, 4)])
+def test_values_that_are_not_finite_stay_in_their_dims(hd, nH, nKV):
+    """An infinity in a V row reaches its own dim only, and a K row with NaN the rows that see it."""
+    S, pos = 70, 30
+    q, k, v = _rows(np.random.default_rng(hd), S, nH, nKV, hd, pos, 0, 0, 0)
+    want = _want(q, k, v, pos)
+    bad = v.copy()
+    bad[pos + 1, :, 5] = np.inf
+    bad[pos + 2, :, 7] = np.nan
+    out = torch.full((S, nH, hd), float("nan"), device="cuda")
+    ops.prefill_kv(dev(q), dev(k), dev(bad), out, S, nH, nKV, hd, pos)
+    rest = [d for d in range(hd) if d not in (5, 7)]
+    got = host(out)
+    assert_close(got[..., rest], want[..., rest], rtol=0.0, atol=ATOL)
+    assert not np.isfinite(got[2:, :, [5, 7]]).any()
+    k[pos + S - 1] = np.nan  # the last row sees it, nobody else
+    ops.prefill_kv(dev(q), dev(k), dev(v), out, S, nH, nKV, hd, pos)
+    got = host(out)
+    assert_close(got[:-1], want[:-1], rtol=0.0, atol=ATOL)
+    assert np.isnan(got[-1]).all()
