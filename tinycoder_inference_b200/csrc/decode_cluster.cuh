@@ -210,6 +210,18 @@ __device__ __forceinline__ void prefetchTile(const uint8_t *k, const uint8_t *v,
 }
 constexpr uint32_t kPrefetchTiles = 2;  // of a warp, ahead of the wait
 
+// What a token brings along (prefetchL2 in tc_common.cuh), a line per thread: `heads` vectors of q, the rows of a kv head to append
+// and -- with a host length -- the table row that rotates them.  Cold, they came out of DRAM behind the wait.
+template <int HD>
+__device__ __forceinline__ void prefetchToken(const float *q, uint32_t heads, const float *k, const float *v, const float *cosRow,
+                                              const float *sinRow, uint32_t thread) {
+    constexpr uint32_t L = HD / 32;  // lines of a row
+    const uint32_t i = thread - heads * L;
+    if (thread < heads * L) prefetchL2(q + 32u * thread);
+    else if (i < 2u * L && k != nullptr) prefetchL2((i < L ? k : v) + 32u * (i % L));
+    else if (i >= 2u * L && i < 3u * L && cosRow != nullptr) prefetchL2((i % L < L / 2u ? cosRow : sinRow) + 32u * (i % (L / 2u)));
+}
+
 // ---- distributed shared memory -------------------------------------------------------------------
 __device__ __forceinline__ uint32_t clusterRank() {
     uint32_t r;

@@ -78,6 +78,11 @@ decodeI8Kernel(const __grid_constant__ DecodeI8Params p) {
             }
         }
     }
+    if (!ROWS) {
+        const size_t row = (static_cast<size_t>(b) * p.nKV + hg) * HD;
+        prefetchToken<HD>(p.q + (static_cast<size_t>(b) * p.nHeads + hg * p.group + p.colBase) * HD, min(8u, p.group - p.colBase),
+                          p.appendK != nullptr ? p.appendK + row : nullptr, p.appendV + row, nullptr, nullptr, threadIdx.x);
+    }
     gridDepWait();
     gridDepLaunch();
 

@@ -67,6 +67,11 @@ decodeI8StreamsKernel(const __grid_constant__ DecodeI8Params p) {
     }
     __syncthreads();
     clusterHello();
+    {
+        const size_t row = static_cast<size_t>(kvHead) * HD;
+        prefetchToken<HD>(p.q + (static_cast<size_t>(kvHead) * p.group + p.colBase) * HD, min(8u, p.group - p.colBase),
+                          p.appendK != nullptr ? p.appendK + row : nullptr, p.appendV + row, nullptr, nullptr, threadIdx.x);
+    }
     gridDepWait();
 
     const uint32_t want = p.devLens ? p.devLens[0] + p.lenAdd : p.lenHost;

@@ -57,6 +57,11 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKv16Kernel(const __grid_co
         const uint8_t *v = static_cast<const uint8_t *>(p.kvV) + static_cast<size_t>(hg) * HD * 2;
         for (uint32_t i = 0, tok = chunk * per + warp * T; i < kPrefetchTiles && tok < min(hint, (chunk + 1u) * per); ++i, tok += NW * T)
             prefetchTile<HD * 2>(k, v, static_cast<size_t>(p.nKV) * HD * 2, tok, p.totalRows - 1, lane);
+        const size_t row = static_cast<size_t>(hg) * HD, table = static_cast<size_t>(p.lenHost - 1u) * (HD / 2);
+        const bool rotates = p.tok.cosT != nullptr && p.devPos == nullptr;
+        prefetchToken<HD>(p.q + (static_cast<size_t>(hg) * p.group + p.colBase) * HD, min(8u, p.group - p.colBase),
+                          p.tok.k != nullptr ? p.tok.k + row : nullptr, p.tok.v + row, rotates ? p.tok.cosT + table : nullptr,
+                          p.tok.sinT + table, threadIdx.x);
     }
     gridDepWait();
     gridDepLaunch();

@@ -26,13 +26,15 @@ kvQuantKernel(const float *__restrict__ k, const float *__restrict__ v, int8_t *
               const uint32_t *__restrict__ devDstBase, uint32_t batchMode, uint64_t rowsPerSeq,
               const uint64_t *__restrict__ rowBase, const uint32_t *__restrict__ devLens, int32_t lenAdd,
               uint64_t maxRows, unsigned int *__restrict__ err) {
-    gridDepWait();  // (no gridDepLaunch: the next grid may request these rows ahead of its own wait)
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t row = static_cast<uint64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (row >= static_cast<uint64_t>(tokens) * nKV) return;
-    if (devDstBase != nullptr) dstTokenBase = devDstBase[0];
+    const bool some = row < static_cast<uint64_t>(tokens) * nKV;
     const uint64_t t = row / nKV, h = row % nKV;
     const uint64_t src = ((srcTokenBase + t) * nKV + h) * hd;
+    if (some && 32u * lane < hd) prefetchL2(k + src + 32u * lane), prefetchL2(v + src + 32u * lane);
+    gridDepWait();  // (no gridDepLaunch: the next grid may request these rows ahead of its own wait)
+    if (!some) return;
+    if (devDstBase != nullptr) dstTokenBase = devDstBase[0];
     uint64_t dst = (dstTokenBase + t) * nKV + h;
     if (batchMode) {
         // source row t is the new token of sequence t; it goes behind that sequence's rows
@@ -134,31 +136,41 @@ kvAppendKernel(float *__restrict__ q, const float *__restrict__ kSrc, const floa
                uint32_t cachePos, uint32_t ropePos, const uint32_t *__restrict__ devPos,
                const float *__restrict__ cosT, const float *__restrict__ sinT, uint32_t maxRows,
                unsigned int *__restrict__ err) {
-    gridDepWait();
-    gridDepLaunch();
     const uint32_t pairs = hd >> 1, perRow = pairs / V;
     const uint32_t rowsPerToken = nHeads + 2 * nKV;
     const uint64_t idx = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const uint64_t rowIdx = idx / perRow;
-    if (rowIdx >= static_cast<uint64_t>(seqLen) * rowsPerToken) return;
+    const bool some = rowIdx < static_cast<uint64_t>(seqLen) * rowsPerToken;
     const uint32_t j = static_cast<uint32_t>(idx - rowIdx * perRow) * V;
     const uint32_t s = static_cast<uint32_t>(rowIdx / rowsPerToken);
     uint32_t row = static_cast<uint32_t>(rowIdx - static_cast<uint64_t>(s) * rowsPerToken);
-    if (devPos != nullptr) {
-        cachePos = devPos[0];
-        ropePos = devPos[0];
-    }
     const bool isQ = row < nHeads;
     if (!isQ) row -= nHeads;
     const bool isV = !isQ && row >= nKV;
     if (isV) row -= nKV;
+    const float *src = isQ ? q + (static_cast<size_t>(s) * nHeads + row) * hd
+                           : (isV ? vSrc : kSrc) + (static_cast<size_t>(s) * nKV + row) * hd;
+    if (some) {
+        prefetchLineOf(src + j, 4 * V);
+        prefetchLineOf(src + j + pairs, 4 * V);
+        if (cosT != nullptr && devPos == nullptr && row == 0) {
+            const size_t at = static_cast<size_t>(ropePos + s) * pairs + j;
+            prefetchLineOf(cosT + at, 4 * V);
+            prefetchLineOf(sinT + at, 4 * V);
+        }
+    }
+    gridDepWait();
+    gridDepLaunch();
+    if (!some) return;
+    if (devPos != nullptr) {
+        cachePos = devPos[0];
+        ropePos = devPos[0];
+    }
     if (!isQ && maxRows != 0 && static_cast<uint64_t>(cachePos) + s >= maxRows) {
         // device-side position outside the window: no store, reported through the error word
         if (j == 0) atomicOr(err, kDevErrRowBound);
         return;
     }
-    const float *src = isQ ? q + (static_cast<size_t>(s) * nHeads + row) * hd
-                           : (isV ? vSrc : kSrc) + (static_cast<size_t>(s) * nKV + row) * hd;
     Vec<V> x0 = loadVec<V>(src + j), x1 = loadVec<V>(src + j + pairs);
     if (!isV && cosT != nullptr) {
         const size_t at = static_cast<size_t>(ropePos + s) * pairs + j;
@@ -189,14 +201,16 @@ kvAppendKernel(float *__restrict__ q, const float *__restrict__ kSrc, const floa
 template <int V>
 __global__ void __launch_bounds__(256)
 sigmoidGateKernel(float *__restrict__ attnOut, const float *__restrict__ qGate, uint64_t units, uint32_t hd) {
-    gridDepWait();
-    gridDepLaunch();
     const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= units) return;
     const uint32_t perHead = hd / V;
     const uint64_t head = i / perHead;  // token x head
     const uint32_t e = static_cast<uint32_t>(i - head * perHead) * V;
-    const Vec<V> g = loadVec<V>(qGate + head * 2 * hd + hd + e);
+    const float *gate = qGate + head * 2 * hd + hd + e;
+    if (i < units) prefetchLineOf(gate, 4 * V);
+    gridDepWait();
+    gridDepLaunch();
+    if (i >= units) return;
+    const Vec<V> g = loadVec<V>(gate);
     Vec<V> x = loadVec<V>(attnOut + head * hd + e);
 #pragma unroll
     for (int k = 0; k < V; ++k) x.x[k] *= 1.0f / (1.0f + __expf(-g.x[k]));

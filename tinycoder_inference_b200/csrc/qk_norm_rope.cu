@@ -33,12 +33,10 @@ qkNormRopeKernel(const float *__restrict__ qIn, uint32_t qInStride, float *qOut,
                  const float *__restrict__ wq, const float *__restrict__ wk, uint32_t hd, uint32_t nDims,
                  uint32_t nHeads, uint32_t nKV, uint32_t seqLen, uint32_t pos, const uint32_t *__restrict__ devPos,
                  const float *__restrict__ cosT, const float *__restrict__ sinT) {
-    gridDepWait();
-    gridDepLaunch();
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t slices = (qIn ? nHeads : 0u) + (k ? nKV : 0u);
     const uint64_t idx = static_cast<uint64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (idx >= static_cast<uint64_t>(seqLen) * slices) return;
+    const bool some = idx < static_cast<uint64_t>(seqLen) * slices;
     const uint32_t s = static_cast<uint32_t>(idx / slices);
     uint32_t h = static_cast<uint32_t>(idx % slices);
     const bool isQ = qIn != nullptr && h < nHeads;
@@ -47,6 +45,19 @@ qkNormRopeKernel(const float *__restrict__ qIn, uint32_t qInStride, float *qOut,
                           : k + (static_cast<uint64_t>(s) * nKV + h) * hd;
     float *op = isQ ? qOut + (static_cast<uint64_t>(s) * nHeads + h) * hd : k + (static_cast<uint64_t>(s) * nKV + h) * hd;
     const float *w = isQ ? wq : wk;
+    if (some) {
+        if (32u * lane < hd) {
+            prefetchL2(rp + 32u * lane);
+            if (s == 0u && h == 0u) prefetchL2(w + 32u * lane);
+        }
+        if (devPos == nullptr && h == 0u && 64u * lane < nDims) {
+            const uint64_t at = static_cast<uint64_t>(pos + s) * (nDims / 2) + 32u * lane;
+            prefetchL2(cosT + at), prefetchL2(sinT + at);
+        }
+    }
+    gridDepWait();
+    gridDepLaunch();
+    if (!some) return;
 
     // element e of a lane is j = lane + 32 e: e = i + 4 kk is the kk-th element of reference thread lane + 32 i
     constexpr int E = 4 * PER;
