@@ -358,6 +358,31 @@ def test_next_pool_hint_changes_nothing_but_timing():
     assert_close(host(b), want, what="decode with a next-pool hint")
 
 
+@pytest.mark.parametrize("appends", [False, True])
+@pytest.mark.parametrize("ctx", [1536, 1537, 1665, 5200])
+def test_next_pool_hint_of_blocks_with_many_tiles(ctx, appends):
+    """A block of more than 12 tiles (one per sequence and kv head here) waits for its last one ahead of the hint, also where that
+    tile takes the new row: the same bits and the same row, with host and device lengths."""
+    nH, nKV, hd, batch = 28, 4, 128, 2
+    g = torch.Generator(device="cuda").manual_seed(ctx)
+    pool = [torch.randint(-127, 128, (batch * ctx, nKV, hd), dtype=torch.int8, device="cuda", generator=g) for _ in range(2)] + \
+           [0.01 + 0.01 * torch.rand((batch * ctx, nKV), device="cuda", generator=g) for _ in range(2)]
+    other = [torch.zeros_like(pool[0]) for _ in range(2)]
+    q = torch.randn((batch, nH, hd), device="cuda", generator=g)
+    rows = tuple(torch.randn((batch, nKV, hd), device="cuda", generator=g) for _ in range(2)) if appends else None
+    lens = torch.tensor([ctx, ctx - 1], dtype=torch.int32, device="cuda")
+    for on_device in (False, True):
+        got = []
+        for hint in (None, tuple(other)):
+            mine, out = [t.clone() for t in pool], torch.empty_like(q)
+            ops.decode_i8_batch(q, *mine, out, ops.workspace(batch, nH, hd, 1), lens if on_device else None, batch, nH, nKV, hd, ctx,
+                                1, rows_per_seq=ctx, next_kv=hint, append=rows)
+            torch.cuda.synchronize()
+            assert ops.device_status() == 0
+            got.append([out] + mine)
+        assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
 def test_context_split_partials_merge_on_one_gpu():
     """The context-axis split as two 'ranks' on one device: each half of the rows yields
     partials-only output, the partials are concatenated as the all-gather would and merged."""

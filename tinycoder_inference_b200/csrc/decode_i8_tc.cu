@@ -65,7 +65,7 @@ struct DecodeTcParams {
     float invSqrt;
     int directOut;
     int dependent;          // TC_DECODE_PDL: the next grid may start ahead of this one's wait
-    int prefetchNext;
+    int prefetchNext;       // 1: yes, 2: only blocks of more than kLateTiles tiles
     uint32_t earlyStages;   // tiles the producer may request before the dependency wait
     int l2Hints;            // bit 0: own tiles evict_first, bit 1: next pools evict_last
     unsigned int *err;
@@ -87,6 +87,7 @@ __device__ __forceinline__ unsigned long long gtime() {
 
 constexpr int kTcTile = 128;      // tokens per tile = MMA M of the score product
 constexpr float kTcLazyLog2 = 8.0f;
+constexpr uint32_t kLateTiles = 12;  // blocks of more tiles pull the next call's rows when their own are in
 
 // NWG softmax warpgroups take the tiles round-robin (tile j belongs to warpgroup j % NWG and uses its
 // buffer (j / NWG) & 1); NS ring stages.  Warps: [0, 4 NWG) softmax, 4 NWG the TMA producer, then
@@ -293,7 +294,7 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
             // the rest.  28 / 4 heads, per layer, all tiles -> these: 32768 rows (7 tiles a block) 11.3 -> 10.7 us, 37000 (8)
             // 12.5 -> 11.7, 4 sequences of 8192 (8) 13.4 -> 12.7, 8 of 4400 (9) 11.9 -> 10.4, 2 of 22000 (10) 14.0 -> 13.0.
             const uint32_t first = nTiles > NS ? min(static_cast<uint32_t>(NS), 2u * (nTiles - NS) + 1u) : 0u;
-            for (uint32_t it = first; it < min(nTiles, NS + 2u); ++it) {
+            for (uint32_t it = first; it < min(nTiles, nTiles > kLateTiles ? NS + 4u : NS + 2u); ++it) {
                 const int row = static_cast<int>(rowBase + t0 + it * T);
                 if (p.l2Hints & 2) {
                     tmaPrefetchL2_3DHint(&tmKn, 0, kvHead, row, polLast);
@@ -406,7 +407,17 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         }
         // all tiles of this block are requested: the next call's rows follow them into L2 (requested
         // earlier they sit in front of this block's own tiles in the queue: 10.2 against 9.1 us)
-        if (p.prefetchNext && lane == 0) prefetchNextPools();
+        // -- and a block of many tiles waits until its last one is in: HBM is what bounds it, and would be idle from there to the
+        // next call's first requests, some 3 us.  That is room for four tiles a block.  Requested with its own last ring they
+        // held that up by as much as they gained.  28 / 4 heads, eight layers, two tiles with the last ring (none above 48 MB a call) ->
+        // four behind it: 8 sequences of 8192 rows (16 tiles a block) 114.0 -> 111.0 us, 16 of 4000 114.3 -> 109.1, 32 of 2000
+        // 107.4 -> 103.9, 2 of 30000 115.0 -> 109.4, 1 of 80000 145.7 -> 140.3.  Below that blocks are bound by latency, and what comes
+        // late comes too late: 2 of 22000 (10 tiles) 91.9 -> 95.1, 8 of 6000 (12 tiles) 87.5 -> 88.2.
+        if (p.prefetchNext == 1 || (p.prefetchNext != 0 && nTiles > kLateTiles)) {
+            const uint32_t last = nTiles - 1u;
+            const bool in = nTiles <= kLateTiles || (okP && mbarWait(&fullBar[last % NS], (last / NS) & 1u, p.err, kDevErrFullWait));
+            if (in && lane == 0) prefetchNextPools();
+        }
     } else if (warp > kProducerWarp) {
         // -------------------------------- MMA issuers --------------------------------
         // Four issuing warps, so that no wait stands in front of another tile's products: score products and P.V products of
@@ -912,9 +923,11 @@ int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, c
     // the next call's pools, pulled into L2 behind this call's rows; larger calls keep HBM busy by themselves.  (With the hint
     // against without it, per layer of pools that do not fit L2 together: 20000 rows 8.70 / 9.25 us, 32768 rows 10.90 /
     // 10.98, 47000 rows (46 MiB) 14.04 / 13.55, 50000 rows 14.25 / 14.02, 80000 rows 18.13 / 18.46; 4 sequences of 8192 rows
-    // 12.2 / 11.7, 8 of 8192 14.24 / 14.60.  It pays where a call is short; from some 30 MB on it is within 4 % either way.)
+    // 12.2 / 11.7, 8 of 8192 14.24 / 14.60.  It pays where a call is short; from some 30 MB on it is within 4 % either way.)  Blocks of many tiles
+    // pull them when their own are in (kLateTiles), which pays up to 80 MB: 2 sequences of 40000 rows (82 MB) 135.5 / 135.7 us for eight
+    // layers, 8 of 12000 (98 MB) 145.3 / 146.0.
     const uint64_t callBytes = static_cast<uint64_t>(d->batch) * d->maxLen * d->nKV * hd * 2ull;
-    const bool prefetchNext = d->nextK8 != nullptr && d->nextV8 != nullptr && callBytes <= (48ull << 20);
+    const int prefetchNext = d->nextK8 == nullptr || d->nextV8 == nullptr || callBytes > (80ull << 20) ? 0 : callBytes <= (48ull << 20) ? 1 : 2;
     if (prefetchNext) {
         TC_REQUIRE(((reinterpret_cast<uintptr_t>(d->nextK8) | reinterpret_cast<uintptr_t>(d->nextV8)) & 15u) == 0,
                    TC_EINVAL, "decode_i8: nextK8/nextV8 need 16-byte alignment");
@@ -960,7 +973,7 @@ int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, c
     prm.invSqrt = d->invSqrt;
     prm.directOut = direct ? 1 : 0;
     prm.dependent = pdl ? 1 : 0;
-    prm.prefetchNext = prefetchNext ? 1 : 0;
+    prm.prefetchNext = prefetchNext;
     // Under programmatic dependent launch the producer requests a whole ring of old rows while the
     // kernels ahead drain (7B shape, 32768 rows, batch 1: 12.4 us per layer against 13.5 with one
     // stage).  The block's own tiles are read once (evict-first); the next call's rows pulled in
