@@ -127,3 +127,27 @@ def test_a_device_position_outside_the_store_writes_no_row(mode, nH, nKV, hd, wi
     assert ops.device_status(raise_on_flags=False) == 32
     for have, want in zip(stores, before):
         assert torch.equal(torch.nan_to_num(have.float()), torch.nan_to_num(want.float()))
+
+
+@pytest.mark.parametrize("nH,nKV,hd,ctx,growth", [(28, 4, 128, 300, 0.0), (28, 4, 128, 4600, 6.0), (14, 2, 128, 4100, 0.4), (16, 2, 256, 2700, 6.0),
+                                                  (8, 4, 256, 1500, 0.4)])
+def test_captured_int8_step_accumulates_like_causal_rows(nH, nKV, hd, ctx, growth):
+    """The launch a captured step replays keeps the causal kernel's roundings over several rounds of tiles, where no tile moves a
+    head's reference point or the bound of the V scales, where all of them do, and where some do: scores and V rows that grow with the
+    position, by `growth` powers of two in 16 rows."""
+    g = torch.Generator(device="cuda").manual_seed(ctx)
+    s = ops.KvSession(nH, nKV, hd, ctx + 100, 1, mode="i8")
+    q = torch.randn((1, nH, hd), device="cuda", generator=g)
+    k, v = (torch.randn((ctx, nKV, hd), device="cuda", generator=g) for _ in range(2))
+    at = torch.arange(ctx, device="cuda", dtype=torch.float32)[:, None, None] / 16.0 * growth
+    mean = q.view(nKV, nH // nKV, hd).mean(1)
+    k += at * math.log(2.0) * math.sqrt(hd) * mean / (mean * mean).sum(1, keepdim=True)
+    v *= torch.exp2(torch.clamp(at / 6.0, max=40.0))
+    ops.kv_quantize_i8(k[:-1].contiguous(), v[:-1].contiguous(), s.k8[0], s.v8[0], s.ks[0], s.vs[0], ctx - 1, nKV, hd)
+    out, want = torch.empty_like(q), torch.empty_like(q)
+    s.attend(0, q, k[-1:].contiguous(), v[-1:].contiguous(), out, ctx - 1, dev_pos=torch.tensor([ctx - 1], dtype=torch.int32, device="cuda"))
+    ops.prefill_i8(q, s.k8[0], s.v8[0], s.ks[0], s.vs[0], want, 1, nH, nKV, hd, ctx - 1)
+    torch.cuda.synchronize()
+    assert ops.device_status() == 0
+    # the eight streams' results are put together in another order: a handful of f32 roundings
+    assert float((out - want).norm() / want.norm()) < 1e-6

@@ -14,8 +14,12 @@
 //     their tiles' maxima and each has walked through them in tile order -- probabilities as MMA operands;
 //   * four value warps own HD / 4 dimensions each and walk through all tiles of the stream: rescale, four to eight products;
 //   * a sum warp walks along with the row sums.
-// A tile costs the walk some 150 cycles where one warp doing all of it took 2500: 5000 rows of 28 q / 4 kv heads of 128
-// (157 tiles of 32 tokens, 20 per stream) take 13.8 us, 26 with a warp per stream, 27.5 with a block per q head.
+// A tile costs the walk some 200 cycles where one warp doing all of it took 2500: 5000 rows of 28 q / 4 kv heads of 128
+// (157 tiles of 32 tokens, 20 per stream) took 13.8 us, 26 with a warp per stream, 27.5 with a block per q head.
+// The walks of values and sums hear of a round of eight tiles at a time, and a round's V tiles are requested when its
+// probabilities are out: the score warps used to stand until the walk was through with the round before, and a wait per
+// tile cost the walk 170 cycles.  Most tiles move no reference point, and are passed over together.  Per layer, 28 / 4 / 128 at 5000 /
+// 8000 / 16000 rows 11.3 / 16.5 / 29.6 -> 10.8 / 14.2 / 23.0 us, 16 / 2 / 256 at 8000 (norm and gate included) 34.4 -> 25.9.
 #include "decode_i8.cuh"
 
 namespace tc {
@@ -34,11 +38,11 @@ struct I8StreamSmem {
     static constexpr int kScales = kRec + kSlots * kRecord;        // [score warp][2][K, V][T]
     static constexpr int kMax = kScales + kScoreWarps * 4 * T * 4; // [2][score warp][12]: column maxima, V scale bits
     static constexpr int kEnd = kMax + 2 * kScoreWarps * 12 * 4;   // m[8], E, then l[8], sums of P x scale [8]
-    static constexpr int kBars = kEnd + 32 * 4;                    // full, empty per slot
+    static constexpr int kBars = kEnd + 32 * 4;                    // full, empty of the even / odd rounds
     // The score warps prepare the query together where it is long (16 / 2 / 256, norm and gate included: 20 / 500 / 2000 / 5000 rows
     // 10.0 / 10.5 / 14.2 / 25.3 -> 9.75 / 10.0 / 13.85 / 24.9 us a layer; 8 / 2 / 128 at 20 rows 5.65 -> 5.9).
     static constexpr bool kShareQuery = HD > 128;
-    static constexpr int kQuery = kBars + 2 * kSlots * 8;          // the query operands
+    static constexpr int kQuery = kBars + 4 * 8;                   // the query operands
     static constexpr int kTotal = kQuery + (kShareQuery ? I8QueryShare<HD, kScoreWarps>::kBytes : 0) + 128;
     static_assert(kQuery % 16 == 0, "16-byte accesses");
     static_assert(FoldScratch<HD>::kWarp * 4 <= kV, "the fold reuses the K tiles");
@@ -56,11 +60,11 @@ decodeI8StreamsKernel(const __grid_constant__ DecodeI8Params p) {
 
     extern __shared__ uint8_t smemRaw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smemRaw) + 127) & ~uintptr_t(127));
-    uint64_t *fullBar = reinterpret_cast<uint64_t *>(smem + L::kBars), *emptyBar = fullBar + NSLOT;
+    uint64_t *fullBar = reinterpret_cast<uint64_t *>(smem + L::kBars), *emptyBar = fullBar + 2;
     float *sEnd = reinterpret_cast<float *>(smem + L::kEnd);
     if (threadIdx.x == 0) {
-        for (uint32_t s = 0; s < NSLOT; ++s) {
-            mbarInit(&fullBar[s], 32);
+        for (uint32_t s = 0; s < 2; ++s) {
+            mbarInit(&fullBar[s], SW);
             mbarInit(&emptyBar[s], VW + 1);
         }
         fenceBarrierInit();
@@ -122,8 +126,8 @@ decodeI8StreamsKernel(const __grid_constant__ DecodeI8Params p) {
         bool ok = true;
         auto requestV = [&](uint32_t i) {
             if (ok && i < n) {
-                // the slot's tile of a round before has been folded by everybody
-                if (i >= NSLOT) ok = mbarWait(&emptyBar[i % NSLOT], (i / NSLOT - 1u) & 1u, p.err, kDevErrEmptyWait);
+                // the tiles of two rounds before have been folded by everybody
+                if (i >= NSLOT) ok = mbarWait(&emptyBar[(i / SW) & 1u], (i / NSLOT - 1u) & 1u, p.err, kDevErrEmptyWait);
                 request(i, true);
             }
             cpAsyncCommit();
@@ -156,13 +160,17 @@ decodeI8StreamsKernel(const __grid_constant__ DecodeI8Params p) {
         uint32_t Ebits = 0;                // running power-of-two scale of the V row scales (0 = unset)
         for (uint32_t round = 0; round * SW < n; ++round) {
             const uint32_t i = round * SW + warp;
-            requestV(i + SW);
-            cpAsyncWait<2>();  // K and V of this tile are in
+            cpAsyncWait<2>();  // K of this tile is in
             const uint32_t tokBase = (stream + 8u * i) * T + g;
             float sc[NR][2], svr[NR];
             float mx0 = -INFINITY, mx1 = -INFINITY, svmax = 0.0f;
             if (i < n) {  // warp-uniform
                 i8Scores<HD, MT>(qf, smemAddr(slotK(i)), scales(i), tokBase, len, len, lane, sc);
+                __syncwarp();
+            }
+            requestK(i + 2 * SW);  // (every lane is through with K)
+            cpAsyncWait<1>();      // V of this tile is in
+            if (i < n) {
 #pragma unroll
                 for (int r = 0; r < NR; ++r) {
                     svr[r] = tokBase + 8 * r < len ? scales(i)[T + g + 8 * r] : 0.0f;
@@ -177,70 +185,93 @@ decodeI8StreamsKernel(const __grid_constant__ DecodeI8Params p) {
                 }
             }
             const uint32_t ebMine = min(__reduce_max_sync(0xffffffffu, __float_as_uint(svmax)) & 0x7f800000u, 253u << 23);
-            requestK(i + 2 * SW);  // (the shuffles above have every lane through with K)
             // ---- the round's maxima, in tile order ----
             float *mine = sMax + ((round & 1u) * SW + warp) * 12u;
             if (g == 0) *reinterpret_cast<float2 *>(mine + 2 * t) = make_float2(mx0, mx1);
             if (lane == 0) mine[8] = __uint_as_float(ebMine);
             namedBarSync(1, SW * 32);
-            float a0 = 1.0f, a1 = 1.0f, fMine = 1.0f, r0 = m0, r1 = m1, invE = 0.0f;
+            float a0 = 1.0f, a1 = 1.0f, fMine = 1.0f, r0 = m0, r1 = m1;
+            uint32_t eMine = Ebits;
             bool moved = false;
+            float2 mx[SW];
+            uint32_t eb[SW];
 #pragma unroll
             for (uint32_t w = 0; w < SW; ++w) {
                 const float *other = sMax + ((round & 1u) * SW + w) * 12u;
-                const float2 mx = *reinterpret_cast<const float2 *>(other + 2 * t);
-                const uint32_t eb = __float_as_uint(other[8]);
+                mx[w] = *reinterpret_cast<const float2 *>(other + 2 * t);
+                eb[w] = __float_as_uint(other[8]);
+            }
+            // Tiles that move nothing for any head -- nearly all behind the first -- are passed over together; the others one
+            // after the other.
+            uint32_t todo = (1u << SW) - 1u;
+            while (true) {
+                uint32_t moves = 0;
+#pragma unroll
+                for (uint32_t w = 0; w < SW; ++w)
+                    moves |= mx[w].x > m0 + kLazyLog2 || mx[w].y > m1 + kLazyLog2 || eb[w] > Ebits ? 1u << w : 0u;
+                moves = __reduce_or_sync(0xffffffffu, moves) & todo;
+                if (moves == 0u) break;
+                const uint32_t f = __ffs(moves) - 1u;
+                float2 top = mx[0];
+                uint32_t e = eb[0];
+#pragma unroll
+                for (uint32_t w = 1; w < SW; ++w)
+                    if (w == f) top = mx[w], e = eb[w];
                 // lazy reference point: move it only when the maximum ran ahead by 2^8
-                const float mn0 = mx.x > m0 + kLazyLog2 ? mx.x : m0;
-                const float mn1 = mx.y > m1 + kLazyLog2 ? mx.y : m1;
+                const float mn0 = top.x > m0 + kLazyLog2 ? top.x : m0;
+                const float mn1 = top.y > m1 + kLazyLog2 ? top.y : m1;
                 float fE = 1.0f;
-                if (eb > Ebits) {
-                    fE = Ebits ? __uint_as_float(Ebits) * __uint_as_float((254u << 23) - eb) : 1.0f;
-                    Ebits = eb;
+                if (e > Ebits) {
+                    fE = Ebits ? __uint_as_float(Ebits) * __uint_as_float((254u << 23) - e) : 1.0f;
+                    Ebits = e;
                 }
-                if (w == warp) {
+                if (f == warp) {
                     a0 = fastExp2(m0 - mn0), a1 = fastExp2(m1 - mn1), fMine = fE;
                     moved = mn0 != m0 || mn1 != m1 || fE != 1.0f;
-                    r0 = mn0, r1 = mn1;
-                    invE = Ebits ? __uint_as_float((254u << 23) - Ebits) : 0.0f;
                 }
                 m0 = mn0, m1 = mn1;
+                if (f <= warp) r0 = m0, r1 = m1, eMine = Ebits;
+                todo = ~((2u << f) - 1u);
             }
+            const float invE = eMine ? __uint_as_float((254u << 23) - eMine) : 0.0f;
             const bool any = __any_sync(0xffffffffu, moved);
-            if (i >= n) continue;
-            // ---- p, then p * sv scaled into fp16 range, hi + lo, transposed to the B layout ----
-            uint8_t *rec = record(i);
-            float *recP = reinterpret_cast<float *>(rec + kRecP) + lane, *recX = reinterpret_cast<float *>(rec + kRecX) + lane;
+            if (i < n) {
+                // ---- p, then p * sv scaled into fp16 range, hi + lo, transposed to the B layout ----
+                uint8_t *rec = record(i);
+                float *recP = reinterpret_cast<float *>(rec + kRecP) + lane, *recX = reinterpret_cast<float *>(rec + kRecX) + lane;
 #pragma unroll
-            for (int mt = 0; mt < MT; ++mt) {
-                uint32_t bh[2], bl[2];
+                for (int mt = 0; mt < MT; ++mt) {
+                    uint32_t bh[2], bl[2];
 #pragma unroll
-                for (int hf = 0; hf < 2; ++hf) {
-                    const int r = 2 * mt + hf;
-                    const float p0 = fastExp2(sc[r][0] - r0), p1 = fastExp2(sc[r][1] - r1);
-                    const float w = svr[r] * invE;
-                    const float x0 = p0 * w, x1 = p1 * w;
-                    const uint32_t hi = packHalf2(x0, x1);
-                    const __half2 hh = *reinterpret_cast<const __half2 *>(&hi);
-                    const float d0 = x0 - __low2float(hh), d1 = x1 - __high2float(hh);
-                    const uint32_t lo = packHalf2(d0, d1);
-                    const __half2 ll = *reinterpret_cast<const __half2 *>(&lo);
-                    recP[(2 * r) * 32] = p0, recP[(2 * r + 1) * 32] = p1;
-                    recX[(2 * r) * 32] = __low2float(hh) + __low2float(ll);
-                    recX[(2 * r + 1) * 32] = __high2float(hh) + __high2float(ll);
-                    bh[hf] = movmatrixTrans(hi);
-                    bl[hf] = movmatrixTrans(lo);
+                    for (int hf = 0; hf < 2; ++hf) {
+                        const int r = 2 * mt + hf;
+                        const float p0 = fastExp2(sc[r][0] - r0), p1 = fastExp2(sc[r][1] - r1);
+                        const float w = svr[r] * invE;
+                        const float x0 = p0 * w, x1 = p1 * w;
+                        const uint32_t hi = packHalf2(x0, x1);
+                        const __half2 hh = *reinterpret_cast<const __half2 *>(&hi);
+                        const float d0 = x0 - __low2float(hh), d1 = x1 - __high2float(hh);
+                        const uint32_t lo = packHalf2(d0, d1);
+                        const __half2 ll = *reinterpret_cast<const __half2 *>(&lo);
+                        recP[(2 * r) * 32] = p0, recP[(2 * r + 1) * 32] = p1;
+                        recX[(2 * r) * 32] = __low2float(hh) + __low2float(ll);
+                        recX[(2 * r + 1) * 32] = __high2float(hh) + __high2float(ll);
+                        bh[hf] = movmatrixTrans(hi);
+                        bl[hf] = movmatrixTrans(lo);
+                    }
+                    *reinterpret_cast<uint4 *>(rec + (mt * 32 + lane) * 16) = make_uint4(bh[0], bh[1], bl[0], bl[1]);
                 }
-                *reinterpret_cast<uint4 *>(rec + (mt * 32 + lane) * 16) = make_uint4(bh[0], bh[1], bl[0], bl[1]);
+                float *fac = reinterpret_cast<float *>(rec + kRecF);
+                if (g == 0) {
+                    *reinterpret_cast<float2 *>(fac + 2 * t) = make_float2(a0 * fMine, a1 * fMine);
+                    *reinterpret_cast<float2 *>(fac + 8 + 2 * t) = make_float2(a0, a1);
+                }
+                if (lane == 0) *reinterpret_cast<uint32_t *>(fac + 16) = any ? 1u : 0u;
             }
-            float *fac = reinterpret_cast<float *>(rec + kRecF);
-            if (g == 0) {
-                *reinterpret_cast<float2 *>(fac + 2 * t) = make_float2(a0 * fMine, a1 * fMine);
-                *reinterpret_cast<float2 *>(fac + 8 + 2 * t) = make_float2(a0, a1);
-            }
-            if (lane == 0) *reinterpret_cast<uint32_t *>(fac + 16) = any ? 1u : 0u;
+            __syncwarp();
             // (a warp whose wait ran out stays with the others' barrier and hands nothing on: their waits end too)
-            if (ok) mbarArrive(&fullBar[i % NSLOT]);
+            if (ok && lane == 0) mbarArrive(&fullBar[round & 1u]);
+            requestV(i + SW);  // (waits for the values of the round before, which are folded under this one)
             if (hasRow && round == 0) {
                 // (here the row's stores are long done: right behind them the fence cost 0.5 us of the step)
                 __threadfence();
@@ -256,71 +287,78 @@ decodeI8StreamsKernel(const __grid_constant__ DecodeI8Params p) {
     } else if (warp < SW + VW) {
         // ---------------------------------- accumulators ----------------------------------
         const uint32_t cp0 = (warp - SW) * CP;  // dims 32 cp0 .. 32 (cp0 + CP) - 1
-        for (uint32_t i = 0; i < n; ++i) {
-            if (!mbarWait(&fullBar[i % NSLOT], (i / NSLOT) & 1u, p.err, kDevErrFullWait)) break;
-            const uint8_t *rec = record(i);
-            const float *fac = reinterpret_cast<const float *>(rec + kRecF);
-            uint4 b[MT];
+        for (uint32_t i0 = 0, round = 0; i0 < n; i0 += SW, ++round) {
+            if (!mbarWait(&fullBar[round & 1u], (round >> 1) & 1u, p.err, kDevErrFullWait)) break;
+            const uint32_t i1 = min(n, i0 + SW);
+#pragma unroll 2
+            for (uint32_t i = i0; i < i1; ++i) {
+                const uint8_t *rec = record(i);
+                const float *fac = reinterpret_cast<const float *>(rec + kRecF);
+                uint4 b[MT];
 #pragma unroll
-            for (int mt = 0; mt < MT; ++mt) b[mt] = *reinterpret_cast<const uint4 *>(rec + (mt * 32 + lane) * 16);
-            uint32_t v[CP][MT][4];
-            const uint32_t vTile = smemAddr(smem + L::kV + (i % NSLOT) * L::kTileBytes) + lr * 128;
+                for (int mt = 0; mt < MT; ++mt) b[mt] = *reinterpret_cast<const uint4 *>(rec + (mt * 32 + lane) * 16);
+                uint32_t v[CP][MT][4];
+                const uint32_t vTile = smemAddr(smem + L::kV + (i % NSLOT) * L::kTileBytes) + lr * 128;
 #pragma unroll
-            for (int c = 0; c < CP; ++c) {
-                const uint32_t cp = cp0 + c;
-                const uint32_t sw = (((2 * (cp & 3u) + lco) ^ (lr & 7u)) << 4) + (cp >> 2) * L::kHalfBytes;
+                for (int c = 0; c < CP; ++c) {
+                    const uint32_t cp = cp0 + c;
+                    const uint32_t sw = (((2 * (cp & 3u) + lco) ^ (lr & 7u)) << 4) + (cp >> 2) * L::kHalfBytes;
 #pragma unroll
-                for (int mt = 0; mt < MT; ++mt)
-                    ldmatrixX4Trans(v[c][mt][0], v[c][mt][1], v[c][mt][2], v[c][mt][3], vTile + mt * 2048 + sw);
-            }
-            if (*reinterpret_cast<const uint32_t *>(fac + 16) != 0u) {
-                const float2 al = *reinterpret_cast<const float2 *>(fac + 2 * t);
+                    for (int mt = 0; mt < MT; ++mt)
+                        ldmatrixX4Trans(v[c][mt][0], v[c][mt][1], v[c][mt][2], v[c][mt][3], vTile + mt * 2048 + sw);
+                }
+                if (*reinterpret_cast<const uint32_t *>(fac + 16) != 0u) {
+                    const float2 al = *reinterpret_cast<const float2 *>(fac + 2 * t);
 #pragma unroll
-                for (int c = 0; c < 2 * CP; ++c) o[c][0] *= al.x, o[c][1] *= al.y, o[c][2] *= al.x, o[c][3] *= al.y;
-            }
-#pragma unroll
-            for (int mt = 0; mt < MT; ++mt) {
-                // rows g / g + 8 of an MMA tile are dims 16 c + 2 g / 16 c + 2 g + 1
-                uint32_t x[2 * CP][4];
-#pragma unroll
-                for (int c = 0; c < 2 * CP; ++c) {
-                    const uint32_t r0 = v[c / 2][mt][c % 2 * 2] ^ 0x80808080u, r1 = v[c / 2][mt][c % 2 * 2 + 1] ^ 0x80808080u;
-                    x[c][0] = subnormalPair<0x4240>(r0), x[c][1] = subnormalPair<0x4341>(r0);
-                    x[c][2] = subnormalPair<0x4240>(r1), x[c][3] = subnormalPair<0x4341>(r1);
+                    for (int c = 0; c < 2 * CP; ++c) o[c][0] *= al.x, o[c][1] *= al.y, o[c][2] *= al.x, o[c][3] *= al.y;
                 }
 #pragma unroll
-                for (int c = 0; c < 2 * CP; ++c) mmaF16(o[c], x[c][0], x[c][1], x[c][2], x[c][3], b[mt].x, b[mt].y);
+                for (int mt = 0; mt < MT; ++mt) {
+                    // rows g / g + 8 of an MMA tile are dims 16 c + 2 g / 16 c + 2 g + 1
+                    uint32_t x[2 * CP][4];
 #pragma unroll
-                for (int c = 0; c < 2 * CP; ++c) mmaF16(o[c], x[c][0], x[c][1], x[c][2], x[c][3], b[mt].z, b[mt].w);
+                    for (int c = 0; c < 2 * CP; ++c) {
+                        const uint32_t r0 = v[c / 2][mt][c % 2 * 2] ^ 0x80808080u, r1 = v[c / 2][mt][c % 2 * 2 + 1] ^ 0x80808080u;
+                        x[c][0] = subnormalPair<0x4240>(r0), x[c][1] = subnormalPair<0x4341>(r0);
+                        x[c][2] = subnormalPair<0x4240>(r1), x[c][3] = subnormalPair<0x4341>(r1);
+                    }
+#pragma unroll
+                    for (int c = 0; c < 2 * CP; ++c) mmaF16(o[c], x[c][0], x[c][1], x[c][2], x[c][3], b[mt].x, b[mt].y);
+#pragma unroll
+                    for (int c = 0; c < 2 * CP; ++c) mmaF16(o[c], x[c][0], x[c][1], x[c][2], x[c][3], b[mt].z, b[mt].w);
+                }
             }
             __syncwarp();
-            if (lane == 0) mbarArrive(&emptyBar[i % NSLOT]);
+            if (lane == 0) mbarArrive(&emptyBar[round & 1u]);
         }
     } else {
         // ---------------------------------- row sums ----------------------------------
         float l0 = 0.0f, l1 = 0.0f, ps0 = 0.0f, ps1 = 0.0f;
-        for (uint32_t i = 0; i < n; ++i) {
-            if (!mbarWait(&fullBar[i % NSLOT], (i / NSLOT) & 1u, p.err, kDevErrFullWait)) break;
-            const uint8_t *rec = record(i);
-            const float *fac = reinterpret_cast<const float *>(rec + kRecF);
-            const float *recP = reinterpret_cast<const float *>(rec + kRecP) + lane;
-            const float *recX = reinterpret_cast<const float *>(rec + kRecX) + lane;
-            float pv[2 * NR], xv[2 * NR];
+        for (uint32_t i0 = 0, round = 0; i0 < n; i0 += SW, ++round) {
+            if (!mbarWait(&fullBar[round & 1u], (round >> 1) & 1u, p.err, kDevErrFullWait)) break;
+            const uint32_t i1 = min(n, i0 + SW);
+            for (uint32_t i = i0; i < i1; ++i) {
+                const uint8_t *rec = record(i);
+                const float *fac = reinterpret_cast<const float *>(rec + kRecF);
+                const float *recP = reinterpret_cast<const float *>(rec + kRecP) + lane;
+                const float *recX = reinterpret_cast<const float *>(rec + kRecX) + lane;
+                float pv[2 * NR], xv[2 * NR];
 #pragma unroll
-            for (int r = 0; r < 2 * NR; ++r) pv[r] = recP[r * 32], xv[r] = recX[r * 32];
-            if (*reinterpret_cast<const uint32_t *>(fac + 16) != 0u) {
-                const float2 al = *reinterpret_cast<const float2 *>(fac + 2 * t);
-                const float2 as = *reinterpret_cast<const float2 *>(fac + 8 + 2 * t);
-                l0 *= as.x, l1 *= as.y;
-                ps0 *= al.x, ps1 *= al.y;
-            }
+                for (int r = 0; r < 2 * NR; ++r) pv[r] = recP[r * 32], xv[r] = recX[r * 32];
+                if (*reinterpret_cast<const uint32_t *>(fac + 16) != 0u) {
+                    const float2 al = *reinterpret_cast<const float2 *>(fac + 2 * t);
+                    const float2 as = *reinterpret_cast<const float2 *>(fac + 8 + 2 * t);
+                    l0 *= as.x, l1 *= as.y;
+                    ps0 *= al.x, ps1 *= al.y;
+                }
 #pragma unroll
-            for (int r = 0; r < NR; ++r) {
-                l0 += pv[2 * r], l1 += pv[2 * r + 1];
-                ps0 += xv[2 * r], ps1 += xv[2 * r + 1];
+                for (int r = 0; r < NR; ++r) {
+                    l0 += pv[2 * r], l1 += pv[2 * r + 1];
+                    ps0 += xv[2 * r], ps1 += xv[2 * r + 1];
+                }
             }
             __syncwarp();
-            if (lane == 0) mbarArrive(&emptyBar[i % NSLOT]);
+            if (lane == 0) mbarArrive(&emptyBar[round & 1u]);
         }
 #pragma unroll
         for (int off = 4; off <= 16; off <<= 1) {
