@@ -383,6 +383,33 @@ def test_next_pool_hint_of_blocks_with_many_tiles(ctx, appends):
         assert all(torch.equal(a, b) for a, b in zip(*got))
 
 
+@pytest.mark.parametrize("nH,nKV,batch,ctx", [(28, 4, 1, 13900), (28, 4, 1, 20001), (28, 4, 1, 22000), (12, 2, 1, 9000), (12, 2, 1, 15900),
+                                              (40, 8, 1, 16000), (28, 4, 3, 12000), (28, 4, 6, 9100), (12, 2, 4, 16001)])
+def test_few_blocks_of_a_cluster_and_many_with_a_merge(nH, nKV, batch, ctx):
+    """On both sides of the line between a cluster per (sequence, kv head) and a merge launch, with host lengths and the new rows
+    handed in, against 64 bits over the dequantised rows.  What counts is that q is held to 2^(e - 21), |q| < 2^e <= 8: off by
+    2^-18 / sqrt(3) = 2.2e-6 an element, a score (K rows of 1.3 on average) by 2.9e-6, and with V rows that are independent the result
+    by as much of its norm on average.  Three and a half times that; an error of a block's weight or rows is thousands of times more."""
+    hd = 128
+    g = torch.Generator(device="cuda").manual_seed(ctx)
+    k8, v8 = (torch.randint(-127, 128, (batch * ctx, nKV, hd), dtype=torch.int8, device="cuda", generator=g) for _ in range(2))
+    ks, vs = (0.008 + 0.02 * torch.rand((batch * ctx, nKV), device="cuda", generator=g) for _ in range(2))
+    q = torch.randn((batch, nH, hd), device="cuda", generator=g)
+    rows = tuple(torch.randn((batch, nKV, hd), device="cuda", generator=g) for _ in range(2))
+    out = torch.full_like(q, float("nan"))
+    slots = ops.split_geometry(ctx, nH, hd)[1]
+    ops.decode_i8_batch(q, k8, v8, ks, vs, out, ops.workspace(batch, nH, hd, slots), None, batch, nH, nKV, hd, ctx, slots,
+                        rows_per_seq=ctx, append=rows)
+    torch.cuda.synchronize()
+    assert ops.device_status() == 0
+    for b in range(batch):
+        k, v = (x[b * ctx:(b + 1) * ctx].double() * s[b * ctx:(b + 1) * ctx].double()[..., None] for x, s in ((k8, ks), (v8, vs)))
+        for h in range(nH):
+            p = torch.softmax(k[:, h // (nH // nKV)] @ q[b, h].double() / math.sqrt(hd), 0)
+            want = p @ v[:, h // (nH // nKV)]
+            assert float((out[b, h].double() - want).norm() / want.norm()) < 1e-5
+
+
 def test_context_split_partials_merge_on_one_gpu():
     """The context-axis split as two 'ranks' on one device: each half of the rows yields
     partials-only output, the partials are concatenated as the all-gather would and merged."""

@@ -871,9 +871,13 @@ int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, c
     using Smem = DecodeTcSmem<2, 6>;
     // A cluster per (sequence, kv head) folds without partials and merge launch.  It is taken when all of them are resident
     // at once (16 blocks: 7, 8: 15, 4: 33, 2: 74, a block filling an SM) and their blocks, fewer than the merge form's, do not
-    // cost more than the launch: a tile more per block takes 0.3 us while latency is what bounds it.  7B shape, per layer in
-    // a graph: 8192 rows 8.4 -> 7.1 us, 8 sequences of 2048 / 8192 rows 10.7 -> 8.3 / 18.1 -> 16.1, 16384 rows 9.0 in
-    // either form.  With ragged device lengths the cluster also shares every sequence evenly among its blocks, where the
+    // cost more than the launch: a tile more per block takes 0.25 - 0.3 us while latency is what bounds it, and a fold over 16 blocks
+    // more than one over 8.  So up to five tiles more per block for 16 of them, nine for fewer.  Merge -> cluster, eight layers in
+    // stream order, 28 / 4 heads: 14000 rows (3 tiles a block -> 7) 69.4 -> 56.6 us, 16000 (4 -> 8) 67.0 -> 59.5, 20000 (5 -> 10) 70.0 ->
+    // 69.0, 30000 (7 -> 15) 79.9 -> 83.1; 12 / 2 heads: 9000 (1 -> 5) 64.0 -> 45.9, 20000 (3 -> 10, four layers of a session) 28.5 -> 32.8;
+    // 16 blocks for 2 sequences of 12 / 2: 20000 (5 -> 10) 68.7 -> 68.2, 30000 (7 -> 15) 79.0 -> 81.6.  Eight blocks: 40 / 8 at 16000 rows
+    // (7 -> 16) 89.3 -> 83.7, 3 sequences of 28 / 4 at 12000 / 20000 / 28000 (8 -> 12, 14 -> 20, 19 -> 28) 91.9 -> 76.8, 121.6 -> 105.9, 150.7 ->
+    // 139.4, 4 of 12 / 2 at 12000 (6 -> 12) 73.2 -> 74.1, the one that lost.  With ragged device lengths the cluster also shares every sequence evenly among its blocks, where the
     // merge form cuts chunks by the longest one.  There the line is 20 tiles per block of the longest sequence: cluster
     // against merge, 2 / 3 / 4 / 8 sequences of up to 6000 rows (6 - 12 tiles) 0.44 / 0.48 / 0.66 / 0.67 of the time, up to 20000
     // (20 tiles, 2 and 3 sequences) 0.83 and 0.87, up to 12000 (24 tiles, 4 and 8) 0.93 and 0.98, up to 32768 (32, 2 and 3) 1.15.
@@ -885,9 +889,9 @@ int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, c
     uint32_t cluster = 1;
     if (pl.chunksPerSeq > 1 && !d->partialsOnly && d->mergeTickets == nullptr) {
         const uint32_t tiles = (d->maxLen + kTcTile - 1) / kTcTile;
-        const uint32_t most = d->lens == nullptr || d->batch == 1 ? pl.chunkTokens / kTcTile + 3u : 20u;  // tiles per block
         for (uint32_t lg = 4; lg >= 1 && cluster == 1; --lg) {
-            const uint32_t n = 1u << lg;
+            const uint32_t n = 1u << lg, more = n == 16u ? 5u : 9u;
+            const uint32_t most = d->lens == nullptr || d->batch == 1 ? pl.chunkTokens / kTcTile + more : 20u;  // tiles per block
             if (n / 2u >= tiles || limits[lg] < d->nKV * d->batch || (tiles + n - 1u) / n > most) continue;
             cluster = n;
             pl.chunksPerSeq = n;
