@@ -50,3 +50,29 @@ def test_fp16_decode(nH, nKV, hd, pos):
         far.append(_far(q, k, v, out, pos))
     # a tile's chain is two products, not twelve: what is left is the rounding of scores, weights and sums
     assert sum(far) / 3 < 4e-7
+
+
+@pytest.mark.parametrize("dtype,nH,nKV,hd,pos", [(torch.float16, 28, 4, 128, 9999), (torch.float16, 28, 4, 128, 16000), (torch.float16, 40, 8, 128, 4000),
+                                                 (torch.float16, 40, 8, 128, 10000), (torch.float16, 14, 2, 64, 5000), (torch.float16, 8, 4, 64, 14000),
+                                                 (torch.float32, 14, 2, 64, 3000), (torch.float32, 8, 4, 64, 5500)])
+def test_decode_on_both_sides_of_the_merge(dtype, nH, nKV, hd, pos):
+    """One token where a cluster of blocks folds a kv head's rows or a merge launch does.  (f32: up to sixteen tiles share a warp's sums, 1.3e-6 at
+    most as measured; the bound is three times what a chain of 32 products drops, 32 x 6e-8.)"""
+    g = torch.Generator(device="cuda").manual_seed(pos)
+    q = torch.randn((1, nH, hd), device="cuda", generator=g)
+    k, v = (torch.randn((pos + 1, nKV, hd), device="cuda", generator=g).to(dtype) for _ in range(2))
+    out = torch.empty_like(q)
+    ops.decode_kv(q, k, v, out, ops.workspace(1, nH, hd, 256), 1, nH, nKV, hd, pos, 256)
+    assert _far(q, k, v, out, pos) < (BOUND if dtype == torch.float16 else 6e-6)
+
+
+@pytest.mark.parametrize("dtype,nH,nKV,hd,pos", [(torch.float16, 40, 8, 128, 6500), (torch.float16, 28, 4, 128, 24000), (torch.float32, 8, 2, 128, 9000)])
+def test_decode_without_partial_buffers(dtype, nH, nKV, hd, pos):
+    """... is one cluster per kv head, in turns where they are not all resident, whatever the call with buffers takes.  Bounds as above; f32 rows
+    of 16 blocks are up to 36 tiles a warp: 72 products in a sum."""
+    g = torch.Generator(device="cuda").manual_seed(pos)
+    q = torch.randn((1, nH, hd), device="cuda", generator=g)
+    k, v = (torch.randn((pos + 1, nKV, hd), device="cuda", generator=g).to(dtype) for _ in range(2))
+    out = torch.empty_like(q)
+    ops.decode_kv(q, k, v, out, (None, None, None), 1, nH, nKV, hd, pos, 256)
+    assert _far(q, k, v, out, pos) < (BOUND if dtype == torch.float16 else 72 * 6e-8 * 3)

@@ -70,7 +70,11 @@ struct ClusterCost {
 
 // The fewest-microseconds split among one cluster of 1 - 16 blocks per kv head and n blocks with a merge behind them:
 // the tiles a warp has to do one after the other, the tiles of an SM or the HBM stream, whichever takes longest, plus
-// what the fold costs (0.5 us in a cluster, 1.7 us as a merge launch and a little more from the 33rd partial on).
+// what the fold costs (0.5 us in a cluster, 2.5 us as a merge launch and a little more from the 33rd partial on), and 3 us for what a
+// block does ahead of its first tile and behind its last one where clusters take turns.  (With 1.7 us for the merge and nothing for
+// turns, per layer -> like this: fp16, 28 / 4 / 128 at 12000 rows 10.5 -> 8.9 us, 12 / 2 / 128 at 4500 6.7 -> 6.0, 40 / 8 / 128 at 5500 / 9000 10.3 /
+// 12.6 -> 8.4 / 11.0, 14 / 2 / 64 at 7000 6.7 -> 5.7; f32, 14 / 2 / 64 at 2500 7.6 -> 6.4.  With 3.4 us for the merge: 28 / 4 / 128 at 20000
+// 12.9 -> 11.9, 8 / 2 / 128 at 11000 7.6 -> 8.4.)
 inline ClusterPlan searchClusterPlan(uint32_t nKV, uint32_t maxLen, uint32_t slots, bool needPartials, const ClusterCost &c) {
     const uint32_t tiles = maxLen == 0 ? 1u : (maxLen + 15) / 16, sms = static_cast<uint32_t>(numSMs());
     const float stream = static_cast<float>(tiles) * static_cast<float>(nKV) * static_cast<float>(c.tileBytes) * (1.0f / 5.6e6f);
@@ -88,19 +92,19 @@ inline ClusterPlan searchClusterPlan(uint32_t nKV, uint32_t maxLen, uint32_t slo
         best.clusters = n;
         best.chunkTokens = (tiles + n * size - 1) / (n * size) * 16;
     };
-    const float merge = needPartials ? 1.7f : 0.0f;
+    const float merge = needPartials ? 2.5f : 0.0f;
     for (uint32_t lg = 0; lg < 5; ++lg) {
         const uint32_t size = 1u << lg;
         if (c.maxClusters[lg] == 0 || (lg > 0 && size / 2 >= tiles)) continue;
-        consider(size, 1, workUs((tiles + size - 1) / size, size * nKV, (nKV + c.maxClusters[lg] - 1) / c.maxClusters[lg]) +
-                                  (lg > 0 ? 0.45f + 0.03f * lg : 0.0f) + merge);
+        const uint32_t turns = (nKV + c.maxClusters[lg] - 1) / c.maxClusters[lg];
+        consider(size, 1, workUs((tiles + size - 1) / size, size * nKV, turns) + 3.0f * (turns - 1u) + (lg > 0 ? 0.45f + 0.03f * lg : 0.0f) + merge);
     }
     uint32_t most = c.maxClusters[0] / nKV;  // blocks per kv head in one wave
     most = most > slots ? slots : most;
     for (uint32_t n = 2; n <= most && n <= tiles; ++n) {
         const uint32_t perBlock = (tiles + n - 1) / n;
         if ((tiles + perBlock - 1) / perBlock != n) continue;  // the last blocks would have no rows
-        consider(1, n, workUs(perBlock, n * nKV, 1) + 1.7f + (n > 32 ? 0.035f * (n - 32) : 0.0f));
+        consider(1, n, workUs(perBlock, n * nKV, 1) + 2.5f + (n > 32 ? 0.035f * (n - 32) : 0.0f));
     }
     return best;
 }
@@ -528,12 +532,14 @@ int launchKvDecode(ClusterSetup &setup, K kern, uint32_t threads, size_t smem, u
     if (rc != TC_OK) return rc;
     ClusterCost cost = {tileUs, smTileUs, warps, tileBytes, {}};
     memcpy(cost.maxClusters, limits, sizeof(cost.maxClusters));
-    const ClusterPlan pl = planCluster(hd / 64u + (prm.kvHalf ? 4u : 0u), prm.nKV, prm.lenHost, prm.numChunks,
+    // (a caller without partial buffers has one cluster per kv head, wherever the line to the merge lies)
+    const bool partials = prm.pAcc && prm.pM && prm.pL;
+    const ClusterPlan pl = planCluster(hd / 64u + (prm.kvHalf ? 4u : 0u), prm.nKV, prm.lenHost, partials ? prm.numChunks : 1u,
                                        q81Out != nullptr, cost);
     prm.directOut = pl.clusters == 1 && q81Out == nullptr ? 1 : 0;
     prm.chunkTokens = pl.chunkTokens;
     if (!prm.directOut)
-        TC_REQUIRE(prm.pAcc && prm.pM && prm.pL, TC_EWORKSPACE, "tc_attn_decode_kv: partial buffers are required");
+        TC_REQUIRE(partials, TC_EWORKSPACE, "tc_attn_decode_kv: partial buffers are required");
     // several clusters read q: the merge writes its rotation behind them
     QRotation rot = {nullptr, nullptr, nullptr, prm.lenHost};
     if (prm.tok.qRot != nullptr && !prm.directOut) {

@@ -405,8 +405,10 @@ template <int HD, int NW, int SLOTS, int BPS>
 static int decodeKv16Hd(const DecodeKvParams &prm, uint8_t *q81Out, cudaStream_t st) {
     using L = DecodeKv16Smem<HD, NW, SLOTS, false>;
     static ClusterSetup setup;
+    // (head_dim 64, 0.73 -> 0.61 with two slots: 14 / 2 at 9000 rows 27.2 -> 24.8 us for four layers, 8 / 4 at 12000 33.5 -> 27.7; with
+    // four slots 14 / 2 at 45000 rows 18.6 -> 19.3 for two)
     return launchKvDecode(setup, decodeKv16Kernel<HD, NW, SLOTS, BPS, false>, NW * 32, L::kTotal, HD, NW, 2 * L::kTileBytes,
-                          HD == 128 ? 0.87f : 0.73f, HD == 128 ? 0.12f : 0.08f, prm, q81Out, st);
+                          HD == 128 ? 0.87f : SLOTS == 4 ? 0.73f : 0.61f, HD == 128 ? 0.12f : 0.08f, prm, q81Out, st);
 }
 
 // Both are called from decode_kv.cu when kvHalf is set; arguments were validated there.
