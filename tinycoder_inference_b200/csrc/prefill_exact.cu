@@ -11,10 +11,11 @@
 //
 // What bounds it: the issue slots.  With 8 query rows at a time (the causal form of the decode kernels, which stays for
 // few rows behind a long prefix: prefillExactWins below) every warp takes K and V apart for itself.  Here a block of 32 query rows of
-// one q head does that once per stage, into planes in shared memory: loader warps (loads, the rows' exponents, the pairs -- 26
-// instructions per four elements) fill one buffer while the computing warps, 16 rows x TG tokens each, work on the other.  Done by the
+// one q head does that once per stage, into planes in shared memory: loader warps (loads, the rows' exponents, the pairs)
+// fill one buffer while the computing warps, 16 rows x TG tokens each, work on the other.  Done by the
 // computing warps between two barriers, as tf32 planes, a stage of 128 tokens at head_dim 64 took 3.9 us (1.6 of them products); with
-// four loader warps and 48 instructions 3.3, with eight of 26 2.0.  The
+// four loader warps and 9900 warp instructions in all 3.3, with eight and 8700 2.2 (half of the issue slots, a third of the
+// tensor pipe).  The
 // four token groups of a block take their share of every stage (a short prompt is a chain of stages, not a matter of
 // bytes) and are put together at the end.  The late rows of all heads come first, so that what starts last is short.
 // Measured, tf32 planes -> this: 512 rows of 14 / 2 / 64 17.7 -> 12.5 us, 512 behind 3000 200 -> 113; 512 rows of 28 / 4 / 128

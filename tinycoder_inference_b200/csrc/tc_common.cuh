@@ -63,7 +63,7 @@ int getTensorMap(const TensorMapKey &key, CUtensorMap *out);
 
 // Launch under programmatic dependent launch: the grid may be scheduled while the one in front of it drains, so
 // the kernel has to call gridDepWait() before it touches anything that grid may have written or may still read --
-// every kernel launched through here does so first thing, but for the int8 decode at head_dim 128 under
+// every kernel launched through here does so first thing (hints towards L2 may go ahead of it), but for the int8 decode at head_dim 128 under
 // TC_DECODE_PDL, which requests rows of its pool that the caller calls old (prefetchRows) ahead of it.  Where the others
 // call gridDepLaunch() decides what such a launch may find unfinished:
 //   * after the wait, so that the kernels ahead of theirs are complete;
