@@ -410,6 +410,31 @@ def test_few_blocks_of_a_cluster_and_many_with_a_merge(nH, nKV, batch, ctx):
             assert float((out[b, h].double() - want).norm() / want.norm()) < 1e-5
 
 
+@pytest.mark.parametrize("nH,nKV,lens", [(28, 4, (12000, 11871, 130, 5000)), (28, 4, (12000, 1, 7000, 127, 128, 129, 3000, 11999)),
+                                         (40, 8, (12000, 300)), (12, 2, (26000, 64, 25999, 128))])
+def test_ragged_sequences_in_clusters_of_few_blocks(nH, nKV, lens):
+    """Device lengths at 24 and 26 tiles per block of the longest sequence, where clusters of 2 - 8 blocks take over from the merge, and sequences
+    that leave blocks of a cluster without tiles: each like a call of its own, up to the f32 roundings of another fold."""
+    hd, batch, total, most = 128, len(lens), sum(lens), max(lens)
+    g = torch.Generator(device="cuda").manual_seed(total)
+    k8, v8 = (torch.randint(-127, 128, (total, nKV, hd), dtype=torch.int8, device="cuda", generator=g) for _ in range(2))
+    ks, vs = (0.008 + 0.02 * torch.rand((total, nKV), device="cuda", generator=g) for _ in range(2))
+    q = torch.randn((batch, nH, hd), device="cuda", generator=g)
+    at = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    base = torch.cumsum(at.long(), 0) - at
+    slots = min(64, ops.split_geometry(most, nH, hd)[1])
+    out = torch.full_like(q, float("nan"))
+    ops.decode_i8_batch(q, k8, v8, ks, vs, out, ops.workspace(batch, nH, hd, slots), at, batch, nH, nKV, hd, most, slots, row_base=base)
+    ws = ops.workspace(1, nH, hd, 64)
+    for b, n in enumerate(lens):
+        a = int(base[b])
+        alone = torch.empty_like(q[:1])
+        ops.decode_i8(q[b:b + 1], k8[a:a + n], v8[a:a + n], ks[a:a + n], vs[a:a + n], alone, ws, nH, nKV, hd, n - 1, 64)
+        # (a tile's reference point may differ: the 24-bit steps of p * sv with it, 2^-24 a token at most)
+        assert float((out[b] - alone[0]).norm() / alone.norm()) < 4e-6
+    assert ops.device_status() == 0
+
+
 def test_context_split_partials_merge_on_one_gpu():
     """The context-axis split as two 'ranks' on one device: each half of the rows yields
     partials-only output, the partials are concatenated as the all-gather would and merged."""

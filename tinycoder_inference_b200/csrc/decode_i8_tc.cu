@@ -878,9 +878,10 @@ int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, c
     // 16 blocks for 2 sequences of 12 / 2: 20000 (5 -> 10) 68.7 -> 68.2, 30000 (7 -> 15) 79.0 -> 81.6.  Eight blocks: 40 / 8 at 16000 rows
     // (7 -> 16) 89.3 -> 83.7, 3 sequences of 28 / 4 at 12000 / 20000 / 28000 (8 -> 12, 14 -> 20, 19 -> 28) 91.9 -> 76.8, 121.6 -> 105.9, 150.7 ->
     // 139.4, 4 of 12 / 2 at 12000 (6 -> 12) 73.2 -> 74.1, the one that lost.  With ragged device lengths the cluster also shares every sequence evenly among its blocks, where the
-    // merge form cuts chunks by the longest one.  There the line is 20 tiles per block of the longest sequence: cluster
+    // merge form cuts chunks by the longest one.  There the line is 20 tiles per block of the longest sequence for 16 blocks: cluster
     // against merge, 2 / 3 / 4 / 8 sequences of up to 6000 rows (6 - 12 tiles) 0.44 / 0.48 / 0.66 / 0.67 of the time, up to 20000
-    // (20 tiles, 2 and 3 sequences) 0.83 and 0.87, up to 12000 (24 tiles, 4 and 8) 0.93 and 0.98, up to 32768 (32, 2 and 3) 1.15.
+    // (20 tiles, 2 and 3 sequences) 0.83 and 0.87, up to 32768 (32, 2 and 3) 1.15; and 26 for fewer: 2 and 3 of up to 26000 (26 tiles) 0.83 and 0.82,
+    // 4 / 5 / 6 / 8 of up to 12000 (24) 0.92 / 0.94 / 0.96 / 0.97, 12 and 16 of up to 6000 (24) 0.91 and 0.92, 4 / 5 / 6 / 8 of up to 16000 (32) 1.19 / 1.19 / 1.09 / 1.05.
     static ClusterSetup setup;
     const uint32_t *limits = nullptr;
     int rc = setupCluster(setup, decodeI8TcKernel<2, 6, 8, true, TcFold::kCluster>, Smem::kThreads, Smem::kTotal, &limits);
@@ -891,7 +892,7 @@ int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, c
         const uint32_t tiles = (d->maxLen + kTcTile - 1) / kTcTile;
         for (uint32_t lg = 4; lg >= 1 && cluster == 1; --lg) {
             const uint32_t n = 1u << lg, more = n == 16u ? 5u : 9u;
-            const uint32_t most = d->lens == nullptr || d->batch == 1 ? pl.chunkTokens / kTcTile + more : 20u;  // tiles per block
+            const uint32_t most = d->lens == nullptr || d->batch == 1 ? pl.chunkTokens / kTcTile + more : n == 16u ? 20u : 26u;  // tiles per block
             if (n / 2u >= tiles || limits[lg] < d->nKV * d->batch || (tiles + n - 1u) / n > most) continue;
             cluster = n;
             pl.chunksPerSeq = n;
