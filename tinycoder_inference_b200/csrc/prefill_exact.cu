@@ -365,18 +365,33 @@ __global__ void __launch_bounds__(ExactShape<HD>::kThreads, 1) prefillExactKerne
         namedBarSync(kFullV + buf, kAll);
         if (active) {
             // ---- O += P V, 16 tokens at a time: the accumulator layout of the scores is the A operand's.  The probabilities take the
-            // scales of V's rows along, the group's largest one out of them ----
+            // scales of V's rows along, and every query row a power of two of its own, out of its largest product: with one for the group a
+            // row of V that is masked, or weighs nothing, pushed the probabilities of the others out of the pairs' range ----
             const float *sv = sf + S::kScaleV + buf * S::kStage + nh * TG;
-            const uint32_t E = __reduce_max_sync(0xffffffffu, __float_as_uint(sv[lane % TG]));
-            const float in = exactScale(E), out = __uint_as_float(E) * 3.7252902984619140625e-9f;  // 2^(14 - E), 2^(E - 28)
-            uint32_t ph[NT / 2][4], pl[NT / 2][4];
+            float top0 = 0.0f, top1 = 0.0f;
 #pragma unroll
             for (int n = 0; n < NT; ++n) {
                 const float2 w = *reinterpret_cast<const float2 *>(sv + 8 * n + 2 * t);
-                const float w0 = w.x * in, w1 = w.y * in;
-                splitPair(s[n][0] * w0, s[n][1] * w1, ph[n / 2][n % 2 * 2], pl[n / 2][n % 2 * 2]);
-                splitPair(s[n][2] * w0, s[n][3] * w1, ph[n / 2][n % 2 * 2 + 1], pl[n / 2][n % 2 * 2 + 1]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) s[n][i] *= i & 1 ? w.y : w.x;
+                top0 = fmaxf(top0, fmaxf(s[n][0], s[n][1]));
+                top1 = fmaxf(top1, fmaxf(s[n][2], s[n][3]));
             }
+#pragma unroll
+            for (int off = 1; off <= 2; off <<= 1) {
+                top0 = fmaxf(top0, __shfl_xor_sync(0xffffffffu, top0, off));
+                top1 = fmaxf(top1, __shfl_xor_sync(0xffffffffu, top1, off));
+            }
+            const uint32_t e0 = max(__float_as_uint(top0) & 0x7f800000u, 15u << 23), e1 = max(__float_as_uint(top1) & 0x7f800000u, 15u << 23);
+            const float in0 = exactScale(e0), in1 = exactScale(e1);
+            uint32_t ph[NT / 2][4], pl[NT / 2][4];
+#pragma unroll
+            for (int n = 0; n < NT; ++n) {
+                splitPair(s[n][0] * in0, s[n][1] * in0, ph[n / 2][n % 2 * 2], pl[n / 2][n % 2 * 2]);
+                splitPair(s[n][2] * in1, s[n][3] * in1, ph[n / 2][n % 2 * 2 + 1], pl[n / 2][n % 2 * 2 + 1]);
+            }
+            constexpr float kPlanes = 3.7252902984619140625e-9f;  // 2^-28: 2^14 in the planes of V, and in the pairs of p
+            const float out0 = __uint_as_float(e0) * kPlanes, out1 = __uint_as_float(e1) * kPlanes;
             constexpr int DB = HD > 128 ? 1 : 2;  // pairs of dim tiles at a time, their chains alternating
 #pragma unroll
             for (int d0 = 0; d0 < HD / 16; d0 += DB) {
@@ -403,7 +418,7 @@ __global__ void __launch_bounds__(ExactShape<HD>::kThreads, 1) prefillExactKerne
 #pragma unroll
                 for (int d = 0; d < 2 * DB; ++d)
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) o[2 * d0 + d][i] = fmaf(sum[d][i] + cross[d][i], out, o[2 * d0 + d][i]);
+                    for (int i = 0; i < 4; ++i) o[2 * d0 + d][i] = fmaf(sum[d][i] + cross[d][i], i & 2 ? out1 : out0, o[2 * d0 + d][i]);
             }
             __syncwarp();
         }
