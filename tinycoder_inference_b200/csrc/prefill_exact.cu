@@ -5,22 +5,26 @@
 // (include/gpu/GpuAttentionKernels.hpp:211-272, 537-599; include/gpu/GpuQwen35Kernels.hpp:2437-2492): row s attends
 // cache rows [0, pos + s], score = dot(q, k) * invSqrt, online softmax with exp2, out = sum p v / sum p.
 //
-// Over the f32 store every operand is an fp16 pair, x = 2^e (hi + lo) with a power of two per row, and a product is three on the
+// Over the f32 store every operand is an fp16 pair, x = 2^e (hi + 2^-11 lo) with a power of two for the rows that a warp takes apart at a
+// time (16, 8, 2 at head_dim 64, 128, 256), and a product is three on the
 // tensor cores (mma.sync.m16n8k16: hi*hi + lo*hi + hi*lo, f32 accumulation): 22 bits of every factor like 3xTF32, at half the
-// products and half the shared memory.  A row's scale is its own: K's goes into the score, V's into the probability.
+// products and half the shared memory.  K's power goes into the score, V's into the probability, which has one of its own per query row.
+// The pairs hold 22 bits over 2^29; f32 has no such limit.  So the warps that make them look for numbers outside it, and where those can count --
+// outliers of 10^8 in a dim, rows of 2^40 next to others, infinities -- the blocks concerned go on in f32 (the second
+// loop of the kernel): right, and some seven times slower (512 rows of 14 / 2 / 64 13.7 -> 78 - 87 us).
 //
-// What bounds it: the issue slots.  With 8 query rows at a time (the causal form of the decode kernels, which stays for
-// few rows behind a long prefix: prefillExactWins below) every warp takes K and V apart for itself.  Here a block of 32 query rows of
-// one q head does that once per stage, into planes in shared memory: loader warps (loads, the rows' exponents, the pairs)
+// What bounds it: shared memory and mma.sync in turn, and the loaders' instructions.  With 8 query rows at a time (the causal form of the decode
+// kernels, which stays for few rows behind a long prefix: prefillExactWins below) every warp takes K and V apart for itself.  Here a block
+// of 32 query rows of one q head does that once per stage, into planes in shared memory: loader warps (loads, exponents, the pairs)
 // fill one buffer while the computing warps, 16 rows x TG tokens each, work on the other.  Done by the
-// computing warps between two barriers, as tf32 planes, a stage of 128 tokens at head_dim 64 took 3.9 us (1.6 of them products); with
-// four loader warps and 9900 warp instructions in all 3.3, with eight and 8700 2.2 (half of the issue slots, a third of the
-// tensor pipe).  The
+// computing warps between two barriers, as tf32 planes, a stage of 128 tokens at head_dim 64 took 3.9 us (1.6 of them products);
+// like this 2.3.  The
 // four token groups of a block take their share of every stage (a short prompt is a chain of stages, not a matter of
 // bytes) and are put together at the end.  The late rows of all heads come first, so that what starts last is short.
-// Measured, tf32 planes -> this: 512 rows of 14 / 2 / 64 17.7 -> 12.5 us, 512 behind 3000 200 -> 113; 512 rows of 28 / 4 / 128
-// 59 -> 41, 512 behind 512 178 -> 116; 512 rows of 16 / 2 / 256 75 -> 46, 512 behind 512 215 -> 120.  fp16 store, 8-row form -> this: 100
-// rows of 28 / 4 / 128 15.0 -> 6.4 us, 512 behind 512 107 -> 71, 2000 rows of 8 / 4 / 64 81 -> 40.
+// Measured, tf32 planes -> this: 512 rows of 14 / 2 / 64 17.7 -> 13.7 us, 512 behind 3000 200 -> 122; 512 rows of 28 / 4 / 128
+// 59 -> 43, 512 behind 512 178 -> 123; 512 rows of 16 / 2 / 256 75 -> 44, 512 behind 512 215 -> 114.  fp16 store, 8-row form -> this: 100
+// rows of 28 / 4 / 128 15.0 -> 6.4 us, 512 behind 512 107 -> 71, 2000 rows of 8 / 4 / 64 81 -> 40.  (The look at the range and the powers per
+// query row cost 6 - 10 % at head_dim 64 and 3 - 6 at 128; a power per row of K and V instead of one per unit as much again.)
 //
 // What keeps it exact: a tensor-core product drops the bits of a running sum that do not fit, and those losses add up
 // along a chain.  So a stage's products are summed by themselves, the small terms apart (f32) or first (fp16), and added to O in
@@ -48,49 +52,106 @@ static constexpr uint32_t kExactThreads = kExactWarps * 32, kFoldBar = 1;  // (n
 template <int HD>
 struct ExactShape {
     static constexpr int TG = HD == 64 ? 32 : 16, kRows = kExactRows, kStage = kExactNH * TG, NB = HD > 128 ? 1 : 2;
-    static constexpr int kLoaders = HD > 128 ? 4 : 8, kThreads = (kExactWarps + kLoaders) * 32;
+    static constexpr int kLoaders = 8, kThreads = (kExactWarps + kLoaders) * 32;
+    // registers of a thread, and of a loader's: together what the launch has (512 x 128, 384 x 168)
+    static constexpr int kRegs = HD > 128 ? 192 : 144, kLoaderRegs = HD > 128 ? 64 : 112;
+    static_assert((kExactWarps * kRegs + kLoaders * kLoaderRegs) * 32 <= kThreads * 128, "registers of the launch");
+    static constexpr int kParts = HD > 128 ? 4 : 1;  // a loader takes its rows of a stage in so many parts; kUnit: rows of one
+    static constexpr int kUnit = kStage / (kLoaders * kParts);
     static constexpr int kLd = HD + 8;  // halves per row of a plane: eight rows hit different banks
     static constexpr int kPlane = kStage * kLd;
     // halves: planes (hi, lo) of q [kRows][kLd], of K [NB][kStage][kLd], of V; then floats: scales of q's, K's and V's rows
     static constexpr int kQ = 0, kK = 2 * kRows * kLd, kV = kK + 2 * NB * kPlane, kHalves = kV + 2 * NB * kPlane;
-    static constexpr int kScaleQ = 0, kScaleK = kRows, kScaleV = kScaleK + NB * kStage, kFloats = kScaleV + NB * kStage;
+    static constexpr int kScaleQ = 0, kScaleK = kRows, kScaleV = kScaleK + NB * kStage;
+    static constexpr int kProb = kScaleV + NB * kStage;  // a warp's probabilities
+    static constexpr int kFloats = kProb + kExactWarps * 16 * TG;
     static constexpr size_t kOperands = 2 * static_cast<size_t>(kHalves) + 4 * kFloats;
     static constexpr size_t kFold = 4 * static_cast<size_t>(kExactNH * kRows * (HD + 4));  // per group: O and (m, l) of every row
     static constexpr size_t kBytes = (kOperands > kFold ? kOperands : kFold) + 16;
     static_assert(kBytes <= 227 * 1024, "shared memory of an SM");
-    static_assert(kHalves % 8 == 0, "16-byte accesses");
+    static_assert(kHalves % 8 == 0 && kProb % 4 == 0, "16-byte accesses");
 };
 
-// two numbers as fp16 hi + lo pairs (22 significant bits)
+// Two numbers as fp16 pairs hi + 2^-11 lo: 22 significant bits from 2^-14 on, 2^-36 off below it.  (Without the factor lo is out of normal
+// numbers from 2^-3 on down.)
+constexpr float kLoScale = 4.8828125e-4f;
 __device__ __forceinline__ void splitPair(float a, float b, uint32_t &hi, uint32_t &lo) {
     hi = packHalf2(a, b);
     const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&hi));
-    const float2 r = __ffma2_rn(f, make_float2(-1.0f, -1.0f), make_float2(a, b));
+    const float2 r = __fmul2_rn(__ffma2_rn(f, make_float2(-1.0f, -1.0f), make_float2(a, b)), make_float2(2048.0f, 2048.0f));
     lo = packHalf2(r.x, r.y);
 }
-// Rows in powers of two: a row whose largest magnitude is in [2^e, 2^(e + 1)) is scaled into [2^14, 2^15), where the pairs keep 22 bits of
-// every element down to 2^-17 of it, and 2^-39 of it of the smaller ones.  `x`: N pieces of such rows by the lanes of a warp; e gets
-// the bits of 2^e of each (the rows that a warp holds at once share theirs).  Infinities and NaN stay out of it: they stay what they are
-// in the planes, and leave the other elements their scale.
+constexpr float kLeast = 6.103515625e-5f;  // 2^-14
+// Rows in powers of two: `x`, the rows that a warp has in its hands (a unit), share one; scaled by it, their largest element is in
+// [2^14, 2^15), and the pairs keep 22 bits of everything down to 2^-29 of that one and 2^-51 of it of what is smaller.  The bits of 2^e for a
+// largest element in [2^e, 2^(e + 1)); infinities make it one.
 template <int N, int NV>
-__device__ __forceinline__ void rowExponents(const float4 (&x)[N][NV], uint32_t (&e)[N]) {
-    auto largest = [&](int i, auto of) {
-        float m = 0.0f;
+__device__ __forceinline__ uint32_t unitExponent(const float4 (&x)[N][NV]) {
+    float m = 0.0f;
 #pragma unroll
-        for (int v = 0; v < NV; ++v) m = fmaxf(fmaxf(m, fmaxf(of(x[i][v].x), of(x[i][v].y))), fmaxf(of(x[i][v].z), of(x[i][v].w)));
-        return __reduce_max_sync(0xffffffffu, __float_as_uint(m));
-    };
-    uint32_t top = 0;
+    for (int i = 0; i < N; ++i)
 #pragma unroll
-    for (int i = 0; i < N; ++i) e[i] = largest(i, [](float a) { return fabsf(a); }), top = max(top, e[i]);
-    if (top >= 0x7f800000u) {  // warp-uniform
-#pragma unroll
-        for (int i = 0; i < N; ++i) e[i] = largest(i, [](float a) { return fabsf(a) < INFINITY ? fabsf(a) : 0.0f; });
-    }
-#pragma unroll
-    for (int i = 0; i < N; ++i) e[i] = max(e[i] & 0x7f800000u, 15u << 23);
+        for (int v = 0; v < NV; ++v) m = fmaxf(fmaxf(m, fmaxf(fabsf(x[i][v].x), fabsf(x[i][v].y))), fmaxf(fabsf(x[i][v].z), fabsf(x[i][v].w)));
+    return max(__reduce_max_sync(0xffffffffu, __float_as_uint(m)) & 0x7f800000u, 15u << 23);
 }
 __device__ __forceinline__ float exactScale(uint32_t e) { return __uint_as_float((268u << 23) - e); }
+
+// Where that is not enough: numbers in a unit below 2^-29 of its largest whose products with large ones elsewhere, or whose place in
+// a dim of their own, let them count.  (One dim of 1e10 is no measure of the others.)  `low` follows the smallest |hi| that a lane has placed, NaN
+// where one is; a unit with less than kLeast is looked at once more (inDoubt), for whether that was more than zeros (anySmall), and how many (isSmall).
+__device__ __forceinline__ uint32_t leastOf(uint32_t a, uint32_t b) {  // magnitudes, the signs multiplied
+    uint32_t r;
+    asm("min.NaN.xorsign.abs.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ bool inDoubt(uint32_t low) {  // (warp-uniform)
+    return __any_sync(0xffffffffu, !__hbge2(__habs2(*reinterpret_cast<const __half2 *>(&low)), __floats2half2_rn(kLeast, kLeast)));
+}
+template <int N, int NV>
+__device__ __forceinline__ bool anySmall(const float4 (&x)[N][NV], uint32_t e, uint32_t low) {  // (warp-uniform)
+    uint32_t m = 0xffffffffu;  // of what is not 0, the bits of the smallest magnitude, times two less one
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+        for (int v = 0; v < NV; ++v)
+            m = min(min(min(m, 2u * __float_as_uint(x[i][v].x) - 1u), min(2u * __float_as_uint(x[i][v].y) - 1u, 2u * __float_as_uint(x[i][v].z) - 1u)),
+                    2u * __float_as_uint(x[i][v].w) - 1u);
+    const uint32_t least = max(max(e, 28u << 23) - (28u << 23), 1u);  // kLeast in the planes
+    return __any_sync(0xffffffffu, m < 2u * least - 1u || (low & 0x7fffu) > 0x7c00u || (low >> 16 & 0x7fffu) > 0x7c00u);
+}
+__device__ __forceinline__ uint32_t isSmall(float x, float scale) {  // (one that is NaN: as many as make a unit's worth)
+    return x == 0.0f || fabsf(x) * scale >= kLeast ? 0u : (x == x ? 1u : 16u);
+}
+__device__ __forceinline__ uint32_t isSmall(const float4 &x, float scale) {
+    return isSmall(x.x, scale) + isSmall(x.y, scale) + isSmall(x.z, scale) + isSmall(x.w, scale);
+}
+template <int N, int NV>
+__device__ __forceinline__ bool zeroDim(const float4 (&x)[N][NV]) {  // a dim that is 0 in all rows that a lane has of it (warp-uniform)
+    bool zero = false;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        float4 m = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+            m.x = fmaxf(m.x, fabsf(x[i][v].x)), m.y = fmaxf(m.y, fabsf(x[i][v].y)), m.z = fmaxf(m.z, fabsf(x[i][v].z)), m.w = fmaxf(m.w, fabsf(x[i][v].w));
+        zero = zero || m.x == 0.0f || m.y == 0.0f || m.z == 0.0f || m.w == 0.0f;
+    }
+    return __any_sync(0xffffffffu, zero);
+}
+// What a unit's scale says besides, for the warps that compute.  q, K: negative, it has small ones, which count when the score of
+// such rows can be large (kSmallCount: HD x 2 x 2^15 x 2^-36 of that is 2^-24).  V: minus infinity, it has as many as it has rows: a
+// dim of its own (fewer stay within 2^-51 of the unit's largest; N(0, 1) has one in 2 x 10^8); negative, a dim of it is zero, of which
+// its weight says nothing: that counts where its scale is far from the others' (kLongScales).
+constexpr float kSmallCount = 2.44140625e-4f, kMostScale = 1.2676506e30f;  // 2^-12; 2^100: a product with more might not fit
+constexpr uint32_t kHugeWord = 240u << 23;   // a scale of q or K of 2^127 or an infinity
+constexpr uint32_t kLongScales = 6u << 23;  // 2^6 of the first one's
+
+// (what is worked out from it stays in the branch that asks for it, and out of the registers of the loop around)
+__device__ __forceinline__ uint32_t opaqueZero() {
+    uint32_t z;
+    asm volatile("mov.u32 %0, 0;" : "=r"(z));
+    return z;
+}
 
 // The token groups of a row put together: every warp's O (unnormalised), row maxima (log2 units) and row sums through
 // shared memory, then out.  `out` is row 0 of the block, `ld` floats from row to row.
@@ -161,115 +222,129 @@ __global__ void __launch_bounds__(ExactShape<HD>::kThreads, 1) prefillExactKerne
     const uint32_t len = static_cast<uint32_t>(wanted < p.totalRows ? wanted : p.totalRows);  // (a device position past the store)
     const uint32_t nStages = (len + S::kStage - 1) / S::kStage;
     const uint32_t unit = HD < 128 ? lane % 16u : lane, sub = HD < 128 ? lane / 16u : 0u;  // this lane's float4 of a row, and which row
-    // hi and lo parts of a piece of a row, into row r of the planes at `plane` (`lo` halves apart)
-    auto place = [&](__half *plane, uint32_t lo, const float4 (&x)[NV], float scale, uint32_t r) {
+    // hi and lo parts of a piece of a row, into row r of the planes at `plane` (`lo` halves apart); `low` follows the smallest |hi|
+    auto place = [&](__half *plane, uint32_t lo, const float4 (&x)[NV], float scale, uint32_t r, uint32_t &low) {
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
             uint2 h, l;
             const float2 s2 = make_float2(scale, scale), a = __fmul2_rn(make_float2(x[v].x, x[v].y), s2), b = __fmul2_rn(make_float2(x[v].z, x[v].w), s2);
             splitPair(a.x, a.y, h.x, l.x);
             splitPair(b.x, b.y, h.y, l.y);
+            low = leastOf(low, leastOf(h.x, h.y));
             __half *at = plane + r * LD + (unit + 32u * v) * 4u;
             *reinterpret_cast<uint2 *>(at) = h;
             *reinterpret_cast<uint2 *>(at + lo) = l;
         }
     };
 
+    constexpr uint32_t kHighest = 0x7c007c00u;  // (infinities)
+
     if (warp >= kExactWarps) {
-        // (8 x 32 x 96 + 8 x 32 x 160 registers = the 512 x 128 of the launch)
-        if constexpr (HD <= 128) asm volatile("setmaxnreg.dec.sync.aligned.u32 96;");
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(S::kLoaderRegs));
         // ---- loaders: rows of a stage through registers into the planes, K and V in turn, the next ones on their way meanwhile ----
-        constexpr uint32_t LW = S::kLoaders, N = S::kStage / (LW * RW), H = HD > 128 ? 2 : 1, NH = N / H;  // units of a warp: H halves of NH
-        static_assert(NH * H * LW * RW == S::kStage, "even shares");
+        constexpr uint32_t LW = S::kLoaders, H = S::kParts, NH = S::kUnit / RW;  // (float4s of a lane per unit: NH x NV)
+        static_assert(NH * RW == S::kUnit && S::kUnit * H * LW == S::kStage, "even shares");
         const uint32_t lw = warp - kExactWarps, kvHead = head / p.group;
         const size_t stride = static_cast<size_t>(p.nKV) * (HD / 4);
         const float4 *gk = static_cast<const float4 *>(p.k) + static_cast<size_t>(kvHead) * (HD / 4);
         const float4 *gv = static_cast<const float4 *>(p.v) + static_cast<size_t>(kvHead) * (HD / 4);
-        auto rowOf = [&](uint32_t i) { return (i * LW + lw) * RW + sub; };
-        // (rows behind the last one attended are zeros: 0 x NaN would be NaN)
-        auto load = [&](float4 (&x)[NH][NV], const float4 *src, uint32_t st, uint32_t half) {
-            const uint32_t tok0 = st * S::kStage + rowOf(half * NH);
+        auto unitRow = [&](uint32_t part) { return (lw * H + part) * S::kUnit; };
+        // (for rows behind the last one attended, that one: whatever is there meets probabilities of 0, and 0 x NaN would be NaN)
+        auto load = [&](float4 (&x)[NH][NV], const float4 *src, uint32_t st, uint32_t part) {
+            const uint32_t tok0 = st * S::kStage + unitRow(part) + sub;
             const float4 *at = src + tok0 * stride + unit;
             if ((st + 1u) * S::kStage <= len) {  // (a branch, not a condition per load)
 #pragma unroll
                 for (uint32_t i = 0; i < NH; ++i)
 #pragma unroll
-                    for (int v = 0; v < NV; ++v) x[i][v] = __ldg(at + i * (LW * RW * stride) + 32u * v);
+                    for (int v = 0; v < NV; ++v) x[i][v] = __ldg(at + i * (RW * stride) + 32u * v);
                 return;
             }
 #pragma unroll
             for (uint32_t i = 0; i < NH; ++i)
 #pragma unroll
-                for (int v = 0; v < NV; ++v)
-                    x[i][v] = tok0 + i * (LW * RW) < len ? __ldg(at + i * (LW * RW * stride) + 32u * v) : make_float4(0.f, 0.f, 0.f, 0.f);
+                for (int v = 0; v < NV; ++v) x[i][v] = __ldg(src + min(tok0 + i * RW, len - 1u) * stride + unit + 32u * v);
         };
-        auto put = [&](const float4 (&x)[NH][NV], __half *plane, float *scales, uint32_t half, bool isV) {
-            uint32_t e[NH];
-            rowExponents<NH, NV>(x, e);
+        auto put = [&](const float4 (&x)[NH][NV], __half *plane, uint32_t *scales, uint32_t st, uint32_t part, bool isV) {
+            const uint32_t e = unitExponent<NH, NV>(x), row = unitRow(part);
+            const float scale = exactScale(e);
+            uint32_t low = kHighest;
 #pragma unroll
-            for (uint32_t i = 0; i < NH; ++i) {
-                const uint32_t r = rowOf(half * NH + i);
-                place(plane, S::kPlane, x[i], exactScale(e[i]), r);
-                // V: 2^e, the probabilities carry it; K: what undoes the scale
-                if (unit == 0) scales[r] = __uint_as_float(isV ? e[i] : e[i] - (14u << 23));
+            for (uint32_t i = 0; i < NH; ++i) place(plane, S::kPlane, x[i], scale, row + i * RW + sub, low);
+            uint32_t word = isV ? e : e - (14u << 23);  // V: 2^e, the probabilities carry it; K: what undoes the scale
+            if (lane < S::kUnit) scales[row + lane] = word;
+            if (inDoubt(low)) {
+                if (isV && e > (15u << 23) && zeroDim<NH, NV>(x)) word |= 0x80000000u;  // (a unit of nothing but zeros weighs nothing)
+                if (anySmall<NH, NV>(x, e, low)) {
+                    uint32_t small = 0u;
+#pragma unroll 1
+                    for (uint32_t i = opaqueZero(); i < NH; ++i)
+#pragma unroll
+                        for (int v = 0; v < NV; ++v)
+                            small += isSmall(__ldg((isV ? gv : gk) + min(st * S::kStage + row + i * RW + sub, len - 1u) * stride + unit + 32u * v), scale);
+                    small = __reduce_add_sync(0xffffffffu, small);
+                    word = isV ? (small >= S::kUnit ? 0xff800000u : word) : word | 0x80000000u;
+                }
+                if (lane < S::kUnit) scales[row + lane] = word;
             }
         };
-        float4 a[NH][NV], b[NH][NV];
-        load(a, gk, 0, 0);
-        load(b, H == 1 ? gv : gk, 0, H - 1);
+        if (nStages == 0u) return;  // (an empty store)
+        // parts in turn: those of K, those of V; two are on their way
+        float4 x[2][NH][NV];
+        load(x[0], gk, 0, 0);
+        load(x[1], H == 1 ? gv : gk, 0, H == 1 ? 0 : 1);
         for (uint32_t st = 0; st < nStages; ++st) {
             const uint32_t buf = st % NB;
-            __half *pk = sh + S::kK + buf * 2 * S::kPlane, *pv = sh + S::kV + buf * 2 * S::kPlane;
-            float *sk = sf + S::kScaleK + buf * S::kStage, *sv = sf + S::kScaleV + buf * S::kStage;
-            if (st >= NB) namedBarSync(kFreeK + buf, kAll);
-            put(a, pk, sk, 0, false);
-            if (H == 1) {
-                if (st + 1 < nStages) load(a, gk, st + 1, 0);
-                namedBarArrive(kFullK + buf, kAll);
-                if (st >= NB) namedBarSync(kFreeV + buf, kAll);
-                put(b, pv, sv, 0, true);
-                if (st + 1 < nStages) load(b, gv, st + 1, 0);
-                namedBarArrive(kFullV + buf, kAll);
-            } else {
-                load(a, gv, st, 0);
-                put(b, pk, sk, 1, false);
-                load(b, gv, st, 1);
-                namedBarArrive(kFullK + buf, kAll);
-                if (st >= NB) namedBarSync(kFreeV + buf, kAll);
-                put(a, pv, sv, 0, true);
-                if (st + 1 < nStages) load(a, gk, st + 1, 0);
-                put(b, pv, sv, 1, true);
-                if (st + 1 < nStages) load(b, gk, st + 1, 1);
-                namedBarArrive(kFullV + buf, kAll);
+            __half *planes[2] = {sh + S::kK + buf * 2 * S::kPlane, sh + S::kV + buf * 2 * S::kPlane};
+            uint32_t *scales[2] = {reinterpret_cast<uint32_t *>(sf + S::kScaleK + buf * S::kStage), reinterpret_cast<uint32_t *>(sf + S::kScaleV + buf * S::kStage)};
+#pragma unroll
+            for (uint32_t j = 0; j < 2 * H; ++j) {
+                const bool isV = j >= H;
+                if (j % H == 0 && st >= NB) namedBarSync((isV ? kFreeV : kFreeK) + buf, kAll);
+                put(x[j & 1u], planes[isV], scales[isV], st, j % H, isV);
+                const uint32_t next = j + 2, nextSt = st + next / (2 * H), part = next % (2 * H);
+                if (nextSt < nStages) load(x[j & 1u], part >= H ? gv : gk, nextSt, part % H);
+                if (j % H == H - 1) namedBarArrive((isV ? kFullV : kFullK) + buf, kAll);
             }
         }
         return;
     }
 
-    if constexpr (HD <= 128) asm volatile("setmaxnreg.inc.sync.aligned.u32 160;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(S::kRegs));
     const uint32_t g = lane >> 2, t = lane & 3u, rt = warp % RT, nh = warp / RT;
     {   // q, the same way
         constexpr uint32_t N = S::kRows / (kExactWarps * RW);
         float4 x[N][NV];
 #pragma unroll
         for (uint32_t i = 0; i < N; ++i) {
-            const uint32_t r = (i * kExactWarps + warp) * RW + sub;
+            const uint32_t r = min((i * kExactWarps + warp) * RW + sub, rows - 1u);  // (no row: the last one)
 #pragma unroll
             for (int v = 0; v < NV; ++v)
-                x[i][v] = r < rows ? __ldg(reinterpret_cast<const float4 *>(p.q + (static_cast<size_t>(row0 + r) * p.nHeads + head) * HD) + unit + 32u * v)
-                                   : make_float4(0.f, 0.f, 0.f, 0.f);
+                x[i][v] = __ldg(reinterpret_cast<const float4 *>(p.q + (static_cast<size_t>(row0 + r) * p.nHeads + head) * HD) + unit + 32u * v);
         }
-        uint32_t e[N];
-        rowExponents<N, NV>(x, e);
+        const uint32_t e = unitExponent<N, NV>(x);
+        const float scale = exactScale(e);
+        uint32_t low = kHighest, word = e - (14u << 23);
 #pragma unroll
-        for (uint32_t i = 0; i < N; ++i) {
-            const uint32_t r = (i * kExactWarps + warp) * RW + sub;
-            place(sh + S::kQ, S::kRows * LD, x[i], exactScale(e[i]), r);
-            if (unit == 0) sf[S::kScaleQ + r] = p.scaleLog2 * __uint_as_float(e[i] - (14u << 23));
+        for (uint32_t i = 0; i < N; ++i) place(sh + S::kQ, S::kRows * LD, x[i], scale, (i * kExactWarps + warp) * RW + sub, low);
+        if (inDoubt(low) && anySmall<N, NV>(x, e, low)) word |= 0x80000000u;
+        if (unit == 0) {
+#pragma unroll
+            for (uint32_t i = 0; i < N; ++i) sf[S::kScaleQ + (i * kExactWarps + warp) * RW + sub] = __uint_as_float(word);
         }
     }
     namedBarSync(kFoldBar, kExactThreads);
-    const float cs0 = sf[S::kScaleQ + rt * 16u + g], cs1 = sf[S::kScaleQ + rt * 16u + g + 8u];
+    const float cs0 = p.scaleLog2 * fabsf(sf[S::kScaleQ + rt * 16u + g]), cs1 = p.scaleLog2 * fabsf(sf[S::kScaleQ + rt * 16u + g + 8u]);
+    // the largest scale of this warp's rows, whether they have small ones, and from where on a word of K's is looked into (a sign above all)
+    uint32_t csTop, kDoubt;
+    bool qSmall;
+    {
+        const uint32_t word = __float_as_uint(sf[S::kScaleQ + rt * 16u + (lane & 15u)]);
+        qSmall = __any_sync(0xffffffffu, word >> 31);
+        const uint32_t top = __reduce_max_sync(0xffffffffu, word & 0x7fffffffu);
+        csTop = top < kHugeWord ? __float_as_uint(fabsf(p.scaleLog2) * __uint_as_float(top)) : 0x7f800000u;
+        kDoubt = qSmall || top >= kHugeWord ? 0u : min(max(354u - (csTop >> 23), 1u), kHugeWord >> 23) << 23;  // (2^99 or 2^100 with csTop)
+    }
 
     float o[HD / 8][4];
 #pragma unroll
@@ -287,12 +362,70 @@ __global__ void __launch_bounds__(ExactShape<HD>::kThreads, 1) prefillExactKerne
     const uint32_t vAddr = smemAddr(sh + S::kV + (nh * TG + (lane & 15u)) * LD + (lane >> 4) * 8u);
     constexpr uint32_t kLoAt = S::kPlane * 2, kBufAt = 2 * kLoAt;  // bytes
 
-    for (uint32_t st = 0; st < nStages; ++st) {
+    float s[NT][4];
+    // scores (log2 units) to probabilities: this thread has tokens 2t, 2t + 1 of every 8, rows g and g + 8
+    constexpr int NU = S::kUnit < 8 ? 1 : TG / S::kUnit;  // a group's units with a largest probability each (smaller ones do it without)
+    float pm0[NU], pm1[NU];
+    auto softmax = [&](uint32_t tok0, uint32_t freeK, bool again) {
+        float mu0[NU], mu1[NU];
+#pragma unroll
+        for (int u = 0; u < NU; ++u) mu0[u] = mu1[u] = kNegBig;
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const uint32_t tok = tok0 + 8 * n + 2 * t + i;
+                s[n][i] = tok < lim0 ? s[n][i] : -INFINITY;
+                s[n][2 + i] = tok < lim1 ? s[n][2 + i] : -INFINITY;
+                mu0[n * NU / NT] = fmaxf(mu0[n * NU / NT], s[n][i]);
+                mu1[n * NU / NT] = fmaxf(mu1[n * NU / NT], s[n][2 + i]);
+            }
+        __syncwarp();  // (every lane has read its part of K and of its scales)
+        if (again) namedBarArrive(freeK, kAll);
+        float mn0 = m0, mn1 = m1;
+#pragma unroll
+        for (int u = 0; u < NU; ++u) {
+#pragma unroll
+            for (int off = 1; off <= 2; off <<= 1) {
+                mu0[u] = fmaxf(mu0[u], __shfl_xor_sync(0xffffffffu, mu0[u], off));
+                mu1[u] = fmaxf(mu1[u], __shfl_xor_sync(0xffffffffu, mu1[u], off));
+            }
+            mn0 = fmaxf(mn0, mu0[u]), mn1 = fmaxf(mn1, mu1[u]);
+        }
+        if (__any_sync(0xffffffffu, mn0 != m0 || mn1 != m1)) {
+            const float a0 = fastExp2(m0 - mn0), a1 = fastExp2(m1 - mn1);
+#pragma unroll
+            for (int i = 0; i < HD / 8; ++i) {
+                o[i][0] *= a0;
+                o[i][1] *= a0;
+                o[i][2] *= a1;
+                o[i][3] *= a1;
+            }
+            l0 *= a0;
+            l1 *= a1;
+            m0 = mn0;
+            m1 = mn1;
+        }
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+            s[n][0] = fastExp2(s[n][0] - m0), s[n][1] = fastExp2(s[n][1] - m0);
+            s[n][2] = fastExp2(s[n][2] - m1), s[n][3] = fastExp2(s[n][3] - m1);
+            l0 += s[n][0] + s[n][1];
+            l1 += s[n][2] + s[n][3];
+        }
+#pragma unroll
+        for (int u = 0; u < NU; ++u) pm0[u] = fastExp2(mu0[u] - m0), pm1[u] = fastExp2(mu1[u] - m1);
+    };
+
+    uint32_t st = 0, at = 0;  // (at: how far the stage is that did not fit -- 1: its K is in, 2: its probabilities and V are)
+    for (; st < nStages; ++st) {
         const uint32_t buf = st % NB, tok0 = st * S::kStage + nh * TG;
         const bool active = tok0 < warpLimit, again = st + NB < nStages;  // (both warp-uniform)
-        float s[NT][4], x[NT][4];  // hi*hi, and the cross terms
         namedBarSync(kFullK + buf, kAll);
         if (active) {
+            const float *sk = sf + S::kScaleK + buf * S::kStage + nh * TG;
+            const uint32_t word = __float_as_uint(sk[lane % TG]);
+            float x[NT][4];  // s: hi*hi, x: the cross terms
 #pragma unroll
             for (int n = 0; n < NT; ++n)
 #pragma unroll
@@ -304,9 +437,9 @@ __global__ void __launch_bounds__(ExactShape<HD>::kThreads, 1) prefillExactKerne
                 ldmatrixX4(al[0], al[1], al[2], al[3], aAddr + S::kRows * LD * 2 + ks * 32);
 #pragma unroll
                 for (int n = 0; n < NT / 2; ++n) {
-                    const uint32_t at = kAddr + buf * kBufAt + n * (16 * LD * 2) + ks * 32;
-                    ldmatrixX4(bh[n][0], bh[n][1], bh[n][2], bh[n][3], at);
-                    ldmatrixX4(bl[n][0], bl[n][1], bl[n][2], bl[n][3], at + kLoAt);
+                    const uint32_t from = kAddr + buf * kBufAt + n * (16 * LD * 2) + ks * 32;
+                    ldmatrixX4(bh[n][0], bh[n][1], bh[n][2], bh[n][3], from);
+                    ldmatrixX4(bl[n][0], bl[n][1], bl[n][2], bl[n][3], from + kLoAt);
                 }
 #pragma unroll
                 for (int n = 0; n < NT; ++n) mmaF16(s[n], ah[0], ah[1], ah[2], ah[3], bh[n / 2][n % 2 * 2], bh[n / 2][n % 2 * 2 + 1]);
@@ -315,80 +448,73 @@ __global__ void __launch_bounds__(ExactShape<HD>::kThreads, 1) prefillExactKerne
 #pragma unroll
                 for (int n = 0; n < NT; ++n) mmaF16(x[n], ah[0], ah[1], ah[2], ah[3], bl[n / 2][n % 2 * 2], bl[n / 2][n % 2 * 2 + 1]);
             }
-            // ---- online softmax: this thread has tokens 2t, 2t + 1 of every 8, rows g and g + 8 ----
-            float mx0 = kNegBig, mx1 = kNegBig;
-#pragma unroll
-            for (int n = 0; n < NT; ++n) {
-                const float2 sk = *reinterpret_cast<const float2 *>(sf + S::kScaleK + buf * S::kStage + nh * TG + 8 * n + 2 * t);
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const uint32_t tok = tok0 + 8 * n + 2 * t + i;
-                    const float sc = i ? sk.y : sk.x;
-                    s[n][i] = tok < lim0 ? (s[n][i] + x[n][i]) * (sc * cs0) : -INFINITY;
-                    s[n][2 + i] = tok < lim1 ? (s[n][2 + i] + x[n][2 + i]) * (sc * cs1) : -INFINITY;
-                    mx0 = fmaxf(mx0, s[n][i]);
-                    mx1 = fmaxf(mx1, s[n][2 + i]);
+            if (__any_sync(0xffffffffu, word >= kDoubt)) {  // (here the vote is no wait)
+                const float top = __uint_as_float(word & 0x7fffffffu) * __uint_as_float(csTop);
+                const bool holds = top <= kMostScale && (word & 0x7fffffffu) < kHugeWord && !((word >> 31 || qSmall) && top > kSmallCount);
+                if (!__all_sync(0xffffffffu, holds)) {
+                    at = 1;
+                    break;
                 }
-            }
-            __syncwarp();  // (every lane has read its part of K and of its scales)
-            if (again) namedBarArrive(kFreeK + buf, kAll);
-#pragma unroll
-            for (int off = 1; off <= 2; off <<= 1) {
-                mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, off));
-                mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, off));
-            }
-            const float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);
-            if (__any_sync(0xffffffffu, mn0 != m0 || mn1 != m1)) {
-                const float a0 = fastExp2(m0 - mn0), a1 = fastExp2(m1 - mn1);
-#pragma unroll
-                for (int i = 0; i < HD / 8; ++i) {
-                    o[i][0] *= a0;
-                    o[i][1] *= a0;
-                    o[i][2] *= a1;
-                    o[i][3] *= a1;
-                }
-                l0 *= a0;
-                l1 *= a1;
-                m0 = mn0;
-                m1 = mn1;
             }
 #pragma unroll
             for (int n = 0; n < NT; ++n) {
-                s[n][0] = fastExp2(s[n][0] - m0), s[n][1] = fastExp2(s[n][1] - m0);
-                s[n][2] = fastExp2(s[n][2] - m1), s[n][3] = fastExp2(s[n][3] - m1);
-                l0 += s[n][0] + s[n][1];
-                l1 += s[n][2] + s[n][3];
+                const float2 w = *reinterpret_cast<const float2 *>(sk + 8 * n + 2 * t);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) s[n][i] = fmaf(x[n][i], kLoScale, s[n][i]) * (fabsf(i & 1 ? w.y : w.x) * (i & 2 ? cs1 : cs0));
             }
+            softmax(tok0, kFreeK + buf, again);
         } else if (again) {
             namedBarArrive(kFreeK + buf, kAll);
         }
         namedBarSync(kFullV + buf, kAll);
         if (active) {
             // ---- O += P V, 16 tokens at a time: the accumulator layout of the scores is the A operand's.  The probabilities take the
-            // scales of V's rows along, and every query row a power of two of its own, out of its largest product: with one for the group a
-            // row of V that is masked, or weighs nothing, pushed the probabilities of the others out of the pairs' range ----
+            // scales of V's units along, and every query row a power of two of its own: the most that one of its products can be ----
             const float *sv = sf + S::kScaleV + buf * S::kStage + nh * TG;
-            float top0 = 0.0f, top1 = 0.0f;
+            const uint32_t word = __float_as_uint(sv[lane % TG]);
+            const bool doubt = __any_sync(0xffffffffu, word >= 0x7f800000u);
+            float top0 = 0.0f, top1 = 0.0f, u[NT][4];
 #pragma unroll
             for (int n = 0; n < NT; ++n) {
                 const float2 w = *reinterpret_cast<const float2 *>(sv + 8 * n + 2 * t);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) s[n][i] *= i & 1 ? w.y : w.x;
-                top0 = fmaxf(top0, fmaxf(s[n][0], s[n][1]));
-                top1 = fmaxf(top1, fmaxf(s[n][2], s[n][3]));
+                for (int i = 0; i < 4; ++i) u[n][i] = s[n][i] * fabsf(i & 1 ? w.y : w.x);
+                if constexpr (S::kUnit >= 8) {  // (w is the same for all of a unit)
+                    top0 = fmaxf(top0, pm0[n * NU / NT] * fabsf(w.x));
+                    top1 = fmaxf(top1, pm1[n * NU / NT] * fabsf(w.x));
+                } else {
+                    top0 = fmaxf(top0, fmaxf(u[n][0], u[n][1]));
+                    top1 = fmaxf(top1, fmaxf(u[n][2], u[n][3]));
+                }
             }
+            if constexpr (S::kUnit < 8) {
 #pragma unroll
-            for (int off = 1; off <= 2; off <<= 1) {
-                top0 = fmaxf(top0, __shfl_xor_sync(0xffffffffu, top0, off));
-                top1 = fmaxf(top1, __shfl_xor_sync(0xffffffffu, top1, off));
+                for (int off = 1; off <= 2; off <<= 1) {
+                    top0 = fmaxf(top0, __shfl_xor_sync(0xffffffffu, top0, off));
+                    top1 = fmaxf(top1, __shfl_xor_sync(0xffffffffu, top1, off));
+                }
             }
             const uint32_t e0 = max(__float_as_uint(top0) & 0x7f800000u, 15u << 23), e1 = max(__float_as_uint(top1) & 0x7f800000u, 15u << 23);
             const float in0 = exactScale(e0), in1 = exactScale(e1);
+            if (doubt) {
+                bool holds = true;
+#pragma unroll
+                for (int n = 0; n < NT; ++n)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) holds = holds && !(u[n][i] != 0.0f && u[n][i] * (i & 2 ? in1 : in0) < kLeast);
+                const uint32_t scale = word & 0x7fffffffu, first = __float_as_uint(sv[0]) & 0x7fffffffu;
+                const bool near = !__any_sync(0xffffffffu, scale - first + kLongScales > 2u * kLongScales);
+                holds = (holds || near) && scale < 0x7f800000u;
+                if (!__all_sync(0xffffffffu, holds)) {
+                    at = 2;
+                    break;
+                }
+            }
             uint32_t ph[NT / 2][4], pl[NT / 2][4];
 #pragma unroll
             for (int n = 0; n < NT; ++n) {
-                splitPair(s[n][0] * in0, s[n][1] * in0, ph[n / 2][n % 2 * 2], pl[n / 2][n % 2 * 2]);
-                splitPair(s[n][2] * in1, s[n][3] * in1, ph[n / 2][n % 2 * 2 + 1], pl[n / 2][n % 2 * 2 + 1]);
+                splitPair(u[n][0] * in0, u[n][1] * in0, ph[n / 2][n % 2 * 2], pl[n / 2][n % 2 * 2]);
+                splitPair(u[n][2] * in1, u[n][3] * in1, ph[n / 2][n % 2 * 2 + 1], pl[n / 2][n % 2 * 2 + 1]);
             }
             constexpr float kPlanes = 3.7252902984619140625e-9f;  // 2^-28: 2^14 in the planes of V, and in the pairs of p
             const float out0 = __uint_as_float(e0) * kPlanes, out1 = __uint_as_float(e1) * kPlanes;
@@ -401,9 +527,9 @@ __global__ void __launch_bounds__(ExactShape<HD>::kThreads, 1) prefillExactKerne
                     uint32_t bh[DB][4], bl[DB][4];
 #pragma unroll
                     for (int d = 0; d < DB; ++d) {
-                        const uint32_t at = vAddr + buf * kBufAt + n * (16 * LD * 2) + (d0 + d) * 32;
-                        ldmatrixX4Trans(bh[d][0], bh[d][1], bh[d][2], bh[d][3], at);
-                        ldmatrixX4Trans(bl[d][0], bl[d][1], bl[d][2], bl[d][3], at + kLoAt);
+                        const uint32_t from = vAddr + buf * kBufAt + n * (16 * LD * 2) + (d0 + d) * 32;
+                        ldmatrixX4Trans(bh[d][0], bh[d][1], bh[d][2], bh[d][3], from);
+                        ldmatrixX4Trans(bl[d][0], bl[d][1], bl[d][2], bl[d][3], from + kLoAt);
                     }
 #pragma unroll
                     for (int d = 0; d < 2 * DB; ++d)
@@ -418,7 +544,73 @@ __global__ void __launch_bounds__(ExactShape<HD>::kThreads, 1) prefillExactKerne
 #pragma unroll
                 for (int d = 0; d < 2 * DB; ++d)
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) o[2 * d0 + d][i] = fmaf(sum[d][i] + cross[d][i], i & 2 ? out1 : out0, o[2 * d0 + d][i]);
+                    for (int i = 0; i < 4; ++i) o[2 * d0 + d][i] = fmaf(fmaf(cross[d][i], kLoScale, sum[d][i]), i & 2 ? out1 : out0, o[2 * d0 + d][i]);
+            }
+            __syncwarp();
+        }
+        if (again) namedBarArrive(kFreeV + buf, kAll);
+    }
+
+    // From the first stage on whose numbers the pairs do not hold: the same in f32, from the rows themselves, hand in hand with the loaders
+    // still.  (In the loop above it cost every stage 4 - 6 %.)
+    for (; st < nStages; ++st, at = 0) {
+        const uint32_t buf = st % NB, tok0 = st * S::kStage + nh * TG;
+        const bool active = tok0 < warpLimit, again = st + NB < nStages;
+        if (at == 0) namedBarSync(kFullK + buf, kAll);
+        if (at < 2) {
+            if (active) {
+                const float4 *qa = reinterpret_cast<const float4 *>(p.q + (static_cast<size_t>(row0 + min(rt * 16u + g, rows - 1u)) * p.nHeads + head) * HD);
+                const float4 *qb = reinterpret_cast<const float4 *>(p.q + (static_cast<size_t>(row0 + min(rt * 16u + g + 8u, rows - 1u)) * p.nHeads + head) * HD);
+                const float4 *gk = static_cast<const float4 *>(p.k) + static_cast<size_t>(head / p.group) * (HD / 4);
+                float x[NT][4];
+#pragma unroll
+                for (int n = 0; n < NT; ++n)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) s[n][i] = x[n][i] = 0.0f;
+#pragma unroll 1
+                for (uint32_t c = 0; c < HD / 4; ++c) {
+                    const float4 a = __ldg(qa + c), b = __ldg(qb + c);
+#pragma unroll
+                    for (int n = 0; n < NT; ++n)
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) {
+                            const uint32_t tok = min(tok0 + 8 * n + 2 * t + i, len - 1u);
+                            const float4 k = __ldg(gk + static_cast<size_t>(tok) * p.nKV * (HD / 4) + c);
+                            s[n][i] = fmaf(a.x, k.x, fmaf(a.y, k.y, s[n][i])), x[n][i] = fmaf(a.z, k.z, fmaf(a.w, k.w, x[n][i]));
+                            s[n][2 + i] = fmaf(b.x, k.x, fmaf(b.y, k.y, s[n][2 + i])), x[n][2 + i] = fmaf(b.z, k.z, fmaf(b.w, k.w, x[n][2 + i]));
+                        }
+                }
+#pragma unroll
+                for (int n = 0; n < NT; ++n)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) s[n][i] = (s[n][i] + x[n][i]) * p.scaleLog2;
+                softmax(tok0, kFreeK + buf, again);
+            } else if (again) {
+                namedBarArrive(kFreeK + buf, kAll);
+            }
+            namedBarSync(kFullV + buf, kAll);
+        }
+        if (active) {
+            // the warp's probabilities through shared memory: a thread takes all tokens of its two rows for the dims it has
+            float *prob = sf + S::kProb + warp * 16 * TG;
+#pragma unroll
+            for (int n = 0; n < NT; ++n) {
+                *reinterpret_cast<float2 *>(prob + g * TG + 8 * n + 2 * t) = make_float2(s[n][0], s[n][1]);
+                *reinterpret_cast<float2 *>(prob + (g + 8u) * TG + 8 * n + 2 * t) = make_float2(s[n][2], s[n][3]);
+            }
+            __syncwarp();
+            const float2 *gv = static_cast<const float2 *>(p.v) + static_cast<size_t>(head / p.group) * (HD / 2) + t;
+#pragma unroll 1
+            for (uint32_t c = 0; c < TG && tok0 + c < warpLimit; ++c) {
+                const float p0 = prob[g * TG + c], p1 = prob[(g + 8u) * TG + c];
+                const bool see0 = tok0 + c < lim0, see1 = tok0 + c < lim1;  // (masked rows stay out: 0 x Inf would be NaN)
+                const float2 *row = gv + static_cast<size_t>(tok0 + c) * p.nKV * (HD / 2);
+#pragma unroll
+                for (int d = 0; d < HD / 8; ++d) {
+                    const float2 v = __ldg(row + 4 * d);
+                    if (see0) o[d][0] = fmaf(p0, v.x, o[d][0]), o[d][1] = fmaf(p0, v.y, o[d][1]);
+                    if (see1) o[d][2] = fmaf(p1, v.x, o[d][2]), o[d][3] = fmaf(p1, v.y, o[d][3]);
+                }
             }
             __syncwarp();
         }
@@ -429,7 +621,7 @@ __global__ void __launch_bounds__(ExactShape<HD>::kThreads, 1) prefillExactKerne
 }
 
 // ---- fp16 store ------------------------------------------------------------------------------------------
-// fp16 K and V are operands as they are (m16n8k16, twice the rate of the tf32 products and no third one); q, normalised by
+// fp16 K and V are operands as they are, in one plane each and two products where the f32 rows need three; q, normalised by
 // a power of two per row, and the probabilities are fp16 hi + lo pairs (two products, ~22 mantissa bits), as in
 // decode_kv16.cu.  Stages come in by cp.async, two deep.
 template <int HD>
@@ -663,7 +855,7 @@ struct ExactCost {
     float end8, token8, end32, token32;
 };
 bool prefillExactWins(uint32_t rows, uint64_t before, uint32_t nHeads, uint32_t hd, int kvHalf) {
-    static constexpr ExactCost k32[3] = {{3.0f, 0.0103f, 3.4f, 0.0164f}, {4.2f, 0.0193f, 3.4f, 0.0365f}, {5.1f, 0.0548f, 6.0f, 0.0727f}};
+    static constexpr ExactCost k32[3] = {{3.0f, 0.0103f, 3.7f, 0.0174f}, {4.2f, 0.0193f, 3.8f, 0.038f}, {5.1f, 0.0548f, 5.8f, 0.069f}};
     static constexpr ExactCost k16[2] = {{3.4f, 0.0032f, 2.9f, 0.0115f}, {4.8f, 0.0049f, 4.3f, 0.019f}};
     const ExactCost &c = kvHalf ? k16[hd == 128] : k32[hd == 64 ? 0 : (hd == 128 ? 1 : 2)];
     const float last = static_cast<float>(before + rows), mean = static_cast<float>(before) + 0.5f * rows;
