@@ -410,6 +410,23 @@ def test_few_blocks_of_a_cluster_and_many_with_a_merge(nH, nKV, batch, ctx):
             assert float((out[b, h].double() - want).norm() / want.norm()) < 1e-5
 
 
+@pytest.mark.parametrize("nH,nKV,batch,ctx,cluster", [(28, 4, 2, 9200, True), (28, 4, 2, 10500, False), (40, 8, 1, 15300, False), (28, 4, 3, 18500, True),
+                                                      (28, 4, 4, 3000, True), (28, 4, 4, 6000, False), (28, 4, 5, 9208, False), (28, 4, 6, 9208, True),
+                                                      (28, 4, 10, 4600, False), (12, 2, 18, 3000, False), (28, 4, 12, 4600, True)])
+def test_clusters_of_few_blocks_only_where_they_fill_the_card(nH, nKV, batch, ctx, cluster):
+    """Sequences of one length: clusters of 8, 4 and 2 blocks on fewer than 5 / 8 of the SMs are left to the merge as soon as their blocks have
+    more than five (three) tiles more than its (one slot used: a cluster)."""
+    hd = 128
+    q = torch.zeros((batch, nH, hd), device="cuda")
+    k8 = torch.zeros((batch * ctx, nKV, hd), dtype=torch.int8, device="cuda")
+    ks = torch.ones((batch * ctx, nKV), device="cuda")
+    slots = min(64, ops.split_geometry(ctx, nH, hd)[1])
+    used = ops.decode_i8_batch(q, k8, k8, ks, ks, torch.empty_like(q), ops.workspace(batch, nH, hd, slots), None, batch, nH, nKV, hd, ctx, slots,
+                               rows_per_seq=ctx)
+    assert (used == 1) == cluster
+    assert ops.device_status() == 0
+
+
 @pytest.mark.parametrize("nH,nKV,lens", [(28, 4, (12000, 11871, 130, 5000)), (28, 4, (12000, 1, 7000, 127, 128, 129, 3000, 11999)),
                                          (40, 8, (12000, 300)), (12, 2, (26000, 64, 25999, 128))])
 def test_ragged_sequences_in_clusters_of_few_blocks(nH, nKV, lens):

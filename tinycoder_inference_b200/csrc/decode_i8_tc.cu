@@ -872,12 +872,17 @@ int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, c
     // A cluster per (sequence, kv head) folds without partials and merge launch.  It is taken when all of them are resident
     // at once (16 blocks: 7, 8: 15, 4: 33, 2: 74, a block filling an SM) and their blocks, fewer than the merge form's, do not
     // cost more than the launch: a tile more per block takes 0.25 - 0.3 us while latency is what bounds it, and a fold over 16 blocks
-    // more than one over 8.  So up to five tiles more per block for 16 of them, nine for fewer.  Merge -> cluster, eight layers in
-    // stream order, 28 / 4 heads: 14000 rows (3 tiles a block -> 7) 69.4 -> 56.6 us, 16000 (4 -> 8) 67.0 -> 59.5, 20000 (5 -> 10) 70.0 ->
-    // 69.0, 30000 (7 -> 15) 79.9 -> 83.1; 12 / 2 heads: 9000 (1 -> 5) 64.0 -> 45.9, 20000 (3 -> 10, four layers of a session) 28.5 -> 32.8;
-    // 16 blocks for 2 sequences of 12 / 2: 20000 (5 -> 10) 68.7 -> 68.2, 30000 (7 -> 15) 79.0 -> 81.6.  Eight blocks: 40 / 8 at 16000 rows
-    // (7 -> 16) 89.3 -> 83.7, 3 sequences of 28 / 4 at 12000 / 20000 / 28000 (8 -> 12, 14 -> 20, 19 -> 28) 91.9 -> 76.8, 121.6 -> 105.9, 150.7 ->
-    // 139.4, 4 of 12 / 2 at 12000 (6 -> 12) 73.2 -> 74.1, the one that lost.  With ragged device lengths the cluster also shares every sequence evenly among its blocks, where the
+    // more than one over 8.  So up to five tiles more per block for 16 of them and nine for fewer -- where the clusters keep 5 / 8 of the
+    // SMs busy.  Where they do not, a tile is not latency alone, the rows come in over those SMs only: five for 8 blocks, three for 4 and 2.
+    // Cluster against merge, 28 / 4 heads unless said, rows asked for early (TC_DECODE_PDL) / plain stream order, per layer, tiles a block in brackets:
+    //   16 blocks: 1 sequence of 12708 - 19749 rows (3 -> 7, 5 -> 10) 0.70 - 0.96 / 0.72 - 1.015; of 30000 (7 -> 15) 1.04;
+    //   8 blocks, 96 of them: 3 sequences of 10520 - 27057 (7 -> 11, 18 -> 27) 0.83 - 0.92 / 0.93 - 1.01;
+    //   8 blocks, 64: 2 of 6357 - 9275 (3 -> 7, 5 -> 10) 0.88 - 0.92 / 0.93 - 0.99, of 15351 (7 -> 15) 1.06 / 1.06; 40 / 8, one of 11204 (5 -> 11) 1.045 / 1.08,
+    //     of 15351 1.09 / 1.10;
+    //   4 blocks, 96 and 112: 6 and 7 of 5262 - 23855 (7 -> 11, 38 -> 47) 0.81 - 0.96 / 0.91 - 1.0; 64: 4 of 5969 (6 -> 12) 1.11 / 1.14, of 7678 1.04 / 1.15;
+    //     80: 5 of 4941 - 9275 (6 -> 10, 11 -> 19) 1.01 - 1.07 / 0.99 - 1.06;
+    //   2 blocks, 96: 12 of 2632 - 6770 (7 -> 11, 18 -> 27) 0.88 - 0.96 / 0.95 - 1.01; 72: 12 / 2, 18 of 2320 - 4356 (5 -> 10, 9 -> 18) 1.03 - 1.08 / 1.07 - 1.09.
+    // With ragged device lengths the cluster also shares every sequence evenly among its blocks, where the
     // merge form cuts chunks by the longest one.  There the line is 20 tiles per block of the longest sequence for 16 blocks: cluster
     // against merge, 2 / 3 / 4 / 8 sequences of up to 6000 rows (6 - 12 tiles) 0.44 / 0.48 / 0.66 / 0.67 of the time, up to 20000
     // (20 tiles, 2 and 3 sequences) 0.83 and 0.87, up to 32768 (32, 2 and 3) 1.15; and 26 for fewer: 2 and 3 of up to 26000 (26 tiles) 0.83 and 0.82,
@@ -891,7 +896,9 @@ int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, c
     if (pl.chunksPerSeq > 1 && !d->partialsOnly && d->mergeTickets == nullptr) {
         const uint32_t tiles = (d->maxLen + kTcTile - 1) / kTcTile;
         for (uint32_t lg = 4; lg >= 1 && cluster == 1; --lg) {
-            const uint32_t n = 1u << lg, more = n == 16u ? 5u : 9u;
+            const uint32_t n = 1u << lg;
+            const bool busy = n * d->nKV * d->batch * 8u >= static_cast<uint32_t>(numSMs()) * 5u;
+            const uint32_t more = n == 16u ? 5u : (busy ? 9u : (n == 8u ? 5u : 3u));
             const uint32_t most = d->lens == nullptr || d->batch == 1 ? pl.chunkTokens / kTcTile + more : n == 16u ? 20u : 26u;  // tiles per block
             if (n / 2u >= tiles || limits[lg] < d->nKV * d->batch || (tiles + n - 1u) / n > most) continue;
             cluster = n;
