@@ -76,3 +76,21 @@ def test_decode_without_partial_buffers(dtype, nH, nKV, hd, pos):
     out = torch.empty_like(q)
     ops.decode_kv(q, k, v, out, (None, None, None), 1, nH, nKV, hd, pos, 256)
     assert _far(q, k, v, out, pos) < (BOUND if dtype == torch.float16 else 72 * 6e-8 * 3)
+
+
+@pytest.mark.parametrize("nH,nKV,pos", [(14, 2, 4000), (8, 4, 4000), (8, 4, 30000)])
+def test_f32_decode_of_many_tiles_a_warp(nH, nKV, pos):
+    """... at head_dim 64 is as near as 1500 rows, a tile a warp: what a warp adds up beyond a tile is f32.  (Means of eight inputs, which differ by some 3 %
+    of each other; with one running sum 1.2 to 2.9 times as far.)"""
+    def mean(pos):
+        far = 0.0
+        for seed in range(8):
+            g = torch.Generator(device="cuda").manual_seed(seed)
+            q = torch.randn((1, nH, 64), device="cuda", generator=g)
+            k, v = (torch.randn((pos + 1, nKV, 64), device="cuda", generator=g) for _ in range(2))
+            out = torch.empty_like(q)
+            ops.decode_kv(q, k, v, out, ops.workspace(1, nH, 64, 256), 1, nH, nKV, 64, pos, 256)
+            far += _far(q, k, v, out, pos) / 8
+        return far
+
+    assert mean(pos) < 1.15 * mean(1500)
