@@ -383,6 +383,35 @@ def test_next_pool_hint_of_blocks_with_many_tiles(ctx, appends):
         assert all(torch.equal(a, b) for a, b in zip(*got))
 
 
+@pytest.mark.parametrize("pdl", [False, True])
+@pytest.mark.parametrize("appends", [False, True])
+def test_next_pool_hint_of_calls_above_48_mb(appends, pdl):
+    """8 sequences of 8192 rows, 64 MB: blocks of 14 tiles ask for the next call's rows behind their last one, in plain order and as a dependent
+    launch behind a call that reads the same pool.  The same bits as without a hint; pointers off 16 bytes are no hint, and no error."""
+    nH, nKV, hd, batch, ctx = 28, 4, 128, 8, 8192
+    g = torch.Generator(device="cuda").manual_seed(5)
+    pool = [torch.randint(-127, 128, (batch * ctx, nKV, hd), dtype=torch.int8, device="cuda", generator=g) for _ in range(2)] + \
+           [0.01 + 0.01 * torch.rand((batch * ctx, nKV), device="cuda", generator=g) for _ in range(2)]
+    flat = [torch.zeros(pool[0].numel() + 16, dtype=torch.int8, device="cuda") for _ in range(2)]
+    n = pool[0].numel()
+    hints = (None, tuple(x[:n].view_as(pool[0]) for x in flat), tuple(x[1:1 + n].view_as(pool[0]) for x in flat))
+    q = torch.randn((batch, nH, hd), device="cuda", generator=g)
+    rows = tuple(torch.randn((batch, nKV, hd), device="cuda", generator=g) for _ in range(2)) if appends else None
+    slots = min(64, ops.split_geometry(ctx, nH, hd)[1])
+    ws = ops.workspace(batch, nH, hd, slots)
+    got = []
+    for hint in hints:
+        mine, out = [t.clone() for t in pool], torch.empty_like(q)
+        for _ in range(2):
+            ops.decode_i8_batch(q, *mine, out, ws, None, batch, nH, nKV, hd, ctx, slots, rows_per_seq=ctx, next_kv=hint, append=rows,
+                                pdl=pdl, prefetch_rows=ctx - 1 if pdl else 0)
+        torch.cuda.synchronize()
+        assert ops.device_status() == 0
+        got.append([out] + mine)
+    for other in got[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(got[0], other))
+
+
 @pytest.mark.parametrize("nH,nKV,batch,ctx", [(28, 4, 1, 13900), (28, 4, 1, 20001), (28, 4, 1, 22000), (12, 2, 1, 9000), (12, 2, 1, 15900),
                                               (40, 8, 1, 16000), (28, 4, 3, 12000), (28, 4, 6, 9100), (12, 2, 4, 16001)])
 def test_few_blocks_of_a_cluster_and_many_with_a_merge(nH, nKV, batch, ctx):
@@ -428,7 +457,8 @@ def test_clusters_of_few_blocks_only_where_they_fill_the_card(nH, nKV, batch, ct
 
 
 @pytest.mark.parametrize("nH,nKV,lens", [(28, 4, (12000, 11871, 130, 5000)), (28, 4, (12000, 1, 7000, 127, 128, 129, 3000, 11999)),
-                                         (40, 8, (12000, 300)), (12, 2, (26000, 64, 25999, 128))])
+                                         (40, 8, (12000, 300)), (12, 2, (26000, 64, 25999, 128)),
+                                         (28, 4, (6000, 1, 130, 5999, 3000, 127, 128, 129, 5889, 256, 4000, 2))])
 def test_ragged_sequences_in_clusters_of_few_blocks(nH, nKV, lens):
     """Device lengths at 24 and 26 tiles per block of the longest sequence, where clusters of 2 - 8 blocks take over from the merge, and sequences
     that leave blocks of a cluster without tiles: each like a call of its own, up to the f32 roundings of another fold."""

@@ -939,10 +939,13 @@ int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, c
     // pull them when their own are in (kLateTiles), which pays up to 80 MB: 2 sequences of 40000 rows (82 MB) 135.5 / 135.7 us for eight
     // layers, 8 of 12000 (98 MB) 145.3 / 146.0.
     const uint64_t callBytes = static_cast<uint64_t>(d->batch) * d->maxLen * d->nKV * hd * 2ull;
-    const int prefetchNext = d->nextK8 == nullptr || d->nextV8 == nullptr || callBytes > (80ull << 20) ? 0 : callBytes <= (48ull << 20) ? 1 : 2;
+    // (Between 48 and 80 MB a hint that a copy could not follow is no error: those calls used to go without one.)
+    const bool nextAligned = ((reinterpret_cast<uintptr_t>(d->nextK8) | reinterpret_cast<uintptr_t>(d->nextV8)) & 15u) == 0;
+    const int prefetchNext = d->nextK8 == nullptr || d->nextV8 == nullptr || callBytes > (80ull << 20) ? 0
+                             : callBytes <= (48ull << 20)                                              ? 1
+                                                                                                       : (nextAligned ? 2 : 0);
     if (prefetchNext) {
-        TC_REQUIRE(((reinterpret_cast<uintptr_t>(d->nextK8) | reinterpret_cast<uintptr_t>(d->nextV8)) & 15u) == 0,
-                   TC_EINVAL, "decode_i8: nextK8/nextV8 need 16-byte alignment");
+        TC_REQUIRE(nextAligned, TC_EINVAL, "decode_i8: nextK8/nextV8 need 16-byte alignment");
         key.base = d->nextK8;
         rc = getTensorMap(key, &tmKn);
         if (rc != TC_OK) return rc;
