@@ -144,7 +144,7 @@ kvAppendKernel(float *__restrict__ q, const float *__restrict__ kSrc, const floa
     const uint32_t j = static_cast<uint32_t>(idx - rowIdx * perRow) * V;
     const uint32_t s = static_cast<uint32_t>(rowIdx / rowsPerToken);
     uint32_t row = static_cast<uint32_t>(rowIdx - static_cast<uint64_t>(s) * rowsPerToken);
-    const bool isQ = row < nHeads;
+    const bool isQ = row < nHeads, isFirst = row == 0;
     if (!isQ) row -= nHeads;
     const bool isV = !isQ && row >= nKV;
     if (isV) row -= nKV;
@@ -153,7 +153,7 @@ kvAppendKernel(float *__restrict__ q, const float *__restrict__ kSrc, const floa
     if (some) {
         prefetchLineOf(src + j, 4 * V);
         prefetchLineOf(src + j + pairs, 4 * V);
-        if (cosT != nullptr && devPos == nullptr && row == 0) {
+        if (cosT != nullptr && devPos == nullptr && isFirst) {  // (the token's table row once, not for q, K and V each)
             const size_t at = static_cast<size_t>(ropePos + s) * pairs + j;
             prefetchLineOf(cosT + at, 4 * V);
             prefetchLineOf(sinT + at, 4 * V);

@@ -39,7 +39,7 @@ qkNormRopeKernel(const float *__restrict__ qIn, uint32_t qInStride, float *qOut,
     const bool some = idx < static_cast<uint64_t>(seqLen) * slices;
     const uint32_t s = static_cast<uint32_t>(idx / slices);
     uint32_t h = static_cast<uint32_t>(idx % slices);
-    const bool isQ = qIn != nullptr && h < nHeads;
+    const bool isQ = qIn != nullptr && h < nHeads, isFirst = h == 0u;
     if (!isQ && qIn != nullptr) h -= nHeads;
     const float *rp = isQ ? qIn + (static_cast<uint64_t>(s) * nHeads + h) * qInStride
                           : k + (static_cast<uint64_t>(s) * nKV + h) * hd;
@@ -50,7 +50,7 @@ qkNormRopeKernel(const float *__restrict__ qIn, uint32_t qInStride, float *qOut,
             prefetchL2(rp + 32u * lane);
             if (s == 0u && h == 0u) prefetchL2(w + 32u * lane);
         }
-        if (devPos == nullptr && h == 0u && 64u * lane < nDims) {
+        if (devPos == nullptr && isFirst && 64u * lane < nDims) {  // (the token's table row once, not for q and K each)
             const uint64_t at = static_cast<uint64_t>(pos + s) * (nDims / 2) + 32u * lane;
             prefetchL2(cosT + at), prefetchL2(sinT + at);
         }
