@@ -78,10 +78,11 @@ __global__ void __launch_bounds__(NW * 32, BPS) decodeKvKernel(const __grid_cons
             prefetchTile<HD * 4>(k, v, static_cast<size_t>(p.nKV) * HD * 4, tok, p.totalRows - 1, lane);
         const size_t row = static_cast<size_t>(hg) * HD, table = static_cast<size_t>(p.lenHost - 1u) * (HD / 2);
         const bool rotates = p.tok.cosT != nullptr && p.devPos == nullptr;
-        if constexpr (HD > 64)  // (14 / 2 / 64 at 2047 rows: 5.66 us without, 5.71 with it)
-            prefetchToken<HD>(p.q + (static_cast<size_t>(hg) * p.group + p.colBase) * HD, min(8u, p.group - p.colBase),
-                              p.tok.k != nullptr ? p.tok.k + row : nullptr, p.tok.v + row, rotates ? p.tok.cosT + table : nullptr,
-                              p.tok.sinT + table, threadIdx.x);
+        // (at head_dim 64, 15 - 20000 rows in a graph, with it / without: one layer 0.97 - 1.06 of the time, mean 1.00, four 0.98 - 1.01, eight 0.98 - 1.01,
+        // mean 0.995, and 0.94 - 0.98 where the inputs are cold at half of the lengths)
+        prefetchToken<HD>(p.q + (static_cast<size_t>(hg) * p.group + p.colBase) * HD, min(8u, p.group - p.colBase),
+                          p.tok.k != nullptr ? p.tok.k + row : nullptr, p.tok.v + row, rotates ? p.tok.cosT + table : nullptr,
+                          p.tok.sinT + table, threadIdx.x);
     }
     gridDepWait();
     gridDepLaunch();
