@@ -456,6 +456,25 @@ def test_clusters_of_few_blocks_only_where_they_fill_the_card(nH, nKV, batch, ct
     assert ops.device_status() == 0
 
 
+@pytest.mark.parametrize("nH,nKV,batch,ctx", [(40, 8, 1, 15300), (28, 4, 4, 6000), (12, 2, 18, 3000)])
+def test_calls_without_partial_buffers_take_the_cluster_that_others_leave(nH, nKV, batch, ctx):
+    """... to the merge: the same result up to the f32 roundings of another fold (a tile's reference point may differ, 2^-24 a token at most)."""
+    hd = 128
+    g = torch.Generator(device="cuda").manual_seed(ctx)
+    k8, v8 = (torch.randint(-127, 128, (batch * ctx, nKV, hd), dtype=torch.int8, device="cuda", generator=g) for _ in range(2))
+    ks, vs = (0.008 + 0.02 * torch.rand((batch * ctx, nKV), device="cuda", generator=g) for _ in range(2))
+    q = torch.randn((batch, nH, hd), device="cuda", generator=g)
+    slots = min(64, ops.split_geometry(ctx, nH, hd)[1])
+    got = []
+    for ws in (ops.workspace(batch, nH, hd, slots), (None, None, None)):
+        out = torch.empty_like(q)
+        used = ops.decode_i8_batch(q, k8, v8, ks, vs, out, ws, None, batch, nH, nKV, hd, ctx, slots, rows_per_seq=ctx)
+        assert (used == 1) == (ws[0] is None)
+        got.append(out)
+    assert ops.device_status() == 0
+    assert float((got[0] - got[1]).norm() / got[0].norm()) < 4e-6
+
+
 @pytest.mark.parametrize("nH,nKV,lens", [(28, 4, (12000, 11871, 130, 5000)), (28, 4, (12000, 1, 7000, 127, 128, 129, 3000, 11999)),
                                          (40, 8, (12000, 300)), (12, 2, (26000, 64, 25999, 128)),
                                          (28, 4, (6000, 1, 130, 5999, 3000, 127, 128, 129, 5889, 256, 4000, 2))])

@@ -893,12 +893,13 @@ int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, c
     if (rc != TC_OK) return rc;
     DecodePlan pl = planDecode(d->batch, d->nKV, d->maxLen, d->numChunks, kTcTile, d->lens == nullptr, 1u);
     uint32_t cluster = 1;
+    const bool partials = d->pAcc && d->pM && d->pL;  // (without them a merge is not to be had: nine for all)
     if (pl.chunksPerSeq > 1 && !d->partialsOnly && d->mergeTickets == nullptr) {
         const uint32_t tiles = (d->maxLen + kTcTile - 1) / kTcTile;
         for (uint32_t lg = 4; lg >= 1 && cluster == 1; --lg) {
             const uint32_t n = 1u << lg;
             const bool busy = n * d->nKV * d->batch * 8u >= static_cast<uint32_t>(numSMs()) * 5u;
-            const uint32_t more = n == 16u ? 5u : (busy ? 9u : (n == 8u ? 5u : 3u));
+            const uint32_t more = n == 16u ? 5u : (busy || !partials ? 9u : (n == 8u ? 5u : 3u));
             const uint32_t most = d->lens == nullptr || d->batch == 1 ? pl.chunkTokens / kTcTile + more : n == 16u ? 20u : 26u;  // tiles per block
             if (n / 2u >= tiles || limits[lg] < d->nKV * d->batch || (tiles + n - 1u) / n > most) continue;
             cluster = n;
@@ -907,7 +908,7 @@ int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, c
     }
     const bool pdl = (d->flags & TC_DECODE_PDL) != 0;
     const bool direct = (pl.chunksPerSeq == 1 || cluster > 1) && !d->partialsOnly;
-    if (!direct) TC_REQUIRE(d->pAcc && d->pM && d->pL, TC_EWORKSPACE, "decode_i8: partial buffers are required");
+    if (!direct) TC_REQUIRE(partials, TC_EWORKSPACE, "decode_i8: partial buffers are required");
     if (d->chunksUsed) *d->chunksUsed = cluster > 1 ? 1u : pl.chunksPerSeq;  // (a cluster's blocks write no slots)
     TC_REQUIRE(d->nKV <= 65535, TC_EUNSUPPORTED, "decode_i8: %u kv heads", d->nKV);
 
