@@ -165,7 +165,10 @@ int tc_attn_decode_i8(const float *q, const int8_t *k8, const int8_t *v8,
  * sequence is exactly maxLen rows long.  q/out: [batch][nHeads][hd].
  * partialsOnly != 0 skips the merge and leaves (m, l, acc) per chunk in
  * pAcc/pM/pL -- the form a context-axis split across GPUs exchanges;
- * *chunksUsed (HOST, nullable) receives the chunk slots written per head. */
+ * *chunksUsed (HOST, nullable) receives the chunk slots written per head (1 where
+ * the call needed none).  pAcc/pM/pL may be NULL for a call that the library does
+ * without partials -- which ones is its own affair and has changed: TC_EWORKSPACE
+ * otherwise, so a caller that is not prepared for it gives them. */
 typedef struct tc_decode_i8_batch {
     const float *q;
     float *out;
@@ -203,8 +206,9 @@ typedef struct tc_decode_i8_batch {
      * the next call's block cannot request by itself while it waits -- so DRAM keeps
      * streaming while this call's blocks fold their partials and the merge runs,
      * instead of idling until the next call's blocks start.  Nothing is read or
-     * written through these pointers by the SMs.  Ignored when a call's rows
-     * (batch * maxLen * nKV * hd * 2 bytes) exceed 48 MB: they would not stay in L2. */
+     * written through these pointers by the SMs.  16-byte aligned (TC_EINVAL
+     * otherwise).  Ignored when a call's rows (batch * maxLen * nKV * hd * 2 bytes)
+     * exceed 80 MB, and from 48 MB on where it is not aligned. */
     const int8_t *nextK8, *nextV8;
     /* Optional (NULL = merge in a second launch): batch * nKV arrival counters in DEVICE memory,
      * zero before the first call (the kernel leaves them zero).  With them the split-KV kernel
@@ -259,7 +263,11 @@ int tc_attn_decode_i8_noalloc(const float *q, const int8_t *k8, const int8_t *v8
  * so a launch captured in a CUDA graph and replayed at growing positions passes
  * the last position of the window (maxSeqLen - 1), as the reference's *Pos
  * launch covers its whole attnChunk x attnChunks grid.  Rows past a bound that
- * was too small are not attended. */
+ * was too small are not attended.
+ * pAcc/pM/pL hold numChunks chunk slots per head.  Without them (any of the three
+ * NULL) a call of seqLen 1 keeps to one cluster of blocks per kv head, slower for
+ * long rows and with longer f32 sums (72 products at 9000 rows of 8 / 2 / 128); with q81Out they are needed
+ * (TC_EWORKSPACE otherwise). */
 int tc_attn_decode_kv(const float *q, const void *kvK, const void *kvV,
                       float *attnOut, float *pAcc, float *pM, float *pL,
                       uint32_t seqLen, uint32_t nHeads, uint32_t nKV, uint32_t hd,
@@ -391,7 +399,10 @@ int tc_attn_prefill_f16_i8(const float *q, const int8_t *k8, const int8_t *v8,
 /* Replaces kWarpAttention / kWarpAttentionPos and kQ35WarpAttention
  * (include/gpu/GpuAttentionKernels.hpp:211-272, 537-599;
  * include/gpu/GpuQwen35Kernels.hpp:2437-2492): causal attention of seqLen query
- * rows, row s over cache rows [0, cachePos + s], f32 or fp16 cache, f32 math. */
+ * rows, row s over cache rows [0, cachePos + s], f32 or fp16 cache, f32 math:
+ * every factor is held to 21 bits and more, and what is large in one row or dim of
+ * an f32 cache takes nothing from another (a 2^-51 of the largest of some rows at
+ * most; numbers further apart than 2^29 are worked on in f32, several times slower). */
 int tc_attn_prefill_kv(const float *q, const void *kvK, const void *kvV,
                        float *out, uint32_t seqLen, uint32_t nHeads,
                        uint32_t nKV, uint32_t hd, uint32_t cachePos,

@@ -409,9 +409,11 @@ decodeI8TcKernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         // earlier they sit in front of this block's own tiles in the queue: 10.2 against 9.1 us)
         // -- and a block of many tiles waits until its last one is in: HBM is what bounds it, and would be idle from there to the
         // next call's first requests, some 3 us.  That is room for four tiles a block.  Requested with its own last ring they
-        // held that up by as much as they gained.  28 / 4 heads, eight layers, two tiles with the last ring (none above 48 MB a call) ->
-        // four behind it: 8 sequences of 8192 rows (16 tiles a block) 114.0 -> 111.0 us, 16 of 4000 114.3 -> 109.1, 32 of 2000
-        // 107.4 -> 103.9, 2 of 30000 115.0 -> 109.4, 1 of 80000 145.7 -> 140.3.  Below that blocks are bound by latency, and what comes
+        // held that up by as much as they gained.  28 / 4 heads, per layer of calls above 48 MB, none -> four tiles behind the last, two / four / eight
+        // layers of pools in turn, dependent launches: 8 sequences of 8192 rows (16 tiles a block) 14.1 / 14.2 / 14.5 -> 13.3 / 13.9 / 14.3 us, 16 of 4000
+        // 13.5 / 14.1 / 14.5 -> 12.8 / 13.4 / 14.05, 2 of 30000 13.4 / 14.1 / 14.6 -> 12.9 / 13.3 / 13.9, 1 of 80000 16.9 / 17.6 / 17.9 -> 16.1 / 16.9 / 17.5; in
+        // plain stream order 1 - 3 % of two and 2 - 4 % of eight layers, while four (L2 twice over) lose 2 - 5 %.  Eight layers of 8 x 8192 with
+        // their session around them: 117.5 -> 116.4 us.  In blocks of fewer tiles, bound by latency, what comes
         // late comes too late: 2 of 22000 (10 tiles) 91.9 -> 95.1, 8 of 6000 (12 tiles) 87.5 -> 88.2.
         if (p.prefetchNext == 1 || (p.prefetchNext != 0 && nTiles > kLateTiles)) {
             const uint32_t last = nTiles - 1u;
@@ -937,8 +939,8 @@ int decodeI8Tc(const tc_decode_i8_batch *d, uint32_t lenHost, uint32_t lenAdd, c
     // against without it, per layer of pools that do not fit L2 together: 20000 rows 8.70 / 9.25 us, 32768 rows 10.90 /
     // 10.98, 47000 rows (46 MiB) 14.04 / 13.55, 50000 rows 14.25 / 14.02, 80000 rows 18.13 / 18.46; 4 sequences of 8192 rows
     // 12.2 / 11.7, 8 of 8192 14.24 / 14.60.  It pays where a call is short; from some 30 MB on it is within 4 % either way.)  Blocks of many tiles
-    // pull them when their own are in (kLateTiles), which pays up to 80 MB: 2 sequences of 40000 rows (82 MB) 135.5 / 135.7 us for eight
-    // layers, 8 of 12000 (98 MB) 145.3 / 146.0.
+    // pull them when their own are in (kLateTiles), which pays up to 80 MB: 2 sequences of 40000 rows (82 MB) 17.1 / 17.0 us a layer of eight,
+    // 8 of 12000 (98 MB) 18.2 / 18.25.
     const uint64_t callBytes = static_cast<uint64_t>(d->batch) * d->maxLen * d->nKV * hd * 2ull;
     // (Between 48 and 80 MB a hint that a copy could not follow is no error: those calls used to go without one.)
     const bool nextAligned = ((reinterpret_cast<uintptr_t>(d->nextK8) | reinterpret_cast<uintptr_t>(d->nextV8)) & 15u) == 0;

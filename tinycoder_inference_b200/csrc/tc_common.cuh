@@ -95,7 +95,7 @@ int launchDependent(void (*kern)(P...), dim3 grid, uint32_t threads, size_t smem
 // What a kernel is handed -- q, new rows, gates, rotation tables -- towards L2 ahead of its dependency wait: where DRAM still holds
 // it, a chain of short launches waited for it at each of them.  Right at any time: it is a hint, and what a kernel in flight
 // still writes is read after the wait.  (Each line once: the norm weights asked for by every warp of a 333-row launch cost 6 us.)
-// Eight layers of 16 / 2 / 256 behind 16383 int8 rows, norm and gate included, 121.7 -> 115.8 us; four of 28 / 4 / 128 behind 8191 fp16
+// Eight layers of 16 / 2 / 256 behind 16383 int8 rows, norm and gate included, 140.0 -> 134.2 us (as a graph 121.7 -> 115.8); four of 28 / 4 / 128 behind 8191 fp16
 // rows 30.0 -> 29.5; four of a 333-row prompt of 16 / 2 / 256 101.3 -> 96.8.
 __device__ __forceinline__ void prefetchL2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 // (`bytes` and the address multiples of 16)
