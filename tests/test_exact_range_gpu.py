@@ -113,3 +113,17 @@ def test_a_large_row_of_v_weighs_what_its_probability_is(scale, S, nH, nKV, hd, 
     k[pos + 34, :, 0] = -(scale + 45.0) * math.log(2.0) * math.sqrt(hd)
     out, want = _run(q, k, v, pos)
     assert _far(out, want) < FAR
+
+
+@pytest.mark.parametrize("past", [0, 5, 1000])
+@pytest.mark.parametrize("S,nH,nKV,hd,rows", [(64, 40, 4, 64, 150), (64, 48, 8, 128, 77), (64, 64, 4, 256, 65)])
+def test_a_device_position_past_the_store_attends_the_rows_there_are(past, S, nH, nKV, hd, rows):
+    """The last stage is filled up with rows that nobody sees, also where the position on the device says that somebody does."""
+    q, k, v = _inputs(S, nH, nKV, hd, rows - S)
+    out = torch.full_like(q, float("nan"))
+    at = torch.tensor([rows + past], dtype=torch.int32, device="cuda")
+    ops.prefill_kv(q, k, v, out, S, nH, nKV, hd, 0, dev_pos=at)
+    for h in range(nH):
+        kv = h * nKV // nH
+        want = torch.softmax(q[:, h].double() @ k[:, kv].double().T / math.sqrt(hd), -1) @ v[:, kv].double()
+        assert _far(out[:, h], want) < FAR

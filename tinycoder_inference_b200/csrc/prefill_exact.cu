@@ -350,8 +350,8 @@ __global__ void __launch_bounds__(ExactShape<HD>::kThreads, 1) prefillExactKerne
 #pragma unroll
     for (int i = 0; i < HD / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
     float m0 = kNegBig, m1 = kNegBig, l0 = 0.0f, l1 = 0.0f;
-    // this thread's query rows (g and g + 8 of the warp's tile) see tokens below:
-    const uint32_t lim0 = pos0 + row0 + rt * 16u + g + 1u, lim1 = lim0 + 8u;
+    // this thread's query rows (g and g + 8 of the warp's tile) see tokens below (with a device position past the store, the rows there are):
+    const uint32_t lim0 = min(len, pos0 + row0 + rt * 16u + g + 1u), lim1 = min(len, pos0 + row0 + rt * 16u + g + 9u);
     const uint32_t warpLimit = min(len, pos0 + row0 + rt * 16u + 16u);  // no row of the warp's tile sees further
 
     // ldmatrix: lane i delivers row i % 8 of 8x8 block i / 8
